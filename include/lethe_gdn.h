@@ -112,6 +112,12 @@ typedef struct LetheGdnArgs {
   /* No counterpart in the reference.                                                                          */
   uint32_t c_begin;
   uint32_t c_count;
+  /* Sequences that do not fill their last chunk, and 64 key channels (delta 0 or 1).  dims.L stays a multiple of  */
+  /* 64 and dims.K 128 (they size the workspaces); l_tokens in (dims.L - 64, dims.L] and k_channels = 64 say how   */
+  /* many tokens and key channels the tensors really have, in the same layouts ([B, l_tokens, H, k_channels] ...,  */
+  /* states [B, H, k_channels, V]).  The rest counts as zero and is neither read nor written.  0: all of dims.     */
+  uint32_t l_tokens;
+  uint32_t k_channels;
 } LetheGdnArgs;
 
 /* Bytes of the forward->backward workspace / of the backward scratch for these sizes (0 = bad dims). */
@@ -164,6 +170,7 @@ typedef struct LetheGdnDecodeArgs {
   const float* beta;
   float* state;
   void* o;
+  uint32_t in_f32;   /* non-zero: q, k, v are fp32; each value is rounded to bf16 as it is read */
 } LetheGdnDecodeArgs;
 int lethe_gdn_decode_step(const LetheGdnDecodeArgs* args, void* cuda_stream);
 
@@ -173,6 +180,7 @@ int lethe_gdn_decode_step(const LetheGdnDecodeArgs* args, void* cuda_stream);
  * src/lethe/kernels/references/gdn2_assemble.py:300-312):
  *   y = x * rsqrt(sum_d x_d^2 + eps);      dx = r (dy - y (y . dy)),  r = rsqrt(sum_d x_d^2 + eps).
  * flags: LETHE_L2_IN_F32  - q, k (and the returned dq, dk) are fp32 instead of bf16;
+ *        LETHE_L2_IN_F16  - ... fp16 (at most one of the two);
  *        LETHE_L2_NORM_F16 - the normalised rows qn, kn and their gradients dqn, dkn are fp16 instead
  *                            of bf16 (pair it with LetheGdnArgs::qk_f16 on the forward / backward
  *                            calls: the rows are then rounded once, to the operand type).
@@ -180,11 +188,28 @@ int lethe_gdn_decode_step(const LetheGdnDecodeArgs* args, void* cuda_stream);
  * qn, kn: 16-bit [rows, D], the tensors lethe_gdn_forward / lethe_gdn_backward then read.
  * dqn, dkn: 16-bit [rows, D], the dq / dk lethe_gdn_backward wrote; dq, dk: [rows, D] in the type of
  * q, k (may alias dqn, dkn when both are bf16).  One launch each; every pointer 16-byte aligned. */
-enum { LETHE_L2_IN_F32 = 1, LETHE_L2_NORM_F16 = 2 };
+enum { LETHE_L2_IN_F32 = 1, LETHE_L2_NORM_F16 = 2, LETHE_L2_IN_F16 = 4 };
 int lethe_gdn_l2norm_qk(const void* q, const void* k, void* qn, void* kn, int64_t rows, int32_t D,
                         int32_t flags, float eps, void* cuda_stream);
 int lethe_gdn_l2norm_qk_vjp(const void* q, const void* k, const void* dqn, const void* dkn, void* dq, void* dk,
                             int64_t rows, int32_t D, int32_t flags, float eps, void* cuda_stream);
+
+/* The six-input surface of the reference (gdn_layer.py:99-111) takes every gate per channel: g, b [rows, K], w
+ * [rows, V], fp32, rows = B L H.  lethe_gdn_gate_regime decides which kernels such a call needs, as the reference
+ * does (cute/gdn2_backward.py:53-60), by bitwise comparison along the channels, and compacts what those kernels read:
+ *   *flags (4-byte device or mapped host word) = LETHE_REGIME_DONE | the tests that hold:
+ *     SCALAR_GATE  g is one value per row;   ONE_BETA  b and w are the same one value per row;
+ *     NO_DELTA     b is 0 and w is 1 everywhere;
+ *   g0 [rows], b0 [rows]: g[:, 0] and b[:, 0], complete when one of the tests that use them holds.
+ * work: 8 bytes of device memory, zero before the call and again after it.
+ * lethe_gdn_gate_spread is the other direction: gradients per row spread evenly over the channels, as the reference's
+ * scalar assembly does (gdn2_assemble.py:343-345): dg[r, :] = dg0[r] / K, db[r, :] = db0[r] / K, dw[r, :] = dw0[r] / V.
+ * A null output is not wanted, a null source counts as zero. */
+enum { LETHE_REGIME_SCALAR_GATE = 1, LETHE_REGIME_ONE_BETA = 2, LETHE_REGIME_NO_DELTA = 4, LETHE_REGIME_DONE = 8 };
+int lethe_gdn_gate_regime(const float* g, const float* b, const float* w, int64_t rows, int32_t K, int32_t V,
+                          float* g0, float* b0, uint32_t* flags, uint32_t* work, void* cuda_stream);
+int lethe_gdn_gate_spread(const float* dg0, const float* db0, const float* dw0, int64_t rows, int32_t K, int32_t V,
+                          float* dg, float* db, float* dw, void* cuda_stream);
 
 /* Text for a return code of the calls above or for a device status code. */
 const char* lethe_gdn_strerror(int code);

@@ -29,12 +29,13 @@ static bool dims_ok(const LetheGdnDims& d) {
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-// Tensor map of a token-major [B, L, H, D] 16-bit tensor; one box = 64 tokens x 64 channels of one head.
-static int token_map(CUtensorMap* m, const void* ptr, const LetheGdnDims& d, int D) {
-  uint64_t dims[4] = {static_cast<uint64_t>(D), static_cast<uint64_t>(d.H), static_cast<uint64_t>(d.L),
-                      static_cast<uint64_t>(d.B)};
-  uint64_t str[3] = {static_cast<uint64_t>(D) * 2, static_cast<uint64_t>(d.H) * D * 2,
-                     static_cast<uint64_t>(d.L) * d.H * D * 2};
+// Tensor map of a token-major [B, L, H, D] 16-bit tensor; one box = 64 tokens x 64 channels of one head.  L and D are
+// the tensor's own: what a box covers beyond them reads as zero and is not stored.
+static int token_map(CUtensorMap* m, const void* ptr, const Problem& p, int D) {
+  uint64_t dims[4] = {static_cast<uint64_t>(D), static_cast<uint64_t>(p.H), static_cast<uint64_t>(p.L),
+                      static_cast<uint64_t>(p.B)};
+  uint64_t str[3] = {static_cast<uint64_t>(D) * 2, static_cast<uint64_t>(p.H) * D * 2,
+                     static_cast<uint64_t>(p.L) * p.H * D * 2};
   uint32_t box[4] = {64, 1, 64, 1};
   return make_tmap_16bit(m, ptr, 4, dims, str, box);
 }
@@ -63,7 +64,12 @@ static int fill_problem(const LetheGdnArgs* a, Problem* p, bool backward) {
   if (backward && a->scratch_bytes < lay.scratch_total) return kErrWorkspace;
   if (!aligned16(a->saved) || (reinterpret_cast<uintptr_t>(a->saved) & 1023u)) return kErrAlign;
   if (backward && (reinterpret_cast<uintptr_t>(a->scratch) & 1023u)) return kErrAlign;
-  p->B = d.B; p->H = d.H; p->L = d.L; p->NT = d.L / kC; p->V = d.V; p->gate = d.gate; p->delta = d.delta ? 1 : 0;
+  p->B = d.B; p->H = d.H; p->NT = d.L / kC;
+  p->L = a->l_tokens ? static_cast<int>(a->l_tokens) : d.L;
+  p->Kr = a->k_channels ? static_cast<int>(a->k_channels) : kK;
+  if (p->L > d.L || p->L <= d.L - kC || (p->Kr != 64 && p->Kr != kK)) return kErrDims;
+  if (d.delta == 2 && (p->L != d.L || p->Kr != kK)) return kErrFlags;
+  p->V = d.V; p->gate = d.gate; p->delta = d.delta ? 1 : 0;
   if (a->bh_count == 0) {
     if (a->bh_begin != 0) return kErrDims;
     p->bh0 = 0;
@@ -127,9 +133,9 @@ extern "C" int lethe_gdn_forward(const LetheGdnArgs* a, void* stream) {
   if (!guard.ok) return kErrDevice;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   CUtensorMap mq, mk, mv;
-  if ((e = token_map(&mq, a->q, a->dims, kK))) return e;
-  if ((e = token_map(&mk, a->k, a->dims, kK))) return e;
-  if ((e = token_map(&mv, a->v, a->dims, a->dims.V))) return e;
+  if ((e = token_map(&mq, a->q, p, p.Kr))) return e;
+  if ((e = token_map(&mk, a->k, p, p.Kr))) return e;
+  if ((e = token_map(&mv, a->v, p, p.V))) return e;
   const uint32_t m = a->kernel_mask ? a->kernel_mask : 7u;
   if ((m & 1u) && (e = (p.gate == LETHE_GATE_CHANNEL ? launch_prepare_cw(p, mq, mk, mv, st)
                                                      : launch_prepare(p, mq, mk, mv, st)))) return e;
@@ -147,10 +153,10 @@ extern "C" int lethe_gdn_backward(const LetheGdnArgs* a, void* stream) {
   if (!guard.ok) return kErrDevice;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   CUtensorMap mq, mk, mv, mdo;
-  if ((e = token_map(&mq, a->q, a->dims, kK))) return e;
-  if ((e = token_map(&mk, a->k, a->dims, kK))) return e;
-  if ((e = token_map(&mv, a->v, a->dims, a->dims.V))) return e;
-  if ((e = token_map(&mdo, a->d_o, a->dims, a->dims.V))) return e;
+  if ((e = token_map(&mq, a->q, p, p.Kr))) return e;
+  if ((e = token_map(&mk, a->k, p, p.Kr))) return e;
+  if ((e = token_map(&mv, a->v, p, p.V))) return e;
+  if ((e = token_map(&mdo, a->d_o, p, p.V))) return e;
   const uint32_t m = a->kernel_mask ? a->kernel_mask : 15u;
   if ((m & 1u) && (e = launch_bwd_pre(p, mq, mdo, st))) return e;
   if ((m & 2u) && (e = launch_scan(p, true, st))) return e;
@@ -159,9 +165,9 @@ extern "C" int lethe_gdn_backward(const LetheGdnArgs* a, void* stream) {
       if ((e = launch_bwd_main_cw(p, mq, mk, mv, mdo, st, m))) return e;
     } else {
       OutMaps mo;
-      if ((e = token_map(&mo.dq, a->dq, a->dims, kK))) return e;
-      if ((e = token_map(&mo.dk, a->dk, a->dims, kK))) return e;
-      if ((e = token_map(&mo.dv, a->dv, a->dims, a->dims.V))) return e;
+      if ((e = token_map(&mo.dq, a->dq, p, p.Kr))) return e;
+      if ((e = token_map(&mo.dk, a->dk, p, p.Kr))) return e;
+      if ((e = token_map(&mo.dv, a->dv, p, p.V))) return e;
       if ((e = launch_bwd_main(p, mq, mk, mv, mdo, mo, st, m))) return e;
     }
   }

@@ -63,7 +63,7 @@ bwd_pre_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
     tmem_relinquish();
   }
   float gval = 0.f;
-  if (tid < 64 && p.gate == LETHE_GATE_SCALAR) gval = p.g[(static_cast<size_t>(b) * p.L + c * kC + tid) * p.H + h];
+  if (tid < p.rows_of(c) && p.gate == LETHE_GATE_SCALAR) gval = p.g[(static_cast<size_t>(b) * p.L + c * kC + tid) * p.H + h];
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -224,7 +224,7 @@ bwd_stageb_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
   }
   const size_t tok0 = (static_cast<size_t>(b) * p.L + c * kC) * p.H + h;   // token index of row 0 (stride H)
   float gval = 0.f;
-  if (tid < 64 && p.gate == LETHE_GATE_SCALAR) gval = p.g[tok0 + static_cast<size_t>(tid) * p.H];
+  if (tid < p.rows_of(c) && p.gate == LETHE_GATE_SCALAR) gval = p.g[tok0 + static_cast<size_t>(tid) * p.H];
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -316,7 +316,7 @@ bwd_stageb_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
         }
         const uint4 pk = pack8_f16(d + 8 * i);
         tile_st_chunk(DD, 64 + r, jb * 4 + i, 128, pk);
-        if (!DELTA) *reinterpret_cast<uint4*>(dv_g + jb * 32 + 8 * i) = pack8_bf16(d + 8 * i);
+        if (!DELTA && r < p.rows_of(c)) *reinterpret_cast<uint4*>(dv_g + jb * 32 + 8 * i) = pack8_bf16(d + 8 * i);
       }
     }
     t3p[half * 64 + r] = t3 + dde;
@@ -419,7 +419,7 @@ bwd_stageb_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
     }
     umma_commit_led(leader, bar_mma);
     if (tid == 0) {
-      for (int a = 0; a < 2; ++a) tma_store_4d(&mdq, SQ + a * 8192, a * 64, h, c * kC, b);
+      for (int a = 0; a < p.Kr / 64; ++a) tma_store_4d(&mdq, SQ + a * 8192, a * 64, h, c * kC, b);
       if (DELTA) bulk_s2g(p.scratch + p.lay.dw + static_cast<size_t>(z) * p.lay.sz_dw, SW, 16384);
       bulk_commit();
     }
@@ -458,7 +458,7 @@ bwd_stageb_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
     if (DELTA) {
       bulk_s2g(p.scratch + p.lay.dkb + static_cast<size_t>(z) * p.lay.sz_dkb, SK, 32768);
     } else {
-      for (int a = 0; a < 2; ++a) tma_store_4d(&mdk, SK + a * 8192, a * 64, h, c * kC, b);
+      for (int a = 0; a < p.Kr / 64; ++a) tma_store_4d(&mdk, SK + a * 8192, a * 64, h, c * kC, b);
     }
     bulk_commit();
   }
@@ -478,7 +478,7 @@ bwd_stageb_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
   }
   if (!DELTA) {
     const float acc = chunk_rev_cumsum(dG, tid, tmp);
-    if (tid < 64 && p.gate == LETHE_GATE_SCALAR) p.dg[tok0 + static_cast<size_t>(tid) * p.H] = acc;
+    if (tid < p.rows_of(c) && p.gate == LETHE_GATE_SCALAR) p.dg[tok0 + static_cast<size_t>(tid) * p.H] = acc;
   }
   if (tid == 0) bulk_wait_read();
   tc_fence_before();

@@ -71,7 +71,7 @@ bwd_wy2_kernel(const Problem p, const __grid_constant__ CUtensorMap mk, const __
   }
   const size_t tok0 = (static_cast<size_t>(b) * p.L + c * kC) * p.H + h;
   float gval = 0.f, bval = 0.f, dgb = 0.f;
-  if (tid < 64) {
+  if (tid < p.rows_of(c)) {
     if (p.gate == LETHE_GATE_SCALAR) gval = p.g[tok0 + static_cast<size_t>(tid) * p.H];
     bval = p.beta[tok0 + static_cast<size_t>(tid) * p.H];
   }
@@ -316,7 +316,7 @@ bwd_wy2_kernel(const Problem p, const __grid_constant__ CUtensorMap mk, const __
   fence_proxy_async();
   __syncthreads();
   if (tid == 0) {
-    for (int a = 0; a < 2; ++a) tma_store_4d(&mdk, SKo + a * 8192, a * 64, h, c * kC, b);
+    for (int a = 0; a < p.Kr / 64; ++a) tma_store_4d(&mdk, SKo + a * 8192, a * 64, h, c * kC, b);
     for (int a = 0; a < V / 64; ++a) tma_store_4d(&mdv, SV + a * 8192, a * 64, h, c * kC, b);
     bulk_commit();
   }
@@ -329,7 +329,8 @@ bwd_wy2_kernel(const Problem p, const __grid_constant__ CUtensorMap mk, const __
     const float rse = prt[2 * 64 + r] + prt[7 * 64 + r];
     const float cse = prt[3 * 64 + r] + prt[8 * 64 + r];
     const float rvs = prt[4 * 64 + r] + prt[9 * 64 + r];
-    if (p.dbeta_w) {
+    if (r >= p.rows_of(c)) {
+    } else if (p.dbeta_w) {
       p.dbeta_w[tok0 + static_cast<size_t>(r) * p.H] = rvs;
       p.dbeta[tok0 + static_cast<size_t>(r) * p.H] = gam * pks + dbm;
     } else {
@@ -339,7 +340,7 @@ bwd_wy2_kernel(const Problem p, const __grid_constant__ CUtensorMap mk, const __
   }
   {
     const float acc = chunk_rev_cumsum(dgv, tid, tmp);
-    if (tid < 64 && p.gate == LETHE_GATE_SCALAR) p.dg[tok0 + static_cast<size_t>(tid) * p.H] = acc;
+    if (tid < p.rows_of(c) && p.gate == LETHE_GATE_SCALAR) p.dg[tok0 + static_cast<size_t>(tid) * p.H] = acc;
   }
   if (tid == 0) bulk_wait_read();
   tc_fence_before();

@@ -98,7 +98,8 @@ __host__ inline Layout make_layout(const LetheGdnDims& d) {
 
 // Everything a kernel needs besides its tensor maps.
 struct Problem {
-  int B, H, L, NT, V, gate, delta;
+  int B, H, L, NT, V, gate, delta;   // L: tokens of the user tensors (the last chunk may be partly filled)
+  int Kr;            // key channels of the user tensors (64 or 128); the kernels work on 128, missing ones are zero
   int bh0, nbh;      // the (batch, head) pairs this call works on: [bh0, bh0 + nbh) of the B * H pairs
   int c0, cn;        // the chunks of every pair this call works on: [c0, c0 + cn) of the NT chunks
   int qk16;          // non-zero: q, k, dq, dk hold fp16 instead of bf16
@@ -114,6 +115,11 @@ struct Problem {
   unsigned char* scratch;
   Layout lay;
   int* status;
+
+  // rows of chunk c that hold tokens (all kC but for the last chunk of a ragged sequence).  The tensor maps end at
+  // the real token and channel counts, so the missing rows and channels of every tile read as zero and are not stored;
+  // a kernel that goes to memory by itself tests the row.  A row with k = v = q = 0, g = 0, beta = 0 leaves the state alone.
+  __device__ __forceinline__ int rows_of(int c) const { return min(kC, L - c * kC); }
 };
 
 // ---------------------------------------------------------------------------------------------

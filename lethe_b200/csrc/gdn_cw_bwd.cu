@@ -200,7 +200,7 @@ bwd_cw_sb1_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
         const uint4 pk = pack8_f16(d + 8 * i);
         tile_st_chunk(DD, 64 + r, jb * 4 + i, 128, pk);
         if (DELTA) *reinterpret_cast<uint4*>(dv2_g + sw128_chunk(r, jb * 4 + i, 64)) = pk;
-        else *reinterpret_cast<uint4*>(dv_g + jb * 32 + 8 * i) = pack8_bf16(d + 8 * i);
+        else if (r < p.rows_of(c)) *reinterpret_cast<uint4*>(dv_g + jb * 32 + 8 * i) = pack8_bf16(d + 8 * i);
       }
     }
   } else if (tid < 64) {
@@ -364,7 +364,8 @@ bwd_cw_wy1_kernel(const Problem p, const __grid_constant__ CUtensorMap mk, const
   const size_t tok0 = (static_cast<size_t>(b) * p.L + c * kC) * p.H + h;
   // full op (per-channel erase gate b, write gate w): the gates enter element by element, beta is one
   const bool full = p.bch != nullptr;
-  if (tid < 64) betas[tid] = full ? 1.f : p.beta[tok0 + static_cast<size_t>(tid) * p.H];
+  const int rows = p.rows_of(c);
+  if (tid < 64) betas[tid] = full ? 1.f : (tid < rows ? p.beta[tok0 + static_cast<size_t>(tid) * p.H] : 0.f);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -506,7 +507,7 @@ bwd_cw_wy1_kernel(const Problem p, const __grid_constant__ CUtensorMap mk, const
             o8[e] = bval * d[8 * i + e];
           }
         }
-        *reinterpret_cast<uint4*>(dv_g + jb * 32 + 8 * i) = pack8_bf16(o8);
+        if (r < rows) *reinterpret_cast<uint4*>(dv_g + jb * 32 + 8 * i) = pack8_bf16(o8);
       }
     }
     // d(beta gamma k) = T^T dw: fp32 -> record; its direct part of the erase-gate gradient,
@@ -541,7 +542,7 @@ bwd_cw_wy1_kernel(const Problem p, const __grid_constant__ CUtensorMap mk, const
     bulk_s2g(p.scratch + p.lay.dqp + static_cast<size_t>(z) * (kC * kK * 4), DQs, kC * kK * 4);
     bulk_commit();
   }
-  if (owner && half == 0 && !full) {
+  if (owner && half == 0 && !full && r < rows) {
     rv += part[r];
     pq += part[64 + r];
     if (p.dbeta_w) {
@@ -618,7 +619,9 @@ bwd_cw_pair_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, cons
   }
   const size_t tok0 = (static_cast<size_t>(b) * p.L + c * kC) * p.H + h;
   const bool full = (MODE == 1) && p.bch != nullptr;    // per-channel erase gate: x = b k element by element
-  if (tid < 64) betas[tid] = (MODE == 1 && !full) ? p.beta[tok0 + static_cast<size_t>(tid) * p.H] : 1.f;
+  const int rows = p.rows_of(c);
+  if (tid < 64)
+    betas[tid] = (MODE == 1 && !full) ? (tid < rows ? p.beta[tok0 + static_cast<size_t>(tid) * p.H] : 0.f) : 1.f;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -821,7 +824,7 @@ bwd_cw_pair_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, cons
     }
   }
   __syncthreads();
-  if (MODE == 1 && !full && tid < 64)      // sum_d d(bk)_m k
+  if (MODE == 1 && !full && tid < rows)    // sum_d d(bk)_m k
     p.dbeta[tok0 + static_cast<size_t>(tid) * p.H] += (red[tid] + red[64 + tid]) + (red[128 + tid] + red[192 + tid]);
   // ---- phase B: every (row, group of four channels) combines the two sums with the fp32 records: the dq / dk
   // parts from their shared-memory copies, the gate-gradient part from global memory.  A warp covers one row
@@ -851,7 +854,8 @@ bwd_cw_pair_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, cons
       ex_ld4(EX2, i, c4, o2);
       unpack4_f16(*reinterpret_cast<const uint2*>(KX + sw128_chunk(i, c4 >> 1, 128) + (c4 & 1) * 8), kv);
       unpack4_f16(*reinterpret_cast<const uint2*>(KX + sw128_chunk(64 + i, c4 >> 1, 128) + (c4 & 1) * 8), xv);
-      const size_t tok = (tok0 + static_cast<size_t>(i) * p.H) * kK + d0;
+      const size_t tok = (tok0 + static_cast<size_t>(i) * p.H) * p.Kr + d0;
+      const bool out = i < rows && d0 < p.Kr;
       float dk[4], dG[4];
       if (MODE == 0) {
         float dq[4];
@@ -861,7 +865,7 @@ bwd_cw_pair_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, cons
           dk[e] = dkb[e] + o2[e];
           dG[e] = dgb[e] + xv[e] * o1[e] - kv[e] * o2[e];          // q~ . dq_intra - k . dk_intra (the scale sits in C)
         }
-        store_out16x4(p.dq + tok, dq, p.qk16);
+        if (out) store_out16x4(p.dq + tok, dq, p.qk16);
       } else {
         const float4 g4 = gt4(Gt, i, d0);
         const float gg[4] = {g4.x, g4.y, g4.z, g4.w};
@@ -883,8 +887,9 @@ bwd_cw_pair_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, cons
         }
         if (full) *reinterpret_cast<float4*>(p.dbch + tok) = make_float4(dbkk[0], dbkk[1], dbkk[2], dbkk[3]);
       }
-      if (kFinalK) store_out16x4(p.dk + tok, dk, p.qk16);
-      else *reinterpret_cast<float4*>(dkb_g + ridx(i, d0)) = make_float4(dk[0], dk[1], dk[2], dk[3]);
+      if (kFinalK) {
+        if (out) store_out16x4(p.dk + tok, dk, p.qk16);
+      } else *reinterpret_cast<float4*>(dkb_g + ridx(i, d0)) = make_float4(dk[0], dk[1], dk[2], dk[3]);
       if (FINAL_G) ex_st4(EX1, i, c4, dG);                         // closed below by the reverse cumulative sum
       else *reinterpret_cast<float4*>(dgb_g + ridx(i, d0)) = make_float4(dG[0], dG[1], dG[2], dG[3]);
     }
@@ -905,7 +910,8 @@ bwd_cw_pair_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, cons
     float below = 0.f;
     for (int g2 = 3; g2 > grp; --g2) below += Cd[g2 * kK + d];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) p.dg[(tok0 + static_cast<size_t>(grp * 16 + j) * p.H) * kK + d] = v[j] + below;
+    for (int j = 0; j < 16; ++j)
+      if (grp * 16 + j < rows && d < p.Kr) p.dg[(tok0 + static_cast<size_t>(grp * 16 + j) * p.H) * p.Kr + d] = v[j] + below;
   }
   tc_fence_before();
   __syncthreads();

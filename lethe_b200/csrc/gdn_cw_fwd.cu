@@ -71,15 +71,17 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq,
   }
   const size_t tok0 = (static_cast<size_t>(b) * p.L + c * kC) * p.H + h;
   const int seg = tid >> 7;
+  const int rows = p.rows_of(c);
   float x[kGateRows];
 #pragma unroll
   for (int i = 0; i < kGateRows; ++i)
-    x[i] = p.g[(tok0 + static_cast<size_t>(seg * kGateRows + i) * p.H) * kK + (tid & 127)];
+    x[i] = (seg * kGateRows + i < rows && (tid & 127) < p.Kr)
+               ? p.g[(tok0 + static_cast<size_t>(seg * kGateRows + i) * p.H) * p.Kr + (tid & 127)] : 0.f;
   // full op (per-channel erase gate b, write gate w): the gates enter the operand tiles element by
   // element and the per-row beta is one
   const bool full = p.bch != nullptr;
   float beta_r = 1.f;
-  if (DELTA && tid < 64 && !full) beta_r = p.beta[tok0 + static_cast<size_t>(tid) * p.H];
+  if (DELTA && tid < rows && !full) beta_r = p.beta[tok0 + static_cast<size_t>(tid) * p.H];
   if (warp == 0) {
     tmem_alloc(&cs->tmem_slot, 256);
     tmem_relinquish();

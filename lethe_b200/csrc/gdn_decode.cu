@@ -21,7 +21,7 @@ constexpr int kDK = 128;
 struct DecodeProblem {
   int BH, H, V, gate, delta;
   float scale;
-  const __nv_bfloat16 *q, *k, *v;
+  const void *q, *k, *v;      // bf16, or fp32 (rounded to bf16 as read)
   const float *g, *beta;
   float* state;
   __nv_bfloat16* o;
@@ -30,14 +30,20 @@ struct DecodeProblem {
 // kSplit threads share a column of S (kDK / kSplit rows each).
 constexpr int kSplit = 4;
 
-template <int V>
+template <bool F32>
+__device__ __forceinline__ float token_in(const void* x, size_t i) {
+  if (F32) return __bfloat162float(__float2bfloat16_rn(static_cast<const float*>(x)[i]));
+  return __bfloat162float(static_cast<const __nv_bfloat16*>(x)[i]);
+}
+
+template <int V, bool F32>
 __global__ void __launch_bounds__(kSplit * V, 1024 / (kSplit * V))
 decode_step_kernel(const DecodeProblem p) {
   __shared__ float ks[kDK], qs[kDK], as[kDK], part[kSplit][V];
   const int bh = blockIdx.x, c = threadIdx.x % V, part_id = threadIdx.x / V;   // rows [kRows part_id, + kRows)
   for (int d = threadIdx.x; d < kDK; d += kSplit * V) {
-    ks[d] = __bfloat162float(p.k[static_cast<size_t>(bh) * kDK + d]);
-    qs[d] = p.scale * __bfloat162float(p.q[static_cast<size_t>(bh) * kDK + d]);
+    ks[d] = token_in<F32>(p.k, static_cast<size_t>(bh) * kDK + d);
+    qs[d] = p.scale * token_in<F32>(p.q, static_cast<size_t>(bh) * kDK + d);
     float a = 1.f;
     if (p.gate == LETHE_GATE_SCALAR) a = __expf(p.g[bh]);
     else if (p.gate == LETHE_GATE_CHANNEL) a = __expf(p.g[static_cast<size_t>(bh) * kDK + d]);
@@ -63,7 +69,7 @@ decode_step_kernel(const DecodeProblem p) {
   ksum = 0.f;
 #pragma unroll
   for (int s = 0; s < kSplit; ++s) ksum += part[s][c];
-  float vn = __bfloat162float(p.v[static_cast<size_t>(bh) * V + c]);
+  float vn = token_in<F32>(p.v, static_cast<size_t>(bh) * V + c);
   if (p.delta) vn = p.beta[bh] * (vn - ksum);
   float o = 0.f;
 #pragma unroll
@@ -81,6 +87,13 @@ decode_step_kernel(const DecodeProblem p) {
     for (int s = 0; s < kSplit; ++s) os += part[s][c];
     p.o[static_cast<size_t>(bh) * V + c] = __float2bfloat16_rn(os);
   }
+}
+
+template <bool F32>
+static int launch_decode(const DecodeProblem& p, cudaStream_t st) {
+  if (p.V == 64) decode_step_kernel<64, F32><<<p.BH, kSplit * 64, 0, st>>>(p);
+  else decode_step_kernel<128, F32><<<p.BH, kSplit * 128, 0, st>>>(p);
+  return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
 }
 
 }  // namespace lg
@@ -101,15 +114,13 @@ extern "C" int lethe_gdn_decode_step(const LetheGdnDecodeArgs* a, void* stream) 
   p.gate = a->gate;
   p.delta = a->delta;
   p.scale = a->scale;
-  p.q = static_cast<const __nv_bfloat16*>(a->q);
-  p.k = static_cast<const __nv_bfloat16*>(a->k);
-  p.v = static_cast<const __nv_bfloat16*>(a->v);
+  p.q = a->q;
+  p.k = a->k;
+  p.v = a->v;
   p.g = a->g;
   p.beta = a->beta;
   p.state = a->state;
   p.o = static_cast<__nv_bfloat16*>(a->o);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (a->V == 64) decode_step_kernel<64><<<p.BH, kSplit * 64, 0, st>>>(p);
-  else decode_step_kernel<128><<<p.BH, kSplit * 128, 0, st>>>(p);
-  return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
+  return a->in_f32 ? launch_decode<true>(p, st) : launch_decode<false>(p, st);
 }

@@ -71,7 +71,7 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq,
     tmem_relinquish();
   }
   float gval = 0.f, bval = 1.f;
-  if (tid < 64) {
+  if (tid < p.rows_of(c)) {
     const size_t tok = (static_cast<size_t>(b) * p.L + c * kC + tid) * p.H + h;
     if (p.gate == LETHE_GATE_SCALAR) gval = p.g[tok];
     if (DELTA) bval = p.beta[tok];
@@ -343,7 +343,7 @@ output_kernel(const Problem p, const __grid_constant__ CUtensorMap mq) {
     tmem_relinquish();
   }
   float gval = 0.f;
-  if (tid < 64 && p.gate == LETHE_GATE_SCALAR)
+  if (tid < p.rows_of(c) && p.gate == LETHE_GATE_SCALAR)
     gval = p.g[(static_cast<size_t>(b) * p.L + c * kC + tid) * p.H + h];
   tc_fence_before();
   __syncthreads();
@@ -433,6 +433,7 @@ output_kernel(const Problem p, const __grid_constant__ CUtensorMap mq) {
   tc_fence_after();
   if (tid >= 64) {
     const int r = tid - 64;
+    const bool live = r < p.rows_of(c);
     __nv_bfloat16* og = p.o + ((static_cast<size_t>(b) * p.L + c * kC + r) * p.H + h) * V;
 #pragma unroll
     for (int jb = 0; jb < V / 32; ++jb) {
@@ -440,7 +441,8 @@ output_kernel(const Problem p, const __grid_constant__ CUtensorMap mq) {
       tmem_ld32(tmem + lane_base + jb * 32, d);
       tmem_ld_wait();
 #pragma unroll
-      for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(og + jb * 32 + 8 * i) = pack8_bf16(d + 8 * i);
+      for (int i = 0; i < 4; ++i)
+        if (live) *reinterpret_cast<uint4*>(og + jb * 32 + 8 * i) = pack8_bf16(d + 8 * i);
     }
   }
   if (tid == 0) bulk_wait_read();

@@ -1,0 +1,150 @@
+// Gates of the six-input surface (reference gdn_layer.py:99-111), where g, b and w come per channel even when a model
+// has one decay and one beta per token-head: the test that finds this out and compacts them, and the way back.  Both
+// are element-wise and bound by HBM: one pass over the gates each.
+#include <algorithm>
+
+#include "../../include/lethe_gdn.h"
+#include "host_util.h"
+
+namespace lg {
+
+constexpr int kGateThreads = 256;
+constexpr int kGateRowsPerWarp = 4;     // rows a warp requests before it looks at the first: 5 KB in flight per warp
+
+struct RegimeProblem {
+  const float *g, *b, *w;
+  float *g0, *b0;
+  long long rows;
+  uint32_t *flags, *work;      // work[0]: tests that have failed somewhere; work[1]: CTAs that are done
+};
+
+// A warp takes kGateRowsPerWarp rows at a time (K = 128: one float4 per lane and row), grid-stride.  Three tests can
+// fail; once all three have, nothing more has to be read, which is what a call with independent gates sees at its
+// first rows.  The last CTA publishes the verdict: `flags` may be a mapped host word that the caller polls, which
+// costs the call no copy and no synchronisation with whatever else the stream holds.
+template <int V>
+__global__ void __launch_bounds__(kGateThreads)
+gate_regime_kernel(const RegimeProblem p) {
+  const int lane = threadIdx.x & 31;
+  const long long warps = static_cast<long long>(gridDim.x) * (kGateThreads / 32);
+  const long long first = static_cast<long long>(blockIdx.x) * (kGateThreads / 32) + (threadIdx.x >> 5);
+  constexpr int R = kGateRowsPerWarp;
+  constexpr int WV = V / 32;
+  uint32_t bad = 0;
+  for (long long r0 = first * R; r0 < p.rows; r0 += warps * R) {
+    float4 g[R], b[R];
+    float w[R][WV];
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+      const long long r = min(r0 + u, p.rows - 1);
+      g[u] = reinterpret_cast<const float4*>(p.g + r * 128)[lane];
+      b[u] = reinterpret_cast<const float4*>(p.b + r * 128)[lane];
+      if (WV == 4) *reinterpret_cast<float4*>(w[u]) = reinterpret_cast<const float4*>(p.w + r * V)[lane];
+      else *reinterpret_cast<float2*>(w[u]) = reinterpret_cast<const float2*>(p.w + r * V)[lane];
+    }
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+      const float gf = __shfl_sync(0xffffffffu, g[u].x, 0), bf = __shfl_sync(0xffffffffu, b[u].x, 0);
+      const bool g_one = g[u].x == gf && g[u].y == gf && g[u].z == gf && g[u].w == gf;
+      bool one = b[u].x == bf && b[u].y == bf && b[u].z == bf && b[u].w == bf;
+      bool none = b[u].x == 0.f && b[u].y == 0.f && b[u].z == 0.f && b[u].w == 0.f;
+#pragma unroll
+      for (int e = 0; e < WV; ++e) {
+        one = one && w[u][e] == bf;
+        none = none && w[u][e] == 1.f;
+      }
+      bad |= (g_one ? 0u : LETHE_REGIME_SCALAR_GATE) | (one ? 0u : LETHE_REGIME_ONE_BETA) | (none ? 0u : LETHE_REGIME_NO_DELTA);
+      if (lane == 0 && r0 + u < p.rows) {
+        p.g0[r0 + u] = gf;
+        p.b0[r0 + u] = bf;
+      }
+    }
+    bad = __reduce_or_sync(0xffffffffu, bad);
+    if (bad == 7u) break;
+    if (*reinterpret_cast<volatile uint32_t*>(p.work) == 7u) break;
+  }
+  __shared__ uint32_t cta_bad;
+  if (threadIdx.x == 0) cta_bad = 0;
+  __syncthreads();
+  if (lane == 0 && bad) atomicOr(&cta_bad, bad);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (cta_bad) atomicOr(p.work, cta_bad);
+    __threadfence();
+    if (atomicAdd(p.work + 1, 1u) == gridDim.x - 1) {
+      const uint32_t failed = atomicExch(p.work, 0u);
+      p.work[1] = 0u;
+      *reinterpret_cast<volatile uint32_t*>(p.flags) = LETHE_REGIME_DONE | (~failed & 7u);
+      __threadfence_system();
+    }
+  }
+}
+
+struct SpreadProblem {
+  const float *dg0, *db0, *dw0;
+  float *dg, *db, *dw;
+  long long rows;
+};
+
+// One warp per row and pass: three coalesced row stores.
+template <int V>
+__global__ void __launch_bounds__(kGateThreads)
+gate_spread_kernel(const SpreadProblem p) {
+  const int lane = threadIdx.x & 31;
+  const long long warps = static_cast<long long>(gridDim.x) * (kGateThreads / 32);
+  for (long long r = static_cast<long long>(blockIdx.x) * (kGateThreads / 32) + (threadIdx.x >> 5); r < p.rows; r += warps) {
+    if (p.dg) {
+      const float x = p.dg0 ? p.dg0[r] * (1.f / 128) : 0.f;
+      reinterpret_cast<float4*>(p.dg + r * 128)[lane] = make_float4(x, x, x, x);
+    }
+    if (p.db) {
+      const float x = p.db0 ? p.db0[r] * (1.f / 128) : 0.f;
+      reinterpret_cast<float4*>(p.db + r * 128)[lane] = make_float4(x, x, x, x);
+    }
+    if (p.dw) {
+      const float x = p.dw0 ? p.dw0[r] * (1.f / V) : 0.f;
+      if (V == 128) reinterpret_cast<float4*>(p.dw + r * V)[lane] = make_float4(x, x, x, x);
+      else reinterpret_cast<float2*>(p.dw + r * V)[lane] = make_float2(x, x);
+    }
+  }
+}
+
+static bool gates_aligned(const void* a) { return (reinterpret_cast<uintptr_t>(a) & 15) == 0; }
+
+}  // namespace lg
+
+extern "C" int lethe_gdn_gate_regime(const float* g, const float* b, const float* w, int64_t rows, int32_t K, int32_t V,
+                                     float* g0, float* b0, uint32_t* flags, uint32_t* work, void* stream) {
+  using namespace lg;
+  if (!g || !b || !w || !g0 || !b0 || !flags || !work) return kErrNull;
+  if (rows <= 0 || K != 128 || (V != 64 && V != 128)) return kErrDims;
+  if (!gates_aligned(g) || !gates_aligned(b) || !gates_aligned(w)) return kErrAlign;
+  DeviceGuard guard(g);
+  const int sms = sm_count();
+  if (!guard.ok || sms <= 0) return kErrDevice;
+  const RegimeProblem p{g, b, w, g0, b0, rows, flags, work};
+  const int64_t per_cta = (kGateThreads / 32) * kGateRowsPerWarp;
+  // four CTAs per SM: enough bytes in flight for HBM, few enough CTAs to finish in one wave
+  const unsigned grid = static_cast<unsigned>(std::min(static_cast<int64_t>(4 * sms), (rows + per_cta - 1) / per_cta));
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (V == 64) gate_regime_kernel<64><<<grid, kGateThreads, 0, st>>>(p);
+  else gate_regime_kernel<128><<<grid, kGateThreads, 0, st>>>(p);
+  return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
+}
+
+extern "C" int lethe_gdn_gate_spread(const float* dg0, const float* db0, const float* dw0, int64_t rows, int32_t K, int32_t V,
+                                     float* dg, float* db, float* dw, void* stream) {
+  using namespace lg;
+  if (!dg && !db && !dw) return kErrNull;
+  if (rows <= 0 || K != 128 || (V != 64 && V != 128)) return kErrDims;
+  if (!gates_aligned(dg) || !gates_aligned(db) || !gates_aligned(dw)) return kErrAlign;
+  DeviceGuard guard(dg ? dg : db ? db : dw);
+  const int sms = sm_count();
+  if (!guard.ok || sms <= 0) return kErrDevice;
+  const SpreadProblem p{dg0, db0, dw0, dg, db, dw, rows};
+  const unsigned grid = static_cast<unsigned>(std::min(static_cast<int64_t>(8 * sms), (rows + kGateThreads / 32 - 1) / (kGateThreads / 32)));
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (V == 64) gate_spread_kernel<64><<<grid, kGateThreads, 0, st>>>(p);
+  else gate_spread_kernel<128><<<grid, kGateThreads, 0, st>>>(p);
+  return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
+}

@@ -18,37 +18,31 @@
 
 namespace lg {
 
-template <bool F32>
+__device__ __forceinline__ void load8_16(const void* base, size_t idx, float* x, int f16);
+__device__ __forceinline__ void store8_16(void* base, size_t idx, const float* x, int f16);
+
+enum { kInBf16 = 0, kInF32 = 1, kInF16 = 2 };   // type of q, k and of the gradients returned for them
+
+template <int IN>
 __device__ __forceinline__ void load8(const void* base, size_t idx, float* x) {
-  if (F32) {
+  if (IN == kInF32) {
     const float4* p = reinterpret_cast<const float4*>(static_cast<const float*>(base) + idx);
     const float4 a = p[0], b = p[1];
     x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
     x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
   } else {
-    const uint4 u = *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(base) + idx);
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float2 f = __bfloat1622float2(h[j]);
-      x[2 * j] = f.x;
-      x[2 * j + 1] = f.y;
-    }
+    load8_16(base, idx, x, IN == kInF16);
   }
 }
 
-template <bool F32>
+template <int IN>
 __device__ __forceinline__ void store8(void* base, size_t idx, const float* x) {
-  if (F32) {
+  if (IN == kInF32) {
     float4* p = reinterpret_cast<float4*>(static_cast<float*>(base) + idx);
     p[0] = make_float4(x[0], x[1], x[2], x[3]);
     p[1] = make_float4(x[4], x[5], x[6], x[7]);
   } else {
-    uint4 u;
-    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&u);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(x[2 * j], x[2 * j + 1]);
-    *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(base) + idx) = u;
+    store8_16(base, idx, x, IN == kInF16);
   }
 }
 
@@ -109,7 +103,7 @@ struct L2Problem {
 // bandwidth that way).
 constexpr int kPieces = 4;
 
-template <int LANES, bool F32, bool BACKWARD>
+template <int LANES, int IN, bool BACKWARD>
 __global__ void __launch_bounds__(256)
 l2norm_qk_kernel(const L2Problem p) {
   const int t = blockIdx.y;
@@ -126,7 +120,7 @@ l2norm_qk_kernel(const L2Problem p) {
     idx[u] = static_cast<size_t>(live[u] ? piece : 0) * 8;
   }
 #pragma unroll
-  for (int u = 0; u < kPieces; ++u) load8<F32>(p.x[t], idx[u], x[u]);
+  for (int u = 0; u < kPieces; ++u) load8<IN>(p.x[t], idx[u], x[u]);
   if (BACKWARD) {
 #pragma unroll
     for (int u = 0; u < kPieces; ++u) load8_16(p.dy[t], idx[u], dy[u], p.norm_f16);
@@ -148,24 +142,26 @@ l2norm_qk_kernel(const L2Problem p) {
       const float c = row_sum<LANES>(dot) * r * r;       // dx = r dy - x r^3 (x . dy)
 #pragma unroll
       for (int j = 0; j < 8; ++j) x[u][j] = r * (dy[u][j] - x[u][j] * c);
-      if (live[u]) store8<F32>(p.out[t], idx[u], x[u]);
+      if (live[u]) store8<IN>(p.out[t], idx[u], x[u]);
     }
   }
 }
 
+template <int LANES, bool BACKWARD>
+void launch_l2norm_t(const L2Problem& p, int in, const dim3& grid, cudaStream_t st) {
+  if (in == kInF32) l2norm_qk_kernel<LANES, kInF32, BACKWARD><<<grid, 256, 0, st>>>(p);
+  else if (in == kInF16) l2norm_qk_kernel<LANES, kInF16, BACKWARD><<<grid, 256, 0, st>>>(p);
+  else l2norm_qk_kernel<LANES, kInBf16, BACKWARD><<<grid, 256, 0, st>>>(p);
+}
 template <bool BACKWARD>
-int launch_l2norm(const L2Problem& p, int D, bool f32, cudaStream_t st) {
+int launch_l2norm(const L2Problem& p, int D, int flags, cudaStream_t st) {
+  const int in = (flags & LETHE_L2_IN_F32) ? kInF32 : (flags & LETHE_L2_IN_F16) ? kInF16 : kInBf16;
   const int lanes = D / 8;
   const long long pieces = p.rows * lanes;
   const int per_cta = 256 * kPieces;
   const dim3 grid(static_cast<unsigned>((pieces + per_cta - 1) / per_cta), 2);
-  if (lanes == 16) {
-    if (f32) l2norm_qk_kernel<16, true, BACKWARD><<<grid, 256, 0, st>>>(p);
-    else l2norm_qk_kernel<16, false, BACKWARD><<<grid, 256, 0, st>>>(p);
-  } else {
-    if (f32) l2norm_qk_kernel<8, true, BACKWARD><<<grid, 256, 0, st>>>(p);
-    else l2norm_qk_kernel<8, false, BACKWARD><<<grid, 256, 0, st>>>(p);
-  }
+  if (lanes == 16) launch_l2norm_t<16, BACKWARD>(p, in, grid, st);
+  else launch_l2norm_t<8, BACKWARD>(p, in, grid, st);
   return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
 }
 
@@ -182,7 +178,7 @@ extern "C" int lethe_gdn_l2norm_qk(const void* q, const void* k, void* qn, void*
   DeviceGuard guard(q);
   if (!guard.ok) return kErrDevice;
   L2Problem p{{q, k}, {nullptr, nullptr}, {qn, kn}, rows, eps, (flags & LETHE_L2_NORM_F16) ? 1 : 0};
-  return launch_l2norm<false>(p, D, (flags & LETHE_L2_IN_F32) != 0, static_cast<cudaStream_t>(stream));
+  return launch_l2norm<false>(p, D, flags, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int lethe_gdn_l2norm_qk_vjp(const void* q, const void* k, const void* dqn, const void* dkn, void* dq,
@@ -196,5 +192,5 @@ extern "C" int lethe_gdn_l2norm_qk_vjp(const void* q, const void* k, const void*
   DeviceGuard guard(q);
   if (!guard.ok) return kErrDevice;
   L2Problem p{{q, k}, {dqn, dkn}, {dq, dk}, rows, eps, (flags & LETHE_L2_NORM_F16) ? 1 : 0};
-  return launch_l2norm<true>(p, D, (flags & LETHE_L2_IN_F32) != 0, static_cast<cudaStream_t>(stream));
+  return launch_l2norm<true>(p, D, flags, static_cast<cudaStream_t>(stream));
 }

@@ -139,8 +139,9 @@ scan_kernel(const Problem p) {
     float x[kVs];
     {
       const float* x0 = seg_first ? (ADJOINT ? p.dhT : p.h0) : carry;
+      const int nrow = seg_first ? p.Kr : kK;      // user states have the real channel count
 #pragma unroll
-      for (int j = 0; j < kVs; ++j) x[j] = x0 ? x0[(static_cast<size_t>(bh) * kK + tid) * V + v0 + j] : 0.f;
+      for (int j = 0; j < kVs; ++j) x[j] = x0 && tid < nrow ? x0[(static_cast<size_t>(bh) * nrow + tid) * V + v0 + j] : 0.f;
     }
     constexpr int kPieces = kVs / 8;             // 16-byte pieces of this thread's row
     uint4 rnext[kPieces];
@@ -211,10 +212,11 @@ scan_kernel(const Problem p) {
         *reinterpret_cast<uint4*>(rec + sw128_chunk(tid, v0 / 8 + q, 128)) = pack8_f16(x + 8 * q);
     }
     float* xT = seg_last ? (ADJOINT ? p.dh0 : p.hT) : carry;
-    if (xT) {
+    const int nrow = seg_last ? p.Kr : kK;
+    if (xT && tid < nrow) {
 #pragma unroll
       for (int j = 0; j < kVs; j += 4)
-        *reinterpret_cast<float4*>(xT + (static_cast<size_t>(bh) * kK + tid) * V + v0 + j) =
+        *reinterpret_cast<float4*>(xT + (static_cast<size_t>(bh) * nrow + tid) * V + v0 + j) =
             make_float4(x[j], x[j + 1], x[j + 2], x[j + 3]);
     }
   }
@@ -252,8 +254,9 @@ scan_nodelta_kernel(const Problem p) {
   float x[8];
   {
     const float* x0 = seg_first ? (ADJOINT ? p.dhT : p.h0) : carry;
+    const int nrow = seg_first ? p.Kr : kK;        // user states have the real channel count
 #pragma unroll
-    for (int j = 0; j < 8; ++j) x[j] = x0 ? x0[(static_cast<size_t>(bh) * kK + d) * V + col0 + j] : 0.f;
+    for (int j = 0; j < 8; ++j) x[j] = x0 && d < nrow ? x0[(static_cast<size_t>(bh) * nrow + d) * V + col0 + j] : 0.f;
   }
   constexpr int kBatch = 8;
   for (int it0 = 0; it0 < n; it0 += kBatch) {
@@ -282,8 +285,9 @@ scan_nodelta_kernel(const Problem p) {
   if (!ADJOINT && seg_last)   // the final state as one more record
     *reinterpret_cast<uint4*>(Xg + (static_cast<size_t>(bh) * (NT + 1) + NT) * szx + off) = pack8_f16(x);
   float* xT = seg_last ? (ADJOINT ? p.dh0 : p.hT) : carry;
-  if (xT) {
-    float* dst = xT + (static_cast<size_t>(bh) * kK + d) * V + col0;
+  const int nrow = seg_last ? p.Kr : kK;
+  if (xT && d < nrow) {
+    float* dst = xT + (static_cast<size_t>(bh) * nrow + d) * V + col0;
     *reinterpret_cast<float4*>(dst) = make_float4(x[0], x[1], x[2], x[3]);
     *reinterpret_cast<float4*>(dst + 4) = make_float4(x[4], x[5], x[6], x[7]);
   }
