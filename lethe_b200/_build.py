@@ -23,6 +23,8 @@ LIB = os.path.join(LIBDIR, "liblethe_gdn.so")
 PROBE_SRC = os.path.join(ROOT, "tests", "native", "probe.cu")
 PROBE_LIBDIR = os.path.join(ROOT, "tests", "native", "_lib")
 PROBE_LIB = os.path.join(PROBE_LIBDIR, "libletheprobe.so")
+TORCH_SRC = os.path.join(CSRC, "torch_ops.cpp")
+TORCH_LIB = os.path.join(LIBDIR, "lethe_gdn_torch.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 # -use_fast_math: subnormal results flush to zero and division / square root are the approximate forms.
 # The gate factors go through exp2 with flush-to-zero instead of the longer subnormal-safe sequence, which
@@ -42,7 +44,7 @@ def _newest(*roots):
     for root in roots:
         for f in os.listdir(root):
             p = os.path.join(root, f)
-            if os.path.isfile(p):
+            if os.path.isfile(p) and not f.endswith(".cpp"):
                 t = max(t, os.path.getmtime(p))
     return t
 
@@ -100,6 +102,34 @@ def build(force: bool = False, verbose: bool = False) -> str:
     return LIB
 
 
+def build_torch(force: bool = False, verbose: bool = False) -> str:
+    """The extension module that binds the CUDA library to PyTorch (``csrc/torch_ops.cpp``, host code only)."""
+    build()
+    deps = [TORCH_SRC, os.path.join(ROOT, "include", "lethe_gdn.h")]
+    fresh = lambda: os.path.exists(TORCH_LIB) and os.path.getmtime(TORCH_LIB) >= max(map(os.path.getmtime, deps))
+    if not force and fresh():
+        return TORCH_LIB
+    with _Lock(os.path.join(LIBDIR, ".build.lock")):
+        if not force and fresh():
+            return TORCH_LIB
+        import sysconfig
+
+        import torch
+        t = os.path.dirname(torch.__file__)
+        cuda = os.path.dirname(os.path.dirname(NVCC))
+        tmp = f"{TORCH_LIB}.{os.getpid()}.tmp"
+        incs = [os.path.join(t, "include"), os.path.join(t, "include", "torch", "csrc", "api", "include"),
+                os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+        _run(["g++", "-shared", "-fPIC", "-O2", "-std=c++17", "-w",
+              f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-DTORCH_EXTENSION_NAME=lethe_gdn_torch",
+              *[f"-I{i}" for i in incs], TORCH_SRC, "-o", tmp, f"-L{LIBDIR}", "-l:" + os.path.basename(LIB),
+              "-Wl,-rpath,$ORIGIN", "-L" + os.path.join(t, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python",
+              "-L" + os.path.join(cuda, "lib64"), "-lcudart_static", "-ldl", "-lrt", "-lpthread"],
+             "g++ torch_ops.cpp", verbose)
+        os.replace(tmp, TORCH_LIB)
+    return TORCH_LIB
+
+
 def build_probe(force: bool = False, verbose: bool = False) -> str:
     """The test-only self-test library (tcgen05 / TMA toolkit probe, starved-wait probe)."""
     os.makedirs(PROBE_LIBDIR, exist_ok=True)
@@ -117,4 +147,5 @@ def build_probe(force: bool = False, verbose: bool = False) -> str:
 
 if __name__ == "__main__":
     print(build(force="--force" in sys.argv, verbose="-v" in sys.argv))
+    print(build_torch(force="--force" in sys.argv, verbose="-v" in sys.argv))
     print(build_probe(force="--force" in sys.argv, verbose="-v" in sys.argv))

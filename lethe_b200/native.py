@@ -1,14 +1,17 @@
-"""ctypes binding of the CUDA library.  There is no fallback: if the library is missing or does not
+"""Loads the CUDA library (ctypes) and the extension module that binds it to PyTorch.  There is no fallback: if the library is missing or does not
 load, importing this module raises."""
 
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 
 from . import _build
 
 _LIB = None
+_EXT = None
 
 
 def lib() -> ctypes.CDLL:
@@ -23,6 +26,23 @@ def lib() -> ctypes.CDLL:
         _LIB = ctypes.CDLL(path)
         _declare(_LIB)
     return _LIB
+
+
+def ext():
+    """Load (once) the extension module that binds the library to PyTorch (``_build.build_torch()``)."""
+    global _EXT
+    if _EXT is None:
+        path = _build.TORCH_LIB
+        if not os.path.exists(path):
+            raise RuntimeError(
+                f"{path} is missing: build it with `python -m lethe_b200._build` (needs nvcc and g++)")
+        loader = importlib.machinery.ExtensionFileLoader("lethe_gdn_torch", path)
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("lethe_gdn_torch", loader))
+        loader.exec_module(mod)
+        from .ops import GdnError
+        mod.set_error_type(GdnError)
+        _EXT = mod
+    return _EXT
 
 
 def _declare(L: ctypes.CDLL) -> None:

@@ -7,7 +7,8 @@ its chunkwise references: an initial state in and the final state out
 (``src/lethe/kernels/references/gdn2_chunkwise.py:77,157-158``).
 
 PyTorch supplies device memory, the stream and autograd bookkeeping; every number is computed by the
-CUDA library behind ``lethe_b200.native`` (there is no other path: a missing library raises).
+CUDA library behind ``lethe_b200.native`` (there is no other path: a missing library raises).  The
+differentiable ops and the decode step are one call each into the native binding (``csrc/torch_ops.cpp``).
 """
 
 from __future__ import annotations
@@ -45,6 +46,7 @@ class _Args(ctypes.Structure):
         ("db_gate", ctypes.c_void_p), ("dw_gate", ctypes.c_void_p),
         ("bh_begin", ctypes.c_uint32), ("bh_count", ctypes.c_uint32), ("qk_f16", ctypes.c_uint32),
         ("c_begin", ctypes.c_uint32), ("c_count", ctypes.c_uint32),
+        ("l_tokens", ctypes.c_uint32), ("k_channels", ctypes.c_uint32),
     ]
 
 
@@ -78,57 +80,6 @@ def check_status(status: Tensor) -> None:
 
 def _prep16(t: Tensor) -> Tensor:
     return t.to(torch.bfloat16).contiguous()
-
-
-def _prep_qk(q: Tensor, k: Tensor) -> tuple[Tensor, Tensor]:
-    """q and k as the kernels read them: fp16 when both came as fp16 (the tensor-core operand type, kept
-    as it is), bf16 otherwise."""
-    if q.dtype == torch.float16 and k.dtype == torch.float16:
-        return q.contiguous(), k.contiguous()
-    return _prep16(q), _prep16(k)
-
-
-class _StatusWatch:
-    """Deferred, sync-free check of the device status words.  After a call the word is copied to a pinned
-    host slot on the call's stream; a later call looks at the slots whose copies have completed and
-    raises if a device-side wait of that earlier call gave up.  Nothing ever waits for the GPU here, so
-    an error surfaces one or two calls late; ``check_status`` is the immediate (synchronising) form."""
-
-    SLOTS = 64
-
-    def __init__(self):
-        self._host = None
-        self._events = [None] * self.SLOTS
-        self._next = 0
-
-    def poll(self) -> None:
-        for i, ev in enumerate(self._events):
-            if ev is not None and ev.query():
-                self._events[i] = None
-                code = int(self._host[i])
-                if code != 0:
-                    raise GdnError(f"lethe_gdn: a device-side wait of an earlier call timed out at site {code}; "
-                                   "the results of that call are invalid")
-
-    def watch(self, status: Tensor) -> None:
-        if self._host is None:
-            self._host = torch.zeros(self.SLOTS, dtype=torch.int32).pin_memory()
-        i = self._next
-        self._next = (i + 1) % self.SLOTS
-        if self._events[i] is not None:      # ring full: this slot's copy is old enough to have landed
-            self._events[i].synchronize()
-            self.poll()
-        self._host[i:i + 1].copy_(status, non_blocking=True)
-        ev = torch.cuda.Event()
-        ev.record(torch.cuda.current_stream(status.device))
-        self._events[i] = ev
-
-
-_watch = _StatusWatch()
-
-
-def _prep32(t: Tensor | None) -> Tensor | None:
-    return None if t is None else t.to(torch.float32).contiguous()
 
 
 class GdnBuffers:
@@ -441,7 +392,7 @@ def gdn_backward_raw(q, k, v, g, beta, h0, do, dhT, saved, status, scale: float)
     return buf.dq, buf.dk, buf.dv, buf.dg, buf.dbeta, buf.dh0, buf.scratch
 
 
-L2_IN_F32, L2_NORM_F16 = 1, 2
+L2_IN_F32, L2_NORM_F16 = 1, 2       # flags of the C calls
 
 
 def _l2_working(q: Tensor, k: Tensor) -> tuple[Tensor, Tensor, bool]:
@@ -513,77 +464,6 @@ def l2norm_qk(q: Tensor, k: Tensor, eps: float = 1e-6) -> tuple[Tensor, Tensor]:
     return _L2NormQK.apply(q, k, eps)
 
 
-class _GdnChunk(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, q, k, v, g, beta, h0, scale):
-        if not q.is_cuda:
-            raise GdnError("lethe_gdn: inputs must live on a CUDA device (there is no CPU path)")
-        _watch.poll()
-        K = q.shape[-1]
-        ctx.in_dtypes = tuple(None if t is None else t.dtype for t in (q, k, v, g, beta, h0))
-        ctx.pad_k = 0
-        (q16, k16), v16 = _prep_qk(q, k), _prep16(v)
-        g32, b32, h32 = _prep32(g), _prep32(beta), _prep32(h0)
-        if K == 64:
-            # the kernels are built for 128 key channels: pad with zero channels (exact)
-            ctx.pad_k = 64
-            q16 = torch.nn.functional.pad(q16, (0, 64))
-            k16 = torch.nn.functional.pad(k16, (0, 64))
-            if g32 is not None and g32.dim() == 4:
-                g32 = torch.nn.functional.pad(g32, (0, 64))
-            if h32 is not None:
-                h32 = torch.nn.functional.pad(h32, (0, 0, 0, 64))
-        L = q.shape[1]
-        ctx.pad_l = (-L) % 64
-        if ctx.pad_l:
-            # The kernels work on chunks of 64 tokens.  Tokens appended with k = v = q = 0, g = 0 and
-            # beta = 0 leave the state untouched (decay 1, nothing erased, nothing written), so the
-            # result on the real tokens and the final state are exact.
-            def pad_tokens(t):
-                return None if t is None else torch.nn.functional.pad(t, (0, 0) * (t.dim() - 2) + (0, ctx.pad_l))
-            q16, k16, v16, g32, b32 = (pad_tokens(t) for t in (q16, k16, v16, g32, b32))
-        o, hT, saved, status = gdn_forward_raw(q16, k16, v16, g32, b32, h32, scale)
-        _watch.watch(status)
-        ctx.save_for_backward(q16, k16, v16, g32, b32, h32, saved, status)
-        ctx.scale = scale
-        if ctx.pad_k:
-            hT = hT[:, :, :K].contiguous()
-        if ctx.pad_l:
-            o = o[:, :L]
-        return o.to(v.dtype), hT
-
-    @staticmethod
-    @once_differentiable
-    def backward(ctx, do, dhT):
-        q16, k16, v16, g32, b32, h32, saved, status = ctx.saved_tensors
-        _watch.poll()
-        do16 = _prep16(do)
-        dhT32 = _prep32(dhT)
-        if ctx.pad_l:
-            do16 = torch.nn.functional.pad(do16, (0, 0, 0, 0, 0, ctx.pad_l))
-        if ctx.pad_k and dhT32 is not None:
-            dhT32 = torch.nn.functional.pad(dhT32, (0, 0, 0, ctx.pad_k))
-        dq, dk, dv, dg, dbeta, dh0, _ = gdn_backward_raw(q16, k16, v16, g32, b32, h32, do16, dhT32,
-                                                        saved, status, ctx.scale)
-        _watch.watch(status)
-        if ctx.pad_k:
-            K = q16.shape[-1] - ctx.pad_k
-            dq, dk, dh0 = dq[..., :K], dk[..., :K], dh0[:, :, :K]
-            if dg is not None and dg.dim() == 4:
-                dg = dg[..., :K]
-        if ctx.pad_l:
-            L = q16.shape[1] - ctx.pad_l
-            dq, dk, dv = dq[:, :L], dk[:, :L], dv[:, :L]
-            dg = None if dg is None else dg[:, :L]
-            dbeta = None if dbeta is None else dbeta[:, :L]
-        dts = ctx.in_dtypes
-        outs = [dq.to(dts[0]), dk.to(dts[1]), dv.to(dts[2]),
-                None if dg is None else dg.to(dts[3]),
-                None if dbeta is None else dbeta.to(dts[4]),
-                None if dts[5] is None else dh0.to(dts[5]), None]
-        return tuple(outs)
-
-
 def gdn_chunk(q: Tensor, k: Tensor, v: Tensor, g: Tensor | None, beta: Tensor | None,
               h0: Tensor | None = None, *, scale: float | None = None,
               use_qk_l2norm: bool = False) -> tuple[Tensor, Tensor]:
@@ -593,15 +473,14 @@ def gdn_chunk(q: Tensor, k: Tensor, v: Tensor, g: Tensor | None, beta: Tensor | 
     ``beta``: ``[B,L,H]`` (erase and write gate) or None for the variants without the delta term
     (linear attention, GLA, SSD).  Gradients flow to q, k, v, g, beta and h0 (first order only: the
     backward is not itself differentiable, asking for a second derivative raises).  ``L`` need not be a
-    multiple of the chunk length and d_k may be 64 or 128: both are met by exact zero padding.  q and k
-    are read as bf16, or as fp16 when both are given as fp16; with ``use_qk_l2norm`` they are normalised
+    multiple of the chunk length and d_k may be 64 or 128: the kernels read what is missing from a chunk
+    as zeros, which is exact (a token with k = v = q = 0, g = 0 and beta = 0 leaves the state untouched).
+    q and k are read as bf16, or as fp16 when both are given as fp16; with ``use_qk_l2norm`` they are normalised
     in fp32 and rounded once to fp16.
     """
-    if scale is None:
-        scale = q.shape[-1] ** -0.5
-    if use_qk_l2norm:
-        q, k = l2norm_qk(q, k)
-    return _GdnChunk.apply(q, k, v, g, beta, h0, float(scale))
+    if not q.is_cuda:
+        raise GdnError("lethe_gdn: inputs must live on a CUDA device (there is no CPU path)")
+    return native.ext().chunk(q, k, v, g, beta, h0, q.shape[-1] ** -0.5 if scale is None else scale, use_qk_l2norm)
 
 
 class _DecodeArgs(ctypes.Structure):
@@ -609,7 +488,7 @@ class _DecodeArgs(ctypes.Structure):
                 ("gate", ctypes.c_int32), ("delta", ctypes.c_int32), ("scale", ctypes.c_float),
                 ("q", ctypes.c_void_p), ("k", ctypes.c_void_p), ("v", ctypes.c_void_p),
                 ("g", ctypes.c_void_p), ("beta", ctypes.c_void_p), ("state", ctypes.c_void_p),
-                ("o", ctypes.c_void_p)]
+                ("o", ctypes.c_void_p), ("in_f32", ctypes.c_uint32)]
 
 
 def gdn_decode_step(q: Tensor, k: Tensor, v: Tensor, g: Tensor | None, beta: Tensor | None, state: Tensor,
@@ -622,64 +501,7 @@ def gdn_decode_step(q: Tensor, k: Tensor, v: Tensor, g: Tensor | None, beta: Ten
     (start from the ``h_T`` that ``gdn_chunk`` returned for the prompt).  Returns ``o [B,H,V]`` bf16.
     Not differentiable.  K must be 128, V 64 or 128.
     """
-    if not state.is_cuda:
-        raise GdnError("lethe_gdn: inputs must live on a CUDA device (there is no CPU path)")
-    if state.dtype != torch.float32 or not state.is_contiguous():
-        raise GdnError("lethe_gdn: the decode state must be a contiguous fp32 tensor (it is updated in place)")
-    B, H, K, V = state.shape
-    q16, k16, v16 = _prep16(q), _prep16(k), _prep16(v)
-    g32, b32 = _prep32(g), _prep32(beta)
-    if q16.shape != (B, H, K) or k16.shape != (B, H, K) or v16.shape != (B, H, V):
-        raise GdnError("lethe_gdn: decode step expects q, k [B,H,K] and v [B,H,V] matching the state")
-    if g32 is not None and g32.shape not in ((B, H), (B, H, K)):
-        raise GdnError("lethe_gdn: decode step expects g [B,H] or [B,H,K]")
-    if b32 is not None and b32.shape != (B, H):
-        raise GdnError("lethe_gdn: decode step expects beta [B,H]")
-    o = torch.empty(B, H, V, dtype=torch.bfloat16, device=state.device)
-    a = _DecodeArgs(B=B, H=H, K=K, V=V, gate=_gate_code(None if g32 is None else g32.unsqueeze(1)),
-                    delta=0 if b32 is None else 1, scale=float(K ** -0.5 if scale is None else scale),
-                    q=_ptr(q16), k=_ptr(k16), v=_ptr(v16), g=_ptr(g32), beta=_ptr(b32), state=_ptr(state), o=_ptr(o))
-    _check(native.lib().lethe_gdn_decode_step(ctypes.byref(a), torch.cuda.current_stream(state.device).cuda_stream))
-    return o
-
-
-class _GdnFull(torch.autograd.Function):
-    """The reference's full recurrence (``src/lethe/kernels/references/gdn_backward.py:45-53``): per-channel
-    log decay ``g`` and erase gate ``b`` (``[B,L,H,K]``), per-channel write gate ``w`` (``[B,L,H,V]``)."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, g, b, w, h0, scale):
-        if not q.is_cuda:
-            raise GdnError("lethe_gdn: inputs must live on a CUDA device (there is no CPU path)")
-        _watch.poll()
-        B, L, H, K = q.shape
-        V = v.shape[-1]
-        if K != 128 or L % 64:
-            raise GdnError("lethe_gdn: the full-gate op needs d_k = 128 and L a multiple of 64")
-        ctx.in_dtypes = tuple(None if t is None else t.dtype for t in (q, k, v, g, b, w, h0))
-        (q16, k16), v16 = _prep_qk(q, k), _prep16(v)
-        g32, b32, w32, h32 = _prep32(g), _prep32(b), _prep32(w), _prep32(h0)
-        buf = GdnBuffers(B, L, H, K, V, GATE_CHANNEL, 2, q.device, backward=False)
-        forward_into(buf, q16, k16, v16, g32, None, h32, scale, b_gate=b32, w_gate=w32)
-        _watch.watch(buf.status)
-        ctx.save_for_backward(q16, k16, v16, g32, b32, w32, h32, buf.saved, buf.status)
-        ctx.scale = scale
-        return buf.o.to(v.dtype), buf.hT
-
-    @staticmethod
-    @once_differentiable
-    def backward(ctx, do, dhT):
-        q16, k16, v16, g32, b32, w32, h32, saved, status = ctx.saved_tensors
-        _watch.poll()
-        B, L, H, K = q16.shape
-        buf = GdnBuffers(B, L, H, K, v16.shape[-1], GATE_CHANNEL, 2, q16.device, saved=saved, status=status,
-                         qk_dtype=q16.dtype)
-        backward_into(buf, q16, k16, v16, g32, None, h32, _prep16(do), _prep32(dhT), ctx.scale,
-                      b_gate=b32, w_gate=w32)
-        _watch.watch(status)
-        dts = ctx.in_dtypes
-        return (buf.dq.to(dts[0]), buf.dk.to(dts[1]), buf.dv.to(dts[2]), buf.dg.to(dts[3]), buf.db.to(dts[4]),
-                buf.dw.to(dts[5]), None if dts[6] is None else buf.dh0.to(dts[6]), None)
+    return native.ext().decode_step(q, k, v, g, beta, state, state.shape[2] ** -0.5 if scale is None else scale)
 
 
 def gdn_chunk_full(q: Tensor, k: Tensor, v: Tensor, g: Tensor, b: Tensor, w: Tensor, h0: Tensor | None = None, *,
@@ -687,11 +509,7 @@ def gdn_chunk_full(q: Tensor, k: Tensor, v: Tensor, g: Tensor, b: Tensor, w: Ten
     """The reference's full six-input recurrence with an initial state in and the final state out:
     ``g, b [B,L,H,K]`` (log decay and erase gate per key channel), ``w [B,L,H,V]`` (write gate per value
     channel).  Returns ``(o, h_T)``; gradients flow to all seven inputs (first order only)."""
-    if scale is None:
-        scale = q.shape[-1] ** -0.5
-    if use_qk_l2norm:
-        q, k = l2norm_qk(q, k)
-    return _GdnFull.apply(q, k, v, g, b, w, h0, float(scale))
+    return native.ext().chunk_full(q, k, v, g, b, w, h0, q.shape[-1] ** -0.5 if scale is None else scale, use_qk_l2norm)
 
 
 # ------------------------------------------------------------------------------------------------
@@ -700,100 +518,32 @@ def gdn_chunk_full(q: Tensor, k: Tensor, v: Tensor, g: Tensor, b: Tensor, w: Ten
 def gate_regime(g: Tensor, b: Tensor, w: Tensor) -> tuple[bool, bool, bool]:
     """``(scalar_gate, one_beta, no_delta)`` of a six-input call, decided as the reference decides
     (``src/lethe/kernels/cute/gdn2_backward.py:53-60``): BITWISE equality along the channel axis, never
-    a tolerance - a gate that is merely close to constant is a channel-wise gate.  One device
-    reduction and one host read for all five tests.
+    a tolerance - a gate that is merely close to constant is a channel-wise gate.  One kernel and one
+    host read for all five tests.
 
     scalar_gate: g is one value per token-head broadcast over the key channels;
     one_beta:    b and w are the same one value per token-head broadcast over their channels;
     no_delta:    b = 0 everywhere and w = 1 everywhere (no erase term, unit write gate)."""
-    with torch.no_grad():
-        flags = torch.stack([
-            (g == g[..., :1]).all(),
-            (b == b[..., :1]).all() & (w == w[..., :1]).all() & (b[..., 0] == w[..., 0]).all(),
-            (b == 0).all() & (w == 1).all(),
-        ]).tolist()
-    return bool(flags[0]), bool(flags[1]), bool(flags[2])
-
-
-class _Gdn2Op(torch.autograd.Function):
-    """``gdn2_op`` of the reference (``src/lethe/kernels/ops/gdn_layer.py:15-111``) on the CUDA library.
-
-    The reference op takes a per-channel log decay ``g``, erase gate ``b`` (both ``[B,L,H,d_k]``) and
-    write gate ``w`` (``[B,L,H,d_v]``).  The kernels cover the regimes its native path covers
-    (``src/lethe/kernels/cute/gdn2_backward.py:53-60,102-134`` and ``cute/gdn2_family.py``):
-    ``b`` and ``w`` both equal to one beta per token-head broadcast over the channels (gated delta
-    rule / KDA), or ``b = 0, w = 1`` (no delta term); ``g`` either constant over the channels
-    (scalar gate) or not (channel-wise gate).  Independent per-channel ``b`` / ``w`` do not come
-    here: ``gdn2_op`` sends them to ``gdn_chunk_full``.
-
-    Gradients of broadcast inputs are spread evenly over the channels, as the reference's scalar
-    assembly does (``gdn2_assemble.py:343-345``); ``grad_b`` carries the erase part and ``grad_w`` the
-    write part of the beta gradient (``gdn2_assemble.py:150-181``).
-    """
-
-    @staticmethod
-    def forward(ctx, q, k, v, g, b, w, scale, use_qk_l2norm, scalar_gate, delta):
-        if not q.is_cuda:
-            raise GdnError("lethe_gdn: inputs must live on a CUDA device (there is no CPU path)")
-        _watch.poll()
-        K, V = q.shape[-1], v.shape[-1]
-        with torch.no_grad():
-            beta = b[..., 0].float().contiguous() if delta else None
-            g_in = (g[..., 0] if scalar_gate else g).float().contiguous()
-        ctx.meta = (q.dtype, k.dtype, v.dtype, g.dtype, b.dtype, w.dtype, K, V, scalar_gate, delta, use_qk_l2norm)
-        q16, k16 = l2norm_qk_raw(q, k) if use_qk_l2norm else _prep_qk(q, k)
-        v16 = _prep16(v)
-        o, _hT, saved, status = gdn_forward_raw(q16, k16, v16, g_in, beta, None, scale)
-        _watch.watch(status)
-        ctx.save_for_backward(q, k, q16, k16, v16, g_in, beta, saved, status)
-        ctx.scale = scale
-        return o.to(v.dtype)
-
-    @staticmethod
-    @once_differentiable
-    def backward(ctx, do):
-        q, k, q16, k16, v16, g_in, beta, saved, status = ctx.saved_tensors
-        _watch.poll()
-        dq_t, dk_t, dv_t, dg_t, db_t, dw_t, K, V, scalar_gate, delta, l2 = ctx.meta
-        B, L, H, _ = q16.shape
-        buf = GdnBuffers(B, L, H, K, V, _gate_code(g_in), delta, q16.device, saved=saved, status=status,
-                         qk_dtype=q16.dtype)
-        if delta:
-            buf.dbeta_write = torch.empty(B, L, H, dtype=torch.float32, device=q16.device)
-        backward_into(buf, q16, k16, v16, g_in, beta, None, _prep16(do), None, ctx.scale)
-        _watch.watch(status)
-        dq, dk = buf.dq, buf.dk
-        if l2:   # VJP of x / sqrt(|x|^2 + eps) (the reference gets it by autograd, gdn2_assemble.py:300-312)
-            dq, dk = l2norm_qk_vjp_raw(q, k, dq, dk)
-        grad_g = (buf.dg.unsqueeze(-1).expand(B, L, H, K) / K) if scalar_gate else buf.dg
-        if delta:
-            grad_b = buf.dbeta.unsqueeze(-1).expand(B, L, H, K) / K
-            grad_w = buf.dbeta_write.unsqueeze(-1).expand(B, L, H, V) / V
-        else:
-            grad_b = torch.zeros(B, L, H, K, device=q16.device)
-            grad_w = torch.zeros(B, L, H, V, device=q16.device)
-        return (dq.to(dq_t), dk.to(dk_t), buf.dv.to(dv_t), grad_g.to(dg_t).contiguous(),
-                grad_b.to(db_t).contiguous(), grad_w.to(dw_t).contiguous(), None, None, None, None)
+    m = native.ext().gate_regime(g, b, w)
+    return bool(m & 1), bool(m & 2), bool(m & 4)
 
 
 def gdn2_op(q: Tensor, k: Tensor, v: Tensor, g: Tensor, b: Tensor, w: Tensor, *, scale: float | None = None,
             use_qk_l2norm: bool = True) -> Tensor:
     """Drop-in for the reference's ``gdn2_op`` (same argument list, same defaults, returns ``o``).
     First-order gradients only: the backward pass is not differentiable (the reference falls back to its
-    eager path for that case, ``cute/gdn2_backward.py:92``; here a second derivative raises)."""
-    if scale is None:
-        scale = q.shape[-1] ** -0.5
-    if q.shape[-1] != 128:
-        raise GdnError("lethe_gdn: gdn2_op needs d_k = 128 (use gdn_chunk for d_k = 64)")
+    eager path for that case, ``cute/gdn2_backward.py:92``; here a second derivative raises).
+
+    The kernels cover the regimes the reference's native path covers (``cute/gdn2_backward.py:53-60,102-134``
+    and ``cute/gdn2_family.py``): ``b`` and ``w`` both equal to one beta per token-head (gated delta rule,
+    KDA), or ``b = 0, w = 1`` (no delta term); ``g`` constant over the channels (scalar gate) or not.  Independent
+    per-channel ``b`` / ``w`` run the full recurrence of ``gdn_chunk_full``.  Gradients of broadcast gates are
+    spread evenly over the channels, as the reference's scalar assembly does (``gdn2_assemble.py:343-345``);
+    ``grad_b`` carries the erase part and ``grad_w`` the write part of the beta gradient
+    (``gdn2_assemble.py:150-181``)."""
     if not q.is_cuda:
         raise GdnError("lethe_gdn: inputs must live on a CUDA device (there is no CPU path)")
-    scalar_gate, one_beta, no_delta = gate_regime(g, b, w)
-    if one_beta or no_delta:
-        # the regimes the scalar-beta kernels cover (cheaper: one gate value per token-head)
-        return _Gdn2Op.apply(q, k, v, g, b, w, float(scale), bool(use_qk_l2norm), scalar_gate, bool(one_beta))
-    # independent per-channel erase / write gates: the full recurrence
-    o, _ = gdn_chunk_full(q, k, v, g, b, w, None, scale=float(scale), use_qk_l2norm=bool(use_qk_l2norm))
-    return o
+    return native.ext().six_inputs(q, k, v, g, b, w, q.shape[-1] ** -0.5 if scale is None else scale, use_qk_l2norm)
 
 
 class Gdn2Grads(NamedTuple):
