@@ -118,6 +118,9 @@ typedef struct LetheGdnArgs {
   /* states [B, H, k_channels, V]).  The rest counts as zero and is neither read nor written.  0: all of dims.     */
   uint32_t l_tokens;
   uint32_t k_channels;
+  /* Non-zero: the call leaves only results in memory, and in the workspaces what its own later kernels and, after a   */
+  /* forward, the backward read.  Zero: also intermediates that a caller may want to look at (dv2, dw).                */
+  uint32_t lean;
 } LetheGdnArgs;
 
 /* Bytes of the forward->backward workspace / of the backward scratch for these sizes (0 = bad dims). */

@@ -15,7 +15,7 @@ int launch_bwd_pre(const Problem&, const CUtensorMap& mq, const CUtensorMap& mdo
 int launch_bwd_main(const Problem&, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                     const CUtensorMap& mdo, const OutMaps& mo, cudaStream_t, uint32_t mask);
 int launch_bwd_main_cw(const Problem&, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
-                       const CUtensorMap& mdo, cudaStream_t, uint32_t mask);
+                       const CUtensorMap& mdo, const CUtensorMap& mg, cudaStream_t, uint32_t mask);
 
 static bool dims_ok(const LetheGdnDims& d) {
   if (d.B <= 0 || d.H <= 0 || d.L <= 0) return false;
@@ -40,6 +40,15 @@ static int token_map(CUtensorMap* m, const void* ptr, const Problem& p, int D) {
   return make_tmap_16bit(m, ptr, 4, dims, str, box);
 }
 
+// Tensor map of the channel-wise gate [B, L, H, K] in fp32; one box = 64 tokens x 32 channels of one head.
+static int gate_map(CUtensorMap* m, const void* ptr, const Problem& p) {
+  const uint64_t K = static_cast<uint64_t>(p.Kr), H = static_cast<uint64_t>(p.H), L = static_cast<uint64_t>(p.L);
+  uint64_t dims[4] = {K, H, L, static_cast<uint64_t>(p.B)};
+  uint64_t str[3] = {K * 4, H * K * 4, L * H * K * 4};
+  uint32_t box[4] = {32, 1, 64, 1};
+  return make_tmap_f32(m, ptr, 4, dims, str, box);
+}
+
 static int fill_problem(const LetheGdnArgs* a, Problem* p, bool backward) {
   if (!a) return kErrNull;
   const LetheGdnDims& d = a->dims;
@@ -55,6 +64,7 @@ static int fill_problem(const LetheGdnArgs* a, Problem* p, bool backward) {
     if (d.delta == 1 && !a->dbeta) return kErrNull;
     if (d.delta == 2 && (!a->db_gate || !a->dw_gate)) return kErrNull;
   }
+  if (d.gate == LETHE_GATE_CHANNEL && !aligned16(a->g)) return kErrAlign;      // read through a tensor map
   const void* ptrs[] = {a->q, a->k, a->v, a->o, a->d_o, a->dq, a->dk, a->dv, a->h0, a->hT, a->dhT, a->dh0,
                         a->saved, a->scratch, a->b_gate, a->w_gate, a->db_gate, a->dw_gate};
   for (const void* x : ptrs)
@@ -90,6 +100,7 @@ static int fill_problem(const LetheGdnArgs* a, Problem* p, bool backward) {
   }
   p->scale = a->scale;
   p->qk16 = a->qk_f16 ? 1 : 0;
+  p->lean = a->lean ? 1 : 0;
   p->q = static_cast<const __nv_bfloat16*>(a->q);
   p->k = static_cast<const __nv_bfloat16*>(a->k);
   p->v = static_cast<const __nv_bfloat16*>(a->v);
@@ -162,7 +173,9 @@ extern "C" int lethe_gdn_backward(const LetheGdnArgs* a, void* stream) {
   if ((m & 2u) && (e = launch_scan(p, true, st))) return e;
   if (m & 12u) {
     if (p.gate == LETHE_GATE_CHANNEL) {
-      if ((e = launch_bwd_main_cw(p, mq, mk, mv, mdo, st, m))) return e;
+      CUtensorMap mg;
+      if ((e = gate_map(&mg, a->g, p))) return e;
+      if ((e = launch_bwd_main_cw(p, mq, mk, mv, mdo, mg, st, m))) return e;
     } else {
       OutMaps mo;
       if ((e = token_map(&mo.dq, a->dq, p, p.Kr))) return e;

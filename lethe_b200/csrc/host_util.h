@@ -65,6 +65,25 @@ inline int make_tmap_16bit(CUtensorMap* map, const void* ptr, int rank, const ui
   return r == CUDA_SUCCESS ? kOk : kErrDriver;
 }
 
+// The same over fp32 elements, without a swizzle (boxes of up to 32 elements: 128-byte rows).
+inline int make_tmap_f32(CUtensorMap* map, const void* ptr, int rank, const uint64_t* dims, const uint64_t* strides_bytes,
+                         const uint32_t* box) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (!fn) return kErrDriver;
+  cuuint64_t gdim[5], gstr[4];
+  cuuint32_t bx[5], es[5];
+  for (int i = 0; i < rank; ++i) {
+    gdim[i] = dims[i];
+    bx[i] = box[i];
+    es[i] = 1;
+    if (i > 0) gstr[i - 1] = strides_bytes[i - 1];
+  }
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, static_cast<cuuint32_t>(rank), const_cast<void*>(ptr), gdim, gstr, bx, es,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? kOk : kErrDriver;
+}
+
 // Tensor maps of the token-major gradient outputs that leave by tensor-map stores.
 struct OutMaps {
   CUtensorMap dq, dk, dv;

@@ -98,6 +98,11 @@ Tensor as(const Tensor& t, at::ScalarType dt) {
   return t.scalar_type() == dt ? t.contiguous() : t.to(dt).contiguous();
 }
 Tensor as32(const Tensor& t) { return t.defined() ? as(t, at::kFloat) : t; }
+// a gate per channel is read through a tensor map, which wants its start on a 16-byte boundary
+Tensor as_gate(const Tensor& t) {
+  const Tensor r = as32(t);
+  return r.defined() && (reinterpret_cast<uintptr_t>(r.data_ptr()) & 15) ? r.clone() : r;
+}
 Tensor opt(const OptTensor& t) { return t.has_value() ? *t : Tensor(); }
 Tensor cast_back(const Tensor& t, at::ScalarType dt) { return t.scalar_type() == dt ? t : t.to(dt); }
 template <typename T = void>
@@ -167,6 +172,7 @@ LetheGdnArgs base_args(const Problem& p, const Operands& x, void* saved, size_t 
   a.saved = saved;
   a.saved_bytes = saved_bytes;
   a.status = status_word(x.q.device().index());
+  a.lean = 1u;
   a.qk_f16 = x.q.scalar_type() == at::kHalf ? 1u : 0u;
   return a;
 }
@@ -405,7 +411,7 @@ std::pair<Tensor, Tensor> chunk(const Tensor& q, const Tensor& k, const Tensor& 
       at::NoGradGuard no_grad;
       prepare_qk(p, q, k, &x);
       x.v = as(v, at::kBFloat16);
-      x.g = as32(g); x.beta = as32(beta); x.h0 = as32(h0);
+      x.g = as_gate(g); x.beta = as32(beta); x.h0 = as32(h0);
     }
     return apply(p, {q, k, v, g, beta, h0, Tensor(), Tensor()}, std::move(x), false);
   });
@@ -420,7 +426,7 @@ std::pair<Tensor, Tensor> full_with(Problem p, Operands x, const Tensor (&in)[kS
     at::NoGradGuard no_grad;
     if (!x.q.defined()) prepare_qk(p, in[kQ], in[kKey], &x);
     x.v = as(in[kV], at::kBFloat16);
-    x.g = as32(in[kG]); x.b = as32(in[kB]); x.w = as32(in[kW]); x.h0 = as32(in[kH0]);
+    x.g = as_gate(in[kG]); x.b = as32(in[kB]); x.w = as32(in[kW]); x.h0 = as32(in[kH0]);
   }
   return apply(p, in, std::move(x), six);
 }
@@ -576,7 +582,7 @@ Tensor six_inputs(const Tensor& q, const Tensor& k, const Tensor& v, const Tenso
       p.delta = one_beta ? 1 : 0;
       if (!one_beta) x.beta = Tensor();
       p.gate = (regime & LETHE_REGIME_SCALAR_GATE) ? LETHE_GATE_SCALAR : LETHE_GATE_CHANNEL;
-      if (!full && p.gate == LETHE_GATE_CHANNEL) x.g = as32(g);
+      if (!full && p.gate == LETHE_GATE_CHANNEL) x.g = as_gate(g);
     }
     return (full ? full_with(p, std::move(x), in, true) : apply(p, in, std::move(x), true)).first;
   });

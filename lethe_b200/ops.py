@@ -47,6 +47,7 @@ class _Args(ctypes.Structure):
         ("bh_begin", ctypes.c_uint32), ("bh_count", ctypes.c_uint32), ("qk_f16", ctypes.c_uint32),
         ("c_begin", ctypes.c_uint32), ("c_count", ctypes.c_uint32),
         ("l_tokens", ctypes.c_uint32), ("k_channels", ctypes.c_uint32),
+        ("lean", ctypes.c_uint32),
     ]
 
 
@@ -272,7 +273,6 @@ class GdnStepGraph:
             bb = [0] + list(self.bwd_cuts) + [NT]
             bsegs = [(bb[i], bb[i + 1] - bb[i]) for i in range(len(bb) - 1)]
             SB = len(bsegs)
-            has_wy = buf.dims.delta != 0
             e_p, e_f, e_o = ([None] * S for _ in range(3))
             e_r, e_a = ([None] * SB for _ in range(2))
             with torch.cuda.stream(side):
@@ -309,15 +309,11 @@ class GdnStepGraph:
                 for e in e_o:
                     st.wait_event(e)
                 with torch.cuda.stream(st):
-                    bwd(4, bsegs[i])
-                    if has_wy:
-                        bwd(8, bsegs[i])
+                    bwd(12, bsegs[i])
             for e in e_o:
                 side.wait_event(e)
             with torch.cuda.stream(side):
-                bwd(4, bsegs[0])
-                if has_wy:
-                    bwd(8, bsegs[0])
+                bwd(12, bsegs[0])
             side.wait_event(mark(other))
             side.wait_event(mark(third))
 

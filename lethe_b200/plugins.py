@@ -69,10 +69,6 @@ def _layout(B, H, L, V, gate):
     for n in ("rb", "dh", "dv2", "dw", "dkb", "dgb"):
         off2[n] = o
         o = al(o + Z * sz2[n])
-    if gate == ops.GATE_CHANNEL:
-        for n, size in (("da", 8192), ("dm", 8192), ("dqp", 64 * 128 * 4)):
-            sz2[n], off2[n] = size, o
-            o = al(o + Z * size)
     return Z, sz, off, sz2, off2
 
 
@@ -202,6 +198,7 @@ def k2_fn_cw(k: Tensor, v: Tensor, b: Tensor, w: Tensor, g2: Tensor, t_mat: Tens
     _record_view(buf.scratch, off2["dw"], sz2["dw"], Z, torch.float16).copy_(to_image(dwy.half()).reshape(Z, -1))
     _record_view(buf.scratch, off2["dkb"], sz2["dkb"], Z, f32).zero_()
     _record_view(buf.scratch, off2["dgb"], sz2["dgb"], Z, f32).zero_()
+    _record_view(buf.scratch, off2["rb"], sz2["rb"], Z, f32).zero_()       # what Stage B would have left: nothing
     k16 = _untok(k).to(torch.bfloat16)
     v16 = _untok(v).to(torch.bfloat16)
     g_cum = g2.to(f32) * LN2
