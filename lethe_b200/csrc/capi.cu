@@ -15,7 +15,7 @@ int launch_bwd_pre(const Problem&, const CUtensorMap& mq, const CUtensorMap& mdo
 int launch_bwd_main(const Problem&, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                     const CUtensorMap& mdo, const OutMaps& mo, cudaStream_t, uint32_t mask);
 int launch_bwd_main_cw(const Problem&, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
-                       const CUtensorMap& mdo, const CUtensorMap& mg, cudaStream_t, uint32_t mask);
+                       const CUtensorMap& mdo, const CUtensorMap& mg, const CwOutMaps& mo, cudaStream_t, uint32_t mask);
 
 static bool dims_ok(const LetheGdnDims& d) {
   if (d.B <= 0 || d.H <= 0 || d.L <= 0) return false;
@@ -64,7 +64,7 @@ static int fill_problem(const LetheGdnArgs* a, Problem* p, bool backward) {
     if (d.delta == 1 && !a->dbeta) return kErrNull;
     if (d.delta == 2 && (!a->db_gate || !a->dw_gate)) return kErrNull;
   }
-  if (d.gate == LETHE_GATE_CHANNEL && !aligned16(a->g)) return kErrAlign;      // read through a tensor map
+  if (d.gate == LETHE_GATE_CHANNEL && (!aligned16(a->g) || !aligned16(a->dg))) return kErrAlign;      // read through a tensor map
   const void* ptrs[] = {a->q, a->k, a->v, a->o, a->d_o, a->dq, a->dk, a->dv, a->h0, a->hT, a->dhT, a->dh0,
                         a->saved, a->scratch, a->b_gate, a->w_gate, a->db_gate, a->dw_gate};
   for (const void* x : ptrs)
@@ -174,8 +174,11 @@ extern "C" int lethe_gdn_backward(const LetheGdnArgs* a, void* stream) {
   if (m & 12u) {
     if (p.gate == LETHE_GATE_CHANNEL) {
       CUtensorMap mg;
-      if ((e = gate_map(&mg, a->g, p))) return e;
-      if ((e = launch_bwd_main_cw(p, mq, mk, mv, mdo, mg, st, m))) return e;
+      CwOutMaps mo;
+      if ((e = gate_map(&mg, a->g, p)) || (e = gate_map(&mo.dg, a->dg, p))) return e;
+      if ((e = token_map(&mo.dq, a->dq, p, p.Kr)) || (e = token_map(&mo.dk, a->dk, p, p.Kr))) return e;
+      if ((e = token_map(&mo.dv, a->dv, p, p.V))) return e;
+      if ((e = launch_bwd_main_cw(p, mq, mk, mv, mdo, mg, mo, st, m))) return e;
     } else {
       OutMaps mo;
       if ((e = token_map(&mo.dq, a->dq, p, p.Kr))) return e;

@@ -116,6 +116,12 @@ __device__ __forceinline__ void write_column(unsigned char* tile, int blk, int d
   *reinterpret_cast<uint4*>(tile + sw128_chunk(d, 2 * blk, 128)) = pack8_f16(x);
   *reinterpret_cast<uint4*>(tile + sw128_chunk(d, 2 * blk + 1, 128)) = pack8_f16(x + 8);
 }
+// one 16-bit result of token r into a token-major tile [64 tokens][channels], the image a tensor-map store takes
+__device__ __forceinline__ void stage16(unsigned char* tile, int r, int d, float x, int f16) {
+  *reinterpret_cast<uint16_t*>(tile + sw128_off(r, d, 64)) =
+      f16 ? static_cast<uint16_t>(f16x2_sat(x, 0.f)) : __bfloat16_as_ushort(__float2bfloat16_rn(x));
+}
+
 // 16 columns of block blk of row r of a [token][token] tile (128-byte rows)
 __device__ __forceinline__ void write_row16(unsigned char* tile, int r, int blk, const float* x) {
   *reinterpret_cast<uint4*>(tile + sw128_chunk(r, 2 * blk, 64)) = pack8_f16(x);
@@ -147,11 +153,11 @@ struct CwSmem {
   static constexpr int oV = oQ + 16384;                  // v (times w)                      token-major
   static constexpr int oG = oV + kVT;                    // g as loaded (32 KB); then kd | gamma k, then dw | ...
   static constexpr int oDO = oG + 32768;                 // do                               token-major
-  static constexpr int oDV = oDO + kVT;                  // dv2                              [value channel][token]
+  static constexpr int oDV = oDO + kVT;                  // dv2  [value channel][token]; then dv on its way out
   static constexpr int oTA = oDV + kVT;                  // [T; A]
-  static constexpr int oC = oTA + 16384;                 // v_new; then C0 / C1 by row block
-  static constexpr int oH = oC + 16384;                  // h
-  static constexpr int oDH = oH + V * 256;               // dh; then (b k) e (16 KB), dT / X (8 KB)
+  static constexpr int oC = oTA + 16384;                 // v_new; then C0 / C1 by row block; then dq on its way out
+  static constexpr int oH = oC + 16384;                  // h; then, 32 KB from here, dg on its way out
+  static constexpr int oDH = oH + 32768;                 // dh; then (b k) e (16 KB), dT / X (8 KB); then dk on its way out
   static constexpr int kDH = V * 256 > 24576 ? V * 256 : 24576;
   static constexpr int oCd = oDH + kDH;                  // diagonal blocks of C0, C1 in fp32: [2][64][16]
   static constexpr int oF = oCd + 8192;                  // floats: Bb [4][128], Af [4][128], S [4][128], red [2][4][64], betas [64]
@@ -160,11 +166,13 @@ struct CwSmem {
   static constexpr int CR = WY ? 32 : 16;        // rows of the C tile per row block
 };
 
-template <int V, CwMode MODE>
+// FULL: per-channel erase and write gates (a compile-time choice: a branch on it in every row of the pair sums kept the
+// compiler from overlapping one row with the next, 8.9 k cycles per chunk instead of the 2.9 k of one sum)
+template <int V, CwMode MODE, bool FULL>
 __global__ void __launch_bounds__(kCwThreads, 1)
 bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,
               const __grid_constant__ CUtensorMap mv, const __grid_constant__ CUtensorMap mdo,
-              const __grid_constant__ CUtensorMap mg) {
+              const __grid_constant__ CUtensorMap mg, const __grid_constant__ CwOutMaps mo) {
   constexpr bool SB = MODE != kCwWy, WY = MODE == kCwAll || MODE == kCwWy, DELTA = MODE != kCwNoDelta;
   constexpr bool CUT = MODE == kCwStageB || MODE == kCwWy;
   using S = CwSmem<V, WY>;
@@ -173,6 +181,8 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
   unsigned char* sm = align1024(smem_raw);
   unsigned char *tK = sm + S::oK, *tQ = sm + S::oQ, *tV = sm + S::oV, *tKD = sm + S::oG, *tGK = sm + S::oG + 16384;
   unsigned char *tDW = tKD, *tDO = sm + S::oDO, *tDV = sm + S::oDV, *tTA = sm + S::oTA, *tVN = sm + S::oC, *tC = sm + S::oC;
+  unsigned char *oQt = tC, *oKt = sm + S::oDH, *oVt = tDV;
+  float* oGt = reinterpret_cast<float*>(sm + S::oH);
   unsigned char *tH = sm + S::oH, *tDH = sm + S::oDH, *tBE = sm + S::oDH, *tDT = sm + S::oDH + 16384;
   const float* G = reinterpret_cast<const float*>(sm + S::oG);
   float* Cd0 = reinterpret_cast<float*>(sm + S::oCd);
@@ -187,7 +197,6 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, quad = warp & 3, blk = warp >> 2, d = quad * 32 + lane;
   CtaCtl ctl{p.status, &bars->abort_flag};
   const int nchunks = p.nbh * p.cn;
-  const bool full = p.bch != nullptr;
   struct At { int bh, c, z, b, h; };
   auto at = [&](int n) {
     At a;
@@ -198,7 +207,7 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     a.h = a.bh % p.H;
     return a;
   };
-  // The loads of a chunk, in two parts by when their destinations are free in the chunk before (tid 0 only).
+  // The loads of a chunk, in three parts by when their destinations are free in the chunk before (tid 0 only).
   auto load_part1 = [&](const At& a) {
     mbar_expect_tx(&bars->in0, 32768u + 16384u + 16384u);
     for (int q = 0; q < 4; ++q) tma_load_4d(sm + S::oG + q * 8192, &mg, &bars->in0, q * 32, a.h, a.c * kC, a.b);
@@ -208,16 +217,19 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     else bulk_g2s(tTA + 8192, p.saved + p.lay.ta + static_cast<size_t>(a.z) * 16384 + 8192, 8192, &bars->in1);
     if (SB) {
       for (int t = 0; t < V / 64; ++t) tma_load_4d(tDO + t * 8192, &mdo, &bars->in1, t * 64, a.h, a.c * kC, a.b);
-      bulk_g2s(tH, p.saved + p.lay.hc + static_cast<size_t>(a.z + a.bh) * p.lay.sz_hc, V * 256, &bars->in1);
     }
   };
-  auto load_part2 = [&](const At& a, bool with_dh) {
+  auto load_part2 = [&](const At& a) {
     for (int t = 0; t < 2; ++t) {
       tma_load_4d(tK + t * 8192, &mk, &bars->in0, t * 64, a.h, a.c * kC, a.b);
       tma_load_4d(tQ + t * 8192, &mq, &bars->in0, t * 64, a.h, a.c * kC, a.b);
     }
-    if (SB) bulk_g2s(tVN, p.saved + p.lay.vn + static_cast<size_t>(a.z) * p.lay.sz_vn, V * 128, &bars->in1);
-    if (SB && with_dh) bulk_g2s(tDH, p.scratch + p.lay.dh + static_cast<size_t>(a.z) * p.lay.sz_dh, V * 256, &bars->in1);
+  };
+  auto load_part3 = [&](const At& a, bool with_dh) {
+    if (!SB) return;
+    bulk_g2s(tVN, p.saved + p.lay.vn + static_cast<size_t>(a.z) * p.lay.sz_vn, V * 128, &bars->in1);
+    bulk_g2s(tH, p.saved + p.lay.hc + static_cast<size_t>(a.z + a.bh) * p.lay.sz_hc, V * 256, &bars->in1);
+    if (with_dh) bulk_g2s(tDH, p.scratch + p.lay.dh + static_cast<size_t>(a.z) * p.lay.sz_dh, V * 256, &bars->in1);
   };
 
   if (tid == 0) {
@@ -231,7 +243,8 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     if (SB) {
       const At a = at(blockIdx.x);
       load_part1(a);
-      load_part2(a, false);
+      load_part2(a);
+      load_part3(a, false);
     }
   }
   if (warp == 0) {
@@ -254,7 +267,7 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       bulk_g2s(tDH, p.scratch + p.lay.dh + static_cast<size_t>(a.z) * p.lay.sz_dh, V * 256, &bars->in1);
     } else {
       load_part1(a);
-      load_part2(a, false);
+      load_part2(a);
     }
   }
   const uint32_t aK = smem_u32(tK), aQ = smem_u32(tQ), aC = smem_u32(tC), aBE = smem_u32(tBE);
@@ -266,7 +279,7 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     const size_t tok0 = (static_cast<size_t>(a.b) * p.L + a.c * kC) * p.H + a.h;
     const size_t tokb = tok0 + static_cast<size_t>(blk * 16) * p.H;       // first token of this thread's block
     float beta_r = 1.f;
-    if (WY && !full && tid < 64) beta_r = tid < rows ? p.beta[tok0 + static_cast<size_t>(tid) * p.H] : 0.f;
+    if (WY && !FULL && tid < 64) beta_r = tid < rows ? p.beta[tok0 + static_cast<size_t>(tid) * p.H] : 0.f;
 
     // ---- this thread's column: decays, k, q
     float al[16];
@@ -284,6 +297,10 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       Af[blk * kK + d] = al[0];
     }
     if (WY && tid < 64) betas[tid] = beta_r;
+    if (tid == 0 && n != static_cast<int>(blockIdx.x)) {
+      bulk_wait_read();                             // the results of the chunk before have left their tiles
+      load_part3(a, true);
+    }
     __syncthreads();          // the raw tiles are read, the block products are there
     float cdn[3], cup[3], pre = 1.f, post = 1.f;    // decays: end of block J -> start of this one; end of this -> start of I
     {
@@ -311,9 +328,13 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     auto kv = [&](int i) { return half_of(kp[i >> 1], i & 1); };
     auto qv = [&](int i) { return half_of(qp[i >> 1], i & 1); };
     auto bg = [&](int i) {                          // erase gate of token i of the block
-      if (full) return p.bch[(tokb + static_cast<size_t>(i) * p.H) * kK + d];
-      return betas[blk * 16 + i];
+      return FULL ? p.bch[(tokb + static_cast<size_t>(i) * p.H) * kK + d] : betas[blk * 16 + i];
     };
+    uint32_t bkp[FULL ? 8 : 1];                     // b k
+    if (FULL)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) bkp[j] = f16x2_sat(kv(2 * j) * bg(2 * j), kv(2 * j + 1) * bg(2 * j + 1));
+    auto bkv = [&](int i) { return FULL ? half_of(bkp[FULL ? i >> 1 : 0], i & 1) : kv(i) * bg(i); };
     // ---- operand tiles
     {
       float x[16], e = 1.f, f = 1.f;
@@ -339,8 +360,7 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           if (i) e *= al[i];
-          x[i] = kv(i) * e;
-          if (full) x[i] *= bg(i);
+          x[i] = (FULL ? bkv(i) : kv(i)) * e;
         }
         write_column(tGK, blk, d, x);
       }
@@ -359,7 +379,7 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
         const int r = idx / (V / 8), ch = idx % (V / 8);
         float x[8];
         unpack8_bf16(tile_ld_chunk(tV, r, ch, 64), x);
-        if (full) {
+        if (FULL) {
           float w[8];
           ld8(p.wch + (tok0 + static_cast<size_t>(r) * p.H) * V + ch * 8, w);
 #pragma unroll
@@ -442,8 +462,7 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
               store_f16_sat(dv2_g + sw128_off(blk * 16 + i, d, 64), x[i]);
         } else {
 #pragma unroll
-          for (int i = 0; i < 16; ++i)
-            if (blk * 16 + i < rows) p.dv[(tokb + static_cast<size_t>(i) * p.H) * V + d] = __float2bfloat16_rn(x[i]);
+          for (int i = 0; i < 16; ++i) stage16(oVt, blk * 16 + i, d, x[i], 0);
         }
       }
       mbar_wait_warp(&bars->mB, ph, ctl, 604);      // v_new and dh are dead from here on
@@ -494,7 +513,7 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         if (i) e *= al[i];
-        x[i] = kv(i) * bg(i) * e;
+        x[i] = bkv(i) * e;
       }
       write_column(tBE, blk, d, x);
     }
@@ -542,7 +561,7 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
         float x[16];
         tmem_ld16(cT + lane_base + blk * 16, x);
         tmem_ld_wait();
-        if (!full)
+        if (!FULL)
 #pragma unroll
           for (int j = 0; j < 16; ++j) x[j] *= betas[blk * 16 + j];
         write_row16(tDT, d, blk, x);
@@ -563,20 +582,19 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
         float x[16];
         tmem_ld16(cDBV + lane_base + blk * 16, x);
         tmem_ld_wait();
-        if (full) {
+        if (FULL) {
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
             const size_t o = (tokb + static_cast<size_t>(i) * p.H) * V + d;
             p.dwch[o] = x[i] * __bfloat162float(p.v[o]);
-            p.dv[o] = __float2bfloat16_rn(p.wch[o] * x[i]);
+            stage16(oVt, blk * 16 + i, d, p.wch[o] * x[i], 0);
           }
         } else {
           uint32_t vp[8];
           read_column(tV, blk, d, 1, vp);
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
-            if (blk * 16 + i < rows)
-              p.dv[(tokb + static_cast<size_t>(i) * p.H) * V + d] = __float2bfloat16_rn(betas[blk * 16 + i] * x[i]);
+            stage16(oVt, blk * 16 + i, d, betas[blk * 16 + i] * x[i], 0);
             x[i] *= half_of(vp[i >> 1], i & 1);
           }
           const float s0 = warp_sum8(x, lane), s1 = warp_sum8(x + 8, lane);
@@ -627,9 +645,13 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       sync_for_issue();
       if (tid == 0 && more) {
         load_part1(nx);
-        load_part2(nx, true);
+        load_part2(nx);
       }
       continue;
+    }
+    if (tid == 0) {                                 // dv (written before the last barrier)
+      for (int t = 0; t < V / 64; ++t) tma_store_4d(&mo.dv, oVt + t * 8192, t * 64, a.h, a.c * kC, a.b);
+      bulk_commit();
     }
     // ---- pair sums of the off-diagonal blocks, one accumulator per block pair.  out1: for source block J the rows of
     // all later blocks are neighbours in the C tile; out2: for row block I the columns of all earlier ones are.
@@ -652,7 +674,7 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       umma_commit_led(leader, &bars->mO);
     }
     __syncwarp();
-    if (tid == 0 && more) load_part1(nx);      // g, v, do, h, [T; A]: their tiles are dead
+    if (tid == 0 && more) load_part1(nx);      // g, v, do, [T; A]: their tiles are dead
 
     // ---- diagonal blocks, column sums: rows from the last to the first, sum(s) <- alpha sum(s) + C x
     const float* c0 = Cd0 + blk * 256;
@@ -664,7 +686,7 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     for (int i = 15; i >= 0; --i) {
       f2 xq, xb;
       { const float x = qv(i); xq = pack2(x, x); }
-      if (WY) { const float x = kv(i) * bg(i); xb = pack2(x, x); }
+      if (WY) { const float x = bkv(i); xb = pack2(x, x); }
       const float an = i < 15 ? al[i + 1] : 1.f;
       const f2 dec = pack2(an, an), dec_lo = pack2(an, 1.f);
 #pragma unroll
@@ -686,7 +708,7 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     }
     mbar_wait_warp(&bars->mO, ph, ctl, 610);
     tc_fence_after();
-    if (tid == 0 && more) load_part2(nx, true);   // k, q, v_new, dh: the last products that read those tiles are done
+    if (tid == 0 && more) load_part2(nx);         // k, q: the last products that read those tiles are done
     // dk' without the gate part: de (v_new dh^T) + out2
     float dkp[16];
     {
@@ -721,14 +743,16 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       }
     }
     // ---- diagonal blocks, row sums (kr(s) = k(s) ratio(i, s)), and the gradients of each row; dG replaces dk'
-    const bool dlive = d < p.Kr;
     f2 kr[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) kr[j] = pack2(0.f, 0.f);
     float e = 1.f, dsum = 0.f;
 #pragma unroll
     for (int hf = 0; hf < 2; ++hf) {
-      float o0[8], o1[WY ? 8 : 1], x[8], val[WY ? 8 : 1];
+      float o0[8], o1[WY ? 8 : 1], x[8], val[WY ? 8 : 1], bi[FULL ? 8 : 1];
+      if (FULL)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) bi[i] = bg(8 * hf + i);
       if (SB) {
         tmem_ld8(cDQ + lane_base + blk * 16 + 8 * hf, x);
         tmem_ld_wait();
@@ -748,15 +772,14 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       for (int J = 0; J < 3; ++J) {
         if (J >= blk) continue;
         const uint32_t at1 = cO1 + lane_base + (J == 0 ? 0 : J == 1 ? 3 * CR : 5 * CR) + (blk - 1 - J) * CR + 8 * hf;
+        float y[WY ? 8 : 1];
         tmem_ld8(at1, x);
+        if (WY) tmem_ld8(at1 + 16, y);
         tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 8; ++i) o0[i] = fmaf(cdn[J], x[i], o0[i]);
-        if (WY) {
-          tmem_ld8(at1 + 16, x);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 8; ++i) o1[i] = fmaf(cdn[J], x[i], o1[i]);
+        for (int i = 0; i < 8; ++i) {
+          o0[i] = fmaf(cdn[J], x[i], o0[i]);
+          if (WY) o1[i] = fmaf(cdn[J], y[i], o1[i]);
         }
       }
 #pragma unroll
@@ -765,7 +788,7 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
         const float ai = i ? al[i] : 1.f, k_i = kv(i);
         e *= ai;
         const f2 dec = pack2(ai, ai);
-        f2 s0 = pack2(0.f, 0.f), s1 = s0;
+        f2 s0[2] = {pack2(0.f, 0.f), pack2(0.f, 0.f)}, s1[2] = {s0[0], s0[0]};     // two chains each
 #pragma unroll
         for (int j4 = 0; j4 <= i / 4; ++j4) {
           f2 u0[2], u1[2];
@@ -782,27 +805,25 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
             } else {
               kr[j] = pack2(k_i, 0.f);
             }
-            s0 = fma2(u0[t], kr[j], s0);
-            if (WY) s1 = fma2(u1[t], kr[j], s1);
+            s0[t] = fma2(u0[t], kr[j], s0[t]);
+            if (WY) s1[t] = fma2(u1[t], kr[j], s1[t]);
           }
         }
-        const bool out = dlive && blk * 16 + i < rows;
-        const size_t o = (tokb + static_cast<size_t>(i) * p.H) * p.Kr + d;
-        const float dq = fmaf(e, o0[i8], sum2(s0));
+        const float dq = fmaf(e, o0[i8], sum2(s0[0]) + sum2(s0[1]));
         float dk = dkp[i], dG = fmaf(qv(i), dq, -k_i * dk);
-        if (out) store_out16(p.dq + o, dq, p.qk16);
+        stage16(oQt, blk * 16 + i, d, dq, p.qk16);
         if (WY) {
-          const float dbk = fmaf(e, o1[i8], sum2(s1)), b_i = bg(i);
-          dG = fmaf(k_i * b_i, dbk, dG);
-          dk = fmaf(b_i, dbk, dk);
+          const float dbk = fmaf(e, o1[i8], sum2(s1[0]) + sum2(s1[1]));
+          dG = fmaf(bkv(i), dbk, dG);
+          dk = fmaf(FULL ? bi[FULL ? i8 : 0] : bg(i), dbk, dk);
           val[i8] = dbk * k_i;
-          if (full) p.dbch[o] = val[i8];
+          if (FULL) p.dbch[(tokb + static_cast<size_t>(i) * p.H) * kK + d] = val[i8];
         }
-        if (out) store_out16(p.dk + o, dk, p.qk16);
+        stage16(oKt, blk * 16 + i, d, dk, p.qk16);
         dsum += dG;
         dkp[i] = dG;
       }
-      if (WY && !full) {
+      if (WY && !FULL) {
         const float s = warp_sum8(val, lane);
         if ((lane & 3) == 0) red[quad * 64 + blk * 16 + 8 * hf + (lane >> 2)] = s;
       }
@@ -821,10 +842,20 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
 #pragma unroll
       for (int i = 15; i >= 0; --i) {
         acc += dkp[i];
-        if (dlive && blk * 16 + i < rows) p.dg[(tokb + static_cast<size_t>(i) * p.H) * p.Kr + d] = acc;
+        oGt[quad * 2048 + (blk * 16 + i) * 32 + lane] = acc;
       }
     }
-    if (WY && !full && tid < rows) {
+    fence_proxy_async();
+    __syncthreads();
+    if (tid == 0) {
+      for (int t = 0; t < p.Kr / 64; ++t) {
+        tma_store_4d(&mo.dq, oQt + t * 8192, t * 64, a.h, a.c * kC, a.b);
+        tma_store_4d(&mo.dk, oKt + t * 8192, t * 64, a.h, a.c * kC, a.b);
+      }
+      for (int t = 0; t < p.Kr / 32; ++t) tma_store_4d(&mo.dg, oGt + t * 2048, t * 32, a.h, a.c * kC, a.b);
+      bulk_commit();
+    }
+    if (WY && !FULL && tid < rows) {
       const float er = (red[tid] + red[64 + tid]) + (red[128 + tid] + red[192 + tid]);
       float wr = red[256 + tid] + red[320 + tid];
       if (V == 128) wr += red[384 + tid] + red[448 + tid];
@@ -837,39 +868,42 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       }
     }
   }
+  if (tid == 0) bulk_wait_read();
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
 // ---------------------------------------------------------------------------------------------
-template <int V, CwMode MODE>
+template <int V, CwMode MODE, bool FULL>
 static int launch_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
-                    const CUtensorMap& mdo, const CUtensorMap& mg, cudaStream_t st) {
+                    const CUtensorMap& mdo, const CUtensorMap& mg, const CwOutMaps& mo, cudaStream_t st) {
   constexpr int smem = CwSmem<V, MODE == kCwAll || MODE == kCwWy>::kBytes;
   static_assert(smem <= 232448, "227 KB per CTA");
   static SmemAttr attr;
-  if (attr.set(bwd_cw_kernel<V, MODE>, smem)) return kErrLaunch;
+  if (attr.set(bwd_cw_kernel<V, MODE, FULL>, smem)) return kErrLaunch;
   const int sms = sm_count();
   if (sms <= 0) return kErrDevice;
   const int n = p.nbh * p.cn;
-  if (launch_dependent(bwd_cw_kernel<V, MODE>, dim3(n < sms ? n : sms), dim3(kCwThreads), smem, st, p, mq, mk, mv, mdo, mg) !=
+  if (launch_dependent(bwd_cw_kernel<V, MODE, FULL>, dim3(n < sms ? n : sms), dim3(kCwThreads), smem, st, p, mq, mk, mv, mdo, mg, mo) !=
       cudaSuccess) return kErrLaunch;
   return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
 }
-template <CwMode MODE>
+template <CwMode MODE, bool FULL = false>
 static int launch_v(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
-                    const CUtensorMap& mdo, const CUtensorMap& mg, cudaStream_t st) {
-  return p.V == 64 ? launch_t<64, MODE>(p, mq, mk, mv, mdo, mg, st) : launch_t<128, MODE>(p, mq, mk, mv, mdo, mg, st);
+                    const CUtensorMap& mdo, const CUtensorMap& mg, const CwOutMaps& mo, cudaStream_t st) {
+  return p.V == 64 ? launch_t<64, MODE, FULL>(p, mq, mk, mv, mdo, mg, mo, st) : launch_t<128, MODE, FULL>(p, mq, mk, mv, mdo, mg, mo, st);
 }
 
 // mask bit 4: Stage B, bit 8: WY VJP (delta variants only); both together are one kernel
 int launch_bwd_main_cw(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
-                       const CUtensorMap& mdo, const CUtensorMap& mg, cudaStream_t st, uint32_t mask) {
+                       const CUtensorMap& mdo, const CUtensorMap& mg, const CwOutMaps& mo, cudaStream_t st, uint32_t mask) {
   const bool sb = mask & 4u, wy = (mask & 8u) && p.delta;
-  if (!p.delta) return sb ? launch_v<kCwNoDelta>(p, mq, mk, mv, mdo, mg, st) : kOk;
-  if (sb && wy) return launch_v<kCwAll>(p, mq, mk, mv, mdo, mg, st);
-  return sb ? launch_v<kCwStageB>(p, mq, mk, mv, mdo, mg, st) : launch_v<kCwWy>(p, mq, mk, mv, mdo, mg, st);
+  if (!p.delta) return sb ? launch_v<kCwNoDelta>(p, mq, mk, mv, mdo, mg, mo, st) : kOk;
+  if (sb && !wy) return launch_v<kCwStageB>(p, mq, mk, mv, mdo, mg, mo, st);
+  if (p.bch)
+    return sb ? launch_v<kCwAll, true>(p, mq, mk, mv, mdo, mg, mo, st) : launch_v<kCwWy, true>(p, mq, mk, mv, mdo, mg, mo, st);
+  return sb ? launch_v<kCwAll>(p, mq, mk, mv, mdo, mg, mo, st) : launch_v<kCwWy>(p, mq, mk, mv, mdo, mg, mo, st);
 }
 
 }  // namespace lg

@@ -88,6 +88,9 @@ inline int make_tmap_f32(CUtensorMap* map, const void* ptr, int rank, const uint
 struct OutMaps {
   CUtensorMap dq, dk, dv;
 };
+struct CwOutMaps {
+  CUtensorMap dq, dk, dv, dg;
+};
 
 // Makes the device that owns `ptr` current on the calling thread for the duration of a call and
 // binds its primary context.  A host framework may call from a worker thread that has never touched
