@@ -8,7 +8,7 @@
 
 namespace lg {
 int launch_prepare(const Problem&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, cudaStream_t);
-int launch_prepare_cw(const Problem&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, cudaStream_t);
+int launch_prepare_cw(const Problem&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap& mg, cudaStream_t);
 int launch_output(const Problem&, const CUtensorMap&, cudaStream_t);
 int launch_scan(const Problem&, bool adjoint, cudaStream_t);
 int launch_bwd_pre(const Problem&, const CUtensorMap& mq, const CUtensorMap& mdo, cudaStream_t);
@@ -148,8 +148,12 @@ extern "C" int lethe_gdn_forward(const LetheGdnArgs* a, void* stream) {
   if ((e = token_map(&mk, a->k, p, p.Kr))) return e;
   if ((e = token_map(&mv, a->v, p, p.V))) return e;
   const uint32_t m = a->kernel_mask ? a->kernel_mask : 7u;
-  if ((m & 1u) && (e = (p.gate == LETHE_GATE_CHANNEL ? launch_prepare_cw(p, mq, mk, mv, st)
-                                                     : launch_prepare(p, mq, mk, mv, st)))) return e;
+  if ((m & 1u) && p.gate == LETHE_GATE_CHANNEL) {
+    CUtensorMap mg;
+    if ((e = gate_map(&mg, a->g, p)) || (e = launch_prepare_cw(p, mq, mk, mv, mg, st))) return e;
+  } else if ((m & 1u) && (e = launch_prepare(p, mq, mk, mv, st))) {
+    return e;
+  }
   if ((m & 2u) && (e = launch_scan(p, false, st))) return e;
   if ((m & 4u) && (e = launch_output(p, mq, st))) return e;
   return kOk;

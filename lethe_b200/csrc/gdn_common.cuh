@@ -16,12 +16,9 @@
 //           the final state, so record index is (b*H + h)*(NT + 1) + c
 //     VN    64 x V  image: v_new = u - w h
 //     AD    128 fp32: exp(G_last) per key channel     (the decay of the chunk)
-//     GT    channel-wise gate only: 64 x 128 fp32, the cumulative decay of the chunk in log2 units in the
-//           swizzled shared-memory arrangement of gidx(), written once by prepare and bulk-loaded
-//           by every later kernel instead of being recomputed
 //     QG    channel-wise gate only: 16 KB image, 64 x 128: scale * gamma * q, the query operand of the output
 //           kernel and of the adjoint scan's input kernel (written by prepare, which has q and the gate in
-//           registers anyway, so that those two kernels need neither the 32 KB gate tile nor a conversion)
+//           registers anyway, so that those two kernels need neither the gate nor a conversion)
 //   scratch (backward only)
 //     RB    128 x V fp16 row-major: (q gamma)^T do - w^T (A^T do)
 //     DH    128 x V image: adjoint of the state leaving the chunk
@@ -44,7 +41,7 @@ constexpr int kK = 128;   // key dimension
 
 struct Layout {
   // byte offsets of the record arrays inside `saved` / `scratch`, and record sizes
-  size_t ta, w, u, p, r, hc, vn, ad, gt, qg, carry_f, saved_total;
+  size_t ta, w, u, p, r, hc, vn, ad, qg, carry_f, saved_total;
   size_t rb, dh, dv2, dw, dkb, dgb, carry_b, scratch_total;
   size_t sz_ta, sz_w, sz_u, sz_p, sz_r, sz_hc, sz_vn, sz_ad;
   size_t sz_rb, sz_dh, sz_dv2, sz_dw, sz_dkb, sz_dgb;
@@ -68,7 +65,6 @@ __host__ inline Layout make_layout(const LetheGdnDims& d) {
   l.vn = o; o = align_up(o + Z * l.sz_vn, 1024);
   l.ad = o; o = align_up(o + Z * l.sz_ad, 1024);
   if (d.gate == LETHE_GATE_CHANNEL) {
-    l.gt = o; o = align_up(o + Z * static_cast<size_t>(kC * kK * 4), 1024);
     l.qg = o; o = align_up(o + Z * static_cast<size_t>(16384), 1024);
   }
   // fp32 master state handed from one chunk-range call of the forward scan to the next ([B, H, K, V])
@@ -147,32 +143,7 @@ __device__ __forceinline__ float chunk_rev_cumsum(float x, int tid, float* tmp) 
   return x;
 }
 
-// Channel-wise gate tile: cumulative decay of the chunk in LOG2 units (G * log2 e, so that every decay
-// factor is one exp2 of a difference), 64 rows x 128 channels of fp32 in shared memory.  Element (row, col)
-// lives at gidx(row, col).  A row is 32 pieces of 16 bytes (four channels).  The even pieces - the first
-// halves of the 8-channel groups that match one 16-byte chunk of an fp16 operand tile - come first, then
-// the odd pieces, and within every 128-byte line the pieces are XOR-ed with the low three row bits (the odd
-// half with 4 more).  All three ways the kernels read the tile then run without bank replays:
-//   "lane = chunk of one row" (operand builds): 16 lanes read 16 neighbouring pieces, twice (gt8);
-//   "thread i reads row i" (epilogues): eight neighbouring rows land in eight different pieces of a line;
-//   "thread d walks column d": 32 channels are 4 + 4 pieces in two lines, on disjoint banks.
 constexpr float kLog2e = 1.4426950408889634f;
-__device__ __forceinline__ int gidx(int row, int col) {
-  const int p = col >> 2;
-  const int piece = ((p >> 1) + ((p & 1) << 4)) ^ ((row & 7) ^ ((p & 1) << 2));
-  return row * kK + (piece << 2) + (col & 3);
-}
-// four / eight consecutive gate values of one row (col0 a multiple of 4 / 8)
-__device__ __forceinline__ float4 gt4(const float* Gt, int row, int col0) {
-  return *reinterpret_cast<const float4*>(Gt + gidx(row, col0));
-}
-__device__ __forceinline__ void gt8(const float* Gt, int row, int col0, float* g) {
-  const float4 a = gt4(Gt, row, col0), b = gt4(Gt, row, col0 + 4);
-  g[0] = a.x; g[1] = a.y; g[2] = a.z; g[3] = a.w; g[4] = b.x; g[5] = b.y; g[6] = b.z; g[7] = b.w;
-}
-// fp32 exchange tiles [64][128] (not the gate tile): the column is XOR-ed with the low five row bits, so that
-// both "thread d walks column d" and "thread i walks row i" with scalar accesses are free of bank conflicts
-__device__ __forceinline__ int exi(int row, int col) { return row * kK + (col ^ (row & 31)); }
 
 // Control block at the start of every kernel: barriers, TMEM slot, abort flag.
 struct CtaShared {

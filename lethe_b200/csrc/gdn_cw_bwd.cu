@@ -34,7 +34,7 @@
 // product groups plus CUDA-core phases.  The CTA is persistent and fetches the next chunk's tiles into the ones that
 // are dead once its last products are issued, under the longest CUDA-core phase.  Measured against the four kernels
 // this replaces (Stage B 1, pair sums, WY 1, pair sums; 887 KB of traffic per chunk) in the notes of launch_main.
-#include "gdn_common.cuh"
+#include "gdn_cw.cuh"
 #include "host_util.h"
 
 namespace lg {
@@ -58,92 +58,6 @@ enum CwMode {
 };
 constexpr int kRecDiag = 8192, kRecEnd = kRecDiag + 4096;     // RB: C0 as a 64-row tile, its diagonal blocks, end terms
 __device__ __forceinline__ size_t rec_at(int i, int d) { return static_cast<size_t>(i) * kK + d; }    // DGB, DKB: fp32 [64][128]
-
-// ---- packed pairs of fp32 ----------------------------------------------------------------------------------------
-struct f2 { unsigned long long u; };
-__device__ __forceinline__ f2 pack2(float lo, float hi) {
-  f2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r.u) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack2(f2 a, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.u)); }
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
-  f2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.u) : "l"(a.u), "l"(b.u));
-  return r;
-}
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-  f2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.u) : "l"(a.u), "l"(b.u), "l"(c.u));
-  return r;
-}
-// two neighbouring pairs from shared memory (16-byte aligned)
-__device__ __forceinline__ void ld_pairs(const float* src, f2* out) {
-  const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(src);
-  out[0].u = v.x;
-  out[1].u = v.y;
-}
-__device__ __forceinline__ float sum2(f2 a) {
-  float lo, hi;
-  unpack2(a, lo, hi);
-  return lo + hi;
-}
-
-__device__ __forceinline__ float half_of(uint32_t pair, int hi) {
-  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&pair));
-  return hi ? f.y : f.x;
-}
-__device__ __forceinline__ float in16(uint16_t x, int f16) {
-  if (f16) return __half2float(__ushort_as_half(x));
-  return __uint_as_float(static_cast<uint32_t>(x) << 16);
-}
-__device__ __forceinline__ void store_f16_sat(unsigned char* dst, float x) {
-  *reinterpret_cast<uint16_t*>(dst) = static_cast<uint16_t>(f16x2_sat(x, 0.f));
-}
-// a 16-bit token-major tile [64 tokens][D channels] as TMA leaves it: this thread's 16-token column, as fp16 pairs
-__device__ __forceinline__ void read_column(const unsigned char* tile, int blk, int d, int f16, uint32_t* out) {
-  const unsigned char* base = tile + (d >> 6) * 8192 + blk * 2048 + (d & 7) * 2;
-  const int ch = (d >> 3) & 7;
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const uint16_t a = *reinterpret_cast<const uint16_t*>(base + (2 * j) * 128 + ((ch ^ ((2 * j) & 7)) << 4));
-    const uint16_t b = *reinterpret_cast<const uint16_t*>(base + (2 * j + 1) * 128 + ((ch ^ ((2 * j + 1) & 7)) << 4));
-    out[j] = f16 ? (static_cast<uint32_t>(b) << 16 | a) : f16x2_sat(in16(a, 0), in16(b, 0));
-  }
-}
-// 16 values of this thread's column into a [channel][token] tile (128-byte rows, SW128)
-__device__ __forceinline__ void write_column(unsigned char* tile, int blk, int d, const float* x) {
-  *reinterpret_cast<uint4*>(tile + sw128_chunk(d, 2 * blk, 128)) = pack8_f16(x);
-  *reinterpret_cast<uint4*>(tile + sw128_chunk(d, 2 * blk + 1, 128)) = pack8_f16(x + 8);
-}
-// one 16-bit result of token r into a token-major tile [64 tokens][channels], the image a tensor-map store takes
-__device__ __forceinline__ void stage16(unsigned char* tile, int r, int d, float x, int f16) {
-  *reinterpret_cast<uint16_t*>(tile + sw128_off(r, d, 64)) =
-      f16 ? static_cast<uint16_t>(f16x2_sat(x, 0.f)) : __bfloat16_as_ushort(__float2bfloat16_rn(x));
-}
-
-// 16 columns of block blk of row r of a [token][token] tile (128-byte rows)
-__device__ __forceinline__ void write_row16(unsigned char* tile, int r, int blk, const float* x) {
-  *reinterpret_cast<uint4*>(tile + sw128_chunk(r, 2 * blk, 64)) = pack8_f16(x);
-  *reinterpret_cast<uint4*>(tile + sw128_chunk(r, 2 * blk + 1, 64)) = pack8_f16(x + 8);
-}
-
-// Sums over the 32 lanes of eight values per lane: lane l ends up with the total of value (l >> 2).
-__device__ __forceinline__ float warp_sum8(float* v, int lane) {
-#pragma unroll
-  for (int w = 4, o = 16; w >= 1; w >>= 1, o >>= 1) {
-    const bool up = (lane & o) != 0;
-#pragma unroll
-    for (int j = 0; j < w; ++j) {
-      const float send = up ? v[j] : v[j + w];
-      const float keep = up ? v[j + w] : v[j];
-      v[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-    }
-  }
-  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
-  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
-  return v[0];
-}
 
 template <int V, bool WY>
 struct CwSmem {
@@ -302,28 +216,8 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       load_part3(a, true);
     }
     __syncthreads();          // the raw tiles are read, the block products are there
-    float cdn[3], cup[3], pre = 1.f, post = 1.f;    // decays: end of block J -> start of this one; end of this -> start of I
-    {
-      float bm[4], am[4];
-#pragma unroll
-      for (int m = 0; m < 4; ++m) {
-        bm[m] = Bb[m * kK + d];
-        am[m] = Af[m * kK + d];
-        if (m < blk) pre *= bm[m];
-        if (m > blk) post *= bm[m];
-      }
-#pragma unroll
-      for (int J = 0; J < 3; ++J) {
-        cdn[J] = al[0];
-#pragma unroll
-        for (int m = J + 1; m < 4; ++m)
-          if (m < blk) cdn[J] *= bm[m];
-        cup[J] = am[J + 1];                         // I = J + 1
-#pragma unroll
-        for (int m = 1; m <= J; ++m)
-          if (m > blk) cup[J] *= bm[m];
-      }
-    }
+    const BlockDecays bd = block_decays(Bb, Af, blk, d);
+    const float pre = bd.pre, post = bd.post;
     const float gam0 = pre * al[0];                 // gamma of the block's first token
     auto kv = [&](int i) { return half_of(kp[i >> 1], i & 1); };
     auto qv = [&](int i) { return half_of(qp[i >> 1], i & 1); };
@@ -724,7 +618,7 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
         tmem_ld16(cO2 + lane_base + (I == 1 ? 0 : I == 2 ? 16 : 48) + 16 * blk, x);
         tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 16; ++i) t2[i] = fmaf(cup[I - 1], x[i], t2[i]);
+        for (int i = 0; i < 16; ++i) t2[i] = fmaf(bd.cup[I - 1], x[i], t2[i]);
       }
       if (SB) {
         tmem_ld16(cDK + lane_base + blk * 16, x);
@@ -778,8 +672,8 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
         tmem_ld_wait();
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          o0[i] = fmaf(cdn[J], x[i], o0[i]);
-          if (WY) o1[i] = fmaf(cdn[J], y[i], o1[i]);
+          o0[i] = fmaf(bd.cdn[J], x[i], o0[i]);
+          if (WY) o1[i] = fmaf(bd.cdn[J], y[i], o1[i]);
         }
       }
 #pragma unroll

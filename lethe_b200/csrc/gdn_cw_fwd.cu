@@ -1,455 +1,504 @@
 // Channel-wise gate (one log decay per token, head and key channel): the `prepare` kernel.
 //
 // With a per-channel decay the ratio exp(G_i,d - G_s,d) sits inside the contraction over d, so
-// M[i,s] = beta_i sum_d k[i,d] k[s,d] exp(G_i,d - G_s,d) and A[i,s] are not plain Gram products
-// (reference: gdn2_chunkwise_cw.py:155-157,168-169).  Splitting the ratio as exp(G_i - G_ref) *
-// exp(G_ref - G_s) is only safe when both exponents are <= 0, i.e. when s <= ref <= i.  The 64-token
-// chunk is therefore cut into four blocks of 16 rows:
-//   * row block I against earlier blocks (s < 16 I): reference row a_I = 16 I.  Left operand rows
-//     x[i] exp(G_i - G_{a_I}) (one tile serves all I: blocks are disjoint row ranges), right operand
-//     rows k[s] exp(G_{a_I} - G_s) for s < 16 I (three row ranges packed into one tile).  Three
-//     tcgen05 products with N = 16, 32, 48.
-//   * the four diagonal 16 x 16 blocks: exact per-pair exponentials on the CUDA cores, while the
-//     products run.
-// Everything after M and A (inverse, WY factors, state map) is the scalar-gate kernel's, with
-// per-channel decays in the operand scalings.
-#include "gdn_common.cuh"
+// M[i,s] = beta_i sum_d k[i,d] k[s,d] ratio(i,s)[d] and A[i,s] are not plain Gram products (reference:
+// gdn2_chunkwise_cw.py:155-157,168-169).  The 64-token chunk is cut into four blocks of 16 rows:
+//   * row block I against earlier blocks: left operand rows x[i] e[i], decayed from the first token of their block, right
+//     operand rows k[s] decayed from s to the first token of block I (96 of them for I = 1, 2, 3); tcgen05 products;
+//   * the four diagonal 16 x 16 blocks: exact fp32 sums on the CUDA cores, while the products run.
+// Everything after M and A (inverse, WY factors, state map) is the scalar-gate kernel's, with per-channel decays in the
+// operand scalings.
+//
+// Layout and decays are those of the backward (gdn_cw_bwd.cu): thread (block of 16 tokens, channel) builds its 16-token
+// columns of every decayed operand in registers from alpha = exp(g), the only exponential, and stores them as
+// [channel][token] tiles; ratios are products of alphas.  The diagonal blocks need sums over channels instead: there a
+// half-warp takes the rows j and 15 - j of a block, a lane eight channels of them, and goes down the source rows with
+// ratio(i, s) = ratio(i, s + 1) alpha(s + 1); a source row is loaded once for both rows.
+//
+// The CTA is persistent: the next chunk's k, q and g are fetched as soon as the diagonal sums have read this chunk's, v
+// and the rest behind the second product.
+#include "gdn_cw.cuh"
 #include "host_util.h"
 
 namespace lg {
 
 constexpr int kMsC = 68;
-constexpr int kPrepCwThreads = 256;
+constexpr int kPrepCwThreads = 512;
 constexpr int kDg = 17;                               // row stride (floats) of the diagonal-block buffers
-constexpr int kGateSegs = kPrepCwThreads / 128;       // row segments of the cumulative sum (thread = segment x channel)
-constexpr int kGateRows = kC / kGateSegs;
 
-template <int V, bool DELTA>
-__global__ void __launch_bounds__(kPrepCwThreads)
-prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq,
-                  const __grid_constant__ CUtensorMap mk, const __grid_constant__ CUtensorMap mv) {
+template <int V>
+struct PrepCwSmem {
+  static constexpr int oK = 0;                           // k as loaded (token-major)
+  static constexpr int oQ = oK + 16384;                  // q as loaded
+  static constexpr int oG = oQ + 16384;                  // g as loaded (four boxes of 32 channels); then alpha
+  static constexpr int oV = oG + 32768;                  // v; then beta v (w v)                token-major
+  static constexpr int oLA = oV + V * 128;               // (b) k e | q e  [channel][token]; then M (fp32), then P
+  static constexpr int oKR = oLA + 32768;                // k to the start of block 3 | 1, 2; then [w | u]
+  static constexpr int oGK = oKR + 32768;                // b gamma k   [channel][token]; with kd behind it, then R
+  static constexpr int oKD = oGK + 16384;                // k exp(G_last - G)
+  static constexpr int oTA = oKD + 16384;                // scale gamma q (token-major record); then [T; A]
+  static constexpr int oF = oTA + 16384;
+  // floats: diagonal blocks of A and M [64][kDg] each, betas [64], Bb and Af [4][128]
+  static constexpr int kFloats = 128 * kDg + 64 + 1024;
+  static constexpr int kBytes = oF + kFloats * 4 + static_cast<int>(sizeof(CtaShared)) + 1024;
+};
+
+// Sums over the 16 lanes of a half-warp of N values per lane (N = 16 or 8): lane l ends up with the total of value l
+// (N = 16) or l >> 1 (N = 8).
+template <int N>
+__device__ __forceinline__ float half_warp_sum(float* v, int lane) {
+#pragma unroll
+  for (int w = N / 2, o = 8; w >= 1; w >>= 1, o >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int j = 0; j < w; ++j) {
+      const float send = up ? v[j] : v[j + w];
+      const float keep = up ? v[j + w] : v[j];
+      v[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  if (N == 8) v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+  return v[0];
+}
+// four neighbouring 16-bit values as two packed pairs
+template <bool F16>
+__device__ __forceinline__ void ld4_pairs(const unsigned char* src, f2* out) {
+  const uint2 u = *reinterpret_cast<const uint2*>(src);
+  if (F16) {
+    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&u.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
+    out[0] = pack2(a.x, a.y);
+    out[1] = pack2(b.x, b.y);
+  } else {
+    out[0] = pack2(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u));
+    out[1] = pack2(__uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
+  }
+}
+
+template <int V, bool DELTA, bool FULL, bool F16>
+__global__ void __launch_bounds__(kPrepCwThreads, 1)
+prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,
+                  const __grid_constant__ CUtensorMap mv, const __grid_constant__ CUtensorMap mg) {
+  using S = PrepCwSmem<V>;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* sm = align1024(smem_raw);
-  unsigned char* KQ = sm;                      // 32 KB: rows 0-63 k, 64-127 q (fp16); later M (fp32), then [w | u]
-  unsigned char* LA = KQ + 32768;              // 32 KB: rows 0-63 k exp(G_i - G_a), rows 64-127 q exp(G_i - G_a)
-  unsigned char* KR = LA + 32768;              // 32 KB: rows [0,16) [16,48) [48,96): k exp(G_{a_I} - G_s), I = 1, 2, 3
-  float* Gt = reinterpret_cast<float*>(KR + 32768);   // 32 KB: cumulative log decay [64][128]
-  unsigned char* BGK = reinterpret_cast<unsigned char*>(Gt) + 32768;   // 16 KB
-  unsigned char* BV = BGK + 16384;             // V*128
-  unsigned char* KD = BV + V * 128;            // 16 KB
-  unsigned char* TA = KD + 16384;              // 16 KB
-  float* fs = reinterpret_cast<float*>(TA + 16384);
-  // diagonal blocks of A and of M, [64][16] with rows kDg floats apart: an odd stride keeps both the epilogue's
-  // reads (thread r reads row r) and the diagonal phase's stores off each other's banks
-  float* Adg = fs;
-  float* Mdg = fs + 64 * kDg;
-  float* betas = fs + 128 * kDg;     // [64]
-  CtaShared* cs = reinterpret_cast<CtaShared*>(fs + 128 * kDg + 64);
-  float* Msm = reinterpret_cast<float*>(KQ);
-  unsigned char* WU = KQ;
+  unsigned char *tK = sm + S::oK, *tQ = sm + S::oQ, *BV = sm + S::oV, *LA = sm + S::oLA, *KR = sm + S::oKR, *GK = sm + S::oGK;
+  unsigned char *KD = sm + S::oKD, *TA = sm + S::oTA, *WU = KR, *SP = LA, *SR = GK;
+  float* G = reinterpret_cast<float*>(sm + S::oG);
+  float* Msm = reinterpret_cast<float*>(LA);
+  float* Adg = reinterpret_cast<float*>(sm + S::oF);
+  float* Mdg = Adg + 64 * kDg;
+  float* betas = Mdg + 64 * kDg;
+  float* Bb = betas + 64;
+  float* Af = Bb + 512;
+  CtaShared* cs = reinterpret_cast<CtaShared*>(Af + 512);
 
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const int bh = p.bh0 + blockIdx.x / p.cn, c = p.c0 + blockIdx.x % p.cn, z = bh * p.NT + c, b = bh / p.H, h = bh % p.H;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, quad = warp & 3, blk = warp >> 2, d = quad * 32 + lane;
   CtaCtl ctl{p.status, &cs->abort_flag};
-  uint64_t* bar_load = &cs->bar[0];
-  uint64_t* bar_mma = &cs->bar[1];
-  // Everything that has to come from global memory is requested first - the tensor-map loads of k, q, v by
-  // the thread that has just initialised their barrier, the gate values and beta by every thread - so that
-  // the one memory latency of the chunk overlaps the tensor-memory allocation and the first barrier.
+  uint64_t *in0 = &cs->bar[0], *in1 = &cs->bar[1], *m1 = &cs->bar[2], *m2 = &cs->bar[3], *m3 = &cs->bar[4];
+  const int nchunks = p.nbh * p.cn;
+  struct At { int bh, c, z, b, h; };
+  auto at = [&](int n) {
+    At a;
+    a.bh = p.bh0 + n / p.cn;
+    a.c = p.c0 + n % p.cn;
+    a.z = a.bh * p.NT + a.c;
+    a.b = a.bh / p.H;
+    a.h = a.bh % p.H;
+    return a;
+  };
+  auto load_kqg = [&](const At& a) {      // (tid 0)
+    mbar_expect_tx(in0, 65536u);
+    for (int q = 0; q < 4; ++q) tma_load_4d(sm + S::oG + q * 8192, &mg, in0, q * 32, a.h, a.c * kC, a.b);
+    for (int t = 0; t < 2; ++t) {
+      tma_load_4d(tK + t * 8192, &mk, in0, t * 64, a.h, a.c * kC, a.b);
+      tma_load_4d(tQ + t * 8192, &mq, in0, t * 64, a.h, a.c * kC, a.b);
+    }
+  };
+  auto load_v = [&](const At& a) {
+    mbar_expect_tx(in1, V * 128u);
+    for (int t = 0; t < V / 64; ++t) tma_load_4d(BV + t * 8192, &mv, in1, t * 64, a.h, a.c * kC, a.b);
+  };
   if (tid == 0) {
     cs->abort_flag = 0;
-    mbar_init(bar_load, 1);
-    mbar_init(bar_mma, 1);
+    for (int i = 0; i < 5; ++i) mbar_init(&cs->bar[i], 1);
     fence_mbar_init();
     fence_proxy_async();
-    mbar_expect_tx(bar_load, 32768u + V * 128u);
-    for (int a = 0; a < 2; ++a) {
-      tma_load_4d(KQ + a * 16384, &mk, bar_load, a * 64, h, c * kC, b);
-      tma_load_4d(KQ + a * 16384 + 8192, &mq, bar_load, a * 64, h, c * kC, b);
-    }
-    for (int a = 0; a < V / 64; ++a) tma_load_4d(BV + a * 8192, &mv, bar_load, a * 64, h, c * kC, b);
+    load_kqg(at(blockIdx.x));
+    load_v(at(blockIdx.x));
   }
-  const size_t tok0 = (static_cast<size_t>(b) * p.L + c * kC) * p.H + h;
-  const int seg = tid >> 7;
-  const int rows = p.rows_of(c);
-  float x[kGateRows];
-#pragma unroll
-  for (int i = 0; i < kGateRows; ++i)
-    x[i] = (seg * kGateRows + i < rows && (tid & 127) < p.Kr)
-               ? p.g[(tok0 + static_cast<size_t>(seg * kGateRows + i) * p.H) * p.Kr + (tid & 127)] : 0.f;
-  // full op (per-channel erase gate b, write gate w): the gates enter the operand tiles element by
-  // element and the per-row beta is one
-  const bool full = p.bch != nullptr;
-  float beta_r = 1.f;
-  if (DELTA && tid < rows && !full) beta_r = p.beta[tok0 + static_cast<size_t>(tid) * p.H];
   if (warp == 0) {
-    tmem_alloc(&cs->tmem_slot, 256);
+    tmem_alloc(&cs->tmem_slot, 512);
     tmem_relinquish();
   }
-  if (DELTA && tid < 64) betas[tid] = beta_r;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = cs->tmem_slot;
-  {
-    // cumulative decay: thread (segment of rows, channel) sums its rows, the segment totals are exchanged
-    // through shared memory (Adg is free until the diagonal blocks), every thread adds the totals of the
-    // segments before its own and writes its entries once, in log2 units
-    const int d = tid & 127;
-#pragma unroll
-    for (int i = 1; i < kGateRows; ++i) x[i] += x[i - 1];
-    Adg[seg * kK + d] = x[kGateRows - 1];
-    __syncthreads();
-    float base = 0.f;
-    for (int s2 = 0; s2 < seg; ++s2) base += Adg[s2 * kK + d];
-#pragma unroll
-    for (int i = 0; i < kGateRows; ++i) Gt[gidx(seg * kGateRows + i, d)] = (base + x[i]) * kLog2e;
-    if (seg == kGateSegs - 1)
-      reinterpret_cast<float*>(p.saved + p.lay.ad)[static_cast<size_t>(z) * kK + d] = __expf(base + x[kGateRows - 1]);
-    fence_proxy_async();
-  }
-  __syncthreads();
+  const uint32_t tmem = cs->tmem_slot, lane_base = static_cast<uint32_t>(quad * 32) << 16;
+  const uint32_t cMA = tmem, cWU = tmem + 256, cPR = tmem;       // M | A blocks; [w | u]; [P | R]
 
-  if (tid == 0) {   // the gate tile becomes a record: later kernels load it instead of rebuilding it
-    bulk_s2g(p.saved + p.lay.gt + static_cast<size_t>(z) * (kC * kK * 4), Gt, 32768);
-    bulk_commit();
-  }
-  // ---- operand tiles
-  mbar_wait_warp(bar_load, 0, ctl, 501);
-  for (int idx = tid; idx < 64 * 16; idx += kPrepCwThreads) {
-    const int r = idx >> 4, ch = idx & 15, d0 = ch * 8;
-    const int blk = r >> 4;
-    float kx[8], qx[8], y[8], gr[8], ga[8], gl[8];
-    unpack8_in(tile_ld_chunk(KQ, r, ch, 128), kx, p.qk16);
-    unpack8_in(tile_ld_chunk(KQ, 64 + r, ch, 128), qx, p.qk16);
-    tile_st_chunk(KQ, r, ch, 128, pack8_f16(kx));
-    tile_st_chunk(KQ, 64 + r, ch, 128, pack8_f16(qx));
-    gt8(Gt, r, d0, gr);
-    gt8(Gt, blk * 16, d0, ga);
-    gt8(Gt, 63, d0, gl);
-    float ea[8], bb[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) ea[e] = exp2f(gr[e] - ga[e]);
-    if (DELTA && full) {
-      ld8(p.bch + (tok0 + static_cast<size_t>(r) * p.H) * kK + d0, bb);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) y[e] = kx[e] * bb[e] * ea[e];     // left factor of M is b k
-    } else {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) y[e] = kx[e] * ea[e];
-    }
-    tile_st_chunk(LA, r, ch, 128, pack8_f16(y));
-#pragma unroll
-    for (int e = 0; e < 8; ++e) y[e] = qx[e] * ea[e];
-    tile_st_chunk(LA, 64 + r, ch, 128, pack8_f16(y));
-    // scale * gamma * q for the output kernel and the adjoint scan's input kernel, staged in the [T; A] tile
-    // (not written before the first epilogue) and stored as a record
-#pragma unroll
-    for (int e = 0; e < 8; ++e) y[e] = qx[e] * (p.scale * exp2f(gr[e]));
-    tile_st_chunk(TA, r, ch, 64, pack8_f16(y));
-#pragma unroll
-    for (int e = 0; e < 8; ++e) y[e] = kx[e] * exp2f(gl[e] - gr[e]);
-    tile_st_chunk(KD, r, ch, 64, pack8_f16(y));
-    if (DELTA) {
-      if (!full) {
-        const float be = betas[r];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) bb[e] = be;
-      }
-#pragma unroll
-      for (int e = 0; e < 8; ++e) y[e] = kx[e] * bb[e] * exp2f(gr[e]);
-      tile_st_chunk(BGK, r, ch, 64, pack8_f16(y));
-    }
-    for (int I = blk + 1; I < 4; ++I) {     // row r is a source row for every later row block I
-      const int off = (I == 1) ? 0 : (I == 2 ? 16 : 48);
-      gt8(Gt, I * 16, d0, ga);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) y[e] = kx[e] * exp2f(ga[e] - gr[e]);
-      tile_st_chunk(KR, off + r, ch, 128, pack8_f16(y));
-    }
-  }
-  for (int idx = tid; idx < 64 * (V / 8); idx += kPrepCwThreads) {
-    const int r = idx / (V / 8), ch = idx % (V / 8);
-    float x[8];
-    unpack8_bf16(tile_ld_chunk(BV, r, ch, 64), x);
-    if (DELTA && full) {
-      float wv[8];
-      ld8(p.wch + (tok0 + static_cast<size_t>(r) * p.H) * V + ch * 8, wv);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) x[i] *= wv[i];
-    } else {
-      const float be = DELTA ? betas[r] : 1.f;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) x[i] *= be;
-    }
-    tile_st_chunk(BV, r, ch, 64, pack8_f16(x));
-  }
-  sync_for_issue();
-
-  // ---- off-diagonal blocks on the tensor cores: columns [0,16) I=1, [16,48) I=2, [48,96) I=3
   uint32_t ph = 0;
-  if (warp == 0) {
-    tc_fence_after();
-    const uint32_t leader = elect_leader();
-    issue_product_led(leader, tmem + 0, Tile{smem_u32(LA), 128, false}, Tile{smem_u32(KR), 128, false}, 16, 128, 0u);
-    issue_product_led(leader, tmem + 16, Tile{smem_u32(LA), 128, false}, Tile{smem_u32(KR) + 16 * 128, 128, false}, 32, 128, 0u);
-    issue_product_led(leader, tmem + 48, Tile{smem_u32(LA), 128, false}, Tile{smem_u32(KR) + 48 * 128, 128, false}, 48, 128, 0u);
-    umma_commit_led(leader, bar_mma);
-    if (tid == 0) {
-      bulk_s2g(p.saved + p.lay.qg + static_cast<size_t>(z) * 16384, TA, 16384);
-      bulk_commit();
-    }
-  }
-  __syncwarp();
-  // ---- diagonal blocks, exact: pairs (i, s) of one 16-row block, s <= i, one exp2 per pair and channel.
-  // Thread (block, row pair j, piece c): rows 16 blk + j and 16 blk + 15 - j - together 17 pairs, the same
-  // count for every thread - over channels [8 c, 8 c + 8) and [64 + 8 c, 64 + 8 c + 8): the eight pieces of a
-  // row read eight neighbouring 16-byte chunks of a tile row (and two whole lines of the gate tile), which
-  // keeps the shared-memory pipe - the limit of this phase - free of replays.  The row operands stay in registers while
-  // the source rows stream by; the eight pieces of a pair sit in neighbouring lanes and are added by a
-  // butterfly (fixed order: deterministic).
-  {
-    static_assert(kPrepCwThreads == 256, "8 row pairs (one per warp) x 4 blocks x 8 pieces");
-    // (a warp holds one row pair j of all four blocks: which source row comes next, and when the thread moves
-    // on to its second row, is then the same for every lane)
-    const int c = tid & 7, blk = (tid >> 3) & 3, j = tid >> 5;
-    float qi[16], ki[16], gi[16];
-    auto load_row = [&](int i) {
-      unpack8_f16(tile_ld_chunk(KQ, 64 + i, c, 128), qi);
-      unpack8_f16(tile_ld_chunk(KQ, 64 + i, c + 8, 128), qi + 8);
-      unpack8_f16(tile_ld_chunk(KQ, i, c, 128), ki);
-      unpack8_f16(tile_ld_chunk(KQ, i, c + 8, 128), ki + 8);
-      gt8(Gt, i, 8 * c, gi);
-      gt8(Gt, i, 64 + 8 * c, gi + 8);
-      if (DELTA && full) {
-        float bi[16];
-        const float* bp = p.bch + (tok0 + static_cast<size_t>(i) * p.H) * kK + 8 * c;
-        ld8(bp, bi);
-        ld8(bp + 64, bi + 8);
-#pragma unroll
-        for (int e = 0; e < 16; ++e) ki[e] *= bi[e];
-      }
-    };
-    int i = blk * 16 + j;
-    load_row(i);
-    // (unrolled: the loads of a pair overlap the arithmetic of the pair before it; the partial sums of all 17
-    // pairs stay in registers and are added across the eight pieces at the end, 34 independent butterflies
-    // instead of one after every pair)
-    float pa[17], pm[17];
-#pragma unroll
-    for (int t = 0; t < 17; ++t) {
-      if (t == j + 1) {               // the first row's pairs are done: on to the mirrored row
-        i = blk * 16 + 15 - j;
-        load_row(i);
-      }
-      const int ss = (t > j) ? t - j - 1 : t;
-      const int s = blk * 16 + ss;
-      float ks[16], gs[16];
-      unpack8_f16(tile_ld_chunk(KQ, s, c, 128), ks);
-      unpack8_f16(tile_ld_chunk(KQ, s, c + 8, 128), ks + 8);
-      gt8(Gt, s, 8 * c, gs);
-      gt8(Gt, s, 64 + 8 * c, gs + 8);
-      float aa0 = 0.f, aa1 = 0.f, mm0 = 0.f, mm1 = 0.f;
-#pragma unroll
-      for (int e = 0; e < 16; e += 2) {
-        const float k0 = ks[e] * exp2f(gi[e] - gs[e]);
-        const float k1 = ks[e + 1] * exp2f(gi[e + 1] - gs[e + 1]);
-        aa0 = fmaf(qi[e], k0, aa0);
-        aa1 = fmaf(qi[e + 1], k1, aa1);
-        mm0 = fmaf(ki[e], k0, mm0);
-        mm1 = fmaf(ki[e + 1], k1, mm1);
-      }
-      pa[t] = aa0 + aa1;
-      pm[t] = mm0 + mm1;
-    }
-#pragma unroll
-    for (int o = 1; o < 8; o <<= 1) {
-#pragma unroll
-      for (int t = 0; t < 17; ++t) {
-        pa[t] += __shfl_xor_sync(0xffffffffu, pa[t], o);
-        pm[t] += __shfl_xor_sync(0xffffffffu, pm[t], o);
-      }
-    }
-    if (c == 0) {
-#pragma unroll
-      for (int t = 0; t < 17; ++t) {
-        const int row = (t > j) ? blk * 16 + 15 - j : blk * 16 + j;
-        const int ss = (t > j) ? t - j - 1 : t;
-        const int ii = row - blk * 16;
-        Adg[row * kDg + ss] = p.scale * pa[t];
-        Mdg[row * kDg + ss] = (DELTA && ss < ii) ? betas[row] * pm[t] : 0.f;
-      }
-    }
-  }
-  if (tid == 0) bulk_wait_read();      // the query record has left the [T; A] tile, which the epilogue now fills
-  __syncthreads();
-  wait_products(bar_mma, ph, ctl, 502);
-  const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
-  {
-    // thread t & 127 owns accumulator lane t & 127 (row r of M for lanes 0-63, of A for lanes 64-127); the two
-    // warps that reach a lane quadrant split the row's 64 columns in halves
-    const int t = tid & 127, half = tid >> 7;
-    float d[96];
-    tmem_ld32(tmem + lane_base, d);
-    tmem_ld32(tmem + lane_base + 32, d + 32);
-    tmem_ld32(tmem + lane_base + 64, d + 64);
-    tmem_ld_wait();
-    const int r = t & 63, I = r >> 4;
-    float row[32];                       // this half's off-diagonal values: columns [32 half, 32 half + 32)
-#pragma unroll
-    for (int s = 0; s < 32; ++s) row[s] = 0.f;
-    if (half == 0) {
-      if (I == 1) {
-#pragma unroll
-        for (int s = 0; s < 16; ++s) row[s] = d[s];
-      } else if (I == 2) {
-#pragma unroll
-        for (int s = 0; s < 32; ++s) row[s] = d[16 + s];
-      } else if (I == 3) {
-#pragma unroll
-        for (int s = 0; s < 32; ++s) row[s] = d[48 + s];
-      }
-    } else if (I == 3) {
-#pragma unroll
-      for (int s = 0; s < 16; ++s) row[s] = d[80 + s];
-    }
-    if (t < 64) {
-      if (DELTA) {
-        const float be = betas[r];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const int s = half * 32 + j;
-          float m = row[j] * be;                               // off-diagonal blocks (zero beyond 16 I)
-          if ((s >> 4) == I) m = (s < r) ? Mdg[r * kDg + (s & 15)] : 0.f;
-          Msm[r * kMsC + s] = m;
-        }
-      }
-    } else {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int s8 = half * 4 + q;
-        float a[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const int s = s8 * 8 + e;
-          float x = row[q * 8 + e] * p.scale;
-          if ((s >> 4) == I) x = (s <= r) ? Adg[r * kDg + (s & 15)] : 0.f;
-          a[e] = x;
-        }
-        tile_st_chunk(TA, 64 + r, s8, 128, pack8_f16(a));
-      }
-    }
-  }
-  tc_fence_before();
-  __syncthreads();
+  for (int n = blockIdx.x; n < nchunks; n += gridDim.x, ph ^= 1u) {
+    const At a = at(n);
+    const bool more = n + static_cast<int>(gridDim.x) < nchunks;
+    const At nx = at(more ? n + gridDim.x : n);
+    const int rows = p.rows_of(a.c);
+    const size_t tok0 = (static_cast<size_t>(a.b) * p.L + a.c * kC) * p.H + a.h;
+    float beta_r = 1.f;
+    if (DELTA && !FULL && tid < 64) beta_r = tid < rows ? p.beta[tok0 + static_cast<size_t>(tid) * p.H] : 0.f;
 
-  // ---- T = (I + M)^-1 (fp32, CUDA cores)
-  if (DELTA) {
-    unit_lower_inverse64_blocked<kMsC>(Msm, Msm + 64 * kMsC, TA, tid);
-  } else if (tid < 64) {
+    // ---- this thread's column: decays, k, q
+    float al[16];
+    uint32_t kp[8], qp[8];
+    mbar_wait_warp(in0, ph, ctl, 501);
     {
+      float B = 1.f;
 #pragma unroll
-      for (int i = 0; i < 64; ++i)
-        *reinterpret_cast<__half*>(TA + sw128_off(i, tid, 128)) = __float2half_rn((i == tid) ? 1.f : 0.f);
+      for (int i = 0; i < 16; ++i) {
+        float* gi = G + quad * 2048 + (blk * 16 + i) * 32 + lane;
+        al[i] = exp2f(*gi * kLog2e);
+        *gi = al[i];                       // for the diagonal sums
+        B *= al[i];
+      }
+      Bb[blk * kK + d] = B;
+      Af[blk * kK + d] = al[0];
     }
-  }
-  sync_for_issue();
+    read_column(tK, blk, d, F16, kp);
+    read_column(tQ, blk, d, F16, qp);
+    if (DELTA && tid < 64) betas[tid] = beta_r;
+    if (tid == 0) bulk_wait_read();        // the chunk before has left its staging tiles
+    __syncthreads();
+    const BlockDecays bd = block_decays(Bb, Af, blk, d);
+    const float gam0 = bd.pre * al[0];     // gamma of the block's first token
+    if (blk == 3) reinterpret_cast<float*>(p.saved + p.lay.ad)[static_cast<size_t>(a.z) * kK + d] = bd.pre * Bb[3 * kK + d];
+    auto kv = [&](int i) { return half_of(kp[i >> 1], i & 1); };
+    auto qv = [&](int i) { return half_of(qp[i >> 1], i & 1); };
+    // ---- operand tiles
+    {
+      float x[16], y[16], f = 1.f, e = 1.f;
+#pragma unroll
+      for (int i = 15; i >= 0; --i) {
+        x[i] = kv(i) * f;                  // k to the end of its block
+        f *= al[i];
+      }
+#pragma unroll
+      for (int i = 0; i < 16; ++i) y[i] = x[i] * bd.post;
+      write_column(KD, blk, d, y);
+#pragma unroll
+      for (int I = 1; I < 4; ++I) {        // ... and on to the start of every later block
+        if (I <= blk) continue;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) y[i] = x[i] * bd.cup[I - 1];
+        // columns: block 3's 48 and block 1's 16 in the first atom, block 2's 32 in the second
+        unsigned char* t = KR + (I == 2 ? 16384 : 0);
+        write_column(t, I == 1 ? 3 : blk, d, y);
+      }
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        if (i) e *= al[i];
+        y[i] = qv(i) * e;
+        stage16(TA, blk * 16 + i, d, y[i] * (p.scale * gam0), 1);
+      }
+      write_column(LA + 16384, blk, d, y);
+      e = 1.f;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        if (i) e *= al[i];
+        x[i] = kv(i) * e;
+        if (FULL) x[i] *= p.bch[(tok0 + static_cast<size_t>(blk * 16 + i) * p.H) * kK + d];
+      }
+      write_column(LA, blk, d, x);         // left factor of M (without the row's beta)
+      if (DELTA) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) x[i] *= FULL ? gam0 : gam0 * betas[blk * 16 + i];
+        write_column(GK, blk, d, x);
+      }
+    }
+    mbar_wait_warp(in1, ph, ctl, 505);
+    for (int idx = tid; idx < 64 * (V / 8); idx += kPrepCwThreads) {
+      const int r = idx / (V / 8), ch = idx % (V / 8);
+      float x[8];
+      unpack8_bf16(tile_ld_chunk(BV, r, ch, 64), x);
+      if (DELTA && FULL) {
+        float wv[8];
+        ld8(p.wch + (tok0 + static_cast<size_t>(r) * p.H) * V + ch * 8, wv);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] *= wv[i];
+      } else {
+        const float be = DELTA ? betas[r] : 1.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] *= be;
+      }
+      tile_st_chunk(BV, r, ch, 64, pack8_f16(x));
+    }
+    sync_for_issue();
 
-  if (DELTA) {
+    // ---- off-diagonal blocks of M (rows 0-63) and A (rows 64-127) on the tensor cores
     if (warp == 0) {
       tc_fence_after();
       const uint32_t leader = elect_leader();
-      issue_product_led(leader, tmem, Tile{smem_u32(TA), 128, false}, Tile{smem_u32(BGK), 64, true}, 128 + V, 64, 0u);
-      umma_commit_led(leader, bar_mma);
-      if (tid == 0) bulk_s2g(p.saved + p.lay.ta + static_cast<size_t>(z) * p.lay.sz_ta, TA, 16384);
-      if (tid == 0) bulk_commit();
-    }
-    wait_products(bar_mma, ph, ctl, 503);
-    if ((tid & 127) < 64) {     // rows 0-63: lane quadrants 0 and 1; the four warps of a quadrant split the columns
-#pragma unroll 1
-      for (int jb = tid >> 7; jb < (128 + V) / 32; jb += kPrepCwThreads / 128) {
-        float d[32];
-        tmem_ld32(tmem + lane_base + jb * 32, d);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 4; ++i) tile_st_chunk(WU, tid & 127, jb * 4 + i, 64, pack8_f16(d + 8 * i));
+      issue_product_led(leader, cMA, Tile{smem_u32(LA), 128, true}, Tile{smem_u32(KR), 128, true}, 64, 128, 0u);
+      issue_product_led(leader, cMA + 64, Tile{smem_u32(LA), 128, true}, Tile{smem_u32(KR) + 16384, 128, true}, 32, 128, 0u);
+      umma_commit_led(leader, m1);
+      if (tid == 0) {
+        bulk_s2g(p.saved + p.lay.qg + static_cast<size_t>(a.z) * 16384, TA, 16384);
+        bulk_commit();
       }
     }
-    sync_for_issue();
-  } else if (tid == 0) {
-    bulk_s2g(p.saved + p.lay.ta + static_cast<size_t>(z) * p.lay.sz_ta, TA, 16384);
-    bulk_commit();
-  }
-
-  constexpr int N3 = DELTA ? 128 + V : V;
-  if (warp == 0) {
-    tc_fence_after();
-    const uint32_t leader = elect_leader();
-    issue_product_led(leader, tmem, Tile{smem_u32(KD), 64, true}, Tile{smem_u32(DELTA ? WU : BV), 64, true}, N3, 64, 0u);
-    umma_commit_led(leader, bar_mma);
-    if (DELTA) {
-      if (tid == 0) bulk_s2g(p.saved + p.lay.w + static_cast<size_t>(z) * p.lay.sz_w, WU, 16384);
-      if (tid == 0) bulk_s2g(p.saved + p.lay.u + static_cast<size_t>(z) * p.lay.sz_u, WU + 16384, V * 128);
-    } else {
-      if (tid == 0) bulk_s2g(p.saved + p.lay.u + static_cast<size_t>(z) * p.lay.sz_u, BV, V * 128);
-    }
-    if (tid == 0) bulk_commit();
-  }
-  wait_products(bar_mma, ph, ctl, 504);
-  {
-    // P and R are staged as their record images in the two ratio-scaled operand tiles (dead now) and
-    // leave by bulk stores; the two thread halves split the columns.
-    unsigned char* SP = LA;
-    unsigned char* SR = KR;
-    const int tq = tid & 127;
-    // warp w reads the lanes of quadrant w & 3; the four warps of a quadrant split the 32-column blocks
+    __syncwarp();
+    // ---- diagonal blocks, exact.  Half-warp (block, j): rows j and 15 - j - 17 pairs for every j; lane: channels
+    // 4 c .. 4 c + 3 of either half.  Source rows from the last to the first; a row's ratio starts at one on the diagonal
+    // and is zero before it, so a step needs no test.  Four source rows' sums are added over the lanes at once.
+    {
+      const int c = lane & 15, j = warp & 7, db = (warp >> 3) * 2 + (lane >> 4);
+      const float* al0 = G + (c >> 3) * 2048 + 4 * (c & 7);        // alpha of row r: + 32 r; the other half: + 4096
+      const unsigned char* kt = tK + (c & 1) * 8;
+      const unsigned char* qt = tQ + (c & 1) * 8;
+      auto at16 = [&](int r) { return r * 128 + (((c >> 1) ^ (r & 7)) << 4); };
+      const int hi = 15 - j;
+      f2 q1[4], k1[4], q2[4], k2[4];
+      auto load_row = [&](int i, f2* qi, f2* ki) {
+        const int r = db * 16 + i;
+        ld4_pairs<F16>(qt + at16(r), qi);
+        ld4_pairs<F16>(qt + 8192 + at16(r), qi + 2);
+        ld4_pairs<F16>(kt + at16(r), ki);
+        ld4_pairs<F16>(kt + 8192 + at16(r), ki + 2);
+        if (FULL) {
+          const float* bp = p.bch + (tok0 + static_cast<size_t>(r) * p.H) * kK + 4 * c;
+          f2 b[4];
+          ld_pairs(bp, b);
+          ld_pairs(bp + 64, b + 2);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) ki[e] = mul2(ki[e], b[e]);
+        }
+      };
+      load_row(hi, q1, k1);
+      load_row(j, q2, k2);
+      const f2 one = pack2(1.f, 1.f), zero = pack2(0.f, 0.f);
+      f2 r1[4] = {zero, zero, zero, zero}, r2[4] = {zero, zero, zero, zero}, an[4] = {zero, zero, zero, zero};
+      // sums of one row against source row s: A, and M where the delta term wants it
+      auto step = [&](const f2* ks, f2* ratio, const f2* qi, const f2* ki, float& sa, float& sm_) {
+        f2 aa = zero, mm = zero;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const f2 t = mul2(ratio[e], ks[e]);
+          aa = fma2(qi[e], t, aa);
+          if (DELTA) mm = fma2(ki[e], t, mm);
+        }
+        sa = sum2(aa);
+        sm_ = DELTA ? sum2(mm) : 0.f;
+      };
+      auto store = [&](int i, int s, bool is_m, float x) {
+        const int r = db * 16 + i;
+        if (is_m) Mdg[r * kDg + s] = s < i ? betas[r] * x : 0.f;
+        else Adg[r * kDg + s] = p.scale * x;
+      };
 #pragma unroll 1
-    for (int jb = tid >> 7; jb < N3 / 32; jb += kPrepCwThreads / 128) {
-      float d[32];
-      tmem_ld32(tmem + lane_base + jb * 32, d);
+      for (int sg = hi >> 2; sg >= 0; --sg) {
+        const bool both = sg <= (j >> 2);
+        float v[16];
+#pragma unroll
+        for (int u = 3; u >= 0; --u) {
+          const int s = 4 * sg + u, r = db * 16 + s;
+          f2 ks[4], as[4];
+          ld4_pairs<F16>(kt + at16(r), ks);
+          ld4_pairs<F16>(kt + 8192 + at16(r), ks + 2);
+          ld_pairs(al0 + 32 * r, as);
+          ld_pairs(al0 + 32 * r + 4096, as + 2);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) r1[e] = s == hi ? one : mul2(r1[e], an[e]);
+          step(ks, r1, q1, k1, v[u], v[4 + u]);
+          if (both) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) r2[e] = s == j ? one : mul2(r2[e], an[e]);
+            step(ks, r2, q2, k2, v[8 + u], v[12 + u]);
+          }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) an[e] = as[e];
+        }
+        if (both) {
+          const float t = half_warp_sum<16>(v, lane);
+          store((c & 8) ? j : hi, 4 * sg + (c & 3), (c & 4) != 0, t);
+        } else {
+          const float t = half_warp_sum<8>(v, lane);
+          store(hi, 4 * sg + ((c >> 1) & 3), (c & 8) != 0, t);
+        }
+      }
+    }
+    fence_proxy_async();
+    if (tid == 0) bulk_wait_read();        // the query record has left the [T; A] tile, which the epilogue now fills
+    __syncthreads();
+    if (tid == 0 && more) load_kqg(nx);    // k, q and alpha of this chunk are read
+    mbar_wait_warp(m1, ph, ctl, 502);
+    tc_fence_after();
+    {
+      // thread: accumulator lane t = quad * 32 + lane (row r of M for lanes 0-63, of A for 64-127), columns of block blk
+      const int t = d, r = t & 63, I = r >> 4, I0 = 2 * (quad & 1);      // a warp's lanes are rows of blocks I0 and I0 + 1
+      float x[16], y[16];
+#pragma unroll
+      for (int e = 0; e < 16; ++e) x[e] = 0.f;
+      auto col = [](int rb, int cb) { return rb == 1 ? 48 : (rb == 2 ? 64 : 0) + 16 * cb; };
+      if (blk < I0 + 1) {
+        tmem_ld16(cMA + lane_base + col(I0 + 1, blk), y);
+        tmem_ld_wait();
+        if (I == I0 + 1)
+#pragma unroll
+          for (int e = 0; e < 16; ++e) x[e] = y[e];
+      }
+      if (blk < I0) {
+        tmem_ld16(cMA + lane_base + col(I0, blk), y);
+        tmem_ld_wait();
+        if (I == I0)
+#pragma unroll
+          for (int e = 0; e < 16; ++e) x[e] = y[e];
+      }
+      if (t < 64) {
+        if (DELTA) {
+          const float be = betas[r];
+#pragma unroll
+          for (int e = 0; e < 16; ++e) {
+            x[e] *= be;
+            if (I == blk) x[e] = blk * 16 + e < r ? Mdg[r * kDg + e] : 0.f;
+          }
+          float* m = Msm + r * kMsC + blk * 16;
+          st8(m, x);
+          st8(m + 8, x + 8);
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+          x[e] *= p.scale;
+          if (I == blk) x[e] = blk * 16 + e <= r ? Adg[r * kDg + e] : 0.f;
+        }
+        write_row16(TA, 64 + r, blk, x);
+      }
+    }
+    tc_fence_before();
+    __syncthreads();
+
+    // ---- T = (I + M)^-1 (fp32, CUDA cores)
+    if (DELTA) {
+      unit_lower_inverse64_blocked<kMsC>(Msm, Msm + 64 * kMsC, TA, tid);
+      sync_for_issue();
+      // ---- [w | u] = T [b gamma k | beta v]
+      if (warp == 0) {
+        tc_fence_after();
+        const uint32_t leader = elect_leader();
+        issue_product_led(leader, cWU, Tile{smem_u32(TA), 128, false}, Tile{smem_u32(GK), 128, false}, 128, 64, 0u);
+        issue_product_led(leader, cWU + 128, Tile{smem_u32(TA), 128, false}, Tile{smem_u32(BV), 64, true}, V, 64, 0u);
+        umma_commit_led(leader, m2);
+        if (tid == 0) {
+          bulk_s2g(p.saved + p.lay.ta + static_cast<size_t>(a.z) * p.lay.sz_ta, TA, 16384);
+          bulk_commit();
+        }
+      }
+      __syncwarp();
+      mbar_wait_warp(m2, ph, ctl, 503);
+      tc_fence_after();
+      if (tid == 0 && more) load_v(nx);    // v is read
+      if (quad < 2) {                      // rows 0-63; the four warps of a quadrant split the columns
+        for (int jb = blk; jb < (128 + V) / 32; jb += 4) {
+          float x[32];
+          tmem_ld32(cWU + lane_base + jb * 32, x);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 4; ++i) tile_st_chunk(WU, d, jb * 4 + i, 64, pack8_f16(x + 8 * i));
+        }
+      }
+      sync_for_issue();
+    } else {
+      fence_proxy_async();
+      __syncthreads();
+      if (tid == 0) {                      // A only: without the delta term nothing reads T
+        bulk_s2g(p.saved + p.lay.ta + static_cast<size_t>(a.z) * p.lay.sz_ta + 8192, TA + 8192, 8192);
+        bulk_commit();
+      }
+    }
+
+    // ---- [P | R] = kd^T [w | u]   (no delta: R = kd^T v)
+    if (warp == 0) {
+      tc_fence_after();
+      const uint32_t leader = elect_leader();
+      issue_product_led(leader, cPR, Tile{smem_u32(KD), 128, false}, Tile{smem_u32(DELTA ? WU : BV), 64, true}, DELTA ? 128 + V : V, 64, 0u);
+      umma_commit_led(leader, m3);
+      if (tid == 0) {
+        if (DELTA) {
+          bulk_s2g(p.saved + p.lay.w + static_cast<size_t>(a.z) * p.lay.sz_w, WU, 16384);
+          bulk_s2g(p.saved + p.lay.u + static_cast<size_t>(a.z) * p.lay.sz_u, WU + 16384, V * 128);
+        } else {
+          bulk_s2g(p.saved + p.lay.u + static_cast<size_t>(a.z) * p.lay.sz_u, BV, V * 128);
+        }
+        bulk_commit();
+      }
+    }
+    __syncwarp();
+    mbar_wait_warp(m3, ph, ctl, 504);
+    tc_fence_after();
+    // P and R leave as their record images through tiles nothing reads any more; the four warps of a lane quadrant split
+    // the columns
+    for (int jb = blk; jb < (DELTA ? 128 + V : V) / 32; jb += 4) {
+      float x[32];
+      tmem_ld32(cPR + lane_base + jb * 32, x);
       tmem_ld_wait();
       if (DELTA && jb < 4) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) tile_st_chunk(SP, tq, jb * 4 + i, 128, pack8_f16(d + 8 * i));
+        for (int i = 0; i < 4; ++i) tile_st_chunk(SP, d, jb * 4 + i, 128, pack8_f16(x + 8 * i));
       } else {
         const int c8 = (jb - (DELTA ? 4 : 0)) * 4;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          if (DELTA) *reinterpret_cast<uint4*>(SR + rrec_off(tq, c8 + i)) = pack8_f16(d + 8 * i);
-          else tile_st_chunk(SR, tq, c8 + i, 128, pack8_f16(d + 8 * i));     // no delta term: plain tile image
+          if (DELTA) *reinterpret_cast<uint4*>(SR + rrec_off(d, c8 + i)) = pack8_f16(x + 8 * i);
+          else tile_st_chunk(SR, d, c8 + i, 128, pack8_f16(x + 8 * i));      // no delta term: plain tile image
         }
       }
     }
     fence_proxy_async();
+    tc_fence_before();
     __syncthreads();
     if (tid == 0) {
-      if (DELTA) bulk_s2g(p.saved + p.lay.p + static_cast<size_t>(z) * p.lay.sz_p, SP, 32768);
-      bulk_s2g(p.saved + p.lay.r + static_cast<size_t>(z) * p.lay.sz_r, SR, V * 256);
+      if (DELTA) bulk_s2g(p.saved + p.lay.p + static_cast<size_t>(a.z) * p.lay.sz_p, SP, 32768);
+      bulk_s2g(p.saved + p.lay.r + static_cast<size_t>(a.z) * p.lay.sz_r, SR, V * 256);
       bulk_commit();
+      if (!DELTA && more) {                // v leaves as u: wait for that before the next v comes
+        bulk_wait_read();
+        load_v(nx);
+      }
     }
   }
   if (tid == 0) bulk_wait_read();
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, 256);
+  if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
-template <int V, bool DELTA>
-static int launch_prepare_cw_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk,
-                               const CUtensorMap& mv, cudaStream_t st) {
-  const int smem = 32768 * 4 + 16384 + V * 128 + 16384 + 16384 + (128 * kDg + 64) * 4 +
-                   static_cast<int>(sizeof(CtaShared)) + 1024;
-  auto kern = prepare_cw_kernel<V, DELTA>;
+template <int V, bool DELTA, bool FULL, bool F16>
+static int launch_prepare_cw_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
+                               const CUtensorMap& mg, cudaStream_t st) {
+  constexpr int smem = PrepCwSmem<V>::kBytes;
+  static_assert(smem <= 232448, "227 KB per CTA");
+  auto kern = prepare_cw_kernel<V, DELTA, FULL, F16>;
   static SmemAttr attr;
   if (attr.set(kern, smem)) return kErrLaunch;
-  kern<<<p.nbh * p.cn, kPrepCwThreads, smem, st>>>(p, mq, mk, mv);
+  const int sms = sm_count(), n = p.nbh * p.cn;
+  if (sms <= 0) return kErrDevice;
+  kern<<<n < sms ? n : sms, kPrepCwThreads, smem, st>>>(p, mq, mk, mv, mg);
   return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
+}
+template <int V, bool DELTA, bool FULL>
+static int launch_prepare_cw_f(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
+                               const CUtensorMap& mg, cudaStream_t st) {
+  return p.qk16 ? launch_prepare_cw_t<V, DELTA, FULL, true>(p, mq, mk, mv, mg, st)
+                : launch_prepare_cw_t<V, DELTA, FULL, false>(p, mq, mk, mv, mg, st);
+}
+template <int V>
+static int launch_prepare_cw_v(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
+                               const CUtensorMap& mg, cudaStream_t st) {
+  if (!p.delta) return launch_prepare_cw_f<V, false, false>(p, mq, mk, mv, mg, st);
+  return p.bch ? launch_prepare_cw_f<V, true, true>(p, mq, mk, mv, mg, st) : launch_prepare_cw_f<V, true, false>(p, mq, mk, mv, mg, st);
 }
 
 int launch_prepare_cw(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
-                      cudaStream_t st) {
-  if (p.V == 64) return p.delta ? launch_prepare_cw_t<64, true>(p, mq, mk, mv, st) : launch_prepare_cw_t<64, false>(p, mq, mk, mv, st);
-  return p.delta ? launch_prepare_cw_t<128, true>(p, mq, mk, mv, st) : launch_prepare_cw_t<128, false>(p, mq, mk, mv, st);
+                      const CUtensorMap& mg, cudaStream_t st) {
+  return p.V == 64 ? launch_prepare_cw_v<64>(p, mq, mk, mv, mg, st) : launch_prepare_cw_v<128>(p, mq, mk, mv, mg, st);
 }
 
 }  // namespace lg

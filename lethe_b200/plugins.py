@@ -61,8 +61,6 @@ def _layout(B, H, L, V, gate):
     for n in ("ta", "w", "u", "p", "r", "hc", "vn", "ad"):
         off[n] = o
         o = al(o + (Z + B * H if n == "hc" else Z) * sz[n])
-    if gate == ops.GATE_CHANNEL:
-        sz["gt"], off["gt"] = 64 * 128 * 4, o
     sz2 = dict(rb=128 * V * 2, dh=128 * V * 2, dv2=64 * V * 2, dw=16384, dkb=64 * 128 * 4,
                dgb=(64 * 128 if gate == ops.GATE_CHANNEL else 64) * 4)
     off2, o = {}, 0
@@ -161,21 +159,6 @@ def k2_fn(k: Tensor, v: Tensor, beta: Tensor, g2: Tensor, t_mat: Tensor, dw: Ten
     return dk2.clone(), dv.clone(), db.clone(), dg.clone()
 
 
-def _gate_tile_image(G: Tensor) -> Tensor:
-    """[Z, 64, 128] fp32 cumulative decay in log2 units -> the record image the kernels read (``gidx`` of
-    ``csrc/gdn_common.cuh``): a row is 32 pieces of four channels, even pieces first, then the odd ones, and
-    within each 128-byte line the pieces are XOR-ed with the low three row bits (the odd half with 4 more)."""
-    Z = G.shape[0]
-    row = torch.arange(64, device=G.device)[:, None]
-    col = torch.arange(128, device=G.device)[None, :]
-    p = col >> 2
-    piece = ((p >> 1) + ((p & 1) << 4)) ^ ((row & 7) ^ ((p & 1) << 2))
-    dst = (row * 128 + (piece << 2) + (col & 3)).reshape(-1)
-    img = torch.empty(Z, 64 * 128, dtype=torch.float32, device=G.device)
-    img[:, dst] = G.reshape(Z, -1)
-    return img
-
-
 def k2_fn_cw(k: Tensor, v: Tensor, b: Tensor, w: Tensor, g2: Tensor, t_mat: Tensor, dwy: Tensor, du: Tensor
              ) -> tuple[Tensor, Tensor, Tensor, Tensor, Tensor]:
     """Channel-wise K#2 with independent per-channel erase gate ``b`` and write gate ``w`` (reference
@@ -193,7 +176,6 @@ def k2_fn_cw(k: Tensor, v: Tensor, b: Tensor, w: Tensor, g2: Tensor, t_mat: Tens
     ta = torch.zeros(B, H, NT, 128, 64, dtype=torch.float16, device=dev)
     ta[..., :64, :] = t_mat.half()
     _record_view(buf.saved, off["ta"], sz["ta"], Z, torch.float16).copy_(to_image(ta).reshape(Z, -1))
-    _record_view(buf.saved, off["gt"], sz["gt"], Z, f32).copy_(_gate_tile_image(g2.to(f32).reshape(Z, C, K)))
     _record_view(buf.scratch, off2["dv2"], sz2["dv2"], Z, torch.float16).copy_(to_image(du.half()).reshape(Z, -1))
     _record_view(buf.scratch, off2["dw"], sz2["dw"], Z, torch.float16).copy_(to_image(dwy.half()).reshape(Z, -1))
     _record_view(buf.scratch, off2["dkb"], sz2["dkb"], Z, f32).zero_()
