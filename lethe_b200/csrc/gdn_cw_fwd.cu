@@ -305,11 +305,11 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
           ld_pairs(al0 + 32 * r, as);
           ld_pairs(al0 + 32 * r + 4096, as + 2);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) r1[e] = s == hi ? one : mul2(r1[e], an[e]);
+          for (int e = 0; e < 4; ++e) r1[e] = fma2(r1[e], an[e], s == hi ? one : zero);
           step(ks, r1, q1, k1, v[u], v[4 + u]);
           if (both) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) r2[e] = s == j ? one : mul2(r2[e], an[e]);
+            for (int e = 0; e < 4; ++e) r2[e] = fma2(r2[e], an[e], s == j ? one : zero);
             step(ks, r2, q2, k2, v[8 + u], v[12 + u]);
           }
 #pragma unroll
