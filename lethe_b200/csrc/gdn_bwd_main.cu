@@ -1,0 +1,685 @@
+// Scalar gate (and none): the chunk-parallel backward after the adjoint state scan, Stage B and the WY / triangular-inverse
+// VJP in one kernel.  With T = (I + strict_lower(M))^-1, A the masked attention, ratio(i, s) = exp(G_i - G_s), de_i =
+// exp(G_last - G_i), gamma_i = exp(G_i):
+//
+//   dv2 = de (k dh) + A^T do              dA = tril(do v_new^T),  DS = scale ratio dA
+//   dq  = scale gamma (do h^T) + DS k     dw = -dv2 h^T
+//   dT  = beta_s [dv2 v^T + gamma_s dw k^T],   dM = strict_lower(-T^T dT T^T),   dkk = beta_i ratio dM
+//   dv  = beta (T^T dv2)                  dbgk = T^T dw,  p_i = <dbgk_i, k_i>
+//   dk  = de (v_new dh^T) + DS^T q + (dkk + dkk^T) k + beta gamma dbgk
+//   dbeta = <T^T dv2, v> + gamma p + sum_s dM ratio KK
+//   dg = reverse cumulative sum of dG, dG_i = <scale gamma (do h^T), q> + rowsum(dA A) - colsum(dA A) - de_i <v_new, k dh>
+//        + rowsum(dkk KK) - colsum(dkk KK) + beta p gamma,   and at the chunk's last row  exp(G_last) <dh, h> + sum_i dde_i
+//
+// The gate gradient is a reverse cumulative sum in which large terms cancel (row sums against column sums, every -dde_i
+// against the + sum dde of the last row); each such pair is formed from the same fp32 numbers: colsum(dA A)_s =
+// <v_new_s, (A^T do)_s>, sum_d dde = <v_new, de (k dh)>, and both sums of dkk KK come from the same products.
+// Reference: closed Stage B gdn2_assemble.py:521-585 (scalar form), K#2 gdn2_assemble.py:102-147.
+//
+// Layout.  What has a key-channel axis on one side and tokens on the other is computed transposed, [128 channels in the
+// lanes][64 tokens in the columns], so that all rows of the M = 128 products count; what is [token][value channel] or
+// [token][token] keeps tokens in the lanes (64 of 128; for dv2 in lanes 64-127, through views that start 64 rows early).
+// Decays and gates are applied in fp32 in the epilogues; no scaled copy of k, q or v is ever an operand.
+//
+// Two CTAs share an SM at d_v = 64 (256 tensor-memory columns, 109 KB): six dependent product groups per chunk are a chain
+// of latencies that one CTA cannot fill.  CTAs are persistent and fetch the next chunk's tiles as theirs fall free.
+#include "gdn_cw.cuh"
+#include "host_util.h"
+
+namespace lg {
+
+constexpr int kBwdThreads = 256;
+
+// What runs in a launch; a call cut into its two halves (kernel_mask 4, then 8) gives the bits of the uncut one.
+enum ScMode {
+  kScAll,        // the backward with the delta term
+  kScNoDelta,    // without it: no WY half
+  kScStageB,     // up to dq and dw; leaves dv2, dw, v_new dh^T (in DKB), the gate gradient so far (in DGB), DS (in RB, which
+                 // nothing reads after the adjoint scan)
+  kScWy          // the rest, from those records
+};
+
+struct ScBars {
+  uint64_t in0, in1, m1, m2, m3, mV, m4, m5, m6;
+  uint32_t tmem_slot;
+  int abort_flag;
+};
+
+template <int V>
+struct ScSmem {
+  static constexpr int kVT = V * 128;
+  static constexpr int oQ = 0;                      // q; then dk on its way out
+  static constexpr int oK = oQ + 16384;             // k (directly behind q: early view)
+  static constexpr int oDO = oK + 16384;            // do; with v_new behind it, then dq on its way out
+  static constexpr int oVN = oDO + kVT;             // v_new
+  static constexpr int oV = oVN + kVT;              // v; then dv on its way out
+  static constexpr int oT = oV + kVT;               // T; then dkk
+  static constexpr int oA = oT + 8192;              // A (directly behind T: early view); then DS
+  static constexpr int oH = oA + 8192;              // h; then dw [channel][token]
+  static constexpr int oDH = oH + V * 256;          // dh; then dv2 [token][V], and dT / X behind it
+  static constexpr int oF = oDH + V * 256;
+  // floats: G, beta, de, beta gamma [64] each; t1q [4][64], pq [4][64]; t2p, t3p, ddep, rsp, dbm, rvp [2][64] each;
+  // csp [2][64]; red [16]
+  static constexpr int kFloats = 4 * 64 + 2 * 256 + 7 * 128 + 16;
+  // An A operand of 64 rows is read as 128: 16 KB from the start of its tile.  The last one is dT / X, kVT into dh.
+  static constexpr int kUsed = oF + kFloats * 4 + static_cast<int>(sizeof(ScBars)), kRead = oDH + kVT + 16384;
+  static constexpr int kBytes = (kUsed > kRead ? kUsed : kRead) + 1024;
+  static constexpr uint32_t kCols = V == 64 ? 256u : 512u;
+};
+
+// 32 values per lane: their sums over the warp's lanes; lane l gets the total of value 8 u + (l >> 2) in out[u]
+__device__ __forceinline__ void warp_sum32(float* v, int lane, float* out) {
+#pragma unroll
+  for (int u = 0; u < 4; ++u) out[u] = warp_sum8(v + 8 * u, lane);
+}
+
+template <int V, ScMode MODE>
+__global__ void __launch_bounds__(kBwdThreads, V == 64 ? 2 : 1)
+bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,
+              const __grid_constant__ CUtensorMap mv, const __grid_constant__ CUtensorMap mdo, const __grid_constant__ OutMaps mo) {
+  using S = ScSmem<V>;
+  constexpr bool SB = MODE != kScWy, WY = MODE == kScAll || MODE == kScWy, DELTA = MODE != kScNoDelta;
+  constexpr bool CUT = MODE == kScStageB || MODE == kScWy;
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* sm = align1024(smem_raw);
+  unsigned char *tQ = sm + S::oQ, *tK = sm + S::oK, *tDO = sm + S::oDO, *tVN = sm + S::oVN, *tV = sm + S::oV, *tT = sm + S::oT;
+  unsigned char *tA = sm + S::oA, *tDS = tA, *tH = sm + S::oH, *tDW = tH, *tDH = sm + S::oDH, *tDV = tDH;
+  unsigned char *tX = tDH + S::kVT, *tKKd = tT, *oQt = tDO, *oKt = tQ, *oVt = tV;
+  float* Gs = reinterpret_cast<float*>(sm + S::oF);
+  float *betas = Gs + 64, *decs = betas + 64, *bgs = decs + 64, *t1q = bgs + 64, *pq = t1q + 256;
+  float *t2p = pq + 256, *t3p = t2p + 128, *ddep = t3p + 128, *rsp = ddep + 128, *dbm = rsp + 128, *rvp = dbm + 128, *csp = rvp + 128;
+  float* red = csp + 128;
+  ScBars* bars = reinterpret_cast<ScBars*>(red + 16);
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, quad = warp & 3, half = warp >> 2, d = quad * 32 + lane;
+  const int c0 = half * 32;                       // this thread's 32 tokens / columns of every 64-column accumulator
+  CtaCtl ctl{p.status, &bars->abort_flag};
+  const int nchunks = p.nbh * p.cn;
+  struct At { int bh, c, z, b, h; };
+  auto at = [&](int n) {
+    At a;
+    a.bh = p.bh0 + n / p.cn;
+    a.c = p.c0 + n % p.cn;
+    a.z = a.bh * p.NT + a.c;
+    a.b = a.bh / p.H;
+    a.h = a.bh % p.H;
+    return a;
+  };
+  // loads of a chunk (tid 0), by when their destinations fall free in the chunk before
+  constexpr uint32_t kIn0 = 32768u + (WY ? V * 128u : 0u) + (DELTA ? 16384u : 8192u) + (SB ? 2u * V * 128 + V * 256 : V * 128u);
+  auto load_a = [&](const At& a) {                // do, v_new, v, h (dv2 where the first half of the call left it)
+    mbar_expect_tx(&bars->in0, kIn0);
+    for (int t = 0; t < V / 64; ++t) {
+      if (SB) {
+        tma_load_4d(tDO + t * 8192, &mdo, &bars->in0, t * 64, a.h, a.c * kC, a.b);
+        if (DELTA) bulk_g2s(tVN + t * 8192, p.saved + p.lay.vn + static_cast<size_t>(a.z) * p.lay.sz_vn + t * 8192, 8192, &bars->in0);
+        else tma_load_4d(tVN + t * 8192, &mv, &bars->in0, t * 64, a.h, a.c * kC, a.b);      // v_new is v
+      }
+      if (WY) tma_load_4d(tV + t * 8192, &mv, &bars->in0, t * 64, a.h, a.c * kC, a.b);
+    }
+    if (SB) bulk_g2s(tH, p.saved + p.lay.hc + static_cast<size_t>(a.z + a.bh) * p.lay.sz_hc, V * 256, &bars->in0);
+    else bulk_g2s(tDV, p.scratch + p.lay.dv2 + static_cast<size_t>(a.z) * p.lay.sz_dv2, V * 128, &bars->in0);
+  };
+  auto load_dh = [&](const At& a) {
+    mbar_expect_tx(&bars->in1, V * 256u);
+    bulk_g2s(tDH, p.scratch + p.lay.dh + static_cast<size_t>(a.z) * p.lay.sz_dh, V * 256, &bars->in1);
+  };
+  auto load_b = [&](const At& a) {                // [T; A], k
+    const unsigned char* ta = p.saved + p.lay.ta + static_cast<size_t>(a.z) * p.lay.sz_ta;
+    if (DELTA) bulk_g2s(tT, ta, 16384, &bars->in0);
+    else bulk_g2s(tA, ta + 8192, 8192, &bars->in0);
+    for (int t = 0; t < 2; ++t) tma_load_4d(tK + t * 8192, &mk, &bars->in0, t * 64, a.h, a.c * kC, a.b);
+  };
+  auto load_q = [&](const At& a) {
+    for (int t = 0; t < 2; ++t) tma_load_4d(tQ + t * 8192, &mq, &bars->in0, t * 64, a.h, a.c * kC, a.b);
+  };
+
+  if (tid == 0) {
+    bars->abort_flag = 0;
+    mbar_init(&bars->in0, 1); mbar_init(&bars->in1, 1); mbar_init(&bars->m1, 2); mbar_init(&bars->m2, 2);
+    mbar_init(&bars->m3, 1); mbar_init(&bars->mV, 1); mbar_init(&bars->m4, 1); mbar_init(&bars->m5, 1); mbar_init(&bars->m6, 1);
+    fence_mbar_init();
+    fence_proxy_async();
+    if (SB) {                  // everything but dh, which the adjoint scan just before this kernel writes, is older
+      const At a = at(blockIdx.x);
+      load_a(a);
+      load_b(a);
+      load_q(a);
+    }
+  }
+  if (warp == 0) {
+    tmem_alloc(&bars->tmem_slot, S::kCols);
+    tmem_relinquish();
+  }
+  float g_next = 0.f, b_next = 1.f;               // gate and beta of token tid of the next chunk
+  auto fetch_gates = [&](const At& a) {
+    g_next = 0.f;
+    b_next = WY ? 0.f : 1.f;
+    if (tid < p.rows_of(a.c)) {
+      const size_t tok = (static_cast<size_t>(a.b) * p.L + a.c * kC + tid) * p.H + a.h;
+      if (p.gate == LETHE_GATE_SCALAR) g_next = p.g[tok];
+      if (WY) b_next = p.beta[tok];
+    }
+  };
+  fetch_gates(at(blockIdx.x));
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = bars->tmem_slot, lane_base = static_cast<uint32_t>(quad * 32) << 16;
+  // columns; an accumulator that shares columns with an earlier one is issued after that one has been read
+  const uint32_t cD = tmem, cAo = tmem + V, cDA = tmem + 2 * V, cDK = tmem + 2 * V + 64;      // k dh, A^T do, dA, (v_new dh^T)^T
+  const uint32_t cDQ = tmem, cDWt = tmem + 64, cQI = tmem + 128;                               // (do h^T)^T, (dv2 h^T)^T, (DS k)^T
+  const uint32_t cT1 = tmem, cT2 = tmem + 64, cBV = V == 64 ? tmem + 128 : tmem + 320 + 64;    // dv2 v^T, dw k^T, T^T dv2
+  const uint32_t cX = tmem, cBK = tmem + 64, cKK = tmem + 128, cAcc = tmem;                    // X / dM, (T^T dw)^T, k k^T, dk sums
+  griddep_wait();
+  griddep_launch();
+  if (tid == 0) {
+    const At a = at(blockIdx.x);
+    if (SB) {
+      load_dh(a);
+    } else {
+      load_a(a);
+      load_b(a);
+      load_q(a);
+    }
+  }
+
+  uint32_t ph = 0;
+  for (int n = blockIdx.x; n < nchunks; n += gridDim.x, ph ^= 1u) {
+    const At a = at(n);
+    const bool more = n + static_cast<int>(gridDim.x) < nchunks;
+    const At nx = at(more ? n + gridDim.x : n);
+    const int rows = p.rows_of(a.c);
+    const size_t tok0 = (static_cast<size_t>(a.b) * p.L + a.c * kC) * p.H + a.h;
+    unsigned char* dv2_g = p.scratch + p.lay.dv2 + static_cast<size_t>(a.z) * p.lay.sz_dv2;
+    unsigned char* dw_g = p.scratch + p.lay.dw + static_cast<size_t>(a.z) * p.lay.sz_dw;
+    unsigned char* rb_g = p.scratch + p.lay.rb + static_cast<size_t>(a.z) * p.lay.sz_rb;
+    float* dkb_g = reinterpret_cast<float*>(p.scratch + p.lay.dkb + static_cast<size_t>(a.z) * p.lay.sz_dkb);
+    float* dgb_g = reinterpret_cast<float*>(p.scratch + p.lay.dgb + static_cast<size_t>(a.z) * p.lay.sz_dgb);
+    const bool keep = CUT || !p.lean;
+
+    // ---- gates
+    if (tid == 0 && n != static_cast<int>(blockIdx.x)) {
+      bulk_wait_read();                             // dk of the chunk before has left the q tile
+      load_q(a);
+    }
+    const float bval = b_next;
+    const float Gt = chunk_cumsum(g_next, tid, red);
+    if (tid < 64) {
+      Gs[tid] = Gt;
+      betas[tid] = bval;
+      bgs[tid] = bval * __expf(Gt);
+    }
+    __syncthreads();
+    const float Glast = Gs[63];
+    if (tid < 64) decs[tid] = __expf(Glast - Gt);
+    if (more) fetch_gates(nx);
+
+    // ---- operands to fp16 in place
+    mbar_wait_warp(&bars->in0, ph, ctl, 411);
+    if (!p.qk16) {
+      for (int idx = tid; idx < 2 * 64 * 16; idx += kBwdThreads) {      // q and k lie behind each other
+        uint4* c = reinterpret_cast<uint4*>(tQ + idx * 16);
+        float x[8];
+        unpack8_bf16(*c, x);
+        *c = pack8_f16(x);
+      }
+    }
+    if (SB) {
+      for (int idx = tid; idx < (DELTA ? 1 : 2) * 64 * (V / 8); idx += kBwdThreads) {      // do (and, without delta, v behind it)
+        uint4* c = reinterpret_cast<uint4*>(tDO + idx * 16);
+        float x[8];
+        unpack8_bf16(*c, x);
+        *c = pack8_f16(x);
+      }
+    }
+    if (WY) {
+      for (int idx = tid; idx < 64 * (V / 8); idx += kBwdThreads) {
+        uint4* c = reinterpret_cast<uint4*>(tV + idx * 16);
+        float x[8];
+        unpack8_bf16(*c, x);
+        *c = pack8_f16(x);
+      }
+    }
+    if (!SB) {                                      // the first half of the call left DS and dw
+      for (int idx = tid; idx < 512; idx += kBwdThreads) reinterpret_cast<uint4*>(tDS)[idx] = reinterpret_cast<const uint4*>(rb_g)[idx];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        float x[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          x[i] = __half2float(*reinterpret_cast<const __half*>(dw_g + sw128_off(c0 + 16 * u + i, d, 64)));
+        write_column(tDW, 2 * half + u, d, x);
+      }
+    }
+    sync_for_issue();
+
+    float dhh = 0.f;
+    if (SB) {
+      mbar_wait_warp(&bars->in1, ph, ctl, 415);
+      // ---- group 1 (two warps issue): k dh (lanes 64-127), (v_new dh^T)^T | A^T do (lanes 64-127), dA
+      if (warp == 0) {
+        tc_fence_after();
+        const uint32_t leader = elect_leader();
+        issue_product_led(leader, cD, Tile{smem_u32(tK) - 8192, 64, false}, Tile{smem_u32(tDH), 128, true}, V, 128, 0u);
+        issue_product_led(leader, cDK, Tile{smem_u32(tDH), 128, false}, Tile{smem_u32(tVN), 64, false}, 64, V, 0u);
+        umma_commit_led(leader, &bars->m1);
+      } else if (warp == 4) {
+        tc_fence_after();
+        const uint32_t leader = elect_leader();
+        issue_product_led(leader, cAo, Tile{smem_u32(tA) - 8192, 64, true}, Tile{smem_u32(tDO), 64, true}, V, 64, 0u);
+        issue_product_led(leader, cDA, Tile{smem_u32(tDO), 64, false}, Tile{smem_u32(tVN), 64, false}, 64, V, 0u);
+        umma_commit_led(leader, &bars->m1);
+      }
+      __syncwarp();
+      // in their shadow: <dh, h>, element by element on two images of one layout
+      for (int idx = tid; idx < kK * V / 8; idx += kBwdThreads) {
+        float x[8], y[8];
+        unpack8_f16(*reinterpret_cast<const uint4*>(tDH + idx * 16), x);
+        unpack8_f16(*reinterpret_cast<const uint4*>(tH + idx * 16), y);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) dhh += x[i] * y[i];
+      }
+      dhh = cta_sum256(dhh, tid, red + 2) * __expf(Glast);      // (its barriers: every thread has read dh)
+      mbar_wait_warp(&bars->m1, ph, ctl, 412);
+      tc_fence_after();
+      if (quad >= 2) {                              // dv2
+        const int r = d - 64;
+        const float de = decs[r];
+        float t3 = 0.f, dde = 0.f;
+#pragma unroll
+        for (int jj = 0; jj < V / 32; ++jj) {
+          const int cb = half * (V / 2) + jj * 16;
+          float x[16], y[16];
+          tmem_ld16(cAo + lane_base + cb, x);
+          tmem_ld16(cD + lane_base + cb, y);
+          tmem_ld_wait();
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            float vn[8];
+            unpack8_f16(tile_ld_chunk(tVN, r, cb / 8 + q, 64), vn);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const float kd_dh = de * y[8 * q + e];
+              t3 += vn[e] * x[8 * q + e];
+              dde += vn[e] * kd_dh;
+              x[8 * q + e] += kd_dh;
+            }
+            if (DELTA) tile_st_chunk(tDV, r, cb / 8 + q, 64, pack8_f16(x + 8 * q));
+            else tile_st_chunk(oVt, r, cb / 8 + q, 64, pack8_bf16(x + 8 * q));
+          }
+        }
+        t3p[half * 64 + r] = t3 + dde;
+        ddep[half * 64 + r] = dde;
+      } else {                                      // dA -> DS, where A was
+        const int r = d;
+        const float Gr = Gs[r];
+        float t2 = 0.f;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          float x[16];
+          tmem_ld16(cDA + lane_base + c0 + 16 * u, x);
+          tmem_ld_wait();
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            const int s8 = c0 / 8 + 2 * u + q;
+            float av[8], y[8];
+            unpack8_f16(tile_ld_chunk(tA, r, s8, 64), av);       // A[r, s] (holds scale * ratio already)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const int s = s8 * 8 + i;
+              const float da = (s <= r) ? x[8 * q + i] : 0.f;
+              t2 += da * av[i];
+              y[i] = (s <= r) ? p.scale * __expf(Gr - Gs[s]) * da : 0.f;
+            }
+            tile_st_chunk(tDS, r, s8, 64, pack8_f16(y));
+          }
+        }
+        t2p[half * 64 + r] = t2;
+      }
+      sync_for_issue();
+
+      // ---- group 2: (do h^T)^T, (DS k)^T | (dv2 h^T)^T
+      if (warp == 0) {
+        tc_fence_after();
+        const uint32_t leader = elect_leader();
+        issue_product_led(leader, cDQ, Tile{smem_u32(tH), 128, false}, Tile{smem_u32(tDO), 64, false}, 64, V, 0u);
+        umma_commit_led(leader, &bars->m2);
+        if (tid == 0) {
+          if (!DELTA) for (int t = 0; t < V / 64; ++t) tma_store_4d(&mo.dv, oVt + t * 8192, t * 64, a.h, a.c * kC, a.b);
+          else if (keep) bulk_s2g(dv2_g, tDV, V * 128);
+          if (CUT) bulk_s2g(rb_g, tDS, 8192);
+          bulk_commit();
+        }
+      } else if (warp == 4) {
+        tc_fence_after();
+        const uint32_t leader = elect_leader();
+        issue_product_led(leader, cQI, Tile{smem_u32(tK), 64, true}, Tile{smem_u32(tDS), 64, false}, 64, 64, 0u);
+        if (DELTA) issue_product_led(leader, cDWt, Tile{smem_u32(tH), 128, false}, Tile{smem_u32(tDV), 64, false}, 64, V, 0u);
+        umma_commit_led(leader, &bars->m2);
+      }
+      __syncwarp();
+      mbar_wait_warp(&bars->m2, ph, ctl, 413);
+      tc_fence_after();
+      float t1[32];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        uint32_t qp[8];
+        float x[16], y[16];
+        read_column(tQ, 2 * half + u, d, 1, qp);
+        tmem_ld16(cDQ + lane_base + c0 + 16 * u, x);
+        tmem_ld16(cQI + lane_base + c0 + 16 * u, y);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const int r = c0 + 16 * u + i;
+          const float dq = p.scale * __expf(Gs[r]) * x[i];
+          t1[16 * u + i] = dq * half_of(qp[i >> 1], i & 1);
+          stage16(oQt, r, d, dq + y[i], p.qk16);
+        }
+        if (DELTA) {
+          tmem_ld16(cDWt + lane_base + c0 + 16 * u, x);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 16; ++i) x[i] = -x[i];
+          if (WY) write_column(tDW, 2 * half + u, d, x);
+          if (keep)
+#pragma unroll
+            for (int i = 0; i < 16; ++i) store_f16_sat(dw_g + sw128_off(c0 + 16 * u + i, d, 64), x[i]);
+        }
+        if (MODE == kScStageB) {
+          tmem_ld16(cDK + lane_base + c0 + 16 * u, x);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 16; ++i) dkb_g[static_cast<size_t>(c0 + 16 * u + i) * kK + d] = x[i];
+        }
+      }
+      {
+        float s[4];
+        warp_sum32(t1, lane, s);
+        if ((lane & 3) == 0)
+#pragma unroll
+          for (int u = 0; u < 4; ++u) t1q[quad * 64 + c0 + 8 * u + (lane >> 2)] = s[u];
+      }
+      sync_for_issue();
+      if (tid == 0) {
+        for (int t = 0; t < p.Kr / 64; ++t) tma_store_4d(&mo.dq, oQt + t * 8192, t * 64, a.h, a.c * kC, a.b);
+        bulk_commit();
+      }
+    }
+    // gate gradient of Stage B (token tid), before the cumulative sum
+    float dG = 0.f;
+    if (SB) {
+      if (tid < 64) {
+        float sdde = ddep[tid] + ddep[64 + tid];    // sum over the chunk's rows, fixed tree
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sdde += __shfl_xor_sync(0xffffffffu, sdde, o);
+        if (lane == 0) red[12 + warp] = sdde;
+        dG = ((t1q[tid] + t1q[64 + tid]) + (t1q[128 + tid] + t1q[192 + tid])) + (t2p[tid] + t2p[64 + tid]) - (t3p[tid] + t3p[64 + tid]);
+      }
+    } else if (tid < 64) {
+      dG = dgb_g[tid];
+    }
+    if (MODE == kScStageB) {
+      __syncthreads();
+      if (tid < 64) dgb_g[tid] = dG + (tid == 63 ? dhh + (red[12] + red[13]) : 0.f);
+      if (tid == 0 && more) {
+        bulk_wait_read();
+        load_a(nx);
+        load_dh(nx);
+        load_b(nx);
+      }
+      tc_fence_before();
+      __syncthreads();
+      continue;
+    }
+    if (WY) {
+      // ---- group 3: dT in two accumulators (its gates are applied in fp32), T^T dv2
+      if (warp == 0) {
+        tc_fence_after();
+        const uint32_t leader = elect_leader();
+        issue_product_led(leader, cT1, Tile{smem_u32(tDV), 64, false}, Tile{smem_u32(tV), 64, false}, 64, V, 0u);
+        issue_product_led(leader, cT2, Tile{smem_u32(tDW), 128, true}, Tile{smem_u32(tK), 64, false}, 64, 128, 0u);
+        umma_commit_led(leader, &bars->m3);
+        issue_product_led(leader, cBV, Tile{smem_u32(tT), 64, true}, Tile{smem_u32(tDV), 64, true}, V, 64, 0u);
+        umma_commit_led(leader, &bars->mV);
+      }
+      __syncwarp();
+      mbar_wait_warp(&bars->m3, ph, ctl, 421);
+      tc_fence_after();
+      if (quad < 2) {
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          float x[16], y[16];
+          tmem_ld16(cT1 + lane_base + c0 + 16 * u, x);
+          tmem_ld16(cT2 + lane_base + c0 + 16 * u, y);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const int s = c0 + 16 * u + j;
+            x[j] = fmaf(bgs[s], y[j], betas[s] * x[j]);
+          }
+          write_row16(tX, d, 2 * half + u, x);
+        }
+      }
+      sync_for_issue();
+      // ---- group 4: X = dT T^T, (T^T dw)^T
+      if (warp == 0) {
+        tc_fence_after();
+        const uint32_t leader = elect_leader();
+        issue_product_led(leader, cX, Tile{smem_u32(tX), 64, false}, Tile{smem_u32(tT), 64, false}, 64, 64, 0u);
+        issue_product_led(leader, cBK, Tile{smem_u32(tDW), 128, false}, Tile{smem_u32(tT), 64, true}, 64, 64, 0u);
+        umma_commit_led(leader, &bars->m4);
+      }
+      __syncwarp();
+      // in its shadow: dv = beta T^T dv2 where v was, and the value part of dbeta
+      mbar_wait_warp(&bars->mV, ph, ctl, 422);
+      tc_fence_after();
+      if (quad < 2) {
+        const int r = d;
+        const float be = betas[r];
+        float rv = 0.f;
+#pragma unroll
+        for (int jj = 0; jj < V / 32; ++jj) {
+          const int cb = half * (V / 2) + jj * 16;
+          float x[16];
+          tmem_ld16(cBV + lane_base + cb, x);
+          tmem_ld_wait();
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            float vv[8];
+            unpack8_f16(tile_ld_chunk(tV, r, cb / 8 + q, 64), vv);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              rv += x[8 * q + e] * vv[e];
+              x[8 * q + e] *= be;
+            }
+            tile_st_chunk(oVt, r, cb / 8 + q, 64, pack8_bf16(x + 8 * q));
+          }
+        }
+        rvp[half * 64 + r] = rv;
+      }
+      mbar_wait_warp(&bars->m4, ph, ctl, 423);
+      tc_fence_after();
+      if (quad < 2) {
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          float x[16];
+          tmem_ld16(cX + lane_base + c0 + 16 * u, x);
+          tmem_ld_wait();
+          write_row16(tX, d, 2 * half + u, x);
+        }
+      }
+      sync_for_issue();
+      // ---- group 5: dM = -T^T X, k k^T
+      if (warp == 0) {
+        tc_fence_after();
+        const uint32_t leader = elect_leader();
+        issue_product_led(leader, cX, Tile{smem_u32(tT), 64, true}, Tile{smem_u32(tX), 64, true}, 64, 64, 0u, true);
+        issue_product_led(leader, cKK, Tile{smem_u32(tK), 64, false}, Tile{smem_u32(tK), 64, false}, 64, 128, 0u);
+        umma_commit_led(leader, &bars->m5);
+        if (tid == 0) {
+          for (int t = 0; t < V / 64; ++t) tma_store_4d(&mo.dv, oVt + t * 8192, t * 64, a.h, a.c * kC, a.b);
+          bulk_commit();
+        }
+      }
+      __syncwarp();
+      // p_i = <(T^T dw)_i, k_i> meanwhile
+      {
+        float v[32], s[4];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          uint32_t kp[8];
+          float x[16];
+          read_column(tK, 2 * half + u, d, 1, kp);
+          tmem_ld16(cBK + lane_base + c0 + 16 * u, x);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 16; ++i) v[16 * u + i] = x[i] * half_of(kp[i >> 1], i & 1);
+        }
+        warp_sum32(v, lane, s);
+        if ((lane & 3) == 0)
+#pragma unroll
+          for (int u = 0; u < 4; ++u) pq[quad * 64 + c0 + 8 * u + (lane >> 2)] = s[u];
+      }
+      mbar_wait_warp(&bars->m5, ph, ctl, 424);
+      tc_fence_after();
+      if (quad < 2) {                               // dkk = beta ratio dM, where T was; row and column sums of e = dkk KK
+        const int r = d;
+        const float Gr = Gs[r], be = betas[r];
+        float rse = 0.f, dbe = 0.f, ev[32], s[4];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          float x[16], y[16];
+          tmem_ld16(cX + lane_base + c0 + 16 * u, x);
+          tmem_ld16(cKK + lane_base + c0 + 16 * u, y);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const int sidx = c0 + 16 * u + j;
+            const float m = (sidx < r) ? x[j] * __expf(Gr - Gs[sidx]) : 0.f;      // dM * ratio, strictly lower
+            dbe += m * y[j];
+            x[j] = m * be;
+            const float e = x[j] * y[j];
+            rse += e;
+            ev[16 * u + j] = e;
+          }
+          write_row16(tKKd, r, 2 * half + u, x);
+        }
+        rsp[half * 64 + r] = rse;
+        dbm[half * 64 + r] = dbe;
+        warp_sum32(ev, lane, s);                    // columns c0 .. c0 + 31 over this warp's 32 rows
+        if ((lane & 3) == 0)
+#pragma unroll
+          for (int u = 0; u < 4; ++u) csp[quad * 64 + c0 + 8 * u + (lane >> 2)] = s[u];
+      }
+      sync_for_issue();
+    }
+    // ---- last group: DS^T q (+ (dkk + dkk^T) k)
+    if (warp == 0) {
+      tc_fence_after();
+      const uint32_t leader = elect_leader();
+      issue_product_led(leader, cAcc, Tile{smem_u32(tQ), 64, true}, Tile{smem_u32(tDS), 64, true}, 64, 64, 0u);
+      if (WY) {
+        issue_product_led(leader, cAcc, Tile{smem_u32(tK), 64, true}, Tile{smem_u32(tKKd), 64, false}, 64, 64, 1u);
+        issue_product_led(leader, cAcc, Tile{smem_u32(tK), 64, true}, Tile{smem_u32(tKKd), 64, true}, 64, 64, 1u);
+      }
+      umma_commit_led(leader, &bars->m6);
+      if (tid == 0 && more) {          // dq and dv have left by now; h / dw, dv2 and X are read
+        bulk_wait_read();
+        load_a(nx);
+        if (SB) load_dh(nx);
+      }
+    }
+    __syncwarp();
+    mbar_wait_warp(&bars->m6, ph, ctl, 425);
+    tc_fence_after();
+    if (tid == 0 && more) load_b(nx);               // [T; A] and k are read
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      float x[16], y[16];
+      if (SB) {
+        tmem_ld16(cDK + lane_base + c0 + 16 * u, y);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) y[i] = dkb_g[static_cast<size_t>(c0 + 16 * u + i) * kK + d];
+      }
+      tmem_ld16(cAcc + lane_base + c0 + 16 * u, x);
+      tmem_ld_wait();
+#pragma unroll
+      for (int i = 0; i < 16; ++i) x[i] = fmaf(decs[c0 + 16 * u + i], y[i], x[i]);
+      if (WY) {
+        tmem_ld16(cBK + lane_base + c0 + 16 * u, y);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) x[i] = fmaf(bgs[c0 + 16 * u + i], y[i], x[i]);
+      }
+#pragma unroll
+      for (int i = 0; i < 16; ++i) stage16(oKt, c0 + 16 * u + i, d, x[i], p.qk16);
+    }
+    fence_proxy_async();
+    tc_fence_before();
+    __syncthreads();
+    if (tid == 0) {
+      for (int t = 0; t < p.Kr / 64; ++t) tma_store_4d(&mo.dk, oKt + t * 8192, t * 64, a.h, a.c * kC, a.b);
+      bulk_commit();
+    }
+    if (tid < 64) {
+      if (SB && tid == 63) dG += dhh + (red[12] + red[13]);
+      if (WY) {
+        const float gam = __expf(Gs[tid]);
+        const float pks = (pq[tid] + pq[64 + tid]) + (pq[128 + tid] + pq[192 + tid]);
+        const float db = dbm[tid] + dbm[64 + tid], rvs = rvp[tid] + rvp[64 + tid];
+        const float rse = rsp[tid] + rsp[64 + tid], cse = csp[tid] + csp[64 + tid];
+        if (tid < rows) {
+          const size_t o = tok0 + static_cast<size_t>(tid) * p.H;
+          if (p.dbeta_w) {
+            p.dbeta_w[o] = rvs;
+            p.dbeta[o] = gam * pks + db;
+          } else {
+            p.dbeta[o] = rvs + gam * pks + db;
+          }
+        }
+        dG = dG + rse - cse + bval * pks * gam;
+      }
+    }
+    const float acc = chunk_rev_cumsum(dG, tid, red);
+    if (tid < rows && p.gate == LETHE_GATE_SCALAR) p.dg[tok0 + static_cast<size_t>(tid) * p.H] = acc;
+  }
+  if (tid == 0) bulk_wait_read();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem, S::kCols);
+}
+
+// ---------------------------------------------------------------------------------------------
+template <int V, ScMode MODE>
+static int launch_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
+                    const CUtensorMap& mdo, const OutMaps& mo, cudaStream_t st) {
+  constexpr int smem = ScSmem<V>::kBytes, per_sm = V == 64 ? 2 : 1;
+  static_assert(per_sm * (smem + 1024) <= 228 * 1024, "CTAs per SM");
+  static SmemAttr attr;
+  if (attr.set(bwd_sc_kernel<V, MODE>, smem)) return kErrLaunch;
+  const int sms = sm_count();
+  if (sms <= 0) return kErrDevice;
+  const int n = p.nbh * p.cn, most = per_sm * sms;
+  if (launch_dependent(bwd_sc_kernel<V, MODE>, dim3(n < most ? n : most), dim3(kBwdThreads), smem, st, p, mq, mk, mv, mdo, mo) !=
+      cudaSuccess) return kErrLaunch;
+  return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
+}
+template <ScMode MODE>
+static int launch_v(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
+                    const CUtensorMap& mdo, const OutMaps& mo, cudaStream_t st) {
+  return p.V == 64 ? launch_t<64, MODE>(p, mq, mk, mv, mdo, mo, st) : launch_t<128, MODE>(p, mq, mk, mv, mdo, mo, st);
+}
+
+// mask bit 4: Stage B, bit 8: WY VJP (delta variants only); both together are one kernel
+int launch_bwd_main(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
+                    const CUtensorMap& mdo, const OutMaps& mo, cudaStream_t st, uint32_t mask) {
+  const bool sb = mask & 4u, wy = (mask & 8u) && p.delta;
+  if (!p.delta) return sb ? launch_v<kScNoDelta>(p, mq, mk, mv, mdo, mo, st) : kOk;
+  if (sb && wy) return launch_v<kScAll>(p, mq, mk, mv, mdo, mo, st);
+  return sb ? launch_v<kScStageB>(p, mq, mk, mv, mdo, mo, st) : launch_v<kScWy>(p, mq, mk, mv, mdo, mo, st);
+}
+
+}  // namespace lg

@@ -24,9 +24,8 @@
 //     DH    128 x V image: adjoint of the state leaving the chunk
 //     DV2   64 x V  image: adjoint of v_new
 //     DW    64 x 128 image: adjoint of w
-//     DKB   64 x 128 fp32: key gradient of Stage B
-//     DGB   64 x 128 fp32 (channel-wise) or 64 fp32 (scalar): gate-gradient of Stage B before the cumsum
-//     (channel-wise gate: DV2, DW, DKB and DGB are only written and read when a call is cut between Stage B and WY)
+//     DKB   64 x 128 fp32, DGB 64 x 128 (channel-wise) or 64 fp32 (scalar): what Stage B leaves for the WY VJP beside DV2
+//           and DW when a call is cut between them (the uncut backward keeps all of it on chip)
 #pragma once
 #include <stddef.h>
 #include <stdint.h>

@@ -143,6 +143,7 @@ def k2_fn(k: Tensor, v: Tensor, beta: Tensor, g2: Tensor, t_mat: Tensor, dw: Ten
     _record_view(buf.scratch, off2["dw"], sz2["dw"], Z, torch.float16).copy_(to_image(dw.half()).reshape(Z, -1))
     _record_view(buf.scratch, off2["dkb"], sz2["dkb"], Z, f32).zero_()
     _record_view(buf.scratch, off2["dgb"], sz2["dgb"], Z, f32).zero_()
+    _record_view(buf.scratch, off2["rb"], sz2["rb"], Z, f32).zero_()       # what Stage B would have left: nothing
     # per-token natural-log decay from the in-chunk cumulative log2 decay
     g_cum = g2.to(f32) * LN2
     g_tok = torch.diff(g_cum, dim=-1, prepend=torch.zeros_like(g_cum[..., :1]))
