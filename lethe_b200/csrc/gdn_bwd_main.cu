@@ -28,7 +28,6 @@
 
 namespace lg {
 
-constexpr int kBwdThreads = 256;
 
 // What runs in a launch; a call cut into its two halves (kernel_mask 4, then 8) gives the bits of the uncut one.
 enum ScMode {
@@ -45,6 +44,8 @@ struct ScBars {
   int abort_flag;
 };
 
+struct ScGates { float G[64], beta[64], de[64], gam[64]; };      // cumulative log decay, beta, de, gamma
+
 template <int V>
 struct ScSmem {
   static constexpr int kVT = V * 128;
@@ -58,41 +59,49 @@ struct ScSmem {
   static constexpr int oH = oA + 8192;              // h; then dw [channel][token]
   static constexpr int oDH = oH + V * 256;          // dh; then dv2 [token][V], and dT / X behind it
   static constexpr int oF = oDH + V * 256;
-  // floats: G, beta, de, beta gamma [64] each; t1q [4][64], pq [4][64]; t2p, t3p, ddep, rsp, dbm, rvp [2][64] each;
-  // csp [2][64]; red [16]
-  static constexpr int kFloats = 4 * 64 + 2 * 256 + 7 * 128 + 16;
+  // warps that reach one lane quadrant: they split the columns of every epilogue
+  static constexpr int kCg = V == 64 ? 2 : 4, kThreads = 128 * kCg;
+  // floats: gates of this chunk and the next; t1q [4][64], pq [4][64]; t2p, t3p, ddep, rsp, dbm, rvp [kCg][64] each;
+  // csp [2][64]; red [32]
+  static constexpr int kFloats = 2 * 256 + 2 * 256 + 6 * 64 * kCg + 128 + 32;
   // An A operand of 64 rows is read as 128: 16 KB from the start of its tile.  The last one is dT / X, kVT into dh.
   static constexpr int kUsed = oF + kFloats * 4 + static_cast<int>(sizeof(ScBars)), kRead = oDH + kVT + 16384;
   static constexpr int kBytes = (kUsed > kRead ? kUsed : kRead) + 1024;
   static constexpr uint32_t kCols = V == 64 ? 256u : 512u;
 };
 
-// 32 values per lane: their sums over the warp's lanes; lane l gets the total of value 8 u + (l >> 2) in out[u]
-__device__ __forceinline__ void warp_sum32(float* v, int lane, float* out) {
+// N values per lane: their sums over the warp's lanes, value i to out[i]
+template <int N>
+__device__ __forceinline__ void warp_sums(float* v, int lane, float* out) {
 #pragma unroll
-  for (int u = 0; u < 4; ++u) out[u] = warp_sum8(v + 8 * u, lane);
+  for (int u = 0; u < N / 8; ++u) {
+    const float s = warp_sum8(v + 8 * u, lane);
+    if ((lane & 3) == 0) out[8 * u + (lane >> 2)] = s;
+  }
 }
 
 template <int V, ScMode MODE>
-__global__ void __launch_bounds__(kBwdThreads, V == 64 ? 2 : 1)
+__global__ void __launch_bounds__(ScSmem<V>::kThreads, V == 64 ? 2 : 1)
 bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,
               const __grid_constant__ CUtensorMap mv, const __grid_constant__ CUtensorMap mdo, const __grid_constant__ OutMaps mo) {
   using S = ScSmem<V>;
   constexpr bool SB = MODE != kScWy, WY = MODE == kScAll || MODE == kScWy, DELTA = MODE != kScNoDelta;
+  constexpr int kCg = S::kCg, kU = 4 / kCg, kThreads = S::kThreads;
   constexpr bool CUT = MODE == kScStageB || MODE == kScWy;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* sm = align1024(smem_raw);
   unsigned char *tQ = sm + S::oQ, *tK = sm + S::oK, *tDO = sm + S::oDO, *tVN = sm + S::oVN, *tV = sm + S::oV, *tT = sm + S::oT;
   unsigned char *tA = sm + S::oA, *tDS = tA, *tH = sm + S::oH, *tDW = tH, *tDH = sm + S::oDH, *tDV = tDH;
   unsigned char *tX = tDH + S::kVT, *tKKd = tT, *oQt = tDO, *oKt = tQ, *oVt = tV;
-  float* Gs = reinterpret_cast<float*>(sm + S::oF);
-  float *betas = Gs + 64, *decs = betas + 64, *bgs = decs + 64, *t1q = bgs + 64, *pq = t1q + 256;
-  float *t2p = pq + 256, *t3p = t2p + 128, *ddep = t3p + 128, *rsp = ddep + 128, *dbm = rsp + 128, *rvp = dbm + 128, *csp = rvp + 128;
+  ScGates* gates = reinterpret_cast<ScGates*>(sm + S::oF);
+  float *t1q = reinterpret_cast<float*>(gates + 2), *pq = t1q + 256;
+  float *t2p = pq + 256, *t3p = t2p + 64 * kCg, *ddep = t3p + 64 * kCg, *rsp = ddep + 64 * kCg, *dbm = rsp + 64 * kCg;
+  float *rvp = dbm + 64 * kCg, *csp = rvp + 64 * kCg;
   float* red = csp + 128;
-  ScBars* bars = reinterpret_cast<ScBars*>(red + 16);
+  ScBars* bars = reinterpret_cast<ScBars*>(red + 32);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, quad = warp & 3, half = warp >> 2, d = quad * 32 + lane;
-  const int c0 = half * 32;                       // this thread's 32 tokens / columns of every 64-column accumulator
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, quad = warp & 3, cg = warp >> 2, d = quad * 32 + lane;
+  const int c0 = cg * 16 * kU;                    // this thread's tokens / columns of every 64-column accumulator
   CtaCtl ctl{p.status, &bars->abort_flag};
   const int nchunks = p.nbh * p.cn;
   struct At { int bh, c, z, b, h; };
@@ -151,17 +160,33 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     tmem_alloc(&bars->tmem_slot, S::kCols);
     tmem_relinquish();
   }
-  float g_next = 0.f, b_next = 1.f;               // gate and beta of token tid of the next chunk
-  auto fetch_gates = [&](const At& a) {
-    g_next = 0.f;
-    b_next = WY ? 0.f : 1.f;
-    if (tid < p.rows_of(a.c)) {
-      const size_t tok = (static_cast<size_t>(a.b) * p.L + a.c * kC + tid) * p.H + a.h;
-      if (p.gate == LETHE_GATE_SCALAR) g_next = p.g[tok];
-      if (WY) b_next = p.beta[tok];
+  // gates of a chunk, by one warp, two neighbouring tokens per lane
+  auto sum_gates = [&](const At& a, ScGates* o) {
+    float g[2] = {0.f, 0.f}, be[2] = {WY ? 0.f : 1.f, WY ? 0.f : 1.f};
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int t = 2 * lane + e;
+      if (t < p.rows_of(a.c)) {
+        const size_t tok = (static_cast<size_t>(a.b) * p.L + a.c * kC + t) * p.H + a.h;
+        if (p.gate == LETHE_GATE_SCALAR) g[e] = p.g[tok];
+        if (WY) be[e] = p.beta[tok];
+      }
     }
+    float sum = g[0] + g[1];
+#pragma unroll
+    for (int w = 1; w < 32; w <<= 1) {
+      const float y = __shfl_up_sync(0xffffffffu, sum, w);
+      if (lane >= w) sum += y;
+    }
+    const float G1 = sum, G0 = sum - g[1], last = __shfl_sync(0xffffffffu, sum, 31);
+    *reinterpret_cast<float2*>(o->G + 2 * lane) = make_float2(G0, G1);
+    *reinterpret_cast<float2*>(o->beta + 2 * lane) = make_float2(be[0], be[1]);
+    *reinterpret_cast<float2*>(o->de + 2 * lane) = make_float2(__expf(last - G0), __expf(last - G1));
+    *reinterpret_cast<float2*>(o->gam + 2 * lane) = make_float2(__expf(G0), __expf(G1));
   };
-  fetch_gates(at(blockIdx.x));
+
+  At a = at(blockIdx.x);
+  if (warp == 2) sum_gates(a, gates);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -174,7 +199,6 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
   griddep_wait();
   griddep_launch();
   if (tid == 0) {
-    const At a = at(blockIdx.x);
     if (SB) {
       load_dh(a);
     } else {
@@ -186,9 +210,8 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
 
   uint32_t ph = 0;
   for (int n = blockIdx.x; n < nchunks; n += gridDim.x, ph ^= 1u) {
-    const At a = at(n);
     const bool more = n + static_cast<int>(gridDim.x) < nchunks;
-    const At nx = at(more ? n + gridDim.x : n);
+    const At nx = more ? at(n + gridDim.x) : a;
     const int rows = p.rows_of(a.c);
     const size_t tok0 = (static_cast<size_t>(a.b) * p.L + a.c * kC) * p.H + a.h;
     unsigned char* dv2_g = p.scratch + p.lay.dv2 + static_cast<size_t>(a.z) * p.lay.sz_dv2;
@@ -198,27 +221,16 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     float* dgb_g = reinterpret_cast<float*>(p.scratch + p.lay.dgb + static_cast<size_t>(a.z) * p.lay.sz_dgb);
     const bool keep = CUT || !p.lean;
 
-    // ---- gates
+    const ScGates& gt = gates[ph];
     if (tid == 0 && n != static_cast<int>(blockIdx.x)) {
       bulk_wait_read();                             // dk of the chunk before has left the q tile
       load_q(a);
     }
-    const float bval = b_next;
-    const float Gt = chunk_cumsum(g_next, tid, red);
-    if (tid < 64) {
-      Gs[tid] = Gt;
-      betas[tid] = bval;
-      bgs[tid] = bval * __expf(Gt);
-    }
-    __syncthreads();
-    const float Glast = Gs[63];
-    if (tid < 64) decs[tid] = __expf(Glast - Gt);
-    if (more) fetch_gates(nx);
 
     // ---- operands to fp16 in place
     mbar_wait_warp(&bars->in0, ph, ctl, 411);
     if (!p.qk16) {
-      for (int idx = tid; idx < 2 * 64 * 16; idx += kBwdThreads) {      // q and k lie behind each other
+      for (int idx = tid; idx < 2 * 64 * 16; idx += kThreads) {      // q and k lie behind each other
         uint4* c = reinterpret_cast<uint4*>(tQ + idx * 16);
         float x[8];
         unpack8_bf16(*c, x);
@@ -226,7 +238,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       }
     }
     if (SB) {
-      for (int idx = tid; idx < (DELTA ? 1 : 2) * 64 * (V / 8); idx += kBwdThreads) {      // do (and, without delta, v behind it)
+      for (int idx = tid; idx < (DELTA ? 1 : 2) * 64 * (V / 8); idx += kThreads) {      // do (and, without delta, v behind it)
         uint4* c = reinterpret_cast<uint4*>(tDO + idx * 16);
         float x[8];
         unpack8_bf16(*c, x);
@@ -234,7 +246,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       }
     }
     if (WY) {
-      for (int idx = tid; idx < 64 * (V / 8); idx += kBwdThreads) {
+      for (int idx = tid; idx < 64 * (V / 8); idx += kThreads) {
         uint4* c = reinterpret_cast<uint4*>(tV + idx * 16);
         float x[8];
         unpack8_bf16(*c, x);
@@ -242,19 +254,18 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       }
     }
     if (!SB) {                                      // the first half of the call left DS and dw
-      for (int idx = tid; idx < 512; idx += kBwdThreads) reinterpret_cast<uint4*>(tDS)[idx] = reinterpret_cast<const uint4*>(rb_g)[idx];
+      for (int idx = tid; idx < 512; idx += kThreads) reinterpret_cast<uint4*>(tDS)[idx] = reinterpret_cast<const uint4*>(rb_g)[idx];
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
+      for (int u = 0; u < kU; ++u) {
         float x[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i)
           x[i] = __half2float(*reinterpret_cast<const __half*>(dw_g + sw128_off(c0 + 16 * u + i, d, 64)));
-        write_column(tDW, 2 * half + u, d, x);
+        write_column(tDW, kU * cg + u, d, x);
       }
     }
     sync_for_issue();
 
-    float dhh = 0.f;
     if (SB) {
       mbar_wait_warp(&bars->in1, ph, ctl, 415);
       // ---- group 1 (two warps issue): k dh (lanes 64-127), (v_new dh^T)^T | A^T do (lanes 64-127), dA
@@ -273,23 +284,27 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       }
       __syncwarp();
       // in their shadow: <dh, h>, element by element on two images of one layout
-      for (int idx = tid; idx < kK * V / 8; idx += kBwdThreads) {
+      float dhh = 0.f;
+      for (int idx = tid; idx < kK * V / 8; idx += kThreads) {
         float x[8], y[8];
         unpack8_f16(*reinterpret_cast<const uint4*>(tDH + idx * 16), x);
         unpack8_f16(*reinterpret_cast<const uint4*>(tH + idx * 16), y);
 #pragma unroll
         for (int i = 0; i < 8; ++i) dhh += x[i] * y[i];
       }
-      dhh = cta_sum256(dhh, tid, red + 2) * __expf(Glast);      // (its barriers: every thread has read dh)
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) dhh += __shfl_xor_sync(0xffffffffu, dhh, o);
+      if (lane == 0) red[16 + warp] = dhh;
+      __syncthreads();                              // every thread has read dh
       mbar_wait_warp(&bars->m1, ph, ctl, 412);
       tc_fence_after();
       if (quad >= 2) {                              // dv2
         const int r = d - 64;
-        const float de = decs[r];
+        const float de = gt.de[r];
         float t3 = 0.f, dde = 0.f;
 #pragma unroll
-        for (int jj = 0; jj < V / 32; ++jj) {
-          const int cb = half * (V / 2) + jj * 16;
+        for (int jj = 0; jj < V / (16 * kCg); ++jj) {
+          const int cb = cg * (V / kCg) + jj * 16;
           float x[16], y[16];
           tmem_ld16(cAo + lane_base + cb, x);
           tmem_ld16(cD + lane_base + cb, y);
@@ -309,14 +324,14 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
             else tile_st_chunk(oVt, r, cb / 8 + q, 64, pack8_bf16(x + 8 * q));
           }
         }
-        t3p[half * 64 + r] = t3 + dde;
-        ddep[half * 64 + r] = dde;
+        t3p[cg * 64 + r] = t3 + dde;
+        ddep[cg * 64 + r] = dde;
       } else {                                      // dA -> DS, where A was
         const int r = d;
-        const float Gr = Gs[r];
+        const float Gr = gt.G[r];
         float t2 = 0.f;
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
+        for (int u = 0; u < kU; ++u) {
           float x[16];
           tmem_ld16(cDA + lane_base + c0 + 16 * u, x);
           tmem_ld_wait();
@@ -330,12 +345,12 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
               const int s = s8 * 8 + i;
               const float da = (s <= r) ? x[8 * q + i] : 0.f;
               t2 += da * av[i];
-              y[i] = (s <= r) ? p.scale * __expf(Gr - Gs[s]) * da : 0.f;
+              y[i] = (s <= r) ? p.scale * __expf(Gr - gt.G[s]) * da : 0.f;
             }
             tile_st_chunk(tDS, r, s8, 64, pack8_f16(y));
           }
         }
-        t2p[half * 64 + r] = t2;
+        t2p[cg * 64 + r] = t2;
       }
       sync_for_issue();
 
@@ -361,19 +376,19 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       __syncwarp();
       mbar_wait_warp(&bars->m2, ph, ctl, 413);
       tc_fence_after();
-      float t1[32];
+      float t1[16 * kU];
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
+      for (int u = 0; u < kU; ++u) {
         uint32_t qp[8];
         float x[16], y[16];
-        read_column(tQ, 2 * half + u, d, 1, qp);
+        read_column(tQ, kU * cg + u, d, 1, qp);
         tmem_ld16(cDQ + lane_base + c0 + 16 * u, x);
         tmem_ld16(cQI + lane_base + c0 + 16 * u, y);
         tmem_ld_wait();
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           const int r = c0 + 16 * u + i;
-          const float dq = p.scale * __expf(Gs[r]) * x[i];
+          const float dq = p.scale * gt.gam[r] * x[i];
           t1[16 * u + i] = dq * half_of(qp[i >> 1], i & 1);
           stage16(oQt, r, d, dq + y[i], p.qk16);
         }
@@ -382,7 +397,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
           tmem_ld_wait();
 #pragma unroll
           for (int i = 0; i < 16; ++i) x[i] = -x[i];
-          if (WY) write_column(tDW, 2 * half + u, d, x);
+          if (WY) write_column(tDW, kU * cg + u, d, x);
           if (keep)
 #pragma unroll
             for (int i = 0; i < 16; ++i) store_f16_sat(dw_g + sw128_off(c0 + 16 * u + i, d, 64), x[i]);
@@ -394,13 +409,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
           for (int i = 0; i < 16; ++i) dkb_g[static_cast<size_t>(c0 + 16 * u + i) * kK + d] = x[i];
         }
       }
-      {
-        float s[4];
-        warp_sum32(t1, lane, s);
-        if ((lane & 3) == 0)
-#pragma unroll
-          for (int u = 0; u < 4; ++u) t1q[quad * 64 + c0 + 8 * u + (lane >> 2)] = s[u];
-      }
+      warp_sums<16 * kU>(t1, lane, t1q + quad * 64 + c0);
       sync_for_issue();
       if (tid == 0) {
         for (int t = 0; t < p.Kr / 64; ++t) tma_store_4d(&mo.dq, oQt + t * 8192, t * 64, a.h, a.c * kC, a.b);
@@ -409,20 +418,32 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     }
     // gate gradient of Stage B (token tid), before the cumulative sum
     float dG = 0.f;
+    auto over_cg = [&](const float* x) {
+      float s = x[tid] + x[64 + tid];
+      if (kCg == 4) s += x[128 + tid] + x[192 + tid];
+      return s;
+    };
+    auto end_term = [&]() {                         // exp(G_last) <dh, h> + sum dde, for the chunk's last row (after a barrier)
+      float s = 0.f;
+#pragma unroll
+      for (int w = 0; w < 4 * kCg; ++w) s += red[16 + w];
+      return s * gt.gam[63] + (red[12] + red[13]);
+    };
     if (SB) {
       if (tid < 64) {
-        float sdde = ddep[tid] + ddep[64 + tid];    // sum over the chunk's rows, fixed tree
+        float sdde = over_cg(ddep);    // sum over the chunk's rows, fixed tree
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) sdde += __shfl_xor_sync(0xffffffffu, sdde, o);
         if (lane == 0) red[12 + warp] = sdde;
-        dG = ((t1q[tid] + t1q[64 + tid]) + (t1q[128 + tid] + t1q[192 + tid])) + (t2p[tid] + t2p[64 + tid]) - (t3p[tid] + t3p[64 + tid]);
+        dG = ((t1q[tid] + t1q[64 + tid]) + (t1q[128 + tid] + t1q[192 + tid])) + over_cg(t2p) - over_cg(t3p);
       }
     } else if (tid < 64) {
       dG = dgb_g[tid];
     }
     if (MODE == kScStageB) {
       __syncthreads();
-      if (tid < 64) dgb_g[tid] = dG + (tid == 63 ? dhh + (red[12] + red[13]) : 0.f);
+      if (tid < 64) dgb_g[tid] = dG + (tid == 63 ? end_term() : 0.f);
+      if (warp == 2 && more) sum_gates(nx, gates + (ph ^ 1u));
       if (tid == 0 && more) {
         bulk_wait_read();
         load_a(nx);
@@ -431,6 +452,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       }
       tc_fence_before();
       __syncthreads();
+      a = nx;
       continue;
     }
     if (WY) {
@@ -449,7 +471,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       tc_fence_after();
       if (quad < 2) {
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
+        for (int u = 0; u < kU; ++u) {
           float x[16], y[16];
           tmem_ld16(cT1 + lane_base + c0 + 16 * u, x);
           tmem_ld16(cT2 + lane_base + c0 + 16 * u, y);
@@ -457,9 +479,9 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             const int s = c0 + 16 * u + j;
-            x[j] = fmaf(bgs[s], y[j], betas[s] * x[j]);
+            x[j] = gt.beta[s] * fmaf(gt.gam[s], y[j], x[j]);
           }
-          write_row16(tX, d, 2 * half + u, x);
+          write_row16(tX, d, kU * cg + u, x);
         }
       }
       sync_for_issue();
@@ -477,11 +499,11 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       tc_fence_after();
       if (quad < 2) {
         const int r = d;
-        const float be = betas[r];
+        const float be = gt.beta[r];
         float rv = 0.f;
 #pragma unroll
-        for (int jj = 0; jj < V / 32; ++jj) {
-          const int cb = half * (V / 2) + jj * 16;
+        for (int jj = 0; jj < V / (16 * kCg); ++jj) {
+          const int cb = cg * (V / kCg) + jj * 16;
           float x[16];
           tmem_ld16(cBV + lane_base + cb, x);
           tmem_ld_wait();
@@ -497,17 +519,17 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
             tile_st_chunk(oVt, r, cb / 8 + q, 64, pack8_bf16(x + 8 * q));
           }
         }
-        rvp[half * 64 + r] = rv;
+        rvp[cg * 64 + r] = rv;
       }
       mbar_wait_warp(&bars->m4, ph, ctl, 423);
       tc_fence_after();
       if (quad < 2) {
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
+        for (int u = 0; u < kU; ++u) {
           float x[16];
           tmem_ld16(cX + lane_base + c0 + 16 * u, x);
           tmem_ld_wait();
-          write_row16(tX, d, 2 * half + u, x);
+          write_row16(tX, d, kU * cg + u, x);
         }
       }
       sync_for_issue();
@@ -526,30 +548,27 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       __syncwarp();
       // p_i = <(T^T dw)_i, k_i> meanwhile
       {
-        float v[32], s[4];
+        float v[16 * kU];
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
+        for (int u = 0; u < kU; ++u) {
           uint32_t kp[8];
           float x[16];
-          read_column(tK, 2 * half + u, d, 1, kp);
+          read_column(tK, kU * cg + u, d, 1, kp);
           tmem_ld16(cBK + lane_base + c0 + 16 * u, x);
           tmem_ld_wait();
 #pragma unroll
           for (int i = 0; i < 16; ++i) v[16 * u + i] = x[i] * half_of(kp[i >> 1], i & 1);
         }
-        warp_sum32(v, lane, s);
-        if ((lane & 3) == 0)
-#pragma unroll
-          for (int u = 0; u < 4; ++u) pq[quad * 64 + c0 + 8 * u + (lane >> 2)] = s[u];
+        warp_sums<16 * kU>(v, lane, pq + quad * 64 + c0);
       }
       mbar_wait_warp(&bars->m5, ph, ctl, 424);
       tc_fence_after();
       if (quad < 2) {                               // dkk = beta ratio dM, where T was; row and column sums of e = dkk KK
         const int r = d;
-        const float Gr = Gs[r], be = betas[r];
-        float rse = 0.f, dbe = 0.f, ev[32], s[4];
+        const float Gr = gt.G[r], be = gt.beta[r];
+        float rse = 0.f, dbe = 0.f, ev[16 * kU];
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
+        for (int u = 0; u < kU; ++u) {
           float x[16], y[16];
           tmem_ld16(cX + lane_base + c0 + 16 * u, x);
           tmem_ld16(cKK + lane_base + c0 + 16 * u, y);
@@ -557,21 +576,18 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             const int sidx = c0 + 16 * u + j;
-            const float m = (sidx < r) ? x[j] * __expf(Gr - Gs[sidx]) : 0.f;      // dM * ratio, strictly lower
+            const float m = (sidx < r) ? x[j] * __expf(Gr - gt.G[sidx]) : 0.f;      // dM * ratio, strictly lower
             dbe += m * y[j];
             x[j] = m * be;
             const float e = x[j] * y[j];
             rse += e;
             ev[16 * u + j] = e;
           }
-          write_row16(tKKd, r, 2 * half + u, x);
+          write_row16(tKKd, r, kU * cg + u, x);
         }
-        rsp[half * 64 + r] = rse;
-        dbm[half * 64 + r] = dbe;
-        warp_sum32(ev, lane, s);                    // columns c0 .. c0 + 31 over this warp's 32 rows
-        if ((lane & 3) == 0)
-#pragma unroll
-          for (int u = 0; u < 4; ++u) csp[quad * 64 + c0 + 8 * u + (lane >> 2)] = s[u];
+        rsp[cg * 64 + r] = rse;
+        dbm[cg * 64 + r] = dbe;
+        warp_sums<16 * kU>(ev, lane, csp + quad * 64 + c0);      // over this warp's 32 rows
       }
       sync_for_issue();
     }
@@ -592,11 +608,12 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       }
     }
     __syncwarp();
+    if (warp == 2 && more) sum_gates(nx, gates + (ph ^ 1u));
     mbar_wait_warp(&bars->m6, ph, ctl, 425);
     tc_fence_after();
     if (tid == 0 && more) load_b(nx);               // [T; A] and k are read
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
+    for (int u = 0; u < kU; ++u) {
       float x[16], y[16];
       if (SB) {
         tmem_ld16(cDK + lane_base + c0 + 16 * u, y);
@@ -607,12 +624,12 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       tmem_ld16(cAcc + lane_base + c0 + 16 * u, x);
       tmem_ld_wait();
 #pragma unroll
-      for (int i = 0; i < 16; ++i) x[i] = fmaf(decs[c0 + 16 * u + i], y[i], x[i]);
+      for (int i = 0; i < 16; ++i) x[i] = fmaf(gt.de[c0 + 16 * u + i], y[i], x[i]);
       if (WY) {
         tmem_ld16(cBK + lane_base + c0 + 16 * u, y);
         tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 16; ++i) x[i] = fmaf(bgs[c0 + 16 * u + i], y[i], x[i]);
+        for (int i = 0; i < 16; ++i) x[i] = fmaf(gt.beta[c0 + 16 * u + i] * gt.gam[c0 + 16 * u + i], y[i], x[i]);
       }
 #pragma unroll
       for (int i = 0; i < 16; ++i) stage16(oKt, c0 + 16 * u + i, d, x[i], p.qk16);
@@ -625,12 +642,11 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       bulk_commit();
     }
     if (tid < 64) {
-      if (SB && tid == 63) dG += dhh + (red[12] + red[13]);
+      if (SB && tid == 63) dG += end_term();
       if (WY) {
-        const float gam = __expf(Gs[tid]);
+        const float gam = gt.gam[tid];
         const float pks = (pq[tid] + pq[64 + tid]) + (pq[128 + tid] + pq[192 + tid]);
-        const float db = dbm[tid] + dbm[64 + tid], rvs = rvp[tid] + rvp[64 + tid];
-        const float rse = rsp[tid] + rsp[64 + tid], cse = csp[tid] + csp[64 + tid];
+        const float db = over_cg(dbm), rvs = over_cg(rvp), rse = over_cg(rsp), cse = csp[tid] + csp[64 + tid];
         if (tid < rows) {
           const size_t o = tok0 + static_cast<size_t>(tid) * p.H;
           if (p.dbeta_w) {
@@ -640,11 +656,12 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
             p.dbeta[o] = rvs + gam * pks + db;
           }
         }
-        dG = dG + rse - cse + bval * pks * gam;
+        dG = dG + rse - cse + gt.beta[tid] * pks * gam;
       }
     }
     const float acc = chunk_rev_cumsum(dG, tid, red);
     if (tid < rows && p.gate == LETHE_GATE_SCALAR) p.dg[tok0 + static_cast<size_t>(tid) * p.H] = acc;
+    a = nx;
   }
   if (tid == 0) bulk_wait_read();
   tc_fence_before();
@@ -663,7 +680,7 @@ static int launch_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& 
   const int sms = sm_count();
   if (sms <= 0) return kErrDevice;
   const int n = p.nbh * p.cn, most = per_sm * sms;
-  if (launch_dependent(bwd_sc_kernel<V, MODE>, dim3(n < most ? n : most), dim3(kBwdThreads), smem, st, p, mq, mk, mv, mdo, mo) !=
+  if (launch_dependent(bwd_sc_kernel<V, MODE>, dim3(n < most ? n : most), dim3(ScSmem<V>::kThreads), smem, st, p, mq, mk, mv, mdo, mo) !=
       cudaSuccess) return kErrLaunch;
   return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
 }
