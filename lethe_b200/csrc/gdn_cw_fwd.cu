@@ -12,11 +12,14 @@
 // Layout and decays are those of the backward (gdn_cw_bwd.cu): thread (block of 16 tokens, channel) builds its 16-token
 // columns of every decayed operand in registers from alpha = exp(g), the only exponential, and stores them as
 // [channel][token] tiles; ratios are products of alphas.  The diagonal blocks need sums over channels instead: there a
-// half-warp takes the rows j and 15 - j of a block, a lane eight channels of them, and goes down the source rows with
-// ratio(i, s) = ratio(i, s + 1) alpha(s + 1); a source row is loaded once for both rows.
+// half-warp takes the rows j and 15 - j of a block, a lane eight channels of them.  The 16 rows fall into groups of four:
+// inside its own group a row goes down the source rows with ratio(i, s) = ratio(i, s + 1) alpha(s + 1); for an earlier
+// group the source rows lie ready in fp32, decayed to the end of their group, and the row carries its decay from there, so
+// that a pair costs two FMAs per channel and no ratio.  All in fp32, and every factor is a decay between two rows that lie
+// between s and i.  (Walking every pair with a running ratio took 6.8 k cycles per chunk, this 4.2 k.)
 //
-// The CTA is persistent: the next chunk's k, q and g are fetched as soon as the diagonal sums have read this chunk's, v
-// and the rest behind the second product.
+// The CTA is persistent: the next chunk's k, q and g are fetched as soon as the diagonal sums have read this chunk's.  v
+// is fetched under the first epilogue: its tile holds the decayed source rows before.
 #include "gdn_cw.cuh"
 #include "host_util.h"
 
@@ -31,8 +34,10 @@ struct PrepCwSmem {
   static constexpr int oK = 0;                           // k as loaded (token-major)
   static constexpr int oQ = oK + 16384;                  // q as loaded
   static constexpr int oG = oQ + 16384;                  // g as loaded (four boxes of 32 channels); then alpha
-  static constexpr int oV = oG + 32768;                  // v; then beta v (w v)                token-major
-  static constexpr int oLA = oV + V * 128;               // (b) k e | q e  [channel][token]; then M (fp32), then P
+  static constexpr int oV = oG + 32768;                  // k to the end of its four rows, fp32, 48 rows of 512 bytes (24 KB);
+                                                         // then v, beta v (w v)                token-major
+  static constexpr int oBg = oV + 24576;                 // decays over four rows, fp32 [16][128]
+  static constexpr int oLA = oBg + 8192;                 // (b) k e | q e  [channel][token]; then M (fp32), then P
   static constexpr int oKR = oLA + 32768;                // k to the start of block 3 | 1, 2; then [w | u]
   static constexpr int oGK = oKR + 32768;                // b gamma k   [channel][token]; with kd behind it, then R
   static constexpr int oKD = oGK + 16384;                // k exp(G_last - G)
@@ -83,7 +88,7 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
   unsigned char* sm = align1024(smem_raw);
   unsigned char *tK = sm + S::oK, *tQ = sm + S::oQ, *BV = sm + S::oV, *LA = sm + S::oLA, *KR = sm + S::oKR, *GK = sm + S::oGK;
   unsigned char *KD = sm + S::oKD, *TA = sm + S::oTA, *WU = KR, *SP = LA, *SR = GK;
-  float* G = reinterpret_cast<float*>(sm + S::oG);
+  float *G = reinterpret_cast<float*>(sm + S::oG), *kfd = reinterpret_cast<float*>(sm + S::oV), *Bg = reinterpret_cast<float*>(sm + S::oBg);
   float* Msm = reinterpret_cast<float*>(LA);
   float* Adg = reinterpret_cast<float*>(sm + S::oF);
   float* Mdg = Adg + 64 * kDg;
@@ -124,7 +129,6 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
     fence_mbar_init();
     fence_proxy_async();
     load_kqg(at(blockIdx.x));
-    load_v(at(blockIdx.x));
   }
   if (warp == 0) {
     tmem_alloc(&cs->tmem_slot, 512);
@@ -176,9 +180,23 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
     {
       float x[16], y[16], f = 1.f, e = 1.f;
 #pragma unroll
-      for (int i = 15; i >= 0; --i) {
-        x[i] = kv(i) * f;                  // k to the end of its block
-        f *= al[i];
+      for (int A = 0; A < 4; ++A) {        // decays over four rows, and k to the end of its four
+        f = 1.f;
+#pragma unroll
+        for (int i = 4 * A + 3; i >= 4 * A; --i) {
+          x[i] = kv(i) * f;
+          if (A < 3) kfd[(blk * 12 + i) * kK + d] = x[i];
+          f *= al[i];
+        }
+        Bg[(blk * 4 + A) * kK + d] = f;
+        y[A] = f;
+      }
+      f = 1.f;
+#pragma unroll
+      for (int A = 3; A >= 0; --A) {       // k to the end of its block
+#pragma unroll
+        for (int i = 4 * A; i < 4 * A + 4; ++i) x[i] *= f;
+        f *= y[A];
       }
 #pragma unroll
       for (int i = 0; i < 16; ++i) y[i] = x[i] * bd.post;
@@ -213,23 +231,6 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
         write_column(GK, blk, d, x);
       }
     }
-    mbar_wait_warp(in1, ph, ctl, 505);
-    for (int idx = tid; idx < 64 * (V / 8); idx += kPrepCwThreads) {
-      const int r = idx / (V / 8), ch = idx % (V / 8);
-      float x[8];
-      unpack8_bf16(tile_ld_chunk(BV, r, ch, 64), x);
-      if (DELTA && FULL) {
-        float wv[8];
-        ld8(p.wch + (tok0 + static_cast<size_t>(r) * p.H) * V + ch * 8, wv);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) x[i] *= wv[i];
-      } else {
-        const float be = DELTA ? betas[r] : 1.f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) x[i] *= be;
-      }
-      tile_st_chunk(BV, r, ch, 64, pack8_f16(x));
-    }
     sync_for_issue();
 
     // ---- off-diagonal blocks of M (rows 0-63) and A (rows 64-127) on the tensor cores
@@ -245,18 +246,35 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
       }
     }
     __syncwarp();
-    // ---- diagonal blocks, exact.  Half-warp (block, j): rows j and 15 - j - 17 pairs for every j; lane: channels
-    // 4 c .. 4 c + 3 of either half.  Source rows from the last to the first; a row's ratio starts at one on the diagonal
-    // and is zero before it, so a step needs no test.  Four source rows' sums are added over the lanes at once.
+    // ---- diagonal blocks, exact.  Half-warp (block, j): rows j and 15 - j - 17 pairs for every j, 5 of them inside the
+    // rows' own groups and 3 x 4 with earlier groups; lane: channels 4 c .. 4 c + 3 of either half.
     {
       const int c = lane & 15, j = warp & 7, db = (warp >> 3) * 2 + (lane >> 4);
       const float* al0 = G + (c >> 3) * 2048 + 4 * (c & 7);        // alpha of row r: + 32 r; the other half: + 4096
       const unsigned char* kt = tK + (c & 1) * 8;
       const unsigned char* qt = tQ + (c & 1) * 8;
       auto at16 = [&](int r) { return r * 128 + (((c >> 1) ^ (r & 7)) << 4); };
-      const int hi = 15 - j;
-      f2 q1[4], k1[4], q2[4], k2[4];
-      auto load_row = [&](int i, f2* qi, f2* ki) {
+      const f2 one = pack2(1.f, 1.f), zero = pack2(0.f, 0.f);
+      // sums of one row against one source row: A, and M where the delta term wants it
+      auto dots = [&](const f2* t, const f2* qi, const f2* ki, float& sa, float& sm_) {
+        f2 aa = zero, mm = zero;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          aa = fma2(qi[e], t[e], aa);
+          if (DELTA) mm = fma2(ki[e], t[e], mm);
+        }
+        sa = sum2(aa);
+        sm_ = DELTA ? sum2(mm) : 0.f;
+      };
+      auto store = [&](int i, int s, bool is_m, float x) {
+        const int r = db * 16 + i;
+        if (is_m) Mdg[r * kDg + s] = s < i ? betas[r] * x : 0.f;
+        else Adg[r * kDg + s] = p.scale * x;
+      };
+      const int i0 = 15 - j, i1 = j;
+      f2 q0[4], k0[4], q1[4], k1[4];               // the two rows; later times their decay
+      float v[16];
+      auto own_group = [&](int i, f2* qi, f2* ki, float* out) {
         const int r = db * 16 + i;
         ld4_pairs<F16>(qt + at16(r), qi);
         ld4_pairs<F16>(qt + 8192 + at16(r), qi + 2);
@@ -270,64 +288,78 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
 #pragma unroll
           for (int e = 0; e < 4; ++e) ki[e] = mul2(ki[e], b[e]);
         }
-      };
-      load_row(hi, q1, k1);
-      load_row(j, q2, k2);
-      const f2 one = pack2(1.f, 1.f), zero = pack2(0.f, 0.f);
-      f2 r1[4] = {zero, zero, zero, zero}, r2[4] = {zero, zero, zero, zero}, an[4] = {zero, zero, zero, zero};
-      // sums of one row against source row s: A, and M where the delta term wants it
-      auto step = [&](const f2* ks, f2* ratio, const f2* qi, const f2* ki, float& sa, float& sm_) {
-        f2 aa = zero, mm = zero;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const f2 t = mul2(ratio[e], ks[e]);
-          aa = fma2(qi[e], t, aa);
-          if (DELTA) mm = fma2(ki[e], t, mm);
-        }
-        sa = sum2(aa);
-        sm_ = DELTA ? sum2(mm) : 0.f;
-      };
-      auto store = [&](int i, int s, bool is_m, float x) {
-        const int r = db * 16 + i;
-        if (is_m) Mdg[r * kDg + s] = s < i ? betas[r] * x : 0.f;
-        else Adg[r * kDg + s] = p.scale * x;
-      };
-#pragma unroll 1
-      for (int sg = hi >> 2; sg >= 0; --sg) {
-        const bool both = sg <= (j >> 2);
-        float v[16];
+        f2 ratio[4] = {one, one, one, one};
 #pragma unroll
         for (int u = 3; u >= 0; --u) {
-          const int s = 4 * sg + u, r = db * 16 + s;
+          out[u] = out[4 + u] = 0.f;
+          if (u > (i & 3)) continue;               // (the same for the whole warp)
+          const int s = (i & ~3) + u, rs = db * 16 + s;
           f2 ks[4], as[4];
-          ld4_pairs<F16>(kt + at16(r), ks);
-          ld4_pairs<F16>(kt + 8192 + at16(r), ks + 2);
-          ld_pairs(al0 + 32 * r, as);
-          ld_pairs(al0 + 32 * r + 4096, as + 2);
+          ld4_pairs<F16>(kt + at16(rs), ks);
+          ld4_pairs<F16>(kt + 8192 + at16(rs), ks + 2);
+          ld_pairs(al0 + 32 * rs, as);
+          ld_pairs(al0 + 32 * rs + 4096, as + 2);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) r1[e] = fma2(r1[e], an[e], s == hi ? one : zero);
-          step(ks, r1, q1, k1, v[u], v[4 + u]);
-          if (both) {
+          for (int e = 0; e < 4; ++e) ks[e] = mul2(ratio[e], ks[e]);
+          dots(ks, qi, ki, out[u], out[4 + u]);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) r2[e] = fma2(r2[e], an[e], s == j ? one : zero);
-            step(ks, r2, q2, k2, v[8 + u], v[12 + u]);
+          for (int e = 0; e < 4; ++e) ratio[e] = mul2(ratio[e], as[e]);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {              // the row's decay from the end of the group before its own
+          qi[e] = mul2(qi[e], ratio[e]);
+          if (DELTA) ki[e] = mul2(ki[e], ratio[e]);
+        }
+      };
+      own_group(i0, q0, k0, v);
+      own_group(i1, q1, k1, v + 8);
+      {
+        const float t = half_warp_sum<16>(v, lane);
+        const int i = (c & 8) ? i1 : i0, s = (i & ~3) + (c & 3);
+        if (s <= i) store(i, s, (c & 4) != 0, t);
+      }
+      // earlier group B of a row; then the row's decay goes on over that group
+      auto earlier = [&](int B, f2* qi, f2* ki, float* out) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          f2 t[4];
+          ld_pairs(kfd + (db * 12 + 4 * B + u) * kK + 4 * c, t);
+          ld_pairs(kfd + (db * 12 + 4 * B + u) * kK + 64 + 4 * c, t + 2);
+          dots(t, qi, ki, out[u], out[4 + u]);
+        }
+        if (B > 0) {
+          f2 g[4];
+          ld_pairs(Bg + (db * 4 + B) * kK + 4 * c, g);
+          ld_pairs(Bg + (db * 4 + B) * kK + 64 + 4 * c, g + 2);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            qi[e] = mul2(qi[e], g[e]);
+            if (DELTA) ki[e] = mul2(ki[e], g[e]);
           }
-#pragma unroll
-          for (int e = 0; e < 4; ++e) an[e] = as[e];
         }
-        if (both) {
-          const float t = half_warp_sum<16>(v, lane);
-          store((c & 8) ? j : hi, 4 * sg + (c & 3), (c & 4) != 0, t);
-        } else {
-          const float t = half_warp_sum<8>(v, lane);
-          store(hi, 4 * sg + ((c >> 1) & 3), (c & 8) != 0, t);
-        }
+      };
+      // row 15 - j has three earlier groups for j < 4 and two otherwise, row j none and one
+      const int B0 = (i0 >> 2) - 1;
+      earlier(B0, q0, k0, v);
+      earlier(B0 - 1, q0, k0, v + 8);
+      {
+        const float t = half_warp_sum<16>(v, lane);
+        store(i0, 4 * (B0 - (c >> 3)) + (c & 3), (c & 4) != 0, t);
+      }
+      if (j < 4) earlier(0, q0, k0, v);
+      else earlier(0, q1, k1, v);
+      {
+        const float t = half_warp_sum<8>(v, lane);
+        store(j < 4 ? i0 : i1, (c >> 1) & 3, (c & 8) != 0, t);
       }
     }
     fence_proxy_async();
     if (tid == 0) bulk_wait_read();        // the query record has left the [T; A] tile, which the epilogue now fills
     __syncthreads();
-    if (tid == 0 && more) load_kqg(nx);    // k, q and alpha of this chunk are read
+    if (tid == 0) {                        // k, q, alpha and the decayed rows of this chunk are read
+      load_v(a);
+      if (more) load_kqg(nx);
+    }
     mbar_wait_warp(m1, ph, ctl, 502);
     tc_fence_after();
     {
@@ -375,6 +407,26 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
     tc_fence_before();
     __syncthreads();
 
+    // ---- beta v (w v) on the warps that have no part in the inverse
+    if (tid >= 256) {
+      mbar_wait_warp(in1, ph, ctl, 505);
+      for (int idx = tid - 256; idx < 64 * (V / 8); idx += kPrepCwThreads - 256) {
+        const int r = idx / (V / 8), ch = idx % (V / 8);
+        float x[8];
+        unpack8_bf16(tile_ld_chunk(BV, r, ch, 64), x);
+        if (DELTA && FULL) {
+          float wv[8];
+          ld8(p.wch + (tok0 + static_cast<size_t>(r) * p.H) * V + ch * 8, wv);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) x[i] *= wv[i];
+        } else {
+          const float be = DELTA ? betas[r] : 1.f;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) x[i] *= be;
+        }
+        tile_st_chunk(BV, r, ch, 64, pack8_f16(x));
+      }
+    }
     // ---- T = (I + M)^-1 (fp32, CUDA cores)
     if (DELTA) {
       unit_lower_inverse64_blocked<kMsC>(Msm, Msm + 64 * kMsC, TA, tid);
@@ -394,7 +446,6 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
       __syncwarp();
       mbar_wait_warp(m2, ph, ctl, 503);
       tc_fence_after();
-      if (tid == 0 && more) load_v(nx);    // v is read
       if (quad < 2) {                      // rows 0-63; the four warps of a quadrant split the columns
         for (int jb = blk; jb < (128 + V) / 32; jb += 4) {
           float x[32];
@@ -458,10 +509,6 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
       if (DELTA) bulk_s2g(p.saved + p.lay.p + static_cast<size_t>(a.z) * p.lay.sz_p, SP, 32768);
       bulk_s2g(p.saved + p.lay.r + static_cast<size_t>(a.z) * p.lay.sz_r, SR, V * 256);
       bulk_commit();
-      if (!DELTA && more) {                // v leaves as u: wait for that before the next v comes
-        bulk_wait_read();
-        load_v(nx);
-      }
     }
   }
   if (tid == 0) bulk_wait_read();
