@@ -18,35 +18,39 @@ namespace lg {
 
 constexpr int kStages = 3;
 constexpr int kMmaWarps = 2;   // warps that issue the step's products (each its own accumulator)
-// Columns of the state per CTA (template parameter kVs of the kernel): 16, or 32 when the 16-column CTAs of a
-// launch could not all be resident at once.  With 32 columns the scan needs half the CTAs and reads P half as
-// often, but a step takes about a fifth longer (measured: 39 against 33 us for 32 chunks), so the narrow form
-// is kept wherever it fits in one wave.
-// warps 0-3 hold the state (thread d = key channel d), warp 4 streams P, warps 5.. issue products
-constexpr int kScanThreads = (5 + kMmaWarps) * 32;
-constexpr int kStepBarrier = 128 + kMmaWarps * 32;
+// Columns of the state per CTA: 16 on four state-holding warps or 64 on sixteen (kGr groups of four warps, 16 columns
+// per thread either way).  The narrow CTA has the shorter step, 0.5 us against 0.7 us; but every CTA of a (batch, head)
+// pair streams all of P, so the wide form moves a quarter of its bytes from L2 - see the rule in launch_scan.
+// warps 0 .. 4 kGr - 1 hold the state (thread d = key channel d), then one warp streams P, two issue products
+constexpr int kVs = 16;
 
 // Step barrier of the delta path: the state-holding warps arrive once the operand is written (and go
 // on to work that does not depend on the product), the issuing warps wait for them.
-__device__ __forceinline__ void step_arrive() { asm volatile("bar.arrive 1, %0;" ::"n"(kStepBarrier) : "memory"); }
-__device__ __forceinline__ void step_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kStepBarrier) : "memory"); }
+template <int kN>
+__device__ __forceinline__ void step_arrive() { asm volatile("bar.arrive 1, %0;" ::"n"(kN) : "memory"); }
+template <int kN>
+__device__ __forceinline__ void step_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kN) : "memory"); }
 
-template <bool ADJOINT, int kVs>
-__global__ void __launch_bounds__(kScanThreads, 2)
+template <int kGr>
+constexpr int kScanThreads = (4 * kGr + 1 + kMmaWarps) * 32;
+
+template <bool ADJOINT, int kGr>
+__global__ void __launch_bounds__(kScanThreads<kGr>, kGr == 1 ? 2 : 1)
 scan_kernel(const Problem p) {
-  constexpr int kTmemCols = kMmaWarps * kVs;        // 32 or 64
-  constexpr int kXB = 128 * kVs * 2;                 // bytes of the state operand tile
+  constexpr int kW = kVs * kGr;                      // columns of this CTA: 16 or 64
+  constexpr int kTmemCols = kMmaWarps * kW;         // 32 or 128
+  constexpr int kXB = 128 * kW * 2;                  // bytes of the state operand tile
+  constexpr int kStateWarps = 4 * kGr, kStepBarrier = (kStateWarps + kMmaWarps) * 32;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* sm = align1024_generic(smem_raw);
   unsigned char* Pst = sm;                          // kStages x 32 KB
-  // x as the B operand, contracted along its rows (row k = key channel k, kVs columns = 32 or 64 bytes):
-  // atoms of 8 rows x 32 (64) bytes with the 32-byte (64-byte) swizzle, so that thread k stores its row as
-  // two (four) 16-byte pieces
-  unsigned char* XB = sm + kStages * 32768;
-  CtaShared* cs = reinterpret_cast<CtaShared*>(XB + kXB);
+  // x as the B operand, contracted along its rows (row k = key channel k, kW columns = 32 or 128 bytes):
+  // atoms of 8 rows with the swizzle of that width, so that thread k stores its row as 16-byte pieces
+  unsigned char* XB0 = sm + kStages * 32768;        // two of them, alternating: the step before's is still being recorded
+  CtaShared* cs = reinterpret_cast<CtaShared*>(XB0 + 2 * kXB);
 
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const int v0 = blockIdx.x * kVs, bh = blockIdx.y + p.bh0;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int v0 = blockIdx.x * kW, bh = blockIdx.y + p.bh0;
   // This launch walks the chunks [c0, c0 + cn) of every pair (all NT of them in an ordinary call), forward in
   // chunk order, the adjoint in reverse.  A launch that does not start at the sequence's first (adjoint: last)
   // chunk takes its fp32 state from the carry buffer the launch before it left, and one that does not end at
@@ -77,16 +81,23 @@ scan_kernel(const Problem p) {
   tc_fence_after();
   const uint32_t tmem = cs->tmem_slot;
   auto chunk_of = [&](int it) { return ADJOINT ? p.c0 + n - 1 - it : p.c0 + it; };
+  // Record of the state a chunk sees: this CTA's columns in the image of [128][V].  At 64 columns the operand tile is that
+  // image and leaves as one bulk copy; stores by the state warps, a row of pieces per thread, held up the step that
+  // followed them (1.08 us a step with them, 0.7 like this).  At 16 columns they cost next to nothing.
+  auto record = [&](int it) {
+    const size_t z = static_cast<size_t>(bh) * NT + chunk_of(it);
+    return (ADJOINT ? p.scratch + p.lay.dh : p.saved + p.lay.hc) + (ADJOINT ? z : z + bh) * p.lay.sz_hc + static_cast<size_t>(v0 >> 6) * 16384;
+  };
   // The kernel before this one wrote R (forward) or Rb (adjoint); P comes from the same kernel in the
   // forward and from the forward call in the adjoint, whose producer may start at once.
-  if (!(ADJOINT && warp == 4)) {
+  if (!(ADJOINT && warp == kStateWarps)) {
     griddep_wait();
     griddep_launch();
   }
 
-  if (warp == 4) {
+  if (warp == kStateWarps) {
     // ---- producer: keeps the ring of P stages full
-    if (tid == 128) {
+    if (lane == 0) {
       const unsigned char* Pg = p.saved + p.lay.p;
       for (int it = 0; it < n; ++it) {
         const int st = it % kStages;
@@ -95,21 +106,22 @@ scan_kernel(const Problem p) {
         bulk_g2s(Pst + st * 32768, Pg + (static_cast<size_t>(bh) * NT + chunk_of(it)) * 32768, 32768u, &bar_full[st]);
       }
     }
-  } else if (warp > 4) {
+  } else if (warp > kStateWarps) {
     // ---- product issue: warp m takes contraction steps [m * 8 / kMmaWarps, ...) into accumulator m.
     // All lanes stay on the path (uniform descriptors); the elected lane issues.
-    const int m = warp - 5;
+    const int m = warp - kStateWarps - 1;
     constexpr int kPer = 8 / kMmaWarps;
     const uint32_t leader = elect_leader();
     // A = the P stage (contracted along its columns forward, along its rows for the adjoint),
     // B = the state operand; one 16-element contraction step moves each by a fixed amount
-    const uint64_t b_desc0 = kVs == 16 ? make_desc_sw32(smem_u32(XB), 16u, 256u) : make_desc_sw64(smem_u32(XB), 16u, 512u);
-    const uint32_t idesc = make_idesc(128, kVs, ADJOINT, true);
-    const uint32_t acc = tmem + static_cast<uint32_t>(m * kVs);
+    const uint64_t b_desc0 = kW == 16 ? make_desc_sw32(smem_u32(XB0), 16u, 256u) : make_desc(smem_u32(XB0), 16384u, 1024u);
+    const uint32_t idesc = make_idesc(128, kW, ADJOINT, true);
+    const uint32_t acc = tmem + static_cast<uint32_t>(m * kW);
     for (int it = 0; it < n; ++it) {
       const int st = it % kStages;
       mbar_wait_warp(&bar_full[st], static_cast<uint32_t>((it / kStages) & 1), ctl, 301);
-      step_sync();
+      if (kW == 64 && m == 0 && lane == 0) bulk_wait_read();     // the other operand tile is recorded: it may be written again
+      step_sync<kStepBarrier>();
       tc_fence_after();
       const uint32_t pa = smem_u32(Pst + st * 32768);
       const uint64_t a_desc0 = ADJOINT ? make_desc(pa, 16384u, 1024u) : make_desc(pa, 16u, 1024u);
@@ -119,21 +131,27 @@ scan_kernel(const Problem p) {
         // byte offsets of contraction step j, in the descriptors' 16-byte units
         const uint32_t aoff = ADJOINT ? static_cast<uint32_t>(j * 2048) >> 4
                                       : static_cast<uint32_t>((j >> 2) * 16384 + (j & 3) * 32) >> 4;
-        const uint32_t boff = static_cast<uint32_t>(j * 32 * kVs) >> 4;     // 16 rows of 2 kVs bytes per step
+        const uint32_t boff = static_cast<uint32_t>(j * 32 * kW + (it & 1) * kXB) >> 4;      // 16 rows of 2 kW bytes per step
         umma_led(leader, acc, a_desc0 + aoff, b_desc0 + boff, idesc, jj > 0 ? 1u : 0u);
       }
       umma_commit_led(leader, bar_mma);
       umma_commit_led(leader, &bar_free[st]);
+      if (kW == 64 && m == 0 && lane == 0) {       // the operand tile is the record's image
+        bulk_s2g(record(it), XB0 + (it & 1) * kXB, kXB);
+        bulk_commit();
+      }
     }
+    if (kW == 64 && m == 0 && lane == 0) bulk_wait_read();
   } else {
-    // ---- the state: thread d holds row d of x (16 columns) in fp32
+    // ---- the state: thread d of a group holds kVs columns of row d of x in fp32
+    const int d = tid & 127, g = tid >> 7, vg = v0 + g * kVs;      // group g: columns [vg, vg + kVs)
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const __half* Rg = reinterpret_cast<const __half*>(ADJOINT ? p.scratch + p.lay.rb : p.saved + p.lay.r);
     const float* ADg = reinterpret_cast<const float*>(p.saved + p.lay.ad);
     unsigned char* Xg = ADJOINT ? p.scratch + p.lay.dh : p.saved + p.lay.hc;
     const size_t szx = p.lay.sz_hc;
     // R / Rb records are [V / 16 column blocks][128 rows][16 columns]: this CTA's block, this thread's row
-    const size_t rofs = (static_cast<size_t>(blockIdx.x) * (kVs / 16) * kK + tid) * 16;
+    const size_t rofs = (static_cast<size_t>(vg / 16) * kK + d) * 16;
 
     float* carry = reinterpret_cast<float*>(ADJOINT ? p.scratch + p.lay.carry_b : p.saved + p.lay.carry_f);
     float x[kVs];
@@ -141,7 +159,7 @@ scan_kernel(const Problem p) {
       const float* x0 = seg_first ? (ADJOINT ? p.dhT : p.h0) : carry;
       const int nrow = seg_first ? p.Kr : kK;      // user states have the real channel count
 #pragma unroll
-      for (int j = 0; j < kVs; ++j) x[j] = x0 && tid < nrow ? x0[(static_cast<size_t>(bh) * nrow + tid) * V + v0 + j] : 0.f;
+      for (int j = 0; j < kVs; ++j) x[j] = x0 && d < nrow ? x0[(static_cast<size_t>(bh) * nrow + d) * V + vg + j] : 0.f;
     }
     constexpr int kPieces = kVs / 8;             // 16-byte pieces of this thread's row
     uint4 rnext[kPieces];
@@ -153,23 +171,22 @@ scan_kernel(const Problem p) {
         rnext[q] = *reinterpret_cast<const uint4*>(r + (q >> 1) * (kK * 16) + (q & 1) * 8);
     };
     load_r(chunk_of(0));
-    float a_next = ADg[(static_cast<size_t>(bh) * NT + chunk_of(0)) * kK + tid];
+    float a_next = ADg[(static_cast<size_t>(bh) * NT + chunk_of(0)) * kK + d];
 
     for (int it = 0; it < n; ++it) {
-      const size_t z = static_cast<size_t>(bh) * NT + chunk_of(it);
+      unsigned char* XB = XB0 + (it & 1) * kXB;
       // critical path: the state as a tensor-core operand
       {
-        // 32-byte swizzle: the two pieces of rows 4-7 of an atom swap; 64-byte swizzle: piece q of row r sits
-        // at q ^ ((r >> 1) & 3)
-        const int sw = kVs == 16 ? (tid >> 2) & 1 : (tid >> 1) & 3;
+        // 32-byte swizzle: the two pieces of rows 4-7 of an atom swap; 128-byte swizzle: piece q of row r sits at q ^ (r & 7)
+        const int sw = kW == 16 ? (d >> 2) & 1 : d & 7;
 #pragma unroll
         for (int q = 0; q < kPieces; ++q)
-          *reinterpret_cast<uint4*>(XB + tid * (2 * kVs) + ((q ^ sw) << 4)) = pack8_f16(x + 8 * q);
+          *reinterpret_cast<uint4*>(XB + d * (2 * kW) + (((g * kPieces + q) ^ sw) << 4)) = pack8_f16(x + 8 * q);
       }
       fence_proxy_async();
       tc_fence_before();
-      step_arrive();
-      // in the shadow of the product: this chunk's input and decay, the next chunk's loads, the record
+      step_arrive<kStepBarrier>();
+      // in the shadow of the product: this chunk's input and decay, the next chunk's loads
       const float a = a_next;
       float rr[kVs];
 #pragma unroll
@@ -179,44 +196,36 @@ scan_kernel(const Problem p) {
       if (it + 1 < n) {
         const int cn = chunk_of(it + 1);
         load_r(cn);
-        a_next = ADg[(static_cast<size_t>(bh) * NT + cn) * kK + tid];
+        a_next = ADg[(static_cast<size_t>(bh) * NT + cn) * kK + d];
       }
-      {
-        unsigned char* rec = Xg + (ADJOINT ? z : z + bh) * szx;
+      if (kW < 64) {
+        unsigned char* rec = record(it);
 #pragma unroll
         for (int q = 0; q < kPieces; ++q)
-          *reinterpret_cast<uint4*>(rec + sw128_chunk(tid, v0 / 8 + q, 128)) = pack8_f16(x + 8 * q);
+          *reinterpret_cast<uint4*>(rec + d * 128 + (((((vg & 63) >> 3) + q) ^ (d & 7)) << 4)) = pack8_f16(x + 8 * q);
       }
       mbar_wait_warp(bar_mma, static_cast<uint32_t>(it & 1), ctl, 302);
       tc_fence_after();
-      static_assert(kMmaWarps == 2, "two accumulators of kVs columns, one per half of the contraction");
-      if (kVs == 16) {
-        float acc[32];
-        tmem_ld32(tmem + lane_base, acc);
-        tmem_ld_wait();
+      static_assert(kMmaWarps == 2, "two accumulators of kW columns, one per half of the contraction");
+      float a0[kVs], a1[kVs];
+      tmem_ld16(tmem + lane_base + g * kVs, a0);
+      tmem_ld16(tmem + lane_base + kW + g * kVs, a1);
+      tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < 16; ++j) x[j] = rr[j] - (acc[j] + acc[16 + j]);
-      } else {
-        float a0[32], a1[32];
-        tmem_ld32(tmem + lane_base, a0);
-        tmem_ld32(tmem + lane_base + 32, a1);
-        tmem_ld_wait();
-#pragma unroll
-        for (int j = 0; j < 32; ++j) x[j] = rr[j] - (a0[j] + a1[j]);
-      }
+      for (int j = 0; j < kVs; ++j) x[j] = rr[j] - (a0[j] + a1[j]);
     }
     if (!ADJOINT && seg_last) {   // the final state as one more record
       unsigned char* rec = Xg + (static_cast<size_t>(bh) * (NT + 1) + NT) * szx;
 #pragma unroll
       for (int q = 0; q < kPieces; ++q)
-        *reinterpret_cast<uint4*>(rec + sw128_chunk(tid, v0 / 8 + q, 128)) = pack8_f16(x + 8 * q);
+        *reinterpret_cast<uint4*>(rec + sw128_chunk(d, vg / 8 + q, 128)) = pack8_f16(x + 8 * q);
     }
     float* xT = seg_last ? (ADJOINT ? p.dh0 : p.hT) : carry;
     const int nrow = seg_last ? p.Kr : kK;
-    if (xT && tid < nrow) {
+    if (xT && d < nrow) {
 #pragma unroll
       for (int j = 0; j < kVs; j += 4)
-        *reinterpret_cast<float4*>(xT + (static_cast<size_t>(bh) * nrow + tid) * V + v0 + j) =
+        *reinterpret_cast<float4*>(xT + (static_cast<size_t>(bh) * nrow + d) * V + vg + j) =
             make_float4(x[j], x[j + 1], x[j + 2], x[j + 3]);
     }
   }
@@ -293,18 +302,18 @@ scan_nodelta_kernel(const Problem p) {
   }
 }
 
-template <int kVs>
+template <int kGr>
 static int launch_scan_t(const Problem& p, bool adjoint, cudaStream_t st) {
-  const int smem = kStages * 32768 + 128 * kVs * 2 + static_cast<int>(sizeof(CtaShared)) + 1024;
-  dim3 grid(p.V / kVs, p.nbh);
+  constexpr int kW = kVs * kGr, smem = kStages * 32768 + 2 * 128 * kW * 2 + static_cast<int>(sizeof(CtaShared)) + 1024;
+  dim3 grid(p.V / kW, p.nbh);
   if (adjoint) {
     static SmemAttr attr;
-    if (attr.set(scan_kernel<true, kVs>, smem)) return kErrLaunch;
-    if (launch_dependent(scan_kernel<true, kVs>, grid, dim3(kScanThreads), smem, st, p) != cudaSuccess) return kErrLaunch;
+    if (attr.set(scan_kernel<true, kGr>, smem)) return kErrLaunch;
+    if (launch_dependent(scan_kernel<true, kGr>, grid, dim3(kScanThreads<kGr>), smem, st, p) != cudaSuccess) return kErrLaunch;
   } else {
     static SmemAttr attr;
-    if (attr.set(scan_kernel<false, kVs>, smem)) return kErrLaunch;
-    if (launch_dependent(scan_kernel<false, kVs>, grid, dim3(kScanThreads), smem, st, p) != cudaSuccess) return kErrLaunch;
+    if (attr.set(scan_kernel<false, kGr>, smem)) return kErrLaunch;
+    if (launch_dependent(scan_kernel<false, kGr>, grid, dim3(kScanThreads<kGr>), smem, st, p) != cudaSuccess) return kErrLaunch;
   }
   return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
 }
@@ -316,12 +325,12 @@ int launch_scan(const Problem& p, bool adjoint, cudaStream_t st) {
                                   : launch_dependent(scan_nodelta_kernel<false>, g, dim3(256), 0, st, p);
     return e == cudaSuccess ? kOk : kErrLaunch;
   }
-  // 32 columns per CTA when the CTAs of the 16-column form could not all be resident at once (two per SM):
-  // the recurrence is serial, so a second wave of CTAs doubles the time of the scan
   const int sms = sm_count();
   if (sms <= 0) return kErrDevice;
-  const bool wide = (p.V / 16) * p.nbh > 2 * sms;
-  return wide ? launch_scan_t<32>(p, adjoint, st) : launch_scan_t<16>(p, adjoint, st);
+  // 16 columns per CTA while every CTA has an SM of its own (B H = 16: 19.7 us for 32 chunks against 25.8); beyond that
+  // the CTAs share the SMs' intake from L2 and P's repeats count (d_v = 128, us for 64 chunks, 16 / 64 columns: B H = 24
+  // 61.8 / 57, 32 63 / 60, 48 119 / 67, 64 122 / 76, 128 252 / 156)
+  return (p.V / 16) * p.nbh <= sms ? launch_scan_t<1>(p, adjoint, st) : launch_scan_t<4>(p, adjoint, st);
 }
 
 }  // namespace lg
