@@ -9,7 +9,7 @@
 namespace lg {
 int launch_prepare(const Problem&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, cudaStream_t);
 int launch_prepare_cw(const Problem&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap& mg, cudaStream_t);
-int launch_output(const Problem&, const CUtensorMap&, cudaStream_t);
+int launch_output(const Problem&, const CUtensorMap& mq, const CUtensorMap& mv, const CUtensorMap& mo, cudaStream_t);
 int launch_scan(const Problem&, bool adjoint, cudaStream_t);
 int launch_bwd_pre(const Problem&, const CUtensorMap& mq, const CUtensorMap& mdo, cudaStream_t);
 int launch_bwd_main(const Problem&, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
@@ -155,7 +155,10 @@ extern "C" int lethe_gdn_forward(const LetheGdnArgs* a, void* stream) {
     return e;
   }
   if ((m & 2u) && (e = launch_scan(p, false, st))) return e;
-  if ((m & 4u) && (e = launch_output(p, mq, st))) return e;
+  if (m & 4u) {
+    CUtensorMap mo;
+    if ((e = token_map(&mo, a->o, p, p.V)) || (e = launch_output(p, mq, mv, mo, st))) return e;
+  }
   return kOk;
 }
 

@@ -64,7 +64,7 @@ struct CwSmem {
   static constexpr int kVT = V * 128;                    // a [64 tokens][V] or [V][64 tokens] tile
   static constexpr int oK = 0;                           // k as loaded; then k f            [channel][token]
   static constexpr int oQ = oK + 16384;                  // q as loaded; then q e
-  static constexpr int oV = oQ + 16384;                  // v (times w)                      token-major
+  static constexpr int oV = oQ + 16384;                  // v (times w; without delta: v_new)  token-major
   static constexpr int oG = oV + kVT;                    // g as loaded (32 KB); then kd | gamma k, then dw | ...
   static constexpr int oDO = oG + 32768;                 // do                               token-major
   static constexpr int oDV = oDO + kVT;                  // dv2  [value channel][token]; then dv on its way out
@@ -94,7 +94,7 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
   extern __shared__ unsigned char smem_raw[];
   unsigned char* sm = align1024(smem_raw);
   unsigned char *tK = sm + S::oK, *tQ = sm + S::oQ, *tV = sm + S::oV, *tKD = sm + S::oG, *tGK = sm + S::oG + 16384;
-  unsigned char *tDW = tKD, *tDO = sm + S::oDO, *tDV = sm + S::oDV, *tTA = sm + S::oTA, *tVN = sm + S::oC, *tC = sm + S::oC;
+  unsigned char *tDW = tKD, *tDO = sm + S::oDO, *tDV = sm + S::oDV, *tTA = sm + S::oTA, *tVN = sm + (DELTA ? S::oC : S::oV), *tC = sm + S::oC;
   unsigned char *oQt = tC, *oKt = sm + S::oDH, *oVt = tDV;
   float* oGt = reinterpret_cast<float*>(sm + S::oH);
   unsigned char *tH = sm + S::oH, *tDH = sm + S::oDH, *tBE = sm + S::oDH, *tDT = sm + S::oDH + 16384;
@@ -126,7 +126,7 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     mbar_expect_tx(&bars->in0, 32768u + 16384u + 16384u);
     for (int q = 0; q < 4; ++q) tma_load_4d(sm + S::oG + q * 8192, &mg, &bars->in0, q * 32, a.h, a.c * kC, a.b);
     mbar_expect_tx(&bars->in1, (SB ? 2u * V * 128 + 2u * V * 256 : 0u) + (DELTA ? 16384u : 8192u) + (WY ? V * 128u : 0u));
-    if (WY) for (int t = 0; t < V / 64; ++t) tma_load_4d(tV + t * 8192, &mv, &bars->in1, t * 64, a.h, a.c * kC, a.b);
+    if (WY || !DELTA) for (int t = 0; t < V / 64; ++t) tma_load_4d(tV + t * 8192, &mv, &bars->in1, t * 64, a.h, a.c * kC, a.b);
     if (DELTA) bulk_g2s(tTA, p.saved + p.lay.ta + static_cast<size_t>(a.z) * 16384, 16384, &bars->in1);
     else bulk_g2s(tTA + 8192, p.saved + p.lay.ta + static_cast<size_t>(a.z) * 16384 + 8192, 8192, &bars->in1);
     if (SB) {
@@ -141,7 +141,7 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
   };
   auto load_part3 = [&](const At& a, bool with_dh) {
     if (!SB) return;
-    bulk_g2s(tVN, p.saved + p.lay.vn + static_cast<size_t>(a.z) * p.lay.sz_vn, V * 128, &bars->in1);
+    if (DELTA) bulk_g2s(tVN, p.saved + p.lay.vn + static_cast<size_t>(a.z) * p.lay.sz_vn, V * 128, &bars->in1);
     bulk_g2s(tH, p.saved + p.lay.hc + static_cast<size_t>(a.z + a.bh) * p.lay.sz_hc, V * 256, &bars->in1);
     if (with_dh) bulk_g2s(tDH, p.scratch + p.lay.dh + static_cast<size_t>(a.z) * p.lay.sz_dh, V * 256, &bars->in1);
   };
@@ -266,6 +266,10 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
         float x[8];
         unpack8_bf16(tile_ld_chunk(tDO, r, ch, 64), x);
         tile_st_chunk(tDO, r, ch, 64, pack8_f16(x));
+        if (!DELTA) {
+          unpack8_bf16(tile_ld_chunk(tVN, r, ch, 64), x);
+          tile_st_chunk(tVN, r, ch, 64, pack8_f16(x));
+        }
       }
     }
     if (WY) {

@@ -475,7 +475,7 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
         if (DELTA) {
           bulk_s2g(p.saved + p.lay.w + static_cast<size_t>(a.z) * p.lay.sz_w, WU, 16384);
           bulk_s2g(p.saved + p.lay.u + static_cast<size_t>(a.z) * p.lay.sz_u, WU + 16384, V * 128);
-        } else {
+        } else if (!p.lean) {            // (u is v)
           bulk_s2g(p.saved + p.lay.u + static_cast<size_t>(a.z) * p.lay.sz_u, BV, V * 128);
         }
         bulk_commit();

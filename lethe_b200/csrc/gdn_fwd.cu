@@ -242,7 +242,7 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq,
       if (tid == 0) bulk_s2g(p.saved + p.lay.w + static_cast<size_t>(z) * p.lay.sz_w, WU, 16384);
       if (tid == 0) bulk_s2g(p.saved + p.lay.u + static_cast<size_t>(z) * p.lay.sz_u, WU + 16384, V * 128);
     } else {
-      if (tid == 0) bulk_s2g(p.saved + p.lay.u + static_cast<size_t>(z) * p.lay.sz_u, BV, V * 128);
+      if (tid == 0 && !p.lean) bulk_s2g(p.saved + p.lay.u + static_cast<size_t>(z) * p.lay.sz_u, BV, V * 128);      // (u is v)
     }
     if (tid == 0) bulk_commit();
   }
@@ -295,154 +295,207 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq,
 //   v_new = u - w h
 //   o = qg h + A v_new                                       (product 2 accumulates onto rows 64-127)
 // Reference: gdn2_chunkwise.py:146-153.
+//
+// Bound by HBM (120 KB per chunk at d_v = 128, channel-wise gate).  Persistent CTAs; results leave as tensor-map / bulk
+// stores from dead tiles (o where w was, v_new where u was).  Channel-wise, d_v = 128: one CTA per SM with two stages, a
+// chunk's tiles arrive while the chunk before is computed (8192 chunks: 193 -> 152 us, 0.99 of the copy bandwidth on its
+// bytes).  Shorter chunks and those whose q and v are converted here are bound by the chain of latencies, which two or
+// three CTAs of one stage each hide better (scalar gate, d_v = 64, 4096 chunks: 59 us against 71 us with two stages;
+// d_v = 128 without the delta term: 78 against 86).
 // ---------------------------------------------------------------------------------------------
+constexpr int kOutThreads = 256;
+
+template <int V, bool CW>
+struct OutSmem {
+  static constexpr int oA = 32768;                   // behind [w; qg]: A (its 128-row view starts 64 rows early)
+  static constexpr int oH = oA + 8192;               // state image
+  static constexpr int oU = oH + V * 256;            // u, then v_new
+  static constexpr int kStage = oU + V * 128, kStages = V == 64 || !CW ? 1 : 2, kCtas = V == 64 ? 3 : CW ? 1 : 2;
+  static constexpr int kBytes = kStages * kStage + 2 * 256 + static_cast<int>(sizeof(CtaShared)) + 1024;
+};
+
 template <int V, bool DELTA, bool CW>
-__global__ void __launch_bounds__(128)
-output_kernel(const Problem p, const __grid_constant__ CUtensorMap mq) {
+__global__ void __launch_bounds__(kOutThreads, OutSmem<V, CW>::kCtas)
+output_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mv,
+              const __grid_constant__ CUtensorMap mo) {
+  using S = OutSmem<V, CW>;
   extern __shared__ unsigned char smem_raw[];
-  unsigned char* sm = CW ? align1024(smem_raw) : align1024_generic(smem_raw);   // measured per variant
-  unsigned char* WQ = sm;                       // 32 KB: rows 0-63 w, rows 64-127 scale gamma q
-  unsigned char* HT = sm + 32768;               // state image 128 x V
-  unsigned char* TAt = HT + V * 256;            // 16 KB [T; A]
-  unsigned char* VN = TAt + 16384;              // v_new 64 x V
-  float* fs = reinterpret_cast<float*>(VN + V * 128);
-  float* Gs = fs;
-  float* tmp = fs + 64;
-  CtaShared* cs = reinterpret_cast<CtaShared*>(fs + 72);
-
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const int bh = p.bh0 + blockIdx.x / p.cn, c = p.c0 + blockIdx.x % p.cn, z = bh * p.NT + c, b = bh / p.H, h = bh % p.H;
+  unsigned char* sm = align1024(smem_raw);
+  float* sgs = reinterpret_cast<float*>(sm + S::kStages * S::kStage);      // [2][64] scale gamma (scalar gate)
+  CtaShared* cs = reinterpret_cast<CtaShared*>(sgs + 128);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, quad = warp & 3, half = warp >> 2;
   CtaCtl ctl{p.status, &cs->abort_flag};
-  const unsigned char* Ug = p.saved + p.lay.u + static_cast<size_t>(z) * p.lay.sz_u;
-  uint64_t* bar_load = &cs->bar[0];
-  uint64_t* bar_mma = &cs->bar[1];
-  uint64_t* bar_ht = &cs->bar[2];       // the state image, loaded once the scan before this kernel is complete
-
-  if (tid == 0) {
-    cs->abort_flag = 0;
-    mbar_init(bar_load, 1);
-    mbar_init(bar_mma, 1);
-    mbar_init(bar_ht, 1);
-    fence_mbar_init();
-    fence_proxy_async();
-    mbar_expect_tx(bar_load, 16384u + (DELTA ? 16384u : V * 128u) + 16384u);
-    for (int a = 0; a < 2; ++a) {
+  uint64_t *full = &cs->bar[0], *m1 = &cs->bar[2], *m2 = &cs->bar[3];
+  const int nchunks = p.nbh * p.cn;
+  struct At { int bh, c, z, b, h; };
+  auto at = [&](int n) {
+    At a;
+    a.bh = p.bh0 + n / p.cn;
+    a.c = p.c0 + n % p.cn;
+    a.z = a.bh * p.NT + a.c;
+    a.b = a.bh / p.H;
+    a.h = a.bh % p.H;
+    return a;
+  };
+  auto load = [&](const At& a, int s) {              // everything but h (tid 0)
+    unsigned char* t = sm + s * S::kStage;
+    mbar_expect_tx(&full[s], 16384u + (DELTA ? 16384u : 0u) + V * 128u + 8192u + V * 256u);
+    for (int i = 0; i < 2; ++i) {
       // the query operand: q from the user tensor (scaled below), or - channel-wise gate - the record of
       // scale * gamma * q that the prepare kernel left (two 64-row atoms of 8 KB)
-      if (CW) bulk_g2s(WQ + a * 16384 + 8192, p.saved + p.lay.qg + static_cast<size_t>(z) * 16384 + a * 8192, 8192, bar_load);
-      else tma_load_4d(WQ + a * 16384 + 8192, &mq, bar_load, a * 64, h, c * kC, b);
-      if (DELTA)
-        bulk_g2s(WQ + a * 16384, p.saved + p.lay.w + static_cast<size_t>(z) * p.lay.sz_w + a * 8192, 8192, bar_load);
+      if (CW) bulk_g2s(t + i * 16384 + 8192, p.saved + p.lay.qg + static_cast<size_t>(a.z) * 16384 + i * 8192, 8192, &full[s]);
+      else tma_load_4d(t + i * 16384 + 8192, &mq, &full[s], i * 64, a.h, a.c * kC, a.b);
+      if (DELTA) bulk_g2s(t + i * 16384, p.saved + p.lay.w + static_cast<size_t>(a.z) * p.lay.sz_w + i * 8192, 8192, &full[s]);
     }
-    if (!DELTA) bulk_g2s(VN, Ug, V * 128, bar_load);   // v_new = u = v
-    bulk_g2s(TAt, p.saved + p.lay.ta + static_cast<size_t>(z) * p.lay.sz_ta, 16384, bar_load);
-    // (the state image, written by the scan just before this kernel, is loaded after griddep_wait)
+    bulk_g2s(t + S::oA, p.saved + p.lay.ta + static_cast<size_t>(a.z) * p.lay.sz_ta + 8192, 8192, &full[s]);
+    if (DELTA) bulk_g2s(t + S::oU, p.saved + p.lay.u + static_cast<size_t>(a.z) * p.lay.sz_u, V * 128, &full[s]);
+    else for (int i = 0; i < V / 64; ++i) tma_load_4d(t + S::oU + i * 8192, &mv, &full[s], i * 64, a.h, a.c * kC, a.b);    // v_new = v
+  };
+  auto load_h = [&](const At& a, int s) {
+    bulk_g2s(sm + s * S::kStage + S::oH, p.saved + p.lay.hc + static_cast<size_t>(a.z + a.bh) * p.lay.sz_hc, V * 256, &full[s]);
+  };
+  // scale * gamma of a chunk by one warp, two neighbouring tokens per lane
+  auto gates = [&](const At& a, float* o) {
+    float g[2] = {0.f, 0.f};
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int t = 2 * lane + e;
+      if (p.gate == LETHE_GATE_SCALAR && t < p.rows_of(a.c)) g[e] = p.g[(static_cast<size_t>(a.b) * p.L + a.c * kC + t) * p.H + a.h];
+    }
+    float sum = g[0] + g[1];
+#pragma unroll
+    for (int w = 1; w < 32; w <<= 1) {
+      const float y = __shfl_up_sync(0xffffffffu, sum, w);
+      if (lane >= w) sum += y;
+    }
+    *reinterpret_cast<float2*>(o + 2 * lane) = make_float2(p.scale * __expf(sum - g[1]), p.scale * __expf(sum));
+  };
+
+  const int n0 = blockIdx.x, n1 = n0 + gridDim.x;
+  if (tid == 0) {
+    cs->abort_flag = 0;
+    for (int i = 0; i < 4; ++i) mbar_init(&cs->bar[i], 1);
+    fence_mbar_init();
+    fence_proxy_async();
+    load(at(n0), 0);                                 // inputs and records older than the scan
+    if (S::kStages == 2 && n1 < nchunks) load(at(n1), 1);
   }
   if (warp == 0) {
     tmem_alloc(&cs->tmem_slot, V);
     tmem_relinquish();
   }
-  float gval = 0.f;
-  if (tid < p.rows_of(c) && p.gate == LETHE_GATE_SCALAR)
-    gval = p.g[(static_cast<size_t>(b) * p.L + c * kC + tid) * p.H + h];
+  if (!CW && warp == 1) gates(at(n0), sgs);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = cs->tmem_slot;
-
-  // u row of this thread (threads 0-63), kept packed
-  uint4 upk[V / 8];
-  if (DELTA && tid < 64) {
-#pragma unroll
-    for (int ch = 0; ch < V / 8; ++ch) upk[ch] = *reinterpret_cast<const uint4*>(Ug + sw128_chunk(tid, ch, 64));
-  }
-  const float G = chunk_cumsum(gval, tid, tmp);
-  if (tid < 64) Gs[tid] = G;
-  __syncthreads();
-
-  // the loads above fetch inputs and records older than the scan; once the scan is complete (at once,
-  // except for the CTAs that started early) its state image is fetched too
+  const uint32_t tmem = cs->tmem_slot, lane_base = static_cast<uint32_t>(quad * 32) << 16;
   griddep_wait();
   griddep_launch();
-  if (tid == 0) {
-    mbar_expect_tx(bar_ht, V * 256u);
-    bulk_g2s(HT, p.saved + p.lay.hc + static_cast<size_t>(z + bh) * p.lay.sz_hc, V * 256, bar_ht);
+  if (tid == 0) {                                    // the state images, written by the scan just before this kernel
+    load_h(at(n0), 0);
+    if (S::kStages == 2 && n1 < nchunks) load_h(at(n1), 1);
   }
-  mbar_wait_warp(bar_load, 0, ctl, 211);
-  for (int idx = tid; idx < 64 * 16; idx += 128) {
-    const int r = idx >> 4, ch = idx & 15;
-    if (!CW) {
-      float x[8];
-      unpack8_in(tile_ld_chunk(WQ, 64 + r, ch, 128), x, p.qk16);
-      const float sg = p.scale * __expf(Gs[r]);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) x[i] *= sg;
-      tile_st_chunk(WQ, 64 + r, ch, 128, pack8_f16(x));
-    }
-    if (!DELTA) tile_st_chunk(WQ, r, ch, 128, make_uint4(0, 0, 0, 0));
-  }
-  fence_proxy_async();
-  __syncthreads();
-  mbar_wait_warp(bar_ht, 0, ctl, 214);
 
-  if (warp == 0) {
-    tc_fence_after();
-    const uint32_t leader = elect_leader();
-    issue_product_led(leader, tmem, Tile{smem_u32(WQ), 128, false}, Tile{smem_u32(HT), 128, true}, V, 128, 0u);
-    umma_commit_led(leader, bar_mma);
-  }
-  __syncwarp();
-  mbar_wait_warp(bar_mma, 0, ctl, 212);
-  tc_fence_after();
-  const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
-  if (DELTA) {
-    if (tid < 64) {
+  int it = 0;
+  for (int n = n0; n < nchunks; n += gridDim.x, ++it) {
+    const At a = at(n);
+    const int s = it % S::kStages, g2 = it & 1;
+    const uint32_t ph = static_cast<uint32_t>(it & 1);
+    unsigned char *WQ = sm + s * S::kStage, *At_ = WQ + S::oA, *HT = WQ + S::oH, *VN = WQ + S::oU;
+    mbar_wait_warp(&full[s], static_cast<uint32_t>((it / S::kStages) & 1), ctl, 211);
+    if (!CW) {
+      const float* sg = sgs + g2 * 64;
+      for (int idx = tid; idx < 64 * 16; idx += kOutThreads) {
+        const int r = idx >> 4, ch = idx & 15;
+        float x[8];
+        unpack8_in(tile_ld_chunk(WQ, 64 + r, ch, 128), x, p.qk16);
 #pragma unroll
-      for (int jb = 0; jb < V / 32; ++jb) {
-        float d[32];
-        tmem_ld32(tmem + lane_base + jb * 32, d);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          float u8[8];
-          unpack8_f16(upk[jb * 4 + i], u8);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) u8[e] -= d[8 * i + e];
-          tile_st_chunk(VN, tid, jb * 4 + i, 64, pack8_f16(u8));
-        }
+        for (int i = 0; i < 8; ++i) x[i] *= sg[r];
+        tile_st_chunk(WQ, 64 + r, ch, 128, pack8_f16(x));
       }
     }
-  }
-  // Every thread must be past its wait on the first product before the second one is committed: a
-  // thread still polling the barrier's first phase when the second phase completes would wait for
-  // a third completion that never comes.
-  tc_fence_before();
-  fence_proxy_async();
-  __syncthreads();
-
-  if (warp == 0) {
+    if (!DELTA) {
+      for (int idx = tid; idx < 64 * (V / 8); idx += kOutThreads) {
+        uint4* c = reinterpret_cast<uint4*>(VN + idx * 16);
+        float x[8];
+        unpack8_bf16(*c, x);
+        *c = pack8_f16(x);
+      }
+    }
+    if (!CW || !DELTA) sync_for_issue();             // (otherwise nothing was written, and the chunk before ended in a barrier)
+    if (warp == 0) {
+      tc_fence_after();
+      const uint32_t leader = elect_leader();
+      issue_product_led(leader, tmem, Tile{smem_u32(WQ), 128, false}, Tile{smem_u32(HT), 128, true}, V, 128, 0u);
+      if (!DELTA) issue_product_led(leader, tmem, Tile{smem_u32(At_) - 8192, 64, false}, Tile{smem_u32(VN), 64, true}, V, 64, 1u);
+      umma_commit_led(leader, DELTA ? m1 : m2);
+      if (S::kStages == 2 && tid == 0 && it > 0 && n + static_cast<int>(gridDim.x) < nchunks) {      // the other stage's results have left it
+        bulk_wait_read();
+        const At nx = at(n + gridDim.x);
+        load(nx, s ^ 1);
+        load_h(nx, s ^ 1);
+      }
+    }
+    __syncwarp();
+    if (!CW && warp == 1 && n + static_cast<int>(gridDim.x) < nchunks) gates(at(n + gridDim.x), sgs + (g2 ^ 1) * 64);
+    if (DELTA) {
+      mbar_wait_warp(m1, ph, ctl, 212);
+      tc_fence_after();
+      if (quad < 2) {                                // v_new, where u was
+        const int r = quad * 32 + lane;
+#pragma unroll
+        for (int jj = 0; jj < V / 64; ++jj) {
+          const int cb = half * (V / 2) + jj * 32;
+          float d[32];
+          tmem_ld32(tmem + lane_base + cb, d);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            float u8[8];
+            unpack8_f16(tile_ld_chunk(VN, r, cb / 8 + i, 64), u8);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) u8[e] -= d[8 * i + e];
+            tile_st_chunk(VN, r, cb / 8 + i, 64, pack8_f16(u8));
+          }
+        }
+      }
+      sync_for_issue();
+      if (warp == 0) {
+        tc_fence_after();
+        const uint32_t leader = elect_leader();
+        issue_product_led(leader, tmem, Tile{smem_u32(At_) - 8192, 64, false}, Tile{smem_u32(VN), 64, true}, V, 64, 1u);
+        umma_commit_led(leader, m2);
+      }
+      __syncwarp();
+    }
+    mbar_wait_warp(m2, ph, ctl, 213);
     tc_fence_after();
-    const uint32_t leader = elect_leader();
-    issue_product_led(leader, tmem, Tile{smem_u32(TAt), 128, false}, Tile{smem_u32(VN), 64, true}, V, 64, 1u);
-    umma_commit_led(leader, bar_mma);
-    if (tid == 0) bulk_s2g(p.saved + p.lay.vn + static_cast<size_t>(z) * p.lay.sz_vn, VN, V * 128);
-    if (tid == 0) bulk_commit();
-  }
-  __syncwarp();
-  mbar_wait_warp(bar_mma, 1, ctl, 213);
-  tc_fence_after();
-  if (tid >= 64) {
-    const int r = tid - 64;
-    const bool live = r < p.rows_of(c);
-    __nv_bfloat16* og = p.o + ((static_cast<size_t>(b) * p.L + c * kC + r) * p.H + h) * V;
+    if (quad >= 2) {                                 // o as a token-major tile where w (without delta: nothing) was
+      const int r = (quad - 2) * 32 + lane;
 #pragma unroll
-    for (int jb = 0; jb < V / 32; ++jb) {
-      float d[32];
-      tmem_ld32(tmem + lane_base + jb * 32, d);
-      tmem_ld_wait();
+      for (int jj = 0; jj < V / 64; ++jj) {
+        const int cb = half * (V / 2) + jj * 32;
+        float d[32];
+        tmem_ld32(tmem + lane_base + cb, d);
+        tmem_ld_wait();
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        if (live) *reinterpret_cast<uint4*>(og + jb * 32 + 8 * i) = pack8_bf16(d + 8 * i);
+        for (int i = 0; i < 4; ++i)
+          *reinterpret_cast<uint4*>(WQ + (cb >> 6) * 16384 + r * 128 + ((((cb >> 3) + i) & 7) ^ (r & 7)) * 16) = pack8_bf16(d + 8 * i);
+      }
+    }
+    fence_proxy_async();
+    tc_fence_before();
+    __syncthreads();
+    if (tid == 0) {
+      for (int i = 0; i < V / 64; ++i) tma_store_4d(&mo, WQ + i * 16384, i * 64, a.h, a.c * kC, a.b);
+      if (DELTA || !p.lean) bulk_s2g(p.saved + p.lay.vn + static_cast<size_t>(a.z) * p.lay.sz_vn, VN, V * 128);
+      bulk_commit();
+      if (S::kStages == 1 && n + static_cast<int>(gridDim.x) < nchunks) {
+        bulk_wait_read();
+        const At nx = at(n + gridDim.x);
+        load(nx, 0);
+        load_h(nx, 0);
+      }
     }
   }
   if (tid == 0) bulk_wait_read();
@@ -465,12 +518,14 @@ static int launch_prepare_t(const Problem& p, const CUtensorMap& mq, const CUten
   return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
 }
 template <int V, bool DELTA, bool CW>
-static int launch_output_t(const Problem& p, const CUtensorMap& mq, cudaStream_t st) {
-  const int smem = 32768 + V * 256 + 16384 + V * 128 + 128 * 4 + 1024;
+static int launch_output_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mv, const CUtensorMap& mo, cudaStream_t st) {
+  constexpr int smem = OutSmem<V, CW>::kBytes;
   auto kern = output_kernel<V, DELTA, CW>;
   static SmemAttr attr;
   if (attr.set(kern, smem)) return kErrLaunch;
-  if (launch_dependent(kern, dim3(p.nbh * p.cn), dim3(128), smem, st, p, mq) != cudaSuccess) return kErrLaunch;
+  const int sms = sm_count(), n = p.nbh * p.cn;
+  if (sms <= 0) return kErrDevice;
+  if (launch_dependent(kern, dim3(n < OutSmem<V, CW>::kCtas * sms ? n : OutSmem<V, CW>::kCtas * sms), dim3(kOutThreads), smem, st, p, mq, mv, mo) != cudaSuccess) return kErrLaunch;
   return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
 }
 
@@ -479,13 +534,13 @@ int launch_prepare(const Problem& p, const CUtensorMap& mq, const CUtensorMap& m
   if (p.V == 64) return p.delta ? launch_prepare_t<64, true>(p, mq, mk, mv, st) : launch_prepare_t<64, false>(p, mq, mk, mv, st);
   return p.delta ? launch_prepare_t<128, true>(p, mq, mk, mv, st) : launch_prepare_t<128, false>(p, mq, mk, mv, st);
 }
-int launch_output(const Problem& p, const CUtensorMap& mq, cudaStream_t st) {
-  if (p.gate == LETHE_GATE_CHANNEL) {
-    if (p.V == 64) return p.delta ? launch_output_t<64, true, true>(p, mq, st) : launch_output_t<64, false, true>(p, mq, st);
-    return p.delta ? launch_output_t<128, true, true>(p, mq, st) : launch_output_t<128, false, true>(p, mq, st);
-  }
-  if (p.V == 64) return p.delta ? launch_output_t<64, true, false>(p, mq, st) : launch_output_t<64, false, false>(p, mq, st);
-  return p.delta ? launch_output_t<128, true, false>(p, mq, st) : launch_output_t<128, false, false>(p, mq, st);
+template <bool CW>
+static int launch_output_cw(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mv, const CUtensorMap& mo, cudaStream_t st) {
+  if (p.V == 64) return p.delta ? launch_output_t<64, true, CW>(p, mq, mv, mo, st) : launch_output_t<64, false, CW>(p, mq, mv, mo, st);
+  return p.delta ? launch_output_t<128, true, CW>(p, mq, mv, mo, st) : launch_output_t<128, false, CW>(p, mq, mv, mo, st);
+}
+int launch_output(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mv, const CUtensorMap& mo, cudaStream_t st) {
+  return p.gate == LETHE_GATE_CHANNEL ? launch_output_cw<true>(p, mq, mv, mo, st) : launch_output_cw<false>(p, mq, mv, mo, st);
 }
 
 }  // namespace lg

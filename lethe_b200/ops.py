@@ -121,23 +121,24 @@ class GdnBuffers:
 
 def forward_into(buf: GdnBuffers, q, k, v, g, beta, h0, scale: float, kernel_mask: int = 0, *,
                  b_gate=None, w_gate=None, bh_range: tuple[int, int] = (0, 0),
-                 c_range: tuple[int, int] = (0, 0)) -> None:
+                 c_range: tuple[int, int] = (0, 0), lean: bool = False) -> None:
     """Enqueue the forward kernels on the current stream; results land in ``buf.o`` / ``buf.hT``.
     ``b_gate [B,L,H,K]`` / ``w_gate [B,L,H,V]`` (fp32) replace ``beta`` for buffers made with ``delta=2``.
     ``bh_range = (begin, count)`` restricts the call to those (batch, head) pairs (count 0: all),
     ``c_range = (begin, count)`` to those 64-token chunks of every sequence (the scans carry their state from
-    one range to the next: forward ranges in ascending order)."""
+    one range to the next: forward ranges in ascending order).  ``lean``: workspace records that no kernel of the
+    forward or the backward reads are not written."""
     a = _Args(dims=buf.dims, scale=scale, q=_ptr(q), k=_ptr(k), v=_ptr(v), g=_ptr(g), beta=_ptr(beta),
               h0=_ptr(h0), o=_ptr(buf.o), hT=_ptr(buf.hT), saved=_ptr(buf.saved),
               saved_bytes=buf.saved.numel(), status=_ptr(buf.status), kernel_mask=kernel_mask,
               b_gate=_ptr(b_gate), w_gate=_ptr(w_gate), bh_begin=bh_range[0], bh_count=bh_range[1],
-              qk_f16=int(q.dtype == torch.float16), c_begin=c_range[0], c_count=c_range[1])
+              qk_f16=int(q.dtype == torch.float16), c_begin=c_range[0], c_count=c_range[1], lean=int(lean))
     _check(native.lib().lethe_gdn_forward(ctypes.byref(a), torch.cuda.current_stream(q.device).cuda_stream))
 
 
 def backward_into(buf: GdnBuffers, q, k, v, g, beta, h0, do, dhT, scale: float, kernel_mask: int = 0, *,
                   b_gate=None, w_gate=None, bh_range: tuple[int, int] = (0, 0),
-                  c_range: tuple[int, int] = (0, 0)) -> None:
+                  c_range: tuple[int, int] = (0, 0), lean: bool = False) -> None:
     """Enqueue the backward kernels; gradients land in ``buf.dq`` ... ``buf.dh0`` (``buf.db`` / ``buf.dw``
     for the per-channel gates of buffers made with ``delta=2``)."""
     a = _Args(dims=buf.dims, scale=scale, q=_ptr(q), k=_ptr(k), v=_ptr(v), g=_ptr(g), beta=_ptr(beta),
@@ -147,7 +148,7 @@ def backward_into(buf: GdnBuffers, q, k, v, g, beta, h0, do, dhT, scale: float, 
               status=_ptr(buf.status), kernel_mask=kernel_mask, dbeta_write=_ptr(buf.dbeta_write),
               b_gate=_ptr(b_gate), w_gate=_ptr(w_gate), db_gate=_ptr(buf.db), dw_gate=_ptr(buf.dw),
               bh_begin=bh_range[0], bh_count=bh_range[1], qk_f16=int(q.dtype == torch.float16),
-              c_begin=c_range[0], c_count=c_range[1])
+              c_begin=c_range[0], c_count=c_range[1], lean=int(lean))
     if buf.dq.dtype != q.dtype:
         raise GdnError("lethe_gdn: dq / dk buffers must have the type of q / k (make GdnBuffers with qk_dtype=)")
     _check(native.lib().lethe_gdn_backward(ctypes.byref(a), torch.cuda.current_stream(q.device).cuda_stream))
@@ -236,7 +237,7 @@ class GdnStepGraph:
         self.bwd_cuts = tuple(sorted(int(c) for c in bwd_cuts))
         if any(c <= 0 or c >= NT for c in self.bwd_cuts) or len(set(self.bwd_cuts)) != len(self.bwd_cuts):
             raise GdnError(f"lethe_gdn: backward cuts {self.bwd_cuts} must be distinct chunk indices inside (0, {NT})")
-        gates = dict(b_gate=b_gate, w_gate=w_gate)
+        gates = dict(b_gate=b_gate, w_gate=w_gate, lean=True)
 
         def chain(rng):
             forward_into(buf, q, k, v, g, beta, h0, scale, bh_range=rng, **gates)
