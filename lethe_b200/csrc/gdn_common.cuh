@@ -216,6 +216,23 @@ __device__ __forceinline__ uint32_t rrec_off(int row, int col8) {
   return static_cast<uint32_t>((col8 >> 1) * 4096 + row * 32 + (col8 & 1) * 16);
 }
 
+// scale * gamma_t of the 64 tokens of chunk c by one warp, two neighbouring tokens per lane (scalar gate or none).
+__device__ __forceinline__ void warp_scaled_gammas(const Problem& p, int b, int c, int h, int lane, float* out) {
+  float g[2] = {0.f, 0.f};
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const int t = 2 * lane + e;
+    if (p.gate == LETHE_GATE_SCALAR && t < p.rows_of(c)) g[e] = p.g[(static_cast<size_t>(b) * p.L + c * kC + t) * p.H + h];
+  }
+  float sum = g[0] + g[1];
+#pragma unroll
+  for (int w = 1; w < 32; w <<= 1) {
+    const float y = __shfl_up_sync(0xffffffffu, sum, w);
+    if (lane >= w) sum += y;
+  }
+  *reinterpret_cast<float2*>(out + 2 * lane) = make_float2(p.scale * __expf(sum - g[1]), p.scale * __expf(sum));
+}
+
 // T = (I + M)^-1 for a strictly lower-triangular 64 x 64 M (fp32, row stride MS floats, zeros on and
 // above the diagonal), by 16 x 16 blocks on threads 0-255 of a CTA (every thread of the CTA must call: four
 // CTA-wide barriers inside; threads beyond 255 only take part in the barriers).  With D_b the inverses of the four diagonal blocks of I + M and N_ba = D_b M_ba

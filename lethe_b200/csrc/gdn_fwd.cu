@@ -354,22 +354,7 @@ output_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
   auto load_h = [&](const At& a, int s) {
     bulk_g2s(sm + s * S::kStage + S::oH, p.saved + p.lay.hc + static_cast<size_t>(a.z + a.bh) * p.lay.sz_hc, V * 256, &full[s]);
   };
-  // scale * gamma of a chunk by one warp, two neighbouring tokens per lane
-  auto gates = [&](const At& a, float* o) {
-    float g[2] = {0.f, 0.f};
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int t = 2 * lane + e;
-      if (p.gate == LETHE_GATE_SCALAR && t < p.rows_of(a.c)) g[e] = p.g[(static_cast<size_t>(a.b) * p.L + a.c * kC + t) * p.H + a.h];
-    }
-    float sum = g[0] + g[1];
-#pragma unroll
-    for (int w = 1; w < 32; w <<= 1) {
-      const float y = __shfl_up_sync(0xffffffffu, sum, w);
-      if (lane >= w) sum += y;
-    }
-    *reinterpret_cast<float2*>(o + 2 * lane) = make_float2(p.scale * __expf(sum - g[1]), p.scale * __expf(sum));
-  };
+  auto gates = [&](const At& a, float* o) { warp_scaled_gammas(p, a.b, a.c, a.h, lane, o); };
 
   const int n0 = blockIdx.x, n1 = n0 + gridDim.x;
   if (tid == 0) {
