@@ -1,6 +1,5 @@
 // Chunk-parallel forward kernels: `prepare` (UT / WY transform and the per-chunk state map) and
-// `output` (v_new and o from the chunk-entry states).  One CTA per chunk: 256 threads in `prepare`,
-// 128 in `output`.
+// `output` (v_new and o from the chunk-entry states).  Persistent CTAs of 256 threads, one chunk at a time.
 //
 // All tensor-core products are tcgen05 with M = 128, fp16 operands in SW128 shared-memory tiles and
 // fp32 accumulators in TMEM; two 64-row operands that share the other operand are stacked into one
@@ -14,272 +13,322 @@ namespace lg {
 constexpr int kMs = 68;  // row stride (floats) of the fp32 copy of M used by the inverse
 
 // ---------------------------------------------------------------------------------------------
-// prepare: per chunk
+// prepare, scalar gate (or none): per chunk
 //   G = cumsum(g), ratio[i,s] = exp(G_i - G_s) (s <= i)
-//   [KK; QK] = [k; q] k^T                                    (product 1)
+//   [KK; QK] = [k; q] k^T                                              (product 1)
 //   M = strict_lower(beta_i ratio KK), A = tril(scale ratio QK), T = (I + M)^-1  (fp32, CUDA cores)
-//   [w | u] = T [beta gamma k | beta v]                      (product 2)
-//   [P | R] = kd^T [w | u],  kd = k exp(G_last - G_i)        (product 3)
+//   w = (T diag(beta gamma)) k,  u = (T diag(beta)) v                  (product 2, both T's stacked)
+//   [P | R] = kd^T [w | u],  kd = k exp(G_last - G_i)                  (product 3)
 // Reference: gdn2_chunkwise.py:130-158 of the reference project; P and R fold its state update
 // h' = exp(G_last) h + kd^T (u - w h) into h' = exp(G_last) h - P h + R.
+//
+// Bound by HBM (128 KB per chunk at d_v = 64) and by the chain of phases of a chunk, about 9 k cycles.  Two persistent CTAs
+// per SM; the next k, q and v are fetched as soon as their tiles are dead (k and q under product 3 and the last epilogue),
+// and the gates are summed a chunk ahead by one warp.  With one CTA per chunk instead, the wait for the first loads and the
+// start of the CTA were 40 % of its time.  The gates are applied to the columns of T, not to k and v: half the elements.
+// PREPARE_NOTE
 // ---------------------------------------------------------------------------------------------
-template <int V, bool DELTA>
-__global__ void __launch_bounds__(256)
-prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq,
-               const __grid_constant__ CUtensorMap mk, const __grid_constant__ CUtensorMap mv) {
-  extern __shared__ unsigned char smem_raw[];
-  unsigned char* sm = DELTA ? align1024(smem_raw) : align1024_generic(smem_raw);   // measured per variant
-  unsigned char* KQ = sm;                      // 32 KB: rows 0-63 k, rows 64-127 q; later M (fp32), then [w | u]
-  unsigned char* BGK = sm + 32768;             // 16 KB: beta gamma k   (64 x 128)
-  unsigned char* BV = BGK + 16384;             // beta v (64 x V), directly behind BGK: one N = 128 + V operand
-  unsigned char* KD = BV + V * 128;            // 16 KB: kd            (64 x 128)
-  unsigned char* TA = KD + 16384;              // 16 KB: [T; A]        (128 x 64)
-  float* fs = reinterpret_cast<float*>(TA + 16384);
-  float* Gs = fs;            // [64] cumulative log decay
-  float* betas = fs + 64;    // [64]
-  float* decs = fs + 128;    // [64] exp(G_last - G_i)
-  float* bgs = fs + 192;     // [64] beta_i exp(G_i)
-  float* tmp = fs + 256;     // [2]
-  CtaShared* cs = reinterpret_cast<CtaShared*>(fs + 264);
-  float* Msm = reinterpret_cast<float*>(KQ);           // [64][kMs]
-  float* Tsm = Msm + 64 * kMs;                          // scratch of the inverse (kInvScratchFloats)
-  unsigned char* WU = KQ;
+constexpr int kPrepThreads = 256;
 
+struct PrepGates {
+  float G[64], beta[64], dec[64], bg[64];     // cumulative log decay; beta; exp(G_last - G); beta exp(G)
+};
+
+// Gates of a chunk by one warp, two neighbouring tokens per lane; also the record of the chunk's whole decay.
+__device__ __forceinline__ void prep_gates(const Problem& p, int b, int c, int h, int z, int lane, PrepGates* o) {
+  float g[2] = {0.f, 0.f}, be[2] = {p.delta ? 0.f : 1.f, p.delta ? 0.f : 1.f};
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const int t = 2 * lane + e;
+    if (t < p.rows_of(c)) {
+      const size_t tok = (static_cast<size_t>(b) * p.L + c * kC + t) * p.H + h;
+      if (p.gate == LETHE_GATE_SCALAR) g[e] = p.g[tok];
+      if (p.delta) be[e] = p.beta[tok];
+    }
+  }
+  float sum = g[0] + g[1];
+#pragma unroll
+  for (int w = 1; w < 32; w <<= 1) {
+    const float y = __shfl_up_sync(0xffffffffu, sum, w);
+    if (lane >= w) sum += y;
+  }
+  const float G1 = sum, G0 = sum - g[1], last = __shfl_sync(0xffffffffu, sum, 31);
+  *reinterpret_cast<float2*>(o->G + 2 * lane) = make_float2(G0, G1);
+  *reinterpret_cast<float2*>(o->beta + 2 * lane) = make_float2(be[0], be[1]);
+  *reinterpret_cast<float2*>(o->dec + 2 * lane) = make_float2(__expf(last - G0), __expf(last - G1));
+  *reinterpret_cast<float2*>(o->bg + 2 * lane) = make_float2(be[0] * __expf(G0), be[1] * __expf(G1));
+  const float a = __expf(last);
+  *reinterpret_cast<float4*>(p.saved + p.lay.ad + static_cast<size_t>(z) * kK * 4 + lane * 16) = make_float4(a, a, a, a);
+}
+
+struct PrepAt {
+  int bh, c, z, b, h;
+  __device__ __forceinline__ PrepAt(const Problem& p, int n)
+      : bh(p.bh0 + n / p.cn), c(p.c0 + n % p.cn), z(bh * p.NT + c), b(bh / p.H), h(bh % p.H) {}
+};
+
+// k and q into the 128-row tile [k; q] (tid 0)
+__device__ __forceinline__ void prep_load_kq(unsigned char* KQ, const CUtensorMap* mk, const CUtensorMap* mq, uint64_t* bar, const PrepAt& a) {
+  mbar_expect_tx(bar, 32768u);
+  for (int t = 0; t < 2; ++t) {
+    tma_load_4d(KQ + t * 16384, mk, bar, t * 64, a.h, a.c * kC, a.b);
+    tma_load_4d(KQ + t * 16384 + 8192, mq, bar, t * 64, a.h, a.c * kC, a.b);
+  }
+}
+template <int V>
+__device__ __forceinline__ void prep_load_v(unsigned char* Vt, const CUtensorMap* mv, uint64_t* bar, const PrepAt& a) {
+  mbar_expect_tx(bar, V * 128u);
+  for (int t = 0; t < V / 64; ++t) tma_load_4d(Vt + t * 8192, mv, bar, t * 64, a.h, a.c * kC, a.b);
+}
+// a tile of bf16 to fp16 in place, whatever its shape
+__device__ __forceinline__ void prep_to_f16(unsigned char* t, int bytes, int tid) {
+  for (int i = tid * 16; i < bytes; i += kPrepThreads * 16) {
+    float x[8];
+    unpack8_bf16(*reinterpret_cast<const uint4*>(t + i), x);
+    *reinterpret_cast<uint4*>(t + i) = pack8_f16(x);
+  }
+}
+// kd = k exp(G_last - G), a 64-row tile
+__device__ __forceinline__ void prep_kd(unsigned char* KD, const unsigned char* KQ, const float* dec, int tid) {
+  for (int idx = tid; idx < 64 * 16; idx += kPrepThreads) {
+    const int r = idx >> 4, ch = idx & 15;
+    float x[8];
+    unpack8_f16(tile_ld_chunk(KQ, r, ch, 128), x);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] *= dec[r];
+    tile_st_chunk(KD, r, ch, 64, pack8_f16(x));
+  }
+}
+// row r of A, 32 columns from 32 half: d holds those of q k^T (live: not all of them right of the diagonal)
+__device__ __forceinline__ void prep_row_a(unsigned char* A, const float* Gs, const float* d, int r, int half, bool live, float scale) {
+  const float Gr = Gs[r];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int s8 = half * 4 + q;
+    float a[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) a[i] = 0.f;
+    if (live) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int s = s8 * 8 + i;
+        a[i] = (s <= r) ? scale * __expf(Gr - Gs[s]) * d[q * 8 + i] : 0.f;
+      }
+    }
+    tile_st_chunk(A, r, s8, 64, pack8_f16(a));
+  }
+}
+
+template <int V>
+struct PrepSmem {
+  static constexpr int oTA = 32768;              // behind [k; q]: [T; A]; then, with kd, P on its way out
+  static constexpr int oKD = oTA + 16384;        // M in fp32 and the scratch of its inverse (30 KB); then kd
+  static constexpr int oW = oKD + 16384;         // [T diag(beta gamma); T diag(beta)]; then w; then R (d_v = 128: with u) on its way out
+  static constexpr int oV = oW + 16384;          // v; then u
+  static constexpr int kUsed = oV + V * 128, kBytes = kUsed + 2 * static_cast<int>(sizeof(PrepGates)) + static_cast<int>(sizeof(CtaShared)) + 1024;
+  static_assert((64 * kMs + kInvScratchFloats) * 4 <= 32768, "scratch of the inverse");
+};
+
+template <int V>
+__global__ void __launch_bounds__(kPrepThreads, 2)
+prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,
+               const __grid_constant__ CUtensorMap mv) {
+  using S = PrepSmem<V>;
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* sm = align1024(smem_raw);
+  unsigned char *KQ = sm, *TA = sm + S::oTA, *KD = sm + S::oKD, *W = sm + S::oW, *Vt = sm + S::oV;
+  float *Msm = reinterpret_cast<float*>(KD), *Tsm = Msm + 64 * kMs;
+  PrepGates* gates = reinterpret_cast<PrepGates*>(sm + S::kUsed);
+  CtaShared* cs = reinterpret_cast<CtaShared*>(gates + 2);
   // Threads 0-127 and 128-255 reach the same TMEM lanes (lane quadrant = warp & 3): the two halves take
   // the same rows and split the columns of every epilogue.
-  const int tid = threadIdx.x, warp = tid >> 5, tq = tid & 127, half = tid >> 7;
-  const int bh = p.bh0 + blockIdx.x / p.cn, c = p.c0 + blockIdx.x % p.cn, z = bh * p.NT + c, b = bh / p.H, h = bh % p.H;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, quad = warp & 3, half = warp >> 2, tq = tid & 127;
   CtaCtl ctl{p.status, &cs->abort_flag};
-  uint64_t* bar_load = &cs->bar[0];
-  uint64_t* bar_mma = &cs->bar[1];
+  uint64_t *full_kq = &cs->bar[0], *full_v = &cs->bar[1], *mma = &cs->bar[2];
+  const int nchunks = p.nbh * p.cn;
 
   if (tid == 0) {
     cs->abort_flag = 0;
-    mbar_init(bar_load, 1);
-    mbar_init(bar_mma, 1);
+    for (int i = 0; i < 3; ++i) mbar_init(&cs->bar[i], 1);
     fence_mbar_init();
     fence_proxy_async();
-    mbar_expect_tx(bar_load, 32768u + V * 128u);
-    for (int a = 0; a < 2; ++a) {
-      tma_load_4d(KQ + a * 16384, &mk, bar_load, a * 64, h, c * kC, b);
-      tma_load_4d(KQ + a * 16384 + 8192, &mq, bar_load, a * 64, h, c * kC, b);
-    }
-    for (int a = 0; a < V / 64; ++a) tma_load_4d(BV + a * 8192, &mv, bar_load, a * 64, h, c * kC, b);
   }
   if (warp == 0) {
     tmem_alloc(&cs->tmem_slot, 256);
     tmem_relinquish();
   }
-  float gval = 0.f, bval = 1.f;
-  if (tid < p.rows_of(c)) {
-    const size_t tok = (static_cast<size_t>(b) * p.L + c * kC + tid) * p.H + h;
-    if (p.gate == LETHE_GATE_SCALAR) gval = p.g[tok];
-    if (DELTA) bval = p.beta[tok];
-  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = cs->tmem_slot;
-
-
-  // ---- gate: cumulative log decay of the chunk
-  const float G = chunk_cumsum(gval, tid, tmp);
-  if (tid < 64) {
-    Gs[tid] = G;
-    betas[tid] = bval;
-  }
-  __syncthreads();
-  const float Glast = Gs[63];
-  if (tid < 64) {
-    decs[tid] = __expf(Glast - G);
-    bgs[tid] = bval * __expf(G);
-  }
-  if (tid < kK) reinterpret_cast<float*>(p.saved + p.lay.ad)[static_cast<size_t>(z) * kK + tid] = __expf(Glast);
-  __syncthreads();
-
-  // ---- operands: k, q -> fp16 in place; kd, beta gamma k, beta v
-  mbar_wait_warp(bar_load, 0, ctl, 201);
-  for (int idx = tid; idx < 64 * 16; idx += 256) {
-    const int r = idx >> 4, ch = idx & 15;
-    float x[8], y[8];
-    unpack8_in(tile_ld_chunk(KQ, r, ch, 128), x, p.qk16);
-    tile_st_chunk(KQ, r, ch, 128, pack8_f16(x));
-    const float de = decs[r];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) y[i] = x[i] * de;
-    tile_st_chunk(KD, r, ch, 64, pack8_f16(y));
-    if (DELTA) {
-      const float bg = bgs[r];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) y[i] = x[i] * bg;
-      tile_st_chunk(BGK, r, ch, 64, pack8_f16(y));
-    }
-    unpack8_in(tile_ld_chunk(KQ, 64 + r, ch, 128), x, p.qk16);
-    tile_st_chunk(KQ, 64 + r, ch, 128, pack8_f16(x));
-  }
-  for (int idx = tid; idx < 64 * (V / 8); idx += 256) {
-    const int r = idx / (V / 8), ch = idx % (V / 8);
-    float x[8];
-    unpack8_bf16(tile_ld_chunk(BV, r, ch, 64), x);
-    const float be = DELTA ? betas[r] : 1.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) x[i] *= be;
-    tile_st_chunk(BV, r, ch, 64, pack8_f16(x));
-  }
-  fence_proxy_async();
-  __syncthreads();
-
-  // ---- product 1: [KK; QK] = [k; q] k^T
-  if (warp == 0) {
-    tc_fence_after();
-    const uint32_t leader = elect_leader();
-    issue_product_led(leader, tmem, Tile{smem_u32(KQ), 128, false}, Tile{smem_u32(KQ), 128, false}, 64, 128, 0u);
-    umma_commit_led(leader, bar_mma);
-  }
-  __syncwarp();
-  mbar_wait_warp(bar_mma, 0, ctl, 202);
-  tc_fence_after();
-  const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
+  const uint32_t tmem = cs->tmem_slot, lane_base = static_cast<uint32_t>(quad * 32) << 16;
+  griddep_wait();
+  griddep_launch();
   {
-    // each half takes 32 of the 64 columns; rows 0-31 (lane quadrant 0 of either operand half) have
-    // nothing right of column 31, so the triangle is cut per warp
-    const bool live = (half == 0) || ((warp & 1) != 0);
-    float d[32];
-    if (live) {
-      tmem_ld32(tmem + lane_base + half * 32, d);
-      tmem_ld_wait();
+    const PrepAt a(p, blockIdx.x);
+    if (tid == 0) {
+      prep_load_kq(KQ, &mk, &mq, full_kq, a);
+      prep_load_v<V>(Vt, &mv, full_v, a);
     }
-    if (tq < 64) {
-      if (DELTA) {
-        const int r = tq;
-        const float Gr = Gs[r], be = betas[r];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const int s = half * 32 + j;
-          float m = 0.f;
-          if (live) m = (s < r) ? be * __expf(Gr - Gs[s]) * d[j] : 0.f;
-          Msm[r * kMs + s] = m;
-        }
-      }
-    } else {
-      const int r = tq - 64;
-      const float Gr = Gs[r];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int s8 = half * 4 + q;
-        float a[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) a[i] = 0.f;
-        if (live) {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int s = s8 * 8 + i;
-            a[i] = (s <= r) ? p.scale * __expf(Gr - Gs[s]) * d[q * 8 + i] : 0.f;
-          }
-        }
-        tile_st_chunk(TA, 64 + r, s8, 128, pack8_f16(a));
-      }
-    }
+    if (warp == 1) prep_gates(p, a.b, a.c, a.h, a.z, lane, gates);
   }
-  tc_fence_before();
   __syncthreads();
 
-  // ---- T = (I + M)^-1 (fp32, CUDA cores)
-  if (DELTA) {
-    unit_lower_inverse64_blocked<kMs>(Msm, Tsm, TA, tid);
-  } else if (tid < 64) {
-    {
-#pragma unroll
-      for (int i = 0; i < 64; ++i)
-        *reinterpret_cast<__half*>(TA + sw128_off(i, tid, 128)) = __float2half_rn((i == tid) ? 1.f : 0.f);
-    }
-  }
-  fence_proxy_async();
-  __syncthreads();
+  uint32_t ph = 0, pm = 0;
+  for (int n = blockIdx.x; n < nchunks; n += gridDim.x, ph ^= 1u) {
+    const PrepAt a(p, n);
+    const bool more = n + static_cast<int>(gridDim.x) < nchunks;
+    const PrepAt nx(p, more ? n + gridDim.x : n);
+    const PrepGates& gt = gates[ph];
 
-  uint32_t ph = 1;
-  if (DELTA) {
-    // ---- product 2: [w | u] = T [beta gamma k | beta v]
+    mbar_wait_warp(full_kq, ph, ctl, 201);
+    if (!p.qk16) prep_to_f16(KQ, 32768, tid);
+    if (tid == 0 && n != static_cast<int>(blockIdx.x)) {
+      bulk_wait_read();                              // P and R of the chunk before have left their tiles
+      if (V == 128) prep_load_v<V>(Vt, &mv, full_v, a);
+    }
+    sync_for_issue();
+
+    // ---- product 1: [KK; QK] = [k; q] k^T
     if (warp == 0) {
       tc_fence_after();
       const uint32_t leader = elect_leader();
-      issue_product_led(leader, tmem, Tile{smem_u32(TA), 128, false}, Tile{smem_u32(BGK), 64, true}, 128 + V, 64, 0u);
-      umma_commit_led(leader, bar_mma);
-      if (tid == 0) bulk_s2g(p.saved + p.lay.ta + static_cast<size_t>(z) * p.lay.sz_ta, TA, 16384);
-      if (tid == 0) bulk_commit();
+      issue_product_led(leader, tmem, Tile{smem_u32(KQ), 128, false}, Tile{smem_u32(KQ), 128, false}, 64, 128, 0u);
+      umma_commit_led(leader, mma);
     }
-    __syncwarp();
-    mbar_wait_warp(bar_mma, ph, ctl, 203);
-    ph ^= 1;
-    tc_fence_after();
-    if (tq < 64) {
-      constexpr int kHalf2 = (128 + V) / 64;
-#pragma unroll
-      for (int jb = half * kHalf2; jb < (half + 1) * kHalf2; ++jb) {
-        float d[32];
-        tmem_ld32(tmem + lane_base + jb * 32, d);
+    wait_products(mma, pm, ctl, 202);
+    {
+      // each half takes 32 of the 64 columns; rows 0-31 (lane quadrant 0 of either operand half) have
+      // nothing right of column 31, so the triangle is cut per warp
+      const bool live = (half == 0) || ((warp & 1) != 0);
+      float d[32];
+      if (live) {
+        tmem_ld32(tmem + lane_base + half * 32, d);
         tmem_ld_wait();
+      }
+      if (tq < 64) {
+        const int r = tq;
+        const float Gr = gt.G[r], be = gt.beta[r];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) tile_st_chunk(WU, tq, jb * 4 + i, 64, pack8_f16(d + 8 * i));
+        for (int j4 = 0; j4 < 8; ++j4) {
+          float m[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int s = half * 32 + 4 * j4 + e;
+            m[e] = 0.f;
+            if (live) m[e] = (s < r) ? be * __expf(Gr - gt.G[s]) * d[4 * j4 + e] : 0.f;
+          }
+          *reinterpret_cast<float4*>(Msm + r * kMs + half * 32 + 4 * j4) = make_float4(m[0], m[1], m[2], m[3]);
+        }
+      } else {
+        prep_row_a(TA + 8192, gt.G, d, tq - 64, half, live, p.scale);
       }
     }
     tc_fence_before();
-    fence_proxy_async();
     __syncthreads();
-  } else if (tid == 0) {
-    bulk_s2g(p.saved + p.lay.ta + static_cast<size_t>(z) * p.lay.sz_ta, TA, 16384);
-    bulk_commit();
-  }
 
-  // ---- product 3: [P | R] = kd^T [w | u]   (no delta: R = kd^T v)
-  constexpr int N3 = DELTA ? 128 + V : V;
-  if (warp == 0) {
-    tc_fence_after();
-    const uint32_t leader = elect_leader();
-    issue_product_led(leader, tmem, Tile{smem_u32(KD), 64, true}, Tile{smem_u32(DELTA ? WU : BV), 64, true}, N3, 64, 0u);
-    umma_commit_led(leader, bar_mma);
-    if (DELTA) {
-      if (tid == 0) bulk_s2g(p.saved + p.lay.w + static_cast<size_t>(z) * p.lay.sz_w, WU, 16384);
-      if (tid == 0) bulk_s2g(p.saved + p.lay.u + static_cast<size_t>(z) * p.lay.sz_u, WU + 16384, V * 128);
-    } else {
-      if (tid == 0 && !p.lean) bulk_s2g(p.saved + p.lay.u + static_cast<size_t>(z) * p.lay.sz_u, BV, V * 128);      // (u is v)
+    // ---- T = (I + M)^-1 (fp32, CUDA cores)
+    unit_lower_inverse64_blocked<kMs>(Msm, Tsm, TA, tid);
+    mbar_wait_warp(full_v, ph, ctl, 203);
+    prep_to_f16(Vt, V * 128, tid);
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int idx = tid + u * kPrepThreads, r = idx >> 3, ch = idx & 7;
+      float t[8], x[8];
+      unpack8_f16(tile_ld_chunk(TA, r, ch, 128), t);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[i] = t[i] * gt.bg[ch * 8 + i];
+      tile_st_chunk(W, r, ch, 128, pack8_f16(x));
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[i] = t[i] * gt.beta[ch * 8 + i];
+      tile_st_chunk(W, 64 + r, ch, 128, pack8_f16(x));
     }
-    if (tid == 0) bulk_commit();
-  }
-  __syncwarp();
-  mbar_wait_warp(bar_mma, ph, ctl, 204);
-  tc_fence_after();
-  // P and R are staged as their record images in tiles nothing reads any more and leave by bulk
-  // stores: P behind BGK (beta gamma k, beta v, kd are dead), R where k and q were once the stores
-  // of [w | u] have finished reading it.
-  if (tid == 0) bulk_wait_read();
-  __syncthreads();
-  {
-    unsigned char* SP = BGK;
-    unsigned char* SR = KQ;
-    constexpr int kHalf3 = N3 / 64;
+    sync_for_issue();
+
+    // ---- product 2: w in rows 0-63, u in rows 64-127
+    if (warp == 0) {
+      tc_fence_after();
+      const uint32_t leader = elect_leader();
+      issue_product_led(leader, tmem, Tile{smem_u32(W), 128, false}, Tile{smem_u32(KQ), 128, true}, 128, 64, 0u);
+      issue_product_led(leader, tmem + 128, Tile{smem_u32(W), 128, false}, Tile{smem_u32(Vt), 64, true}, V, 64, 0u);
+      umma_commit_led(leader, mma);
+      if (tid == 0) {
+        bulk_s2g(p.saved + p.lay.ta + static_cast<size_t>(a.z) * p.lay.sz_ta, TA, 16384);
+        bulk_commit();
+      }
+      __syncwarp();
+    }
+    prep_kd(KD, KQ, gt.dec, tid);                    // in its shadow
+    wait_products(mma, pm, ctl, 204);
+    if (quad < 2) {
+#pragma unroll
+      for (int jj = 0; jj < 2; ++jj) {
+        const int cb = half * 64 + jj * 32;
+        float d[32];
+        tmem_ld32(tmem + lane_base + cb, d);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) tile_st_chunk(W, tq, cb / 8 + i, 64, pack8_f16(d + 8 * i));
+      }
+    } else {
+#pragma unroll
+      for (int jj = 0; jj < V / 64; ++jj) {
+        const int cb = half * (V / 2) + jj * 32;
+        float d[32];
+        tmem_ld32(tmem + 128 + lane_base + cb, d);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) tile_st_chunk(Vt, tq - 64, cb / 8 + i, 64, pack8_f16(d + 8 * i));
+      }
+    }
+    sync_for_issue();
+
+    // ---- product 3: [P | R] = kd^T [w | u]
+    if (warp == 0) {
+      tc_fence_after();
+      const uint32_t leader = elect_leader();
+      issue_product_led(leader, tmem, Tile{smem_u32(KD), 64, true}, Tile{smem_u32(W), 64, true}, 128, 64, 0u);
+      issue_product_led(leader, tmem + 128, Tile{smem_u32(KD), 64, true}, Tile{smem_u32(Vt), 64, true}, V, 64, 0u);
+      umma_commit_led(leader, mma);
+      if (tid == 0) {
+        if (more) prep_load_kq(KQ, &mk, &mq, full_kq, nx);        // nothing reads k and q any more
+        bulk_s2g(p.saved + p.lay.w + static_cast<size_t>(a.z) * p.lay.sz_w, W, 16384);
+        bulk_s2g(p.saved + p.lay.u + static_cast<size_t>(a.z) * p.lay.sz_u, Vt, V * 128);
+        bulk_commit();
+      }
+    }
+    __syncwarp();
+    if (warp == 1 && more) prep_gates(p, nx.b, nx.c, nx.h, nx.z, lane, gates + (ph ^ 1u));
+    wait_products(mma, pm, ctl, 205);
+    // P and R leave from tiles that nothing reads any more, once the stores of w and u have read them
+    if (tid == 0) {
+      bulk_wait_read();
+      if (V == 64 && more) prep_load_v<V>(Vt, &mv, full_v, nx);
+    }
+    __syncthreads();
+    {
+      unsigned char *SP = TA, *SR = W;
+      constexpr int kHalf = (128 + V) / 64;
 #pragma unroll 1
-    for (int jb = half * kHalf3; jb < (half + 1) * kHalf3; ++jb) {
-      float d[32];
-      tmem_ld32(tmem + lane_base + jb * 32, d);
-      tmem_ld_wait();
-      if (DELTA && jb < 4) {
+      for (int jb = half * kHalf; jb < (half + 1) * kHalf; ++jb) {
+        float d[32];
+        tmem_ld32(tmem + lane_base + jb * 32, d);
+        tmem_ld_wait();
+        if (jb < 4) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) tile_st_chunk(SP, tq, jb * 4 + i, 128, pack8_f16(d + 8 * i));
-      } else {
-        const int c8 = (jb - (DELTA ? 4 : 0)) * 4;
+          for (int i = 0; i < 4; ++i) tile_st_chunk(SP, tq, jb * 4 + i, 128, pack8_f16(d + 8 * i));
+        } else {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          if (DELTA) *reinterpret_cast<uint4*>(SR + rrec_off(tq, c8 + i)) = pack8_f16(d + 8 * i);
-          else tile_st_chunk(SR, tq, c8 + i, 128, pack8_f16(d + 8 * i));     // no delta term: plain tile image
+          for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(SR + rrec_off(tq, (jb - 4) * 4 + i)) = pack8_f16(d + 8 * i);
         }
       }
     }
     fence_proxy_async();
+    tc_fence_before();
     __syncthreads();
     if (tid == 0) {
-      if (DELTA) bulk_s2g(p.saved + p.lay.p + static_cast<size_t>(z) * p.lay.sz_p, SP, 32768);
-      bulk_s2g(p.saved + p.lay.r + static_cast<size_t>(z) * p.lay.sz_r, SR, V * 256);
+      bulk_s2g(p.saved + p.lay.p + static_cast<size_t>(a.z) * p.lay.sz_p, TA, 32768);
+      bulk_s2g(p.saved + p.lay.r + static_cast<size_t>(a.z) * p.lay.sz_r, W, V * 256);
       bulk_commit();
     }
   }
@@ -287,6 +336,133 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq,
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, 256);
+}
+
+// Without the delta term u = v, and only A and R = kd^T v are left: two independent products, one wait.
+template <int V>
+struct PrepNdSmem {
+  static constexpr int oA = 32768, oKD = oA + 8192, oV = oKD + 16384;    // R leaves from where kd (d_v = 128: and v) was
+  static constexpr int kUsed = oV + V * 128, kBytes = kUsed + 2 * static_cast<int>(sizeof(PrepGates)) + static_cast<int>(sizeof(CtaShared)) + 1024;
+  static constexpr int kCols = V == 64 ? 128 : 256, kCtas = V == 64 ? 3 : 2;      // q k^T and R side by side in tensor memory
+};
+
+template <int V>
+__global__ void __launch_bounds__(kPrepThreads, PrepNdSmem<V>::kCtas)
+prepare_nodelta_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,
+                       const __grid_constant__ CUtensorMap mv) {
+  using S = PrepNdSmem<V>;
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* sm = align1024(smem_raw);
+  unsigned char *KQ = sm, *A = sm + S::oA, *KD = sm + S::oKD, *Vt = sm + S::oV;
+  PrepGates* gates = reinterpret_cast<PrepGates*>(sm + S::kUsed);
+  CtaShared* cs = reinterpret_cast<CtaShared*>(gates + 2);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, quad = warp & 3, half = warp >> 2, tq = tid & 127;
+  CtaCtl ctl{p.status, &cs->abort_flag};
+  uint64_t *full_kq = &cs->bar[0], *full_v = &cs->bar[1], *mma = &cs->bar[2];
+  const int nchunks = p.nbh * p.cn;
+
+  if (tid == 0) {
+    cs->abort_flag = 0;
+    for (int i = 0; i < 3; ++i) mbar_init(&cs->bar[i], 1);
+    fence_mbar_init();
+    fence_proxy_async();
+  }
+  if (warp == 0) {
+    tmem_alloc(&cs->tmem_slot, S::kCols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = cs->tmem_slot, lane_base = static_cast<uint32_t>(quad * 32) << 16;
+  griddep_wait();
+  griddep_launch();
+  {
+    const PrepAt a(p, blockIdx.x);
+    if (tid == 0) {
+      prep_load_kq(KQ, &mk, &mq, full_kq, a);
+      prep_load_v<V>(Vt, &mv, full_v, a);
+    }
+    if (warp == 1) prep_gates(p, a.b, a.c, a.h, a.z, lane, gates);
+  }
+  __syncthreads();
+
+  uint32_t ph = 0, pm = 0;
+  for (int n = blockIdx.x; n < nchunks; n += gridDim.x, ph ^= 1u) {
+    const PrepAt a(p, n);
+    const bool more = n + static_cast<int>(gridDim.x) < nchunks;
+    const PrepAt nx(p, more ? n + gridDim.x : n);
+    const PrepGates& gt = gates[ph];
+
+    mbar_wait_warp(full_kq, ph, ctl, 206);
+    for (int idx = tid; idx < 64 * 16; idx += kPrepThreads) {
+      const int r = idx >> 4, ch = idx & 15;
+      float x[8];
+      unpack8_in(tile_ld_chunk(KQ, r, ch, 128), x, p.qk16);
+      if (!p.qk16) tile_st_chunk(KQ, r, ch, 128, pack8_f16(x));
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[i] *= gt.dec[r];
+      tile_st_chunk(KD, r, ch, 64, pack8_f16(x));
+      if (!p.qk16) {
+        unpack8_bf16(tile_ld_chunk(KQ, 64 + r, ch, 128), x);
+        tile_st_chunk(KQ, 64 + r, ch, 128, pack8_f16(x));
+      }
+    }
+    mbar_wait_warp(full_v, ph, ctl, 207);
+    prep_to_f16(Vt, V * 128, tid);
+    sync_for_issue();
+    if (warp == 0) {
+      tc_fence_after();
+      const uint32_t leader = elect_leader();
+      issue_product_led(leader, tmem, Tile{smem_u32(KQ), 128, false}, Tile{smem_u32(KQ), 128, false}, 64, 128, 0u);
+      issue_product_led(leader, tmem + 64, Tile{smem_u32(KD), 64, true}, Tile{smem_u32(Vt), 64, true}, V, 64, 0u);
+      umma_commit_led(leader, mma);
+      if (tid == 0 && !p.lean) {
+        bulk_s2g(p.saved + p.lay.u + static_cast<size_t>(a.z) * p.lay.sz_u, Vt, V * 128);      // (u is v)
+        bulk_commit();
+      }
+    }
+    __syncwarp();
+    if (warp == 1 && more) prep_gates(p, nx.b, nx.c, nx.h, nx.z, lane, gates + (ph ^ 1u));
+    wait_products(mma, pm, ctl, 208);
+    if (tid == 0 && more) prep_load_kq(KQ, &mk, &mq, full_kq, nx);
+    if (!p.lean) {
+      if (tid == 0) bulk_wait_read();
+      __syncthreads();
+    }
+    if (quad >= 2) {
+      const bool live = (half == 0) || ((warp & 1) != 0);
+      float d[32];
+      if (live) {
+        tmem_ld32(tmem + lane_base + half * 32, d);
+        tmem_ld_wait();
+      }
+      prep_row_a(A, gt.G, d, tq - 64, half, live, p.scale);
+    }
+#pragma unroll
+    for (int jj = 0; jj < V / 64; ++jj) {
+      const int cb = half * (V / 2) + jj * 32;
+      float d[32];
+      tmem_ld32(tmem + 64 + lane_base + cb, d);
+      tmem_ld_wait();
+#pragma unroll
+      for (int i = 0; i < 4; ++i) tile_st_chunk(KD, tq, cb / 8 + i, 128, pack8_f16(d + 8 * i));
+    }
+    fence_proxy_async();
+    tc_fence_before();
+    __syncthreads();
+    if (tid == 0) {
+      bulk_s2g(p.saved + p.lay.r + static_cast<size_t>(a.z) * p.lay.sz_r, KD, V * 256);
+      bulk_s2g(p.saved + p.lay.ta + static_cast<size_t>(a.z) * p.lay.sz_ta + 8192, A, 8192);
+      bulk_commit();
+      bulk_wait_read();
+      if (more) prep_load_v<V>(Vt, &mv, full_v, nx);
+    }
+    __syncthreads();
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem, S::kCols);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -492,32 +668,30 @@ output_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
 // ---------------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------------
-template <int V, bool DELTA>
-static int launch_prepare_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk,
-                            const CUtensorMap& mv, cudaStream_t st) {
-  const int smem = 32768 + 16384 + V * 128 + 16384 + 16384 + 264 * 4 + static_cast<int>(sizeof(CtaShared)) + 1024;
-  auto kern = prepare_kernel<V, DELTA>;
-  static SmemAttr attr;
-  if (attr.set(kern, smem)) return kErrLaunch;
-  kern<<<p.nbh * p.cn, 256, smem, st>>>(p, mq, mk, mv);
-  return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
-}
-template <int V, bool DELTA, bool CW>
-static int launch_output_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mv, const CUtensorMap& mo, cudaStream_t st) {
-  constexpr int smem = OutSmem<V, CW>::kBytes;
-  auto kern = output_kernel<V, DELTA, CW>;
-  static SmemAttr attr;
+template <typename Kern>
+static int launch_persistent(Kern kern, SmemAttr& attr, int smem, int ctas, const Problem& p, const CUtensorMap& m0, const CUtensorMap& m1,
+                             const CUtensorMap& m2, cudaStream_t st) {
   if (attr.set(kern, smem)) return kErrLaunch;
   const int sms = sm_count(), n = p.nbh * p.cn;
   if (sms <= 0) return kErrDevice;
-  if (launch_dependent(kern, dim3(n < OutSmem<V, CW>::kCtas * sms ? n : OutSmem<V, CW>::kCtas * sms), dim3(kOutThreads), smem, st, p, mq, mv, mo) != cudaSuccess) return kErrLaunch;
+  if (launch_dependent(kern, dim3(n < ctas * sms ? n : ctas * sms), dim3(256), smem, st, p, m0, m1, m2) != cudaSuccess) return kErrLaunch;
   return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
+}
+template <int V>
+static int launch_prepare_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, cudaStream_t st) {
+  static SmemAttr attr[2];
+  return p.delta ? launch_persistent(prepare_kernel<V>, attr[0], PrepSmem<V>::kBytes, 2, p, mq, mk, mv, st)
+                 : launch_persistent(prepare_nodelta_kernel<V>, attr[1], PrepNdSmem<V>::kBytes, PrepNdSmem<V>::kCtas, p, mq, mk, mv, st);
+}
+template <int V, bool DELTA, bool CW>
+static int launch_output_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mv, const CUtensorMap& mo, cudaStream_t st) {
+  static SmemAttr attr;
+  return launch_persistent(output_kernel<V, DELTA, CW>, attr, OutSmem<V, CW>::kBytes, OutSmem<V, CW>::kCtas, p, mq, mv, mo, st);
 }
 
 int launch_prepare(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                    cudaStream_t st) {
-  if (p.V == 64) return p.delta ? launch_prepare_t<64, true>(p, mq, mk, mv, st) : launch_prepare_t<64, false>(p, mq, mk, mv, st);
-  return p.delta ? launch_prepare_t<128, true>(p, mq, mk, mv, st) : launch_prepare_t<128, false>(p, mq, mk, mv, st);
+  return p.V == 64 ? launch_prepare_t<64>(p, mq, mk, mv, st) : launch_prepare_t<128>(p, mq, mk, mv, st);
 }
 template <bool CW>
 static int launch_output_cw(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mv, const CUtensorMap& mo, cudaStream_t st) {

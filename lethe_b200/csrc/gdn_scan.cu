@@ -238,7 +238,8 @@ scan_kernel(const Problem p) {
 // Without the delta term the recurrence is x <- a x + R per element: no product, nothing serial but the
 // chunk order, and the kernel is bound by reading R and writing the state records once.  Every thread
 // owns one 16-byte piece (8 columns) of one row of the state; a warp covers four whole 128-byte rows
-// of a record atom, so every access is a full line.  R / Rb and the state records are 128-row tile images.
+// of a record atom, so every access is a full line.  A thread keeps the R of the next 16 chunks on the way (in batches of
+// 8 without overlap a scan of 47 chunks after the kernel that wrote R took SCAN_NOTE).  R / Rb and the state records are 128-row tile images.
 // Grid: (V / 64 atoms x 4 row blocks, pairs) x 256 threads.
 // ---------------------------------------------------------------------------------------------
 template <bool ADJOINT>
@@ -267,27 +268,29 @@ scan_nodelta_kernel(const Problem p) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) x[j] = x0 && d < nrow ? x0[(static_cast<size_t>(bh) * nrow + d) * V + col0 + j] : 0.f;
   }
-  constexpr int kBatch = 8;
-  for (int it0 = 0; it0 < n; it0 += kBatch) {
-    uint4 rb[kBatch];
-    float ab[kBatch];
-#pragma unroll
-    for (int j = 0; j < kBatch; ++j) {
-      if (it0 + j < n) {
-        const size_t zj = static_cast<size_t>(bh) * NT + chunk_of(it0 + j);
-        rb[j] = *reinterpret_cast<const uint4*>(Rg + zj * p.lay.sz_r + off);
-        ab[j] = ADg[zj * kK + d];
-      }
+  constexpr int kDepth = 16;
+  uint4 rb[kDepth];
+  float ab[kDepth];
+  auto load = [&](int j, int it) {
+    if (it < n) {
+      const size_t zj = static_cast<size_t>(bh) * NT + chunk_of(it);
+      rb[j] = *reinterpret_cast<const uint4*>(Rg + zj * p.lay.sz_r + off);
+      ab[j] = ADg[zj * kK + d];
     }
+  };
 #pragma unroll
-    for (int j = 0; j < kBatch; ++j) {
+  for (int j = 0; j < kDepth; ++j) load(j, j);
+  for (int it0 = 0; it0 < n; it0 += kDepth) {
+#pragma unroll
+    for (int j = 0; j < kDepth; ++j) {
       if (it0 + j < n) {
         const size_t zj = static_cast<size_t>(bh) * NT + chunk_of(it0 + j);
         *reinterpret_cast<uint4*>(Xg + (ADJOINT ? zj : zj + bh) * szx + off) = pack8_f16(x);
         float rr[8];
         unpack8_f16(rb[j], rr);
 #pragma unroll
-        for (int n = 0; n < 8; ++n) x[n] = fmaf(ab[j], x[n], rr[n]);
+        for (int e = 0; e < 8; ++e) x[e] = fmaf(ab[j], x[e], rr[e]);
+        load(j, it0 + j + kDepth);
       }
     }
   }
