@@ -5,36 +5,6 @@
 
 namespace lg {
 
-// ---- packed pairs of fp32 ----------------------------------------------------------------------------------------
-struct f2 { unsigned long long u; };
-__device__ __forceinline__ f2 pack2(float lo, float hi) {
-  f2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r.u) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack2(f2 a, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.u)); }
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
-  f2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.u) : "l"(a.u), "l"(b.u));
-  return r;
-}
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-  f2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.u) : "l"(a.u), "l"(b.u), "l"(c.u));
-  return r;
-}
-// two neighbouring pairs from shared memory (16-byte aligned)
-__device__ __forceinline__ void ld_pairs(const float* src, f2* out) {
-  const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(src);
-  out[0].u = v.x;
-  out[1].u = v.y;
-}
-__device__ __forceinline__ float sum2(f2 a) {
-  float lo, hi;
-  unpack2(a, lo, hi);
-  return lo + hi;
-}
-
 __device__ __forceinline__ float half_of(uint32_t pair, int hi) {
   const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&pair));
   return hi ? f.y : f.x;

@@ -21,11 +21,11 @@
 // The CTA is persistent: the next chunk's k, q and g are fetched as soon as the diagonal sums have read this chunk's.  v
 // is fetched under the first epilogue: its tile holds the decayed source rows before.
 #include "gdn_cw.cuh"
+#include "gdn_inverse.cuh"
 #include "host_util.h"
 
 namespace lg {
 
-constexpr int kMsC = 68;
 constexpr int kPrepCwThreads = 512;
 constexpr int kDg = 17;                               // row stride (floats) of the diagonal-block buffers
 
@@ -89,7 +89,7 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
   unsigned char *tK = sm + S::oK, *tQ = sm + S::oQ, *BV = sm + S::oV, *LA = sm + S::oLA, *KR = sm + S::oKR, *GK = sm + S::oGK;
   unsigned char *KD = sm + S::oKD, *TA = sm + S::oTA, *WU = KR, *SP = LA, *SR = GK;
   float *G = reinterpret_cast<float*>(sm + S::oG), *kfd = reinterpret_cast<float*>(sm + S::oV), *Bg = reinterpret_cast<float*>(sm + S::oBg);
-  float* Msm = reinterpret_cast<float*>(LA);
+  float* Mt = reinterpret_cast<float*>(LA);
   float* Adg = reinterpret_cast<float*>(sm + S::oF);
   float* Mdg = Adg + 64 * kDg;
   float* betas = Mdg + 64 * kDg;
@@ -391,9 +391,8 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
             x[e] *= be;
             if (I == blk) x[e] = blk * 16 + e < r ? Mdg[r * kDg + e] : 0.f;
           }
-          float* m = Msm + r * kMsC + blk * 16;
-          st8(m, x);
-          st8(m + 8, x + 8);
+#pragma unroll
+          for (int e = 0; e < 16; ++e) Mt[(blk * 16 + e) * kMt + r] = x[e];
         }
       } else {
 #pragma unroll
@@ -429,7 +428,7 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
     }
     // ---- T = (I + M)^-1 (fp32, CUDA cores)
     if (DELTA) {
-      unit_lower_inverse64_blocked<kMsC>(Msm, Msm + 64 * kMsC, TA, tid);
+      unit_lower_inverse64(Mt, Mt + kInvMtFloats, TA, tid);
       sync_for_issue();
       // ---- [w | u] = T [b gamma k | beta v]
       if (warp == 0) {

@@ -5,12 +5,10 @@
 // fp32 accumulators in TMEM; two 64-row operands that share the other operand are stacked into one
 // 128-row tile so that a single product serves both (rows 0-63 of the accumulator belong to the
 // first, rows 64-127 to the second).
-#include "gdn_common.cuh"
+#include "gdn_inverse.cuh"
 #include "host_util.h"
 
 namespace lg {
-
-constexpr int kMs = 68;  // row stride (floats) of the fp32 copy of M used by the inverse
 
 // ---------------------------------------------------------------------------------------------
 // prepare, scalar gate (or none): per chunk
@@ -99,34 +97,34 @@ __device__ __forceinline__ void prep_kd(unsigned char* KD, const unsigned char* 
     tile_st_chunk(KD, r, ch, 64, pack8_f16(x));
   }
 }
-// row r of A, 32 columns from 32 half: d holds those of q k^T (live: not all of them right of the diagonal)
-__device__ __forceinline__ void prep_row_a(unsigned char* A, const float* Gs, const float* d, int r, int half, bool live, float scale) {
+// 32 columns (from 32 half) of row r of a product, times the decay between the tokens and `f`; zero from column `end` on.
+// Everything in registers first: with a store or a branch between them the exponentials run one at a time (2.7 k cycles).
+__device__ __forceinline__ void prep_decay_row(float* d, const float* Gs, int r, int half, int end, float f) {
   const float Gr = Gs[r];
+  float g[32];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int s8 = half * 4 + q;
-    float a[8];
+  for (int q = 0; q < 4; ++q) ld8(Gs + half * 32 + 8 * q, g + 8 * q);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) a[i] = 0.f;
-    if (live) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int s = s8 * 8 + i;
-        a[i] = (s <= r) ? scale * __expf(Gr - Gs[s]) * d[q * 8 + i] : 0.f;
-      }
-    }
-    tile_st_chunk(A, r, s8, 64, pack8_f16(a));
+  for (int j = 0; j < 32; ++j) {
+    const float x = f * __expf(fminf(Gr - g[j], 0.f)) * d[j];
+    d[j] = half * 32 + j < end ? x : 0.f;
   }
+}
+// the 32 columns of row r of A: lane quadrants 0 of either half have nothing right of column 31 (live)
+__device__ __forceinline__ void prep_row_a(unsigned char* A, const float* Gs, float* d, int r, int half, bool live, float scale) {
+  if (live) prep_decay_row(d, Gs, r, half, r + 1, scale);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) tile_st_chunk(A, r, half * 4 + q, 64, live ? pack8_f16(d + 8 * q) : make_uint4(0u, 0u, 0u, 0u));
 }
 
 template <int V>
 struct PrepSmem {
   static constexpr int oTA = 32768;              // behind [k; q]: [T; A]; then, with kd, P on its way out
-  static constexpr int oKD = oTA + 16384;        // M in fp32 and the scratch of its inverse (30 KB); then kd
+  static constexpr int oKD = oTA + 16384;        // M in fp32 and the scratch of its inverse (29 KB); then kd
   static constexpr int oW = oKD + 16384;         // [T diag(beta gamma); T diag(beta)]; then w; then R (d_v = 128: with u) on its way out
   static constexpr int oV = oW + 16384;          // v; then u
   static constexpr int kUsed = oV + V * 128, kBytes = kUsed + 2 * static_cast<int>(sizeof(PrepGates)) + static_cast<int>(sizeof(CtaShared)) + 1024;
-  static_assert((64 * kMs + kInvScratchFloats) * 4 <= 32768, "scratch of the inverse");
+  static_assert((kInvMtFloats + kInvScratchFloats) * 4 <= 32768, "scratch of the inverse");
 };
 
 template <int V>
@@ -137,7 +135,7 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
   extern __shared__ unsigned char smem_raw[];
   unsigned char* sm = align1024(smem_raw);
   unsigned char *KQ = sm, *TA = sm + S::oTA, *KD = sm + S::oKD, *W = sm + S::oW, *Vt = sm + S::oV;
-  float *Msm = reinterpret_cast<float*>(KD), *Tsm = Msm + 64 * kMs;
+  float* Mt = reinterpret_cast<float*>(KD);
   PrepGates* gates = reinterpret_cast<PrepGates*>(sm + S::kUsed);
   CtaShared* cs = reinterpret_cast<CtaShared*>(gates + 2);
   // Threads 0-127 and 128-255 reach the same TMEM lanes (lane quadrant = warp & 3): the two halves take
@@ -206,19 +204,9 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
         tmem_ld_wait();
       }
       if (tq < 64) {
-        const int r = tq;
-        const float Gr = gt.G[r], be = gt.beta[r];
+        if (live) prep_decay_row(d, gt.G, tq, half, tq, gt.beta[tq]);
 #pragma unroll
-        for (int j4 = 0; j4 < 8; ++j4) {
-          float m[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int s = half * 32 + 4 * j4 + e;
-            m[e] = 0.f;
-            if (live) m[e] = (s < r) ? be * __expf(Gr - gt.G[s]) * d[4 * j4 + e] : 0.f;
-          }
-          *reinterpret_cast<float4*>(Msm + r * kMs + half * 32 + 4 * j4) = make_float4(m[0], m[1], m[2], m[3]);
-        }
+        for (int j = 0; j < 32; ++j) Mt[(half * 32 + j) * kMt + tq] = live ? d[j] : 0.f;
       } else {
         prep_row_a(TA + 8192, gt.G, d, tq - 64, half, live, p.scale);
       }
@@ -227,20 +215,22 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
     __syncthreads();
 
     // ---- T = (I + M)^-1 (fp32, CUDA cores)
-    unit_lower_inverse64_blocked<kMs>(Msm, Tsm, TA, tid);
+    unit_lower_inverse64(Mt, Mt + kInvMtFloats, TA, tid);
     mbar_wait_warp(full_v, ph, ctl, 203);
     prep_to_f16(Vt, V * 128, tid);
     __syncthreads();
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const int idx = tid + u * kPrepThreads, r = idx >> 3, ch = idx & 7;
-      float t[8], x[8];
+      float t[8], x[8], b[8];
       unpack8_f16(tile_ld_chunk(TA, r, ch, 128), t);
+      ld8(gt.bg + ch * 8, b);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) x[i] = t[i] * gt.bg[ch * 8 + i];
+      for (int i = 0; i < 8; ++i) x[i] = t[i] * b[i];
+      ld8(gt.beta + ch * 8, b);
       tile_st_chunk(W, r, ch, 128, pack8_f16(x));
 #pragma unroll
-      for (int i = 0; i < 8; ++i) x[i] = t[i] * gt.beta[ch * 8 + i];
+      for (int i = 0; i < 8; ++i) x[i] = t[i] * b[i];
       tile_st_chunk(W, 64 + r, ch, 128, pack8_f16(x));
     }
     sync_for_issue();
@@ -281,6 +271,7 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
         for (int i = 0; i < 4; ++i) tile_st_chunk(Vt, tq - 64, cb / 8 + i, 64, pack8_f16(d + 8 * i));
       }
     }
+    if (tid == 0) bulk_wait_read();                  // [T; A] have left their tile
     sync_for_issue();
 
     // ---- product 3: [P | R] = kd^T [w | u]
@@ -300,34 +291,39 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
     __syncwarp();
     if (warp == 1 && more) prep_gates(p, nx.b, nx.c, nx.h, nx.z, lane, gates + (ph ^ 1u));
     wait_products(mma, pm, ctl, 205);
-    // P and R leave from tiles that nothing reads any more, once the stores of w and u have read them
+    // P leaves from where [T; A] and kd were, R from where w (and u) were once their stores have read them
+#pragma unroll
+    for (int jj = 0; jj < 2; ++jj) {
+      const int cb = half * 64 + jj * 32;
+      float d[32];
+      tmem_ld32(tmem + lane_base + cb, d);
+      tmem_ld_wait();
+#pragma unroll
+      for (int i = 0; i < 4; ++i) tile_st_chunk(TA, tq, cb / 8 + i, 128, pack8_f16(d + 8 * i));
+    }
+    fence_proxy_async();
     if (tid == 0) {
       bulk_wait_read();
       if (V == 64 && more) prep_load_v<V>(Vt, &mv, full_v, nx);
     }
     __syncthreads();
-    {
-      unsigned char *SP = TA, *SR = W;
-      constexpr int kHalf = (128 + V) / 64;
-#pragma unroll 1
-      for (int jb = half * kHalf; jb < (half + 1) * kHalf; ++jb) {
-        float d[32];
-        tmem_ld32(tmem + lane_base + jb * 32, d);
-        tmem_ld_wait();
-        if (jb < 4) {
+    if (tid == 0) {
+      bulk_s2g(p.saved + p.lay.p + static_cast<size_t>(a.z) * p.lay.sz_p, TA, 32768);
+      bulk_commit();
+    }
 #pragma unroll
-          for (int i = 0; i < 4; ++i) tile_st_chunk(SP, tq, jb * 4 + i, 128, pack8_f16(d + 8 * i));
-        } else {
+    for (int jj = 0; jj < V / 64; ++jj) {
+      const int cb = half * (V / 2) + jj * 32;
+      float d[32];
+      tmem_ld32(tmem + 128 + lane_base + cb, d);
+      tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(SR + rrec_off(tq, (jb - 4) * 4 + i)) = pack8_f16(d + 8 * i);
-        }
-      }
+      for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(W + rrec_off(tq, cb / 8 + i)) = pack8_f16(d + 8 * i);
     }
     fence_proxy_async();
     tc_fence_before();
     __syncthreads();
     if (tid == 0) {
-      bulk_s2g(p.saved + p.lay.p + static_cast<size_t>(a.z) * p.lay.sz_p, TA, 32768);
       bulk_s2g(p.saved + p.lay.r + static_cast<size_t>(a.z) * p.lay.sz_r, W, V * 256);
       bulk_commit();
     }
