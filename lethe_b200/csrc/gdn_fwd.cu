@@ -24,7 +24,7 @@ namespace lg {
 // per SM; the next k, q and v are fetched as soon as their tiles are dead (k and q under product 3 and the last epilogue),
 // and the gates are summed a chunk ahead by one warp.  With one CTA per chunk instead, the wait for the first loads and the
 // start of the CTA were 40 % of its time.  The gates are applied to the columns of T, not to k and v: half the elements.
-// PREPARE_NOTE
+// 4096 chunks: d_v = 64 167 -> 132 us, d_v = 128 183 -> 143; without the delta term (below) d_v = 128 121 -> 85.
 // ---------------------------------------------------------------------------------------------
 constexpr int kPrepThreads = 256;
 
@@ -666,11 +666,13 @@ output_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
 // ---------------------------------------------------------------------------------------------
 template <typename Kern>
 static int launch_persistent(Kern kern, SmemAttr& attr, int smem, int ctas, const Problem& p, const CUtensorMap& m0, const CUtensorMap& m1,
-                             const CUtensorMap& m2, cudaStream_t st) {
+                             const CUtensorMap& m2, cudaStream_t st, bool early = true) {
   if (attr.set(kern, smem)) return kErrLaunch;
   const int sms = sm_count(), n = p.nbh * p.cn;
   if (sms <= 0) return kErrDevice;
-  if (launch_dependent(kern, dim3(n < ctas * sms ? n : ctas * sms), dim3(256), smem, st, p, m0, m1, m2) != cudaSuccess) return kErrLaunch;
+  const int grid = n < ctas * sms ? n : ctas * sms;
+  if (!early) kern<<<grid, 256, smem, st>>>(p, m0, m1, m2);
+  else if (launch_dependent(kern, dim3(grid), dim3(256), smem, st, p, m0, m1, m2) != cudaSuccess) return kErrLaunch;
   return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
 }
 template <int V>
@@ -682,7 +684,10 @@ static int launch_prepare_t(const Problem& p, const CUtensorMap& mq, const CUten
 template <int V, bool DELTA, bool CW>
 static int launch_output_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mv, const CUtensorMap& mo, cudaStream_t st) {
   static SmemAttr attr;
-  return launch_persistent(output_kernel<V, DELTA, CW>, attr, OutSmem<V, CW>::kBytes, OutSmem<V, CW>::kCtas, p, mq, mv, mo, st);
+  // A part of the sequences (a captured step that overlaps parts): early CTAs would wait in room that a scan or a chunk kernel
+  // of another part needs (B H = 16, 32 chunks: 112 -> 109 us, 4096 chunks 584 -> 571; without the delta term nothing is that long)
+  const bool early = !DELTA || p.cn == p.NT;
+  return launch_persistent(output_kernel<V, DELTA, CW>, attr, OutSmem<V, CW>::kBytes, OutSmem<V, CW>::kCtas, p, mq, mv, mo, st, early);
 }
 
 int launch_prepare(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,

