@@ -678,8 +678,13 @@ static int launch_persistent(Kern kern, SmemAttr& attr, int smem, int ctas, cons
 template <int V>
 static int launch_prepare_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, cudaStream_t st) {
   static SmemAttr attr[2];
-  return p.delta ? launch_persistent(prepare_kernel<V>, attr[0], PrepSmem<V>::kBytes, 2, p, mq, mk, mv, st)
-                 : launch_persistent(prepare_nodelta_kernel<V>, attr[1], PrepNdSmem<V>::kBytes, PrepNdSmem<V>::kCtas, p, mq, mk, mv, st);
+  // Not early for a later part of the sequences of at most two rounds: its CTAs would take the SMs that the scan of the first
+  // part starts on (captured step of B H = 16, 32 chunks: 108.5 -> 105.6 us).  With more rounds the time saved at its start
+  // counts for more (4096 chunks: 572 us early, 582 not).
+  const int sms = sm_count();
+  const bool early = p.c0 == 0 || p.nbh * p.cn > 4 * sms;
+  return p.delta ? launch_persistent(prepare_kernel<V>, attr[0], PrepSmem<V>::kBytes, 2, p, mq, mk, mv, st, early)
+                 : launch_persistent(prepare_nodelta_kernel<V>, attr[1], PrepNdSmem<V>::kBytes, PrepNdSmem<V>::kCtas, p, mq, mk, mv, st, early);
 }
 template <int V, bool DELTA, bool CW>
 static int launch_output_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mv, const CUtensorMap& mo, cudaStream_t st) {

@@ -5,7 +5,7 @@ import torch
 
 from lethe_b200 import ops
 from lethe_b200.synth import make_inputs
-from oracle.gdn_oracle import scale_rel, serial_forward
+from oracle.gdn_oracle import scale_rel, serial_backward, serial_backward_full, serial_forward
 
 from .wsview import report
 
@@ -32,3 +32,64 @@ def test_decode_of_many_pairs(gate, delta, dtype, extra, shift):
     errs = {"o": scale_rel(o.double().cpu(), o_ref[:, 0]), "state": scale_rel(state.double().cpu(), hT_ref)}
     report(f"decode gate={gate} delta={delta} pairs={H}", errs)
     assert max(errs.values()) <= TOL, errs
+
+
+@pytest.mark.parametrize("gate,delta,V,K,H,L,dtype", [
+    # more chunks than any persistent grid has CTAs (up to four per SM), the last of every sequence ragged
+    ("scalar", True, 64, 128, 450, 100, torch.bfloat16), ("scalar", True, 128, 128, 310, 128, torch.bfloat16),
+    ("scalar", False, 64, 64, 450, 100, torch.bfloat16), ("none", False, 128, 128, 310, 128, torch.float16),
+    ("channel", True, 128, 128, 155, 100, torch.bfloat16), ("channel", True, 64, 64, 155, 128, torch.float16),
+    ("channel", False, 64, 128, 155, 100, torch.bfloat16),
+    # state scans: 16 columns per CTA for the last time, 64 for the first; without the delta term 16 and 8 records ahead
+    ("scalar", True, 64, 128, 37, 320, torch.bfloat16), ("scalar", True, 64, 128, 38, 320, torch.bfloat16),
+    ("none", False, 64, 128, 74, 1088, torch.bfloat16), ("none", False, 64, 128, 75, 1088, torch.bfloat16)])
+def test_persistent_grids_and_scan_rules(gate, delta, V, K, H, L, dtype):
+    dev = torch.device("cuda")
+    inp = make_inputs(1, L, H, K, V, gate=gate, delta=delta, seed=9, mild=True)
+    heads = [0, H // 2, H - 1]               # the pairs are independent: the oracle takes three of them
+    pick = lambda n, t: None if t is None else t[:, heads] if n == "h0" else t[:, :, heads]      # noqa: E731
+    f64 = {n: (None if t is None else pick(n, t).double()) for n, t in inp.items()}
+    o_ref, hT_ref, gr = serial_backward(*(f64[n] for n in ("q", "k", "v", "g", "beta", "h0", "do")))
+    names = [n for n in ("q", "k", "v", "g", "beta", "h0") if inp[n] is not None]
+    cast = lambda n, t: t.to(dev, dtype) if n in ("q", "k") else t.to(dev)      # noqa: E731
+    d = {n: cast(n, inp[n]).requires_grad_(True) for n in names}
+    o, hT = ops.gdn_chunk(*(d.get(n) for n in ("q", "k", "v", "g", "beta", "h0")))
+    got = dict(zip(names, torch.autograd.grad(o, [d[n] for n in names], inp["do"].to(dev))))
+    back = lambda n, t: pick(n, t.detach().double().cpu())      # noqa: E731
+    ref = {"q": gr.dq, "k": gr.dk, "v": gr.dv, "g": gr.dg, "beta": gr.dbeta, "h0": gr.dh0}
+    errs = {"o": scale_rel(back("o", o), o_ref), "hT": scale_rel(back("h0", hT), hT_ref)}
+    errs.update({"d" + n: scale_rel(back(n, got[n]), ref[n]) for n in names})
+    report(f"edges gate={gate} delta={delta} V={V} K={K} H={H} L={L}", errs)
+    assert max(errs.values()) <= TOL, errs
+
+
+@pytest.mark.parametrize("V,H,dtype", [(64, 150, torch.float32), (128, 150, torch.bfloat16)])
+def test_per_channel_gates_with_more_chunks_than_ctas(V, H, dtype):
+    dev = torch.device("cuda")
+    inp = make_inputs(1, 128, H, 128, V, gate="channel", seed=6, mild=True, full=True)
+    heads = [0, H - 1]
+    names = ("q", "k", "v", "g", "b", "w")
+    f64 = {n: inp[n][:, :, heads].double() for n in names}
+    o_ref, _, ref = serial_backward_full(*(f64[n] for n in names), None, inp["do"][:, :, heads].double())
+    d = {n: inp[n].to(dev, dtype if n in "qkv" else torch.float32).requires_grad_(True) for n in names}
+    o = ops.gdn2_op(*(d[n] for n in names), use_qk_l2norm=False)
+    got = dict(zip(names, torch.autograd.grad(o, [d[n] for n in names], inp["do"].to(dev, o.dtype))))
+    errs = {"o": scale_rel(o.detach().double().cpu()[:, :, heads], o_ref)}
+    errs.update({"d" + n: scale_rel(got[n].double().cpu()[:, :, heads], ref[n]) for n in names})
+    report(f"per-channel gates V={V} {dtype}", errs)
+    assert max(errs.values()) <= TOL, errs
+
+
+@pytest.mark.parametrize("rows,K,V", [(1, 64, 64), (97, 128, 64), (5000, 128, 128)])
+def test_gate_regime_sees_one_differing_channel(rows, K, V):
+    dev = torch.device("cuda")
+    g = -torch.rand(1, rows, 1, 1, device=dev).expand(1, rows, 1, K).contiguous()
+    b = torch.rand(1, rows, 1, 1, device=dev).expand(1, rows, 1, K).contiguous()
+    w = b[..., :1].expand(1, rows, 1, V).contiguous()
+    assert ops.gate_regime(g, b, w) == (True, True, False)
+    assert ops.gate_regime(g, torch.zeros_like(b), torch.ones_like(w)) == (True, False, True)
+    for t, want in ((g, (False, True, False)), (b, (True, False, False)), (w, (True, False, False))):
+        last = t[0, -1, 0, -1].clone()
+        t[0, -1, 0, -1] = torch.nextafter(last, torch.zeros_like(last))
+        assert ops.gate_regime(g, b, w) == want
+        t[0, -1, 0, -1] = last
