@@ -257,46 +257,33 @@ def path_fractions(workload: str, fwd_ms: float, bwd_ms: float, step_ms: float, 
 # ------------------------------------------------------------------------------------------------
 # DRAM traffic per chunk (dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture / chunks of that
 # launch), from the captures summarised under profiles/ (2048- and 4096-chunk workloads, records larger than L2;
-# every kernel's traffic grows in proportion to its chunks).  Keyed by (kernel, gate, d_v, delta); the
-# channel-wise "stageb" and "wy" are two launches each, summed.  Absent combinations report null.
+# every kernel's traffic grows in proportion to its chunks).  Keyed by (kernel, gate, d_v, delta).
+# Absent combinations report null.
 NCU_DRAM_BYTES_PER_CHUNK = {
-    # scalar-gate GDN, B4 H8 L4096 d_v 64 (2048 chunks)
-    ("prepare", "scalar", 64, True): (85.0e6 + 127.6e6) / 2048,
-    ("scan_fwd", "scalar", 64, True): (102.8e6 + 14.0e6) / 2048,
-    ("output", "scalar", 64, True): (151.5e6 + 18.1e6) / 2048,
-    ("bwd_pre", "scalar", 64, True): (118.0e6 + 14.1e6) / 2048,
-    ("scan_bwd", "scalar", 64, True): (101.7e6 + 14.0e6) / 2048,
-    ("stageb", "scalar", 64, True): (185.1e6 + 104.6e6) / 2048,
-    ("wy", "scalar", 64, True): (203.0e6 + 35.3e6) / 2048,
-    # KDA, B4 H8 L4096 d_v 128 (2048 chunks)
-    ("prepare", "channel", 128, True): (168.5e6 + 279.2e6) / 2048,
-    ("scan_fwd", "channel", 128, True): (137.4e6 + 38.2e6) / 2048,
-    ("output", "channel", 128, True): (201.4e6 + 43.8e6) / 2048,
-    ("bwd_pre", "channel", 128, True): (134.2e6 + 36.5e6) / 2048,
-    ("scan_bwd", "channel", 128, True): (135.3e6 + 37.6e6) / 2048,
-    ("stageb", "channel", 128, True): (369.2e6 + 240.3e6 + 352.4e6 + 129.5e6) / 2048,
-    ("wy", "channel", 128, True): (235.5e6 + 87.9e6 + 319.9e6 + 81.0e6) / 2048,
-    # GLA, B4 H16 L4096 d_v 128 (4096 chunks)
-    ("prepare", "channel", 128, False): (335.6e6 + 418.7e6) / 4096,
-    ("scan_fwd", "channel", 128, False): (141.0e6 + 93.5e6) / 4096,
-    ("output", "channel", 128, False): (335.6e6 + 105.7e6) / 4096,
-    ("bwd_pre", "channel", 128, False): (134.2e6 + 89.7e6) / 4096,
-    ("scan_bwd", "channel", 128, False): (136.4e6 + 90.6e6) / 4096,
-    ("stageb", "channel", 128, False): (738.3e6 + 460.8e6 + 704.7e6 + 244.6e6) / 4096,
-    # SSD, B4 H16 L4096 d_v 128 (4096 chunks)
-    ("prepare", "scalar", 128, False): (202.5e6 + 217.3e6) / 4096,
-    ("scan_fwd", "scalar", 128, False): (141.0e6 + 92.5e6) / 4096,
-    ("output", "scalar", 128, False): (336.6e6 + 106.5e6) / 4096,
-    ("bwd_pre", "scalar", 128, False): (135.3e6 + 90.4e6) / 4096,
-    ("scan_bwd", "scalar", 128, False): (136.4e6 + 91.0e6) / 4096,
-    ("stageb", "scalar", 128, False): (571.6e6 + 179.6e6) / 4096,
-    # LA, B4 H16 L4096 d_v 128 (4096 chunks)
-    ("prepare", "none", 128, False): (201.4e6 + 216.9e6) / 4096,
-    ("scan_fwd", "none", 128, False): (141.0e6 + 93.0e6) / 4096,
-    ("output", "none", 128, False): (335.6e6 + 105.9e6) / 4096,
-    ("bwd_pre", "none", 128, False): (134.2e6 + 90.8e6) / 4096,
-    ("scan_bwd", "none", 128, False): (136.4e6 + 89.7e6) / 4096,
-    ("stageb", "none", 128, False): (570.5e6 + 178.0e6) / 4096,
+    ("prepare", "scalar", 64, True): (85.0e6 + 125.3e6) / 2048,
+    ("scan_fwd", "scalar", 64, True): (102.8e6 + 10.0e6) / 2048,
+    ("output", "scalar", 64, True): (134.8e6 + 12.0e6) / 2048,
+    ("bwd_pre", "scalar", 64, True): (101.2e6 + 4.1e6) / 2048,
+    ("scan_bwd", "scalar", 64, True): (101.7e6 + 9.9e6) / 2048,
+    ("main", "scalar", 64, True): (219.3e6 + 52.3e6) / 2048,
+    ("prepare", "channel", 128, True): (168.4e6 + 211.3e6) / 2048,
+    ("scan_fwd", "channel", 128, True): (137.4e6 + 37.2e6) / 2048,
+    ("output", "channel", 128, True): (184.6e6 + 35.7e6) / 2048,
+    ("bwd_pre", "channel", 128, True): (117.5e6 + 25.4e6) / 2048,
+    ("scan_bwd", "channel", 128, True): (135.3e6 + 36.4e6) / 2048,
+    ("main", "channel", 128, True): (403.4e6 + 136.8e6) / 2048,
+    ("prepare", "channel", 128, False): (335.6e6 + 198.6e6) / 4096,
+    ("scan_fwd", "channel", 128, False): (140.6e6 + 86.7e6) / 4096,
+    ("output", "channel", 128, False): (302.0e6 + 48.6e6) / 4096,
+    ("bwd_pre", "channel", 128, False): (134.2e6 + 78.0e6) / 4096,
+    ("scan_bwd", "channel", 128, False): (136.4e6 + 83.7e6) / 4096,
+    ("main", "channel", 128, False): (704.8e6 + 300.8e6) / 4096,
+    ("prepare", "scalar", 128, False): (202.5e6 + 123.3e6) / 4096,
+    ("scan_fwd", "scalar", 128, False): (140.5e6 + 86.5e6) / 4096,
+    ("output", "scalar", 128, False): (303.1e6 + 47.4e6) / 4096,
+    ("bwd_pre", "scalar", 128, False): (135.6e6 + 78.6e6) / 4096,
+    ("scan_bwd", "scalar", 128, False): (136.3e6 + 82.3e6) / 4096,
+    ("main", "scalar", 128, False): (571.6e6 + 173.0e6) / 4096,
 }
 
 
@@ -308,34 +295,29 @@ def measured_traffic(kernel: str, gate: str, V: int, delta: bool, Z: int):
 # ------------------------------------------------------------------------------------------------
 def algorithmic_bytes(kernel: str, Z: int, BH: int, V: int, delta: bool, cw: bool = False) -> int:
     """Bytes one launch of `kernel` must move: each input tile and each record read once, each
-    result written once (Z chunks, 64 tokens each; K = 128).  With the channel-wise gate "prepare" also
-    writes the chunk's 32 KB tile of cumulative gate values and the 16 KB record of the scaled, decayed
-    query (which "output" and "bwd_pre" read in place of q), the Stage B and WY kernels read the gate
-    tile, and "stageb" and "wy" are two launches each that pass three fp32 64 x 128 records (dq / dk / dg
-    parts) between them."""
+    result written once (Z chunks, 64 tokens each; K = 128), as a training step keeps records.  With the
+    channel-wise gate "prepare" also writes the 16 KB record of the scaled, decayed query, which "output" and
+    "bwd_pre" read in place of q.  Without the delta term v_new is v itself."""
     qk, vv, img = 64 * 128 * 2, 64 * V * 2, 128 * V * 2
     ta, w, p_, r, f32k = 16384, 16384, 32768, 128 * V * 2, 64 * 128 * 4
     if cw:
         g = f32k
         per = {
-            "prepare": g + 2 * qk + vv + g + qk + ta + vv + r + ((w + p_) if delta else 0) + 512,
+            "prepare": g + 2 * qk + vv + qk + ta + r + ((w + p_ + vv) if delta else 0) + 512,
             "scan_fwd": (p_ if delta else 0) + r + img + 512,
-            "output": qk + ta + img + vv + vv + vv + (w if delta else 0),
-            "bwd_pre": qk + vv + r + ((w + ta) if delta else 0),
+            "output": qk + ta // 2 + img + vv + vv + ((vv + w) if delta else 0),
+            "bwd_pre": qk + vv + r + ((w + ta // 2) if delta else 0),
             "scan_bwd": (p_ if delta else 0) + r + img + 512,
-            "stageb": (g + 2 * qk + vv + ta + vv + 2 * img + 8192 + 3 * f32k + (vv + w if delta else vv))
-                      + (g + 2 * qk + 8192 + 3 * f32k + qk + (2 * f32k if delta else qk + f32k)),
-            "wy": (g + qk + vv + ta + vv + w + 8192 + f32k + vv) + (g + qk + 8192 + 3 * f32k + qk + f32k),
+            "main": g + 2 * qk + vv + 2 * img + vv + 2 * qk + vv + g + ((ta + vv) if delta else ta // 2),
         }[kernel]
         return per * Z
     per = {
-        "prepare": 2 * qk + vv + ta + vv + r + ((w + p_) if delta else 0) + 512,
+        "prepare": 2 * qk + vv + r + 512 + ((ta + w + p_ + vv) if delta else ta // 2),
         "scan_fwd": (p_ if delta else 0) + r + img + 512,
-        "output": qk + ta + img + vv + vv + vv + (w if delta else 0),
-        "bwd_pre": qk + vv + r + ((w + ta) if delta else 0),
+        "output": qk + ta // 2 + img + vv + vv + ((vv + w) if delta else 0),
+        "bwd_pre": qk + vv + r + ((w + ta // 2) if delta else 0),
         "scan_bwd": (p_ if delta else 0) + r + img + 512,
-        "stageb": 2 * qk + vv + ta + vv + 2 * img + qk + (vv + w + f32k if delta else qk + vv),
-        "wy": qk + vv + ta + vv + w + f32k + qk + vv,
+        "main": 2 * qk + vv + 2 * img + vv + 2 * qk + vv + ((ta + vv) if delta else ta // 2),
     }[kernel]
     return per * Z
 
@@ -343,7 +325,7 @@ def algorithmic_bytes(kernel: str, Z: int, BH: int, V: int, delta: bool, cw: boo
 def io_bytes(kernel: str, Z: int, V: int, delta, gate: str) -> int:
     """The part of `algorithmic_bytes` that the path itself requires whatever the kernel decomposition: the
     first read of each user tensor in a pass, the final outputs, and the chunk-entry state (written once by
-    the forward scan, read once by Stage B).  The rest of a kernel's bytes are records the kernels hand to
+    the forward scan, read once by the backward's main kernel).  The rest of a kernel's bytes are records the kernels hand to
     one another and re-reads of inputs - traffic this design chose, not traffic the path needs."""
     qk, vv, img = 64 * 128 * 2, 64 * V * 2, 128 * V * 2
     gin = {"none": 0, "scalar": 64 * 4, "channel": 64 * 128 * 4}[gate]      # gate values of a chunk
@@ -354,9 +336,7 @@ def io_bytes(kernel: str, Z: int, V: int, delta, gate: str) -> int:
         "output": vv,                                              # o
         "bwd_pre": qk + vv,                                        # q, do (first touch of the backward)
         "scan_bwd": 0,
-        # k, state; dq; without the delta term also dk, dv, dg
-        "stageb": qk + img + qk + ((qk + vv + gin) if not delta else 0),
-        "wy": vv + qk + vv + gin + bin_,                           # v; dk, dv, dg, dbeta
+        "main": qk + vv + img + 2 * qk + vv + gin + bin_,          # k, v, state; dq, dk, dv, dg, dbeta
     }[kernel]
     return per * Z
 
@@ -556,7 +536,7 @@ def sp_main(args, rank, world, dev, B, L, H, K, V, gate, delta, config):
                           "ms_per_step": float(ms), "higher_is_better": True, "scaling": "strong",
                           "vs_baseline": None, "dtype": "fp16 operands, fp32 accumulate (bf16 in/out)",
                           "data": "synthetic", "config": config,
-                          "gpu_launches": args.steps * (9 if gate == "channel" and delta else 7)}))
+                          "gpu_launches": args.steps * 6}))
     dist.destroy_process_group()
 
 
@@ -686,7 +666,7 @@ def main():
     # ---- per-kernel timing (each kernel alone, same records in place), for the roofline
     kern = {}
     names_f = [("prepare", 1), ("scan_fwd", 2), ("output", 4)]
-    names_b = [("bwd_pre", 1), ("scan_bwd", 2), ("stageb", 4)] + ([("wy", 8)] if delta else [])
+    names_b = [("bwd_pre", 1), ("scan_bwd", 2), ("main", 12)]
     step()
     for name, m in names_f:
         kern[name] = timed(lambda m=m: ops.forward_into(buf, d["q"], d["k"], d["v"], g, beta, h0, scale, m, **gates),
@@ -814,9 +794,8 @@ def main():
                     "host_link": pcie,
                     "host_link_floor_ms": max(h2d, d2h) / (pcie["both"]["slowest_rank_gbs"] * 1e9) * 1e3},
             "autograd_op_ms": op_ms,
-            # kernels per replayed step: three per forward segment of the step graph, the backward kernels per
-            # backward segment
-            "gpu_launches": args.steps * ((3 * graph.segments + ((6 if delta else 4) if gate == "channel" else (4 if delta else 3)) * (len(graph.bwd_cuts) + 1))),
+            # kernels per replayed step: three per forward and per backward segment of the step graph
+            "gpu_launches": args.steps * 3 * (graph.segments + len(graph.bwd_cuts) + 1),
             "clocks": clocks,
             "roofline": {"kernel": top, "bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
                          "frac": achieved / hbm, "peak_source": which,

@@ -121,6 +121,12 @@ typedef struct LetheGdnArgs {
   /* Non-zero: the call leaves only results in memory, and in the workspaces what its own later kernels and, after a   */
   /* forward, the backward read.  Zero: also intermediates that a caller may want to look at (dv2, dw).                */
   uint32_t lean;
+  /* Forward, LETHE_GATE_CHANNEL only.  l2_eps > 0: q and k are normalised as they are read, x rsqrt(sum x^2 + l2_eps)   */
+  /* per token-head, in fp32 and rounded once to fp16 (what lethe_gdn_l2norm_qk does, without its pass over memory);    */
+  /* q_norm, k_norm (both or neither) take the normalised rows, fp16, for the backward.                                 */
+  float l2_eps;
+  void* q_norm;
+  void* k_norm;
 } LetheGdnArgs;
 
 /* Bytes of the forward->backward workspace / of the backward scratch for these sizes (0 = bad dims). */

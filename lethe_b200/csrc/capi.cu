@@ -8,7 +8,8 @@
 
 namespace lg {
 int launch_prepare(const Problem&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, cudaStream_t);
-int launch_prepare_cw(const Problem&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap& mg, cudaStream_t);
+int launch_prepare_cw(const Problem&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap& mg,
+                      const NormMaps&, cudaStream_t);
 int launch_output(const Problem&, const CUtensorMap& mq, const CUtensorMap& mv, const CUtensorMap& mo, cudaStream_t);
 int launch_scan(const Problem&, bool adjoint, cudaStream_t);
 int launch_bwd_pre(const Problem&, const CUtensorMap& mq, const CUtensorMap& mdo, cudaStream_t);
@@ -101,6 +102,12 @@ static int fill_problem(const LetheGdnArgs* a, Problem* p, bool backward) {
   p->scale = a->scale;
   p->qk16 = a->qk_f16 ? 1 : 0;
   p->lean = a->lean ? 1 : 0;
+  if (!backward && a->l2_eps != 0.f) {
+    if (!(a->l2_eps > 0.f) || d.gate != LETHE_GATE_CHANNEL || !a->q_norm != !a->k_norm) return kErrFlags;
+    if (a->q_norm && (!aligned16(a->q_norm) || !aligned16(a->k_norm))) return kErrAlign;
+    p->l2_eps = a->l2_eps;
+    p->keep_norm = a->q_norm ? 1 : 0;
+  }
   p->q = static_cast<const __nv_bfloat16*>(a->q);
   p->k = static_cast<const __nv_bfloat16*>(a->k);
   p->v = static_cast<const __nv_bfloat16*>(a->v);
@@ -150,7 +157,10 @@ extern "C" int lethe_gdn_forward(const LetheGdnArgs* a, void* stream) {
   const uint32_t m = a->kernel_mask ? a->kernel_mask : 7u;
   if ((m & 1u) && p.gate == LETHE_GATE_CHANNEL) {
     CUtensorMap mg;
-    if ((e = gate_map(&mg, a->g, p)) || (e = launch_prepare_cw(p, mq, mk, mv, mg, st))) return e;
+    NormMaps mn;
+    memset(&mn, 0, sizeof(mn));
+    if (p.keep_norm && ((e = token_map(&mn.q, a->q_norm, p, p.Kr)) || (e = token_map(&mn.k, a->k_norm, p, p.Kr)))) return e;
+    if ((e = gate_map(&mg, a->g, p)) || (e = launch_prepare_cw(p, mq, mk, mv, mg, mn, st))) return e;
   } else if ((m & 1u) && (e = launch_prepare(p, mq, mk, mv, st))) {
     return e;
   }

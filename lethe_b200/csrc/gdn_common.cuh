@@ -92,6 +92,8 @@ struct Problem {
   int lean;          // non-zero: intermediates that no later kernel of the call reads are not written
   int qk16;          // non-zero: q, k, dq, dk hold fp16 instead of bf16
   float scale;
+  float l2_eps;      // > 0: the channel-wise prepare kernel normalises q and k
+  int keep_norm;     // ... and stores the normalised rows
   const __nv_bfloat16 *q, *k, *v, *d_o;
   const float *g, *beta, *h0, *dhT;
   __nv_bfloat16 *o, *dq, *dk, *dv;

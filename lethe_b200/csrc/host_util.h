@@ -84,6 +84,7 @@ inline int make_tmap_f32(CUtensorMap* map, const void* ptr, int rank, const uint
   return r == CUDA_SUCCESS ? kOk : kErrDriver;
 }
 
+struct NormMaps { CUtensorMap q, k; };      // normalised rows of q and k on their way out
 // Tensor maps of the token-major gradient outputs that leave by tensor-map stores.
 struct OutMaps {
   CUtensorMap dq, dk, dv;

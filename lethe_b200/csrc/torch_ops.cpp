@@ -157,6 +157,7 @@ struct Problem {
 // What both directions hand to the library.
 struct Operands {
   Tensor q, k, v, g, beta, h0, b, w;      // q, k bf16 or fp16; v bf16; the rest fp32
+  bool raw = false;                       // q, k are still to be normalised, by the forward's first kernel
 };
 
 LetheGdnArgs base_args(const Problem& p, const Operands& x, void* saved, size_t saved_bytes) {
@@ -183,7 +184,8 @@ struct Forward {
   Workspace saved;
 };
 
-Forward run_forward(const Problem& p, Operands x) {
+// `keep`: a backward follows, which reads the normalised rows
+Forward run_forward(const Problem& p, Operands x, bool keep) {
   Forward f;
   const LetheGdnDims d = p.dims();
   const size_t need = lethe_gdn_saved_bytes(&d);
@@ -198,7 +200,22 @@ Forward run_forward(const Problem& p, Operands x) {
   LetheGdnArgs a = base_args(p, x, f.saved.start(), need);
   a.o = ptr(f.o);
   a.hT = ptr<float>(f.hT);
+  Tensor qn, kn;
+  if (x.raw) {
+    a.l2_eps = kL2Eps;
+    if (keep) {
+      qn = at::empty(x.q.sizes(), o16.dtype(at::kHalf));
+      kn = at::empty(x.k.sizes(), o16.dtype(at::kHalf));
+      a.q_norm = ptr(qn);
+      a.k_norm = ptr(kn);
+    }
+  }
   check(lethe_gdn_forward(&a, stream_of(x.q)));
+  if (qn.defined()) {
+    x.q = qn;
+    x.k = kn;
+    x.raw = false;
+  }
   f.x = std::move(x);
   return f;
 }
@@ -322,7 +339,7 @@ std::pair<Tensor, Tensor> apply(const Problem& p, const Tensor (&in)[kSlots], Op
   Forward f;
   {
     at::NoGradGuard no_grad;
-    f = run_forward(p, std::move(x));
+    f = run_forward(p, std::move(x), need);
     f.o = cast_back(f.o, in[kV].scalar_type());
   }
   if (need) {
@@ -369,10 +386,17 @@ Problem describe(const Tensor& q, const Tensor& k, const Tensor& v, double scale
 
 // q and k as the kernels read them: normalised rows in fp16 (rounded once from fp32), fp16 when both came as fp16,
 // bf16 otherwise
-void prepare_qk(const Problem& p, const Tensor& q, const Tensor& k, Operands* x) {
+// `fuse`: the channel-wise prepare kernel may normalise 16-bit rows itself
+void prepare_qk(const Problem& p, const Tensor& q, const Tensor& k, Operands* x, bool fuse = false) {
   if (p.l2) {
     Tensor qc, kc;
     const int flags = l2_inputs(q, k, &qc, &kc) | LETHE_L2_NORM_F16;
+    if (fuse && p.gate == LETHE_GATE_CHANNEL && !(flags & LETHE_L2_IN_F32)) {
+      x->q = qc;
+      x->k = kc;
+      x->raw = true;
+      return;
+    }
     x->q = at::empty(qc.sizes(), qc.options().dtype(at::kHalf));
     x->k = at::empty(kc.sizes(), kc.options().dtype(at::kHalf));
     check(lethe_gdn_l2norm_qk(qc.data_ptr(), kc.data_ptr(), x->q.data_ptr(), x->k.data_ptr(), qc.numel() / p.K,
@@ -409,7 +433,7 @@ std::pair<Tensor, Tensor> chunk(const Tensor& q, const Tensor& k, const Tensor& 
     Operands x;
     {
       at::NoGradGuard no_grad;
-      prepare_qk(p, q, k, &x);
+      prepare_qk(p, q, k, &x, true);
       x.v = as(v, at::kBFloat16);
       x.g = as_gate(g); x.beta = as32(beta); x.h0 = as32(h0);
     }
@@ -424,7 +448,7 @@ std::pair<Tensor, Tensor> full_with(Problem p, Operands x, const Tensor (&in)[kS
   p.delta = 2;
   {
     at::NoGradGuard no_grad;
-    if (!x.q.defined()) prepare_qk(p, in[kQ], in[kKey], &x);
+    if (!x.q.defined()) prepare_qk(p, in[kQ], in[kKey], &x, true);
     x.v = as(in[kV], at::kBFloat16);
     x.g = as_gate(in[kG]); x.b = as32(in[kB]); x.w = as32(in[kW]); x.h0 = as32(in[kH0]);
   }

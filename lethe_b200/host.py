@@ -173,9 +173,9 @@ class HostPipeline:
                 if self.pre_run is not None:
                     self.pre_run()
                 ops.forward_into(slot.buf, i["q"], i["k"], i["v"], i.get("g"), i.get("beta"), i.get("h0"), self.scale,
-                                 b_gate=i.get("b"), w_gate=i.get("w"))
+                                 b_gate=i.get("b"), w_gate=i.get("w"), lean=True)
                 ops.backward_into(slot.buf, i["q"], i["k"], i["v"], i.get("g"), i.get("beta"), i.get("h0"), i["do"],
-                                  i.get("dhT"), self.scale, b_gate=i.get("b"), w_gate=i.get("w"))
+                                  i.get("dhT"), self.scale, b_gate=i.get("b"), w_gate=i.get("w"), lean=True)
                 slot.computed.record(self.s_run)
             with torch.cuda.stream(self.s_out):
                 self.s_out.wait_event(slot.computed)

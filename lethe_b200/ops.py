@@ -48,6 +48,7 @@ class _Args(ctypes.Structure):
         ("c_begin", ctypes.c_uint32), ("c_count", ctypes.c_uint32),
         ("l_tokens", ctypes.c_uint32), ("k_channels", ctypes.c_uint32),
         ("lean", ctypes.c_uint32),
+        ("l2_eps", ctypes.c_float), ("q_norm", ctypes.c_void_p), ("k_norm", ctypes.c_void_p),
     ]
 
 

@@ -93,3 +93,24 @@ def test_gate_regime_sees_one_differing_channel(rows, K, V):
         t[0, -1, 0, -1] = torch.nextafter(last, torch.zeros_like(last))
         assert ops.gate_regime(g, b, w) == want
         t[0, -1, 0, -1] = last
+
+
+@pytest.mark.parametrize("K,V,L,H,dtype,delta", [(128, 128, 200, 150, torch.bfloat16, True), (64, 64, 130, 3, torch.float16, True),
+                                                 (128, 64, 64, 5, torch.bfloat16, False)])
+def test_rows_normalised_on_the_way_in(K, V, L, H, dtype, delta):
+    """Channel-wise gate: the prepare kernel normalises q and k itself; same op on rows normalised beforehand."""
+    dev = torch.device("cuda")
+    inp = make_inputs(1, L, H, K, V, gate="channel", delta=delta, seed=12, mild=True)
+    d = {n: (None if inp[n] is None else inp[n].to(dev)) for n in ("v", "g", "beta", "h0", "do")}
+    q, k = ((3 * inp[n]).to(dev, dtype).requires_grad_(True) for n in ("q", "k"))
+    rest = (d["v"], d["g"], d["beta"], d["h0"])
+    o, hT = ops.gdn_chunk(q, k, *rest, use_qk_l2norm=True)
+    o_ref, hT_ref = ops.gdn_chunk(*ops.l2norm_qk(q, k), *rest)
+    with torch.no_grad():
+        o_eval, hT_eval = ops.gdn_chunk(q, k, *rest, use_qk_l2norm=True)
+    assert torch.equal(o, o_eval) and torch.equal(hT, hT_eval)
+    got, ref = (torch.autograd.grad(x, (q, k), d["do"]) for x in (o, o_ref))
+    errs = {"o": scale_rel(o.detach().double(), o_ref.detach().double()), "hT": scale_rel(hT.detach().double(), hT_ref.detach().double()),
+            "dq": scale_rel(got[0].double(), ref[0].double()), "dk": scale_rel(got[1].double(), ref[1].double())}
+    report(f"normalised on the way in K={K} V={V} {dtype}", errs)
+    assert max(errs.values()) <= TOL, errs
