@@ -768,9 +768,9 @@ def main():
     if rank == 0:
         hbm, tf_burst, tf_sustained, which = peaks()
         Z, BH = B * H * (L // 64), B * H
-        # the roofline kernel is named, not picked by max() over noisy timings: the forward's prepare kernel is
-        # the longest single launch of the delta-rule variants, Stage B of the variants without the delta term
-        top = "prepare" if delta else "stageb"
+        # the roofline kernel is named, not picked by max() over noisy timings: the backward's main kernel is the
+        # longest launch of every variant
+        top = "main"
         total_b = algorithmic_bytes(top, Z, BH, V, delta, gate == "channel")
         ab = io_bytes(top, Z, V, delta, gate)
         achieved = ab / (kern[top] * 1e-3) / 1e9

@@ -1,15 +1,15 @@
 // Shared definitions of the GDN kernels: problem description, workspace layout, small device helpers.
 //
 // Work decomposition.  A "chunk" is 64 consecutive tokens of one (batch, head) pair; chunks are
-// numbered z = (b*H + h)*NT + c.  Chunk-parallel kernels run one CTA (128 or 256 threads) per chunk;
-// the scan kernel runs one CTA per (b, h, 16-column slice of V) and walks the chunks in order.
+// numbered z = (b*H + h)*NT + c.  Chunk-parallel kernels run persistent CTAs, one chunk at a time;
+// the scan kernel runs one CTA per (b, h, slice of 16 or 64 columns of V) and walks the chunks in order.
 //
 // Per-chunk records in the workspaces ("image" = the SW128 shared-memory tile image, so that a
 // record moves between global and shared memory with one contiguous bulk copy):
 //   saved (forward -> backward)
 //     TA    16 KB   image, 128 rows x 64: rows 0-63 T = (I + strict_lower(M))^-1, rows 64-127 A
 //     W     16 KB   image, 64 x 128: WY factor w = T (beta gamma k)
-//     U     64 x V  image: u = T (beta v)
+//     U     64 x V  image: u = T (beta v)             (no delta term: v itself, left out of a lean call, as is VN)
 //     P     32 KB   image, 128 x 128: kd^T w           (state transition, without the decay)
 //     R     128 x V fp16 row-major: kd^T u            (state input)
 //     Hc    128 x V image: state entering the chunk; NT + 1 records per (b, h), the last one being
@@ -115,22 +115,8 @@ struct Problem {
 // ---------------------------------------------------------------------------------------------
 // device helpers
 // ---------------------------------------------------------------------------------------------
-// Inclusive prefix sum of one value per thread over threads 0..63 (two warps); every thread of the
-// CTA must call it (it contains __syncthreads).  `tmp` is a shared float[2].
-__device__ __forceinline__ float chunk_cumsum(float x, int tid, float* tmp) {
-  const int lane = tid & 31;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const float y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  if (tid == 31) tmp[0] = x;
-  __syncthreads();
-  if (tid >= 32 && tid < 64) x += tmp[0];
-  return x;
-}
-
-// Inclusive suffix sum over threads 0..63 (x_t + x_{t+1} + ... + x_63), same calling rules.
+// Inclusive suffix sum of one value per thread over threads 0..63 (x_t + x_{t+1} + ... + x_63; two warps); every thread of
+// the CTA must call it (it contains __syncthreads).  `tmp` is a shared float[2].
 __device__ __forceinline__ float chunk_rev_cumsum(float x, int tid, float* tmp) {
   const int lane = tid & 31;
 #pragma unroll
@@ -158,9 +144,8 @@ struct CtaShared {
 // pointer arithmetic on the shared symbol, so the compiler keeps the shared address space and emits
 // shared-memory loads and stores; `align1024_generic` goes through an integer, after which every
 // access is a generic one.  Same addresses, different instruction selection and scheduling: the
-// channel-wise kernels run 10-15 % faster with the first, the scalar kernels 3-5 % except the prepare
-// kernel without the delta term, which is 10 % faster with the second, as are the scans by 1-3 %
-// (measured per kernel on a B200), so each kernel names the one it wants.
+// channel-wise kernels run 10-15 % faster with the first, the scalar kernels 3-6 %, the scans 1-3 % faster with
+// the second (measured per kernel on a B200), so each kernel names the one it wants.
 __device__ __forceinline__ unsigned char* align1024_s_(unsigned char* p) {
   const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(p));
   return p + ((1024u - (a & 1023u)) & 1023u);
@@ -263,26 +248,6 @@ __device__ __forceinline__ void warp_scaled_gammas(const Problem& p, int b, int 
     if (lane >= w) sum += y;
   }
   *reinterpret_cast<float2*>(out + 2 * lane) = make_float2(p.scale * __expf(sum - g[1]), p.scale * __expf(sum));
-}
-
-// Deterministic sum over the 128 threads of a CTA (fixed tree).  `red` is a shared float[4].
-__device__ __forceinline__ float cta_sum128(float x, int tid, float* red) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-  __syncthreads();
-  if ((tid & 31) == 0) red[tid >> 5] = x;
-  __syncthreads();
-  return (red[0] + red[1]) + (red[2] + red[3]);
-}
-
-// The same over 256 threads.  `red` is a shared float[8].
-__device__ __forceinline__ float cta_sum256(float x, int tid, float* red) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-  __syncthreads();
-  if ((tid & 31) == 0) red[tid >> 5] = x;
-  __syncthreads();
-  return ((red[0] + red[1]) + (red[2] + red[3])) + ((red[4] + red[5]) + (red[6] + red[7]));
 }
 
 }  // namespace lg
