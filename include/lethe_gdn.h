@@ -118,8 +118,9 @@ typedef struct LetheGdnArgs {
   /* states [B, H, k_channels, V]).  The rest counts as zero and is neither read nor written.  0: all of dims.     */
   uint32_t l_tokens;
   uint32_t k_channels;
-  /* Non-zero: the call leaves only results in memory, and in the workspaces what its own later kernels and, after a   */
-  /* forward, the backward read.  Zero: also intermediates that a caller may want to look at (dv2, dw).                */
+  /* 1: the call leaves only results in memory, and in the workspaces what its own later kernels and, after a forward, */
+  /* the backward read.  2 (forward only): not even the latter, no backward can follow.  0: also intermediates that a  */
+  /* caller may want to look at (dv2, dw).                                                                             */
   uint32_t lean;
   /* Forward, LETHE_GATE_CHANNEL only.  l2_eps > 0: q and k are normalised as they are read, x rsqrt(sum x^2 + l2_eps)   */
   /* per token-head, in fp32 and rounded once to fp16 (what lethe_gdn_l2norm_qk does, without its pass over memory);    */

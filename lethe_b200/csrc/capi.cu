@@ -101,7 +101,8 @@ static int fill_problem(const LetheGdnArgs* a, Problem* p, bool backward) {
   }
   p->scale = a->scale;
   p->qk16 = a->qk_f16 ? 1 : 0;
-  p->lean = a->lean ? 1 : 0;
+  p->lean = a->lean;
+  if (p->lean > 2u || (backward && p->lean == 2u)) return kErrFlags;
   if (!backward && a->l2_eps != 0.f) {
     if (!(a->l2_eps > 0.f) || d.gate != LETHE_GATE_CHANNEL || !a->q_norm != !a->k_norm) return kErrFlags;
     if (a->q_norm && (!aligned16(a->q_norm) || !aligned16(a->k_norm))) return kErrAlign;

@@ -89,7 +89,7 @@ struct Problem {
   int Kr;            // key channels of the user tensors (64 or 128); the kernels work on 128, missing ones are zero
   int bh0, nbh;      // the (batch, head) pairs this call works on: [bh0, bh0 + nbh) of the B * H pairs
   int c0, cn;        // the chunks of every pair this call works on: [c0, c0 + cn) of the NT chunks
-  int lean;          // non-zero: intermediates that no later kernel of the call reads are not written
+  uint32_t lean;     // 1: intermediates that no later kernel of the call reads are not written; 2: nor what only a backward reads
   int qk16;          // non-zero: q, k, dq, dk hold fp16 instead of bf16
   float scale;
   float l2_eps;      // > 0: the channel-wise prepare kernel normalises q and k

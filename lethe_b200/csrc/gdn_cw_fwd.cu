@@ -477,7 +477,8 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
         issue_product_led(leader, cWU + 128, Tile{smem_u32(TA), 128, false}, Tile{smem_u32(BV), 64, true}, V, 64, 0u);
         umma_commit_led(leader, m2);
         if (tid == 0) {
-          bulk_s2g(p.saved + p.lay.ta + static_cast<size_t>(a.z) * p.lay.sz_ta, TA, 16384);
+          if (p.lean < 2) bulk_s2g(p.saved + p.lay.ta + static_cast<size_t>(a.z) * p.lay.sz_ta, TA, 16384);
+          else bulk_s2g(p.saved + p.lay.ta + static_cast<size_t>(a.z) * p.lay.sz_ta + 8192, TA + 8192, 8192);      // A only
           bulk_commit();
         }
       }

@@ -243,7 +243,8 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
       issue_product_led(leader, tmem + 128, Tile{smem_u32(W), 128, false}, Tile{smem_u32(Vt), 64, true}, V, 64, 0u);
       umma_commit_led(leader, mma);
       if (tid == 0) {
-        bulk_s2g(p.saved + p.lay.ta + static_cast<size_t>(a.z) * p.lay.sz_ta, TA, 16384);
+        if (p.lean < 2) bulk_s2g(p.saved + p.lay.ta + static_cast<size_t>(a.z) * p.lay.sz_ta, TA, 16384);
+        else bulk_s2g(p.saved + p.lay.ta + static_cast<size_t>(a.z) * p.lay.sz_ta + 8192, TA + 8192, 8192);      // A only
         bulk_commit();
       }
       __syncwarp();
@@ -645,7 +646,7 @@ output_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     __syncthreads();
     if (tid == 0) {
       for (int i = 0; i < V / 64; ++i) tma_store_4d(&mo, WQ + i * 16384, i * 64, a.h, a.c * kC, a.b);
-      if (DELTA || !p.lean) bulk_s2g(p.saved + p.lay.vn + static_cast<size_t>(a.z) * p.lay.sz_vn, VN, V * 128);
+      if (DELTA ? p.lean < 2 : !p.lean) bulk_s2g(p.saved + p.lay.vn + static_cast<size_t>(a.z) * p.lay.sz_vn, VN, V * 128);
       bulk_commit();
       if (S::kStages == 1 && n + static_cast<int>(gridDim.x) < nchunks) {
         bulk_wait_read();

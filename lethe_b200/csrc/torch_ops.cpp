@@ -200,6 +200,7 @@ Forward run_forward(const Problem& p, Operands x, bool keep) {
   LetheGdnArgs a = base_args(p, x, f.saved.start(), need);
   a.o = ptr(f.o);
   a.hT = ptr<float>(f.hT);
+  if (!keep) a.lean = 2u;
   Tensor qn, kn;
   if (x.raw) {
     a.l2_eps = kL2Eps;
