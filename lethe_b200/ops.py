@@ -192,7 +192,7 @@ class GdnStepGraph:
 
     A training step at fixed shapes calls the library with the same pointers every time; replaying the
     captured kernels removes the launch gaps between them.  Two ways to fill the SMs the serial state scans
-    leave idle (a scan occupies V / 16 CTAs per (batch, head) pair, V / 32 for very many pairs), both bitwise
+    leave idle (a scan occupies V / 16 CTAs per (batch, head) pair, V / 64 for many pairs), both bitwise
     equal to the plain chain:
 
     ``pipeline`` (default): only the serial chain of the step - prepare, forward scan, adjoint scan, Stage B
