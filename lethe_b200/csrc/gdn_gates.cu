@@ -74,8 +74,10 @@ gate_regime_kernel(const RegimeProblem p) {
     if (atomicAdd(p.work + 1, 1u) == gridDim.x - 1) {
       const uint32_t failed = atomicExch(p.work, 0u);
       p.work[1] = 0u;
-      *reinterpret_cast<volatile uint32_t*>(p.flags) = LETHE_REGIME_DONE | (~failed & 7u);
+      // Whoever sees the word may hand `work` to a kernel on another stream at once, which nothing but this fence orders
+      // behind the two stores that clear it.
       __threadfence_system();
+      *reinterpret_cast<volatile uint32_t*>(p.flags) = LETHE_REGIME_DONE | (~failed & 7u);
     }
   }
 }
