@@ -483,6 +483,7 @@ struct RegimeSlot {
 struct RegimePool {
   std::mutex mu;
   std::vector<RegimeSlot> free[kMaxDevices];
+  int made = 0;
   RegimeSlot take(int dev) {
     {
       std::lock_guard<std::mutex> lock(mu);
@@ -495,15 +496,26 @@ struct RegimePool {
     RegimeSlot s;
     void *h = nullptr, *d = nullptr;
     if (cudaHostAlloc(&h, 64, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess ||
-        cudaMalloc(&d, 8) != cudaSuccess || cudaMemset(d, 0, 8) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess)
+        cudaMalloc(&d, 8) != cudaSuccess || cudaMemset(d, 0, 8) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
+      cudaFree(d);
+      cudaFreeHost(h);
       fail("no memory for the gate test");
+    }
     s.word = static_cast<volatile uint32_t*>(h);
     s.work = static_cast<uint32_t*>(d);
+    std::lock_guard<std::mutex> lock(mu);
+    ++made;
     return s;
   }
   void give(int dev, RegimeSlot s) {
     std::lock_guard<std::mutex> lock(mu);
     free[dev].push_back(s);
+  }
+  std::pair<int, int> count() {      // slots made, slots free
+    std::lock_guard<std::mutex> lock(mu);
+    size_t n = 0;
+    for (const auto& f : free) n += f.size();
+    return {made, static_cast<int>(n)};
   }
 };
 RegimePool& regime_pool() {
@@ -511,11 +523,13 @@ RegimePool& regime_pool() {
   return *pool;
 }
 
-// The gate test of one call: enqueue, then wait.
+// The gate test of one call: enqueue, then wait.  A call that fails in between waits as well: the slot goes back when the
+// kernel that uses it is done.
 struct RegimeTest {
   int dev;
   cudaStream_t st;
   RegimeSlot slot;
+  bool pending = false;
   Tensor g0, b0;
   RegimeTest(const Tensor& g, const Tensor& b, const Tensor& w) : dev(g.device().index()), st(stream_of(g)) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -525,12 +539,27 @@ struct RegimeTest {
     b0 = at::empty_like(g0);
     slot = regime_pool().take(dev);
     *slot.word = 0;
-    check(lethe_gdn_gate_regime(ptr<float>(g), ptr<float>(b), ptr<float>(w), g0.numel(), static_cast<int32_t>(g.size(3)),
-                                static_cast<int32_t>(w.size(3)), ptr<float>(g0), ptr<float>(b0),
-                                const_cast<uint32_t*>(slot.word), slot.work, st));
+    const int rc = lethe_gdn_gate_regime(ptr<float>(g), ptr<float>(b), ptr<float>(w), g0.numel(), static_cast<int32_t>(g.size(3)),
+                                         static_cast<int32_t>(w.size(3)), ptr<float>(g0), ptr<float>(b0),
+                                         const_cast<uint32_t*>(slot.word), slot.work, st);
+    if (rc != 0) regime_pool().give(dev, slot);      // nothing was launched
+    check(rc);
+    pending = true;
+  }
+  ~RegimeTest() {
+    if (pending) finish();
   }
   uint32_t wait() {
+    const uint32_t v = finish();
+    if (!(v & LETHE_REGIME_DONE)) fail("the gate test did not complete");
+    return v;
+  }
+
+ private:
+  // the verdict, or 0 after a failed kernel, whose slot is not used again
+  uint32_t finish() {
     uint32_t v = 0;
+    pending = false;
     {
       pybind11::gil_scoped_release nogil;
       for (uint32_t n = 1; !((v = *slot.word) & LETHE_REGIME_DONE); ++n) {
@@ -542,8 +571,7 @@ struct RegimeTest {
         break;
       }
     }
-    if (!(v & LETHE_REGIME_DONE)) fail("the gate test did not complete");    // (the slot is not reused)
-    regime_pool().give(dev, slot);
+    if (v & LETHE_REGIME_DONE) regime_pool().give(dev, slot);
     return v;
   }
 };
@@ -659,5 +687,6 @@ PYBIND11_MODULE(lethe_gdn_torch, m) {
   m.def("chunk_full", &chunk_full);
   m.def("six_inputs", &six_inputs);
   m.def("gate_regime", &gate_regime);
+  m.def("gate_test_slots", [] { return regime_pool().count(); });
   m.def("decode_step", &decode_step);
 }
