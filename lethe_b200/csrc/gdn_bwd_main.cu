@@ -116,16 +116,18 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
   };
   // loads of a chunk (tid 0), by when their destinations fall free in the chunk before
   constexpr uint32_t kIn0 = 32768u + (WY ? V * 128u : 0u) + (DELTA ? 16384u : 8192u) + (SB ? 2u * V * 128 + V * 256 : V * 128u);
-  auto load_a = [&](const At& a) {                // do, v_new, v, h (dv2 where the first half of the call left it)
+  auto load_a = [&](const At& a) {                // do, v
     mbar_expect_tx(&bars->in0, kIn0);
     for (int t = 0; t < V / 64; ++t) {
       if (SB) {
         tma_load_4d(tDO + t * 8192, &mdo, &bars->in0, t * 64, a.h, a.c * kC, a.b);
-        if (DELTA) bulk_g2s(tVN + t * 8192, p.saved + p.lay.vn + static_cast<size_t>(a.z) * p.lay.sz_vn + t * 8192, 8192, &bars->in0);
-        else tma_load_4d(tVN + t * 8192, &mv, &bars->in0, t * 64, a.h, a.c * kC, a.b);      // v_new is v
+        if (!DELTA) tma_load_4d(tVN + t * 8192, &mv, &bars->in0, t * 64, a.h, a.c * kC, a.b);      // v_new is v
       }
       if (WY) tma_load_4d(tV + t * 8192, &mv, &bars->in0, t * 64, a.h, a.c * kC, a.b);
     }
+  };
+  auto load_rec = [&](const At& a) {              // v_new, h (dv2 where the first half of the call left it)
+    if (SB && DELTA) bulk_g2s(tVN, p.saved + p.lay.vn + static_cast<size_t>(a.z) * p.lay.sz_vn, V * 128, &bars->in0);
     if (SB) bulk_g2s(tH, p.saved + p.lay.hc + static_cast<size_t>(a.z + a.bh) * p.lay.sz_hc, V * 256, &bars->in0);
     else bulk_g2s(tDV, p.scratch + p.lay.dv2 + static_cast<size_t>(a.z) * p.lay.sz_dv2, V * 128, &bars->in0);
   };
@@ -149,7 +151,9 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     mbar_init(&bars->m3, 1); mbar_init(&bars->mV, 1); mbar_init(&bars->m4, 1); mbar_init(&bars->m5, 1); mbar_init(&bars->m6, 1);
     fence_mbar_init();
     fence_proxy_async();
-    if (SB) {                  // everything but dh, which the adjoint scan just before this kernel writes, is older
+    // Older than whatever kernel of the path comes just before this one: the caller's tensors and [T; A].  Not dh (the adjoint
+    // scan), v_new (the output kernel) and h (the forward scan): which of the three ran last is up to the caller.
+    if (SB) {
       const At a = at(blockIdx.x);
       load_a(a);
       load_b(a);
@@ -199,13 +203,13 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
   griddep_wait();
   griddep_launch();
   if (tid == 0) {
-    if (SB) {
-      load_dh(a);
-    } else {
+    if (!SB) {
       load_a(a);
       load_b(a);
       load_q(a);
     }
+    load_rec(a);
+    if (SB) load_dh(a);
   }
 
   uint32_t ph = 0;
@@ -447,6 +451,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       if (tid == 0 && more) {
         bulk_wait_read();
         load_a(nx);
+        load_rec(nx);
         load_dh(nx);
         load_b(nx);
       }
@@ -604,6 +609,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       if (tid == 0 && more) {          // dq and dv have left by now; h / dw, dv2 and X are read
         bulk_wait_read();
         load_a(nx);
+        load_rec(nx);
         if (SB) load_dh(nx);
       }
     }

@@ -252,10 +252,10 @@ scan_nodelta_kernel(const Problem p) {
   const int bh = blockIdx.y + p.bh0, V = p.V, NT = p.NT, n = p.cn;
   const bool seg_first = ADJOINT ? (p.c0 + p.cn == NT) : (p.c0 == 0);        // chunk ranges as in scan_kernel
   const bool seg_last = ADJOINT ? (p.c0 == 0) : (p.c0 + p.cn == NT);
-  float* carry = reinterpret_cast<float*>(ADJOINT ? p.scratch + p.lay.carry_b : p.saved + p.lay.carry_f);
   const int col0 = atom * 64 + c8 * 8;
   griddep_wait();
   griddep_launch();
+  float* carry = reinterpret_cast<float*>(ADJOINT ? p.scratch + p.lay.carry_b : p.saved + p.lay.carry_f);
   const unsigned char* Rg = ADJOINT ? p.scratch + p.lay.rb : p.saved + p.lay.r;
   const float* ADg = reinterpret_cast<const float*>(p.saved + p.lay.ad);
   unsigned char* Xg = ADJOINT ? p.scratch + p.lay.dh : p.saved + p.lay.hc;

@@ -85,11 +85,15 @@ __device__ __forceinline__ void mbar_wait_warp(uint64_t* bar, uint32_t parity, c
 
 // ---------------------------------------------------------------------------------------------
 // Programmatic dependent launch.  A kernel launched with the attribute may start while the kernel
-// before it in the stream is still running; `griddep_wait` blocks until that kernel has completed and
-// its writes are visible (a no-op for a plain launch), `griddep_launch` lets the next kernel of the
-// stream start its own prologue.  Every kernel here triggers only after its own wait, so when a
-// kernel starts, everything older than its immediate predecessor is complete: before the wait it
-// may read anything except what the immediate predecessor writes.
+// before it in the stream (in a captured graph: any kernel it depends on, through events too) is still
+// running; `griddep_wait` blocks until those kernels have completed and their writes are visible (a
+// no-op for a plain launch), `griddep_launch` lets the next kernel start its own prologue.  Every
+// kernel here triggers only after its own wait, so when a kernel starts, everything older than its
+// immediate predecessors is complete: before the wait it may read anything except what those write.
+// Calls can be cut into kernels and ranges of chunks, so which kernels these are depends on the
+// caller.  The kernels therefore read, before they wait, only the caller's tensors and records of
+// prepare, behind which another kernel of the same chunks always comes first (prepare, scan, output;
+// prepare, scan input, adjoint scan, main).
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -264,9 +264,11 @@ class GdnStepGraph:
             # `other` prepares the later segment and builds the adjoint scan's input while the forward scan
             # runs, computes the outputs behind the scan, and runs Stage B / WY of the later segment under the
             # adjoint scan of the first; `third` computes the output of the last segment while the adjoint scan
-            # has already started.  Stream order is chosen so that no kernel launched with the
-            # programmatic-dependency attribute follows, on its own stream, the kernel whose result it loads
-            # before its wait (Stage B loads v_new early: it never follows an output kernel of its own segment).
+            # has already started.  Every edge into a kernel with the programmatic-dependency attribute, the ones
+            # from events too, is a programmatic one in the captured graph: such a kernel may start while the ones
+            # it depends on still run, and waits for them itself.  Until then it reads the caller's tensors and
+            # records of prepare only (the adjoint scan: P), and whatever the cuts, a kernel that has waited for
+            # prepare lies in between (tests/test_launch_order_cpu.py goes through the schedule).
             other, third = self._streams[0], self._streams[1]
             segs = [(0, self.cut), (self.cut, NT - self.cut)] if self.segments == 2 else [(0, NT)]
             S = len(segs)

@@ -117,6 +117,36 @@ def test_chunk_ranges_and_the_pipelined_graph_give_the_same_bits(gate, delta, V)
         ops.forward_into(part, *args, sc, c_range=(NT - 1, 2))          # beyond the last chunk
 
 
+@pytest.mark.parametrize("gate,delta,V", [("scalar", True, 64), ("scalar", True, 128), ("channel", True, 128), ("scalar", False, 64),
+                                          ("channel", False, 128)])
+def test_the_main_kernel_may_follow_any_kernel_of_the_forward(gate, delta, V):
+    """Kernels picked one by one, the adjoint scan ahead of the forward's: the backward's main kernel then comes right
+    behind the output kernel, whose v_new it reads (without the delta term: behind the forward scan, whose states)."""
+    B, L, H, K = 2, 4096, 3, 128
+    dev = torch.device("cuda")
+    code = {"scalar": ops.GATE_SCALAR, "channel": ops.GATE_CHANNEL}[gate]
+    inp = make_inputs(B, L, H, K, V, gate=gate, delta=delta, seed=12)
+    d = {n: (None if t is None else t.to(dev)) for n, t in inp.items()}
+    args = (d["q"], d["k"], d["v"], d["g"], d["beta"], d["h0"])
+    sc = K ** -0.5
+    ref = ops.GdnBuffers(B, L, H, K, V, code, delta, dev)
+    ops.forward_into(ref, *args, sc)
+    ops.backward_into(ref, *args, d["do"], None, sc)
+    buf = ops.GdnBuffers(B, L, H, K, V, code, delta, dev)
+    buf.saved.fill_(0x7f), buf.scratch.fill_(0x7f)               # (fp16 0x7f7f is a NaN)
+    ops.forward_into(buf, *args, sc, 1)
+    ops.backward_into(buf, *args, d["do"], None, sc, 1)
+    ops.backward_into(buf, *args, d["do"], None, sc, 2)
+    ops.forward_into(buf, *args, sc, 2)
+    if delta:
+        ops.forward_into(buf, *args, sc, 4)
+    ops.backward_into(buf, *args, d["do"], None, sc, 12)
+    torch.cuda.synchronize()
+    ops.check_status(buf.status)
+    for n in ["dq", "dk", "dv", "dg", "dh0"] + (["dbeta"] if delta else []):
+        assert torch.equal(getattr(buf, n), getattr(ref, n)), n
+
+
 @pytest.mark.parametrize("gate,V,B,L,H", [("scalar", 64, 2, 2048, 8), ("channel", 128, 2, 2048, 8), ("scalar", 128, 4, 4096, 16)])
 def test_step_graph_at_benchmark_shapes_equals_the_plain_chain_on_every_replay(gate, V, B, L, H):
     """The overlapped schedule at the shapes the benchmark times (the default cut, full grids, every stream of
