@@ -687,6 +687,10 @@ PYBIND11_MODULE(lethe_gdn_torch, m) {
   m.def("chunk_full", &chunk_full);
   m.def("six_inputs", &six_inputs);
   m.def("gate_regime", &gate_regime);
+  m.def("status_address", [](int dev) {      // of a GPU's status word, for tests of what an expired wait leads to
+    TORCH_CHECK(dev >= 0 && dev < kMaxDevices);
+    return reinterpret_cast<uintptr_t>(host_words().status + dev);
+  });
   m.def("gate_test_slots", [] { return regime_pool().count(); });
   m.def("decode_step", &decode_step);
 }
