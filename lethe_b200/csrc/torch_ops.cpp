@@ -36,11 +36,11 @@ constexpr int kMaxDevices = 64;
 // ---------------------------------------------------------------------------------------------
 PyObject* g_error_type = nullptr;
 
-[[noreturn]] void fail(const std::string& msg) {
+[[noreturn]] void fail(const std::string& msg, PyObject* type = g_error_type) {
   python_error e;
   {
     pybind11::gil_scoped_acquire gil;
-    PyErr_SetString(g_error_type ? g_error_type : PyExc_RuntimeError, ("lethe_gdn: " + msg).c_str());
+    PyErr_SetString(type ? type : PyExc_RuntimeError, ("lethe_gdn: " + msg).c_str());
     e.persist();
   }
   throw e;
@@ -334,6 +334,9 @@ struct GdnBackward : public torch::autograd::Node {
 
 // Runs the forward and, when something asks for gradients, hangs the node on the results.
 std::pair<Tensor, Tensor> apply(const Problem& p, const Tensor (&in)[kSlots], Operands x, bool six) {
+  for (const Tensor& t : in)      // (the kernels would return the value without its tangent)
+    if (t.defined() && t._fw_grad(/*level=*/0).defined())
+      fail("forward-mode differentiation is not implemented", PyExc_NotImplementedError);
   bool need = false;
   if (torch::autograd::GradMode::is_enabled())
     for (const Tensor& t : in) need = need || (t.defined() && t.requires_grad());

@@ -1,0 +1,43 @@
+"""GPU: the differentiable ops under what PyTorch wraps around an autograd function."""
+import pytest
+import torch
+import torch.autograd.forward_ad as fwd_ad
+
+from lethe_b200 import ops
+from lethe_b200.synth import make_inputs
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(L=128, V=64, seed=6):
+    inp = make_inputs(1, L, 2, 128, V, gate="channel", delta=True, seed=seed)
+    d = {n: (None if t is None else t.cuda()) for n, t in inp.items()}
+    d["b"] = d["beta"][..., None].expand(1, L, 2, 128).contiguous()
+    d["w"] = d["beta"][..., None].expand(1, L, 2, V).contiguous()
+    d["bf"], d["wf"] = d["b"] * torch.rand_like(d["b"]), d["w"] * torch.rand_like(d["w"])
+    return d
+
+
+# name: (op on its tensors, their names)
+OPS = {
+    "gdn_chunk": (lambda *t, **kw: ops.gdn_chunk(*t, **kw)[0], ("q", "k", "v", "g", "beta", "h0")),
+    "gdn_chunk_full": (lambda *t, **kw: ops.gdn_chunk_full(*t, **kw)[0], ("q", "k", "v", "g", "bf", "wf", "h0")),
+    "gdn2_op": (ops.gdn2_op, ("q", "k", "v", "g", "b", "w")),
+    "gdn2_op, independent gates": (ops.gdn2_op, ("q", "k", "v", "g", "bf", "wf")),
+}
+every_op = pytest.mark.parametrize("name", sorted(OPS))
+
+
+@every_op
+def test_forward_mode_is_refused(name):
+    """There is no forward-mode rule: an input with a tangent is refused, not answered without one."""
+    op, names = OPS[name]
+    d = _inputs()
+    for dual in names:
+        with fwd_ad.dual_level():
+            args = [fwd_ad.make_dual(d[n], torch.ones_like(d[n])) if n == dual else d[n] for n in names]
+            with pytest.raises(NotImplementedError, match="forward-mode"):
+                op(*args)
+            with torch.no_grad(), pytest.raises(NotImplementedError, match="forward-mode"):
+                op(*args)
+    op(*[d[n] for n in names])
