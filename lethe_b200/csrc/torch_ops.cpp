@@ -108,17 +108,17 @@ Tensor cast_back(const Tensor& t, at::ScalarType dt) { return t.scalar_type() ==
 template <typename T = void>
 T* ptr(const Tensor& t) { return t.defined() ? static_cast<T*>(t.data_ptr()) : nullptr; }
 
-// Byte buffer for a workspace; the library wants its start on a 1024-byte boundary.
-struct Workspace {
-  Tensor raw;
-  size_t bytes = 0;
-  void* start() const {
-    const uintptr_t a = reinterpret_cast<uintptr_t>(raw.data_ptr());
-    return reinterpret_cast<void*>((a + 1023) & ~static_cast<uintptr_t>(1023));
-  }
-};
-Workspace workspace(size_t bytes, const at::TensorOptions& o) {
-  return {at::empty({static_cast<int64_t>(bytes + 1024)}, o.dtype(at::kByte)), bytes};
+// Byte buffer for a workspace.  The library wants its start on a 1024-byte boundary, the allocator gives 512: the tensor
+// is cut to the part that begins there.
+constexpr int64_t kWorkspaceAlign = 1024;
+bool workspace_aligned(const Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % kWorkspaceAlign == 0; }
+Tensor workspace(size_t bytes, const at::TensorOptions& o) {
+  const int64_t n = static_cast<int64_t>(bytes);
+  Tensor t = at::empty({n + kWorkspaceAlign}, o.dtype(at::kByte));
+  const auto past = static_cast<int64_t>(reinterpret_cast<uintptr_t>(t.data_ptr()) % kWorkspaceAlign);
+  t.unsafeGetTensorImpl()->set_storage_offset(past ? kWorkspaceAlign - past : 0);
+  t.unsafeGetTensorImpl()->set_sizes_contiguous({n});
+  return t;
 }
 
 // q and k as the normalisation kernels read them: as they are when both are bf16, fp32 or fp16, else both as fp32.
@@ -181,7 +181,7 @@ LetheGdnArgs base_args(const Problem& p, const Operands& x, void* saved, size_t 
 struct Forward {
   Tensor o, hT;
   Operands x;
-  Workspace saved;
+  Tensor saved;
 };
 
 // `keep`: a backward follows, which reads the normalised rows
@@ -197,7 +197,7 @@ Forward run_forward(const Problem& p, Operands x, bool keep) {
   f.saved = workspace(need, o16);
   f.o = at::empty({p.B, p.L, p.H, p.V}, o16);
   f.hT = at::empty({p.B, p.H, p.K, p.V}, o32);
-  LetheGdnArgs a = base_args(p, x, f.saved.start(), need);
+  LetheGdnArgs a = base_args(p, x, f.saved.data_ptr(), need);
   a.o = ptr(f.o);
   a.hT = ptr<float>(f.hT);
   if (!keep) a.lean = 2u;
@@ -225,19 +225,19 @@ struct Grads {
   Tensor dq, dk, dv, dg, dbeta, dbeta_w, dh0, db, dw;
 };
 
-Grads run_backward(const Problem& p, const Operands& x, const Workspace& saved, const Tensor& d_o, const Tensor& dhT,
+Grads run_backward(const Problem& p, const Operands& x, const Tensor& saved, const Tensor& d_o, const Tensor& dhT,
                    bool split_beta) {
   Grads r;
   const LetheGdnDims d = p.dims();
   const auto o16 = x.v.options();
   const auto o32 = o16.dtype(at::kFloat);
-  const Workspace scratch = workspace(lethe_gdn_scratch_bytes(&d), o16);
+  const Tensor scratch = workspace(lethe_gdn_scratch_bytes(&d), o16);
   r.dq = at::empty_like(x.q);
   r.dk = at::empty_like(x.k);
   r.dv = at::empty_like(x.v);
   if (x.g.defined()) r.dg = at::empty_like(x.g);
   if (x.h0.defined()) r.dh0 = at::empty_like(x.h0);
-  LetheGdnArgs a = base_args(p, x, saved.start(), saved.bytes);
+  LetheGdnArgs a = base_args(p, x, saved.data_ptr(), static_cast<size_t>(saved.numel()));
   if (p.delta == 2) {
     r.db = at::empty_like(x.b);
     r.dw = at::empty_like(x.w);
@@ -249,8 +249,8 @@ Grads run_backward(const Problem& p, const Operands& x, const Workspace& saved, 
   a.dq = ptr(r.dq); a.dk = ptr(r.dk); a.dv = ptr(r.dv); a.dg = ptr<float>(r.dg); a.dh0 = ptr<float>(r.dh0);
   a.dbeta = ptr<float>(r.dbeta); a.dbeta_write = ptr<float>(r.dbeta_w);
   a.db_gate = ptr<float>(r.db); a.dw_gate = ptr<float>(r.dw);
-  a.scratch = scratch.start();
-  a.scratch_bytes = scratch.bytes;
+  a.scratch = scratch.data_ptr();
+  a.scratch_bytes = static_cast<size_t>(scratch.numel());
   check(lethe_gdn_backward(&a, stream_of(x.q)));
   return r;
 }
@@ -261,14 +261,13 @@ struct GdnBackward : public torch::autograd::Node {
   bool six = false;                        // gates came per channel: gradients go back per channel
   torch::autograd::SavedVariable q_in, k_in;            // inputs of the normalisation
   torch::autograd::SavedVariable q, k, v, g, beta, h0, b, w;
-  Workspace saved;
+  torch::autograd::SavedVariable saved;    // the workspace, most of what is kept: hooks that move or recompute it see it
   at::ScalarType dtypes[kSlots];
   bool released = false;
 
   std::string name() const override { return "GdnBackward"; }
   void release_variables() override {
-    for (auto* s : {&q_in, &k_in, &q, &k, &v, &g, &beta, &h0, &b, &w}) s->reset_data();
-    saved = Workspace();
+    for (auto* s : {&q_in, &k_in, &q, &k, &v, &g, &beta, &h0, &b, &w, &saved}) s->reset_data();
     released = true;
   }
   variable_list apply(variable_list&& grads) override {
@@ -295,9 +294,14 @@ struct GdnBackward : public torch::autograd::Node {
     Operands x{q.unpack(self), k.unpack(self), v.unpack(self), g.unpack(self), beta.unpack(self), h0.unpack(self),
                b.unpack(self), w.unpack(self)};
     c10::cuda::CUDAGuard guard(x.q.device());
+    Tensor ws = saved.unpack(self);
+    if (!workspace_aligned(ws)) {            // a hook brought it back somewhere else
+      Tensor t = workspace(static_cast<size_t>(ws.numel()), ws.options());
+      ws = t.copy_(ws);
+    }
     const Tensor d_o = d_o_in.defined() ? as(d_o_in, at::kBFloat16) : at::zeros({p.B, p.L, p.H, p.V}, x.v.options());
     const Tensor dhT = as32(dhT_in);
-    Grads r = run_backward(p, x, saved, d_o, dhT, six && p.delta == 1);
+    Grads r = run_backward(p, x, ws, d_o, dhT, six && p.delta == 1);
     if (p.l2) {     // VJP of x / sqrt(|x|^2 + eps) (the reference gets it by autograd, gdn2_assemble.py:300-312)
       Tensor qc, kc;
       const int flags = l2_inputs(q_in.unpack(self), k_in.unpack(self), &qc, &kc) | LETHE_L2_NORM_F16;
@@ -365,7 +369,7 @@ std::pair<Tensor, Tensor> apply(const Problem& p, const Tensor (&in)[kSlots], Op
     node->h0 = SavedVariable(f.x.h0, false);
     node->b = SavedVariable(f.x.b, false);
     node->w = SavedVariable(f.x.w, false);
-    node->saved = f.saved;
+    node->saved = SavedVariable(f.saved, false);
     torch::autograd::set_history(f.o, node);
     torch::autograd::set_history(f.hT, node);
   }

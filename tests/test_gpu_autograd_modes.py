@@ -41,3 +41,47 @@ def test_forward_mode_is_refused(name):
             with torch.no_grad(), pytest.raises(NotImplementedError, match="forward-mode"):
                 op(*args)
     op(*[d[n] for n in names])
+
+
+
+
+@every_op
+@pytest.mark.parametrize("l2norm", [False, True])
+def test_hooks_that_move_saved_tensors_see_all_of_them(name, l2norm):
+    """Everything the backward needs goes through the hooks, the workspace included, and may come back at any address."""
+    op, names = OPS[name]
+    d = _inputs()
+    kw = dict(use_qk_l2norm=l2norm)
+    leaves = [d[n].clone().requires_grad_(True) for n in names]
+    want = torch.autograd.grad(op(*leaves, **kw), leaves, d["do"])
+    packed = []
+
+    def pack(t):
+        packed.append(t.nbytes)
+        return t.cpu()
+
+    def unpack(t):                       # 512 bytes past whatever the allocator gives, which is on a 512-byte boundary
+        room = torch.empty(t.nbytes + 512, dtype=torch.uint8, device="cuda")
+        return room[512:].view(t.dtype).view(t.shape).copy_(t)
+
+    for move in (unpack, lambda t: t.cuda()):
+        with torch.autograd.graph.saved_tensors_hooks(pack, move):
+            o = op(*leaves, **kw)
+        for a, b in zip(torch.autograd.grad(o, leaves, d["do"]), want):
+            assert torch.equal(a, b)
+    assert max(packed) > 4 * d["q"].nbytes                 # the workspace: 100 KB and more per chunk
+
+
+@every_op
+def test_a_checkpointed_call_keeps_nothing_but_its_inputs_and_output(name):
+    from torch.utils.checkpoint import checkpoint
+    op, names = OPS[name]
+    d = _inputs(L=512)
+    leaves = [d[n].clone().requires_grad_(True) for n in names]
+    want = torch.autograd.grad(op(*leaves), leaves, d["do"])
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    o = checkpoint(lambda *t: op(*t), *leaves, use_reentrant=False)
+    assert torch.cuda.memory_allocated() - before <= o.nbytes + 4096
+    for a, b in zip(torch.autograd.grad(o, leaves, d["do"]), want):
+        assert torch.equal(a, b)
