@@ -464,6 +464,28 @@ def l2norm_qk(q: Tensor, k: Tensor, eps: float = 1e-6) -> tuple[Tensor, Tensor]:
     return _L2NormQK.apply(q, k, eps)
 
 
+class _Traced(torch.autograd.Function):
+    """A call under ``torch.jit.trace``.  The tracer records the tensor operations that it sees, which of a native call are
+    only the allocations of its results; an autograd function it records as a call, so this one stands around it."""
+
+    @staticmethod
+    def forward(ctx, call, scale, l2norm, *tensors):
+        inner = [None if t is None else t.detach().requires_grad_(t.requires_grad) for t in tensors]
+        with torch.enable_grad():
+            out = getattr(native.ext(), call)(*inner, scale, l2norm)
+        outs = (out,) if isinstance(out, Tensor) else out
+        ctx.outs, ctx.inner = outs, [t for t in inner if t is not None and t.requires_grad]
+        ctx.wanted = [t is not None and t.requires_grad for t in inner]
+        detached = tuple(t.detach() for t in outs)
+        return detached[0] if isinstance(out, Tensor) else detached
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, *grads):
+        got = iter(torch.autograd.grad(ctx.outs, ctx.inner, grads, retain_graph=True, allow_unused=True))
+        return (None, None, None, *(next(got) if w else None for w in ctx.wanted))
+
+
 def gdn_chunk(q: Tensor, k: Tensor, v: Tensor, g: Tensor | None, beta: Tensor | None,
               h0: Tensor | None = None, *, scale: float | None = None,
               use_qk_l2norm: bool = False) -> tuple[Tensor, Tensor]:
@@ -480,7 +502,10 @@ def gdn_chunk(q: Tensor, k: Tensor, v: Tensor, g: Tensor | None, beta: Tensor | 
     """
     if not q.is_cuda:
         raise GdnError("lethe_gdn: inputs must live on a CUDA device (there is no CPU path)")
-    return native.ext().chunk(q, k, v, g, beta, h0, q.shape[-1] ** -0.5 if scale is None else scale, use_qk_l2norm)
+    scale = q.shape[-1] ** -0.5 if scale is None else scale
+    if torch._C._is_tracing():
+        return _Traced.apply("chunk", float(scale), bool(use_qk_l2norm), q, k, v, g, beta, h0)
+    return native.ext().chunk(q, k, v, g, beta, h0, scale, use_qk_l2norm)
 
 
 class _DecodeArgs(ctypes.Structure):
@@ -509,7 +534,10 @@ def gdn_chunk_full(q: Tensor, k: Tensor, v: Tensor, g: Tensor, b: Tensor, w: Ten
     """The reference's full six-input recurrence with an initial state in and the final state out:
     ``g, b [B,L,H,K]`` (log decay and erase gate per key channel), ``w [B,L,H,V]`` (write gate per value
     channel).  Returns ``(o, h_T)``; gradients flow to all seven inputs (first order only)."""
-    return native.ext().chunk_full(q, k, v, g, b, w, h0, q.shape[-1] ** -0.5 if scale is None else scale, use_qk_l2norm)
+    scale = q.shape[-1] ** -0.5 if scale is None else scale
+    if torch._C._is_tracing():
+        return _Traced.apply("chunk_full", float(scale), bool(use_qk_l2norm), q, k, v, g, b, w, h0)
+    return native.ext().chunk_full(q, k, v, g, b, w, h0, scale, use_qk_l2norm)
 
 
 # ------------------------------------------------------------------------------------------------
@@ -543,7 +571,10 @@ def gdn2_op(q: Tensor, k: Tensor, v: Tensor, g: Tensor, b: Tensor, w: Tensor, *,
     (``gdn2_assemble.py:150-181``)."""
     if not q.is_cuda:
         raise GdnError("lethe_gdn: inputs must live on a CUDA device (there is no CPU path)")
-    return native.ext().six_inputs(q, k, v, g, b, w, q.shape[-1] ** -0.5 if scale is None else scale, use_qk_l2norm)
+    scale = q.shape[-1] ** -0.5 if scale is None else scale
+    if torch._C._is_tracing():
+        return _Traced.apply("six_inputs", float(scale), bool(use_qk_l2norm), q, k, v, g, b, w)
+    return native.ext().six_inputs(q, k, v, g, b, w, scale, use_qk_l2norm)
 
 
 class Gdn2Grads(NamedTuple):

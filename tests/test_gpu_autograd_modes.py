@@ -85,3 +85,18 @@ def test_a_checkpointed_call_keeps_nothing_but_its_inputs_and_output(name):
     assert torch.cuda.memory_allocated() - before <= o.nbytes + 4096
     for a, b in zip(torch.autograd.grad(o, leaves, d["do"]), want):
         assert torch.equal(a, b)
+
+
+@every_op
+@pytest.mark.filterwarnings("ignore")
+def test_a_traced_call_computes(name):
+    """torch.jit.trace: other inputs through the trace give what the op gives, and its gradients."""
+    op, names = OPS[name]
+    d, e = _inputs(), _inputs(seed=7)
+    traced = torch.jit.trace(lambda *t: op(*t) * 1, tuple(d[n] for n in names), check_trace=False)
+    leaves = [e[n].clone().requires_grad_(True) for n in names]
+    again = [e[n].clone().requires_grad_(True) for n in names]
+    o, want = traced(*leaves), op(*again)
+    assert torch.equal(o, want)
+    for a, b in zip(torch.autograd.grad(o, leaves, e["do"]), torch.autograd.grad(want, again, e["do"])):
+        assert torch.equal(a, b)
