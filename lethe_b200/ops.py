@@ -156,34 +156,43 @@ def backward_into(buf: GdnBuffers, q, k, v, g, beta, h0, do, dhT, scale: float, 
 
 
 def default_cut(gate: int, V: int, NT: int, BH: int, sms: int) -> int:
-    """Chunk index at which ``GdnStepGraph`` cuts every sequence: the whole number of CTA waves of the chunk
-    kernels nearest to half of the sequence.  A chunk kernel runs one CTA per chunk, two per SM for the scalar
-    gate at d_v = 64 and one otherwise; when the early segment fills whole waves, the kernels on the serial
-    chain (its prepare, its Stage B and WY) do not end on a nearly empty wave, which is worth 7 % of the step
-    at B=2, H=8, L=2048.  ``NT`` chunks per sequence, ``BH`` (batch, head) pairs, ``sms`` SMs."""
+    """Chunk index at which ``GdnStepGraph`` cuts every sequence: near half of its ``NT`` chunks, on a multiple of
+    as many chunks as two CTAs per SM (scalar gate or none, d_v = 64) or one (otherwise) cover when every one of
+    the ``BH`` (batch, head) pairs takes the same number; half where that is nothing or everything.  ``sms``: SMs.
+
+    That unit was a wave of the chunk kernels when they ran one CTA per chunk.  They are persistent now, with one
+    to four CTAs per SM, and no wave ends at the cut: the unit is where the cut lies, not a reason for it.  Replay
+    in us, not cut / cut at half / cut here, BH x NT: scalar gate, d_v = 64: 8 x 32 71 / 83 / 83, 16 x 32 115 / 107
+    / 106, 36 x 47 285 / 281 / 284, 32 x 64 339 / 328 / 337, 64 x 64 575 / 574 / 574; d_v = 128: 16 x 32 153 / 144 /
+    144, 64 x 64 806 / 842 / 842; channel-wise, d_v = 64: 16 x 32 167 / 157 / 149; d_v = 128: 16 x 32 191 / 193 /
+    193, 32 x 64 568 / 578 / 578, 64 x 128 2048 / 2075 / 2075; without the delta term, d_v = 128, 64 x 64: scalar
+    545 / 542 / 542, channel-wise 726 / 696 / 696.  So a cut is worth up to 11 % at 512 chunks and without the
+    delta term, and costs up to 4 % with it from 2048 chunks on, and 16 % for 8 pairs, whose scans leave most SMs
+    free."""
     if NT < 8:
         return 0
     per_sm = 2 if (gate != GATE_CHANNEL and V == 64) else 1
-    wave = (sms * per_sm) // BH                  # chunks of every (batch, head) pair in one wave
-    if wave == 0 or wave >= NT:
+    unit = (sms * per_sm) // BH                  # chunks of every (batch, head) pair
+    if unit == 0 or unit >= NT:
         return NT // 2
-    cut = max(1, int(NT / 2 / wave + 0.5)) * wave
+    cut = max(1, int(NT / 2 / unit + 0.5)) * unit
     if cut >= NT:
-        cut -= wave
+        cut -= unit
     return cut if cut > 0 else NT // 2
 
 
 def default_bwd_cuts(gate: int, V: int, delta: bool, NT: int, BH: int, sms: int, cut: int) -> tuple:
-    """Where the backward is cut: at the forward's cut, and - when the whole problem is at most two waves of
-    two CTAs per SM - once more at half a wave.  The last Stage B and WY launches of a step have nothing to
-    hide behind; with half a wave of chunks their CTAs have an SM each and finish sooner (measured at
-    B=2, H=8, L=2048, d_v=64: 0.1185 -> 0.1125 ms; larger problems and the one-CTA-per-SM kernels lose)."""
+    """Where the backward is cut: at the forward's cut, and - scalar gate, d_v = 64, two units of ``default_cut`` at
+    most - once more at half a unit, so that the last main kernel, which has nothing to hide behind, is short.
+    At B=2, H=8, L=2048 that cut, placed when Stage B and the WY VJP were kernels of their own, is worth nothing
+    any more: 107.2-108.6 us with it, 105.4-106.0 without.  Elsewhere a second cut at half of the first costs 1 to
+    9 % (d_v = 128, 512 chunks: 144 -> 153; channel-wise 193 -> 198; 4096 chunks 574 -> 587)."""
     if not cut:
         return ()
     two_per_sm = gate != GATE_CHANNEL and V == 64 and delta
-    wave = (sms * 2) // BH
-    if two_per_sm and wave >= 2 and cut == wave and wave < NT <= 2 * wave:
-        return (wave // 2, cut)
+    unit = (sms * 2) // BH
+    if two_per_sm and unit >= 2 and cut == unit and unit < NT <= 2 * unit:
+        return (unit // 2, cut)
     return (cut,)
 
 
@@ -198,14 +207,12 @@ class GdnStepGraph:
     ``pipeline`` (default): only the serial chain of the step - prepare, forward scan, adjoint scan, Stage B
     and WY - stays on one stream; the output kernel and the kernel that builds the adjoint scan's input run
     on other streams of the graph beside the scans (the adjoint scan needs neither the outputs nor the
-    forward scan).  ``cut`` (default: about half of the chunks, on a whole number of CTA waves, for
-    sequences of at least 8 chunks; 0 = no cut) splits every sequence into an early and a late segment of
+    forward scan).  ``cut`` (default: ``default_cut``, about half of the chunks, for sequences of at least 8
+    chunks; 0 = no cut) splits every sequence into an early and a late segment of
     chunks (``c_range`` of the C ABI): the late segment is prepared under the forward scan of the early one,
     and its Stage B and WY kernels run under the adjoint scan of the early one.  The scans hand their fp32
-    state from segment to segment through the workspace.  ``bwd_cuts`` (default: the forward's cut, plus one
-    at half a wave for problems of at most two waves) cuts the backward at places of its own.  (More
-    segments than that, and a stream per segment, measured slower: every extra segment adds a scan prologue
-    to the serial chain.)
+    state from segment to segment through the workspace.  ``bwd_cuts`` (default: ``default_bwd_cuts``) cuts the backward at
+    places of its own; every further segment adds a scan prologue to the serial chain.
 
     ``groups > 1``: the (batch, head) pairs are cut into that many ranges and every range runs its own
     kernel chain on its own stream inside the graph (the pairs are independent recurrences).

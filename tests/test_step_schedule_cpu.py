@@ -1,7 +1,8 @@
 """CPU: where the step graph cuts the sequences (pure host logic of ``lethe_b200.ops``).
 
 The cut points only move kernels between streams of the captured step - results are bit-identical for any
-cut (``tests/test_gpu_step_graph.py``) - so what is pinned here is the rule, on the shapes it was measured on."""
+cut (``tests/test_gpu_step_graph.py``) - so what is pinned here is what the rule gives.  Its unit is 296 (scalar gate,
+d_v = 64) or 148 chunks over the (batch, head) pairs; what the cuts are worth stands at the rule."""
 import pytest
 
 from lethe_b200 import ops
@@ -10,15 +11,15 @@ B200_SMS = 148
 
 
 @pytest.mark.parametrize("gate,V,delta,NT,BH,cut,bwd", [
-    (ops.GATE_SCALAR, 64, True, 32, 16, 18, (9, 18)),       # configuration 1: two CTAs per SM, 18 chunks per wave
-    (ops.GATE_CHANNEL, 128, True, 32, 16, 18, (18,)),       # configuration 2: one CTA per SM, 9 chunks per wave
-    (ops.GATE_SCALAR, 64, True, 64, 32, 36, (36,)),         # 2048 chunks: four waves, no second backward cut
-    (ops.GATE_SCALAR, 128, True, 32, 16, 18, (18,)),        # d_v = 128: Stage B holds an SM alone
-    (ops.GATE_CHANNEL, 128, True, 128, 64, 64, (64,)),      # configuration 4a share: two pairs per wave
+    (ops.GATE_SCALAR, 64, True, 32, 16, 18, (9, 18)),       # configuration 1: one unit of 18 chunks, the backward once more at half of it
+    (ops.GATE_CHANNEL, 128, True, 32, 16, 18, (18,)),       # configuration 2: two units of 9
+    (ops.GATE_SCALAR, 64, True, 64, 32, 36, (36,)),         # 2048 chunks: four units of 9, no second backward cut
+    (ops.GATE_SCALAR, 128, True, 32, 16, 18, (18,)),        # d_v = 128: two units of 9
+    (ops.GATE_CHANNEL, 128, True, 128, 64, 64, (64,)),      # configuration 4a share: units of 2
     (ops.GATE_SCALAR, 128, False, 64, 64, 32, (32,)),       # SSD of configuration 3
     (ops.GATE_SCALAR, 64, True, 4, 2, 0, ()),               # short sequences are not cut
-    (ops.GATE_SCALAR, 64, True, 16, 2, 8, (8,)),            # everything fits one wave: halves
-    (ops.GATE_SCALAR, 64, True, 16, 400, 8, (8,)),          # more pairs than CTA slots: halves
+    (ops.GATE_SCALAR, 64, True, 16, 2, 8, (8,)),            # the unit covers everything: half
+    (ops.GATE_SCALAR, 64, True, 16, 400, 8, (8,)),          # more pairs than the unit covers: half
 ])
 def test_default_cuts(gate, V, delta, NT, BH, cut, bwd):
     assert ops.default_cut(gate, V, NT, BH, B200_SMS) == cut
