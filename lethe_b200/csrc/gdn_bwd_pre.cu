@@ -179,8 +179,10 @@ static int launch_pre_t(const Problem& p, const CUtensorMap& mq, const CUtensorM
   if (attr.set(bwd_pre_kernel<V, DELTA, CW>, S::kBytes)) return kErrLaunch;
   const int sms = sm_count(), n = p.nbh * p.cn;
   if (sms <= 0) return kErrDevice;
-  // (not launched early: its CTAs would hold room that the kernel before, or one of another stream, could use - captured step
-  // of B H = 16, 32 chunks: 126 -> 112 us, forward and backward 136 -> 130)
+  // Not launched early: its CTAs would hold room that the kernel before, or one of another stream, could use.  Captured step,
+  // us, plain / early, scalar gate, d_v = 64: 512 chunks 107 / 116, 2048 335 / 341, 4096 572 / 597; channel-wise, d_v = 128: 512
+  // 190 / 199, 8192 2074 / 2046 (early is the better one at the largest, scalar d_v = 128 at 4096 842 / 815 too); one chain: no
+  // more than 1 % either way up to 2048 chunks, 4096 596 / 614.
   bwd_pre_kernel<V, DELTA, CW><<<n < S::kCtas * sms ? n : S::kCtas * sms, kPreThreads, S::kBytes, st>>>(p, mq, mdo);
   return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
 }

@@ -680,8 +680,9 @@ template <int V>
 static int launch_prepare_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, cudaStream_t st) {
   static SmemAttr attr[2];
   // Not early for a later part of the sequences of at most two rounds: its CTAs would take the SMs that the scan of the first
-  // part starts on (captured step of B H = 16, 32 chunks: 108.5 -> 105.6 us).  With more rounds the time saved at its start
-  // counts for more (4096 chunks: 572 us early, 582 not).
+  // part starts on.  Captured step, us, plain / early, by chunks of the later part: 224 (d_v = 64) 107.0 / 108.2, 224 (d_v = 128)
+  // 143 / 140, 828 281 / 284, 896 328 / 336, 2048 584 / 573.  So the line could lie between 900 and 2000 as well; below it the
+  // two differ by less than two captures of the same step do (2 %).
   const int sms = sm_count();
   const bool early = p.c0 == 0 || p.nbh * p.cn > 4 * sms;
   return p.delta ? launch_persistent(prepare_kernel<V>, attr[0], PrepSmem<V>::kBytes, 2, p, mq, mk, mv, st, early)
@@ -691,7 +692,9 @@ template <int V, bool DELTA, bool CW>
 static int launch_output_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mv, const CUtensorMap& mo, cudaStream_t st) {
   static SmemAttr attr;
   // A part of the sequences (a captured step that overlaps parts): early CTAs would wait in room that a scan or a chunk kernel
-  // of another part needs (B H = 16, 32 chunks: 112 -> 109 us, 4096 chunks 584 -> 571; without the delta term nothing is that long)
+  // of another part needs.  Captured step, us, plain / early, scalar gate, d_v = 64: 256 chunks 83 / 89, 512 107 / 111, 2048
+  // 335 / 341, 4096 572 / 586; channel-wise: 512 150 / 157 (d_v = 64) and 190 / 191 (128), 8192 2074 / 2057 (early is the better
+  // one there).  Without the delta term the kernels are short and the gaps count: 512 59 / 57, 4096 553 / 541 and 727 / 695.
   const bool early = !DELTA || p.cn == p.NT;
   return launch_persistent(output_kernel<V, DELTA, CW>, attr, OutSmem<V, CW>::kBytes, OutSmem<V, CW>::kCtas, p, mq, mv, mo, st, early);
 }

@@ -312,8 +312,9 @@ static int launch_scan_t(const Problem& p, bool adjoint, cudaStream_t st) {
   constexpr int kW = kVs * kGr;
   int smem = kStages * 32768 + 2 * 128 * kW * 2 + static_cast<int>(sizeof(CtaShared)) + 1024;
   // Launched early, CTAs of 16 columns settle in pairs on the first SMs that the kernel before leaves, and share their intake;
-  // asking for more than half of an SM's memory keeps them apart (B H = 16, 32 chunks: forward and backward 130 -> 120 us).
-  // Not when the sequences are cut: the next range's scan then waits on the SMs of this one, not on others.
+  // asking for more than half of an SM's memory keeps them apart (one chain, us: 16 pairs x 32 chunks 131 -> 122, d_v = 128 166
+  // -> 152, 32 x 64 373 -> 357).  Not when the sequences are cut: the next range's scan then waits on the SMs of this one, not
+  // on others (captured step, alone / in pairs: 16 x 32 116 / 107, channel-wise 199 / 190; 8 x 32, with room for all, 75 / 83).
   if (kGr == 1 && p.cn == p.NT) smem = kScanAloneBytes;
   dim3 grid(p.V / kW, p.nbh);
   if (adjoint) {
