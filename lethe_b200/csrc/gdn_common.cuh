@@ -143,30 +143,17 @@ struct CtaShared {
 // Next 1024-byte boundary of the dynamic shared memory window, two ways.  `align1024` is plain
 // pointer arithmetic on the shared symbol, so the compiler keeps the shared address space and emits
 // shared-memory loads and stores; `align1024_generic` goes through an integer, after which every
-// access is a generic one.  Same addresses, different instruction selection and scheduling: the
-// channel-wise kernels run 10-15 % faster with the first, the scalar kernels 3-6 %, the scans 1-3 % faster with
-// the second (measured per kernel on a B200), so each kernel names the one it wants.
-__device__ __forceinline__ unsigned char* align1024_s_(unsigned char* p) {
+// access is a generic one.  Same addresses, different instruction selection and scheduling.  The chunk
+// kernels want the first (us, generic against shared: prepare 148 / 135 at 4096 chunks, channel-wise 667 /
+// 590 at 8192; main 270 / 224 and 1051 / 915; output and scan input within 3 %, once 78 / 70).  The scan of
+// 64 columns per CTA is 1-3 % faster with the second (64.7 / 63.4 for 32 pairs x 64 chunks); at 16 columns
+// the forward scan is as well (17.2 / 16.8 at 16 x 32, d_v = 128 17.6 / 18.0), the adjoint is not (16.5 / 17.3).
+__device__ __forceinline__ unsigned char* align1024(unsigned char* p) {
   const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(p));
   return p + ((1024u - (a & 1023u)) & 1023u);
 }
-__device__ __forceinline__ unsigned char* align1024_g_(unsigned char* p) {
-  return reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(p) + 1023) & ~static_cast<uintptr_t>(1023));
-}
-// (-DLETHE_ALL_SHARED / -DLETHE_ALL_GENERIC force one flavour everywhere, to repeat the comparison)
-__device__ __forceinline__ unsigned char* align1024(unsigned char* p) {
-#ifdef LETHE_ALL_GENERIC
-  return align1024_g_(p);
-#else
-  return align1024_s_(p);
-#endif
-}
 __device__ __forceinline__ unsigned char* align1024_generic(unsigned char* p) {
-#ifdef LETHE_ALL_SHARED
-  return align1024_s_(p);
-#else
-  return align1024_g_(p);
-#endif
+  return reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(p) + 1023) & ~static_cast<uintptr_t>(1023));
 }
 
 // Called by all threads before one thread issues products that read tiles written by this CTA's
