@@ -102,11 +102,6 @@ __device__ __forceinline__ void unpack8_in(const uint4& u, float* v, int f16) {
   if (f16) unpack8_f16(u, v);
   else unpack8_bf16(u, v);
 }
-__device__ __forceinline__ uint4 pack8_out(const float* v, int f16) { return f16 ? pack8_f16(v) : pack8_bf16(v); }
-__device__ __forceinline__ void store_out16(__nv_bfloat16* dst, float x, int f16) {
-  if (f16) *reinterpret_cast<__half*>(dst) = __float2half_rn(x);
-  else *dst = __float2bfloat16_rn(x);
-}
 
 // chunk access on a tile given as a generic pointer to its first byte
 __device__ __forceinline__ uint4 tile_ld_chunk(const unsigned char* tile, int r, int ch, int rows) {

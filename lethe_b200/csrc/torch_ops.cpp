@@ -15,8 +15,6 @@
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/extension.h>
 
-#include <atomic>
-#include <chrono>
 #include <mutex>
 #include <string>
 #include <vector>
