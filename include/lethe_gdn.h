@@ -26,7 +26,8 @@
  *   beta        [B, L, H] fp32 (delta = 1)
  *   h0, hT, dhT, dh0   [B, H, K, V] fp32
  *   dg          like g, fp32;   dbeta like beta, fp32
- * Sizes: K = 128, V in {64, 128}, L a multiple of 64 (the chunk length).
+ * Sizes: dims.K = 128, dims.V in {64, 128}, dims.L a multiple of 64 (the chunk length); tensors with 64 key
+ * channels or another number of tokens say so in k_channels and l_tokens.
  */
 #ifndef LETHE_GDN_H_
 #define LETHE_GDN_H_

@@ -289,7 +289,7 @@ extern "C" const char* lethe_gdn_strerror(int code) {
   switch (code) {
     case kOk: return "ok";
     case kErrNull: return "a required pointer is null";
-    case kErrDims: return "unsupported sizes (need K = 128, V in {64, 128}, L a multiple of 64)";
+    case kErrDims: return "unsupported sizes or ranges (dims: K = 128, V in {64, 128}, L a multiple of 64; l_tokens and k_channels for less)";
     case kErrAlign: return "a pointer is not aligned (16 bytes for tensors, 1024 for workspaces)";
     case kErrWorkspace: return "workspace too small";
     case kErrDriver: return "tensor-map encoding failed (driver entry point missing or bad tensor geometry)";

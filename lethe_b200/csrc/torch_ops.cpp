@@ -189,7 +189,7 @@ Forward run_forward(const Problem& p, Operands x, bool keep) {
   const size_t need = lethe_gdn_saved_bytes(&d);
   if (need == 0)
     fail("unsupported sizes B=" + std::to_string(p.B) + " H=" + std::to_string(p.H) + " L=" + std::to_string(p.L) +
-         " K=" + std::to_string(p.K) + " V=" + std::to_string(p.V) + " (need K = 128, V in {64, 128}, L a multiple of 64)");
+         " K=" + std::to_string(p.K) + " V=" + std::to_string(p.V) + " (need V = 64 or 128, and at least one of B, H, L)");
   const auto o16 = x.v.options();
   const auto o32 = o16.dtype(at::kFloat);
   f.saved = workspace(need, o16);

@@ -73,3 +73,13 @@ def test_lengths_off_the_chunk_grid(gate, delta, L):
         errs["d" + n] = scale_rel(got[n].double().cpu(), ref[n])
     report(f"ragged gate={gate} delta={delta} L={L}", errs)
     assert max(errs.values()) <= TOL, errs
+
+
+@pytest.mark.parametrize("shape,says", [((1, 70, 2, 64, 32), "need V = 64 or 128"), ((1, 0, 2, 128, 64), "at least one of B, H, L"),
+                                        ((1, 64, 2, 96, 64), "need K = 64 or 128")])
+def test_unsupported_sizes_are_named_as_the_op_takes_them(shape, says):
+    """The op takes 64 key channels and any length; its messages must not ask for less."""
+    B, L, H, K, V = shape
+    q, v = (torch.zeros(B, L, H, n, device="cuda", dtype=torch.bfloat16) for n in (K, V))
+    with pytest.raises(ops.GdnError, match=says):
+        ops.gdn_chunk(q, q, v, None, None)
