@@ -21,8 +21,9 @@ timed alone with CUDA events, plus the whole step against the algorithmic bytes 
 (HBM and tensor-core fractions for forward, backward and both).  `cpu_baseline`: the reference project's
 own PyTorch CPU chunkwise path (its backward assembly, imported from `oracle/_ref`, the reference compiled
 to bytecode) timed on this machine's host cores on a bounded sample; the CPU oracle port stands in only
-where `oracle/_ref` is absent.  `--impl reference` times that CPU path only (rank 0; other ranks exit):
-W warm-up passes, then K timed passes, every pass really executed.
+where `oracle/_ref` is absent (its `kind` then says "port").  `--impl reference` times that CPU path only (rank 0;
+other ranks exit): W warm-up passes, then K timed passes, every pass really executed; where `oracle/_ref` is absent
+it says that the reference is unavailable, since the port is this repository's own code.
 """
 
 from __future__ import annotations
@@ -546,17 +547,17 @@ def main():
     ap.add_argument("--steps", type=int, default=20)
     ap.add_argument("--warmup", type=int, default=5)
     ap.add_argument("--impl", default="ours", choices=["ours", "reference", "fla", "aux"],
-                    help="reference: the reference's own CPU path (oracle/_ref) or its CPU port; fla: third-party "
+                    help="reference: the reference's own CPU path (oracle/_ref), or that it is unavailable; fla: third-party "
                          "comparator (see fla_main); aux: the L2-normalisation and decode-step kernels")
     ap.add_argument("--groups", type=int, default=1,
                     help="cut the (batch, head) pairs into this many ranges that run as concurrent kernel chains "
                          "inside the step graph (helps when the scans leave SMs idle: a few % on the larger workloads)")
     ap.add_argument("--cut", type=int, default=-1,
                     help="chunk index at which the step graph cuts every sequence into an early and a late segment "
-                         "(0: no cut; -1: the library's default, about half of the chunks on a whole number of CTA waves)")
+                         "(0: no cut; -1: the library's default, about half of the chunks)")
     ap.add_argument("--bwd-cuts", default="",
                     help="comma-separated chunk indices at which the backward of the step graph is cut (default: the "
-                         "forward's cut)")
+                         "library's)")
     ap.add_argument("--plain-chain", action="store_true",
                     help="capture the step as one chain of kernels on one stream (no overlap inside the graph)")
     ap.add_argument("--mild-gate", action="store_true",
@@ -585,6 +586,11 @@ def main():
         return
     if args.impl == "reference":
         if rank != 0:
+            return
+        from oracle import make_ref
+        if make_ref.import_reference() is None:
+            print(json.dumps({"impl": "reference", "unavailable": "the reference's files are not on this machine: "
+                              "oracle/_ref, its byte-compiled copy, is absent and there is nothing to build it from"}))
             return
         t_run = time.perf_counter()
         cb, ts = cpu_time_passes(args.workload, steps=args.steps, warmup=args.warmup)
