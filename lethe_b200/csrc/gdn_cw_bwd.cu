@@ -32,8 +32,12 @@
 //
 // What bounds it: 272 KB of traffic per chunk (12 k cycles of an SM's share of HBM) against the chain of six dependent
 // product groups plus CUDA-core phases.  The CTA is persistent and fetches the next chunk's tiles into the ones that
-// are dead once its last products are issued, under the longest CUDA-core phase.  Measured against the four kernels
-// this replaces (Stage B 1, pair sums, WY 1, pair sums; 887 KB of traffic per chunk) in the notes of launch_main.
+// are dead once its last products are issued, under the longest CUDA-core phase.  8192 chunks, d_v = 128: 915 us; the four
+// kernels that this replaced (Stage B 1, pair sums, WY 1, pair sums; 887 KB of traffic per chunk) took 2489.
+// Cycles per chunk by clock samples of one CTA (d_v = 128): operand columns and waits for the tiles 5.1 k, group 1 and its
+// epilogues 4.2 k, the four dependent groups from dw to dM 6.3 k, column sums with the decay assembly 5.3 k, row sums with
+// the gradients 5.3 k, gate gradient and stores 2.4 k; 28.6 k in all.  Without the delta term 6.5, 3.9, 0, 3.7, 2.5, 1.9:
+// 18.5 k; with per-channel gates 10.8, 4.6, 12.9, 6.1, 7.0, 1.8: 43.3 k.
 #include "gdn_cw.cuh"
 #include "host_util.h"
 

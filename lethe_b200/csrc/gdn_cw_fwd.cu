@@ -16,10 +16,13 @@
 // inside its own group a row goes down the source rows with ratio(i, s) = ratio(i, s + 1) alpha(s + 1); for an earlier
 // group the source rows lie ready in fp32, decayed to the end of their group, and the row carries its decay from there, so
 // that a pair costs two FMAs per channel and no ratio.  All in fp32, and every factor is a decay between two rows that lie
-// between s and i.  (Walking every pair with a running ratio took 6.8 k cycles per chunk, this 4.2 k.)
+// between s and i.  (Walking every pair with a running ratio took 6.8 k cycles per chunk, this 4.8 k.)
 //
 // The CTA is persistent: the next chunk's k, q and g are fetched as soon as the diagonal sums have read this chunk's.  v
 // is fetched under the first epilogue: its tile holds the decayed source rows before.
+// Cycles per chunk by clock samples of one CTA (d_v = 128): loads and operand columns 4.8 k, diagonal blocks 4.8 k, epilogue
+// of M and A 1.8 k, inverse 3.5 k, WY factors, P and R 3.8 k; 18.8 k in all.  Without the delta term 4.6, 4.0 and, for A and R,
+// 4.2: 12.8 k.
 #include "gdn_cw.cuh"
 #include "gdn_inverse.cuh"
 #include "host_util.h"
