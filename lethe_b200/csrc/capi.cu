@@ -189,6 +189,7 @@ extern "C" int lethe_gdn_backward(const LetheGdnArgs* a, void* stream) {
   const uint32_t m = a->kernel_mask ? a->kernel_mask : 15u;
   if ((m & 1u) && (e = launch_bwd_pre(p, mq, mdo, st))) return e;
   if ((m & 2u) && (e = launch_scan(p, true, st))) return e;
+  p.after_scan = (m & 2u) ? 1 : 0;
   if (m & 12u) {
     if (p.gate == LETHE_GATE_CHANNEL) {
       CUtensorMap mg;

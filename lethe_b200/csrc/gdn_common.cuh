@@ -92,6 +92,7 @@ struct Problem {
   uint32_t lean;     // 1: intermediates that no later kernel of the call reads are not written; 2: nor what only a backward reads
   int qk16;          // non-zero: q, k, dq, dk hold fp16 instead of bf16
   float scale;
+  int after_scan;    // the same call launched the adjoint scan just before the main kernel
   float l2_eps;      // > 0: the channel-wise prepare kernel normalises q and k
   int keep_norm;     // ... and stores the normalised rows
   const __nv_bfloat16 *q, *k, *v, *d_o;

@@ -143,10 +143,11 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       tma_load_4d(tQ + t * 8192, &mq, &bars->in0, t * 64, a.h, a.c * kC, a.b);
     }
   };
-  auto load_part3 = [&](const At& a) {
-    if (!SB) return;
+  auto load_rec = [&](const At& a) {      // v_new, h
     if (DELTA) bulk_g2s(tVN, p.saved + p.lay.vn + static_cast<size_t>(a.z) * p.lay.sz_vn, V * 128, &bars->in1);
     bulk_g2s(tH, p.saved + p.lay.hc + static_cast<size_t>(a.z + a.bh) * p.lay.sz_hc, V * 256, &bars->in1);
+  };
+  auto load_dh = [&](const At& a) {
     bulk_g2s(tDH, p.scratch + p.lay.dh + static_cast<size_t>(a.z) * p.lay.sz_dh, V * 256, &bars->in1);
   };
 
@@ -157,12 +158,15 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     mbar_init(&bars->mO, 1);
     fence_mbar_init();
     fence_proxy_async();
-    // Older than whatever kernel of the path comes just before this one: the caller's tensors and [T; A].  Not dh (the adjoint
-    // scan), v_new (the output kernel) and h (the forward scan): which of the three ran last is up to the caller.
+    // Older than whatever kernel of the path comes just before this one: the caller's tensors and [T; A].  v_new (the output
+    // kernel) and h (the forward scan) only where this call has put the adjoint scan in between; with kernels picked one by one
+    // any of the three may be the last.  (Late everywhere: SSD forward and backward 175.1 us instead of 172.3 at 1692 chunks, 557.8
+    // instead of 555.3 at 4096; with the delta term no difference.)
     if (SB) {
       const At a = at(blockIdx.x);
       load_part1(a);
       load_part2(a);
+      if (p.after_scan) load_rec(a);
     }
   }
   if (warp == 0) {
@@ -181,11 +185,13 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
   griddep_launch();
   if (tid == 0) {
     const At a = at(blockIdx.x);
-    if (!SB) {
+    if (SB) {
+      if (!p.after_scan) load_rec(a);
+      load_dh(a);
+    } else {
       load_part1(a);
       load_part2(a);
     }
-    load_part3(a);
   }
   const uint32_t aK = smem_u32(tK), aQ = smem_u32(tQ), aC = smem_u32(tC), aBE = smem_u32(tBE);
 
@@ -216,7 +222,10 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     if (WY && tid < 64) betas[tid] = beta_r;
     if (tid == 0 && n != static_cast<int>(blockIdx.x)) {
       bulk_wait_read();                             // the results of the chunk before have left their tiles
-      load_part3(a);
+      if (SB) {
+        load_rec(a);
+        load_dh(a);
+      }
     }
     __syncthreads();          // the raw tiles are read, the block products are there
     const BlockDecays bd = block_decays(Bb, Af, blk, d);

@@ -18,10 +18,13 @@ from .cusource import block, kernel_body, source
 MAIN = 12      # Stage B and the WY VJP
 
 
-def early_reads(name, kernel):
-    """Records that a kernel reads before its first wait for the kernel before it (as text: every branch counts)."""
+def early_reads(name, kernel, after_scan=False):
+    """Records that a kernel reads before its first wait for the kernel before it (as text: every branch counts, but for
+    what a call does only when it has launched the adjoint scan itself)."""
     body = kernel_body(name, kernel)
     body = body[:body.index("griddep_wait();")]
+    if not after_scan:
+        body = re.sub(r"if \(p\.after_scan\) \w+\(a\);", "", body)
     lambdas = {}
     for m in reversed(list(re.finditer(r"auto (\w+) = \[&\]", body))):
         inner, end = block(body, m.end())
@@ -38,8 +41,15 @@ def early_reads(name, kernel):
 def test_what_the_kernels_read_before_they_wait():
     """Before its wait a kernel may read the caller's tensors and what the prepare kernel wrote: the calls that need a
     chunk's other records all lie between prepare and the reader, on any stream."""
-    assert early_reads("gdn_bwd_main.cu", "bwd_sc_kernel") == {"ta"}
-    assert early_reads("gdn_cw_bwd.cu", "bwd_cw_kernel") == {"ta"}
+    for main in (("gdn_bwd_main.cu", "bwd_sc_kernel"), ("gdn_cw_bwd.cu", "bwd_cw_kernel")):
+        assert early_reads(*main) == {"ta"}
+        # in one call with the adjoint scan also what is older than that scan
+        assert early_reads(*main, after_scan=True) <= {"ta", "vn", "hc", "dv2"}
+    backward = source("capi.cu")
+    backward = backward[backward.index("int lethe_gdn_backward("):]
+    assert re.search(r"if \(\(m & 2u\) && \(e = launch_scan\(p, true, st\)\)\) return e;\s*p\.after_scan = \(m & 2u\) \? 1 : 0;\s*"
+                     r"if \(m & 12u\)", backward)
+    assert sum(s.count("after_scan =") for s in map(source, ("capi.cu", "gdn_bwd_main.cu", "gdn_cw_bwd.cu"))) == 1
     assert early_reads("gdn_fwd.cu", "output_kernel") == {"qg", "w", "ta", "u"}
     for name, kernel in (("gdn_fwd.cu", "prepare_kernel"), ("gdn_fwd.cu", "prepare_nodelta_kernel"),
                          ("gdn_scan.cu", "scan_nodelta_kernel")):
