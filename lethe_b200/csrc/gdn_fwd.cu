@@ -99,6 +99,8 @@ __device__ __forceinline__ void prep_kd(unsigned char* KD, const unsigned char* 
 }
 // 32 columns (from 32 half) of row r of a product, times the decay between the tokens and `f`; zero from column `end` on.
 // Everything in registers first: with a store or a branch between them the exponentials run one at a time (2.7 k cycles).
+// The exponent is not clamped: what it gives right of `end` is dropped, and left of it a clamp would hide a log decay above
+// zero, and make "no decay" of the NaN between two tokens behind a decay of minus infinity.
 __device__ __forceinline__ void prep_decay_row(float* d, const float* Gs, int r, int half, int end, float f) {
   const float Gr = Gs[r];
   float g[32];
@@ -106,7 +108,7 @@ __device__ __forceinline__ void prep_decay_row(float* d, const float* Gs, int r,
   for (int q = 0; q < 4; ++q) ld8(Gs + half * 32 + 8 * q, g + 8 * q);
 #pragma unroll
   for (int j = 0; j < 32; ++j) {
-    const float x = f * __expf(fminf(Gr - g[j], 0.f)) * d[j];
+    const float x = f * __expf(Gr - g[j]) * d[j];
     d[j] = half * 32 + j < end ? x : 0.f;
   }
 }
