@@ -377,6 +377,15 @@ std::pair<Tensor, Tensor> apply(const Problem& p, const Tensor (&in)[kSlots], Op
 void need_shape(bool ok, const char* what) {
   if (!ok) fail(std::string("shapes do not match: ") + what);
 }
+// a pointer from somewhere else would fault in a kernel
+template <typename... T>
+void need_device(const Tensor& like, const T&... ts) {
+  auto one = [&](const Tensor& t) {
+    if (t.defined() && t.device() != like.device())
+      fail("all inputs must live on one CUDA device (" + like.device().str() + " and " + t.device().str() + ")");
+  };
+  (one(ts), ...);
+}
 
 Problem describe(const Tensor& q, const Tensor& k, const Tensor& v, double scale, bool l2) {
   if (!q.is_cuda()) fail("inputs must live on a CUDA device (there is no CPU path)");
@@ -430,6 +439,7 @@ std::pair<Tensor, Tensor> chunk(const Tensor& q, const Tensor& k, const Tensor& 
   return guarded([&] {
     const Tensor g = opt(g_), beta = opt(beta_), h0 = opt(h0_);
     Problem p = describe(q, k, v, scale, l2);
+    need_device(q, k, v, g, beta, h0);
     check_gate(p, g);
     check_state(p, h0);
     if (beta.defined()) need_shape(beta.sizes() == q.sizes().slice(0, 3), "beta [B, L, H]");
@@ -468,6 +478,7 @@ std::pair<Tensor, Tensor> chunk_full(const Tensor& q, const Tensor& k, const Ten
   return guarded([&] {
     const Tensor h0 = opt(h0_);
     const Problem p = describe(q, k, v, scale, l2);
+    need_device(q, k, v, g, b, w, h0);
     check_channel_gates(p, q, v, g, b, w);
     check_state(p, h0);
     c10::cuda::CUDAGuard guard(q.device());
@@ -598,6 +609,7 @@ uint32_t regime_by_ops(const Tensor& g, const Tensor& b, const Tensor& w) {
 uint32_t gate_regime(const Tensor& g, const Tensor& b, const Tensor& w) {
   return guarded([&]() -> uint32_t {
     at::NoGradGuard no_grad;
+    need_device(g, b, w);
     const int64_t V = w.size(-1);
     if (!(g.is_cuda() && g.dim() == 4 && b.dim() == 4 && w.dim() == 4 && g.size(3) == 128 && (V == 64 || V == 128) &&
           g.sizes() == b.sizes() && plain32(g) && plain32(b) && plain32(w)))
@@ -612,6 +624,7 @@ Tensor six_inputs(const Tensor& q, const Tensor& k, const Tensor& v, const Tenso
   return guarded([&]() -> Tensor {
     Problem p = describe(q, k, v, scale, l2);
     if (p.K != 128) fail("gdn2_op needs d_k = 128 (use gdn_chunk for d_k = 64)");
+    need_device(q, k, v, g, b, w);
     check_channel_gates(p, q, v, g, b, w);
     c10::cuda::CUDAGuard guard(q.device());
     const Tensor in[kSlots] = {q, k, v, g, Tensor(), Tensor(), b, w};
@@ -659,7 +672,9 @@ Tensor decode_step(const Tensor& q, const Tensor& k, const Tensor& v, const OptT
     const int64_t B = state.size(0), H = state.size(1), K = state.size(2), V = state.size(3);
     if (q.sizes() != at::IntArrayRef({B, H, K}) || k.sizes() != q.sizes() || v.sizes() != at::IntArrayRef({B, H, V}))
       fail("decode step expects q, k [B,H,K] and v [B,H,V] matching the state");
-    const Tensor g = as32(opt(g_)), beta = as32(opt(beta_));
+    const Tensor g_in = opt(g_), beta_in = opt(beta_);
+    need_device(state, q, k, v, g_in, beta_in);
+    const Tensor g = as32(g_in), beta = as32(beta_in);
     if (g.defined() && g.sizes() != at::IntArrayRef({B, H}) && g.sizes() != q.sizes())
       fail("decode step expects g [B,H] or [B,H,K]");
     if (beta.defined() && beta.sizes() != at::IntArrayRef({B, H})) fail("decode step expects beta [B,H]");

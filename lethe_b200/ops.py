@@ -80,6 +80,15 @@ def check_status(status: Tensor) -> None:
         raise GdnError(f"lethe_gdn: device-side wait timed out at site {code}; results are invalid")
 
 
+def _same_device(q: Tensor, *tensors) -> None:
+    """A pointer from somewhere else would fault in a kernel."""
+    if not q.is_cuda:
+        raise GdnError("lethe_gdn: inputs must live on a CUDA device (there is no CPU path)")
+    for t in tensors:
+        if t is not None and t.device != q.device:
+            raise GdnError(f"lethe_gdn: all tensors must live on one CUDA device ({q.device} and {t.device})")
+
+
 def _prep16(t: Tensor) -> Tensor:
     return t.to(torch.bfloat16).contiguous()
 
@@ -129,6 +138,7 @@ def forward_into(buf: GdnBuffers, q, k, v, g, beta, h0, scale: float, kernel_mas
     ``c_range = (begin, count)`` to those 64-token chunks of every sequence (the scans carry their state from
     one range to the next: forward ranges in ascending order).  ``lean``: workspace records that no kernel of the
     forward or the backward reads are not written."""
+    _same_device(q, k, v, g, beta, h0, b_gate, w_gate, buf.saved)
     a = _Args(dims=buf.dims, scale=scale, q=_ptr(q), k=_ptr(k), v=_ptr(v), g=_ptr(g), beta=_ptr(beta),
               h0=_ptr(h0), o=_ptr(buf.o), hT=_ptr(buf.hT), saved=_ptr(buf.saved),
               saved_bytes=buf.saved.numel(), status=_ptr(buf.status), kernel_mask=kernel_mask,
@@ -142,6 +152,7 @@ def backward_into(buf: GdnBuffers, q, k, v, g, beta, h0, do, dhT, scale: float, 
                   c_range: tuple[int, int] = (0, 0), lean: bool = False) -> None:
     """Enqueue the backward kernels; gradients land in ``buf.dq`` ... ``buf.dh0`` (``buf.db`` / ``buf.dw``
     for the per-channel gates of buffers made with ``delta=2``)."""
+    _same_device(q, k, v, g, beta, h0, do, dhT, b_gate, w_gate, buf.saved)
     a = _Args(dims=buf.dims, scale=scale, q=_ptr(q), k=_ptr(k), v=_ptr(v), g=_ptr(g), beta=_ptr(beta),
               h0=_ptr(h0), d_o=_ptr(do), dhT=_ptr(dhT), dq=_ptr(buf.dq), dk=_ptr(buf.dk), dv=_ptr(buf.dv),
               dg=_ptr(buf.dg), dbeta=_ptr(buf.dbeta), dh0=_ptr(buf.dh0), saved=_ptr(buf.saved),
@@ -414,8 +425,7 @@ def l2norm_qk_raw(q: Tensor, k: Tensor, eps: float = 1e-6, norm_dtype=torch.floa
     the reference, ``gdn_backward.py:9-10``).  The rows are formed in fp32 and rounded once: to fp16 by
     default (the operand type of the GDN kernels, which then read them unchanged; the reference rounds
     at the same point, ``gdn2_bwd_dhu_l3.py:477-479``), or to bf16 with ``norm_dtype=torch.bfloat16``."""
-    if not q.is_cuda:
-        raise GdnError("lethe_gdn: inputs must live on a CUDA device (there is no CPU path)")
+    _same_device(q, k)
     if q.shape != k.shape:
         raise GdnError("lethe_gdn: q and k must have the same shape")
     if norm_dtype not in (torch.float16, torch.bfloat16):
@@ -433,6 +443,7 @@ def l2norm_qk_raw(q: Tensor, k: Tensor, eps: float = 1e-6, norm_dtype=torch.floa
 def l2norm_qk_vjp_raw(q: Tensor, k: Tensor, dqn: Tensor, dkn: Tensor, eps: float = 1e-6) -> tuple[Tensor, Tensor]:
     """Gradients with respect to q and k given those with respect to the normalised rows (fp16 or bf16,
     as the backward kernels wrote them).  Returned in the working type of q, k (bf16 or fp32)."""
+    _same_device(q, k, dqn, dkn)
     qc, kc, f32 = _l2_working(q, k)
     f16 = dqn.dtype == torch.float16 and dkn.dtype == torch.float16
     if f16:
