@@ -18,34 +18,28 @@
 // that a pair costs two FMAs per channel and no ratio.  All in fp32, and every factor is a decay between two rows that lie
 // between s and i.  (Walking every pair with a running ratio took 6.8 k cycles per chunk, this 4.8 k.)
 //
-// The CTA is persistent: the next chunk's k, q and g are fetched as soon as the diagonal sums have read this chunk's.  v
-// is fetched under the first epilogue: its tile holds the decayed source rows before.
-// Cycles per chunk by clock samples of one CTA (d_v = 128): loads and operand columns 4.8 k, diagonal blocks 4.8 k, epilogue
-// of M and A 1.8 k, inverse 3.5 k, WY factors, P and R 3.8 k; 18.8 k in all.  Without the delta term 4.6, 4.0 and, for A and R,
-// 4.2: 12.8 k.
+// NB: blocks of 16 tokens per thread.  2: 256 threads on six tiles that change hands, two persistent CTAs per SM, so that
+// one chunk's barriers, product waits and loads lie under the other's arithmetic; k, q and alpha go to registers after the diagonal
+// sums and the operands take their tiles.  1: 512 threads, for a launch that gives every SM one chunk at most, where only the
+// length of a chunk's own chain counts.  Measured (us, d_v = 128; one CTA of 512 threads with twice the memory before): 8192
+// chunks 590 -> 559, 8000 chunks 582 -> 547, 512 chunks 54 -> 49, without the delta term 4096 chunks 209 -> 190, per-channel gates 512
+// chunks 70 -> 59; 128 chunks 20.5 either way.
 #include "gdn_cw.cuh"
 #include "gdn_inverse.cuh"
 #include "host_util.h"
 
 namespace lg {
 
-constexpr int kPrepCwThreads = 512;
 constexpr int kDg = 17;                               // row stride (floats) of the diagonal-block buffers
 
-template <int V>
+// Six tiles of 16 KB that change hands:
+//   tile       0            1            2                3            4                        5
+//   loaded     k            q            g, then alpha (fp32)          k to the end of its four rows (fp32), decays over four rows
+//   products   k e          q e          k to the start of later blocks   k exp(G_last - G)     b gamma k
+//   inverse    M and scratch             [T; A]           v, beta v    "                        "
+//   then       w            u            "                "            P (without the delta term R)
 struct PrepCwSmem {
-  static constexpr int oK = 0;                           // k as loaded (token-major)
-  static constexpr int oQ = oK + 16384;                  // q as loaded
-  static constexpr int oG = oQ + 16384;                  // g as loaded (four boxes of 32 channels); then alpha
-  static constexpr int oV = oG + 32768;                  // k to the end of its four rows, fp32, 48 rows of 512 bytes (24 KB);
-                                                         // then v, beta v (w v)                token-major
-  static constexpr int oBg = oV + 24576;                 // decays over four rows, fp32 [16][128]
-  static constexpr int oLA = oBg + 8192;                 // (b) k e | q e  [channel][token]; then M (fp32), then P
-  static constexpr int oKR = oLA + 32768;                // k to the start of block 3 | 1, 2; then [w | u]
-  static constexpr int oGK = oKR + 32768;                // b gamma k   [channel][token]; with kd behind it, then R
-  static constexpr int oKD = oGK + 16384;                // k exp(G_last - G)
-  static constexpr int oTA = oKD + 16384;                // scale gamma q (token-major record); then [T; A]
-  static constexpr int oF = oTA + 16384;
+  static constexpr int kTile = 16384, oF = 6 * kTile;
   // floats: diagonal blocks of A and M [64][kDg] each, betas [64], Bb and Af [4][128]
   static constexpr int kFloats = 128 * kDg + 64 + 1024;
   static constexpr int kBytes = oF + kFloats * 4 + static_cast<int>(sizeof(CtaShared)) + 1024;
@@ -86,9 +80,8 @@ __device__ __forceinline__ void ld4_pairs(const unsigned char* src, f2* out) {
 // same 16-byte piece at a time, so the swizzle keeps them off one another's banks.  A kernel of its own reads and writes q and k
 // once more: 84 us of the 1036 us of a forward over 16000 tokens and 32 heads, against 978 us with the rows normalised here.
 enum CwIn { kInBf16, kInF16, kInNorm };
-__device__ __forceinline__ void normalise_rows(unsigned char* tK, unsigned char* tQ, int tid, int f16, float eps) {
-  const int warp = tid >> 5, lane = tid & 31, part = lane >> 3;
-  unsigned char* t = warp < 8 ? tK : tQ;
+__device__ __forceinline__ void normalise_rows(unsigned char* t, int warp, int lane, int f16, float eps) {
+  const int part = lane >> 3;
   const int r = (warp & 7) * 8 + (lane & 7);
   float x[4][8], ss = 0.f;
 #pragma unroll
@@ -108,18 +101,21 @@ __device__ __forceinline__ void normalise_rows(unsigned char* tK, unsigned char*
   }
 }
 
-template <int V, bool DELTA, bool FULL, CwIn IN>
-__global__ void __launch_bounds__(kPrepCwThreads, 1)
+template <int V, bool DELTA, bool FULL, CwIn IN, int NB>
+__global__ void __launch_bounds__(512 / NB, NB)
 prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,
                   const __grid_constant__ CUtensorMap mv, const __grid_constant__ CUtensorMap mg, const __grid_constant__ NormMaps mn) {
   constexpr bool F16 = IN != kInBf16, NORM = IN == kInNorm;      // the type of the tiles once they are here
-  using S = PrepCwSmem<V>;
+  constexpr int kThreads = 512 / NB;
+  using S = PrepCwSmem;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* sm = align1024(smem_raw);
-  unsigned char *tK = sm + S::oK, *tQ = sm + S::oQ, *BV = sm + S::oV, *LA = sm + S::oLA, *KR = sm + S::oKR, *GK = sm + S::oGK;
-  unsigned char *KD = sm + S::oKD, *TA = sm + S::oTA, *WU = KR, *SP = LA, *SR = GK;
-  float *G = reinterpret_cast<float*>(sm + S::oG), *kfd = reinterpret_cast<float*>(sm + S::oV), *Bg = reinterpret_cast<float*>(sm + S::oBg);
-  float* Mt = reinterpret_cast<float*>(LA);
+  auto tile = [&](int i) { return sm + i * S::kTile; };
+  unsigned char *tK = tile(0), *tQ = tile(1), *LA = tile(0), *KR = tile(2), *KD = tile(4), *GK = tile(5);
+  unsigned char *TA = tile(2), *BV = tile(3), *WU = tile(0), *SP = tile(4);
+  float *G = reinterpret_cast<float*>(tile(2)), *kfd = reinterpret_cast<float*>(tile(4)), *Bg = kfd + 48 * kK;
+  float* Mt = reinterpret_cast<float*>(tile(0));
+  static_assert((kInvMtFloats + kInvScratchFloats) * 4 <= 2 * S::kTile, "M and the inverse's scratch");
   float* Adg = reinterpret_cast<float*>(sm + S::oF);
   float* Mdg = Adg + 64 * kDg;
   float* betas = Mdg + 64 * kDg;
@@ -127,7 +123,7 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
   float* Af = Bb + 512;
   CtaShared* cs = reinterpret_cast<CtaShared*>(Af + 512);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, quad = warp & 3, blk = warp >> 2, d = quad * 32 + lane;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, quad = warp & 3, b0 = (warp >> 2) * NB, d = quad * 32 + lane;
   CtaCtl ctl{p.status, &cs->abort_flag};
   uint64_t *in0 = &cs->bar[0], *in1 = &cs->bar[1], *m1 = &cs->bar[2], *m2 = &cs->bar[3], *m3 = &cs->bar[4];
   const int nchunks = p.nbh * p.cn;
@@ -143,7 +139,7 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
   };
   auto load_kqg = [&](const At& a) {      // (tid 0)
     mbar_expect_tx(in0, 65536u);
-    for (int q = 0; q < 4; ++q) tma_load_4d(sm + S::oG + q * 8192, &mg, in0, q * 32, a.h, a.c * kC, a.b);
+    for (int q = 0; q < 4; ++q) tma_load_4d(tile(2) + q * 8192, &mg, in0, q * 32, a.h, a.c * kC, a.b);
     for (int t = 0; t < 2; ++t) {
       tma_load_4d(tK + t * 8192, &mk, in0, t * 64, a.h, a.c * kC, a.b);
       tma_load_4d(tQ + t * 8192, &mq, in0, t * 64, a.h, a.c * kC, a.b);
@@ -161,50 +157,35 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
     load_kqg(at(blockIdx.x));
   }
   if (warp == 0) {
-    tmem_alloc(&cs->tmem_slot, 512);
+    tmem_alloc(&cs->tmem_slot, 256);
     tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = cs->tmem_slot, lane_base = static_cast<uint32_t>(quad * 32) << 16;
-  const uint32_t cMA = tmem, cWU = tmem + 256, cPR = tmem;       // M | A blocks; [w | u]; [P | R]
+  const uint32_t tmem = cs->tmem_slot, lane_base = static_cast<uint32_t>(quad * 32) << 16;      // M | A blocks; [w | u]; [P | R]
 
   uint32_t ph = 0;
   for (int n = blockIdx.x; n < nchunks; n += gridDim.x, ph ^= 1u) {
     const At a = at(n);
     const bool more = n + static_cast<int>(gridDim.x) < nchunks;
-    const At nx = at(more ? n + gridDim.x : n);
     const int rows = p.rows_of(a.c);
     const size_t tok0 = (static_cast<size_t>(a.b) * p.L + a.c * kC) * p.H + a.h;
     float beta_r = 1.f;
     if (DELTA && !FULL && tid < 64) beta_r = tid < rows ? p.beta[tok0 + static_cast<size_t>(tid) * p.H] : 0.f;
 
-    // ---- this thread's column: decays, k, q
-    float al[16];
-    uint32_t kp[8], qp[8];
+    // ---- alphas, in place of g; decays of the blocks
     mbar_wait_warp(in0, ph, ctl, 501);
-    {
-      float B = 1.f;
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        float* gi = G + quad * 2048 + (blk * 16 + i) * 32 + lane;
-        al[i] = exp2f(*gi * kLog2e);
-        *gi = al[i];                       // for the diagonal sums
-        B *= al[i];
-      }
-      Bb[blk * kK + d] = B;
-      Af[blk * kK + d] = al[0];
-    }
     if (NORM) {
-      normalise_rows(tK, tQ, tid, p.qk16, p.l2_eps);
+#pragma unroll
+      for (int w = 0; w < NB; ++w) {
+        const int wq = warp + w * (16 / NB);
+        normalise_rows(wq < 8 ? tK : tQ, wq & 7, lane, p.qk16, p.l2_eps);
+      }
       fence_proxy_async();
-      __syncthreads();
     }
-    read_column(tK, blk, d, F16, kp);
-    read_column(tQ, blk, d, F16, qp);
     if (DELTA && tid < 64) betas[tid] = beta_r;
-    if (tid == 0) bulk_wait_read();        // the chunk before has left its staging tiles
+    if (tid == 0) bulk_wait_read();        // the chunk before has left tiles 4 and 5
     __syncthreads();
     if (NORM && tid == 0 && p.keep_norm) {
       for (int t = 0; t < p.Kr / 64; ++t) {
@@ -213,85 +194,37 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
       }
       bulk_commit();
     }
-    const BlockDecays bd = block_decays(Bb, Af, blk, d);
-    const float gam0 = bd.pre * al[0];     // gamma of the block's first token
-    if (blk == 3) reinterpret_cast<float*>(p.saved + p.lay.ad)[static_cast<size_t>(a.z) * kK + d] = bd.pre * Bb[3 * kK + d];
-    auto kv = [&](int i) { return half_of(kp[i >> 1], i & 1); };
-    auto qv = [&](int i) { return half_of(qp[i >> 1], i & 1); };
-    // ---- operand tiles
-    {
-      float x[16], y[16], f = 1.f, e = 1.f;
+#pragma unroll 1
+    for (int blk = b0; blk < b0 + NB; ++blk) {
+      float al[16], B = 1.f;
+      uint32_t kp[8];
+      read_column(tK, blk, d, F16, kp);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        float* gi = G + quad * 2048 + (blk * 16 + i) * 32 + lane;
+        al[i] = exp2f(*gi * kLog2e);
+        *gi = al[i];
+      }
 #pragma unroll
       for (int A = 0; A < 4; ++A) {        // decays over four rows, and k to the end of its four
-        f = 1.f;
+        float f = 1.f;
 #pragma unroll
         for (int i = 4 * A + 3; i >= 4 * A; --i) {
-          x[i] = kv(i) * f;
-          if (A < 3) kfd[(blk * 12 + i) * kK + d] = x[i];
+          if (A < 3) kfd[(blk * 12 + i) * kK + d] = half_of(kp[i >> 1], i & 1) * f;
           f *= al[i];
         }
         Bg[(blk * 4 + A) * kK + d] = f;
-        y[A] = f;
+        B *= f;
       }
-      f = 1.f;
-#pragma unroll
-      for (int A = 3; A >= 0; --A) {       // k to the end of its block
-#pragma unroll
-        for (int i = 4 * A; i < 4 * A + 4; ++i) x[i] *= f;
-        f *= y[A];
-      }
-#pragma unroll
-      for (int i = 0; i < 16; ++i) y[i] = x[i] * bd.post;
-      write_column(KD, blk, d, y);
-#pragma unroll
-      for (int I = 1; I < 4; ++I) {        // ... and on to the start of every later block
-        if (I <= blk) continue;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) y[i] = x[i] * bd.cup[I - 1];
-        // columns: block 3's 48 and block 1's 16 in the first atom, block 2's 32 in the second
-        unsigned char* t = KR + (I == 2 ? 16384 : 0);
-        write_column(t, I == 1 ? 3 : blk, d, y);
-      }
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        if (i) e *= al[i];
-        y[i] = qv(i) * e;
-        stage16(TA, blk * 16 + i, d, y[i] * (p.scale * gam0), 1);
-      }
-      write_column(LA + 16384, blk, d, y);
-      e = 1.f;
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        if (i) e *= al[i];
-        x[i] = kv(i) * e;
-        if (FULL) x[i] *= p.bch[(tok0 + static_cast<size_t>(blk * 16 + i) * p.H) * kK + d];
-      }
-      write_column(LA, blk, d, x);         // left factor of M (without the row's beta)
-      if (DELTA) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) x[i] *= FULL ? gam0 : gam0 * betas[blk * 16 + i];
-        write_column(GK, blk, d, x);
-      }
+      Bb[blk * kK + d] = B;
+      Af[blk * kK + d] = al[0];
     }
-    sync_for_issue();
-
-    // ---- off-diagonal blocks of M (rows 0-63) and A (rows 64-127) on the tensor cores
-    if (warp == 0) {
-      tc_fence_after();
-      const uint32_t leader = elect_leader();
-      issue_product_led(leader, cMA, Tile{smem_u32(LA), 128, true}, Tile{smem_u32(KR), 128, true}, 64, 128, 0u);
-      issue_product_led(leader, cMA + 64, Tile{smem_u32(LA), 128, true}, Tile{smem_u32(KR) + 16384, 128, true}, 32, 128, 0u);
-      umma_commit_led(leader, m1);
-      if (tid == 0) {
-        bulk_s2g(p.saved + p.lay.qg + static_cast<size_t>(a.z) * 16384, TA, 16384);
-        bulk_commit();
-      }
-    }
-    __syncwarp();
+    __syncthreads();
     // ---- diagonal blocks, exact.  Half-warp (block, j): rows j and 15 - j - 17 pairs for every j, 5 of them inside the
     // rows' own groups and 3 x 4 with earlier groups; lane: channels 4 c .. 4 c + 3 of either half.
-    {
-      const int c = lane & 15, j = warp & 7, db = (warp >> 3) * 2 + (lane >> 4);
+#pragma unroll 1
+    for (int it = 0; it < NB; ++it) {
+      const int c = lane & 15, j = warp & 7, db = (NB == 1 ? warp >> 3 : it) * 2 + (lane >> 4);
       const float* al0 = G + (c >> 3) * 2048 + 4 * (c & 7);        // alpha of row r: + 32 r; the other half: + 4096
       const unsigned char* kt = tK + (c & 1) * 8;
       const unsigned char* qt = tQ + (c & 1) * 8;
@@ -395,16 +328,83 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
         store(j < 4 ? i0 : i1, (c >> 1) & 3, (c & 8) != 0, t);
       }
     }
-    fence_proxy_async();
-    if (tid == 0) bulk_wait_read();        // the query record has left the [T; A] tile, which the epilogue now fills
-    __syncthreads();
-    if (tid == 0) {                        // k, q, alpha and the decayed rows of this chunk are read
-      load_v(a);
-      if (more) load_kqg(nx);
+    // ---- this thread's columns: decays, k, q
+    float al[NB][16];
+    uint32_t kp[NB][8], qp[NB][8];
+#pragma unroll
+    for (int bb = 0; bb < NB; ++bb) {
+      read_column(tK, b0 + bb, d, F16, kp[bb]);
+      read_column(tQ, b0 + bb, d, F16, qp[bb]);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) al[bb][i] = G[quad * 2048 + ((b0 + bb) * 16 + i) * 32 + lane];
     }
+    if (NORM && tid == 0) bulk_wait_read();      // the normalised rows have left
+    __syncthreads();                             // k, q, alpha and the decayed rows are read: their tiles become operands
+    // ---- operand tiles
+#pragma unroll
+    for (int bb = 0; bb < NB; ++bb) {
+      const int blk = b0 + bb;
+      const BlockDecays bd = block_decays(Bb, Af, blk, d);
+      const float gam0 = bd.pre * al[bb][0];     // gamma of the block's first token
+      if (blk == 3) reinterpret_cast<float*>(p.saved + p.lay.ad)[static_cast<size_t>(a.z) * kK + d] = bd.pre * Bb[3 * kK + d];
+      float x[16], y[16], f = 1.f, e = 1.f;
+#pragma unroll
+      for (int i = 15; i >= 0; --i) {            // k to the end of its block ...
+        x[i] = half_of(kp[bb][i >> 1], i & 1) * f;
+        f *= al[bb][i];
+      }
+#pragma unroll
+      for (int i = 0; i < 16; ++i) y[i] = x[i] * bd.post;
+      write_column(KD, blk, d, y);
+#pragma unroll
+      for (int I = 1; I < 4; ++I) {              // ... and on to the start of every later block
+        if (I <= blk) continue;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) y[i] = x[i] * bd.cup[I - 1];
+        // columns: block 3's 48 and block 1's 16 in the first atom, block 2's 32 in the second
+        unsigned char* t = KR + (I == 2 ? 16384 : 0);
+        write_column(t, I == 1 ? 3 : blk, d, y);
+      }
+      // scale gamma q leaves for its record, the image of a [64 tokens][128 channels] tile: a warp writes 64 bytes of a row
+      unsigned char* qg = p.saved + p.lay.qg + static_cast<size_t>(a.z) * 16384;
+      const float sg = p.scale * gam0;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        if (i) e *= al[bb][i];
+        y[i] = half_of(qp[bb][i >> 1], i & 1) * e;
+        store_f16_sat(qg + sw128_off(blk * 16 + i, d, 64), y[i] * sg);
+      }
+      write_column(LA + 16384, blk, d, y);
+      if (DELTA) {
+        e = 1.f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          if (i) e *= al[bb][i];
+          x[i] = half_of(kp[bb][i >> 1], i & 1) * e;
+          if (FULL) x[i] *= p.bch[(tok0 + static_cast<size_t>(blk * 16 + i) * p.H) * kK + d];
+        }
+        write_column(LA, blk, d, x);             // left factor of M (without the row's beta)
+#pragma unroll
+        for (int i = 0; i < 16; ++i) x[i] *= FULL ? gam0 : gam0 * betas[blk * 16 + i];
+        write_column(GK, blk, d, x);
+      }
+    }
+    sync_for_issue();
+
+    // ---- off-diagonal blocks of M (rows 0-63) and A (rows 64-127) on the tensor cores
+    if (warp == 0) {
+      tc_fence_after();
+      const uint32_t leader = elect_leader();
+      issue_product_led(leader, tmem, Tile{smem_u32(LA), 128, true}, Tile{smem_u32(KR), 128, true}, 64, 128, 0u);
+      issue_product_led(leader, tmem + 64, Tile{smem_u32(LA), 128, true}, Tile{smem_u32(KR) + 16384, 128, true}, 32, 128, 0u);
+      umma_commit_led(leader, m1);
+    }
+    __syncwarp();
     mbar_wait_warp(m1, ph, ctl, 502);
     tc_fence_after();
-    {
+    if (tid == 0) load_v(a);
+#pragma unroll 1
+    for (int blk = b0; blk < b0 + NB; ++blk) {
       // thread: accumulator lane t = quad * 32 + lane (row r of M for lanes 0-63, of A for 64-127), columns of block blk
       const int t = d, r = t & 63, I = r >> 4, I0 = 2 * (quad & 1);      // a warp's lanes are rows of blocks I0 and I0 + 1
       float x[16], y[16];
@@ -412,14 +412,14 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
       for (int e = 0; e < 16; ++e) x[e] = 0.f;
       auto col = [](int rb, int cb) { return rb == 1 ? 48 : (rb == 2 ? 64 : 0) + 16 * cb; };
       if (blk < I0 + 1) {
-        tmem_ld16(cMA + lane_base + col(I0 + 1, blk), y);
+        tmem_ld16(tmem + lane_base + col(I0 + 1, blk), y);
         tmem_ld_wait();
         if (I == I0 + 1)
 #pragma unroll
           for (int e = 0; e < 16; ++e) x[e] = y[e];
       }
       if (blk < I0) {
-        tmem_ld16(cMA + lane_base + col(I0, blk), y);
+        tmem_ld16(tmem + lane_base + col(I0, blk), y);
         tmem_ld_wait();
         if (I == I0)
 #pragma unroll
@@ -448,10 +448,11 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
     tc_fence_before();
     __syncthreads();
 
-    // ---- beta v (w v) on the warps that have no part in the inverse
-    if (tid >= 256) {
+    // ---- beta v (w v) on the warps that have no part in the inverse, or not in its first step
+    constexpr int kFirst = NB == 1 ? 256 : 64;
+    if (tid >= kFirst) {
       mbar_wait_warp(in1, ph, ctl, 505);
-      for (int idx = tid - 256; idx < 64 * (V / 8); idx += kPrepCwThreads - 256) {
+      for (int idx = tid - kFirst; idx < 64 * (V / 8); idx += kThreads - kFirst) {
         const int r = idx / (V / 8), ch = idx % (V / 8);
         float x[8];
         unpack8_bf16(tile_ld_chunk(BV, r, ch, 64), x);
@@ -476,8 +477,8 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
       if (warp == 0) {
         tc_fence_after();
         const uint32_t leader = elect_leader();
-        issue_product_led(leader, cWU, Tile{smem_u32(TA), 128, false}, Tile{smem_u32(GK), 128, false}, 128, 64, 0u);
-        issue_product_led(leader, cWU + 128, Tile{smem_u32(TA), 128, false}, Tile{smem_u32(BV), 64, true}, V, 64, 0u);
+        issue_product_led(leader, tmem, Tile{smem_u32(TA), 128, false}, Tile{smem_u32(GK), 128, false}, 128, 64, 0u);
+        issue_product_led(leader, tmem + 128, Tile{smem_u32(TA), 128, false}, Tile{smem_u32(BV), 64, true}, V, 64, 0u);
         umma_commit_led(leader, m2);
         if (tid == 0) {
           if (p.lean < 2) bulk_s2g(p.saved + p.lay.ta + static_cast<size_t>(a.z) * p.lay.sz_ta, TA, 16384);
@@ -488,10 +489,11 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
       __syncwarp();
       mbar_wait_warp(m2, ph, ctl, 503);
       tc_fence_after();
-      if (quad < 2) {                      // rows 0-63; the four warps of a quadrant split the columns
-        for (int jb = blk; jb < (128 + V) / 32; jb += 4) {
+      if (quad < 2) {                      // rows 0-63; the warps of a quadrant split the columns
+#pragma unroll 1
+        for (int jb = warp >> 2; jb < (128 + V) / 32; jb += 4 / NB) {
           float x[32];
-          tmem_ld32(cWU + lane_base + jb * 32, x);
+          tmem_ld32(tmem + lane_base + jb * 32, x);
           tmem_ld_wait();
 #pragma unroll
           for (int i = 0; i < 4; ++i) tile_st_chunk(WU, d, jb * 4 + i, 64, pack8_f16(x + 8 * i));
@@ -511,7 +513,7 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
     if (warp == 0) {
       tc_fence_after();
       const uint32_t leader = elect_leader();
-      issue_product_led(leader, cPR, Tile{smem_u32(KD), 128, false}, Tile{smem_u32(DELTA ? WU : BV), 64, true}, DELTA ? 128 + V : V, 64, 0u);
+      issue_product_led(leader, tmem, Tile{smem_u32(KD), 128, false}, Tile{smem_u32(DELTA ? WU : BV), 64, true}, DELTA ? 128 + V : V, 64, 0u);
       umma_commit_led(leader, m3);
       if (tid == 0) {
         if (DELTA) {
@@ -526,22 +528,25 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
     __syncwarp();
     mbar_wait_warp(m3, ph, ctl, 504);
     tc_fence_after();
-    // P and R leave as their record images through tiles nothing reads any more; the four warps of a lane quadrant split
-    // the columns
-    for (int jb = blk; jb < (DELTA ? 128 + V : V) / 32; jb += 4) {
+    if (tid == 0 && more) {                // tiles 0 to 3 are dead once their records have left
+      bulk_wait_read();
+      load_kqg(at(n + gridDim.x));
+    }
+    // P leaves as its record image through the tiles of the last operands, R (16 columns of a row are 32 bytes of its record,
+    // the rows of a warp 1 KB) directly; the warps of a lane quadrant split the columns
+    unsigned char* r_g = p.saved + p.lay.r + static_cast<size_t>(a.z) * p.lay.sz_r;
+#pragma unroll 1
+    for (int jb = warp >> 2; jb < (DELTA ? 128 + V : V) / 32; jb += 4 / NB) {
       float x[32];
-      tmem_ld32(cPR + lane_base + jb * 32, x);
+      tmem_ld32(tmem + lane_base + jb * 32, x);
       tmem_ld_wait();
-      if (DELTA && jb < 4) {
+      if (!DELTA || jb < 4) {              // P; R without the delta term, a plain tile image
 #pragma unroll
         for (int i = 0; i < 4; ++i) tile_st_chunk(SP, d, jb * 4 + i, 128, pack8_f16(x + 8 * i));
       } else {
-        const int c8 = (jb - (DELTA ? 4 : 0)) * 4;
+        const int c8 = (jb - 4) * 4;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          if (DELTA) *reinterpret_cast<uint4*>(SR + rrec_off(d, c8 + i)) = pack8_f16(x + 8 * i);
-          else tile_st_chunk(SR, d, c8 + i, 128, pack8_f16(x + 8 * i));      // no delta term: plain tile image
-        }
+        for (int i = 0; i < 4; i += 2) st_global_32(r_g + rrec_off(d, c8 + i), pack8_f16(x + 8 * i), pack8_f16(x + 8 * i + 8));
       }
     }
     fence_proxy_async();
@@ -549,28 +554,36 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
     __syncthreads();
     if (tid == 0) {
       if (DELTA) bulk_s2g(p.saved + p.lay.p + static_cast<size_t>(a.z) * p.lay.sz_p, SP, 32768);
-      bulk_s2g(p.saved + p.lay.r + static_cast<size_t>(a.z) * p.lay.sz_r, SR, V * 256);
+      else bulk_s2g(r_g, SP, V * 256);
       bulk_commit();
     }
   }
   if (tid == 0) bulk_wait_read();
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, 512);
+  if (warp == 0) tmem_dealloc(tmem, 256);
 }
 
+template <int V, bool DELTA, bool FULL, CwIn IN, int NB>
+static int launch_prepare_cw_n(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
+                               const CUtensorMap& mg, const NormMaps& mn, int sms, cudaStream_t st) {
+  constexpr int smem = PrepCwSmem::kBytes;
+  static_assert(2 * (smem + 1024) <= 228 * 1024, "two CTAs per SM");
+  auto kern = prepare_cw_kernel<V, DELTA, FULL, IN, NB>;
+  static SmemAttr attr;
+  if (attr.set(kern, smem)) return kErrLaunch;
+  const int n = p.nbh * p.cn, most = NB * sms;
+  kern<<<n < most ? n : most, 512 / NB, smem, st>>>(p, mq, mk, mv, mg, mn);
+  return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
+}
 template <int V, bool DELTA, bool FULL, CwIn IN>
 static int launch_prepare_cw_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                                const CUtensorMap& mg, const NormMaps& mn, cudaStream_t st) {
-  constexpr int smem = PrepCwSmem<V>::kBytes;
-  static_assert(smem <= 232448, "227 KB per CTA");
-  auto kern = prepare_cw_kernel<V, DELTA, FULL, IN>;
-  static SmemAttr attr;
-  if (attr.set(kern, smem)) return kErrLaunch;
-  const int sms = sm_count(), n = p.nbh * p.cn;
+  const int sms = sm_count();
   if (sms <= 0) return kErrDevice;
-  kern<<<n < sms ? n : sms, kPrepCwThreads, smem, st>>>(p, mq, mk, mv, mg, mn);
-  return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
+  // (the line between the two: see NB above)
+  return p.nbh * p.cn <= sms ? launch_prepare_cw_n<V, DELTA, FULL, IN, 1>(p, mq, mk, mv, mg, mn, sms, st)
+                             : launch_prepare_cw_n<V, DELTA, FULL, IN, 2>(p, mq, mk, mv, mg, mn, sms, st);
 }
 template <int V, bool DELTA, bool FULL>
 static int launch_prepare_cw_f(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,

@@ -40,6 +40,9 @@ def test_decode_of_many_pairs(gate, delta, dtype, extra, shift):
     ("scalar", False, 64, 64, 450, 100, torch.bfloat16), ("none", False, 128, 128, 310, 128, torch.float16),
     ("channel", True, 128, 128, 155, 100, torch.bfloat16), ("channel", True, 64, 64, 155, 128, torch.float16),
     ("channel", False, 64, 128, 155, 100, torch.bfloat16),
+    # channel-wise prepare: one chunk per SM for the last time, two CTAs per SM for the first
+    ("channel", True, 128, 128, 148, 64, torch.bfloat16), ("channel", True, 64, 64, 149, 60, torch.float16),
+    ("channel", False, 128, 128, 149, 64, torch.bfloat16),
     # state scans: 16 columns per CTA for the last time, 64 for the first; without the delta term 16 and 8 records ahead
     ("scalar", True, 64, 128, 37, 320, torch.bfloat16), ("scalar", True, 64, 128, 38, 320, torch.bfloat16),
     ("none", False, 64, 128, 74, 1088, torch.bfloat16), ("none", False, 64, 128, 75, 1088, torch.bfloat16)])
