@@ -41,12 +41,12 @@ static int token_map(CUtensorMap* m, const void* ptr, const Problem& p, int D) {
   return make_tmap_16bit(m, ptr, 4, dims, str, box);
 }
 
-// Tensor map of the channel-wise gate [B, L, H, K] in fp32; one box = 64 tokens x 32 channels of one head.
+// Tensor map of the channel-wise gate [B, L, H, K] in fp32; one box = 64 tokens x 128 channels of one head.
 static int gate_map(CUtensorMap* m, const void* ptr, const Problem& p) {
   const uint64_t K = static_cast<uint64_t>(p.Kr), H = static_cast<uint64_t>(p.H), L = static_cast<uint64_t>(p.L);
   uint64_t dims[4] = {K, H, L, static_cast<uint64_t>(p.B)};
   uint64_t str[3] = {K * 4, H * K * 4, L * H * K * 4};
-  uint32_t box[4] = {32, 1, 64, 1};
+  uint32_t box[4] = {kK, 1, 64, 1};
   return make_tmap_f32(m, ptr, 4, dims, str, box);
 }
 

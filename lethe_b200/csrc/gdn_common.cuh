@@ -186,6 +186,11 @@ __device__ __forceinline__ f2 mul2(f2 a, f2 b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.u) : "l"(a.u), "l"(b.u));
   return r;
 }
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.u) : "l"(a.u), "l"(b.u));
+  return r;
+}
 __device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
   f2 r;
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.u) : "l"(a.u), "l"(b.u), "l"(c.u));
@@ -219,6 +224,13 @@ __device__ __forceinline__ void st_global_32(unsigned char* dst, const uint4& a,
                "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
                : "memory");
 }
+
+// Four bytes of global memory to shared memory behind this thread's back, or zero.
+__device__ __forceinline__ void async_copy4(float* dst, const float* src, bool valid) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(valid ? 4 : 0) : "memory");
+}
+__device__ __forceinline__ void async_copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // With the delta term the scan's input records R / Rb (128 rows x V columns, fp16) are stored as V / 16 column blocks of
 // [128 rows][16 columns]: one contiguous 4 KB block per scan CTA, 32 bytes per thread.  Byte offset of

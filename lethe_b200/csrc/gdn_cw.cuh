@@ -38,6 +38,20 @@ __device__ __forceinline__ void stage16(unsigned char* tile, int r, int d, float
       f16 ? static_cast<uint16_t>(f16x2_sat(x, 0.f)) : __bfloat16_as_ushort(__float2bfloat16_rn(x));
 }
 
+// two such results, of tokens r and r + 1
+__device__ __forceinline__ void stage16_two(unsigned char* tile, int r, int d, f2 x, int f16) {
+  float lo, hi;
+  unpack2(x, lo, hi);
+  const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
+  const uint32_t u = f16 ? f16x2_sat(lo, hi) : *reinterpret_cast<const uint32_t*>(&b);
+  *reinterpret_cast<uint16_t*>(tile + sw128_off(r, d, 64)) = static_cast<uint16_t>(u);
+  *reinterpret_cast<uint16_t*>(tile + sw128_off(r + 1, d, 64)) = static_cast<uint16_t>(u >> 16);
+}
+__device__ __forceinline__ f2 pair_of(uint32_t halves) {
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&halves));
+  return pack2(f.x, f.y);
+}
+
 // 16 columns of block blk of row r of a [token][token] tile (128-byte rows)
 __device__ __forceinline__ void write_row16(unsigned char* tile, int r, int blk, const float* x) {
   *reinterpret_cast<uint4*>(tile + sw128_chunk(r, 2 * blk, 64)) = pack8_f16(x);
@@ -58,6 +72,23 @@ __device__ __forceinline__ float warp_sum8(float* v, int lane) {
   }
   v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
   v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+  return v[0];
+}
+
+// The same of four values: lane l ends up with the total of value (l >> 3).
+__device__ __forceinline__ float warp_sum4(float* v, int lane) {
+#pragma unroll
+  for (int w = 2, o = 16; w >= 1; w >>= 1, o >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int j = 0; j < w; ++j) {
+      const float send = up ? v[j] : v[j + w];
+      const float keep = up ? v[j + w] : v[j];
+      v[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+#pragma unroll
+  for (int o = 4; o >= 1; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
   return v[0];
 }
 
@@ -89,6 +120,19 @@ __device__ __forceinline__ BlockDecays block_decays(const float* Bb, const float
       if (m > blk) r.cup[J] *= bm[m];
   }
   return r;
+}
+
+// Where the n-th chunk of a call is: record index, and batch, head and chunk in the user's tensors.  One thread works it out
+// (divisions) and leaves it in shared memory for the others.
+struct __align__(16) ChunkAt { int z, b, h, c; };
+__device__ __forceinline__ ChunkAt chunk_at(const Problem& p, int n) {
+  const int q = n / p.cn, bh = p.bh0 + q;
+  ChunkAt a;
+  a.c = p.c0 + n - q * p.cn;
+  a.z = bh * p.NT + a.c;
+  a.b = bh / p.H;
+  a.h = bh - a.b * p.H;
+  return a;
 }
 
 }  // namespace lg

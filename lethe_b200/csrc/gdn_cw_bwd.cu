@@ -3,8 +3,8 @@
 // ratio(i, s)[d] the decay of channel d from token s to token i:
 //
 //   dv2  = kd dh + A^T do                         dA = do v_new^T,  C0 = scale tril(dA)
-//   dw   = -dv2 h^T                               dT = dv2 (w v)^T + dw (b gamma k)^T,  C1 = dM = strict_lower(-T^T dT T^T)
-//   dbv  = T^T dv2,  dbgk = T^T dw
+//   dw   = -dv2 h^T                               dbv = T^T dv2,  dbgk = T^T dw
+//   C1 = dM = strict_lower(-(dbv u^T + dbgk w^T)),  u = T (w v), w = T (b gamma k)       (the forward's WY factors)
 //   out1_c[i,d] = sum_{s<=i} C_c[i,s] k[s,d] ratio(i,s)[d]
 //   out2[s,d]   = sum_{i>=s} (C0[i,s] q[i,d] + C1[i,s] (b k)[i,d]) ratio(i,s)[d]
 //   dq = scale gamma (do h^T) + out1_0            dbk = gamma dbgk + out1_1
@@ -30,14 +30,20 @@
 // exact fp32 recurrences: going down the rows, k[s] ratio(i,s) is multiplied by alpha_i per row; going up, the column
 // sums are (Horner).  No exponentials, one packed multiply and two packed FMAs per two pairs and sum.
 //
-// What bounds it: 272 KB of traffic per chunk (12 k cycles of an SM's share of HBM) against the chain of six dependent
-// product groups plus CUDA-core phases.  The CTA is persistent and fetches the next chunk's tiles into the ones that
-// are dead once its last products are issued, under the longest CUDA-core phase.  8192 chunks, d_v = 128: 915 us; the four
-// kernels that this replaced (Stage B 1, pair sums, WY 1, pair sums; 887 KB of traffic per chunk) took 2489.
-// Cycles per chunk by clock samples of one CTA (d_v = 128): operand columns and waits for the tiles 5.1 k, group 1 and its
-// epilogues 4.2 k, the four dependent groups from dw to dM 6.3 k, column sums with the decay assembly 5.3 k, row sums with
-// the gradients 5.3 k, gate gradient and stores 2.4 k; 28.6 k in all.  Without the delta term 6.5, 3.9, 0, 3.7, 2.5, 1.9:
-// 18.5 k; with per-channel gates 10.8, 4.6, 12.9, 6.1, 7.0, 1.8: 43.3 k.
+// dM.  The VJP of the inverse is -T^T dT T^T with dT = dv2 (w v)^T + dw (b gamma k)^T; since T^T dv2 = dbv, T^T dw = dbgk, T (w v)
+// = u and T (b gamma k) = w, that is -(dbv u^T + dbgk w^T): one product behind dbv and dbgk, which are wanted anyway, instead of
+// three in a row, for 32 KB more to read per chunk.
+//
+// What bounds it: the chain of four dependent product groups and the CUDA-core phases (issue slots 43 % busy); 300 KB of traffic
+// per chunk are 12 k cycles of an SM's share of HBM.  The CTA is persistent and fetches the next chunk's tiles into the ones that
+// are dead once its last products are issued, under the longest CUDA-core phase.  Inside a group the products that the chain waits
+// for are issued first and the rest of the epilogue before lies in the next group's shadow.
+// us at d_v = 128, before (dT, X = dT T^T and dM as three groups, 100 bytes of registers a thread in local memory, all copies
+// issued by one thread, beta and the per-channel gates read when they were needed) and now: 8192 chunks 920 -> 789; 4096 without the
+// delta term 301 -> 267; 512 with per-channel gates 113 -> 79.
+// Cycles per chunk by clock samples of one CTA (d_v = 128): operand columns and waits for the tiles 4.9 k, group 1 2.5 k, the rest
+// up to dM 7.0 k, column sums with the decay assembly 5.0 k, row sums with the gradients 5.6 k, gate gradient and stores 2.2 k; 27.1 k
+// in all.  Without the delta term 5.1, 3.1, 0.6, 3.5, 2.8, 1.7: 16.8 k; with per-channel gates 30.9 k.
 #include "gdn_cw.cuh"
 #include "host_util.h"
 
@@ -46,7 +52,7 @@ namespace lg {
 constexpr int kCwThreads = 512;
 
 struct CwBars {
-  uint64_t in0, in1, mA, mB, mW, mT, mV, mX, mM, mO;
+  uint64_t in0, in1, inU, mA, mB, mW, mV, mX, mO;
   uint32_t tmem_slot;
   int abort_flag;
 };
@@ -68,19 +74,19 @@ struct CwSmem {
   static constexpr int kVT = V * 128;                    // a [64 tokens][V] or [V][64 tokens] tile
   static constexpr int oK = 0;                           // k as loaded; then k f            [channel][token]
   static constexpr int oQ = oK + 16384;                  // q as loaded; then q e
-  static constexpr int oV = oQ + 16384;                  // v (times w; without delta: v_new)  token-major
-  static constexpr int oG = oV + kVT;                    // g as loaded (32 KB); then kd | gamma k, then dw | ...
+  static constexpr int oV = oQ + 16384;                  // v (without delta: v_new)         token-major
+  static constexpr int oG = oV + kVT;                    // g as loaded (32 KB); then kd, then dw | WY factor w
   static constexpr int oDO = oG + 32768;                 // do                               token-major
   static constexpr int oDV = oDO + kVT;                  // dv2  [value channel][token]; then dv on its way out
   static constexpr int oTA = oDV + kVT;                  // [T; A]
   static constexpr int oC = oTA + 16384;                 // v_new; then C0 / C1 by row block; then dq on its way out
-  static constexpr int oH = oC + 16384;                  // h; then, 32 KB from here, dg on its way out
-  static constexpr int oDH = oH + 32768;                 // dh; then (b k) e (16 KB), dT / X (8 KB); then dk on its way out
-  static constexpr int kDH = V * 256 > 24576 ? V * 256 : 24576;
+  static constexpr int oH = oC + 16384;                  // h; then T^T dw, T^T dv2 [channel][token]; then dg on its way out
+  static constexpr int oDH = oH + 32768;                 // dh; then (b k) e (16 KB), WY factor u; then dk on its way out
+  static constexpr int kDH = 16384 + kVT;
   static constexpr int oCd = oDH + kDH;                  // diagonal blocks of C0, C1 in fp32: [2][64][16]
-  static constexpr int oF = oCd + 8192;                  // floats: Bb [4][128], Af [4][128], S [4][128], red [2][4][64], betas [64]
-  static constexpr int kFloats = 3 * 512 + 512 + 64;
-  static constexpr int kBytes = oF + kFloats * 4 + static_cast<int>(sizeof(CwBars)) + 1024;
+  static constexpr int oF = oCd + 8192;                  // floats: Bb [4][128], Af [4][128], Et [4][128], red [2][4][64], betas [2][64]
+  static constexpr int kFloats = 3 * 512 + 512 + 128;
+  static constexpr int kBytes = oF + kFloats * 4 + static_cast<int>(sizeof(CwBars)) + 2 * static_cast<int>(sizeof(ChunkAt)) + 1024;
   static constexpr int CR = WY ? 32 : 16;        // rows of the C tile per row block
 };
 
@@ -97,77 +103,67 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
   constexpr int CR = S::CR;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* sm = align1024(smem_raw);
-  unsigned char *tK = sm + S::oK, *tQ = sm + S::oQ, *tV = sm + S::oV, *tKD = sm + S::oG, *tGK = sm + S::oG + 16384;
+  unsigned char *tK = sm + S::oK, *tQ = sm + S::oQ, *tV = sm + S::oV, *tKD = sm + S::oG, *tW = sm + S::oG + 16384;
   unsigned char *tDW = tKD, *tDO = sm + S::oDO, *tDV = sm + S::oDV, *tTA = sm + S::oTA, *tVN = sm + (DELTA ? S::oC : S::oV), *tC = sm + S::oC;
   unsigned char *oQt = tC, *oKt = sm + S::oDH, *oVt = tDV;
   float* oGt = reinterpret_cast<float*>(sm + S::oH);
-  unsigned char *tH = sm + S::oH, *tDH = sm + S::oDH, *tBE = sm + S::oDH, *tDT = sm + S::oDH + 16384;
+  unsigned char *tH = sm + S::oH, *tDH = sm + S::oDH, *tBE = sm + S::oDH, *tU = sm + S::oDH + 16384;
+  unsigned char *tBK = tH, *tBV = tH + 16384;
   const float* G = reinterpret_cast<const float*>(sm + S::oG);
   float* Cd0 = reinterpret_cast<float*>(sm + S::oCd);
   float* Cd1 = Cd0 + 1024;
-  float* Bb = reinterpret_cast<float*>(sm + S::oF);      // products of a block's alphas; later the end terms
+  float* Bb = reinterpret_cast<float*>(sm + S::oF);      // products of a block's alphas
   float* Af = Bb + 512;                                  // first alpha of a block
-  float* St = Af + 512;                                  // gate-gradient totals of a block
-  float* red = St + 512;
-  float* betas = red + 512;
-  CwBars* bars = reinterpret_cast<CwBars*>(betas + 64);
+  float* Et = Af + 512;                                  // a block's part of the end term
+  float* St = reinterpret_cast<float*>(tU);              // gate-gradient totals of a block, once u is dead
+  float* red = Et + 512;
+  float* betas2 = red + 512;                             // of this chunk and the next
+  ChunkAt* where = reinterpret_cast<ChunkAt*>(betas2 + 128);      // this chunk and the next
+  CwBars* bars = reinterpret_cast<CwBars*>(where + 2);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, quad = warp & 3, blk = warp >> 2, d = quad * 32 + lane;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, quad = warp & 3, blk = warp >> 2;
   CtaCtl ctl{p.status, &bars->abort_flag};
   const int nchunks = p.nbh * p.cn;
-  struct At { int bh, c, z, b, h; };
-  auto at = [&](int n) {
-    At a;
-    a.bh = p.bh0 + n / p.cn;
-    a.c = p.c0 + n % p.cn;
-    a.z = a.bh * p.NT + a.c;
-    a.b = a.bh / p.H;
-    a.h = a.bh % p.H;
-    return a;
-  };
-  // The loads of a chunk, in three parts by when their destinations are free in the chunk before (tid 0 only).
-  auto load_part1 = [&](const At& a) {
-    mbar_expect_tx(&bars->in0, 32768u + 16384u + 16384u);
-    for (int q = 0; q < 4; ++q) tma_load_4d(sm + S::oG + q * 8192, &mg, &bars->in0, q * 32, a.h, a.c * kC, a.b);
-    mbar_expect_tx(&bars->in1, (SB ? 2u * V * 128 + 2u * V * 256 : 0u) + (DELTA ? 16384u : 8192u) + (WY ? V * 128u : 0u));
-    if (WY || !DELTA) for (int t = 0; t < V / 64; ++t) tma_load_4d(tV + t * 8192, &mv, &bars->in1, t * 64, a.h, a.c * kC, a.b);
-    if (DELTA) bulk_g2s(tTA, p.saved + p.lay.ta + static_cast<size_t>(a.z) * 16384, 16384, &bars->in1);
-    else bulk_g2s(tTA + 8192, p.saved + p.lay.ta + static_cast<size_t>(a.z) * 16384 + 8192, 8192, &bars->in1);
-    if (SB) {
-      for (int t = 0; t < V / 64; ++t) tma_load_4d(tDO + t * 8192, &mdo, &bars->in1, t * 64, a.h, a.c * kC, a.b);
+  // The loads of a chunk, in parts by when their destinations are free in the chunk before, and its stores are shared by four
+  // threads, the first of every block's warps: one thread would issue for some 1 k cycles while the others wait for it.  A tile
+  // that a store reads is loaded by the thread that issued the store.
+  const bool lead = (warp & 3) == 0 && lane == 0;
+  auto load_part1 = [&](const ChunkAt& a) {
+    const int l0 = a.c * kC;
+    if (blk == 0) {
+      mbar_expect_tx(&bars->in0, 32768u + 16384u + 16384u);
+      mbar_expect_tx(&bars->in1, (SB ? 2u * V * 128 + 2u * V * 256 : 0u) + (DELTA ? 16384u : 8192u) + (WY ? V * 128u : 0u));
+      tma_load_4d(sm + S::oG, &mg, &bars->in0, 0, a.h, l0, a.b);
+    } else if (blk == 1) {
+      if (WY || !DELTA) for (int t = 0; t < V / 64; ++t) tma_load_4d(tV + t * 8192, &mv, &bars->in1, t * 64, a.h, l0, a.b);
+    } else if (blk == 2) {
+      if (DELTA) bulk_g2s(tTA, p.saved + p.lay.ta + static_cast<size_t>(a.z) * 16384, 16384, &bars->in1);
+      else bulk_g2s(tTA + 8192, p.saved + p.lay.ta + static_cast<size_t>(a.z) * 16384 + 8192, 8192, &bars->in1);
+    } else if (SB) {
+      for (int t = 0; t < V / 64; ++t) tma_load_4d(tDO + t * 8192, &mdo, &bars->in1, t * 64, a.h, l0, a.b);
     }
   };
-  auto load_part2 = [&](const At& a) {
+  auto load_part2 = [&](const ChunkAt& a) {
     for (int t = 0; t < 2; ++t) {
-      tma_load_4d(tK + t * 8192, &mk, &bars->in0, t * 64, a.h, a.c * kC, a.b);
-      tma_load_4d(tQ + t * 8192, &mq, &bars->in0, t * 64, a.h, a.c * kC, a.b);
+      if (blk == 2) tma_load_4d(tK + t * 8192, &mk, &bars->in0, t * 64, a.h, a.c * kC, a.b);
+      if (blk == 3) tma_load_4d(tQ + t * 8192, &mq, &bars->in0, t * 64, a.h, a.c * kC, a.b);
     }
   };
-  auto load_rec = [&](const At& a) {      // v_new, h
-    if (DELTA) bulk_g2s(tVN, p.saved + p.lay.vn + static_cast<size_t>(a.z) * p.lay.sz_vn, V * 128, &bars->in1);
-    bulk_g2s(tH, p.saved + p.lay.hc + static_cast<size_t>(a.z + a.bh) * p.lay.sz_hc, V * 256, &bars->in1);
+  auto load_rec = [&](const ChunkAt& a) {      // v_new, h
+    if (blk == 0 && DELTA) bulk_g2s(tVN, p.saved + p.lay.vn + static_cast<size_t>(a.z) * p.lay.sz_vn, V * 128, &bars->in1);
+    if (blk == 2) bulk_g2s(tH, p.saved + p.lay.hc + static_cast<size_t>(a.z + a.b * p.H + a.h) * p.lay.sz_hc, V * 256, &bars->in1);
   };
-  auto load_dh = [&](const At& a) {
-    bulk_g2s(tDH, p.scratch + p.lay.dh + static_cast<size_t>(a.z) * p.lay.sz_dh, V * 256, &bars->in1);
+  auto load_dh = [&](const ChunkAt& a) {
+    if (blk == 1) bulk_g2s(tDH, p.scratch + p.lay.dh + static_cast<size_t>(a.z) * p.lay.sz_dh, V * 256, &bars->in1);
   };
 
   if (tid == 0) {
+    where[0] = chunk_at(p, blockIdx.x);
     bars->abort_flag = 0;
-    mbar_init(&bars->in0, 1); mbar_init(&bars->in1, 1); mbar_init(&bars->mA, 1); mbar_init(&bars->mB, 1);
-    mbar_init(&bars->mW, 1); mbar_init(&bars->mT, 1); mbar_init(&bars->mV, 1); mbar_init(&bars->mX, 1);
-    mbar_init(&bars->mO, 1);
+    mbar_init(&bars->in0, 1); mbar_init(&bars->in1, 1); mbar_init(&bars->inU, 1); mbar_init(&bars->mA, 1); mbar_init(&bars->mB, 1);
+    mbar_init(&bars->mW, 1); mbar_init(&bars->mV, 1); mbar_init(&bars->mX, 1); mbar_init(&bars->mO, 1);
     fence_mbar_init();
     fence_proxy_async();
-    // Older than whatever kernel of the path comes just before this one: the caller's tensors and [T; A].  v_new (the output
-    // kernel) and h (the forward scan) only where this call has put the adjoint scan in between; with kernels picked one by one
-    // any of the three may be the last.  (Late everywhere: SSD forward and backward 175.1 us instead of 172.3 at 1692 chunks, 557.8
-    // instead of 555.3 at 4096; with the delta term no difference.)
-    if (SB) {
-      const At a = at(blockIdx.x);
-      load_part1(a);
-      load_part2(a);
-      if (p.after_scan) load_rec(a);
-    }
   }
   if (warp == 0) {
     tmem_alloc(&bars->tmem_slot, 512);
@@ -176,15 +172,27 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if (lead) {
+    // Older than whatever kernel of the path comes just before this one: the caller's tensors and [T; A].  v_new (the output
+    // kernel) and h (the forward scan) only where this call has put the adjoint scan in between; with kernels picked one by one
+    // any of the three may be the last.  (Late everywhere: SSD forward and backward 175.1 us instead of 172.3 at 1692 chunks, 557.8
+    // instead of 555.3 at 4096; with the delta term no difference.)
+    if (SB) {
+      const ChunkAt a = where[0];
+      load_part1(a);
+      load_part2(a);
+      if (p.after_scan) load_rec(a);
+    }
+  }
   const uint32_t tmem = bars->tmem_slot, lane_base = static_cast<uint32_t>(quad * 32) << 16;
-  // accumulators, [lane = channel][column = token] except dA / dT / X / dM ([token][token], lanes 0-63); what shares
+  // accumulators, [lane = channel][column = token] except dA and dM ([token][token], lanes 0-63); what shares
   // columns has been read before it is overwritten
   const uint32_t cDV = tmem, cDA = tmem + 64, cDQ = tmem + 128, cDWt = tmem + 192, cDK = tmem + 256, cO1 = tmem + 320;
   const uint32_t cDBV = tmem, cT = tmem + 64, cDBK = tmem + 192, cO2 = tmem;
   griddep_wait();
   griddep_launch();
-  if (tid == 0) {
-    const At a = at(blockIdx.x);
+  if (lead) {
+    const ChunkAt a = where[0];
     if (SB) {
       if (!p.after_scan) load_rec(a);
       load_dh(a);
@@ -195,21 +203,37 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
   }
   const uint32_t aK = smem_u32(tK), aQ = smem_u32(tQ), aC = smem_u32(tC), aBE = smem_u32(tBE);
 
+  // gates of a chunk, fetched while the chunk before is worked on: beta to shared memory; per channel to L2, a line of 128 bytes a thread
+  auto fetch_gates = [&](const ChunkAt& a, float* betas) {
+    const int t = tid & 255, r = FULL ? t >> 2 : tid, last = p.rows_of(a.c) - 1;
+    const size_t tok = (static_cast<size_t>(a.b) * p.L + a.c * kC + min(r, last)) * p.H + a.h;
+    if (FULL) prefetch_l2(tid < 256 ? p.bch + tok * kK + (t & 3) * 32 : p.wch + tok * V + (t & (V / 32 - 1)) * 32);
+    else if (tid < 64) async_copy4(betas + tid, p.beta + tok, r <= last);
+  };
+  if (WY) fetch_gates(where[0], betas2);
   uint32_t ph = 0;
   for (int n = blockIdx.x; n < nchunks; n += gridDim.x, ph ^= 1u) {
-    const At a = at(n);
-    const int rows = p.rows_of(a.c);
-    const size_t tok0 = (static_cast<size_t>(a.b) * p.L + a.c * kC) * p.H + a.h;
-    const size_t tokb = tok0 + static_cast<size_t>(blk * 16) * p.H;       // first token of this thread's block
-    float beta_r = 1.f;
-    if (WY && !FULL && tid < 64) beta_r = tid < rows ? p.beta[tok0 + static_cast<size_t>(tid) * p.H] : 0.f;
+    const float* betas = betas2 + 64 * ph;
+    int d = quad * 32 + lane;                       // this thread's channel
+    const bool more = n + static_cast<int>(gridDim.x) < nchunks;
+    auto token = [&](int r) {                       // row r of the chunk in the user's tensors
+      const ChunkAt a = where[ph];
+      return (static_cast<size_t>(a.b) * p.L + a.c * kC + r) * p.H + a.h;
+    };
 
     // ---- this thread's column: decays, k, q
     float al[16];
     uint32_t kp[8], qp[8];
+    // Between two phases: what the compiler has made from the channel (tile addresses) and from k and q (fp32 values) is made anew
+    // in the next one; kept, it goes to local memory (100 bytes a thread), which misses L1 beside 226 KB of shared memory.
+    auto anew = [&]() {
+      asm volatile("" : "+r"(d));
+#pragma unroll
+      for (int j = 0; j < 8; ++j) asm volatile("" : "+r"(kp[j]), "+r"(qp[j]));
+    };
     mbar_wait_warp(&bars->in0, ph, ctl, 601);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) al[i] = exp2f(G[quad * 2048 + (blk * 16 + i) * 32 + lane] * kLog2e);
+    for (int i = 0; i < 16; ++i) al[i] = exp2f(G[(blk * 16 + i) * kK + d] * kLog2e);
     read_column(tK, blk, d, p.qk16, kp);
     read_column(tQ, blk, d, p.qk16, qp);
     {
@@ -219,28 +243,32 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       Bb[blk * kK + d] = B;
       Af[blk * kK + d] = al[0];
     }
-    if (WY && tid < 64) betas[tid] = beta_r;
-    if (tid == 0 && n != static_cast<int>(blockIdx.x)) {
+    if (WY && !FULL) async_copy_wait();
+    if (lead && n != static_cast<int>(blockIdx.x)) {
       bulk_wait_read();                             // the results of the chunk before have left their tiles
       if (SB) {
-        load_rec(a);
-        load_dh(a);
+        load_rec(where[ph]);
+        load_dh(where[ph]);
       }
     }
     __syncthreads();          // the raw tiles are read, the block products are there
-    const BlockDecays bd = block_decays(Bb, Af, blk, d);
-    const float pre = bd.pre, post = bd.post;
-    const float gam0 = pre * al[0];                 // gamma of the block's first token
+    if (WY && tid == 0) {
+      mbar_expect_tx(&bars->inU, 16384u + V * 128u);
+      bulk_g2s(tW, p.saved + p.lay.w + static_cast<size_t>(where[ph].z) * 16384, 16384, &bars->inU);
+      if (!SB) bulk_g2s(tU, p.saved + p.lay.u + static_cast<size_t>(where[ph].z) * p.lay.sz_u, V * 128, &bars->inU);
+    }
     auto kv = [&](int i) { return half_of(kp[i >> 1], i & 1); };
     auto qv = [&](int i) { return half_of(qp[i >> 1], i & 1); };
-    auto bg = [&](int i) {                          // erase gate of token i of the block
-      return FULL ? p.bch[(tokb + static_cast<size_t>(i) * p.H) * kK + d] : betas[blk * 16 + i];
-    };
     uint32_t bkp[FULL ? 8 : 1];                     // b k
-    if (FULL)
+    if (FULL) {
+      const float* bg = p.bch + token(blk * 16) * kK + d;
+      float b[16];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) bkp[j] = f16x2_sat(kv(2 * j) * bg(2 * j), kv(2 * j + 1) * bg(2 * j + 1));
-    auto bkv = [&](int i) { return FULL ? half_of(bkp[FULL ? i >> 1 : 0], i & 1) : kv(i) * bg(i); };
+      for (int i = 0; i < 16; ++i) b[i] = bg[static_cast<size_t>(i) * p.H * kK];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) bkp[FULL ? j : 0] = f16x2_sat(kv(2 * j) * b[2 * j], kv(2 * j + 1) * b[2 * j + 1]);
+    }
+    auto bkv = [&](int i) { return FULL ? half_of(bkp[FULL ? i >> 1 : 0], i & 1) : kv(i) * betas[blk * 16 + i]; };
     // ---- operand tiles
     {
       float x[16], e = 1.f, f = 1.f;
@@ -251,6 +279,7 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       }
       write_column(tK, blk, d, x);
       if (SB) {
+        const float post = block_decays(Bb, Af, blk, d).post;
 #pragma unroll
         for (int i = 0; i < 16; ++i) x[i] *= post;
         write_column(tKD, blk, d, x);
@@ -261,16 +290,8 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
         x[i] = qv(i) * e;
       }
       write_column(tQ, blk, d, x);
-      if (WY) {
-        e = gam0;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          if (i) e *= al[i];
-          x[i] = (FULL ? bkv(i) : kv(i)) * e;
-        }
-        write_column(tGK, blk, d, x);
-      }
     }
+    anew();
     mbar_wait_warp(&bars->in1, ph, ctl, 602);
     if (SB) {
       for (int idx = tid; idx < 64 * (V / 8); idx += kCwThreads) {
@@ -284,27 +305,12 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
         }
       }
     }
-    if (WY) {
-      for (int idx = tid; idx < 64 * (V / 8); idx += kCwThreads) {
-        const int r = idx / (V / 8), ch = idx % (V / 8);
-        float x[8];
-        unpack8_bf16(tile_ld_chunk(tV, r, ch, 64), x);
-        if (FULL) {
-          float w[8];
-          ld8(p.wch + (tok0 + static_cast<size_t>(r) * p.H) * V + ch * 8, w);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) x[i] *= w[i];
-        }
-        tile_st_chunk(tV, r, ch, 64, pack8_f16(x));
-      }
-    }
-    unsigned char* dv2_g = p.scratch + p.lay.dv2 + static_cast<size_t>(a.z) * p.lay.sz_dv2;
-    unsigned char* rb_g = p.scratch + p.lay.rb + static_cast<size_t>(a.z) * p.lay.sz_rb;
-    float* dkb_g = reinterpret_cast<float*>(p.scratch + p.lay.dkb + static_cast<size_t>(a.z) * p.lay.sz_dkb);
-    float* dgb_g = reinterpret_cast<float*>(p.scratch + p.lay.dgb + static_cast<size_t>(a.z) * p.lay.sz_dgb);
+    // records of a call that is cut, or that keeps everything
+    auto rec = [&](size_t off, size_t size) { return p.scratch + off + static_cast<size_t>(where[ph].z) * size; };
+    auto rec32 = [&](size_t off, size_t size) { return reinterpret_cast<float*>(rec(off, size)); };
     const bool keep = CUT || !p.lean;
-    unsigned char* dw_g = p.scratch + p.lay.dw + static_cast<size_t>(a.z) * p.lay.sz_dw;
     if (!SB) {      // the first half of the call left dv2 and dw as token-major records
+      const unsigned char *dw_g = rec(p.lay.dw, p.lay.sz_dw), *dv2_g = rec(p.lay.dv2, p.lay.sz_dv2), *rb_g = rec(p.lay.rb, p.lay.sz_rb);
       float x[16];
 #pragma unroll
       for (int i = 0; i < 16; ++i) x[i] = __half2float(*reinterpret_cast<const __half*>(dw_g + sw128_off(blk * 16 + i, d, 64)));
@@ -321,25 +327,24 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
                         *reinterpret_cast<const uint4*>(rb_g + sw128_chunk(d, 2 * blk + j, 64)));
       }
       for (int idx = tid; idx < 1024; idx += kCwThreads) Cd0[idx] = reinterpret_cast<const float*>(rb_g + kRecDiag)[idx];
-      Bb[blk * kK + d] = reinterpret_cast<const float*>(rb_g + kRecEnd)[blk * kK + d];
+      Et[blk * kK + d] = reinterpret_cast<const float*>(rb_g + kRecEnd)[blk * kK + d];
     }
     sync_for_issue();
 
-    // ---- group 1 (two warps issue): dv2^T, dA | dq_inter^T, (v_new dh^T)^T
+    if (tid == kCwThreads - 1 && more) where[ph ^ 1u] = chunk_at(p, n + gridDim.x);
+    // ---- group 1: dv2^T, dA; (v_new dh^T)^T; dq_inter^T.  What the chain needs first is issued first.
     if (SB) {
       if (warp == 0) {
         tc_fence_after();
         const uint32_t leader = elect_leader();
         issue_product_led(leader, cDV, Tile{smem_u32(tDH), 128, true}, Tile{smem_u32(tKD), 128, true}, 64, 128, 0u);
         issue_product_led(leader, cDV, Tile{smem_u32(tDO), 64, true}, Tile{smem_u32(tTA) + 8192, 64, true}, 64, 64, 1u);
-        issue_product_led(leader, cDA, Tile{smem_u32(tDO), 64, false}, Tile{smem_u32(tVN), 64, false}, 64, V, 0u);
         umma_commit_led(leader, &bars->mA);
-      } else if (warp == 4) {
-        tc_fence_after();
-        const uint32_t leader = elect_leader();
-        issue_product_led(leader, cDQ, Tile{smem_u32(tH), 128, false}, Tile{smem_u32(tDO), 64, false}, 64, V, 0u);
+        issue_product_led(leader, cDA, Tile{smem_u32(tDO), 64, false}, Tile{smem_u32(tVN), 64, false}, 64, V, 0u);
         issue_product_led(leader, cDK, Tile{smem_u32(tDH), 128, false}, Tile{smem_u32(tVN), 64, false}, 64, V, 0u);
-        umma_commit_led(leader, &bars->mB);
+        if (MODE == kCwAll) umma_commit_led(leader, &bars->mB);
+        issue_product_led(leader, cDQ, Tile{smem_u32(tH), 128, false}, Tile{smem_u32(tDO), 64, false}, 64, V, 0u);
+        if (MODE != kCwAll) umma_commit_led(leader, &bars->mB);
       }
       __syncwarp();
       // in their shadow: this block's quarter of <dh, h> of channel d (both images are only read)
@@ -352,12 +357,9 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
 #pragma unroll
         for (int e = 0; e < 8; ++e) endt = fmaf(x[e], y[e], endt);
       }
-      {
-        float B = 1.f;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) B *= al[i];
-        endt *= pre * B * post;                     // exp(G_last) <dh, h>
-      }
+      const BlockDecays bd = block_decays(Bb, Af, blk, d);
+      endt *= bd.pre * Bb[blk * kK + d] * bd.post;  // exp(G_last) <dh, h>
+      anew();
       mbar_wait_warp(&bars->mA, ph, ctl, 603);
       tc_fence_after();
       if (d < V) {
@@ -366,31 +368,47 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
         tmem_ld_wait();
         if (DELTA) {
           write_column(tDV, blk, d, x);
-          if (keep)
+          if (keep) {
+            unsigned char* dv2_g = rec(p.lay.dv2, p.lay.sz_dv2);
 #pragma unroll
-            for (int i = 0; i < 16; ++i)
-              store_f16_sat(dv2_g + sw128_off(blk * 16 + i, d, 64), x[i]);
+            for (int i = 0; i < 16; ++i) store_f16_sat(dv2_g + sw128_off(blk * 16 + i, d, 64), x[i]);
+          }
         } else {
 #pragma unroll
           for (int i = 0; i < 16; ++i) stage16(oVt, blk * 16 + i, d, x[i], 0);
         }
       }
+      // ---- group 2: dw^T = -h dv2^T, and T^T dv2
+      if (DELTA) {
+        sync_for_issue();
+        if (warp == 0) {
+          tc_fence_after();
+          const uint32_t leader = elect_leader();
+          issue_product_led(leader, cDWt, Tile{smem_u32(tH), 128, false}, Tile{smem_u32(tDV), V, true}, 64, V, 0u);
+          if (WY) issue_product_led(leader, cDBV, Tile{smem_u32(tDV), V, false}, Tile{smem_u32(tTA), 64, true}, 64, 64, 0u);
+          umma_commit_led(leader, &bars->mW);
+        }
+        __syncwarp();
+      }
+      // in its shadow: the rest of the end term, C0, (b k) e
       mbar_wait_warp(&bars->mB, ph, ctl, 604);      // v_new and dh are dead from here on
       tc_fence_after();
+      if (WY && tid == 0) bulk_g2s(tU, p.saved + p.lay.u + static_cast<size_t>(where[ph].z) * p.lay.sz_u, V * 128, &bars->inU);
       {
-        float x[16], f = 1.f;
+        float x[16], f = bd.post;
         tmem_ld16(cDK + lane_base + blk * 16, x);
         tmem_ld_wait();
 #pragma unroll
         for (int i = 15; i >= 0; --i) {             // + sum_i k (v_new dh^T) exp(G_last - G_i)
-          endt = fmaf(x[i] * kv(i), f * post, endt);
+          endt = fmaf(x[i] * kv(i), f, endt);
           f *= al[i];
         }
-        Bb[blk * kK + d] = endt;
+        Et[blk * kK + d] = endt;
         if (MODE == kCwStageB) {
+          float *dkb_g = rec32(p.lay.dkb, p.lay.sz_dkb), *dgb_g = rec32(p.lay.dgb, p.lay.sz_dgb);
 #pragma unroll
           for (int i = 0; i < 16; ++i) dkb_g[rec_at(blk * 16 + i, d)] = x[i];
-          reinterpret_cast<float*>(rb_g + kRecEnd)[blk * kK + d] = endt;
+          reinterpret_cast<float*>(rec(p.lay.rb, p.lay.sz_rb) + kRecEnd)[blk * kK + d] = endt;
           tmem_ld16(cDQ + lane_base + blk * 16, x);
           tmem_ld_wait();
 #pragma unroll
@@ -410,6 +428,7 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
           st8(Cd0 + i * 16 + 8, x + 8);
         }
         if (MODE == kCwStageB) {
+          unsigned char* rb_g = rec(p.lay.rb, p.lay.sz_rb);
           write_row16(rb_g, i, blk, x);
           if (ib == blk) {
             st8(reinterpret_cast<float*>(rb_g + kRecDiag) + i * 16, x);
@@ -417,7 +436,13 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
           }
         }
       }
+    } else if (warp == 0) {
+      tc_fence_after();
+      const uint32_t leader = elect_leader();
+      issue_product_led(leader, cDBV, Tile{smem_u32(tDV), V, false}, Tile{smem_u32(tTA), 64, true}, 64, 64, 0u);
+      umma_commit_led(leader, &bars->mW);
     }
+    __syncwarp();
     if (WY) {                                       // (b k) e, where dh was
       float x[16], e = 1.f;
 #pragma unroll
@@ -427,86 +452,84 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       }
       write_column(tBE, blk, d, x);
     }
-    sync_for_issue();
-
-    // ---- dw^T = -h dv2^T
-    if (SB && DELTA) {
-      if (warp == 0) {
-        tc_fence_after();
-        const uint32_t leader = elect_leader();
-        issue_product_led(leader, cDWt, Tile{smem_u32(tH), 128, false}, Tile{smem_u32(tDV), V, true}, 64, V, 0u);
-        umma_commit_led(leader, &bars->mW);
-      }
-      __syncwarp();
-      mbar_wait_warp(&bars->mW, ph, ctl, 605);
+    anew();
+    if (DELTA) {
+      mbar_wait_warp(&bars->mW, ph, ctl, 605);      // h is dead from here on
       tc_fence_after();
+    }
+    if (SB && DELTA) {
       float x[16];
       tmem_ld16(cDWt + lane_base + blk * 16, x);
       tmem_ld_wait();
 #pragma unroll
       for (int i = 0; i < 16; ++i) x[i] = -x[i];
       if (WY) write_column(tDW, blk, d, x);
-      if (keep)
+      if (keep) {
+        unsigned char* dw_g = rec(p.lay.dw, p.lay.sz_dw);
 #pragma unroll
-        for (int i = 0; i < 16; ++i)
-          store_f16_sat(dw_g + sw128_off(blk * 16 + i, d, 64), x[i]);
-      if (WY) sync_for_issue();
+        for (int i = 0; i < 16; ++i) store_f16_sat(dw_g + sw128_off(blk * 16 + i, d, 64), x[i]);
+      }
     }
     if (WY) {
-      // ---- dT; T^T dv2, T^T dw
-      if (warp == 0) {
-        tc_fence_after();
-        const uint32_t leader = elect_leader();
-        issue_product_led(leader, cT, Tile{smem_u32(tDV), V, true}, Tile{smem_u32(tV), 64, false}, 64, V, 0u);
-        issue_product_led(leader, cT, Tile{smem_u32(tDW), 128, true}, Tile{smem_u32(tGK), 128, true}, 64, 128, 1u);
-        umma_commit_led(leader, &bars->mT);
-        issue_product_led(leader, cDBV, Tile{smem_u32(tDV), V, false}, Tile{smem_u32(tTA), 64, true}, 64, 64, 0u);
-        issue_product_led(leader, cDBK, Tile{smem_u32(tDW), 128, false}, Tile{smem_u32(tTA), 64, true}, 64, 64, 0u);
-        umma_commit_led(leader, &bars->mV);
-      }
-      __syncwarp();
-      mbar_wait_warp(&bars->mT, ph, ctl, 606);
-      tc_fence_after();
-      if (quad < 2) {                               // the scalar write and erase gates are one factor per source token
-        float x[16];
-        tmem_ld16(cT + lane_base + blk * 16, x);
-        tmem_ld_wait();
-        if (!FULL)
-#pragma unroll
-          for (int j = 0; j < 16; ++j) x[j] *= betas[blk * 16 + j];
-        write_row16(tDT, d, blk, x);
-      }
-      sync_for_issue();
-      // ---- X = dT T^T
-      if (warp == 0) {
-        tc_fence_after();
-        const uint32_t leader = elect_leader();
-        issue_product_led(leader, cT, Tile{smem_u32(tDT), 64, false}, Tile{smem_u32(tTA), 128, false}, 64, 64, 0u);
-        umma_commit_led(leader, &bars->mX);
-      }
-      __syncwarp();
-      // in its shadow: dv and the value part of the gate gradients
-      mbar_wait_warp(&bars->mV, ph, ctl, 607);
-      tc_fence_after();
       if (d < V) {
         float x[16];
         tmem_ld16(cDBV + lane_base + blk * 16, x);
         tmem_ld_wait();
+        write_column(tBV, blk, d, x);
+      }
+      mbar_wait_warp(&bars->inU, ph, ctl, 606);
+      sync_for_issue();
+      // ---- group 3: T^T dw; the first part of dM = -(dbv u^T + dbgk w^T)
+      if (warp == 0) {
+        tc_fence_after();
+        const uint32_t leader = elect_leader();
+        issue_product_led(leader, cDBK, Tile{smem_u32(tDW), 128, false}, Tile{smem_u32(tTA), 64, true}, 64, 64, 0u);
+        umma_commit_led(leader, &bars->mV);
+        issue_product_led(leader, cT, Tile{smem_u32(tBV), V, true}, Tile{smem_u32(tU), 64, false}, 64, V, 0u, true);
+      }
+      __syncwarp();
+      if (more) fetch_gates(where[ph ^ 1u], betas2 + 64 * (ph ^ 1u));
+      mbar_wait_warp(&bars->mV, ph, ctl, 607);
+      tc_fence_after();
+      {
+        float x[16];
+        tmem_ld16(cDBK + lane_base + blk * 16, x);
+        tmem_ld_wait();
+        write_column(tBK, blk, d, x);
+      }
+      sync_for_issue();
+      // ---- group 4: the second part
+      if (warp == 0) {
+        tc_fence_after();
+        const uint32_t leader = elect_leader();
+        issue_product_led(leader, cT, Tile{smem_u32(tBK), 128, true}, Tile{smem_u32(tW), 64, false}, 64, 128, 1u, true);
+        umma_commit_led(leader, &bars->mX);
+      }
+      __syncwarp();
+      anew();
+      // in its shadow: dv and the value part of the gate gradients
+      if (d < V) {
+        float x[16], wv[FULL ? 16 : 1];
+        const size_t step = static_cast<size_t>(p.H) * V, first = FULL ? token(blk * 16) * V + d : 0;
+        if (FULL)
+#pragma unroll
+          for (int i = 0; i < 16; ++i) wv[FULL ? i : 0] = p.wch[first + i * step];
+        uint32_t vp[8];
+        read_column(tV, blk, d, 0, vp);
+        tmem_ld16(cDBV + lane_base + blk * 16, x);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          f2 g, y = pack2(x[2 * j], x[2 * j + 1]);
+          if (FULL) g = pack2(wv[FULL ? 2 * j : 0], wv[FULL ? 2 * j + 1 : 0]);
+          else g.u = *reinterpret_cast<const unsigned long long*>(betas + blk * 16 + 2 * j);
+          stage16_two(oVt, blk * 16 + 2 * j, d, mul2(g, y), 0);
+          unpack2(mul2(y, pair_of(vp[j])), x[2 * j], x[2 * j + 1]);
+        }
         if (FULL) {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const size_t o = (tokb + static_cast<size_t>(i) * p.H) * V + d;
-            p.dwch[o] = x[i] * __bfloat162float(p.v[o]);
-            stage16(oVt, blk * 16 + i, d, p.wch[o] * x[i], 0);
-          }
+          for (int i = 0; i < 16; ++i) p.dwch[first + i * step] = x[i];
         } else {
-          uint32_t vp[8];
-          read_column(tV, blk, d, 1, vp);
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            stage16(oVt, blk * 16 + i, d, betas[blk * 16 + i] * x[i], 0);
-            x[i] *= half_of(vp[i >> 1], i & 1);
-          }
           const float s0 = warp_sum8(x, lane), s1 = warp_sum8(x + 8, lane);
           if ((lane & 3) == 0) {
             red[256 + quad * 64 + blk * 16 + (lane >> 2)] = s0;
@@ -514,24 +537,7 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
           }
         }
       }
-      mbar_wait_warp(&bars->mX, 0, ctl, 608);
-      tc_fence_after();
-      if (quad < 2) {
-        float x[16];
-        tmem_ld16(cT + lane_base + blk * 16, x);
-        tmem_ld_wait();
-        write_row16(tDT, d, blk, x);
-      }
-      sync_for_issue();
-      // ---- dM = -T^T X
-      if (warp == 0) {
-        tc_fence_after();
-        const uint32_t leader = elect_leader();
-        issue_product_led(leader, cT, Tile{smem_u32(tTA), 64, true}, Tile{smem_u32(tDT), 64, true}, 64, 64, 0u, true);
-        umma_commit_led(leader, &bars->mX);
-      }
-      __syncwarp();
-      mbar_wait_warp(&bars->mX, 1, ctl, 609);
+      mbar_wait_warp(&bars->mX, ph, ctl, 609);
       tc_fence_after();
       if (quad < 2) {
         const int i = d, ib = i >> 4;
@@ -549,17 +555,17 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       sync_for_issue();
     }
 
-    const bool more = n + static_cast<int>(gridDim.x) < nchunks;
-    const At nx = at(more ? n + gridDim.x : n);
+    if (!DELTA) sync_for_issue();
     if (MODE == kCwStageB) {
       sync_for_issue();
-      if (tid == 0 && more) {
-        load_part1(nx);
-        load_part2(nx);
+      if (lead && more) {
+        load_part1(where[ph ^ 1u]);
+        load_part2(where[ph ^ 1u]);
       }
       continue;
     }
     if (tid == 0) {                                 // dv (written before the last barrier)
+      const ChunkAt a = where[ph];
       for (int t = 0; t < V / 64; ++t) tma_store_4d(&mo.dv, oVt + t * 8192, t * 64, a.h, a.c * kC, a.b);
       bulk_commit();
     }
@@ -584,8 +590,9 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       umma_commit_led(leader, &bars->mO);
     }
     __syncwarp();
-    if (tid == 0 && more) load_part1(nx);      // g, v, do, [T; A]: their tiles are dead
+    if (lead && more) load_part1(where[ph ^ 1u]);      // g, v, do, [T; A]: their tiles are dead
 
+    anew();
     // ---- diagonal blocks, column sums: rows from the last to the first, sum(s) <- alpha sum(s) + C x
     const float* c0 = Cd0 + blk * 256;
     const float* c1 = Cd1 + blk * 256;
@@ -618,7 +625,9 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     }
     mbar_wait_warp(&bars->mO, ph, ctl, 610);
     tc_fence_after();
-    if (tid == 0 && more) load_part2(nx);         // k, q: the last products that read those tiles are done
+    if (lead && more) load_part2(where[ph ^ 1u]);         // k, q: the last products that read those tiles are done
+    const BlockDecays bd = block_decays(Bb, Af, blk, d);
+    const float gam0 = bd.pre * al[0];              // gamma of the block's first token
     // dk' without the gate part: de (v_new dh^T) + out2
     float dkp[16];
     {
@@ -640,11 +649,12 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
         tmem_ld16(cDK + lane_base + blk * 16, x);
         tmem_ld_wait();
       } else {
+        const float* dkb_g = rec32(p.lay.dkb, p.lay.sz_dkb);
 #pragma unroll
         for (int i = 0; i < 16; ++i) x[i] = dkb_g[rec_at(blk * 16 + i, d)];
       }
 #pragma unroll
-      for (int i = 0; i < 16; ++i) t2[i] = fmaf(post, x[i], t2[i]);
+      for (int i = 0; i < 16; ++i) t2[i] = fmaf(bd.post, x[i], t2[i]);
       float f = 1.f;
 #pragma unroll
       for (int i = 15; i >= 0; --i) {
@@ -652,49 +662,54 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
         f *= al[i];
       }
     }
-    // ---- diagonal blocks, row sums (kr(s) = k(s) ratio(i, s)), and the gradients of each row; dG replaces dk'
+    anew();
+    // ---- diagonal blocks, row sums (kr(s) = k(s) ratio(i, s)), and the gradients of each row; dG where dg will be
     f2 kr[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) kr[j] = pack2(0.f, 0.f);
-    float e = 1.f, dsum = 0.f;
+    float e = 1.f;
+    f2 dsum = pack2(0.f, 0.f);
+    const f2 minus = pack2(-1.f, -1.f);
 #pragma unroll
-    for (int hf = 0; hf < 2; ++hf) {
-      float o0[8], o1[WY ? 8 : 1], x[8], val[WY ? 8 : 1], bi[FULL ? 8 : 1];
-      if (FULL)
+    for (int qt = 0; qt < 4; ++qt) {                // four rows at a time: eight spill
+      float o0[4], o1[WY ? 4 : 1], x[4], bi[FULL ? 4 : 1];
+      if (FULL) {
+        const float* bg = p.bch + token(blk * 16 + 4 * qt) * kK + d;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) bi[i] = bg(8 * hf + i);
+        for (int i = 0; i < 4; ++i) bi[FULL ? i : 0] = bg[static_cast<size_t>(i) * p.H * kK];
+      }
       if (SB) {
-        tmem_ld8(cDQ + lane_base + blk * 16 + 8 * hf, x);
+        tmem_ld4(cDQ + lane_base + blk * 16 + 4 * qt, x);
         tmem_ld_wait();
       } else {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) x[i] = dgb_g[rec_at(blk * 16 + 8 * hf + i, d)];
+        for (int i = 0; i < 4; ++i) x[i] = rec32(p.lay.dgb, p.lay.sz_dgb)[rec_at(blk * 16 + 4 * qt + i, d)];
       }
 #pragma unroll
-      for (int i = 0; i < 8; ++i) o0[i] = p.scale * gam0 * x[i];
+      for (int i = 0; i < 4; ++i) o0[i] = p.scale * gam0 * x[i];
       if (WY) {
-        tmem_ld8(cDBK + lane_base + blk * 16 + 8 * hf, x);
+        tmem_ld4(cDBK + lane_base + blk * 16 + 4 * qt, x);
         tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 8; ++i) o1[i] = gam0 * x[i];
+        for (int i = 0; i < 4; ++i) o1[i] = gam0 * x[i];
       }
 #pragma unroll
       for (int J = 0; J < 3; ++J) {
         if (J >= blk) continue;
-        const uint32_t at1 = cO1 + lane_base + (J == 0 ? 0 : J == 1 ? 3 * CR : 5 * CR) + (blk - 1 - J) * CR + 8 * hf;
-        float y[WY ? 8 : 1];
-        tmem_ld8(at1, x);
-        if (WY) tmem_ld8(at1 + 16, y);
+        const uint32_t at1 = cO1 + lane_base + (J == 0 ? 0 : J == 1 ? 3 * CR : 5 * CR) + (blk - 1 - J) * CR + 4 * qt;
+        float y[WY ? 4 : 1];
+        tmem_ld4(at1, x);
+        if (WY) tmem_ld4(at1 + 16, y);
         tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < 4; ++i) {
           o0[i] = fmaf(bd.cdn[J], x[i], o0[i]);
           if (WY) o1[i] = fmaf(bd.cdn[J], y[i], o1[i]);
         }
       }
 #pragma unroll
-      for (int i8 = 0; i8 < 8; ++i8) {
-        const int i = 8 * hf + i8;
+      for (int i4 = 0; i4 < 4; ++i4) {
+        const int i = 4 * qt + i4;
         const float ai = i ? al[i] : 1.f, k_i = kv(i);
         e *= ai;
         const f2 dec = pack2(ai, ai);
@@ -719,28 +734,43 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
             if (WY) s1[t] = fma2(u1[t], kr[j], s1[t]);
           }
         }
-        const float dq = fmaf(e, o0[i8], sum2(s0[0]) + sum2(s0[1]));
-        float dk = dkp[i], dG = fmaf(qv(i), dq, -k_i * dk);
-        stage16(oQt, blk * 16 + i, d, dq, p.qk16);
+        o0[i4] = fmaf(e, o0[i4], sum2(s0[0]) + sum2(s0[1]));             // dq
+        if (WY) o1[i4] = fmaf(e, o1[i4], sum2(s1[0]) + sum2(s1[1]));     // d(b k)
+      }
+      float val[WY ? 4 : 1];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {                 // two rows: dG = q dq + (b k) dbk - k dk',  dk = dk' + b dbk
+        const int i = 4 * qt + 2 * j;
+        const f2 k2 = pair_of(kp[i >> 1]), dq2 = pack2(o0[2 * j], o0[2 * j + 1]);
+        f2 dk2 = pack2(dkp[i], dkp[i + 1]), u = mul2(minus, dk2);
         if (WY) {
-          const float dbk = fmaf(e, o1[i8], sum2(s1[0]) + sum2(s1[1]));
-          dG = fmaf(bkv(i), dbk, dG);
-          dk = fmaf(FULL ? bi[FULL ? i8 : 0] : bg(i), dbk, dk);
-          val[i8] = dbk * k_i;
-          if (FULL) p.dbch[(tokb + static_cast<size_t>(i) * p.H) * kK + d] = val[i8];
+          const f2 dbk = pack2(o1[WY ? 2 * j : 0], o1[WY ? 2 * j + 1 : 0]), v2 = mul2(dbk, k2);
+          f2 b2;
+          if (FULL) b2 = pack2(bi[FULL ? 2 * j : 0], bi[FULL ? 2 * j + 1 : 0]);
+          else b2.u = *reinterpret_cast<const unsigned long long*>(betas + blk * 16 + i);
+          u = fma2(b2, dbk, u);
+          dk2 = fma2(b2, dbk, dk2);
+          unpack2(v2, val[WY ? 2 * j : 0], val[WY ? 2 * j + 1 : 0]);
         }
-        stage16(oKt, blk * 16 + i, d, dk, p.qk16);
-        dsum += dG;
-        dkp[i] = dG;
+        const f2 dG = fma2(k2, u, mul2(pair_of(qp[i >> 1]), dq2));
+        dsum = add2(dsum, dG);
+        stage16_two(oQt, blk * 16 + i, d, dq2, p.qk16);
+        stage16_two(oKt, blk * 16 + i, d, dk2, p.qk16);
+        unpack2(dG, oGt[(blk * 16 + i) * kK + d], oGt[(blk * 16 + i + 1) * kK + d]);
+      }
+      if (FULL) {
+        float* db = p.dbch + token(blk * 16 + 4 * qt) * kK + d;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) db[static_cast<size_t>(i) * p.H * kK] = val[WY ? i : 0];
       }
       if (WY && !FULL) {
-        const float s = warp_sum8(val, lane);
-        if ((lane & 3) == 0) red[quad * 64 + blk * 16 + 8 * hf + (lane >> 2)] = s;
+        const float s = warp_sum4(val, lane);
+        if ((lane & 7) == 0) red[quad * 64 + blk * 16 + 4 * qt + (lane >> 3)] = s;
       }
     }
     // ---- gate gradient: reverse cumulative sum over the chunk, the end term counting for every row
-    const float endt = (Bb[d] + Bb[kK + d]) + (Bb[2 * kK + d] + Bb[3 * kK + d]);
-    St[blk * kK + d] = dsum;
+    const float endt = (Et[d] + Et[kK + d]) + (Et[2 * kK + d] + Et[3 * kK + d]);
+    St[blk * kK + d] = sum2(dsum);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -751,25 +781,27 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
         if (m > blk) acc += St[m * kK + d];
 #pragma unroll
       for (int i = 15; i >= 0; --i) {
-        acc += dkp[i];
-        oGt[quad * 2048 + (blk * 16 + i) * 32 + lane] = acc;
+        float* g = oGt + (blk * 16 + i) * kK + d;
+        acc += *g;
+        *g = acc;
       }
     }
     fence_proxy_async();
     __syncthreads();
-    if (tid == 0) {
-      for (int t = 0; t < p.Kr / 64; ++t) {
-        tma_store_4d(&mo.dq, oQt + t * 8192, t * 64, a.h, a.c * kC, a.b);
-        tma_store_4d(&mo.dk, oKt + t * 8192, t * 64, a.h, a.c * kC, a.b);
-      }
-      for (int t = 0; t < p.Kr / 32; ++t) tma_store_4d(&mo.dg, oGt + t * 2048, t * 32, a.h, a.c * kC, a.b);
+    if (lead && blk < 3) {
+      const ChunkAt a = where[ph];
+      if (blk < 2)
+        for (int t = 0; t < p.Kr / 64; ++t)
+          tma_store_4d(blk == 0 ? &mo.dq : &mo.dk, (blk == 0 ? oQt : oKt) + t * 8192, t * 64, a.h, a.c * kC, a.b);
+      else
+        tma_store_4d(&mo.dg, oGt, 0, a.h, a.c * kC, a.b);
       bulk_commit();
     }
-    if (WY && !FULL && tid < rows) {
+    if (WY && !FULL && tid < p.rows_of(where[ph].c)) {
       const float er = (red[tid] + red[64 + tid]) + (red[128 + tid] + red[192 + tid]);
       float wr = red[256 + tid] + red[320 + tid];
       if (V == 128) wr += red[384 + tid] + red[448 + tid];
-      const size_t o = tok0 + static_cast<size_t>(tid) * p.H;
+      const size_t o = token(tid);
       if (p.dbeta_w) {
         p.dbeta_w[o] = wr;
         p.dbeta[o] = er;
@@ -778,7 +810,7 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       }
     }
   }
-  if (tid == 0) bulk_wait_read();
+  if (lead) bulk_wait_read();
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, 512);

@@ -139,7 +139,7 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
   };
   auto load_kqg = [&](const At& a) {      // (tid 0)
     mbar_expect_tx(in0, 65536u);
-    for (int q = 0; q < 4; ++q) tma_load_4d(tile(2) + q * 8192, &mg, in0, q * 32, a.h, a.c * kC, a.b);
+    tma_load_4d(tile(2), &mg, in0, 0, a.h, a.c * kC, a.b);
     for (int t = 0; t < 2; ++t) {
       tma_load_4d(tK + t * 8192, &mk, in0, t * 64, a.h, a.c * kC, a.b);
       tma_load_4d(tQ + t * 8192, &mq, in0, t * 64, a.h, a.c * kC, a.b);
@@ -201,7 +201,7 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
       read_column(tK, blk, d, F16, kp);
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
-        float* gi = G + quad * 2048 + (blk * 16 + i) * 32 + lane;
+        float* gi = G + (blk * 16 + i) * kK + d;
         al[i] = exp2f(*gi * kLog2e);
         *gi = al[i];
       }
@@ -225,7 +225,7 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
 #pragma unroll 1
     for (int it = 0; it < NB; ++it) {
       const int c = lane & 15, j = warp & 7, db = (NB == 1 ? warp >> 3 : it) * 2 + (lane >> 4);
-      const float* al0 = G + (c >> 3) * 2048 + 4 * (c & 7);        // alpha of row r: + 32 r; the other half: + 4096
+      const float* al0 = G + 4 * c;        // alpha of row r: + 128 r; the other half: + 64
       const unsigned char* kt = tK + (c & 1) * 8;
       const unsigned char* qt = tQ + (c & 1) * 8;
       auto at16 = [&](int r) { return r * 128 + (((c >> 1) ^ (r & 7)) << 4); };
@@ -272,8 +272,8 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
           f2 ks[4], as[4];
           ld4_pairs<F16>(kt + at16(rs), ks);
           ld4_pairs<F16>(kt + 8192 + at16(rs), ks + 2);
-          ld_pairs(al0 + 32 * rs, as);
-          ld_pairs(al0 + 32 * rs + 4096, as + 2);
+          ld_pairs(al0 + kK * rs, as);
+          ld_pairs(al0 + kK * rs + 64, as + 2);
 #pragma unroll
           for (int e = 0; e < 4; ++e) ks[e] = mul2(ratio[e], ks[e]);
           dots(ks, qi, ki, out[u], out[4 + u]);
@@ -336,7 +336,7 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
       read_column(tK, b0 + bb, d, F16, kp[bb]);
       read_column(tQ, b0 + bb, d, F16, qp[bb]);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) al[bb][i] = G[quad * 2048 + ((b0 + bb) * 16 + i) * 32 + lane];
+      for (int i = 0; i < 16; ++i) al[bb][i] = G[((b0 + bb) * 16 + i) * kK + d];
     }
     if (NORM && tid == 0) bulk_wait_read();      // the normalised rows have left
     __syncthreads();                             // k, q, alpha and the decayed rows are read: their tiles become operands

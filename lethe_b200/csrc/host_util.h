@@ -65,7 +65,7 @@ inline int make_tmap_16bit(CUtensorMap* map, const void* ptr, int rank, const ui
   return r == CUDA_SUCCESS ? kOk : kErrDriver;
 }
 
-// The same over fp32 elements, without a swizzle (boxes of up to 32 elements: 128-byte rows).
+// The same over fp32 elements, without a swizzle.
 inline int make_tmap_f32(CUtensorMap* map, const void* ptr, int rank, const uint64_t* dims, const uint64_t* strides_bytes,
                          const uint32_t* box) {
   EncodeTiledFn fn = encode_tiled_fn();

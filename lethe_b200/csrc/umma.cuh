@@ -268,6 +268,13 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
 // TMEM -> registers.  taddr = base + (lane << 16) + column; the lane field must be the first lane
 // of the calling warp's quadrant (32 * (warp & 3)).  Thread l of the warp receives lane base + l.
 // ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, float* v) {
+  uint32_t* r = reinterpret_cast<uint32_t*>(v);
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(taddr)
+               : "memory");
+}
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
   uint32_t* r = reinterpret_cast<uint32_t*>(v);
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"

@@ -70,6 +70,13 @@ def _layout(B, H, L, V, gate):
     return Z, sz, off, sz2, off2
 
 
+def _wy_factors(buf, sz, off, Z, t_mat: Tensor, gated_k: Tensor, gated_v: Tensor) -> None:
+    """Records of the forward that the VJP reads: w = T (gated k), u = T (gated v)."""
+    for n, x in (("w", gated_k), ("u", gated_v)):
+        img = to_image((t_mat.float() @ x).half()).reshape(Z, -1)
+        _record_view(buf.saved, off[n], sz[n], Z, torch.float16).copy_(img)
+
+
 def _untok(x: Tensor) -> Tensor:
     """[B, H, NT, C, D] -> [B, L, H, D]"""
     B, H, NT, C, D = x.shape
@@ -177,6 +184,7 @@ def k2_fn_cw(k: Tensor, v: Tensor, b: Tensor, w: Tensor, g2: Tensor, t_mat: Tens
     ta = torch.zeros(B, H, NT, 128, 64, dtype=torch.float16, device=dev)
     ta[..., :64, :] = t_mat.half()
     _record_view(buf.saved, off["ta"], sz["ta"], Z, torch.float16).copy_(to_image(ta).reshape(Z, -1))
+    _wy_factors(buf, sz, off, Z, t_mat, b.to(f32) * torch.exp2(g2.to(f32)) * k.to(f32), w.to(f32) * v.to(f32))
     _record_view(buf.scratch, off2["dv2"], sz2["dv2"], Z, torch.float16).copy_(to_image(du.half()).reshape(Z, -1))
     _record_view(buf.scratch, off2["dw"], sz2["dw"], Z, torch.float16).copy_(to_image(dwy.half()).reshape(Z, -1))
     _record_view(buf.scratch, off2["dkb"], sz2["dkb"], Z, f32).zero_()
