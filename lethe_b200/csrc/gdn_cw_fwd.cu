@@ -5,44 +5,53 @@
 // gdn2_chunkwise_cw.py:155-157,168-169).  The 64-token chunk is cut into four blocks of 16 rows:
 //   * row block I against earlier blocks: left operand rows x[i] e[i], decayed from the first token of their block, right
 //     operand rows k[s] decayed from s to the first token of block I (96 of them for I = 1, 2, 3); tcgen05 products;
-//   * the four diagonal 16 x 16 blocks: exact fp32 sums on the CUDA cores, while the products run.
+//   * the four diagonal 16 x 16 blocks: exact fp32 sums on the CUDA cores.
 // Everything after M and A (inverse, WY factors, state map) is the scalar-gate kernel's, with per-channel decays in the
 // operand scalings.
 //
 // Layout and decays are those of the backward (gdn_cw_bwd.cu): thread (block of 16 tokens, channel) builds its 16-token
 // columns of every decayed operand in registers from alpha = exp(g), the only exponential, and stores them as
 // [channel][token] tiles; ratios are products of alphas.  The diagonal blocks need sums over channels instead: there a
-// half-warp takes the rows j and 15 - j of a block, a lane eight channels of them.  The 16 rows fall into groups of four:
-// inside its own group a row goes down the source rows with ratio(i, s) = ratio(i, s + 1) alpha(s + 1); for an earlier
-// group the source rows lie ready in fp32, decayed to the end of their group, and the row carries its decay from there, so
-// that a pair costs two FMAs per channel and no ratio.  All in fp32, and every factor is a decay between two rows that lie
-// between s and i.  (Walking every pair with a running ratio took 6.8 k cycles per chunk, this 4.8 k.)
+// half-warp has a block, a lane eight channels of it.  The 16 rows fall into groups of four.  Inside a group the source rows
+// are carried along, decayed to the row in hand.  For an earlier group they lie ready in fp32, decayed to the end of their
+// group, and the four rows of the later group, decayed from there, stay in registers while the source rows go by: a pair costs
+// two packed FMAs per two channels, and a source row is loaded once for four rows.  All in fp32, and every factor is a decay
+// between two rows that lie between s and i.  (Two rows of a block per half-warp, each loading its source rows: 11 k warp
+// instructions per chunk, now 7 k; 35 k against 29 k for the whole kernel.)
 //
 // NB: blocks of 16 tokens per thread.  2: 256 threads on six tiles that change hands, two persistent CTAs per SM, so that
 // one chunk's barriers, product waits and loads lie under the other's arithmetic; k, q and alpha go to registers after the diagonal
 // sums and the operands take their tiles.  1: 512 threads, for a launch that gives every SM one chunk at most, where only the
-// length of a chunk's own chain counts.  Measured (us, d_v = 128; one CTA of 512 threads with twice the memory before): 8192
-// chunks 590 -> 559, 8000 chunks 582 -> 547, 512 chunks 54 -> 49, without the delta term 4096 chunks 209 -> 190, per-channel gates 512
-// chunks 70 -> 59; 128 chunks 20.5 either way.
+// length of a chunk's own chain counts.  Measured (us, d_v = 128; one CTA of 512 threads with twice the memory / two of 256 /
+// these diagonal sums, loads that come early, beta a chunk ahead): 8192 chunks 590 / 559 / 486; 512 chunks 54 / 49 / 44; without the
+// delta term 4096 chunks 209 / 190 / 158; per-channel gates 512 chunks 70 / 59 / 52; 128 chunks 20 in each.
+//
+// Loads: k and q of the next chunk as soon as the inverse is done, g when w and u have left its tiles, behind a prefetch to L2 that
+// was issued before the inverse; the write gates of the full op are requested under the first products.
+// Bound by the chain of phases of a chunk and by shared memory (LSU data pipe 57 % busy, issue slots 46 %).  Cycles per chunk by
+// clock samples of one of two CTAs (d_v = 128): waits for loads 1.9 k, alphas 1.9 k, diagonal blocks 6.3 k, columns and operands
+// 4.6 k, products and epilogue of M and A 3.1 k, inverse 5.6 k, w and u 2.3 k, P and R 3.7 k.
 #include "gdn_cw.cuh"
 #include "gdn_inverse.cuh"
 #include "host_util.h"
 
 namespace lg {
 
-constexpr int kDg = 17;                               // row stride (floats) of the diagonal-block buffers
+// row strides (floats) of the diagonal blocks: A by rows, M by columns (transposed, as the inverse reads it)
+constexpr int kDg = 17, kDm = 20;
 
 // Six tiles of 16 KB that change hands:
-//   tile       0            1            2                3            4                        5
-//   loaded     k            q            g, then alpha (fp32)          k to the end of its four rows (fp32), decays over four rows
-//   products   k e          q e          k to the start of later blocks   k exp(G_last - G)     b gamma k
-//   inverse    M and scratch             [T; A]           v, beta v    "                        "
-//   then       w            u            "                "            P (without the delta term R)
+//   tile       0            1            2                3                4                    5
+//   loaded     k            q            g, then alpha (fp32)              k to the end of its four rows (fp32), decays over four rows
+//   products   k e          q e          b gamma k        k to blocks 3, 1 k exp(G_last - G)    k to block 2
+//   inverse    M and scratch             "                v, beta v        "                    [T; A]  (without delta: 2)
+//   then       the next k   and q        w                u                P                    (without delta: R)
+//   then       "            "            the next g                        "
 struct PrepCwSmem {
   static constexpr int kTile = 16384, oF = 6 * kTile;
-  // floats: diagonal blocks of A and M [64][kDg] each, betas [64], Bb and Af [4][128]
-  static constexpr int kFloats = 128 * kDg + 64 + 1024;
-  static constexpr int kBytes = oF + kFloats * 4 + static_cast<int>(sizeof(CtaShared)) + 1024;
+  // floats: diagonal blocks of M [64][kDm] and A [64][kDg], betas [2][64], Bb and Af [4][128]
+  static constexpr int kFloats = 64 * (kDm + kDg) + 128 + 1024;
+  static constexpr int kBytes = oF + kFloats * 4 + 2 * static_cast<int>(sizeof(ChunkAt)) + static_cast<int>(sizeof(CtaShared)) + 1024;
 };
 
 // Sums over the 16 lanes of a half-warp of N values per lane (N = 16 or 8): lane l ends up with the total of value l
@@ -111,50 +120,44 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
   extern __shared__ unsigned char smem_raw[];
   unsigned char* sm = align1024(smem_raw);
   auto tile = [&](int i) { return sm + i * S::kTile; };
-  unsigned char *tK = tile(0), *tQ = tile(1), *LA = tile(0), *KR = tile(2), *KD = tile(4), *GK = tile(5);
-  unsigned char *TA = tile(2), *BV = tile(3), *WU = tile(0), *SP = tile(4);
+  unsigned char *tK = tile(0), *tQ = tile(1), *LA = tile(0), *KR = tile(3), *KR2 = tile(5), *KD = tile(4), *GK = tile(2);
+  unsigned char *TA = tile(DELTA ? 5 : 2), *BV = tile(3), *WU = tile(2), *SP = tile(4);
   float *G = reinterpret_cast<float*>(tile(2)), *kfd = reinterpret_cast<float*>(tile(4)), *Bg = kfd + 48 * kK;
   float* Mt = reinterpret_cast<float*>(tile(0));
   static_assert((kInvMtFloats + kInvScratchFloats) * 4 <= 2 * S::kTile, "M and the inverse's scratch");
-  float* Adg = reinterpret_cast<float*>(sm + S::oF);
-  float* Mdg = Adg + 64 * kDg;
-  float* betas = Mdg + 64 * kDg;
-  float* Bb = betas + 64;
+  float* Mdg = reinterpret_cast<float*>(sm + S::oF);
+  float* Adg = Mdg + 64 * kDm;
+  float* betas2 = Adg + 64 * kDg;                      // of this chunk and the next
+  float* Bb = betas2 + 128;
   float* Af = Bb + 512;
-  CtaShared* cs = reinterpret_cast<CtaShared*>(Af + 512);
+  ChunkAt* where = reinterpret_cast<ChunkAt*>(Af + 512);      // this chunk and the next
+  CtaShared* cs = reinterpret_cast<CtaShared*>(where + 2);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, quad = warp & 3, b0 = (warp >> 2) * NB, d = quad * 32 + lane;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, quad = warp & 3, b0 = (warp >> 2) * NB;
   CtaCtl ctl{p.status, &cs->abort_flag};
   uint64_t *in0 = &cs->bar[0], *in1 = &cs->bar[1], *m1 = &cs->bar[2], *m2 = &cs->bar[3], *m3 = &cs->bar[4];
   const int nchunks = p.nbh * p.cn;
-  struct At { int bh, c, z, b, h; };
-  auto at = [&](int n) {
-    At a;
-    a.bh = p.bh0 + n / p.cn;
-    a.c = p.c0 + n % p.cn;
-    a.z = a.bh * p.NT + a.c;
-    a.b = a.bh / p.H;
-    a.h = a.bh % p.H;
-    return a;
-  };
-  auto load_kqg = [&](const At& a) {      // (tid 0)
+  auto load_k = [&](const ChunkAt& a) {      // (one thread each)
     mbar_expect_tx(in0, 65536u);
-    tma_load_4d(tile(2), &mg, in0, 0, a.h, a.c * kC, a.b);
-    for (int t = 0; t < 2; ++t) {
-      tma_load_4d(tK + t * 8192, &mk, in0, t * 64, a.h, a.c * kC, a.b);
-      tma_load_4d(tQ + t * 8192, &mq, in0, t * 64, a.h, a.c * kC, a.b);
-    }
+    for (int t = 0; t < 2; ++t) tma_load_4d(tK + t * 8192, &mk, in0, t * 64, a.h, a.c * kC, a.b);
   };
-  auto load_v = [&](const At& a) {
+  auto load_q = [&](const ChunkAt& a) {
+    for (int t = 0; t < 2; ++t) tma_load_4d(tQ + t * 8192, &mq, in0, t * 64, a.h, a.c * kC, a.b);
+  };
+  auto load_g = [&](const ChunkAt& a) { tma_load_4d(tile(2), &mg, in0, 0, a.h, a.c * kC, a.b); };
+  auto load_v = [&](const ChunkAt& a) {
     mbar_expect_tx(in1, V * 128u);
     for (int t = 0; t < V / 64; ++t) tma_load_4d(BV + t * 8192, &mv, in1, t * 64, a.h, a.c * kC, a.b);
   };
   if (tid == 0) {
+    where[0] = chunk_at(p, blockIdx.x);
     cs->abort_flag = 0;
     for (int i = 0; i < 5; ++i) mbar_init(&cs->bar[i], 1);
     fence_mbar_init();
     fence_proxy_async();
-    load_kqg(at(blockIdx.x));
+    load_k(where[0]);
+    load_q(where[0]);
+    load_g(where[0]);
   }
   if (warp == 0) {
     tmem_alloc(&cs->tmem_slot, 256);
@@ -165,14 +168,33 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
   tc_fence_after();
   const uint32_t tmem = cs->tmem_slot, lane_base = static_cast<uint32_t>(quad * 32) << 16;      // M | A blocks; [w | u]; [P | R]
 
+  // gates of a chunk, fetched while the chunk before is worked on: beta to shared memory; per channel to L2, by lines of 128 bytes
+  auto fetch_gates = [&](const ChunkAt& a, float* betas) {
+    const int last = p.rows_of(a.c) - 1;
+    const size_t tok0 = (static_cast<size_t>(a.b) * p.L + a.c * kC) * p.H + a.h;
+    if (FULL) {
+      for (int t = tid; t < 256; t += kThreads) {
+        const size_t tok = tok0 + static_cast<size_t>(t >> 2) * p.H;
+        prefetch_l2(p.bch + tok * kK + (t & 3) * 32);
+        prefetch_l2(p.wch + tok * V + (t & (V / 32 - 1)) * 32);
+      }
+    } else if (tid < 64) {
+      async_copy4(betas + tid, p.beta + tok0 + static_cast<size_t>(min(tid, last)) * p.H, tid <= last);
+    }
+  };
+  if (DELTA) fetch_gates(where[0], betas2);
   uint32_t ph = 0;
   for (int n = blockIdx.x; n < nchunks; n += gridDim.x, ph ^= 1u) {
-    const At a = at(n);
+    const float* betas = betas2 + 64 * ph;
     const bool more = n + static_cast<int>(gridDim.x) < nchunks;
-    const int rows = p.rows_of(a.c);
-    const size_t tok0 = (static_cast<size_t>(a.b) * p.L + a.c * kC) * p.H + a.h;
-    float beta_r = 1.f;
-    if (DELTA && !FULL && tid < 64) beta_r = tid < rows ? p.beta[tok0 + static_cast<size_t>(tid) * p.H] : 0.f;
+    int d = quad * 32 + lane;                  // this thread's channel; addresses made from it are made anew in every phase
+    auto anew = [&]() { asm volatile("" : "+r"(d)); };
+    anew();
+    auto token = [&](int r) {                  // row r of the chunk in the user's tensors
+      const ChunkAt a = where[ph];
+      return (static_cast<size_t>(a.b) * p.L + a.c * kC + r) * p.H + a.h;
+    };
+    auto rec = [&](size_t off, size_t size) { return p.saved + off + static_cast<size_t>(where[ph].z) * size; };
 
     // ---- alphas, in place of g; decays of the blocks
     mbar_wait_warp(in0, ph, ctl, 501);
@@ -184,10 +206,11 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
       }
       fence_proxy_async();
     }
-    if (DELTA && tid < 64) betas[tid] = beta_r;
+    if (DELTA && !FULL) async_copy_wait();
     if (tid == 0) bulk_wait_read();        // the chunk before has left tiles 4 and 5
     __syncthreads();
     if (NORM && tid == 0 && p.keep_norm) {
+      const ChunkAt a = where[ph];
       for (int t = 0; t < p.Kr / 64; ++t) {
         tma_store_4d(&mn.k, tK + t * 8192, t * 64, a.h, a.c * kC, a.b);
         tma_store_4d(&mn.q, tQ + t * 8192, t * 64, a.h, a.c * kC, a.b);
@@ -220,114 +243,138 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
       Af[blk * kK + d] = al[0];
     }
     __syncthreads();
-    // ---- diagonal blocks, exact.  Half-warp (block, j): rows j and 15 - j - 17 pairs for every j, 5 of them inside the
-    // rows' own groups and 3 x 4 with earlier groups; lane: channels 4 c .. 4 c + 3 of either half.
-#pragma unroll 1
-    for (int it = 0; it < NB; ++it) {
-      const int c = lane & 15, j = warp & 7, db = (NB == 1 ? warp >> 3 : it) * 2 + (lane >> 4);
-      const float* al0 = G + 4 * c;        // alpha of row r: + 128 r; the other half: + 64
+    if (tid == kThreads - 1 && more) where[ph ^ 1u] = chunk_at(p, n + gridDim.x);
+    // ---- diagonal blocks, exact.  A half-warp has one block, a lane its channels 4 c .. 4 c + 3 of either half.  Work comes in two
+    // kinds: the ten pairs of a group of four rows, and the sixteen of a group's rows with an earlier group, whose rows lie ready,
+    // decayed to the end of their group.  A warp takes the same of either kind for its two blocks; a block's ten pieces are dealt
+    // out by their length.
+    {
+      constexpr int kW = 16 / NB / 2;              // warps per two blocks
+      const int db = 2 * (warp / kW) + (lane >> 4);
+      int c = lane & 15;
+      asm volatile("" : "+r"(c));
+      const int w = NB == 2 ? (warp + 2 * (warp / kW)) & 3 : warp & 7;      // (the SM's quarters get the same)
+      // own group of rows, or none; rows A with the earlier groups B, B - 1, ... (nB of them)
+      const int own = NB == 2 || w < 4 ? w : -1;
+      const int A = NB == 2 ? (w == 0 ? 3 : w == 1 ? 2 : w == 2 ? 3 : 1) : (w == 0 || w == 7 ? 2 : w == 1 ? 1 : 3);
+      int B = NB == 2 ? (w == 0 ? 2 : w == 1 ? 1 : 0) : (w == 4 ? 2 : w == 5 || w == 7 ? 1 : 0);
+      int nB = NB == 2 ? (w < 2 ? 2 : 1) : (w == 2 || w == 3 ? 0 : 1);
       const unsigned char* kt = tK + (c & 1) * 8;
       const unsigned char* qt = tQ + (c & 1) * 8;
       auto at16 = [&](int r) { return r * 128 + (((c >> 1) ^ (r & 7)) << 4); };
-      const f2 one = pack2(1.f, 1.f), zero = pack2(0.f, 0.f);
-      // sums of one row against one source row: A, and M where the delta term wants it
-      auto dots = [&](const f2* t, const f2* qi, const f2* ki, float& sa, float& sm_) {
-        f2 aa = zero, mm = zero;
+      auto row = [&](const unsigned char* t, int r, f2* x) {
+        ld4_pairs<F16>(t + at16(r), x);
+        ld4_pairs<F16>(t + 8192 + at16(r), x + 2);
+      };
+      auto row32 = [&](const float* x, int r, f2* y) {
+        ld_pairs(x + r * kK + 4 * c, y);
+        ld_pairs(x + r * kK + 64 + 4 * c, y + 2);
+      };
+      auto times = [&](f2* x, const f2* y) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          aa = fma2(qi[e], t[e], aa);
-          if (DELTA) mm = fma2(ki[e], t[e], mm);
-        }
-        sa = sum2(aa);
-        sm_ = DELTA ? sum2(mm) : 0.f;
+        for (int e = 0; e < 4; ++e) x[e] = mul2(x[e], y[e]);
+      };
+      auto erase = [&](int r, f2* x) {             // per-channel erase gate of the row
+        const float* bp = p.bch + token(r) * kK + 4 * c;
+        f2 b[4];
+        ld_pairs(bp, b);
+        ld_pairs(bp + 64, b + 2);
+        times(x, b);
+      };
+      auto dot = [&](const f2* x, const f2* y) {
+        f2 s = mul2(x[0], y[0]);
+#pragma unroll
+        for (int e = 1; e < 4; ++e) s = fma2(x[e], y[e], s);
+        return sum2(s);
       };
       auto store = [&](int i, int s, bool is_m, float x) {
         const int r = db * 16 + i;
-        if (is_m) Mdg[r * kDg + s] = s < i ? betas[r] * x : 0.f;
+        if (is_m) Mdg[(db * 16 + s) * kDm + i] = FULL ? x : betas[r] * x;
         else Adg[r * kDg + s] = p.scale * x;
       };
-      const int i0 = 15 - j, i1 = j;
-      f2 q0[4], k0[4], q1[4], k1[4];               // the two rows; later times their decay
-      float v[16];
-      auto own_group = [&](int i, f2* qi, f2* ki, float* out) {
-        const int r = db * 16 + i;
-        ld4_pairs<F16>(qt + at16(r), qi);
-        ld4_pairs<F16>(qt + 8192 + at16(r), qi + 2);
-        ld4_pairs<F16>(kt + at16(r), ki);
-        ld4_pairs<F16>(kt + 8192 + at16(r), ki + 2);
-        if (FULL) {
-          const float* bp = p.bch + (tok0 + static_cast<size_t>(r) * p.H) * kK + 4 * c;
-          f2 b[4];
-          ld_pairs(bp, b);
-          ld_pairs(bp + 64, b + 2);
+      if (own >= 0) {
+        f2 t[4][4];                                // source rows, decayed to the row in hand
+        float v[16];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) ki[e] = mul2(ki[e], b[e]);
-        }
-        f2 ratio[4] = {one, one, one, one};
+        for (int r = 0; r < 4; ++r) {
+          const int rr = db * 16 + 4 * own + r;
+          f2 q[4], k[4], a4[4];
+          row(qt, rr, q);
+          row(kt, rr, k);
+          if (r) {
+            row32(G, rr, a4);
 #pragma unroll
-        for (int u = 3; u >= 0; --u) {
-          out[u] = out[4 + u] = 0.f;
-          if (u > (i & 3)) continue;               // (the same for the whole warp)
-          const int s = (i & ~3) + u, rs = db * 16 + s;
-          f2 ks[4], as[4];
-          ld4_pairs<F16>(kt + at16(rs), ks);
-          ld4_pairs<F16>(kt + 8192 + at16(rs), ks + 2);
-          ld_pairs(al0 + kK * rs, as);
-          ld_pairs(al0 + kK * rs + 64, as + 2);
+            for (int s = 0; s < r; ++s) times(t[s], a4);
+          }
 #pragma unroll
-          for (int e = 0; e < 4; ++e) ks[e] = mul2(ratio[e], ks[e]);
-          dots(ks, qi, ki, out[u], out[4 + u]);
+          for (int e = 0; e < 4; ++e) t[r][e] = k[e];
+          if (DELTA && FULL) erase(rr, k);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) ratio[e] = mul2(ratio[e], as[e]);
-        }
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {              // the row's decay from the end of the group before its own
-          qi[e] = mul2(qi[e], ratio[e]);
-          if (DELTA) ki[e] = mul2(ki[e], ratio[e]);
-        }
-      };
-      own_group(i0, q0, k0, v);
-      own_group(i1, q1, k1, v + 8);
-      {
-        const float t = half_warp_sum<16>(v, lane);
-        const int i = (c & 8) ? i1 : i0, s = (i & ~3) + (c & 3);
-        if (s <= i) store(i, s, (c & 4) != 0, t);
-      }
-      // earlier group B of a row; then the row's decay goes on over that group
-      auto earlier = [&](int B, f2* qi, f2* ki, float* out) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          f2 t[4];
-          ld_pairs(kfd + (db * 12 + 4 * B + u) * kK + 4 * c, t);
-          ld_pairs(kfd + (db * 12 + 4 * B + u) * kK + 64 + 4 * c, t + 2);
-          dots(t, qi, ki, out[u], out[4 + u]);
-        }
-        if (B > 0) {
-          f2 g[4];
-          ld_pairs(Bg + (db * 4 + B) * kK + 4 * c, g);
-          ld_pairs(Bg + (db * 4 + B) * kK + 64 + 4 * c, g + 2);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            qi[e] = mul2(qi[e], g[e]);
-            if (DELTA) ki[e] = mul2(ki[e], g[e]);
+          for (int s = 0; s <= r; ++s) {
+            v[r * (r + 1) / 2 + s] = dot(q, t[s]);
+            if (s < r) v[10 + r * (r - 1) / 2 + s] = DELTA ? dot(k, t[s]) : 0.f;
           }
         }
-      };
-      // row 15 - j has three earlier groups for j < 4 and two otherwise, row j none and one
-      const int B0 = (i0 >> 2) - 1;
-      earlier(B0, q0, k0, v);
-      earlier(B0 - 1, q0, k0, v + 8);
-      {
-        const float t = half_warp_sum<16>(v, lane);
-        store(i0, 4 * (B0 - (c >> 3)) + (c & 3), (c & 4) != 0, t);
+        const float x = half_warp_sum<16>(v, lane);
+        // lane c: rows and source rows of A's ten values, then of M's six, two bits each
+        constexpr uint32_t kOwnRow = 0xfe9ffa94u, kOwnSrc = 0x910e4910u;
+        const int r = static_cast<int>(kOwnRow >> (2 * c)) & 3, s = static_cast<int>(kOwnSrc >> (2 * c)) & 3;
+        if (DELTA || c < 10) store(4 * own + r, 4 * own + s, c >= 10, x);
+        if (DELTA && c < 10 && r == s) Mdg[(db * 16 + 4 * own + s) * kDm + 4 * own + s] = 0.f;
       }
-      if (j < 4) earlier(0, q0, k0, v);
-      else earlier(0, q1, k1, v);
-      {
-        const float t = half_warp_sum<8>(v, lane);
-        store(j < 4 ? i0 : i1, (c >> 1) & 3, (c & 8) != 0, t);
+      if (nB > 0) {
+        f2 q[4][4], k[4][4], e4[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {              // the rows, decayed from the end of the group before theirs
+          const int rr = db * 16 + 4 * A + r;
+          row(qt, rr, q[r]);
+          if (DELTA) row(kt, rr, k[r]);
+          if (DELTA && FULL) erase(rr, k[r]);
+          if (r == 0) {
+            row32(G, rr, e4);
+          } else {
+            f2 a4[4];
+            row32(G, rr, a4);
+            times(e4, a4);
+          }
+          times(q[r], e4);
+          if (DELTA) times(k[r], e4);
+        }
+        auto over = [&](int m) {                   // ... and over group m
+          f2 g[4];
+          row32(Bg, db * 4 + m, g);
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            times(q[r], g);
+            if (DELTA) times(k[r], g);
+          }
+        };
+#pragma unroll 1
+        for (int m = A - 1; m > B; --m) over(m);
+#pragma unroll 1
+        for (;;) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            float v[16];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              f2 t[4];
+              row32(kfd, db * 12 + 4 * B + 2 * h + u, t);
+#pragma unroll
+              for (int r = 0; r < 4; ++r) {
+                v[8 * u + 2 * r] = dot(q[r], t);
+                v[8 * u + 2 * r + 1] = DELTA ? dot(k[r], t) : 0.f;
+              }
+            }
+            const float x = half_warp_sum<16>(v, lane);
+            if (DELTA || !(c & 1)) store(4 * A + ((c >> 1) & 3), 4 * B + 2 * h + (c >> 3), c & 1, x);
+          }
+          if (--nB == 0) break;
+          over(B--);
+        }
       }
     }
+    anew();
     // ---- this thread's columns: decays, k, q
     float al[NB][16];
     uint32_t kp[NB][8], qp[NB][8];
@@ -346,7 +393,7 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
       const int blk = b0 + bb;
       const BlockDecays bd = block_decays(Bb, Af, blk, d);
       const float gam0 = bd.pre * al[bb][0];     // gamma of the block's first token
-      if (blk == 3) reinterpret_cast<float*>(p.saved + p.lay.ad)[static_cast<size_t>(a.z) * kK + d] = bd.pre * Bb[3 * kK + d];
+      if (blk == 3) reinterpret_cast<float*>(p.saved + p.lay.ad)[static_cast<size_t>(where[ph].z) * kK + d] = bd.pre * Bb[3 * kK + d];
       float x[16], y[16], f = 1.f, e = 1.f;
 #pragma unroll
       for (int i = 15; i >= 0; --i) {            // k to the end of its block ...
@@ -361,12 +408,11 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
         if (I <= blk) continue;
 #pragma unroll
         for (int i = 0; i < 16; ++i) y[i] = x[i] * bd.cup[I - 1];
-        // columns: block 3's 48 and block 1's 16 in the first atom, block 2's 32 in the second
-        unsigned char* t = KR + (I == 2 ? 16384 : 0);
-        write_column(t, I == 1 ? 3 : blk, d, y);
+        // columns: block 3's 48 and block 1's 16 in one tile, block 2's 32 in the other
+        write_column(I == 2 ? KR2 : KR, I == 1 ? 3 : blk, d, y);
       }
       // scale gamma q leaves for its record, the image of a [64 tokens][128 channels] tile: a warp writes 64 bytes of a row
-      unsigned char* qg = p.saved + p.lay.qg + static_cast<size_t>(a.z) * 16384;
+      unsigned char* qg = rec(p.lay.qg, 16384);
       const float sg = p.scale * gam0;
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
@@ -377,11 +423,16 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
       write_column(LA + 16384, blk, d, y);
       if (DELTA) {
         e = 1.f;
+        if (FULL) {
+          const float* bp = p.bch + token(blk * 16) * kK + d;
+#pragma unroll
+          for (int i = 0; i < 16; ++i) y[i] = bp[static_cast<size_t>(i) * p.H * kK];
+        }
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           if (i) e *= al[bb][i];
           x[i] = half_of(kp[bb][i >> 1], i & 1) * e;
-          if (FULL) x[i] *= p.bch[(tok0 + static_cast<size_t>(blk * 16 + i) * p.H) * kK + d];
+          if (FULL) x[i] *= y[i];
         }
         write_column(LA, blk, d, x);             // left factor of M (without the row's beta)
 #pragma unroll
@@ -391,88 +442,107 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
     }
     sync_for_issue();
 
+    anew();
     // ---- off-diagonal blocks of M (rows 0-63) and A (rows 64-127) on the tensor cores
     if (warp == 0) {
       tc_fence_after();
       const uint32_t leader = elect_leader();
       issue_product_led(leader, tmem, Tile{smem_u32(LA), 128, true}, Tile{smem_u32(KR), 128, true}, 64, 128, 0u);
-      issue_product_led(leader, tmem + 64, Tile{smem_u32(LA), 128, true}, Tile{smem_u32(KR) + 16384, 128, true}, 32, 128, 0u);
+      issue_product_led(leader, tmem + 64, Tile{smem_u32(LA), 128, true}, Tile{smem_u32(KR2), 128, true}, 32, 128, 0u);
       umma_commit_led(leader, m1);
+    } else if (warp == 1 && lane == 0 && more) {      // the next g and v to L2: g's tiles are free late, and v is wanted soon then
+      const ChunkAt a = where[ph ^ 1u];
+      tma_prefetch_4d(&mg, 0, a.h, a.c * kC, a.b);
+      for (int t = 0; t < V / 64; ++t) tma_prefetch_4d(&mv, t * 64, a.h, a.c * kC, a.b);
     }
     __syncwarp();
+    constexpr int kWv = 64 * (V / 8) / kThreads;
+    float wv[FULL ? kWv : 1][8];               // write gates of this thread's pieces of v, requested in the products' shadow
+    if (FULL)
+#pragma unroll
+      for (int j = 0; j < kWv; ++j) {
+        const int idx = tid + j * kThreads;
+        ld8(p.wch + token(idx / (V / 8)) * V + (idx % (V / 8)) * 8, wv[FULL ? j : 0]);
+      }
     mbar_wait_warp(m1, ph, ctl, 502);
     tc_fence_after();
-    if (tid == 0) load_v(a);
-#pragma unroll 1
-    for (int blk = b0; blk < b0 + NB; ++blk) {
-      // thread: accumulator lane t = quad * 32 + lane (row r of M for lanes 0-63, of A for 64-127), columns of block blk
-      const int t = d, r = t & 63, I = r >> 4, I0 = 2 * (quad & 1);      // a warp's lanes are rows of blocks I0 and I0 + 1
-      float x[16], y[16];
-#pragma unroll
-      for (int e = 0; e < 16; ++e) x[e] = 0.f;
+    if (tid == 0) load_v(where[ph]);
+    if (DELTA && more) fetch_gates(where[ph ^ 1u], betas2 + 64 * (ph ^ 1u));
+    // thread: accumulator lane quad * 32 + lane (row r of M for lanes 0-63, of A for 64-127), columns of block blk.  A warp's lanes are
+    // rows of blocks I0 and I0 + 1.  Of M only the blocks below the diagonal ones go to Mt, which has it transposed.
+    {
+      const int r = d & 63, I = r >> 4, I0 = 2 * (quad & 1);
       auto col = [](int rb, int cb) { return rb == 1 ? 48 : (rb == 2 ? 64 : 0) + 16 * cb; };
-      if (blk < I0 + 1) {
-        tmem_ld16(tmem + lane_base + col(I0 + 1, blk), y);
-        tmem_ld_wait();
-        if (I == I0 + 1)
+#pragma unroll 1
+      for (int blk = b0; blk < b0 + NB; ++blk) {
+        float x[16];
+        if (blk <= I0) {
+          float y[16];
+          tmem_ld16(tmem + lane_base + col(I0 + 1, blk), x);
+          tmem_ld16(tmem + lane_base + col(I0, blk < I0 ? blk : 0), y);      // (not used for blk = I0)
+          tmem_ld_wait();
 #pragma unroll
-          for (int e = 0; e < 16; ++e) x[e] = y[e];
-      }
-      if (blk < I0) {
-        tmem_ld16(tmem + lane_base + col(I0, blk), y);
-        tmem_ld_wait();
-        if (I == I0)
+          for (int e = 0; e < 16; ++e) x[e] = I == I0 ? y[e] : x[e];
+        } else {
 #pragma unroll
-          for (int e = 0; e < 16; ++e) x[e] = y[e];
-      }
-      if (t < 64) {
-        if (DELTA) {
-          const float be = betas[r];
+          for (int e = 0; e < 16; ++e) x[e] = 0.f;
+        }
+        if (quad < 2) {
+          if (DELTA && blk < I) {
+            const float be = betas[r];
 #pragma unroll
-          for (int e = 0; e < 16; ++e) {
-            x[e] *= be;
-            if (I == blk) x[e] = blk * 16 + e < r ? Mdg[r * kDg + e] : 0.f;
+            for (int e = 0; e < 16; ++e) Mt[(blk * 16 + e) * kMt + r] = FULL ? x[e] : x[e] * be;
           }
+        } else {
+          if (blk < I) {
 #pragma unroll
-          for (int e = 0; e < 16; ++e) Mt[(blk * 16 + e) * kMt + r] = x[e];
-        }
-      } else {
+            for (int e = 0; e < 16; ++e) x[e] *= p.scale;
+          } else if (blk == I) {
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          x[e] *= p.scale;
-          if (I == blk) x[e] = blk * 16 + e <= r ? Adg[r * kDg + e] : 0.f;
+            for (int e = 0; e < 16; ++e) x[e] = e <= (r & 15) ? Adg[r * kDg + e] : 0.f;
+          } else if (blk > I) {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) x[e] = 0.f;
+          }
+          write_row16(TA, 64 + r, blk, x);
         }
-        write_row16(TA, 64 + r, blk, x);
       }
     }
     tc_fence_before();
     __syncthreads();
 
+    anew();
     // ---- beta v (w v) on the warps that have no part in the inverse, or not in its first step
-    constexpr int kFirst = NB == 1 ? 256 : 64;
+    constexpr int kFirst = FULL ? 0 : NB == 1 ? 256 : 64, kStep = kThreads - kFirst;
     if (tid >= kFirst) {
       mbar_wait_warp(in1, ph, ctl, 505);
-      for (int idx = tid - kFirst; idx < 64 * (V / 8); idx += kThreads - kFirst) {
-        const int r = idx / (V / 8), ch = idx % (V / 8);
+#pragma unroll
+      for (int j = 0; j < (64 * (V / 8) + kStep - 1) / kStep; ++j) {
+        const int idx = tid - kFirst + j * kStep, r = idx / (V / 8), ch = idx % (V / 8);
+        if (idx >= 64 * (V / 8)) break;
         float x[8];
         unpack8_bf16(tile_ld_chunk(BV, r, ch, 64), x);
-        if (DELTA && FULL) {
-          float wv[8];
-          ld8(p.wch + (tok0 + static_cast<size_t>(r) * p.H) * V + ch * 8, wv);
+        if (FULL) {
 #pragma unroll
-          for (int i = 0; i < 8; ++i) x[i] *= wv[i];
-        } else {
-          const float be = DELTA ? betas[r] : 1.f;
+          for (int i = 0; i < 8; ++i) x[i] *= wv[FULL ? j : 0][i];
+        } else if (DELTA) {
+          const float be = betas[r];
 #pragma unroll
           for (int i = 0; i < 8; ++i) x[i] *= be;
         }
         tile_st_chunk(BV, r, ch, 64, pack8_f16(x));
       }
     }
+    auto next_kq = [&]() {                 // tiles 0 and 1 are dead; by warps that have no part in the next step
+      if (more && lane == 0 && warp == 2) load_k(where[ph ^ 1u]);
+      if (more && lane == 0 && warp == 3) load_q(where[ph ^ 1u]);
+      __syncwarp();
+    };
     // ---- T = (I + M)^-1 (fp32, CUDA cores)
     if (DELTA) {
-      unit_lower_inverse64(Mt, Mt + kInvMtFloats, TA, tid);
+      unit_lower_inverse64<kDm, 16 * kDm>(Mt, Mdg, Mt + kInvMtFloats, TA, tid);
       sync_for_issue();
+      next_kq();
       // ---- [w | u] = T [b gamma k | beta v]
       if (warp == 0) {
         tc_fence_after();
@@ -481,30 +551,34 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
         issue_product_led(leader, tmem + 128, Tile{smem_u32(TA), 128, false}, Tile{smem_u32(BV), 64, true}, V, 64, 0u);
         umma_commit_led(leader, m2);
         if (tid == 0) {
-          if (p.lean < 2) bulk_s2g(p.saved + p.lay.ta + static_cast<size_t>(a.z) * p.lay.sz_ta, TA, 16384);
-          else bulk_s2g(p.saved + p.lay.ta + static_cast<size_t>(a.z) * p.lay.sz_ta + 8192, TA + 8192, 8192);      // A only
+          if (p.lean < 2) bulk_s2g(rec(p.lay.ta, p.lay.sz_ta), TA, 16384);
+          else bulk_s2g(rec(p.lay.ta, p.lay.sz_ta) + 8192, TA + 8192, 8192);      // A only
           bulk_commit();
         }
       }
       __syncwarp();
+    anew();
       mbar_wait_warp(m2, ph, ctl, 503);
       tc_fence_after();
       if (quad < 2) {                      // rows 0-63; the warps of a quadrant split the columns
 #pragma unroll 1
-        for (int jb = warp >> 2; jb < (128 + V) / 32; jb += 4 / NB) {
-          float x[32];
+        for (int jb = 2 * (warp >> 2); jb < (128 + V) / 32; jb += 8 / NB) {
+          float x[64];
           tmem_ld32(tmem + lane_base + jb * 32, x);
+          tmem_ld32(tmem + lane_base + jb * 32 + 32, x + 32);
           tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 4; ++i) tile_st_chunk(WU, d, jb * 4 + i, 64, pack8_f16(x + 8 * i));
+          for (int i = 0; i < 8; ++i) tile_st_chunk(WU, d, jb * 4 + i, 64, pack8_f16(x + 8 * i));
         }
       }
+      if (tid == 0) bulk_wait_read();      // [T; A] has left tile 5
       sync_for_issue();
     } else {
       fence_proxy_async();
       __syncthreads();
+      next_kq();
       if (tid == 0) {                      // A only: without the delta term nothing reads T
-        bulk_s2g(p.saved + p.lay.ta + static_cast<size_t>(a.z) * p.lay.sz_ta + 8192, TA + 8192, 8192);
+        bulk_s2g(rec(p.lay.ta, p.lay.sz_ta) + 8192, TA + 8192, 8192);
         bulk_commit();
       }
     }
@@ -517,43 +591,45 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
       umma_commit_led(leader, m3);
       if (tid == 0) {
         if (DELTA) {
-          bulk_s2g(p.saved + p.lay.w + static_cast<size_t>(a.z) * p.lay.sz_w, WU, 16384);
-          bulk_s2g(p.saved + p.lay.u + static_cast<size_t>(a.z) * p.lay.sz_u, WU + 16384, V * 128);
+          bulk_s2g(rec(p.lay.w, p.lay.sz_w), WU, 16384);
+          bulk_s2g(rec(p.lay.u, p.lay.sz_u), WU + 16384, V * 128);
         } else if (!p.lean) {            // (u is v)
-          bulk_s2g(p.saved + p.lay.u + static_cast<size_t>(a.z) * p.lay.sz_u, BV, V * 128);
+          bulk_s2g(rec(p.lay.u, p.lay.sz_u), BV, V * 128);
         }
         bulk_commit();
       }
     }
     __syncwarp();
+    anew();
     mbar_wait_warp(m3, ph, ctl, 504);
     tc_fence_after();
-    if (tid == 0 && more) {                // tiles 0 to 3 are dead once their records have left
+    if (tid == 0 && more) {                // tiles 2 and 3 are dead once their records have left
       bulk_wait_read();
-      load_kqg(at(n + gridDim.x));
+      load_g(where[ph ^ 1u]);
     }
     // P leaves as its record image through the tiles of the last operands, R (16 columns of a row are 32 bytes of its record,
     // the rows of a warp 1 KB) directly; the warps of a lane quadrant split the columns
-    unsigned char* r_g = p.saved + p.lay.r + static_cast<size_t>(a.z) * p.lay.sz_r;
+    unsigned char* r_g = rec(p.lay.r, p.lay.sz_r);
 #pragma unroll 1
-    for (int jb = warp >> 2; jb < (DELTA ? 128 + V : V) / 32; jb += 4 / NB) {
-      float x[32];
+    for (int jb = 2 * (warp >> 2); jb < (DELTA ? 128 + V : V) / 32; jb += 8 / NB) {
+      float x[64];
       tmem_ld32(tmem + lane_base + jb * 32, x);
+      tmem_ld32(tmem + lane_base + jb * 32 + 32, x + 32);
       tmem_ld_wait();
       if (!DELTA || jb < 4) {              // P; R without the delta term, a plain tile image
 #pragma unroll
-        for (int i = 0; i < 4; ++i) tile_st_chunk(SP, d, jb * 4 + i, 128, pack8_f16(x + 8 * i));
+        for (int i = 0; i < 8; ++i) tile_st_chunk(SP, d, jb * 4 + i, 128, pack8_f16(x + 8 * i));
       } else {
         const int c8 = (jb - 4) * 4;
 #pragma unroll
-        for (int i = 0; i < 4; i += 2) st_global_32(r_g + rrec_off(d, c8 + i), pack8_f16(x + 8 * i), pack8_f16(x + 8 * i + 8));
+        for (int i = 0; i < 8; i += 2) st_global_32(r_g + rrec_off(d, c8 + i), pack8_f16(x + 8 * i), pack8_f16(x + 8 * i + 8));
       }
     }
     fence_proxy_async();
     tc_fence_before();
     __syncthreads();
     if (tid == 0) {
-      if (DELTA) bulk_s2g(p.saved + p.lay.p + static_cast<size_t>(a.z) * p.lay.sz_p, SP, 32768);
+      if (DELTA) bulk_s2g(rec(p.lay.p, p.lay.sz_p), SP, 32768);
       else bulk_s2g(r_g, SP, V * 256);
       bulk_commit();
     }

@@ -217,7 +217,7 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
     __syncthreads();
 
     // ---- T = (I + M)^-1 (fp32, CUDA cores)
-    unit_lower_inverse64(Mt, Mt + kInvMtFloats, TA, tid);
+    unit_lower_inverse64(Mt, Mt, Mt + kInvMtFloats, TA, tid);
     mbar_wait_warp(full_v, ph, ctl, 203);
     prep_to_f16(Vt, V * 128, tid);
     __syncthreads();

@@ -49,7 +49,10 @@ __device__ __forceinline__ void store_tile(const f2 (*c)[R], float* dst, int str
 }
 
 // Mt: kInvMtFloats, overwritten.  scratch: kInvScratchFloats.  T leaves as fp16 in rows 0-63 of the 128-row tile TA.
-__device__ __forceinline__ void unit_lower_inverse64(float* Mt, float* scratch, unsigned char* TA, int tid) {
+// diag: the diagonal 16 x 16 blocks, transposed like Mt, SD floats between rows and DB between blocks; of what is not below the
+// diagonal only the diagonal itself is read, as zero.
+template <int SD = kMt, int DB = 16 * kMt + 16>
+__device__ __forceinline__ void unit_lower_inverse64(float* Mt, const float* diag, float* scratch, unsigned char* TA, int tid) {
   const int warp = tid >> 5, lane = tid & 31;
   float* T11 = scratch;                     // rows 0-31 of T
   float* T22t = T11 + 32 * kT32;            // rows 32-63 of its right half, transposed
@@ -58,7 +61,7 @@ __device__ __forceinline__ void unit_lower_inverse64(float* Mt, float* scratch, 
   float* Y = Mt + 32 * kMt;                 // 32 x 32 at stride kMt, where M has zeros
   if (tid < 64) {                           // forward substitution, two rows per packed FMA
     const int b = tid >> 4, j = tid & 15;
-    const float* M = Mt + b * (16 * kMt + 16);
+    const float* M = diag + b * DB;
     f2 x[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) x[q] = pack2(2 * q == j ? 1.f : 0.f, 2 * q + 1 == j ? 1.f : 0.f);
@@ -71,7 +74,7 @@ __device__ __forceinline__ void unit_lower_inverse64(float* Mt, float* scratch, 
 #pragma unroll
       for (int p4 = (k + 1) >> 2; p4 < 4; ++p4) {
         f2 m[2];
-        ld_pairs(M + k * kMt + 4 * p4, m);
+        ld_pairs(M + k * SD + 4 * p4, m);
 #pragma unroll
         for (int t = 0; t < 2; ++t)
           if (2 * (2 * p4 + t) + 1 > k) x[2 * p4 + t] = fma2(m[t], xx, x[2 * p4 + t]);
