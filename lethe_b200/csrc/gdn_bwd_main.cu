@@ -4,10 +4,10 @@
 //
 //   dv2 = de (k dh) + A^T do              dA = tril(do v_new^T),  DS = scale ratio dA
 //   dq  = scale gamma (do h^T) + DS k     dw = -dv2 h^T
-//   dT  = beta_s [dv2 v^T + gamma_s dw k^T],   dM = strict_lower(-T^T dT T^T),   dkk = beta_i ratio dM
-//   dv  = beta (T^T dv2)                  dbgk = T^T dw,  p_i = <dbgk_i, k_i>
+//   dbv = T^T dv2,  dv = beta dbv         dbgk = T^T dw,  p_i = <dbgk_i, k_i>
+//   dM  = strict_lower(-(dbv u^T + dbgk w^T)),   dkk = beta_i ratio dM       (u, w: the forward's WY factors)
 //   dk  = de (v_new dh^T) + DS^T q + (dkk + dkk^T) k + beta gamma dbgk
-//   dbeta = <T^T dv2, v> + gamma p + sum_s dM ratio KK
+//   dbeta = <dbv, v> + gamma p + sum_s dM ratio KK
 //   dg = reverse cumulative sum of dG, dG_i = <scale gamma (do h^T), q> + rowsum(dA A) - colsum(dA A) - de_i <v_new, k dh>
 //        + rowsum(dkk KK) - colsum(dkk KK) + beta p gamma,   and at the chunk's last row  exp(G_last) <dh, h> + sum_i dde_i
 //
@@ -21,8 +21,15 @@
 // [token][token] keeps tokens in the lanes (64 of 128; for dv2 in lanes 64-127, through views that start 64 rows early).
 // Decays and gates are applied in fp32 in the epilogues; no scaled copy of k, q or v is ever an operand.
 //
-// Two CTAs share an SM at d_v = 64 (256 tensor-memory columns, 109 KB): six dependent product groups per chunk are a chain
-// of latencies that one CTA cannot fill.  CTAs are persistent and fetch the next chunk's tiles as theirs fall free.
+// dM.  The VJP of the inverse is -T^T dT T^T with dT = dv2 (beta v)^T + dw (beta gamma k)^T; since T^T dv2 = dbv, T^T dw = dbgk,
+// T (beta v) = u and T (beta gamma k) = w, that is -(dbv u^T + dbgk w^T): one product behind two that are wanted anyway, instead of
+// dT, X = dT T^T and -T^T X in a row.
+//
+// Two CTAs share an SM at d_v = 64 (256 tensor-memory columns, 112 KB): five dependent product groups per chunk are a chain
+// of latencies that one CTA cannot fill.  CTAs are persistent and fetch the next chunk's tiles as theirs fall free, which is late
+// for most of them: all are prefetched to L2 under the first products, and copies are issued by threads that issue no products.
+// us, with six groups and without the prefetch, and now: d_v = 64, 512 chunks 44 -> 40, 4096 230 -> 226; d_v = 128, 512 chunks 62
+// -> 54; without the delta term d_v = 128, 4096 chunks 265 -> 191, d_v = 64, 1692 chunks 75 -> 64.
 #include "gdn_cw.cuh"
 #include "host_util.h"
 
@@ -39,7 +46,7 @@ enum ScMode {
 };
 
 struct ScBars {
-  uint64_t in0, in1, m1, m2, m3, mV, m4, m5, m6;
+  uint64_t in0, in1, inU, m1, m2, m3, m4, m5;
   uint32_t tmem_slot;
   int abort_flag;
 };
@@ -49,23 +56,26 @@ struct ScGates { float G[64], beta[64], de[64], gam[64]; };      // cumulative l
 template <int V>
 struct ScSmem {
   static constexpr int kVT = V * 128;
-  static constexpr int oQ = 0;                      // q; then dk on its way out
+  static constexpr int oQ = 0;                      // q; then (d_v = 64) dk on its way out
   static constexpr int oK = oQ + 16384;             // k (directly behind q: early view)
-  static constexpr int oDO = oK + 16384;            // do; with v_new behind it, then dq on its way out
+  static constexpr int oDO = oK + 16384;            // do; with v_new behind it, then dq on its way out, then (d_v = 64) w
   static constexpr int oVN = oDO + kVT;             // v_new
   static constexpr int oV = oVN + kVT;              // v; then dv on its way out
   static constexpr int oT = oV + kVT;               // T; then dkk
   static constexpr int oA = oT + 8192;              // A (directly behind T: early view); then DS
-  static constexpr int oH = oA + 8192;              // h; then dw [channel][token]
-  static constexpr int oDH = oH + V * 256;          // dh; then dv2 [token][V], and dT / X behind it
-  static constexpr int oF = oDH + V * 256;
+  static constexpr int oH = oA + 8192;              // h; then dw, then dbgk [channel][token]
+  static constexpr int oDH = oH + V * 256;          // dh; then dv2, then dbv [token][V], and (d_v = 64) u behind it
+  static constexpr int oOwn = oDH + V * 256;        // d_v = 128 has room for tiles of their own: dk, w, u
+  static constexpr bool kOwn = V == 128;
+  static constexpr int oDK = kOwn ? oOwn : oQ, oW = kOwn ? oOwn + 16384 : oDO, oU = kOwn ? oOwn + 32768 : oDH + kVT;
+  static constexpr int oF = kOwn ? oOwn + 49152 : oOwn;
   // warps that reach one lane quadrant: they split the columns of every epilogue
   static constexpr int kCg = V == 64 ? 2 : 4, kThreads = 128 * kCg;
   // floats: gates of this chunk and the next; t1q [4][64], pq [4][64]; t2p, t3p, ddep, rsp, dbm, rvp [kCg][64] each;
   // csp [2][64]; red [32]
   static constexpr int kFloats = 2 * 256 + 2 * 256 + 6 * 64 * kCg + 128 + 32;
-  // An A operand of 64 rows is read as 128: 16 KB from the start of its tile.  The last one is dT / X, kVT into dh.
-  static constexpr int kUsed = oF + kFloats * 4 + static_cast<int>(sizeof(ScBars)), kRead = oDH + kVT + 16384;
+  // An A operand of 64 rows is read as 128: 16 KB from the start of its tile, dbv the last of them.
+  static constexpr int kUsed = oF + kFloats * 4 + static_cast<int>(sizeof(ScBars)), kRead = oDH + kVT + 8192;
   static constexpr int kBytes = (kUsed > kRead ? kUsed : kRead) + 1024;
   static constexpr uint32_t kCols = V == 64 ? 256u : 512u;
 };
@@ -92,7 +102,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
   unsigned char* sm = align1024(smem_raw);
   unsigned char *tQ = sm + S::oQ, *tK = sm + S::oK, *tDO = sm + S::oDO, *tVN = sm + S::oVN, *tV = sm + S::oV, *tT = sm + S::oT;
   unsigned char *tA = sm + S::oA, *tDS = tA, *tH = sm + S::oH, *tDW = tH, *tDH = sm + S::oDH, *tDV = tDH;
-  unsigned char *tX = tDH + S::kVT, *tKKd = tT, *oQt = tDO, *oKt = tQ, *oVt = tV;
+  unsigned char *tBV = tDH, *tBK = tH, *tW = sm + S::oW, *tU = sm + S::oU, *tKKd = tT, *oQt = tDO, *oKt = sm + S::oDK, *oVt = tV;
   ScGates* gates = reinterpret_cast<ScGates*>(sm + S::oF);
   float *t1q = reinterpret_cast<float*>(gates + 2), *pq = t1q + 256;
   float *t2p = pq + 256, *t3p = t2p + 64 * kCg, *ddep = t3p + 64 * kCg, *rsp = ddep + 64 * kCg, *dbm = rsp + 64 * kCg;
@@ -116,15 +126,15 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
   };
   // loads of a chunk (tid 0), by when their destinations fall free in the chunk before
   constexpr uint32_t kIn0 = 32768u + (WY ? V * 128u : 0u) + (DELTA ? 16384u : 8192u) + (SB ? 2u * V * 128 + V * 256 : V * 128u);
-  auto load_a = [&](const At& a) {                // do, v
+  auto load_do = [&](const At& a) {               // do, and without the delta term v as v_new
     mbar_expect_tx(&bars->in0, kIn0);
     for (int t = 0; t < V / 64; ++t) {
-      if (SB) {
-        tma_load_4d(tDO + t * 8192, &mdo, &bars->in0, t * 64, a.h, a.c * kC, a.b);
-        if (!DELTA) tma_load_4d(tVN + t * 8192, &mv, &bars->in0, t * 64, a.h, a.c * kC, a.b);      // v_new is v
-      }
-      if (WY) tma_load_4d(tV + t * 8192, &mv, &bars->in0, t * 64, a.h, a.c * kC, a.b);
+      if (SB) tma_load_4d(tDO + t * 8192, &mdo, &bars->in0, t * 64, a.h, a.c * kC, a.b);
+      if (!DELTA) tma_load_4d(tVN + t * 8192, &mv, &bars->in0, t * 64, a.h, a.c * kC, a.b);
     }
+  };
+  auto load_v = [&](const At& a) {
+    if (WY) for (int t = 0; t < V / 64; ++t) tma_load_4d(tV + t * 8192, &mv, &bars->in0, t * 64, a.h, a.c * kC, a.b);
   };
   auto load_rec = [&](const At& a) {              // v_new, h (dv2 where the first half of the call left it)
     if (SB && DELTA) bulk_g2s(tVN, p.saved + p.lay.vn + static_cast<size_t>(a.z) * p.lay.sz_vn, V * 128, &bars->in0);
@@ -141,6 +151,33 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     else bulk_g2s(tA, ta + 8192, 8192, &bars->in0);
     for (int t = 0; t < 2; ++t) tma_load_4d(tK + t * 8192, &mk, &bars->in0, t * 64, a.h, a.c * kC, a.b);
   };
+  auto load_w = [&](const At& a) {                // the forward's WY factors
+    mbar_expect_tx(&bars->inU, 16384u);
+    bulk_g2s(tW, p.saved + p.lay.w + static_cast<size_t>(a.z) * 16384, 16384, &bars->inU);
+  };
+  auto load_u = [&](const At& a) {
+    mbar_expect_tx(&bars->inU, V * 128u);
+    bulk_g2s(tU, p.saved + p.lay.u + static_cast<size_t>(a.z) * p.lay.sz_u, V * 128, &bars->inU);
+  };
+  // what a chunk will load, to L2: its tiles are free late (before this its loads were waited for, 2 to 5 k cycles per chunk)
+  auto prefetch = [&](const At& a) {
+    for (int t = 0; t < 2; ++t) {
+      tma_prefetch_4d(&mq, t * 64, a.h, a.c * kC, a.b);
+      tma_prefetch_4d(&mk, t * 64, a.h, a.c * kC, a.b);
+    }
+    for (int t = 0; t < V / 64; ++t) {
+      tma_prefetch_4d(&mdo, t * 64, a.h, a.c * kC, a.b);
+      tma_prefetch_4d(&mv, t * 64, a.h, a.c * kC, a.b);
+    }
+    if (DELTA) bulk_prefetch(p.saved + p.lay.vn + static_cast<size_t>(a.z) * p.lay.sz_vn, V * 128);
+    bulk_prefetch(p.saved + p.lay.hc + static_cast<size_t>(a.z + a.bh) * p.lay.sz_hc, V * 256);
+    bulk_prefetch(p.scratch + p.lay.dh + static_cast<size_t>(a.z) * p.lay.sz_dh, V * 256);
+    if (WY) {
+      bulk_prefetch(p.saved + p.lay.w + static_cast<size_t>(a.z) * 16384, 16384);
+      bulk_prefetch(p.saved + p.lay.u + static_cast<size_t>(a.z) * p.lay.sz_u, V * 128);
+    }
+    bulk_prefetch(p.saved + p.lay.ta + static_cast<size_t>(a.z) * p.lay.sz_ta, 16384);
+  };
   auto load_q = [&](const At& a) {
     for (int t = 0; t < 2; ++t) tma_load_4d(tQ + t * 8192, &mq, &bars->in0, t * 64, a.h, a.c * kC, a.b);
   };
@@ -148,7 +185,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
   if (tid == 0) {
     bars->abort_flag = 0;
     mbar_init(&bars->in0, 1); mbar_init(&bars->in1, 1); mbar_init(&bars->m1, 2); mbar_init(&bars->m2, 2);
-    mbar_init(&bars->m3, 1); mbar_init(&bars->mV, 1); mbar_init(&bars->m4, 1); mbar_init(&bars->m5, 1); mbar_init(&bars->m6, 1);
+    mbar_init(&bars->m3, 1); mbar_init(&bars->m4, 1); mbar_init(&bars->m5, 1); mbar_init(&bars->inU, 2);
     fence_mbar_init();
     fence_proxy_async();
     // Older than whatever kernel of the path comes just before this one: the caller's tensors and [T; A].  v_new (the output
@@ -157,7 +194,8 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     // instead of 555.3 at 4096; with the delta term no difference.)
     if (SB) {
       const At a = at(blockIdx.x);
-      load_a(a);
+      load_do(a);
+      load_v(a);
       load_b(a);
       load_q(a);
       if (p.after_scan) load_rec(a);
@@ -201,13 +239,14 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
   // columns; an accumulator that shares columns with an earlier one is issued after that one has been read
   const uint32_t cD = tmem, cAo = tmem + V, cDA = tmem + 2 * V, cDK = tmem + 2 * V + 64;      // k dh, A^T do, dA, (v_new dh^T)^T
   const uint32_t cDQ = tmem, cDWt = tmem + 64, cQI = tmem + 128;                               // (do h^T)^T, (dv2 h^T)^T, (DS k)^T
-  const uint32_t cT1 = tmem, cT2 = tmem + 64, cBV = V == 64 ? tmem + 128 : tmem + 320 + 64;    // dv2 v^T, dw k^T, T^T dv2
-  const uint32_t cX = tmem, cBK = tmem + 64, cKK = tmem + 128, cAcc = tmem;                    // X / dM, (T^T dw)^T, k k^T, dk sums
+  const uint32_t cKK = tmem, cBK = tmem + 64, cBV = V == 64 ? tmem + 128 : tmem + 320 + 64;    // k k^T, (T^T dw)^T, T^T dv2
+  const uint32_t cX = tmem + 128, cAcc = tmem;                                                 // dM, dk sums
   griddep_wait();
   griddep_launch();
   if (tid == 0) {
     if (!SB) {
-      load_a(a);
+      load_do(a);
+      load_v(a);
       load_b(a);
       load_q(a);
     }
@@ -230,8 +269,12 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
 
     const ScGates& gt = gates[ph];
     if (tid == 0 && n != static_cast<int>(blockIdx.x)) {
-      bulk_wait_read();                             // dk of the chunk before has left the q tile
-      load_q(a);
+      bulk_wait_read();                             // dk of the chunk before has left its tile
+      if (!S::kOwn) load_q(a);
+    }
+    if (WY && tid == 0 && (S::kOwn || !SB)) {       // w and u where their tiles are free already
+      load_w(a);
+      load_u(a);
     }
 
     // ---- operands to fp16 in place
@@ -247,14 +290,6 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     if (SB) {
       for (int idx = tid; idx < (DELTA ? 1 : 2) * 64 * (V / 8); idx += kThreads) {      // do (and, without delta, v behind it)
         uint4* c = reinterpret_cast<uint4*>(tDO + idx * 16);
-        float x[8];
-        unpack8_bf16(*c, x);
-        *c = pack8_f16(x);
-      }
-    }
-    if (WY) {
-      for (int idx = tid; idx < 64 * (V / 8); idx += kThreads) {
-        uint4* c = reinterpret_cast<uint4*>(tV + idx * 16);
         float x[8];
         unpack8_bf16(*c, x);
         *c = pack8_f16(x);
@@ -288,6 +323,8 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
         issue_product_led(leader, cAo, Tile{smem_u32(tA) - 8192, 64, true}, Tile{smem_u32(tDO), 64, true}, V, 64, 0u);
         issue_product_led(leader, cDA, Tile{smem_u32(tDO), 64, false}, Tile{smem_u32(tVN), 64, false}, 64, V, 0u);
         umma_commit_led(leader, &bars->m1);
+      } else if (warp == 1 && lane == 0 && more) {
+        prefetch(nx);
       }
       __syncwarp();
       // in their shadow: <dh, h>, element by element on two images of one layout
@@ -360,6 +397,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
         t2p[cg * 64 + r] = t2;
       }
       sync_for_issue();
+      if (WY && !S::kOwn && tid == 32) load_u(a);   // dh is dead
 
       // ---- group 2: (do h^T)^T, (DS k)^T | (dv2 h^T)^T
       if (warp == 0) {
@@ -384,6 +422,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       mbar_wait_warp(&bars->m2, ph, ctl, 413);
       tc_fence_after();
       float t1[16 * kU];
+      const f2 scale2 = pack2(p.scale, p.scale);
 #pragma unroll
       for (int u = 0; u < kU; ++u) {
         uint32_t qp[8];
@@ -393,11 +432,13 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
         tmem_ld16(cQI + lane_base + c0 + 16 * u, y);
         tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const int r = c0 + 16 * u + i;
-          const float dq = p.scale * gt.gam[r] * x[i];
-          t1[16 * u + i] = dq * half_of(qp[i >> 1], i & 1);
-          stage16(oQt, r, d, dq + y[i], p.qk16);
+        for (int j = 0; j < 8; ++j) {               // two tokens
+          const int r = c0 + 16 * u + 2 * j;
+          f2 g;
+          g.u = *reinterpret_cast<const unsigned long long*>(gt.gam + r);
+          const f2 dq = mul2(mul2(scale2, g), pack2(x[2 * j], x[2 * j + 1]));
+          unpack2(mul2(dq, pair_of(qp[j])), t1[16 * u + 2 * j], t1[16 * u + 2 * j + 1]);
+          stage16_two(oQt, r, d, add2(dq, pack2(y[2 * j], y[2 * j + 1])), p.qk16);
         }
         if (DELTA) {
           tmem_ld16(cDWt + lane_base + c0 + 16 * u, x);
@@ -417,11 +458,15 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
         }
       }
       warp_sums<16 * kU>(t1, lane, t1q + quad * 64 + c0);
+      if (tid == 0 && keep) bulk_wait_read();       // dv2 has left its tile, which becomes dbv
       sync_for_issue();
-      if (tid == 0) {
+      if (tid == 96) {                              // (a thread that issues no products: it waits)
         for (int t = 0; t < p.Kr / 64; ++t) tma_store_4d(&mo.dq, oQt + t * 8192, t * 64, a.h, a.c * kC, a.b);
         bulk_commit();
+        bulk_wait_read();
+        if (WY && !S::kOwn) load_w(a);
       }
+      __syncwarp();
     }
     // gate gradient of Stage B (token tid), before the cumulative sum
     float dG = 0.f;
@@ -453,10 +498,12 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       if (warp == 2 && more) sum_gates(nx, gates + (ph ^ 1u));
       if (tid == 0 && more) {
         bulk_wait_read();
-        load_a(nx);
+        load_do(nx);
+        load_v(nx);
         load_rec(nx);
         load_dh(nx);
         load_b(nx);
+        if (S::kOwn) load_q(nx);
       }
       tc_fence_before();
       __syncthreads();
@@ -464,51 +511,30 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       continue;
     }
     if (WY) {
-      // ---- group 3: dT in two accumulators (its gates are applied in fp32), T^T dv2
+      // ---- group 3: T^T dv2, (T^T dw)^T; k k^T
       if (warp == 0) {
         tc_fence_after();
         const uint32_t leader = elect_leader();
-        issue_product_led(leader, cT1, Tile{smem_u32(tDV), 64, false}, Tile{smem_u32(tV), 64, false}, 64, V, 0u);
-        issue_product_led(leader, cT2, Tile{smem_u32(tDW), 128, true}, Tile{smem_u32(tK), 64, false}, 64, 128, 0u);
-        umma_commit_led(leader, &bars->m3);
         issue_product_led(leader, cBV, Tile{smem_u32(tT), 64, true}, Tile{smem_u32(tDV), 64, true}, V, 64, 0u);
-        umma_commit_led(leader, &bars->mV);
+        issue_product_led(leader, cBK, Tile{smem_u32(tDW), 128, false}, Tile{smem_u32(tT), 64, true}, 64, 64, 0u);
+        umma_commit_led(leader, &bars->m3);
+        issue_product_led(leader, cKK, Tile{smem_u32(tK), 64, false}, Tile{smem_u32(tK), 64, false}, 64, 128, 0u);
       }
       __syncwarp();
       mbar_wait_warp(&bars->m3, ph, ctl, 421);
       tc_fence_after();
-      if (quad < 2) {
 #pragma unroll
-        for (int u = 0; u < kU; ++u) {
-          float x[16], y[16];
-          tmem_ld16(cT1 + lane_base + c0 + 16 * u, x);
-          tmem_ld16(cT2 + lane_base + c0 + 16 * u, y);
-          tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const int s = c0 + 16 * u + j;
-            x[j] = gt.beta[s] * fmaf(gt.gam[s], y[j], x[j]);
-          }
-          write_row16(tX, d, kU * cg + u, x);
-        }
+      for (int u = 0; u < kU; ++u) {                // dbgk, where dw was
+        float x[16];
+        tmem_ld16(cBK + lane_base + c0 + 16 * u, x);
+        tmem_ld_wait();
+        write_column(tBK, kU * cg + u, d, x);
       }
-      sync_for_issue();
-      // ---- group 4: X = dT T^T, (T^T dw)^T
-      if (warp == 0) {
-        tc_fence_after();
-        const uint32_t leader = elect_leader();
-        issue_product_led(leader, cX, Tile{smem_u32(tX), 64, false}, Tile{smem_u32(tT), 64, false}, 64, 64, 0u);
-        issue_product_led(leader, cBK, Tile{smem_u32(tDW), 128, false}, Tile{smem_u32(tT), 64, true}, 64, 64, 0u);
-        umma_commit_led(leader, &bars->m4);
-      }
-      __syncwarp();
-      // in its shadow: dv = beta T^T dv2 where v was, and the value part of dbeta
-      mbar_wait_warp(&bars->mV, ph, ctl, 422);
-      tc_fence_after();
-      if (quad < 2) {
+      // dbv (lanes 0-63) as an operand, where dv2 was; dv = beta dbv where v was, and the value part of dbeta
+      float rv = 0.f;
+      auto dbv_columns = [&](bool operand, bool result) {
         const int r = d;
         const float be = gt.beta[r];
-        float rv = 0.f;
 #pragma unroll
         for (int jj = 0; jj < V / (16 * kCg); ++jj) {
           const int cb = cg * (V / kCg) + jj * 16;
@@ -517,8 +543,10 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
           tmem_ld_wait();
 #pragma unroll
           for (int q = 0; q < 2; ++q) {
+            if (operand) tile_st_chunk(tBV, r, cb / 8 + q, 64, pack8_f16(x + 8 * q));
+            if (!result) continue;
             float vv[8];
-            unpack8_f16(tile_ld_chunk(tV, r, cb / 8 + q, 64), vv);
+            unpack8_bf16(tile_ld_chunk(tV, r, cb / 8 + q, 64), vv);
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
               rv += x[8 * q + e] * vv[e];
@@ -527,34 +555,21 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
             tile_st_chunk(oVt, r, cb / 8 + q, 64, pack8_bf16(x + 8 * q));
           }
         }
-        rvp[cg * 64 + r] = rv;
-      }
-      mbar_wait_warp(&bars->m4, ph, ctl, 423);
-      tc_fence_after();
-      if (quad < 2) {
-#pragma unroll
-        for (int u = 0; u < kU; ++u) {
-          float x[16];
-          tmem_ld16(cX + lane_base + c0 + 16 * u, x);
-          tmem_ld_wait();
-          write_row16(tX, d, kU * cg + u, x);
-        }
-      }
+        if (result) rvp[cg * 64 + r] = rv;
+      };
+      if (quad < 2) dbv_columns(true, V == 64);     // (d_v = 64: dM takes the columns)
+      mbar_wait_warp(&bars->inU, ph, ctl, 422);
       sync_for_issue();
-      // ---- group 5: dM = -T^T X, k k^T
+      // ---- group 4: dM = -(dbv u^T + dbgk w^T)
       if (warp == 0) {
         tc_fence_after();
         const uint32_t leader = elect_leader();
-        issue_product_led(leader, cX, Tile{smem_u32(tT), 64, true}, Tile{smem_u32(tX), 64, true}, 64, 64, 0u, true);
-        issue_product_led(leader, cKK, Tile{smem_u32(tK), 64, false}, Tile{smem_u32(tK), 64, false}, 64, 128, 0u);
-        umma_commit_led(leader, &bars->m5);
-        if (tid == 0) {
-          for (int t = 0; t < V / 64; ++t) tma_store_4d(&mo.dv, oVt + t * 8192, t * 64, a.h, a.c * kC, a.b);
-          bulk_commit();
-        }
+        issue_product_led(leader, cX, Tile{smem_u32(tBV), 64, false}, Tile{smem_u32(tU), 64, false}, 64, V, 0u, true);
+        issue_product_led(leader, cX, Tile{smem_u32(tBK), 128, true}, Tile{smem_u32(tW), 64, false}, 64, 128, 1u, true);
+        umma_commit_led(leader, &bars->m4);
       }
       __syncwarp();
-      // p_i = <(T^T dw)_i, k_i> meanwhile
+      // in its shadow: p_i = <(T^T dw)_i, k_i>, and dv at d_v = 128
       {
         float v[16 * kU];
 #pragma unroll
@@ -569,7 +584,8 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
         }
         warp_sums<16 * kU>(v, lane, pq + quad * 64 + c0);
       }
-      mbar_wait_warp(&bars->m5, ph, ctl, 424);
+      if (V == 128 && quad < 2) dbv_columns(false, true);
+      mbar_wait_warp(&bars->m4, ph, ctl, 424);
       tc_fence_after();
       if (quad < 2) {                               // dkk = beta ratio dM, where T was; row and column sums of e = dkk KK
         const int r = d;
@@ -600,6 +616,20 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       sync_for_issue();
     }
     // ---- last group: DS^T q (+ (dkk + dkk^T) k)
+    if (tid == 96) {
+      if (WY) {                                     // dv, staged before the last barrier
+        for (int t = 0; t < V / 64; ++t) tma_store_4d(&mo.dv, oVt + t * 8192, t * 64, a.h, a.c * kC, a.b);
+        bulk_commit();
+      }
+      if (more) {
+        load_do(nx);                                // dq has left (this thread has waited for it), w is read
+        if (WY) {
+          bulk_wait_read();
+          load_v(nx);
+        }
+      }
+    }
+    __syncwarp();
     if (warp == 0) {
       tc_fence_after();
       const uint32_t leader = elect_leader();
@@ -608,19 +638,21 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
         issue_product_led(leader, cAcc, Tile{smem_u32(tK), 64, true}, Tile{smem_u32(tKKd), 64, false}, 64, 64, 1u);
         issue_product_led(leader, cAcc, Tile{smem_u32(tK), 64, true}, Tile{smem_u32(tKKd), 64, true}, 64, 64, 1u);
       }
-      umma_commit_led(leader, &bars->m6);
-      if (tid == 0 && more) {          // dq and dv have left by now; h / dw, dv2 and X are read
-        bulk_wait_read();
-        load_a(nx);
+      umma_commit_led(leader, &bars->m5);
+      if (tid == 0 && more) {          // h / dw / dbgk, dv2 / dbv and u are read
         load_rec(nx);
         if (SB) load_dh(nx);
       }
     }
     __syncwarp();
     if (warp == 2 && more) sum_gates(nx, gates + (ph ^ 1u));
-    mbar_wait_warp(&bars->m6, ph, ctl, 425);
+    mbar_wait_warp(&bars->m5, ph, ctl, 425);
     tc_fence_after();
-    if (tid == 0 && more) load_b(nx);               // [T; A] and k are read
+    if (tid == 0 && more) {                         // [T; A], k and q are read
+      load_b(nx);
+      if (S::kOwn) load_q(nx);
+    }
+    __syncwarp();
 #pragma unroll
     for (int u = 0; u < kU; ++u) {
       float x[16], y[16];
@@ -632,16 +664,26 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       }
       tmem_ld16(cAcc + lane_base + c0 + 16 * u, x);
       tmem_ld_wait();
+      auto pair_at = [](const float* t) {
+        f2 r;
+        r.u = *reinterpret_cast<const unsigned long long*>(t);
+        return r;
+      };
+      f2 acc[8];
 #pragma unroll
-      for (int i = 0; i < 16; ++i) x[i] = fmaf(gt.de[c0 + 16 * u + i], y[i], x[i]);
+      for (int j = 0; j < 8; ++j)
+        acc[j] = fma2(pair_at(gt.de + c0 + 16 * u + 2 * j), pack2(y[2 * j], y[2 * j + 1]), pack2(x[2 * j], x[2 * j + 1]));
       if (WY) {
         tmem_ld16(cBK + lane_base + c0 + 16 * u, y);
         tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 16; ++i) x[i] = fmaf(gt.beta[c0 + 16 * u + i] * gt.gam[c0 + 16 * u + i], y[i], x[i]);
+        for (int j = 0; j < 8; ++j) {
+          const int r = c0 + 16 * u + 2 * j;
+          acc[j] = fma2(mul2(pair_at(gt.beta + r), pair_at(gt.gam + r)), pack2(y[2 * j], y[2 * j + 1]), acc[j]);
+        }
       }
 #pragma unroll
-      for (int i = 0; i < 16; ++i) stage16(oKt, c0 + 16 * u + i, d, x[i], p.qk16);
+      for (int j = 0; j < 8; ++j) stage16_two(oKt, c0 + 16 * u + 2 * j, d, acc[j], p.qk16);
     }
     fence_proxy_async();
     tc_fence_before();
@@ -672,7 +714,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     if (tid < rows && p.gate == LETHE_GATE_SCALAR) p.dg[tok0 + static_cast<size_t>(tid) * p.H] = acc;
     a = nx;
   }
-  if (tid == 0) bulk_wait_read();
+  if (tid == 0 || tid == 96) bulk_wait_read();
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, S::kCols);

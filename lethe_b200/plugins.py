@@ -146,6 +146,8 @@ def k2_fn(k: Tensor, v: Tensor, beta: Tensor, g2: Tensor, t_mat: Tensor, dw: Ten
     ta = torch.zeros(B, H, NT, 128, 64, dtype=torch.float16, device=dev)
     ta[..., :64, :] = t_mat.half()
     _record_view(buf.saved, off["ta"], sz["ta"], Z, torch.float16).copy_(to_image(ta).reshape(Z, -1))
+    bt = beta.to(f32)[..., None]
+    _wy_factors(buf, sz, off, Z, t_mat, bt * torch.exp2(g2.to(f32))[..., None] * k.to(f32), bt * v.to(f32))
     _record_view(buf.scratch, off2["dv2"], sz2["dv2"], Z, torch.float16).copy_(to_image(du.half()).reshape(Z, -1))
     _record_view(buf.scratch, off2["dw"], sz2["dw"], Z, torch.float16).copy_(to_image(dw.half()).reshape(Z, -1))
     _record_view(buf.scratch, off2["dkb"], sz2["dkb"], Z, f32).zero_()
