@@ -205,17 +205,18 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     tmem_alloc(&bars->tmem_slot, S::kCols);
     tmem_relinquish();
   }
-  // gates of a chunk, by one warp, two neighbouring tokens per lane
-  auto sum_gates = [&](const At& a, ScGates* o) {
-    float g[2] = {0.f, 0.f}, be[2] = {WY ? 0.f : 1.f, WY ? 0.f : 1.f};
+  // gates of a chunk, by one warp, two neighbouring tokens per lane: fetched a chunk ahead, then summed
+  auto fetch_gates = [&](const At& a, ScGates* o) {
+    if (p.gate == LETHE_GATE_SCALAR) warp_copy_gates(p, p.g, a.b, a.c, a.h, lane, o->G);
+    if (WY) warp_copy_gates(p, p.beta, a.b, a.c, a.h, lane, o->beta);
+  };
+  auto sum_gates = [&](ScGates* o) {
+    async_copy_wait();
+    float g[2] = {0.f, 0.f}, be[2] = {1.f, 1.f};
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-      const int t = 2 * lane + e;
-      if (t < p.rows_of(a.c)) {
-        const size_t tok = (static_cast<size_t>(a.b) * p.L + a.c * kC + t) * p.H + a.h;
-        if (p.gate == LETHE_GATE_SCALAR) g[e] = p.g[tok];
-        if (WY) be[e] = p.beta[tok];
-      }
+      if (p.gate == LETHE_GATE_SCALAR) g[e] = o->G[2 * lane + e];
+      if (WY) be[e] = o->beta[2 * lane + e];
     }
     float sum = g[0] + g[1];
 #pragma unroll
@@ -231,7 +232,10 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
   };
 
   At a = at(blockIdx.x);
-  if (warp == 2) sum_gates(a, gates);
+  if (warp == 2) {
+    fetch_gates(a, gates);
+    sum_gates(gates);
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -268,6 +272,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     const bool keep = CUT || !p.lean;
 
     const ScGates& gt = gates[ph];
+    if (warp == 2 && more) fetch_gates(nx, gates + (ph ^ 1u));
     if (tid == 0 && n != static_cast<int>(blockIdx.x)) {
       bulk_wait_read();                             // dk of the chunk before has left its tile
       if (!S::kOwn) load_q(a);
@@ -495,7 +500,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     if (MODE == kScStageB) {
       __syncthreads();
       if (tid < 64) dgb_g[tid] = dG + (tid == 63 ? end_term() : 0.f);
-      if (warp == 2 && more) sum_gates(nx, gates + (ph ^ 1u));
+      if (warp == 2 && more) sum_gates(gates + (ph ^ 1u));
       if (tid == 0 && more) {
         bulk_wait_read();
         load_do(nx);
@@ -645,7 +650,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       }
     }
     __syncwarp();
-    if (warp == 2 && more) sum_gates(nx, gates + (ph ^ 1u));
+    if (warp == 2 && more) sum_gates(gates + (ph ^ 1u));
     mbar_wait_warp(&bars->m5, ph, ctl, 425);
     tc_fence_after();
     if (tid == 0 && more) {                         // [T; A], k and q are read

@@ -5,7 +5,8 @@
 // Bound by HBM (88 KB per chunk at d_v = 128) and, per chunk, by a chain of load, conversion, two dependent products and
 // store.  Persistent CTAs of 256 threads, three or four per SM, fill each other's gaps; a CTA fetches the next do
 // and A once its last products are done, q and w once the result, staged where they were, has left.  8192 chunks,
-// channel-wise, d_v = 128: 150 -> 128 us; 4096 chunks, scalar, d_v = 64: 56 -> 51.
+// channel-wise, d_v = 128: 150 -> 128 us; 4096 chunks, scalar, d_v = 64: 56 -> 51.  With gates and (scalar gate) tiles
+// requested a chunk ahead: scalar, d_v = 128, 512 chunks 19.4 -> 17.3; without the delta term d_v = 64, 1692 chunks 22.6 -> 19.5.
 #include "gdn_common.cuh"
 #include "host_util.h"
 
@@ -57,7 +58,19 @@ bwd_pre_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
     else for (int i = 0; i < 2; ++i) tma_load_4d(QG + i * 8192, &mq, full, i * 64, a.h, a.c * kC, a.b);
     if (DELTA) bulk_g2s(Wt, p.saved + p.lay.w + static_cast<size_t>(a.z) * p.lay.sz_w, 16384, full);
   };
-  auto gates = [&](const At& a, float* o) { warp_scaled_gammas(p, a.b, a.c, a.h, lane, o); };
+  auto fetch_gates = [&](const At& a, float* o) {
+    if (p.gate == LETHE_GATE_SCALAR) warp_copy_gates(p, p.g, a.b, a.c, a.h, lane, o);
+  };
+  // what the loads will want, to L2; not channel-wise, where nothing is converted and HBM is the bound (8192 chunks: 127 us without, 134
+  // with; scalar gate without the delta term, d_v = 64, 1692 chunks 22.5 without, 20 with)
+  auto prefetch = [&](const At& a) {
+    for (int i = 0; i < V / 64; ++i) tma_prefetch_4d(&mdo, i * 64, a.h, a.c * kC, a.b);
+    for (int i = 0; i < 2; ++i) tma_prefetch_4d(&mq, i * 64, a.h, a.c * kC, a.b);
+    if (DELTA) {
+      bulk_prefetch(p.saved + p.lay.ta + static_cast<size_t>(a.z) * p.lay.sz_ta + 8192, 8192);
+      bulk_prefetch(p.saved + p.lay.w + static_cast<size_t>(a.z) * p.lay.sz_w, 16384);
+    }
+  };
 
   if (tid == 0) {
     cs->abort_flag = 0;
@@ -80,13 +93,17 @@ bwd_pre_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
     load_do(a);
     load_q(a);
   }
-  if (!CW && warp == 1) gates(at(blockIdx.x), sgs);
+  if (!CW && warp == 1) {
+    fetch_gates(at(blockIdx.x), sgs);
+    warp_scaled_gammas(p, lane, sgs);
+  }
   if (!CW) __syncthreads();
 
   uint32_t ph = 0, pm = 0;
   for (int n = blockIdx.x; n < nchunks; n += gridDim.x, ph ^= 1u) {
     const At a = at(n);
     const bool more = n + static_cast<int>(gridDim.x) < nchunks;
+    if (!CW && warp == 1 && more) fetch_gates(at(n + gridDim.x), sgs + (ph ^ 1u) * 64);
     mbar_wait_warp(full, ph, ctl, 401);
     if (!CW) {
       const float* sg = sgs + ph * 64;
@@ -114,7 +131,7 @@ bwd_pre_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
         umma_commit_led(leader, mma);
       }
       __syncwarp();
-      if (!CW && warp == 1 && more) gates(at(n + gridDim.x), sgs + (ph ^ 1u) * 64);
+      if (!CW && warp == 1 && more) warp_scaled_gammas(p, lane, sgs + (ph ^ 1u) * 64);
       wait_products(mma, pm, ctl, 402);
       if (quad >= 2) {
 #pragma unroll
@@ -135,9 +152,11 @@ bwd_pre_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
       issue_product_led(leader, tmem, Tile{smem_u32(QG), 64, true}, Tile{smem_u32(DO), 64, true}, V, 64, 0u);
       if (DELTA) issue_product_led(leader, tmem, Tile{smem_u32(Wt), 64, true}, Tile{smem_u32(DVL), 64, true}, V, 64, 1u, true);
       umma_commit_led(leader, mma);
+    } else if (!CW && warp == 2 && lane == 0 && more) {
+      prefetch(at(n + gridDim.x));
     }
     __syncwarp();
-    if (!DELTA && !CW && warp == 1 && more) gates(at(n + gridDim.x), sgs + (ph ^ 1u) * 64);
+    if (!DELTA && !CW && warp == 1 && more) warp_scaled_gammas(p, lane, sgs + (ph ^ 1u) * 64);
     wait_products(mma, pm, ctl, 403);
     if (tid == 0 && more) load_do(at(n + gridDim.x));
     unsigned char* SR = QG;   // q and w are dead: Rb is staged there as its record image

@@ -240,13 +240,24 @@ __device__ __forceinline__ uint32_t rrec_off(int row, int col8) {
   return static_cast<uint32_t>((col8 >> 1) * 4096 + row * 32 + (col8 & 1) * 16);
 }
 
-// scale * gamma_t of the 64 tokens of chunk c by one warp, two neighbouring tokens per lane (scalar gate or none).
-__device__ __forceinline__ void warp_scaled_gammas(const Problem& p, int b, int c, int h, int lane, float* out) {
-  float g[2] = {0.f, 0.f};
+// One value per token of chunk c to shared memory by one warp, two neighbouring tokens per lane, zero behind the last token; each
+// lane waits for its own (async_copy_wait) and reads them.  A chunk's gates are fetched like this a chunk ahead: a load to registers
+// is waited for by the warp that issues it, and by all others at the next barrier.
+__device__ __forceinline__ void warp_copy_gates(const Problem& p, const float* src, int b, int c, int h, int lane, float* dst) {
+  const int last = p.rows_of(c) - 1;
 #pragma unroll
   for (int e = 0; e < 2; ++e) {
     const int t = 2 * lane + e;
-    if (p.gate == LETHE_GATE_SCALAR && t < p.rows_of(c)) g[e] = p.g[(static_cast<size_t>(b) * p.L + c * kC + t) * p.H + h];
+    async_copy4(dst + t, src + (static_cast<size_t>(b) * p.L + c * kC + min(t, last)) * p.H + h, t <= last);
+  }
+}
+// scale * gamma_t of the 64 tokens of a chunk by one warp (scalar gate or none): from the decays that warp_copy_gates brought
+__device__ __forceinline__ void warp_scaled_gammas(const Problem& p, int lane, float* io) {
+  float g[2] = {0.f, 0.f};
+  if (p.gate == LETHE_GATE_SCALAR) {
+    async_copy_wait();
+    g[0] = io[2 * lane];
+    g[1] = io[2 * lane + 1];
   }
   float sum = g[0] + g[1];
 #pragma unroll
@@ -254,7 +265,7 @@ __device__ __forceinline__ void warp_scaled_gammas(const Problem& p, int b, int 
     const float y = __shfl_up_sync(0xffffffffu, sum, w);
     if (lane >= w) sum += y;
   }
-  *reinterpret_cast<float2*>(out + 2 * lane) = make_float2(p.scale * __expf(sum - g[1]), p.scale * __expf(sum));
+  *reinterpret_cast<float2*>(io + 2 * lane) = make_float2(p.scale * __expf(sum - g[1]), p.scale * __expf(sum));
 }
 
 }  // namespace lg

@@ -25,6 +25,8 @@ namespace lg {
 // and the gates are summed a chunk ahead by one warp.  With one CTA per chunk instead, the wait for the first loads and the
 // start of the CTA were 40 % of its time.  The gates are applied to the columns of T, not to k and v: half the elements.
 // 4096 chunks: d_v = 64 167 -> 132 us, d_v = 128 183 -> 143; without the delta term (below) d_v = 128 121 -> 85.
+// The gates of the next chunk come by asynchronous copies to shared memory, and what its late loads will want is prefetched to L2
+// under product 1: without the delta term d_v = 128 79 -> 70, with it within 1 %.
 // ---------------------------------------------------------------------------------------------
 constexpr int kPrepThreads = 256;
 
@@ -32,17 +34,19 @@ struct PrepGates {
   float G[64], beta[64], dec[64], bg[64];     // cumulative log decay; beta; exp(G_last - G); beta exp(G)
 };
 
-// Gates of a chunk by one warp, two neighbouring tokens per lane; also the record of the chunk's whole decay.
-__device__ __forceinline__ void prep_gates(const Problem& p, int b, int c, int h, int z, int lane, PrepGates* o) {
-  float g[2] = {0.f, 0.f}, be[2] = {p.delta ? 0.f : 1.f, p.delta ? 0.f : 1.f};
+// Gates of a chunk by one warp, two neighbouring tokens per lane: fetched a chunk ahead, then summed; also the record of the
+// chunk's whole decay.
+__device__ __forceinline__ void prep_fetch_gates(const Problem& p, int b, int c, int h, int lane, PrepGates* o) {
+  if (p.gate == LETHE_GATE_SCALAR) warp_copy_gates(p, p.g, b, c, h, lane, o->G);
+  if (p.delta) warp_copy_gates(p, p.beta, b, c, h, lane, o->beta);
+}
+__device__ __forceinline__ void prep_gates(const Problem& p, int z, int lane, PrepGates* o) {
+  async_copy_wait();
+  float g[2] = {0.f, 0.f}, be[2] = {1.f, 1.f};
 #pragma unroll
   for (int e = 0; e < 2; ++e) {
-    const int t = 2 * lane + e;
-    if (t < p.rows_of(c)) {
-      const size_t tok = (static_cast<size_t>(b) * p.L + c * kC + t) * p.H + h;
-      if (p.gate == LETHE_GATE_SCALAR) g[e] = p.g[tok];
-      if (p.delta) be[e] = p.beta[tok];
-    }
+    if (p.gate == LETHE_GATE_SCALAR) g[e] = o->G[2 * lane + e];
+    if (p.delta) be[e] = o->beta[2 * lane + e];
   }
   float sum = g[0] + g[1];
 #pragma unroll
@@ -72,6 +76,15 @@ __device__ __forceinline__ void prep_load_kq(unsigned char* KQ, const CUtensorMa
     tma_load_4d(KQ + t * 16384, mk, bar, t * 64, a.h, a.c * kC, a.b);
     tma_load_4d(KQ + t * 16384 + 8192, mq, bar, t * 64, a.h, a.c * kC, a.b);
   }
+}
+// ... and what a chunk will load to L2, under the products of the chunk before: its tiles are free late
+template <int V>
+__device__ __forceinline__ void prep_prefetch(const CUtensorMap* mk, const CUtensorMap* mq, const CUtensorMap* mv, const PrepAt& a) {
+  for (int t = 0; t < 2; ++t) {
+    tma_prefetch_4d(mk, t * 64, a.h, a.c * kC, a.b);
+    tma_prefetch_4d(mq, t * 64, a.h, a.c * kC, a.b);
+  }
+  for (int t = 0; t < V / 64; ++t) tma_prefetch_4d(mv, t * 64, a.h, a.c * kC, a.b);
 }
 template <int V>
 __device__ __forceinline__ void prep_load_v(unsigned char* Vt, const CUtensorMap* mv, uint64_t* bar, const PrepAt& a) {
@@ -169,7 +182,10 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
       prep_load_kq(KQ, &mk, &mq, full_kq, a);
       prep_load_v<V>(Vt, &mv, full_v, a);
     }
-    if (warp == 1) prep_gates(p, a.b, a.c, a.h, a.z, lane, gates);
+    if (warp == 1) {
+      prep_fetch_gates(p, a.b, a.c, a.h, lane, gates);
+      prep_gates(p, a.z, lane, gates);
+    }
   }
   __syncthreads();
 
@@ -179,6 +195,7 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
     const bool more = n + static_cast<int>(gridDim.x) < nchunks;
     const PrepAt nx(p, more ? n + gridDim.x : n);
     const PrepGates& gt = gates[ph];
+    if (warp == 1 && more) prep_fetch_gates(p, nx.b, nx.c, nx.h, lane, gates + (ph ^ 1u));
 
     mbar_wait_warp(full_kq, ph, ctl, 201);
     if (!p.qk16) prep_to_f16(KQ, 32768, tid);
@@ -194,6 +211,8 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
       const uint32_t leader = elect_leader();
       issue_product_led(leader, tmem, Tile{smem_u32(KQ), 128, false}, Tile{smem_u32(KQ), 128, false}, 64, 128, 0u);
       umma_commit_led(leader, mma);
+    } else if (warp == 2 && lane == 0 && more) {
+      prep_prefetch<V>(&mk, &mq, &mv, nx);
     }
     wait_products(mma, pm, ctl, 202);
     {
@@ -292,7 +311,7 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
       }
     }
     __syncwarp();
-    if (warp == 1 && more) prep_gates(p, nx.b, nx.c, nx.h, nx.z, lane, gates + (ph ^ 1u));
+    if (warp == 1 && more) prep_gates(p, nx.z, lane, gates + (ph ^ 1u));
     wait_products(mma, pm, ctl, 205);
     // P leaves from where [T; A] and kd were, R from where w (and u) were once their stores have read them
 #pragma unroll
@@ -382,7 +401,10 @@ prepare_nodelta_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, 
       prep_load_kq(KQ, &mk, &mq, full_kq, a);
       prep_load_v<V>(Vt, &mv, full_v, a);
     }
-    if (warp == 1) prep_gates(p, a.b, a.c, a.h, a.z, lane, gates);
+    if (warp == 1) {
+      prep_fetch_gates(p, a.b, a.c, a.h, lane, gates);
+      prep_gates(p, a.z, lane, gates);
+    }
   }
   __syncthreads();
 
@@ -392,6 +414,7 @@ prepare_nodelta_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, 
     const bool more = n + static_cast<int>(gridDim.x) < nchunks;
     const PrepAt nx(p, more ? n + gridDim.x : n);
     const PrepGates& gt = gates[ph];
+    if (warp == 1 && more) prep_fetch_gates(p, nx.b, nx.c, nx.h, lane, gates + (ph ^ 1u));
 
     mbar_wait_warp(full_kq, ph, ctl, 206);
     for (int idx = tid; idx < 64 * 16; idx += kPrepThreads) {
@@ -420,9 +443,11 @@ prepare_nodelta_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, 
         bulk_s2g(p.saved + p.lay.u + static_cast<size_t>(a.z) * p.lay.sz_u, Vt, V * 128);      // (u is v)
         bulk_commit();
       }
+    } else if (warp == 2 && lane == 0 && more) {
+      prep_prefetch<V>(&mk, &mq, &mv, nx);
     }
     __syncwarp();
-    if (warp == 1 && more) prep_gates(p, nx.b, nx.c, nx.h, nx.z, lane, gates + (ph ^ 1u));
+    if (warp == 1 && more) prep_gates(p, nx.z, lane, gates + (ph ^ 1u));
     wait_products(mma, pm, ctl, 208);
     if (tid == 0 && more) prep_load_kq(KQ, &mk, &mq, full_kq, nx);
     if (!p.lean) {
@@ -476,7 +501,8 @@ prepare_nodelta_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, 
 // chunk's tiles arrive while the chunk before is computed (8192 chunks: 193 -> 152 us, 0.99 of the copy bandwidth on its
 // bytes).  Shorter chunks and those whose q and v are converted here are bound by the chain of latencies, which two or
 // three CTAs of one stage each hide better (scalar gate, d_v = 64, 4096 chunks: 59 us against 71 us with two stages;
-// d_v = 128 without the delta term: 78 against 86).
+// d_v = 128 without the delta term: 78 against 86).  With one stage a chunk's loads start when the chunk before has left;
+// they are prefetched to L2 and its gates fetched ahead (d_v = 128 without the delta term, 4096 chunks: 76 -> 71.6).
 // ---------------------------------------------------------------------------------------------
 constexpr int kOutThreads = 256;
 
@@ -529,7 +555,19 @@ output_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
   auto load_h = [&](const At& a, int s) {
     bulk_g2s(sm + s * S::kStage + S::oH, p.saved + p.lay.hc + static_cast<size_t>(a.z + a.bh) * p.lay.sz_hc, V * 256, &full[s]);
   };
-  auto gates = [&](const At& a, float* o) { warp_scaled_gammas(p, a.b, a.c, a.h, lane, o); };
+  auto fetch_gates = [&](const At& a, float* o) {
+    if (p.gate == LETHE_GATE_SCALAR) warp_copy_gates(p, p.g, a.b, a.c, a.h, lane, o);
+  };
+  auto prefetch = [&](const At& a) {                 // what load and load_h will want, to L2
+    for (int i = 0; i < 2; ++i)
+      if (!CW) tma_prefetch_4d(&mq, i * 64, a.h, a.c * kC, a.b);
+    if (CW) bulk_prefetch(p.saved + p.lay.qg + static_cast<size_t>(a.z) * 16384, 16384);
+    if (DELTA) bulk_prefetch(p.saved + p.lay.w + static_cast<size_t>(a.z) * p.lay.sz_w, 16384);
+    bulk_prefetch(p.saved + p.lay.ta + static_cast<size_t>(a.z) * p.lay.sz_ta + 8192, 8192);
+    if (DELTA) bulk_prefetch(p.saved + p.lay.u + static_cast<size_t>(a.z) * p.lay.sz_u, V * 128);
+    else for (int i = 0; i < V / 64; ++i) tma_prefetch_4d(&mv, i * 64, a.h, a.c * kC, a.b);
+    bulk_prefetch(p.saved + p.lay.hc + static_cast<size_t>(a.z + a.bh) * p.lay.sz_hc, V * 256);
+  };
 
   const int n0 = blockIdx.x, n1 = n0 + gridDim.x;
   if (tid == 0) {
@@ -544,7 +582,10 @@ output_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     tmem_alloc(&cs->tmem_slot, V);
     tmem_relinquish();
   }
-  if (!CW && warp == 1) gates(at(n0), sgs);
+  if (!CW && warp == 1) {
+    fetch_gates(at(n0), sgs);
+    warp_scaled_gammas(p, lane, sgs);
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -562,6 +603,8 @@ output_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     const int s = it % S::kStages, g2 = it & 1;
     const uint32_t ph = static_cast<uint32_t>(it & 1);
     unsigned char *WQ = sm + s * S::kStage, *At_ = WQ + S::oA, *HT = WQ + S::oH, *VN = WQ + S::oU;
+    const bool more = n + static_cast<int>(gridDim.x) < nchunks;
+    if (!CW && warp == 1 && more) fetch_gates(at(n + gridDim.x), sgs + (g2 ^ 1) * 64);
     mbar_wait_warp(&full[s], static_cast<uint32_t>((it / S::kStages) & 1), ctl, 211);
     if (!CW) {
       const float* sg = sgs + g2 * 64;
@@ -595,9 +638,11 @@ output_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
         load(nx, s ^ 1);
         load_h(nx, s ^ 1);
       }
+    } else if (S::kStages == 1 && warp == 2 && lane == 0 && more) {
+      prefetch(at(n + gridDim.x));
     }
     __syncwarp();
-    if (!CW && warp == 1 && n + static_cast<int>(gridDim.x) < nchunks) gates(at(n + gridDim.x), sgs + (g2 ^ 1) * 64);
+    if (!CW && warp == 1 && more) warp_scaled_gammas(p, lane, sgs + (g2 ^ 1) * 64);
     if (DELTA) {
       mbar_wait_warp(m1, ph, ctl, 212);
       tc_fence_after();
