@@ -147,8 +147,7 @@ struct CtaShared {
 // access is a generic one.  Same addresses, different instruction selection and scheduling.  The chunk
 // kernels want the first (us, generic against shared: prepare 148 / 135 at 4096 chunks, channel-wise 667 /
 // 590 at 8192; main 270 / 224 and 1051 / 915; output and scan input within 3 %, once 78 / 70).  The scan of
-// 64 columns per CTA is 1-3 % faster with the second (64.7 / 63.4 for 32 pairs x 64 chunks); at 16 columns
-// the forward scan is as well (17.2 / 16.8 at 16 x 32, d_v = 128 17.6 / 18.0), the adjoint is not (16.5 / 17.3).
+// 64 columns per CTA is 1-3 % faster with the second (64.7 / 63.4 for 32 pairs x 64 chunks).
 __device__ __forceinline__ unsigned char* align1024(unsigned char* p) {
   const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(p));
   return p + ((1024u - (a & 1023u)) & 1023u);

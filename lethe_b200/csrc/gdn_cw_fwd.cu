@@ -152,7 +152,7 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
   if (tid == 0) {
     where[0] = chunk_at(p, blockIdx.x);
     cs->abort_flag = 0;
-    for (int i = 0; i < 5; ++i) mbar_init(&cs->bar[i], 1);
+    for (int i = 0; i < 5; ++i) mbar_init(&cs->bar[i], i == 2 || i == 3 ? 2 : 1);
     fence_mbar_init();
     fence_proxy_async();
     load_k(where[0]);
@@ -448,9 +448,13 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
       tc_fence_after();
       const uint32_t leader = elect_leader();
       issue_product_led(leader, tmem, Tile{smem_u32(LA), 128, true}, Tile{smem_u32(KR), 128, true}, 64, 128, 0u);
+      umma_commit_led(leader, m1);
+    } else if (warp == 1) {                      // (two warps share the issue, some 45 cycles per product)
+      tc_fence_after();
+      const uint32_t leader = elect_leader();
       issue_product_led(leader, tmem + 64, Tile{smem_u32(LA), 128, true}, Tile{smem_u32(KR2), 128, true}, 32, 128, 0u);
       umma_commit_led(leader, m1);
-    } else if (warp == 1 && lane == 0 && more) {      // the next g and v to L2: g's tiles are free late, and v is wanted soon then
+    } else if (warp == 2 && lane == 0 && more) {      // the next g and v to L2: g's tiles are free late, and v is wanted soon then
       const ChunkAt a = where[ph ^ 1u];
       tma_prefetch_4d(&mg, 0, a.h, a.c * kC, a.b);
       for (int t = 0; t < V / 64; ++t) tma_prefetch_4d(&mv, t * 64, a.h, a.c * kC, a.b);
@@ -548,16 +552,20 @@ prepare_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const
         tc_fence_after();
         const uint32_t leader = elect_leader();
         issue_product_led(leader, tmem, Tile{smem_u32(TA), 128, false}, Tile{smem_u32(GK), 128, false}, 128, 64, 0u);
-        issue_product_led(leader, tmem + 128, Tile{smem_u32(TA), 128, false}, Tile{smem_u32(BV), 64, true}, V, 64, 0u);
         umma_commit_led(leader, m2);
         if (tid == 0) {
           if (p.lean < 2) bulk_s2g(rec(p.lay.ta, p.lay.sz_ta), TA, 16384);
           else bulk_s2g(rec(p.lay.ta, p.lay.sz_ta) + 8192, TA + 8192, 8192);      // A only
           bulk_commit();
         }
+      } else if (warp == 1) {
+        tc_fence_after();
+        const uint32_t leader = elect_leader();
+        issue_product_led(leader, tmem + 128, Tile{smem_u32(TA), 128, false}, Tile{smem_u32(BV), 64, true}, V, 64, 0u);
+        umma_commit_led(leader, m2);
       }
       __syncwarp();
-    anew();
+      anew();
       mbar_wait_warp(m2, ph, ctl, 503);
       tc_fence_after();
       if (quad < 2) {                      // rows 0-63; the warps of a quadrant split the columns

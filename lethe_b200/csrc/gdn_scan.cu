@@ -5,10 +5,11 @@
 //
 // a_c is the chunk's decay per key channel, P_c = kd^T w (128 x 128) and R_c / Rb_c (128 x V) come
 // from the chunk-parallel kernels.  The recurrence is independent per column of x, so the grid is
-// (V / 16) x (B*H): every CTA owns 16 columns, keeps them as fp32 in registers (thread d = key
-// channel d) and does ONE tcgen05 product per chunk, with P streamed through a ring of shared-memory
-// stages by bulk copies that run ahead of the recurrence.  The state seen by chunk c is written out
-// as a shared-memory tile image for the chunk-parallel kernels.
+// (V / columns) x (B*H): every CTA owns some columns, keeps them as fp32 in registers and does ONE product per chunk, with
+// P streamed through a ring of shared-memory stages by bulk copies that run ahead of the recurrence.  The state seen by
+// chunk c is written out as a shared-memory tile image for the chunk-parallel kernels.  Three kernels: 64 columns per CTA on
+// tcgen05 (few CTAs, P read once or twice per pair), 8 to 32 on warp-level matrix instructions (the shorter step), and one without
+// a product where there is no delta term; the rules stand at launch_scan.
 // Reference: the forward recurrence gdn2_chunkwise.py:155-158 and the reverse scan K#1
 // gdn2_assemble.py:71-99 of the reference project, after substituting v_new / dv2.
 #include "gdn_common.cuh"
@@ -18,11 +19,9 @@ namespace lg {
 
 constexpr int kStages = 3;
 constexpr int kMmaWarps = 2;   // warps that issue the step's products (each its own accumulator)
-// Columns of the state per CTA: 16 on four state-holding warps or 64 on sixteen (kGr groups of four warps, 16 columns
-// per thread either way).  The narrow CTA has the shorter step, 0.5 us against 0.7 us; but every CTA of a (batch, head)
-// pair streams all of P, so the wide form moves a quarter of its bytes from L2 - see the rule in launch_scan.
-// warps 0 .. 4 kGr - 1 hold the state (thread d = key channel d), then one warp streams P, two issue products
-constexpr int kVs = 16;
+// 64 columns of the state per CTA on sixteen state-holding warps, 16 columns of a row per thread (four groups of four warps, thread
+// d = key channel d), then one warp that streams P and two that issue products
+constexpr int kVs = 16, kGr = 4, kW = kVs * kGr;
 
 // Step barrier of the delta path: the state-holding warps arrive once the operand is written (and go
 // on to work that does not depend on the product), the issuing warps wait for them.
@@ -31,21 +30,18 @@ __device__ __forceinline__ void step_arrive() { asm volatile("bar.arrive 1, %0;"
 template <int kN>
 __device__ __forceinline__ void step_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kN) : "memory"); }
 
-template <int kGr>
 constexpr int kScanThreads = (4 * kGr + 1 + kMmaWarps) * 32;
 
-template <bool ADJOINT, int kGr>
-__global__ void __launch_bounds__(kScanThreads<kGr>, kGr == 1 ? 2 : 1)
+template <bool ADJOINT>
+__global__ void __launch_bounds__(kScanThreads, 1)
 scan_kernel(const Problem p) {
-  constexpr int kW = kVs * kGr;                      // columns of this CTA: 16 or 64
-  constexpr int kTmemCols = kMmaWarps * kW;         // 32 or 128
+  constexpr int kTmemCols = kMmaWarps * kW;
   constexpr int kXB = 128 * kW * 2;                  // bytes of the state operand tile
   constexpr int kStateWarps = 4 * kGr, kStepBarrier = (kStateWarps + kMmaWarps) * 32;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* sm = align1024_generic(smem_raw);
   unsigned char* Pst = sm;                          // kStages x 32 KB
-  // x as the B operand, contracted along its rows (row k = key channel k, kW columns = 32 or 128 bytes):
-  // atoms of 8 rows with the swizzle of that width, so that thread k stores its row as 16-byte pieces
+  // x as the B operand, contracted along its rows (row k = key channel k, 64 columns): thread k stores pieces of row k
   unsigned char* XB0 = sm + kStages * 32768;        // two of them, alternating: the step before's is still being recorded
   CtaShared* cs = reinterpret_cast<CtaShared*>(XB0 + 2 * kXB);
 
@@ -81,9 +77,9 @@ scan_kernel(const Problem p) {
   tc_fence_after();
   const uint32_t tmem = cs->tmem_slot;
   auto chunk_of = [&](int it) { return ADJOINT ? p.c0 + n - 1 - it : p.c0 + it; };
-  // Record of the state a chunk sees: this CTA's columns in the image of [128][V].  At 64 columns the operand tile is that
-  // image and leaves as one bulk copy; stores by the state warps, a row of pieces per thread, held up the step that
-  // followed them (1.08 us a step with them, 0.7 like this).  At 16 columns they cost next to nothing.
+  // Record of the state a chunk sees: this CTA's columns in the image of [128][V].  The operand tile is that image and
+  // leaves as one bulk copy; stores by the state warps, a row of pieces per thread, held up the step that followed them (1.08 us
+  // a step with them, 0.7 like this).
   auto record = [&](int it) {
     const size_t z = static_cast<size_t>(bh) * NT + chunk_of(it);
     return (ADJOINT ? p.scratch + p.lay.dh : p.saved + p.lay.hc) + (ADJOINT ? z : z + bh) * p.lay.sz_hc + static_cast<size_t>(v0 >> 6) * 16384;
@@ -114,13 +110,13 @@ scan_kernel(const Problem p) {
     const uint32_t leader = elect_leader();
     // A = the P stage (contracted along its columns forward, along its rows for the adjoint),
     // B = the state operand; one 16-element contraction step moves each by a fixed amount
-    const uint64_t b_desc0 = kW == 16 ? make_desc_sw32(smem_u32(XB0), 16u, 256u) : make_desc(smem_u32(XB0), 16384u, 1024u);
+    const uint64_t b_desc0 = make_desc(smem_u32(XB0), 16384u, 1024u);
     const uint32_t idesc = make_idesc(128, kW, ADJOINT, true);
     const uint32_t acc = tmem + static_cast<uint32_t>(m * kW);
     for (int it = 0; it < n; ++it) {
       const int st = it % kStages;
       mbar_wait_warp(&bar_full[st], static_cast<uint32_t>((it / kStages) & 1), ctl, 301);
-      if (kW == 64 && m == 0 && lane == 0) bulk_wait_read();     // the other operand tile is recorded: it may be written again
+      if (m == 0 && lane == 0) bulk_wait_read();     // the other operand tile is recorded: it may be written again
       step_sync<kStepBarrier>();
       tc_fence_after();
       const uint32_t pa = smem_u32(Pst + st * 32768);
@@ -136,12 +132,12 @@ scan_kernel(const Problem p) {
       }
       umma_commit_led(leader, bar_mma);
       umma_commit_led(leader, &bar_free[st]);
-      if (kW == 64 && m == 0 && lane == 0) {       // the operand tile is the record's image
+      if (m == 0 && lane == 0) {       // the operand tile is the record's image
         bulk_s2g(record(it), XB0 + (it & 1) * kXB, kXB);
         bulk_commit();
       }
     }
-    if (kW == 64 && m == 0 && lane == 0) bulk_wait_read();
+    if (m == 0 && lane == 0) bulk_wait_read();
   } else {
     // ---- the state: thread d of a group holds kVs columns of row d of x in fp32
     const int d = tid & 127, g = tid >> 7, vg = v0 + g * kVs;      // group g: columns [vg, vg + kVs)
@@ -177,11 +173,9 @@ scan_kernel(const Problem p) {
       unsigned char* XB = XB0 + (it & 1) * kXB;
       // critical path: the state as a tensor-core operand
       {
-        // 32-byte swizzle: the two pieces of rows 4-7 of an atom swap; 128-byte swizzle: piece q of row r sits at q ^ (r & 7)
-        const int sw = kW == 16 ? (d >> 2) & 1 : d & 7;
 #pragma unroll
         for (int q = 0; q < kPieces; ++q)
-          *reinterpret_cast<uint4*>(XB + d * (2 * kW) + (((g * kPieces + q) ^ sw) << 4)) = pack8_f16(x + 8 * q);
+          *reinterpret_cast<uint4*>(XB + d * (2 * kW) + (((g * kPieces + q) ^ (d & 7)) << 4)) = pack8_f16(x + 8 * q);
       }
       fence_proxy_async();
       tc_fence_before();
@@ -197,12 +191,6 @@ scan_kernel(const Problem p) {
         const int cn = chunk_of(it + 1);
         load_r(cn);
         a_next = ADg[(static_cast<size_t>(bh) * NT + cn) * kK + d];
-      }
-      if (kW < 64) {
-        unsigned char* rec = record(it);
-#pragma unroll
-        for (int q = 0; q < kPieces; ++q)
-          *reinterpret_cast<uint4*>(rec + d * 128 + (((((vg & 63) >> 3) + q) ^ (d & 7)) << 4)) = pack8_f16(x + 8 * q);
       }
       mbar_wait_warp(bar_mma, static_cast<uint32_t>(it & 1), ctl, 302);
       tc_fence_after();
@@ -232,6 +220,270 @@ scan_kernel(const Problem p) {
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, kTmemCols);
+}
+
+// ---------------------------------------------------------------------------------------------
+// The same recurrence for few columns per CTA, on warp-level matrix instructions (mma.sync): a step is a chain of latencies, not a
+// matter of throughput, and there the accumulator that lies in the registers which also hold the state, and the operand that
+// is loaded to registers ahead, beat tcgen05 with its commit, mbarrier and tensor-memory read.  Warps own 16 kM rows of the
+// state in the accumulator layout of m16n8k16; per step they leave them as fp16 in shared memory, and after one barrier of the
+// state warps each reads all rows as the other operand.  Its rows of P (forward; columns, adjoint), R and the decays of the next
+// step are fetched to registers between the products; a producer warp keeps a ring of stages.
+// With y = -x the step is y <- (a y - R) + P fp16(x): the accumulator starts as the bracket and ends as the new state.
+//
+// Bound by the matrix pipe (17 cycles for a product of 16 x 8 x 16 per SM quarter, so 0.14 us per 8 columns) behind 0.25 us of
+// barrier, operand loads and P's way to registers: 0.39 us a step with 8 columns, 0.53 with 16, 0.85 with 32; tcgen05 took 0.69
+// with 16 (same measure: slope over the number of chunks, L2 cold) and takes 0.88 with 64.  With the fetch behind the products
+// instead of between them 16 columns took 0.62, with four warps of kM = 2 at 32 columns the step is 0.92.
+// ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t* r) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+__device__ __forceinline__ void ldsm4t(uint32_t addr, uint32_t* r) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+__device__ __forceinline__ void mma_f16(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+template <int kW, int kSt>
+struct ScanMmaSmem {
+  static constexpr int kR = kW < 16 ? 4096 : kW * 256;                            // whole blocks of 16 columns
+  static constexpr int oR = 32768, oA = oR + kR, kStage = oA + 512;               // P, R, decays of a chunk
+  static constexpr int oX = kSt * kStage, kX = 128 * kW * 2;                      // two operand tiles, alternating
+  static constexpr int oBar = oX + 2 * kX, kBytes = oBar + 2 * kSt * 8 + 16 + 1024;
+};
+
+template <bool ADJOINT, int kW, int kSt, int kM>
+__global__ void __launch_bounds__(32 * (8 / kM + 1), 1)
+scan_mma_kernel(const Problem p) {
+  using S = ScanMmaSmem<kW, kSt>;
+  constexpr int kN = kW / 8, kWarps = 8 / kM, kThreads = 32 * kWarps;      // n-tiles; warps of kM m-tiles each
+  constexpr int kRec = (128 * kN + kThreads - 1) / kThreads;      // 16-byte pieces of a record per thread
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* sm = align1024(smem_raw);
+  uint64_t* full = reinterpret_cast<uint64_t*>(sm + S::oBar);
+  uint64_t* empty = full + kSt;
+  int* abort_flag = reinterpret_cast<int*>(empty + kSt);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int v0 = blockIdx.x * kW, bh = blockIdx.y + p.bh0, V = p.V, NT = p.NT, n = p.cn;
+  const bool seg_first = ADJOINT ? (p.c0 + p.cn == NT) : (p.c0 == 0);        // chunk ranges as in scan_kernel
+  const bool seg_last = ADJOINT ? (p.c0 == 0) : (p.c0 + p.cn == NT);
+  CtaCtl ctl{p.status, abort_flag};
+  if (tid == 0) {
+    *abort_flag = 0;
+    for (int s = 0; s < kSt; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], kWarps);
+    }
+    fence_mbar_init();
+  }
+  __syncthreads();
+  auto chunk_of = [&](int it) { return ADJOINT ? p.c0 + n - 1 - it : p.c0 + it; };
+  const unsigned char* Rg = ADJOINT ? p.scratch + p.lay.rb : p.saved + p.lay.r;
+
+  if (warp == kWarps) {
+    // ---- producer.  P and the decays are older than the kernel before in the adjoint scan, whose R is not.
+    if (lane == 0) {
+      auto load_p = [&](int it) {
+        unsigned char* st = sm + (it % kSt) * S::kStage;
+        const size_t z = static_cast<size_t>(bh) * NT + chunk_of(it);
+        mbar_expect_tx(&full[it % kSt], S::kStage);
+        bulk_g2s(st, p.saved + p.lay.p + z * 32768, 32768u, &full[it % kSt]);
+        bulk_g2s(st + S::oA, p.saved + p.lay.ad + z * 512, 512u, &full[it % kSt]);
+      };
+      auto load_r = [&](int it) {
+        const size_t z = static_cast<size_t>(bh) * NT + chunk_of(it);
+        bulk_g2s(sm + (it % kSt) * S::kStage + S::oR, Rg + z * p.lay.sz_r + static_cast<size_t>(v0 / 16) * 4096, S::kR, &full[it % kSt]);
+      };
+      const int first = n < kSt ? n : kSt;
+      if (!ADJOINT) griddep_wait();
+      for (int it = 0; it < first; ++it) load_p(it);
+      if (ADJOINT) griddep_wait();
+      for (int it = 0; it < first; ++it) load_r(it);
+      for (int it = kSt; it < n; ++it) {
+        mbar_wait(&empty[it % kSt], static_cast<uint32_t>(((it / kSt) - 1) & 1), ctl, 303);
+        load_p(it);
+        load_r(it);
+      }
+    }
+    return;
+  }
+
+  // ---- the state
+  griddep_wait();
+  griddep_launch();
+  const int g = lane >> 2, t = lane & 3, m0 = 16 * kM * warp;
+  float* carry = reinterpret_cast<float*>(ADJOINT ? p.scratch + p.lay.carry_b : p.saved + p.lay.carry_f);
+  unsigned char* Xg = ADJOINT ? p.scratch + p.lay.dh : p.saved + p.lay.hc;
+  float y[kM][kN][4];
+  {
+    const float* x0 = seg_first ? (ADJOINT ? p.dhT : p.h0) : carry;
+    const int nrow = seg_first ? p.Kr : kK;          // user states have the real channel count
+#pragma unroll
+    for (int m = 0; m < kM; ++m)
+#pragma unroll
+      for (int j = 0; j < kN; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int d = m0 + 16 * m + 8 * e + g;
+          float2 v = make_float2(0.f, 0.f);
+          if (x0 && d < nrow) v = *reinterpret_cast<const float2*>(x0 + (static_cast<size_t>(bh) * nrow + d) * V + v0 + 8 * j + 2 * t);
+          y[m][j][2 * e] = -v.x;
+          y[m][j][2 * e + 1] = -v.y;
+        }
+  }
+  // operand tile: rows of kW columns, 16-byte pieces swizzled so that eight rows of one piece lie on different banks
+  auto piece = [](int r, int q) { return r * (2 * kW) + ((q ^ (kW == 8 ? 0 : kW == 16 ? (r >> 2) & 1 : (r >> 1) & 3)) << 4); };
+  constexpr int kB = (kN + 1) / 2;                   // blocks of 16 columns
+  // rows (adjoint: columns) m0 .. m0 + 31 of P, contraction step j
+  auto fetch_a = [&](uint32_t P, int j, uint32_t (*A)[8][4]) {
+#pragma unroll
+    for (int m = 0; m < kM; ++m) {
+      if (ADJOINT) {
+        const int r = 16 * j + (lane & 7) + ((lane >> 4) << 3), ch = (m0 + 16 * m) / 8 + ((lane >> 3) & 1);
+        ldsm4t(P + sw128_chunk(r, ch, 128), A[m][j]);
+      } else {
+        ldsm4(P + sw128_chunk(m0 + 16 * m + (lane & 15), 2 * j + (lane >> 4), 128), A[m][j]);
+      }
+    }
+  };
+  auto fetch_r = [&](int s, uint32_t (*R)[kB][4], float (*a)[2]) {      // ... and R and the decays; then the stage is free
+    const uint32_t P = smem_u32(sm + s * S::kStage);
+#pragma unroll
+    for (int m = 0; m < kM; ++m) {
+#pragma unroll
+      for (int b = 0; b < kB; ++b)
+        ldsm4(P + S::oR + b * 4096 + (m0 + 16 * m + (lane & 15)) * 32 + (kW == 8 ? (v0 >> 3) & 1 : lane >> 4) * 16, R[m][b]);
+      const float* ad = reinterpret_cast<const float*>(sm + s * S::kStage + S::oA) + m0 + 16 * m + g;
+      a[m][0] = ad[0];
+      a[m][1] = ad[8];
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&empty[s]);
+  };
+  auto wait_stage = [&](int it) { mbar_wait_warp(&full[it % kSt], static_cast<uint32_t>((it / kSt) & 1), ctl, 301); };
+  uint4 rec[kRec];
+  auto record_at = [&](int i, const unsigned char* X) {      // this thread's i-th piece of the operand tile
+    const int idx = (tid + kThreads * i) % (128 * kN);
+    return X + piece(idx / (kW / 8), idx % (kW / 8));
+  };
+  auto record = [&](int record, int i) {             // ... into the image of [128][V]
+    unsigned char* dst = Xg + static_cast<size_t>(record) * p.lay.sz_hc + static_cast<size_t>(v0 >> 6) * 16384;
+    const int idx = tid + kThreads * i, r = idx / (kW / 8), q = idx % (kW / 8);
+    if (idx < 128 * kN) *reinterpret_cast<uint4*>(dst + r * 128 + (((((v0 & 63) >> 3) + q) ^ (r & 7)) << 4)) = rec[i];
+  };
+  auto store_x = [&](unsigned char* X) {
+#pragma unroll
+    for (int m = 0; m < kM; ++m)
+#pragma unroll
+      for (int j = 0; j < kN; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          *reinterpret_cast<uint32_t*>(X + piece(m0 + 16 * m + 8 * e + g, j) + 4 * t) = f16x2_sat(-y[m][j][2 * e], -y[m][j][2 * e + 1]);
+  };
+  auto sync4 = [] { asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory"); };
+  uint32_t A0[kM][8][4], A1[kM][8][4], R[kM][kB][4];
+  float a[kM][2];
+  auto step = [&](int it, uint32_t (*A)[8][4], uint32_t (*An)[8][4]) {
+    unsigned char* X = sm + S::oX + (it & 1) * S::kX;
+    store_x(X);
+    // (a y - R) while the other warps arrive
+#pragma unroll
+    for (int m = 0; m < kM; ++m)
+#pragma unroll
+      for (int j = 0; j < kN; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const float2 r = __half22float2(*reinterpret_cast<const __half2*>(&R[m][j >> 1][2 * (j & 1) + e]));
+          y[m][j][2 * e] = fmaf(a[m][e], y[m][j][2 * e], -r.x);
+          y[m][j][2 * e + 1] = fmaf(a[m][e], y[m][j][2 * e + 1], -r.y);
+        }
+    const bool more = it + 1 < n;
+    if (more) wait_stage(it + 1);
+    const uint32_t Pn = smem_u32(sm + ((it + 1) % kSt) * S::kStage), xa = smem_u32(X);
+    sync4();
+    // products, and between them what the next step needs: the matrix pipe takes some 16 cycles for each
+    constexpr int kJ = kW == 32 ? 4 : 8;             // contraction steps whose operand is in registers at a time
+#pragma unroll
+    for (int h = 0; h < 8 / kJ; ++h) {
+      uint32_t B[kJ][kN][2];
+#pragma unroll
+      for (int j = 0; j < kJ; ++j) {
+        if (kW == 8) {
+          if (j % 2 == 0) {
+            uint32_t r[4];
+            ldsm4t(xa + piece(16 * (h * kJ + j) + lane, 0), r);
+            B[j][0][0] = r[0]; B[j][0][1] = r[1];
+            B[(j + 1) % kJ][0][0] = r[2]; B[(j + 1) % kJ][0][1] = r[3];
+          }
+        } else {
+#pragma unroll
+          for (int b = 0; b < kB; ++b) {
+            uint32_t r[4];
+            ldsm4t(xa + piece(16 * (h * kJ + j) + (lane & 15), 2 * b + (lane >> 4)), r);
+            B[j][(2 * b) % kN][0] = r[0]; B[j][(2 * b) % kN][1] = r[1];
+            B[j][(2 * b + 1) % kN][0] = r[2]; B[j][(2 * b + 1) % kN][1] = r[3];
+          }
+        }
+      }
+      if (h == 0)
+#pragma unroll
+        for (int i = 0; i < kRec; ++i) rec[i] = *reinterpret_cast<const uint4*>(record_at(i, X));
+#pragma unroll
+      for (int j = 0; j < kJ; ++j) {
+#pragma unroll
+        for (int b = 0; b < kN; ++b)
+#pragma unroll
+          for (int m = 0; m < kM; ++m) mma_f16(y[m][b], A[m][h * kJ + j], B[j][b][0], B[j][b][1]);
+        if (more) fetch_a(Pn, h * kJ + j, An);
+      }
+    }
+    if (more) fetch_r((it + 1) % kSt, R, a);
+#pragma unroll
+    for (int i = 0; i < kRec; ++i) record(bh * (ADJOINT ? NT : NT + 1) + chunk_of(it), i);
+  };
+  wait_stage(0);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) fetch_a(smem_u32(sm), j, A0);
+  fetch_r(0, R, a);
+  for (int it = 0; it < n; it += 2) {
+    step(it, A0, A1);
+    if (it + 1 < n) step(it + 1, A1, A0);
+  }
+  if (!ADJOINT && seg_last) {                        // the final state as one more record
+    unsigned char* X = sm + S::oX + (n & 1) * S::kX;
+    store_x(X);
+    sync4();
+#pragma unroll
+    for (int i = 0; i < kRec; ++i) {
+      rec[i] = *reinterpret_cast<const uint4*>(record_at(i, X));
+      record(bh * (NT + 1) + NT, i);
+    }
+  }
+  float* xT = seg_last ? (ADJOINT ? p.dh0 : p.hT) : carry;
+  const int nrow = seg_last ? p.Kr : kK;
+  if (xT) {
+#pragma unroll
+    for (int m = 0; m < kM; ++m)
+#pragma unroll
+      for (int j = 0; j < kN; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int d = m0 + 16 * m + 8 * e + g;
+          if (d < nrow)
+            *reinterpret_cast<float2*>(xT + (static_cast<size_t>(bh) * nrow + d) * V + v0 + 8 * j + 2 * t) =
+                make_float2(-y[m][j][2 * e], -y[m][j][2 * e + 1]);
+        }
+  }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -306,29 +558,31 @@ scan_nodelta_kernel(const Problem p) {
   }
 }
 
-constexpr int kScanAloneBytes = 118000;
-template <int kGr>
-static int launch_scan_t(const Problem& p, bool adjoint, cudaStream_t st) {
-  constexpr int kW = kVs * kGr;
-  int smem = kStages * 32768 + 2 * 128 * kW * 2 + static_cast<int>(sizeof(CtaShared)) + 1024;
-  // Launched early, CTAs of 16 columns settle in pairs on the first SMs that the kernel before leaves, and share their intake;
-  // asking for more than half of an SM's memory keeps them apart (one chain, us: 16 pairs x 32 chunks 131 -> 122, d_v = 128 166
-  // -> 152, 32 x 64 373 -> 357).  Not when the sequences are cut: the next range's scan then waits on the SMs of this one, not
-  // on others (captured step, alone / in pairs: 16 x 32 116 / 107, channel-wise 199 / 190; 8 x 32, with room for all, 75 / 83).
-  if (kGr == 1 && p.cn == p.NT) smem = kScanAloneBytes;
-  dim3 grid(p.V / kW, p.nbh);
-  if (adjoint) {
-    static SmemAttr attr;
-    if (attr.set(scan_kernel<true, kGr>, kGr == 1 ? kScanAloneBytes : smem)) return kErrLaunch;
-    if (launch_dependent(scan_kernel<true, kGr>, grid, dim3(kScanThreads<kGr>), smem, st, p) != cudaSuccess) return kErrLaunch;
-  } else {
-    static SmemAttr attr;
-    if (attr.set(scan_kernel<false, kGr>, kGr == 1 ? kScanAloneBytes : smem)) return kErrLaunch;
-    if (launch_dependent(scan_kernel<false, kGr>, grid, dim3(kScanThreads<kGr>), smem, st, p) != cudaSuccess) return kErrLaunch;
-  }
-  return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
+static int launch_scan_wide(const Problem& p, bool adjoint, cudaStream_t st) {
+  constexpr int smem = kStages * 32768 + 2 * 128 * kW * 2 + static_cast<int>(sizeof(CtaShared)) + 1024;
+  const dim3 grid(p.V / kW, p.nbh);
+  static SmemAttr attr[2];
+  if (attr[0].set(scan_kernel<false>, smem) || attr[1].set(scan_kernel<true>, smem)) return kErrLaunch;
+  const cudaError_t e = adjoint ? launch_dependent(scan_kernel<true>, grid, dim3(kScanThreads), smem, st, p)
+                                : launch_dependent(scan_kernel<false>, grid, dim3(kScanThreads), smem, st, p);
+  return e == cudaSuccess ? kOk : kErrLaunch;
 }
 
+template <int kCols>
+static int launch_scan_few(const Problem& p, bool adjoint, cudaStream_t st) {
+  // Four stages (three to five are within 3 %, two are 20 to 40 % slower).  More than half of an SM's memory on purpose: launched
+  // early, CTAs settle in pairs on the first SMs that the kernel before leaves, and share their intake.
+  constexpr int kM = kCols == 32 ? 1 : 2, kSt = 4, smem = ScanMmaSmem<kCols, kSt>::kBytes;
+  static_assert(smem > 118000 && smem <= 232448, "one CTA per SM");
+  const dim3 grid(p.V / kCols, p.nbh), block(32 * (8 / kM + 1));
+  static SmemAttr attr[2];
+  if (attr[0].set(scan_mma_kernel<false, kCols, kSt, kM>, smem) || attr[1].set(scan_mma_kernel<true, kCols, kSt, kM>, smem)) return kErrLaunch;
+  const cudaError_t e = adjoint ? launch_dependent(scan_mma_kernel<true, kCols, kSt, kM>, grid, block, smem, st, p)
+                                : launch_dependent(scan_mma_kernel<false, kCols, kSt, kM>, grid, block, smem, st, p);
+  return e == cudaSuccess ? kOk : kErrLaunch;
+}
+
+constexpr int kScanAloneBytes = 118000;      // more than half of an SM's memory, as above
 template <int kDepth>
 static int launch_scan_nodelta(const Problem& p, bool adjoint, bool alone, cudaStream_t st) {
   const dim3 g((p.V / 64) * 4, p.nbh);
@@ -347,10 +601,26 @@ int launch_scan(const Problem& p, bool adjoint, cudaStream_t st) {
     const int ctas = (p.V / 64) * 4 * p.nbh;
     return ctas <= 2 * sms ? launch_scan_nodelta<16>(p, adjoint, ctas <= sms, st) : launch_scan_nodelta<8>(p, adjoint, false, st);
   }
-  // 16 columns per CTA while every CTA has an SM of its own (B H = 16: 19.7 us for 32 chunks against 25.8); beyond that
-  // the CTAs share the SMs' intake from L2 and P's repeats count (d_v = 128, us for 64 chunks, 16 / 64 columns: B H = 24
-  // 61.8 / 57, 32 63 / 60, 48 119 / 67, 64 122 / 76, 128 252 / 156)
-  return (p.V / 16) * p.nbh <= sms ? launch_scan_t<1>(p, adjoint, st) : launch_scan_t<4>(p, adjoint, st);
+  // Warp-level products or tcgen05: by the whole problem, whatever part of it this call works on.  8, 16 and 32 columns give the same
+  // bits, tcgen05 others, and ranges of the pairs and of the sequences are to give those of one call.  The line is where 16 columns
+  // no longer give every CTA an SM of its own.  Beyond it 32 columns are the faster kernel (scan alone, us, 32 / 64 columns, 64 chunks,
+  // d_v = 64: 64 pairs 61 / 75; d_v = 128: 20 59 / 67, 32 60 / 70), but not in a chain, where P is read twice as often (32 pairs, d_v =
+  // 128, forward over 250 chunks 869 / 861, 64 chunks 181 / 179; training step 20 pairs x 32 chunks 220 / 223; d_v = 64, 64 x 32 314 / 318,
+  // 48 x 128 942 / 936).
+  if ((p.V / 16) * p.B * p.H > sms) return launch_scan_wide(p, adjoint, st);
+  const int c8 = (p.V / 8) * p.nbh;            // CTAs with 8 columns each
+  if (p.cn < p.NT) {
+    // A range of the sequences (captured step): chunk kernels of another range run beside the scan, and an SM that a scan CTA sits
+    // on is lost to them.  Few CTAs then count for more than a short step.  Captured step, us, 8 / 32 columns, d_v = 64, pairs x chunks:
+    // 8 x 32 68 / 84, 12 x 32 97 / 95, 12 x 64 155 / 169, 14 x 32 113 / 99, 16 x 32 119 / 102, 24 x 64 283 / 250, 32 x 64 353 / 314; d_v =
+    // 128: 3 x 16 51 / 61, 6 x 32 74 / 86, 7 x 32 93 / 88, 10 x 32 121 / 103, 16 x 32 172 / 133 (channel-wise 207 / 173; 64 columns, were
+    // the bits no matter, 161).
+    return 3 * c8 <= 2 * sms ? launch_scan_few<8>(p, adjoint, st) : launch_scan_few<32>(p, adjoint, st);
+  }
+  // A whole sequence: the fewest columns with which every CTA has an SM of its own.  Chain of a step, us, 8 / 16 columns (16 or 64 on
+  // tcgen05 before), d_v = 64: 16 x 32 120 / 137 (128); 18 x 64 211 / 228 (254); 32 x 32 207 / 191 (205); d_v = 128: 9 x 64 196 / 210 (227);
+  // 18 x 32 171 / 152 (163).
+  return c8 <= sms ? launch_scan_few<8>(p, adjoint, st) : launch_scan_few<16>(p, adjoint, st);
 }
 
 }  // namespace lg

@@ -47,6 +47,9 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                : "memory");
 }
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
 __device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -199,18 +202,6 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo, uint
   d |= static_cast<uint64_t>((sbo >> 4) & 0x3FFF) << 32;
   d |= 1ull << 46;  // descriptor version of this architecture
   d |= 2ull << 61;  // 128-byte swizzle
-  return d;
-}
-
-// The same for tiles in the 32-byte swizzle (atoms of 8 rows x 32 bytes; 16-byte piece c of row r stored
-// at c ^ ((r >> 2) & 1)), used for a 16-column operand that is contracted along its rows.
-__device__ __forceinline__ uint64_t make_desc_sw32(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((saddr & 0x3FFFF) >> 4);
-  d |= static_cast<uint64_t>((lbo >> 4) & 0x3FFF) << 16;
-  d |= static_cast<uint64_t>((sbo >> 4) & 0x3FFF) << 32;
-  d |= 1ull << 46;  // descriptor version of this architecture
-  d |= 6ull << 61;  // 32-byte swizzle
   return d;
 }
 

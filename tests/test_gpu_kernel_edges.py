@@ -43,7 +43,11 @@ def test_decode_of_many_pairs(gate, delta, dtype, extra, shift):
     # channel-wise prepare: one chunk per SM for the last time, two CTAs per SM for the first
     ("channel", True, 128, 128, 148, 64, torch.bfloat16), ("channel", True, 64, 64, 149, 60, torch.float16),
     ("channel", False, 128, 128, 149, 64, torch.bfloat16),
-    # state scans: 16 columns per CTA for the last time, 64 for the first; without the delta term 16 and 8 records ahead
+    # state scans: 8 and 16 columns per CTA for the last time, 16 and 64 for the first, on fewer chunks than stages and more; without
+    # the delta term 16 and 8 records ahead
+    ("scalar", True, 64, 128, 18, 70, torch.bfloat16), ("scalar", True, 64, 64, 19, 448, torch.float16),
+    ("none", True, 128, 128, 9, 320, torch.bfloat16), ("channel", True, 128, 128, 10, 192, torch.bfloat16),
+    ("scalar", True, 128, 128, 18, 100, torch.bfloat16), ("scalar", True, 128, 64, 19, 320, torch.bfloat16),
     ("scalar", True, 64, 128, 37, 320, torch.bfloat16), ("scalar", True, 64, 128, 38, 320, torch.bfloat16),
     ("none", False, 64, 128, 74, 1088, torch.bfloat16), ("none", False, 64, 128, 75, 1088, torch.bfloat16)])
 def test_persistent_grids_and_scan_rules(gate, delta, V, K, H, L, dtype):

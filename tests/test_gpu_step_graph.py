@@ -177,3 +177,27 @@ def test_step_graph_at_benchmark_shapes_equals_the_plain_chain_on_every_replay(g
         ops.check_status(buf.status)
         for n in names:
             assert torch.equal(getattr(buf, n), getattr(ref, n)), (rep, n)
+
+
+@pytest.mark.parametrize("V,H,L", [(64, 12, 640), (64, 13, 640), (64, 37, 640), (64, 38, 512), (128, 6, 640), (128, 18, 640)])
+def test_scan_kernels_of_parts_and_of_the_whole_give_the_same_bits(V, H, L):
+    """Gentle decays, so that the product of the state scan counts: a whole sequence (8 or 16 columns per CTA, or 64 for many
+    pairs), the captured step's ranges (8, 32 or 64) and ranges of the pairs, on either side of the lines between them."""
+    K = 128
+    dev = torch.device("cuda")
+    inp = make_inputs(1, L, H, K, V, gate="scalar", delta=True, seed=8, mild=True)
+    args = tuple(inp[n].to(dev) for n in ("q", "k", "v", "g", "beta", "h0"))
+    do = inp["do"].to(dev)
+    ref, buf, part = (ops.GdnBuffers(1, L, H, K, V, ops.GATE_SCALAR, True, dev) for _ in range(3))
+    ops.forward_into(ref, *args, K ** -0.5)
+    ops.backward_into(ref, *args, do, None, K ** -0.5)
+    graph = ops.GdnStepGraph(buf, *args, do, None, K ** -0.5)
+    assert graph.cut > 0
+    graph.replay()
+    for rng in ((0, 1), (1, H - 1)):
+        ops.forward_into(part, *args, K ** -0.5, bh_range=rng)
+        ops.backward_into(part, *args, do, None, K ** -0.5, bh_range=rng)
+    torch.cuda.synchronize()
+    for n in ("o", "hT", "dq", "dk", "dv", "dh0", "dg", "dbeta"):
+        assert torch.equal(getattr(buf, n), getattr(ref, n)), n
+        assert torch.equal(getattr(part, n), getattr(ref, n)), n
