@@ -75,7 +75,7 @@ struct ScSmem {
   // csp [2][64]; red [32]
   static constexpr int kFloats = 2 * 256 + 2 * 256 + 6 * 64 * kCg + 128 + 32;
   // An A operand of 64 rows is read as 128: 16 KB from the start of its tile, dbv the last of them.
-  static constexpr int kUsed = oF + kFloats * 4 + static_cast<int>(sizeof(ScBars)), kRead = oDH + kVT + 8192;
+  static constexpr int kUsed = oF + kFloats * 4 + static_cast<int>(sizeof(ScBars) + 2 * sizeof(ChunkAt)), kRead = oDH + kVT + 8192;
   static constexpr int kBytes = (kUsed > kRead ? kUsed : kRead) + 1024;
   static constexpr uint32_t kCols = V == 64 ? 256u : 512u;
 };
@@ -108,59 +108,50 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
   float *t2p = pq + 256, *t3p = t2p + 64 * kCg, *ddep = t3p + 64 * kCg, *rsp = ddep + 64 * kCg, *dbm = rsp + 64 * kCg;
   float *rvp = dbm + 64 * kCg, *csp = rvp + 64 * kCg;
   float* red = csp + 128;
-  ScBars* bars = reinterpret_cast<ScBars*>(red + 32);
+  ChunkAt* where = reinterpret_cast<ChunkAt*>(red + 32);      // this chunk and the next
+  ScBars* bars = reinterpret_cast<ScBars*>(where + 2);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, quad = warp & 3, cg = warp >> 2, d = quad * 32 + lane;
   const int c0 = cg * 16 * kU;                    // this thread's tokens / columns of every 64-column accumulator
   CtaCtl ctl{p.status, &bars->abort_flag};
   const int nchunks = p.nbh * p.cn;
-  struct At { int bh, c, z, b, h; };
-  auto at = [&](int n) {
-    At a;
-    a.bh = p.bh0 + n / p.cn;
-    a.c = p.c0 + n % p.cn;
-    a.z = a.bh * p.NT + a.c;
-    a.b = a.bh / p.H;
-    a.h = a.bh % p.H;
-    return a;
-  };
   // loads of a chunk (tid 0), by when their destinations fall free in the chunk before
   constexpr uint32_t kIn0 = 32768u + (WY ? V * 128u : 0u) + (DELTA ? 16384u : 8192u) + (SB ? 2u * V * 128 + V * 256 : V * 128u);
-  auto load_do = [&](const At& a) {               // do, and without the delta term v as v_new
+  auto load_do = [&](const ChunkAt& a) {               // do, and without the delta term v as v_new
     mbar_expect_tx(&bars->in0, kIn0);
     for (int t = 0; t < V / 64; ++t) {
       if (SB) tma_load_4d(tDO + t * 8192, &mdo, &bars->in0, t * 64, a.h, a.c * kC, a.b);
       if (!DELTA) tma_load_4d(tVN + t * 8192, &mv, &bars->in0, t * 64, a.h, a.c * kC, a.b);
     }
   };
-  auto load_v = [&](const At& a) {
+  auto load_v = [&](const ChunkAt& a) {
     if (WY) for (int t = 0; t < V / 64; ++t) tma_load_4d(tV + t * 8192, &mv, &bars->in0, t * 64, a.h, a.c * kC, a.b);
   };
-  auto load_rec = [&](const At& a) {              // v_new, h (dv2 where the first half of the call left it)
+  auto load_rec = [&](const ChunkAt& a) {              // v_new, h (dv2 where the first half of the call left it)
     if (SB && DELTA) bulk_g2s(tVN, p.saved + p.lay.vn + static_cast<size_t>(a.z) * p.lay.sz_vn, V * 128, &bars->in0);
-    if (SB) bulk_g2s(tH, p.saved + p.lay.hc + static_cast<size_t>(a.z + a.bh) * p.lay.sz_hc, V * 256, &bars->in0);
+    if (SB) bulk_g2s(tH, p.saved + p.lay.hc + static_cast<size_t>(a.z + a.b * p.H + a.h) * p.lay.sz_hc, V * 256, &bars->in0);
     else bulk_g2s(tDV, p.scratch + p.lay.dv2 + static_cast<size_t>(a.z) * p.lay.sz_dv2, V * 128, &bars->in0);
   };
-  auto load_dh = [&](const At& a) {
+  auto load_dh = [&](const ChunkAt& a) {
     mbar_expect_tx(&bars->in1, V * 256u);
     bulk_g2s(tDH, p.scratch + p.lay.dh + static_cast<size_t>(a.z) * p.lay.sz_dh, V * 256, &bars->in1);
   };
-  auto load_b = [&](const At& a) {                // [T; A], k
+  auto load_b = [&](const ChunkAt& a) {                // [T; A], k
     const unsigned char* ta = p.saved + p.lay.ta + static_cast<size_t>(a.z) * p.lay.sz_ta;
     if (DELTA) bulk_g2s(tT, ta, 16384, &bars->in0);
     else bulk_g2s(tA, ta + 8192, 8192, &bars->in0);
     for (int t = 0; t < 2; ++t) tma_load_4d(tK + t * 8192, &mk, &bars->in0, t * 64, a.h, a.c * kC, a.b);
   };
-  auto load_w = [&](const At& a) {                // the forward's WY factors
+  auto load_w = [&](const ChunkAt& a) {                // the forward's WY factors
     mbar_expect_tx(&bars->inU, 16384u);
     bulk_g2s(tW, p.saved + p.lay.w + static_cast<size_t>(a.z) * 16384, 16384, &bars->inU);
   };
-  auto load_u = [&](const At& a) {
+  auto load_u = [&](const ChunkAt& a) {
     mbar_expect_tx(&bars->inU, V * 128u);
     bulk_g2s(tU, p.saved + p.lay.u + static_cast<size_t>(a.z) * p.lay.sz_u, V * 128, &bars->inU);
   };
   // what a chunk will load, to L2: its tiles are free late (before this its loads were waited for, 2 to 5 k cycles per chunk)
-  auto prefetch = [&](const At& a) {
+  auto prefetch = [&](const ChunkAt& a) {
     for (int t = 0; t < 2; ++t) {
       tma_prefetch_4d(&mq, t * 64, a.h, a.c * kC, a.b);
       tma_prefetch_4d(&mk, t * 64, a.h, a.c * kC, a.b);
@@ -170,7 +161,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       tma_prefetch_4d(&mv, t * 64, a.h, a.c * kC, a.b);
     }
     if (DELTA) bulk_prefetch(p.saved + p.lay.vn + static_cast<size_t>(a.z) * p.lay.sz_vn, V * 128);
-    bulk_prefetch(p.saved + p.lay.hc + static_cast<size_t>(a.z + a.bh) * p.lay.sz_hc, V * 256);
+    bulk_prefetch(p.saved + p.lay.hc + static_cast<size_t>(a.z + a.b * p.H + a.h) * p.lay.sz_hc, V * 256);
     bulk_prefetch(p.scratch + p.lay.dh + static_cast<size_t>(a.z) * p.lay.sz_dh, V * 256);
     if (WY) {
       bulk_prefetch(p.saved + p.lay.w + static_cast<size_t>(a.z) * 16384, 16384);
@@ -178,7 +169,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     }
     bulk_prefetch(p.saved + p.lay.ta + static_cast<size_t>(a.z) * p.lay.sz_ta, 16384);
   };
-  auto load_q = [&](const At& a) {
+  auto load_q = [&](const ChunkAt& a) {
     for (int t = 0; t < 2; ++t) tma_load_4d(tQ + t * 8192, &mq, &bars->in0, t * 64, a.h, a.c * kC, a.b);
   };
 
@@ -193,7 +184,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     // any of the three may be the last.  (Late everywhere: SSD forward and backward 175.1 us instead of 172.3 at 1692 chunks, 557.8
     // instead of 555.3 at 4096; with the delta term no difference.)
     if (SB) {
-      const At a = at(blockIdx.x);
+      const ChunkAt a = chunk_at(p, blockIdx.x);
       load_do(a);
       load_v(a);
       load_b(a);
@@ -206,7 +197,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     tmem_relinquish();
   }
   // gates of a chunk, by one warp, two neighbouring tokens per lane: fetched a chunk ahead, then summed
-  auto fetch_gates = [&](const At& a, ScGates* o) {
+  auto fetch_gates = [&](const ChunkAt& a, ScGates* o) {
     if (p.gate == LETHE_GATE_SCALAR) warp_copy_gates(p, p.g, a.b, a.c, a.h, lane, o->G);
     if (WY) warp_copy_gates(p, p.beta, a.b, a.c, a.h, lane, o->beta);
   };
@@ -231,7 +222,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     *reinterpret_cast<float2*>(o->gam + 2 * lane) = make_float2(__expf(G0), __expf(G1));
   };
 
-  At a = at(blockIdx.x);
+  ChunkAt a = chunk_at(p, blockIdx.x);
   if (warp == 2) {
     fetch_gates(a, gates);
     sum_gates(gates);
@@ -261,7 +252,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
   uint32_t ph = 0;
   for (int n = blockIdx.x; n < nchunks; n += gridDim.x, ph ^= 1u) {
     const bool more = n + static_cast<int>(gridDim.x) < nchunks;
-    const At nx = more ? at(n + gridDim.x) : a;
+    if (tid == kThreads - 1 && more) where[ph ^ 1u] = chunk_at(p, n + gridDim.x);      // (read behind the next barrier)
     const int rows = p.rows_of(a.c);
     const size_t tok0 = (static_cast<size_t>(a.b) * p.L + a.c * kC) * p.H + a.h;
     unsigned char* dv2_g = p.scratch + p.lay.dv2 + static_cast<size_t>(a.z) * p.lay.sz_dv2;
@@ -272,7 +263,6 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     const bool keep = CUT || !p.lean;
 
     const ScGates& gt = gates[ph];
-    if (warp == 2 && more) fetch_gates(nx, gates + (ph ^ 1u));
     if (tid == 0 && n != static_cast<int>(blockIdx.x)) {
       bulk_wait_read();                             // dk of the chunk before has left its tile
       if (!S::kOwn) load_q(a);
@@ -312,6 +302,8 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       }
     }
     sync_for_issue();
+    const ChunkAt& nx = where[ph ^ 1u];
+    if (warp == 2 && more) fetch_gates(nx, gates + (ph ^ 1u));
 
     if (SB) {
       mbar_wait_warp(&bars->in1, ph, ctl, 415);
@@ -512,7 +504,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       }
       tc_fence_before();
       __syncthreads();
-      a = nx;
+      if (more) a = nx;
       continue;
     }
     if (WY) {
@@ -717,7 +709,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     }
     const float acc = chunk_rev_cumsum(dG, tid, red);
     if (tid < rows && p.gate == LETHE_GATE_SCALAR) p.dg[tok0 + static_cast<size_t>(tid) * p.H] = acc;
-    a = nx;
+    if (more) a = nx;
   }
   if (tid == 0 || tid == 96) bulk_wait_read();
   tc_fence_before();

@@ -239,6 +239,19 @@ __device__ __forceinline__ uint32_t rrec_off(int row, int col8) {
   return static_cast<uint32_t>((col8 >> 1) * 4096 + row * 32 + (col8 & 1) * 16);
 }
 
+// Where the n-th chunk of a call is: record index, and batch, head and chunk in the user's tensors.  One thread works it out
+// (divisions) and leaves it in shared memory for the others.
+struct __align__(16) ChunkAt { int z, b, h, c; };
+__device__ __forceinline__ ChunkAt chunk_at(const Problem& p, int n) {
+  const int q = n / p.cn, bh = p.bh0 + q;
+  ChunkAt a;
+  a.c = p.c0 + n - q * p.cn;
+  a.z = bh * p.NT + a.c;
+  a.b = bh / p.H;
+  a.h = bh - a.b * p.H;
+  return a;
+}
+
 // One value per token of chunk c to shared memory by one warp, two neighbouring tokens per lane, zero behind the last token; each
 // lane waits for its own (async_copy_wait) and reads them.  A chunk's gates are fetched like this a chunk ahead: a load to registers
 // is waited for by the warp that issues it, and by all others at the next barrier.

@@ -122,17 +122,4 @@ __device__ __forceinline__ BlockDecays block_decays(const float* Bb, const float
   return r;
 }
 
-// Where the n-th chunk of a call is: record index, and batch, head and chunk in the user's tensors.  One thread works it out
-// (divisions) and leaves it in shared memory for the others.
-struct __align__(16) ChunkAt { int z, b, h, c; };
-__device__ __forceinline__ ChunkAt chunk_at(const Problem& p, int n) {
-  const int q = n / p.cn, bh = p.bh0 + q;
-  ChunkAt a;
-  a.c = p.c0 + n - q * p.cn;
-  a.z = bh * p.NT + a.c;
-  a.b = bh / p.H;
-  a.h = bh - a.b * p.H;
-  return a;
-}
-
 }  // namespace lg

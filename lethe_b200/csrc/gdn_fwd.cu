@@ -25,8 +25,8 @@ namespace lg {
 // and the gates are summed a chunk ahead by one warp.  With one CTA per chunk instead, the wait for the first loads and the
 // start of the CTA were 40 % of its time.  The gates are applied to the columns of T, not to k and v: half the elements.
 // 4096 chunks: d_v = 64 167 -> 132 us, d_v = 128 183 -> 143; without the delta term (below) d_v = 128 121 -> 85.
-// The gates of the next chunk come by asynchronous copies to shared memory, and what its late loads will want is prefetched to L2
-// under product 1: without the delta term d_v = 128 79 -> 70, with it within 1 %.
+// The gates of the next chunk come by asynchronous copies to shared memory, its place from one thread, and (not at d_v = 128) its
+// tiles are prefetched to L2 under product 1: without the delta term d_v = 128 79 -> 70, with it within 2 %.
 // ---------------------------------------------------------------------------------------------
 constexpr int kPrepThreads = 256;
 
@@ -63,14 +63,8 @@ __device__ __forceinline__ void prep_gates(const Problem& p, int z, int lane, Pr
   *reinterpret_cast<float4*>(p.saved + p.lay.ad + static_cast<size_t>(z) * kK * 4 + lane * 16) = make_float4(a, a, a, a);
 }
 
-struct PrepAt {
-  int bh, c, z, b, h;
-  __device__ __forceinline__ PrepAt(const Problem& p, int n)
-      : bh(p.bh0 + n / p.cn), c(p.c0 + n % p.cn), z(bh * p.NT + c), b(bh / p.H), h(bh % p.H) {}
-};
-
 // k and q into the 128-row tile [k; q] (tid 0)
-__device__ __forceinline__ void prep_load_kq(unsigned char* KQ, const CUtensorMap* mk, const CUtensorMap* mq, uint64_t* bar, const PrepAt& a) {
+__device__ __forceinline__ void prep_load_kq(unsigned char* KQ, const CUtensorMap* mk, const CUtensorMap* mq, uint64_t* bar, const ChunkAt& a) {
   mbar_expect_tx(bar, 32768u);
   for (int t = 0; t < 2; ++t) {
     tma_load_4d(KQ + t * 16384, mk, bar, t * 64, a.h, a.c * kC, a.b);
@@ -79,7 +73,7 @@ __device__ __forceinline__ void prep_load_kq(unsigned char* KQ, const CUtensorMa
 }
 // ... and what a chunk will load to L2, under the products of the chunk before: its tiles are free late
 template <int V>
-__device__ __forceinline__ void prep_prefetch(const CUtensorMap* mk, const CUtensorMap* mq, const CUtensorMap* mv, const PrepAt& a) {
+__device__ __forceinline__ void prep_prefetch(const CUtensorMap* mk, const CUtensorMap* mq, const CUtensorMap* mv, const ChunkAt& a) {
   for (int t = 0; t < 2; ++t) {
     tma_prefetch_4d(mk, t * 64, a.h, a.c * kC, a.b);
     tma_prefetch_4d(mq, t * 64, a.h, a.c * kC, a.b);
@@ -87,13 +81,14 @@ __device__ __forceinline__ void prep_prefetch(const CUtensorMap* mk, const CUten
   for (int t = 0; t < V / 64; ++t) tma_prefetch_4d(mv, t * 64, a.h, a.c * kC, a.b);
 }
 template <int V>
-__device__ __forceinline__ void prep_load_v(unsigned char* Vt, const CUtensorMap* mv, uint64_t* bar, const PrepAt& a) {
+__device__ __forceinline__ void prep_load_v(unsigned char* Vt, const CUtensorMap* mv, uint64_t* bar, const ChunkAt& a) {
   mbar_expect_tx(bar, V * 128u);
   for (int t = 0; t < V / 64; ++t) tma_load_4d(Vt + t * 8192, mv, bar, t * 64, a.h, a.c * kC, a.b);
 }
 // a tile of bf16 to fp16 in place, whatever its shape
-__device__ __forceinline__ void prep_to_f16(unsigned char* t, int bytes, int tid) {
-  for (int i = tid * 16; i < bytes; i += kPrepThreads * 16) {
+template <int N = kPrepThreads>
+__device__ __forceinline__ void prep_to_f16(unsigned char* t, int bytes, int tid) {      // on N threads
+  for (int i = tid * 16; i < bytes; i += N * 16) {
     float x[8];
     unpack8_bf16(*reinterpret_cast<const uint4*>(t + i), x);
     *reinterpret_cast<uint4*>(t + i) = pack8_f16(x);
@@ -138,7 +133,7 @@ struct PrepSmem {
   static constexpr int oKD = oTA + 16384;        // M in fp32 and the scratch of its inverse (29 KB); then kd
   static constexpr int oW = oKD + 16384;         // [T diag(beta gamma); T diag(beta)]; then w; then R (d_v = 128: with u) on its way out
   static constexpr int oV = oW + 16384;          // v; then u
-  static constexpr int kUsed = oV + V * 128, kBytes = kUsed + 2 * static_cast<int>(sizeof(PrepGates)) + static_cast<int>(sizeof(CtaShared)) + 1024;
+  static constexpr int kUsed = oV + V * 128, kBytes = kUsed + 2 * static_cast<int>(sizeof(PrepGates) + sizeof(ChunkAt)) + static_cast<int>(sizeof(CtaShared)) + 1024;
   static_assert((kInvMtFloats + kInvScratchFloats) * 4 <= 32768, "scratch of the inverse");
 };
 
@@ -152,7 +147,8 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
   unsigned char *KQ = sm, *TA = sm + S::oTA, *KD = sm + S::oKD, *W = sm + S::oW, *Vt = sm + S::oV;
   float* Mt = reinterpret_cast<float*>(KD);
   PrepGates* gates = reinterpret_cast<PrepGates*>(sm + S::kUsed);
-  CtaShared* cs = reinterpret_cast<CtaShared*>(gates + 2);
+  ChunkAt* where = reinterpret_cast<ChunkAt*>(gates + 2);      // this chunk and the next
+  CtaShared* cs = reinterpret_cast<CtaShared*>(where + 2);
   // Threads 0-127 and 128-255 reach the same TMEM lanes (lane quadrant = warp & 3): the two halves take
   // the same rows and split the columns of every epilogue.
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, quad = warp & 3, half = warp >> 2, tq = tid & 127;
@@ -177,8 +173,9 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
   griddep_wait();
   griddep_launch();
   {
-    const PrepAt a(p, blockIdx.x);
+    const ChunkAt a = chunk_at(p, blockIdx.x);
     if (tid == 0) {
+      where[0] = a;
       prep_load_kq(KQ, &mk, &mq, full_kq, a);
       prep_load_v<V>(Vt, &mv, full_v, a);
     }
@@ -191,11 +188,10 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
 
   uint32_t ph = 0, pm = 0;
   for (int n = blockIdx.x; n < nchunks; n += gridDim.x, ph ^= 1u) {
-    const PrepAt a(p, n);
+    const ChunkAt a = where[ph];
     const bool more = n + static_cast<int>(gridDim.x) < nchunks;
-    const PrepAt nx(p, more ? n + gridDim.x : n);
     const PrepGates& gt = gates[ph];
-    if (warp == 1 && more) prep_fetch_gates(p, nx.b, nx.c, nx.h, lane, gates + (ph ^ 1u));
+    if (tid == kPrepThreads - 1 && more) where[ph ^ 1u] = chunk_at(p, n + gridDim.x);
 
     mbar_wait_warp(full_kq, ph, ctl, 201);
     if (!p.qk16) prep_to_f16(KQ, 32768, tid);
@@ -211,8 +207,11 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
       const uint32_t leader = elect_leader();
       issue_product_led(leader, tmem, Tile{smem_u32(KQ), 128, false}, Tile{smem_u32(KQ), 128, false}, 64, 128, 0u);
       umma_commit_led(leader, mma);
-    } else if (warp == 2 && lane == 0 && more) {
-      prep_prefetch<V>(&mk, &mq, &mv, nx);
+    } else if (warp == 1 && more) {
+      const ChunkAt nx = where[ph ^ 1u];
+      prep_fetch_gates(p, nx.b, nx.c, nx.h, lane, gates + (ph ^ 1u));
+    } else if (V == 64 && warp == 2 && lane == 0 && more) {      // (4096 chunks, us, without / with: d_v = 64 135 / 131, 128 143 / 148)
+      prep_prefetch<V>(&mk, &mq, &mv, where[ph ^ 1u]);
     }
     wait_products(mma, pm, ctl, 202);
     {
@@ -235,10 +234,17 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
     tc_fence_before();
     __syncthreads();
 
-    // ---- T = (I + M)^-1 (fp32, CUDA cores)
+    // ---- T = (I + M)^-1 (fp32, CUDA cores); v to fp16 on the warps that have no part in its first step (d_v = 128: behind it, v
+    // was requested late)
+    if (V == 64 && tid >= 64) {
+      mbar_wait_warp(full_v, ph, ctl, 203);
+      prep_to_f16<kPrepThreads - 64>(Vt, V * 128, tid - 64);
+    }
     unit_lower_inverse64(Mt, Mt, Mt + kInvMtFloats, TA, tid);
-    mbar_wait_warp(full_v, ph, ctl, 203);
-    prep_to_f16(Vt, V * 128, tid);
+    if (V == 128) {
+      mbar_wait_warp(full_v, ph, ctl, 203);
+      prep_to_f16(Vt, V * 128, tid);
+    }
     __syncthreads();
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
@@ -304,14 +310,14 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
       issue_product_led(leader, tmem + 128, Tile{smem_u32(KD), 64, true}, Tile{smem_u32(Vt), 64, true}, V, 64, 0u);
       umma_commit_led(leader, mma);
       if (tid == 0) {
-        if (more) prep_load_kq(KQ, &mk, &mq, full_kq, nx);        // nothing reads k and q any more
+        if (more) prep_load_kq(KQ, &mk, &mq, full_kq, where[ph ^ 1u]);        // nothing reads k and q any more
         bulk_s2g(p.saved + p.lay.w + static_cast<size_t>(a.z) * p.lay.sz_w, W, 16384);
         bulk_s2g(p.saved + p.lay.u + static_cast<size_t>(a.z) * p.lay.sz_u, Vt, V * 128);
         bulk_commit();
       }
     }
     __syncwarp();
-    if (warp == 1 && more) prep_gates(p, nx.z, lane, gates + (ph ^ 1u));
+    if (warp == 1 && more) prep_gates(p, where[ph ^ 1u].z, lane, gates + (ph ^ 1u));
     wait_products(mma, pm, ctl, 205);
     // P leaves from where [T; A] and kd were, R from where w (and u) were once their stores have read them
 #pragma unroll
@@ -326,7 +332,7 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
     fence_proxy_async();
     if (tid == 0) {
       bulk_wait_read();
-      if (V == 64 && more) prep_load_v<V>(Vt, &mv, full_v, nx);
+      if (V == 64 && more) prep_load_v<V>(Vt, &mv, full_v, where[ph ^ 1u]);
     }
     __syncthreads();
     if (tid == 0) {
@@ -360,7 +366,7 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
 template <int V>
 struct PrepNdSmem {
   static constexpr int oA = 32768, oKD = oA + 8192, oV = oKD + 16384;    // R leaves from where kd (d_v = 128: and v) was
-  static constexpr int kUsed = oV + V * 128, kBytes = kUsed + 2 * static_cast<int>(sizeof(PrepGates)) + static_cast<int>(sizeof(CtaShared)) + 1024;
+  static constexpr int kUsed = oV + V * 128, kBytes = kUsed + 2 * static_cast<int>(sizeof(PrepGates) + sizeof(ChunkAt)) + static_cast<int>(sizeof(CtaShared)) + 1024;
   static constexpr int kCols = V == 64 ? 128 : 256, kCtas = V == 64 ? 3 : 2;      // q k^T and R side by side in tensor memory
 };
 
@@ -373,7 +379,8 @@ prepare_nodelta_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, 
   unsigned char* sm = align1024(smem_raw);
   unsigned char *KQ = sm, *A = sm + S::oA, *KD = sm + S::oKD, *Vt = sm + S::oV;
   PrepGates* gates = reinterpret_cast<PrepGates*>(sm + S::kUsed);
-  CtaShared* cs = reinterpret_cast<CtaShared*>(gates + 2);
+  ChunkAt* where = reinterpret_cast<ChunkAt*>(gates + 2);      // this chunk and the next
+  CtaShared* cs = reinterpret_cast<CtaShared*>(where + 2);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, quad = warp & 3, half = warp >> 2, tq = tid & 127;
   CtaCtl ctl{p.status, &cs->abort_flag};
   uint64_t *full_kq = &cs->bar[0], *full_v = &cs->bar[1], *mma = &cs->bar[2];
@@ -396,8 +403,9 @@ prepare_nodelta_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, 
   griddep_wait();
   griddep_launch();
   {
-    const PrepAt a(p, blockIdx.x);
+    const ChunkAt a = chunk_at(p, blockIdx.x);
     if (tid == 0) {
+      where[0] = a;
       prep_load_kq(KQ, &mk, &mq, full_kq, a);
       prep_load_v<V>(Vt, &mv, full_v, a);
     }
@@ -410,11 +418,10 @@ prepare_nodelta_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, 
 
   uint32_t ph = 0, pm = 0;
   for (int n = blockIdx.x; n < nchunks; n += gridDim.x, ph ^= 1u) {
-    const PrepAt a(p, n);
+    const ChunkAt a = where[ph];
     const bool more = n + static_cast<int>(gridDim.x) < nchunks;
-    const PrepAt nx(p, more ? n + gridDim.x : n);
     const PrepGates& gt = gates[ph];
-    if (warp == 1 && more) prep_fetch_gates(p, nx.b, nx.c, nx.h, lane, gates + (ph ^ 1u));
+    if (tid == kPrepThreads - 1 && more) where[ph ^ 1u] = chunk_at(p, n + gridDim.x);
 
     mbar_wait_warp(full_kq, ph, ctl, 206);
     for (int idx = tid; idx < 64 * 16; idx += kPrepThreads) {
@@ -443,13 +450,15 @@ prepare_nodelta_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, 
         bulk_s2g(p.saved + p.lay.u + static_cast<size_t>(a.z) * p.lay.sz_u, Vt, V * 128);      // (u is v)
         bulk_commit();
       }
+    } else if (warp == 1 && more) {
+      const ChunkAt nx = where[ph ^ 1u];
+      prep_fetch_gates(p, nx.b, nx.c, nx.h, lane, gates + (ph ^ 1u));
     } else if (warp == 2 && lane == 0 && more) {
-      prep_prefetch<V>(&mk, &mq, &mv, nx);
+      prep_prefetch<V>(&mk, &mq, &mv, where[ph ^ 1u]);
     }
     __syncwarp();
-    if (warp == 1 && more) prep_gates(p, nx.z, lane, gates + (ph ^ 1u));
     wait_products(mma, pm, ctl, 208);
-    if (tid == 0 && more) prep_load_kq(KQ, &mk, &mq, full_kq, nx);
+    if (tid == 0 && more) prep_load_kq(KQ, &mk, &mq, full_kq, where[ph ^ 1u]);
     if (!p.lean) {
       if (tid == 0) bulk_wait_read();
       __syncthreads();
@@ -480,8 +489,9 @@ prepare_nodelta_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, 
       bulk_s2g(p.saved + p.lay.ta + static_cast<size_t>(a.z) * p.lay.sz_ta + 8192, A, 8192);
       bulk_commit();
       bulk_wait_read();
-      if (more) prep_load_v<V>(Vt, &mv, full_v, nx);
+      if (more) prep_load_v<V>(Vt, &mv, full_v, where[ph ^ 1u]);
     }
+    if (warp == 1 && more) prep_gates(p, where[ph ^ 1u].z, lane, gates + (ph ^ 1u));
     __syncthreads();
   }
   tc_fence_before();
