@@ -261,30 +261,30 @@ def path_fractions(workload: str, fwd_ms: float, bwd_ms: float, step_ms: float, 
 # every kernel's traffic grows in proportion to its chunks).  Keyed by (kernel, gate, d_v, delta).
 # Absent combinations report null.
 NCU_DRAM_BYTES_PER_CHUNK = {
-    ("prepare", "scalar", 64, True): (85.0e6 + 125.3e6) / 2048,
-    ("scan_fwd", "scalar", 64, True): (102.8e6 + 10.0e6) / 2048,
-    ("output", "scalar", 64, True): (134.8e6 + 12.0e6) / 2048,
-    ("bwd_pre", "scalar", 64, True): (101.2e6 + 4.1e6) / 2048,
-    ("scan_bwd", "scalar", 64, True): (101.7e6 + 9.9e6) / 2048,
-    ("main", "scalar", 64, True): (219.3e6 + 52.3e6) / 2048,
-    ("prepare", "channel", 128, True): (168.4e6 + 211.3e6) / 2048,
-    ("scan_fwd", "channel", 128, True): (137.4e6 + 37.2e6) / 2048,
-    ("output", "channel", 128, True): (184.6e6 + 35.7e6) / 2048,
-    ("bwd_pre", "channel", 128, True): (117.5e6 + 25.4e6) / 2048,
-    ("scan_bwd", "channel", 128, True): (135.3e6 + 36.4e6) / 2048,
-    ("main", "channel", 128, True): (403.4e6 + 136.8e6) / 2048,
-    ("prepare", "channel", 128, False): (335.6e6 + 198.6e6) / 4096,
-    ("scan_fwd", "channel", 128, False): (140.6e6 + 86.7e6) / 4096,
-    ("output", "channel", 128, False): (302.0e6 + 48.6e6) / 4096,
-    ("bwd_pre", "channel", 128, False): (134.2e6 + 78.0e6) / 4096,
-    ("scan_bwd", "channel", 128, False): (136.4e6 + 83.7e6) / 4096,
-    ("main", "channel", 128, False): (704.8e6 + 300.8e6) / 4096,
-    ("prepare", "scalar", 128, False): (202.5e6 + 123.3e6) / 4096,
-    ("scan_fwd", "scalar", 128, False): (140.5e6 + 86.5e6) / 4096,
-    ("output", "scalar", 128, False): (303.1e6 + 47.4e6) / 4096,
-    ("bwd_pre", "scalar", 128, False): (135.6e6 + 78.6e6) / 4096,
-    ("scan_bwd", "scalar", 128, False): (136.3e6 + 82.3e6) / 4096,
-    ("main", "scalar", 128, False): (571.6e6 + 173.0e6) / 4096,
+    ("prepare", "scalar", 64, True): (85.1e6 + 125.6e6) / 2048,
+    ("scan_fwd", "scalar", 64, True): (101.7e6 + 12.3e6) / 2048,
+    ("output", "scalar", 64, True): (134.8e6 + 11.3e6) / 2048,
+    ("bwd_pre", "scalar", 64, True): (101.2e6 + 5.3e6) / 2048,
+    ("scan_bwd", "scalar", 64, True): (101.7e6 + 10.3e6) / 2048,
+    ("main", "scalar", 64, True): (275.9e6 + 56.7e6) / 2048,
+    ("prepare", "channel", 128, True): (175.5e6 + 214.4e6) / 2048,
+    ("scan_fwd", "channel", 128, True): (135.3e6 + 37.1e6) / 2048,
+    ("output", "channel", 128, True): (184.6e6 + 36.3e6) / 2048,
+    ("bwd_pre", "channel", 128, True): (117.5e6 + 24.3e6) / 2048,
+    ("scan_bwd", "channel", 128, True): (135.3e6 + 35.0e6) / 2048,
+    ("main", "channel", 128, True): (470.5e6 + 135.5e6) / 2048,
+    ("prepare", "channel", 128, False): (337.1e6 + 195.5e6) / 4096,
+    ("scan_fwd", "channel", 128, False): (136.3e6 + 86.5e6) / 4096,
+    ("output", "channel", 128, False): (302.0e6 + 48.8e6) / 4096,
+    ("bwd_pre", "channel", 128, False): (134.2e6 + 77.8e6) / 4096,
+    ("scan_bwd", "channel", 128, False): (136.3e6 + 81.5e6) / 4096,
+    ("main", "channel", 128, False): (704.8e6 + 299.2e6) / 4096,
+    ("prepare", "scalar", 128, False): (202.4e6 + 124.1e6) / 4096,
+    ("scan_fwd", "scalar", 128, False): (136.4e6 + 86.4e6) / 4096,
+    ("output", "scalar", 128, False): (303.1e6 + 48.1e6) / 4096,
+    ("bwd_pre", "scalar", 128, False): (135.7e6 + 81.4e6) / 4096,
+    ("scan_bwd", "scalar", 128, False): (136.3e6 + 80.9e6) / 4096,
+    ("main", "scalar", 128, False): (603.6e6 + 175.7e6) / 4096,
 }
 
 
@@ -309,7 +309,7 @@ def algorithmic_bytes(kernel: str, Z: int, BH: int, V: int, delta: bool, cw: boo
             "output": qk + ta // 2 + img + vv + vv + ((vv + w) if delta else 0),
             "bwd_pre": qk + vv + r + ((w + ta // 2) if delta else 0),
             "scan_bwd": (p_ if delta else 0) + r + img + 512,
-            "main": g + 2 * qk + vv + 2 * img + vv + 2 * qk + vv + g + ((ta + vv) if delta else ta // 2),
+            "main": g + 2 * qk + vv + 2 * img + vv + 2 * qk + vv + g + ((ta + w + 2 * vv) if delta else ta // 2),
         }[kernel]
         return per * Z
     per = {
@@ -318,7 +318,7 @@ def algorithmic_bytes(kernel: str, Z: int, BH: int, V: int, delta: bool, cw: boo
         "output": qk + ta // 2 + img + vv + vv + ((vv + w) if delta else 0),
         "bwd_pre": qk + vv + r + ((w + ta // 2) if delta else 0),
         "scan_bwd": (p_ if delta else 0) + r + img + 512,
-        "main": 2 * qk + vv + 2 * img + vv + 2 * qk + vv + ((ta + vv) if delta else ta // 2),
+        "main": 2 * qk + vv + 2 * img + vv + 2 * qk + vv + ((ta + w + 2 * vv) if delta else ta // 2),
     }[kernel]
     return per * Z
 

@@ -2,7 +2,7 @@
 //
 // Work decomposition.  A "chunk" is 64 consecutive tokens of one (batch, head) pair; chunks are
 // numbered z = (b*H + h)*NT + c.  Chunk-parallel kernels run persistent CTAs, one chunk at a time;
-// the scan kernel runs one CTA per (b, h, slice of 16 or 64 columns of V) and walks the chunks in order.
+// the scan kernels run one CTA per (b, h, slice of 8 to 64 columns of V) and walk the chunks in order.
 //
 // Per-chunk records in the workspaces ("image" = the SW128 shared-memory tile image, so that a
 // record moves between global and shared memory with one contiguous bulk copy):
@@ -232,7 +232,7 @@ __device__ __forceinline__ void async_copy_wait() { asm volatile("cp.async.wait_
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // With the delta term the scan's input records R / Rb (128 rows x V columns, fp16) are stored as V / 16 column blocks of
-// [128 rows][16 columns]: one contiguous 4 KB block per scan CTA, 32 bytes per thread.  Byte offset of
+// [128 rows][16 columns]: a scan CTA takes whole blocks, contiguous pieces of 4 KB.  Byte offset of
 // the 8-column piece `col8` of `row` (without the delta term they are plain 128-row tile images, read by
 // scan_nodelta_kernel with full-line accesses):
 __device__ __forceinline__ uint32_t rrec_off(int row, int col8) {
