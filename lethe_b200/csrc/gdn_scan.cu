@@ -200,7 +200,7 @@ scan_kernel(const Problem p) {
       tmem_ld16(tmem + lane_base + kW + g * kVs, a1);
       tmem_ld_wait();
 #pragma unroll
-      for (int j = 0; j < kVs; ++j) x[j] = rr[j] - (a0[j] + a1[j]);
+      for (int j = 0; j < kVs; ++j) x[j] = rr[j] - a0[j] - a1[j];      // (in the order of scan_mma_kernel)
     }
     if (!ADJOINT && seg_last) {   // the final state as one more record
       unsigned char* rec = Xg + (static_cast<size_t>(bh) * (NT + 1) + NT) * szx;
@@ -229,11 +229,17 @@ scan_kernel(const Problem p) {
 // state in the accumulator layout of m16n8k16; per step they leave them as fp16 in shared memory, and after one barrier of the
 // state warps each reads all rows as the other operand.  Its rows of P (forward; columns, adjoint), R and the decays of the next
 // step are fetched to registers between the products; a producer warp keeps a ring of stages.
-// With y = -x the step is y <- (a y - R) + P fp16(x): the accumulator starts as the bracket and ends as the new state.
+// With y = -x the step is y <- (a y - R) + P fp16(x).
+//
+// The sums are those of scan_kernel, bit for bit (a chain of 16-long products rounds alike in either kind of matrix instruction; the
+// tests compare them): each half of the contraction from zero, then bracket + first half + second half.  So a pair's results do
+// not depend on how many others are in the call, and heads cut over several GPUs give the bits of the whole.  Starting the
+// accumulator with the bracket instead saved the two additions and gave bits that tcgen05 cannot (us a step, so / as here: 8 columns
+// 0.39 / 0.40, 16 0.53 / 0.51, 32 0.79 / 0.80; fetching R and storing the record between the products pays for the additions).
 //
 // Bound by the matrix pipe (17 cycles for a product of 16 x 8 x 16 per SM quarter, so 0.14 us per 8 columns) behind 0.25 us of
-// barrier, operand loads and P's way to registers: 0.39 us a step with 8 columns, 0.53 with 16, 0.85 with 32; tcgen05 took 0.69
-// with 16 (same measure: slope over the number of chunks, L2 cold) and takes 0.88 with 64.  With the fetch behind the products
+// barrier, operand loads and P's way to registers: 0.40 us a step with 8 columns, 0.51 with 16, 0.80 with 32; tcgen05 took 0.69
+// with 16 (same measure: slope over the number of chunks, L2 cold) and takes 0.83 with 64.  With the fetch behind the products
 // instead of between them 16 columns took 0.62, with four warps of kM = 2 at 32 columns the step is 0.92.
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t* r) {
@@ -252,6 +258,11 @@ __device__ __forceinline__ void mma_f16(float* c, const uint32_t* a, uint32_t b0
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma_f16_first(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {      // the same from zero
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+               : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
 }
 
 template <int kW, int kSt>
@@ -356,7 +367,7 @@ scan_mma_kernel(const Problem p) {
       }
     }
   };
-  auto fetch_r = [&](int s, uint32_t (*R)[kB][4], float (*a)[2]) {      // ... and R and the decays; then the stage is free
+  auto fetch_r = [&](int s, uint32_t (*R)[kB][4], float (*a)[2]) {      // ... and R and the decays
     const uint32_t P = smem_u32(sm + s * S::kStage);
 #pragma unroll
     for (int m = 0; m < kM; ++m) {
@@ -367,6 +378,8 @@ scan_mma_kernel(const Problem p) {
       a[m][0] = ad[0];
       a[m][1] = ad[8];
     }
+  };
+  auto free_stage = [&](int s) {
     __syncwarp();
     if (lane == 0) mbar_arrive(&empty[s]);
   };
@@ -392,7 +405,15 @@ scan_mma_kernel(const Problem p) {
   };
   auto sync4 = [] { asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory"); };
   uint32_t A0[kM][8][4], A1[kM][8][4], R[kM][kB][4];
-  float a[kM][2];
+  float a[kM][2], acc[kM][kN][4];
+  auto add_half = [&]() {
+#pragma unroll
+    for (int m = 0; m < kM; ++m)
+#pragma unroll
+      for (int j = 0; j < kN; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[m][j][e] += acc[m][j][e];
+  };
   auto step = [&](int it, uint32_t (*A)[8][4], uint32_t (*An)[8][4]) {
     unsigned char* X = sm + S::oX + (it & 1) * S::kX;
     store_x(X);
@@ -413,6 +434,14 @@ scan_mma_kernel(const Problem p) {
     sync4();
     // products, and between them what the next step needs: the matrix pipe takes some 16 cycles for each
     constexpr int kJ = kW == 32 ? 4 : 8;             // contraction steps whose operand is in registers at a time
+    // Contraction step behind which R is fetched and the record stored (8: behind the last).  us for 128 chunks, forward / adjoint,
+    // all behind the last and like this: 8 columns 57 / 59 (and with either in between up to 67 / 63), 16 columns 85 / 85 and 75 / 77,
+    // 32 columns 115 / 115 and 113 / 107.
+    constexpr int kFetch = kW == 8 ? 8 : kW == 16 ? 3 : 5, kStore = kW == 16 ? 5 : 8;
+    auto store_record = [&]() {
+#pragma unroll
+      for (int i = 0; i < kRec; ++i) record(bh * (ADJOINT ? NT : NT + 1) + chunk_of(it), i);
+    };
 #pragma unroll
     for (int h = 0; h < 8 / kJ; ++h) {
       uint32_t B[kJ][kN][2];
@@ -443,18 +472,26 @@ scan_mma_kernel(const Problem p) {
 #pragma unroll
         for (int b = 0; b < kN; ++b)
 #pragma unroll
-          for (int m = 0; m < kM; ++m) mma_f16(y[m][b], A[m][h * kJ + j], B[j][b][0], B[j][b][1]);
+          for (int m = 0; m < kM; ++m) {
+            if (j % 4) mma_f16(acc[m][b], A[m][h * kJ + j], B[j][b][0], B[j][b][1]);
+            else mma_f16_first(acc[m][b], A[m][h * kJ + j], B[j][b][0], B[j][b][1]);
+          }
         if (more) fetch_a(Pn, h * kJ + j, An);
+        if (h * kJ + j == 3) add_half();
+        if (h * kJ + j == kFetch && more) fetch_r((it + 1) % kSt, R, a);
+        if (h * kJ + j == kStore) store_record();
       }
     }
-    if (more) fetch_r((it + 1) % kSt, R, a);
-#pragma unroll
-    for (int i = 0; i < kRec; ++i) record(bh * (ADJOINT ? NT : NT + 1) + chunk_of(it), i);
+    if (kFetch == 8 && more) fetch_r((it + 1) % kSt, R, a);
+    add_half();
+    if (more) free_stage((it + 1) % kSt);
+    if (kStore == 8) store_record();
   };
   wait_stage(0);
 #pragma unroll
   for (int j = 0; j < 8; ++j) fetch_a(smem_u32(sm), j, A0);
   fetch_r(0, R, a);
+  free_stage(0);
   for (int it = 0; it < n; it += 2) {
     step(it, A0, A1);
     if (it + 1 < n) step(it + 1, A1, A0);
@@ -601,9 +638,8 @@ int launch_scan(const Problem& p, bool adjoint, cudaStream_t st) {
     const int ctas = (p.V / 64) * 4 * p.nbh;
     return ctas <= 2 * sms ? launch_scan_nodelta<16>(p, adjoint, ctas <= sms, st) : launch_scan_nodelta<8>(p, adjoint, false, st);
   }
-  // Warp-level products or tcgen05: by the whole problem, whatever part of it this call works on.  8, 16 and 32 columns give the same
-  // bits, tcgen05 others, and ranges of the pairs and of the sequences are to give those of one call.  The line is where 16 columns
-  // no longer give every CTA an SM of its own.  Beyond it 32 columns are the faster kernel (scan alone, us, 32 / 64 columns, 64 chunks,
+  // Warp-level products or tcgen05 (the same bits): by the whole problem, since calls on ranges of its pairs run beside one another.
+  // The line is where 16 columns no longer give every CTA an SM of its own.  Beyond it 32 columns are the faster kernel (scan alone, us, 32 / 64 columns, 64 chunks,
   // d_v = 64: 64 pairs 61 / 75; d_v = 128: 20 59 / 67, 32 60 / 70), but not in a chain, where P is read twice as often (32 pairs, d_v =
   // 128, forward over 250 chunks 869 / 861, 64 chunks 181 / 179; training step 20 pairs x 32 chunks 220 / 223; d_v = 64, 64 x 32 314 / 318,
   // 48 x 128 942 / 936).
@@ -613,8 +649,8 @@ int launch_scan(const Problem& p, bool adjoint, cudaStream_t st) {
     // A range of the sequences (captured step): chunk kernels of another range run beside the scan, and an SM that a scan CTA sits
     // on is lost to them.  Few CTAs then count for more than a short step.  Captured step, us, 8 / 32 columns, d_v = 64, pairs x chunks:
     // 8 x 32 68 / 84, 12 x 32 97 / 95, 12 x 64 155 / 169, 14 x 32 113 / 99, 16 x 32 119 / 102, 24 x 64 283 / 250, 32 x 64 353 / 314; d_v =
-    // 128: 3 x 16 51 / 61, 6 x 32 74 / 86, 7 x 32 93 / 88, 10 x 32 121 / 103, 16 x 32 172 / 133 (channel-wise 207 / 173; 64 columns, were
-    // the bits no matter, 161).
+    // 128: 3 x 16 51 / 61, 6 x 32 74 / 86, 7 x 32 93 / 88, 10 x 32 121 / 103, 16 x 32 172 / 133 (channel-wise 207 / 173; 64
+    // columns, left out here while their bits differed, 161).
     return 3 * c8 <= 2 * sms ? launch_scan_few<8>(p, adjoint, st) : launch_scan_few<32>(p, adjoint, st);
   }
   // A whole sequence: the fewest columns with which every CTA has an SM of its own.  Chain of a step, us, 8 / 16 columns (16 or 64 on

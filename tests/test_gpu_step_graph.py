@@ -201,3 +201,28 @@ def test_scan_kernels_of_parts_and_of_the_whole_give_the_same_bits(V, H, L):
     for n in ("o", "hT", "dq", "dk", "dv", "dh0", "dg", "dbeta"):
         assert torch.equal(getattr(buf, n), getattr(ref, n)), n
         assert torch.equal(getattr(part, n), getattr(ref, n)), n
+
+
+@pytest.mark.parametrize("gate,V,parts", [("scalar", 64, (18, 20)), ("scalar", 64, (1, 37)), ("scalar", 128, (9, 10)),
+                                          ("channel", 128, (1, 18)), ("none", 128, (3, 10, 10))])
+def test_a_shard_gives_the_bits_of_the_whole(gate, V, parts):
+    """Heads cut into problems of their own, as over several GPUs: the whole takes the state scan of 64 columns per CTA, the parts
+    those of 8 and 16 (and one pair the shortest).  Gentle decays, so that the scan's products count; the last chunk is ragged."""
+    K, L, H = 128, 620, sum(parts)
+    dev = torch.device("cuda")
+    inp = make_inputs(1, L, H, K, V, gate=gate, delta=True, seed=8, mild=True)
+    dhT = 0.1 * torch.randn(1, H, K, V, generator=torch.Generator().manual_seed(7))
+
+    def run(heads):
+        names = [n for n in ("q", "k", "v", "g", "beta", "h0") if inp[n] is not None]
+        d = {n: (inp[n][:, heads] if n == "h0" else inp[n][:, :, heads]).contiguous().to(dev).requires_grad_(True) for n in names}
+        o, hT = ops.gdn_chunk(*(d.get(n) for n in ("q", "k", "v", "g", "beta", "h0")))
+        grads = torch.autograd.grad((o, hT), [d[n] for n in names], (inp["do"][:, :, heads].to(dev), dhT[:, heads].to(dev)))
+        return {"o": o.detach(), "hT": hT.detach(), **{"d" + n: t for n, t in zip(names, grads)}}
+
+    whole, at = run(slice(0, H)), 0
+    for n in parts:
+        part, heads = run(slice(at, at + n)), slice(at, at + n)
+        for name, t in part.items():
+            assert torch.equal(t, (whole[name][:, heads] if name in ("hT", "dh0") else whole[name][:, :, heads])), (name, at, n)
+        at += n
