@@ -32,7 +32,7 @@
 //
 // dM.  The VJP of the inverse is -T^T dT T^T with dT = dv2 (w v)^T + dw (b gamma k)^T; since T^T dv2 = dbv, T^T dw = dbgk, T (w v)
 // = u and T (b gamma k) = w, that is -(dbv u^T + dbgk w^T): one product behind dbv and dbgk, which are wanted anyway, instead of
-// three in a row, for 32 KB more to read per chunk.
+// three in a row, for 32 KB more to read per chunk.  Its error, and that v_new is to be made of the same u and w: gdn_bwd_main.cu.
 //
 // What bounds it: the chain of four dependent product groups and the CUDA-core phases (issue slots 43 % busy); 300 KB of traffic
 // per chunk are 12 k cycles of an SM's share of HBM.  The CTA is persistent and fetches the next chunk's tiles into the ones that

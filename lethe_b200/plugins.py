@@ -5,11 +5,18 @@ driven by the CUDA kernels of this package unchanged, and so that each kernel ca
 reference's own "micro-gate" granularity (``build_microgate_bundles``, ``gdn2_chunkwise.py:318-388``).
 
 Both callables take and return head-major chunked fp32 tensors ``[B, H, NT, C, ...]`` (C = 64,
-d_k = 128) and return fresh tensors, like the reference's.  They stage their arguments into the
-per-chunk records the kernels read (PyTorch is used for that restaging only) and run exactly one
-kernel of the backward call each: the adjoint state scan for K#1, the WY / triangular-inverse VJP for
-K#2 (``k2_fn`` for the scalar gate, ``k2_fn_cw`` for the channel-wise gate with independent erase and
-write gates).
+d_k = 128) and return fresh tensors, like the reference's.  They lay their arguments out as the
+per-chunk records the kernels read and run one kernel of the backward call each: the adjoint state scan
+for K#1, the WY / triangular-inverse VJP for K#2 (``k2_fn`` for the scalar gate, ``k2_fn_cw`` for the
+channel-wise gate with independent erase and write gates).  Records that the arguments do not contain and
+an ordinary call has from its prepare kernel are products formed with PyTorch here, from the arguments as
+given (``t_mat`` need not be the inverse the prepare kernel would find): P and Rb for K#1, w and u for K#2.
+
+K#2 runs its kernel three times.  The gradient of the inverse is a product with w and u, which the
+records hold in fp16; in an ordinary call the same two records make v_new, and most of what their rounding does
+to dg cancels between the two (see ``gdn_bwd_main.cu``).  K#2 by itself would keep it: 2-norm error of dg for
+the scalar gate, over four kinds of keys, 1.4e-4 to 9.4e-4, and 0.9e-4 to 4.7e-4 like this.  The result is linear
+in w and u, so their remainders go through a second run, and a third without either takes out what the two share.
 """
 
 from __future__ import annotations
@@ -70,11 +77,22 @@ def _layout(B, H, L, V, gate):
     return Z, sz, off, sz2, off2
 
 
-def _wy_factors(buf, sz, off, Z, t_mat: Tensor, gated_k: Tensor, gated_v: Tensor) -> None:
-    """Records of the forward that the VJP reads: w = T (gated k), u = T (gated v)."""
-    for n, x in (("w", gated_k), ("u", gated_v)):
-        img = to_image((t_mat.float() @ x).half()).reshape(Z, -1)
-        _record_view(buf.saved, off[n], sz[n], Z, torch.float16).copy_(img)
+def _wy_vjp(buf, sz, off, Z, t_mat: Tensor, gated_k: Tensor, gated_v: Tensor, run, outs) -> list[Tensor]:
+    """The WY kernel on w = T (gated k), u = T (gated v) to fp32 precision: ``run`` launches it on the records W and U, ``outs``
+    names the buffers that hold its results."""
+    x = {n: t_mat.float() @ y for n, y in (("w", gated_k), ("u", gated_v))}
+    hi = {n: y.half() for n, y in x.items()}
+    up = 2.0 ** 11                                   # the remainder of an fp16 rounding is at most 2^-11 of the value
+
+    def results(records):
+        for n, y in records.items():
+            _record_view(buf.saved, off[n], sz[n], Z, torch.float16).copy_(to_image(y).reshape(Z, -1))
+        run()
+        return [getattr(buf, n).float().clone() for n in outs]
+
+    whole, rest = results(hi), results({n: ((x[n] - hi[n].float()) * up).half() for n in x})
+    none = results({n: torch.zeros_like(y) for n, y in hi.items()})
+    return [a + (b - c) / up for a, b, c in zip(whole, rest, none)]
 
 
 def _untok(x: Tensor) -> Tensor:
@@ -146,8 +164,6 @@ def k2_fn(k: Tensor, v: Tensor, beta: Tensor, g2: Tensor, t_mat: Tensor, dw: Ten
     ta = torch.zeros(B, H, NT, 128, 64, dtype=torch.float16, device=dev)
     ta[..., :64, :] = t_mat.half()
     _record_view(buf.saved, off["ta"], sz["ta"], Z, torch.float16).copy_(to_image(ta).reshape(Z, -1))
-    bt = beta.to(f32)[..., None]
-    _wy_factors(buf, sz, off, Z, t_mat, bt * torch.exp2(g2.to(f32))[..., None] * k.to(f32), bt * v.to(f32))
     _record_view(buf.scratch, off2["dv2"], sz2["dv2"], Z, torch.float16).copy_(to_image(du.half()).reshape(Z, -1))
     _record_view(buf.scratch, off2["dw"], sz2["dw"], Z, torch.float16).copy_(to_image(dw.half()).reshape(Z, -1))
     _record_view(buf.scratch, off2["dkb"], sz2["dkb"], Z, f32).zero_()
@@ -161,12 +177,11 @@ def k2_fn(k: Tensor, v: Tensor, beta: Tensor, g2: Tensor, t_mat: Tensor, dw: Ten
     g_t = _untok(g_tok[..., None])[..., 0].contiguous()
     b_t = _untok(beta.to(f32)[..., None])[..., 0].contiguous()
     dov = torch.zeros(B, L, H, V, dtype=torch.bfloat16, device=dev)
-    ops.backward_into(buf, k16, k16, v16, g_t, b_t, None, dov, None, 1.0, kernel_mask=8)
-    dk2 = _tok(buf.dk.to(f32))
-    dv = _tok(buf.dv.to(f32))
-    db = _tok(buf.dbeta[..., None])[..., 0]
-    dg = _tok(buf.dg[..., None])[..., 0]
-    return dk2.clone(), dv.clone(), db.clone(), dg.clone()
+    bt = beta.to(f32)[..., None]
+    dk2, dv, db, dg = _wy_vjp(
+        buf, sz, off, Z, t_mat, bt * torch.exp2(g2.to(f32))[..., None] * k.to(f32), bt * v.to(f32),
+        lambda: ops.backward_into(buf, k16, k16, v16, g_t, b_t, None, dov, None, 1.0, kernel_mask=8), ("dk", "dv", "dbeta", "dg"))
+    return _tok(dk2), _tok(dv), _tok(db[..., None])[..., 0], _tok(dg[..., None])[..., 0]
 
 
 def k2_fn_cw(k: Tensor, v: Tensor, b: Tensor, w: Tensor, g2: Tensor, t_mat: Tensor, dwy: Tensor, du: Tensor
@@ -186,7 +201,6 @@ def k2_fn_cw(k: Tensor, v: Tensor, b: Tensor, w: Tensor, g2: Tensor, t_mat: Tens
     ta = torch.zeros(B, H, NT, 128, 64, dtype=torch.float16, device=dev)
     ta[..., :64, :] = t_mat.half()
     _record_view(buf.saved, off["ta"], sz["ta"], Z, torch.float16).copy_(to_image(ta).reshape(Z, -1))
-    _wy_factors(buf, sz, off, Z, t_mat, b.to(f32) * torch.exp2(g2.to(f32)) * k.to(f32), w.to(f32) * v.to(f32))
     _record_view(buf.scratch, off2["dv2"], sz2["dv2"], Z, torch.float16).copy_(to_image(du.half()).reshape(Z, -1))
     _record_view(buf.scratch, off2["dw"], sz2["dw"], Z, torch.float16).copy_(to_image(dwy.half()).reshape(Z, -1))
     _record_view(buf.scratch, off2["dkb"], sz2["dkb"], Z, f32).zero_()
@@ -199,6 +213,7 @@ def k2_fn_cw(k: Tensor, v: Tensor, b: Tensor, w: Tensor, g2: Tensor, t_mat: Tens
     g_t = _untok(g_tok)
     b_t, w_t = _untok(b.to(f32)), _untok(w.to(f32))
     dov = torch.zeros(B, L, H, V, dtype=torch.bfloat16, device=dev)
-    ops.backward_into(buf, k16, k16, v16, g_t, None, None, dov, None, 1.0, kernel_mask=8, b_gate=b_t, w_gate=w_t)
-    return (_tok(buf.dk.to(f32)).clone(), _tok(buf.dv.to(f32)).clone(), _tok(buf.db).clone(), _tok(buf.dw).clone(),
-            _tok(buf.dg).clone())
+    return tuple(map(_tok, _wy_vjp(
+        buf, sz, off, Z, t_mat, b.to(f32) * torch.exp2(g2.to(f32)) * k.to(f32), w.to(f32) * v.to(f32),
+        lambda: ops.backward_into(buf, k16, k16, v16, g_t, None, None, dov, None, 1.0, kernel_mask=8, b_gate=b_t, w_gate=w_t),
+        ("dk", "dv", "db", "dw", "dg"))))
