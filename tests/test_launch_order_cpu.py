@@ -18,10 +18,15 @@ from .cusource import block, kernel_body, source
 MAIN = 12      # Stage B and the WY VJP
 
 
-def early_reads(name, kernel, after_scan=False):
+def early_reads(name, kernel, after_scan=False, adjoint=None):
     """Records that a kernel reads before its first wait for the kernel before it (as text: every branch counts, but for
     what a call does only when it has launched the adjoint scan itself)."""
     body = kernel_body(name, kernel)
+    if adjoint is not None:                    # scan_mma_kernel: which of its producer's two waits comes first
+        assert "if (!ADJOINT) griddep_wait();" in body and "if (ADJOINT) griddep_wait();" in body
+        body = body.replace("if (%sADJOINT) griddep_wait();" % ("!" if adjoint else ""), "")
+    for m in list(re.finditer(r"const unsigned char\* (\w+) = ([^;]*);", body)):        # a pointer is no read
+        body = re.sub(r"\b%s\b" % m.group(1), "(%s)" % m.group(2), body.replace(m.group(0), ""))
     body = body[:body.index("griddep_wait();")]
     if not after_scan:
         body = re.sub(r"if \(p\.after_scan\) \w+\(a\);", "", body)
@@ -36,6 +41,11 @@ def early_reads(name, kernel, after_scan=False):
             if re.search(r"\b%s\(" % n, text):
                 text += lambdas.pop(n)
     return {r for r in re.findall(r"\bp\.lay\.(\w+)", text) if not r.startswith("sz_")}
+
+
+def adjoint_early():
+    """Of either kernel with a product: scan_kernel's P, as asserted below, and what scan_mma_kernel reads."""
+    return {"p"} | early_reads("gdn_scan.cu", "scan_mma_kernel", adjoint=True)
 
 
 def test_what_the_kernels_read_before_they_wait():
@@ -58,8 +68,10 @@ def test_what_the_kernels_read_before_they_wait():
                                  ("gdn_cw_fwd.cu", "prepare_cw_kernel", r"\bkern<<<")):
         assert "griddep_wait" not in kernel_body(name, kernel)             # launched plainly: nothing to wait for
         assert re.search(launch, source(name)) and "launch_dependent" not in source(name)
-    # the scan's warp that streams P does not wait in the adjoint
+    # the scans' warp that streams P does not wait in the adjoint (on warp-level products it brings the decays along)
     assert "if (!(ADJOINT && warp == kStateWarps)) {" in kernel_body("gdn_scan.cu", "scan_kernel")
+    assert early_reads("gdn_scan.cu", "scan_mma_kernel", adjoint=False) == set()
+    assert adjoint_early() == {"p", "ad"}
 
 
 # ---- stand-ins ---------------------------------------------------------------------------------------------------
@@ -158,7 +170,7 @@ def schedule(monkeypatch, NT, cut, bwd_cuts, gate=ops.GATE_SCALAR, V=64):
 
 # records a kernel reads early, reads after its wait, writes; "carry" and "end" belong to no chunk
 READS = {"prepare": set(), "scan": {"p", "r", "ad", "carry_f"}, "output": {"qg", "w", "ta", "u", "hc"},
-         "pre": {"ta", "w", "qg"}, "adjoint": {"p", "ad", "rb", "carry_b"}, "main": {"ta", "vn", "hc", "dh"}}
+         "pre": {"ta", "w", "qg"}, "adjoint": {"p", "ad", "rb", "carry_b"}, "main": {"ta", "vn", "hc", "dh", "w", "u"}}
 WRITES = {"prepare": {"ta", "w", "u", "p", "r", "ad", "qg"}, "scan": {"hc", "carry_f"}, "output": {"vn", "o"},
           "pre": {"rb"}, "adjoint": {"dh", "carry_b"}, "main": {"dq", "dv2", "dw"}}
 SEQUENCE = {"carry_f", "carry_b"}
@@ -190,11 +202,13 @@ CUTS = [(32, None, None), (64, None, None), (1, None, None), (32, 18, (9, 18)), 
 @pytest.mark.parametrize("NT,cut,bwd_cuts", CUTS)
 def test_no_kernel_of_the_captured_step_reads_what_may_still_be_written(monkeypatch, NT, cut, bwd_cuts):
     main = early_reads("gdn_bwd_main.cu", "bwd_sc_kernel") | early_reads("gdn_cw_bwd.cu", "bwd_cw_kernel")
-    early = {"output": early_reads("gdn_fwd.cu", "output_kernel"), "adjoint": {"p"}, "main": main}
+    early = {"output": early_reads("gdn_fwd.cu", "output_kernel"), "adjoint": adjoint_early(), "main": main}
     check(schedule(monkeypatch, NT, cut, bwd_cuts), NT, early)
 
 
-def test_the_check_sees_a_reader_that_starts_too_soon(monkeypatch):
-    """A main kernel that read v_new before its wait would race with the output kernels, at the default cuts too."""
-    with pytest.raises(AssertionError, match="'early', 'output'"):
-        check(schedule(monkeypatch, 32, None, None), 32, {"main": {"ta", "vn"}})
+@pytest.mark.parametrize("early,writer", [({"main": {"ta", "vn"}}, "output"), ({"adjoint": {"p", "rb"}}, "pre")])
+def test_the_check_sees_a_reader_that_starts_too_soon(monkeypatch, early, writer):
+    """A main kernel that read v_new before its wait would race with the output kernels, at the default cuts too; an adjoint scan
+    that read its input, with the kernel that makes it."""
+    with pytest.raises(AssertionError, match="'early', '%s'" % writer):
+        check(schedule(monkeypatch, 32, None, None), 32, early)
