@@ -82,7 +82,12 @@ typedef struct LetheGdnArgs {
   int32_t* status;        /* device word, see above                                         */
   /* Profiling aid: 0 runs every kernel of the call.  Otherwise bit i selects kernel i of the call  */
   /* (forward: 1 prepare, 2 state scan, 4 output; backward: 1 scan input, 2 adjoint scan,           */
-  /* 4 Stage B, 8 WY VJP); a partial call relies on the records left by an earlier full call.       */
+  /* 4 Stage B, 8 WY VJP); a partial call relies on the records left by an earlier full call (names   */
+  /* and layout: csrc/gdn_common.cuh).  Backward with the delta term, records read: 1: A (of TA), W,   */
+  /* QG (channel-wise gate); 2: P, AD, RB; 4: A, VN, Hc, DH; 8: T (of TA), W and U (the WY factors     */
+  /* w = T (beta gamma k) and u = T (beta v), which the gradient of the inverse is formed with), and   */
+  /* DV2, DW, DKB, DGB, RB as bit 4 left them.  A caller that lays records down for 8 alone has to     */
+  /* supply W and U too.  Without the delta term 4 reads A, Hc and DH, and 8 is empty.                 */
   uint32_t kernel_mask;
   /* Optional split of the beta gradient (delta = 1).  NULL: `dbeta` receives the whole gradient.     */
   /* Non-NULL: `dbeta` receives the erase-gate part and `dbeta_write` the write-gate part, the two    */

@@ -121,3 +121,20 @@ def test_op_refuses_cpu_tensors():
     q = torch.zeros(1, 64, 1, 128)
     with pytest.raises(ops.GdnError):
         ops.gdn_chunk(q, q, torch.zeros(1, 64, 1, 64), None, None)
+
+
+def test_header_names_the_records_that_a_partial_backward_reads():
+    """A caller may run Stage B or the WY VJP alone on records it has laid down: the contract names every one they use."""
+    import re
+
+    from .cusource import kernel_body
+
+    with open(os.path.join(ROOT, "include", "lethe_gdn.h")) as f:
+        text = f.read()
+    text = text[text.index("Profiling aid:"):text.index("uint32_t kernel_mask;")]
+    named = {w.lower() for w in re.findall(r"\b[A-Z][A-Zc0-9]*\b", text)}
+    for name, kernel in (("gdn_bwd_pre.cu", "bwd_pre_kernel"), ("gdn_scan.cu", "scan_mma_kernel"), ("gdn_bwd_main.cu", "bwd_sc_kernel"),
+                         ("gdn_cw_bwd.cu", "bwd_cw_kernel")):
+        used = {r for r in re.findall(r"\bp\.lay\.(\w+)", kernel_body(name, kernel)) if not r.startswith("sz_")}
+        used -= {"carry_f", "carry_b", "r"}            # handed on within the workspace; the forward scan's input
+        assert used and used <= named, (kernel, used - named)
