@@ -24,12 +24,14 @@
 // dM.  The VJP of the inverse is -T^T dT T^T with dT = dv2 (beta v)^T + dw (beta gamma k)^T; since T^T dv2 = dbv, T^T dw = dbgk,
 // T (beta v) = u and T (beta gamma k) = w, that is -(dbv u^T + dbgk w^T): one product behind two that are wanted anyway, instead of
 // dT, X = dT T^T and -T^T X in a row.
-// The fp16 records u and w are also what the forward makes v_new = u - w h of.  The rounding e_u, e_w of a row of theirs is one vector
-// for a whole column of dM and adds up in dg, more so the more the keys resemble one another.  But rowsum(dkk KK) - colsum(dkk KK)
-// has <dv2, e_u> + <dw, e_w> from it (and <dbv, (I + M) e_u> + .., which stays), and -<v_new, dv2> in Stage B the negative of that:
-// with the same records in both places it cancels.  2-norm error of dg in 1e-4, dM from dT (or from dbv v^T and dbgk k^T, T^T applied first) / as here: independent keys 4.3 / 4.25,
-// behind a SiLU 5.9 / 5.3, a ReLU 12.6 / 10.0, around a common direction 8.3 / 7.0; channel-wise gate 5.4 / 5.35, 5.6 / 5.5, 6.65 / 6.3,
-// 8.2 / 8.2.  By itself, without v_new beside it, this form has up to twice the error of the other.
+// The fp16 records u and w are also what the forward makes v_new = u - w h of.  The rounding e_u, e_w of a row of theirs is one
+// vector for a whole column of dM and adds up in dg, more so the more the keys resemble one another.  But what it leaves in
+// rowsum(dkk KK) - colsum(dkk KK) is <dv2, e_u> + <dw, e_w> (less <dbv, (I + M) e_u> and the same of w), and in Stage B's -<v_new, dv2>
+// the negative of that: with the same records in both places it cancels.  2-norm error of dg in 1e-4, with dM from dT (from
+// dbv v^T and dbgk k^T: the same) / as here, for independent keys 4.3 / 4.25, behind a SiLU 5.8 / 5.3, behind a ReLU 12.6 / 10.0, around a
+// common direction 8.3 / 7.0; channel-wise gate 5.4 / 5.35, 5.6 / 5.5, 6.65 / 6.3, 8.2 / 8.2.  dbeta: 3.19 / 3.20, 3.8 / 3.8, 5.9 / 5.7, 7.1 /
+// 6.65, and at decays near zero around a common direction 9.2 / 9.5.  By itself, without v_new beside it, this form has up to
+// twice the error of the other in dg.
 //
 // Two CTAs share an SM at d_v = 64 (256 tensor-memory columns, 112 KB): five dependent product groups per chunk are a chain
 // of latencies that one CTA cannot fill.  CTAs are persistent and fetch the next chunk's tiles as theirs fall free, which is late

@@ -235,10 +235,10 @@ scan_kernel(const Problem p) {
 // tests compare them): each half of the contraction from zero, then bracket + first half + second half.  So a pair's results do
 // not depend on how many others are in the call, and heads cut over several GPUs give the bits of the whole.  Starting the
 // accumulator with the bracket instead saved the two additions and gave bits that tcgen05 cannot (us a step, so / as here: 8 columns
-// 0.39 / 0.40, 16 0.53 / 0.51, 32 0.79 / 0.80; fetching R and storing the record between the products pays for the additions).
+// 0.39 / 0.39, 16 0.53 / 0.51, 32 0.79 / 0.79; fetching R and storing the record between the products pays for the additions).
 //
 // Bound by the matrix pipe (17 cycles for a product of 16 x 8 x 16 per SM quarter, so 0.14 us per 8 columns) behind 0.25 us of
-// barrier, operand loads and P's way to registers: 0.40 us a step with 8 columns, 0.51 with 16, 0.80 with 32; tcgen05 took 0.69
+// barrier, operand loads and P's way to registers: 0.39 us a step with 8 columns, 0.51 with 16, 0.79 with 32; tcgen05 took 0.69
 // with 16 (same measure: slope over the number of chunks, L2 cold) and takes 0.83 with 64.  With the fetch behind the products
 // instead of between them 16 columns took 0.62, with four warps of kM = 2 at 32 columns the step is 0.92.
 // ---------------------------------------------------------------------------------------------
@@ -435,9 +435,9 @@ scan_mma_kernel(const Problem p) {
     // products, and between them what the next step needs: the matrix pipe takes some 16 cycles for each
     constexpr int kJ = kW == 32 ? 4 : 8;             // contraction steps whose operand is in registers at a time
     // Contraction step behind which R is fetched and the record stored (8: behind the last).  us for 128 chunks, forward / adjoint,
-    // all behind the last and like this: 8 columns 57 / 59 (and with either in between up to 67 / 63), 16 columns 85 / 85 and 75 / 77,
-    // 32 columns 115 / 115 and 113 / 107.
-    constexpr int kFetch = kW == 8 ? 8 : kW == 16 ? 3 : 5, kStore = kW == 16 ? 5 : 8;
+    // both behind the last and like this: 8 columns 57 / 59 and 57 / 57 (other places up to 67 / 63), 16 columns 85 / 85 and 75 / 77,
+    // 32 columns 115 / 115 and 111 / 107.
+    constexpr int kFetch = kW == 8 ? (ADJOINT ? 1 : 8) : kW == 16 ? 3 : ADJOINT ? 5 : 2, kStore = kW == 16 ? 5 : 8;
     auto store_record = [&]() {
 #pragma unroll
       for (int i = 0; i < kRec; ++i) record(bh * (ADJOINT ? NT : NT + 1) + chunk_of(it), i);
@@ -639,23 +639,23 @@ int launch_scan(const Problem& p, bool adjoint, cudaStream_t st) {
     return ctas <= 2 * sms ? launch_scan_nodelta<16>(p, adjoint, ctas <= sms, st) : launch_scan_nodelta<8>(p, adjoint, false, st);
   }
   // Warp-level products or tcgen05 (the same bits): by the whole problem, since calls on ranges of its pairs run beside one another.
-  // The line is where 16 columns no longer give every CTA an SM of its own.  Beyond it 32 columns are the faster kernel (scan alone, us, 32 / 64 columns, 64 chunks,
-  // d_v = 64: 64 pairs 61 / 75; d_v = 128: 20 59 / 67, 32 60 / 70), but not in a chain, where P is read twice as often (32 pairs, d_v =
-  // 128, forward over 250 chunks 869 / 861, 64 chunks 181 / 179; training step 20 pairs x 32 chunks 220 / 223; d_v = 64, 64 x 32 314 / 318,
-  // 48 x 128 942 / 936).
+  // The line is where 16 columns no longer give every CTA an SM of its own.  Beyond it 32 columns are the shorter scan (alone, us,
+  // 32 / 64 columns, 64 chunks, d_v = 64: 64 pairs 63 / 76; d_v = 128: 20 61 / 66, 32 63 / 70) and in calls that repeat on the same
+  // inputs (32 pairs, d_v = 128, forward over 250 chunks 814 / 825; training step d_v = 64, 64 x 32 311 / 328, 48 x 128 889 / 914), but not
+  // where the inputs change from call to call, since P is read twice as often: the same forward 873 / 857.
   if ((p.V / 16) * p.B * p.H > sms) return launch_scan_wide(p, adjoint, st);
   const int c8 = (p.V / 8) * p.nbh;            // CTAs with 8 columns each
   if (p.cn < p.NT) {
     // A range of the sequences (captured step): chunk kernels of another range run beside the scan, and an SM that a scan CTA sits
-    // on is lost to them.  Few CTAs then count for more than a short step.  Captured step, us, 8 / 32 columns, d_v = 64, pairs x chunks:
-    // 8 x 32 68 / 84, 12 x 32 97 / 95, 12 x 64 155 / 169, 14 x 32 113 / 99, 16 x 32 119 / 102, 24 x 64 283 / 250, 32 x 64 353 / 314; d_v =
-    // 128: 3 x 16 51 / 61, 6 x 32 74 / 86, 7 x 32 93 / 88, 10 x 32 121 / 103, 16 x 32 172 / 133 (channel-wise 207 / 173; 64
-    // columns, left out here while their bits differed, 161).
+    // on is lost to them.  Few CTAs then count for more than a short step.  Captured step, us, 8 / 32 / 64 columns, d_v = 64, pairs x
+    // chunks: 8 x 32 66 / 86 / 90, 12 x 32 98 / 96 / 107, 12 x 64 154 / 168 / 174, 14 x 32 115 / 100 / 113, 16 x 32 126 / 105 / 117, 24 x 64 277 /
+    // 254 / 276, 32 x 64 351 / 317 / 344; d_v = 128: 3 x 16 50 / 60 / 70, 6 x 32 75 / 87 / 96, 7 x 32 94 / 88 / 97, 10 x 32 120 / 102 / 111, 16 x 32
+    // 171 / 133 / 138; the same with the channel-wise gate 207 / 174 / 161: its chunk kernels would be better off with 64, which this
+    // rule has not been fitted to (64 columns were out of the question here while their bits differed).
     return 3 * c8 <= 2 * sms ? launch_scan_few<8>(p, adjoint, st) : launch_scan_few<32>(p, adjoint, st);
   }
-  // A whole sequence: the fewest columns with which every CTA has an SM of its own.  Chain of a step, us, 8 / 16 columns (16 or 64 on
-  // tcgen05 before), d_v = 64: 16 x 32 120 / 137 (128); 18 x 64 211 / 228 (254); 32 x 32 207 / 191 (205); d_v = 128: 9 x 64 196 / 210 (227);
-  // 18 x 32 171 / 152 (163).
+  // A whole sequence: the fewest columns with which every CTA has an SM of its own.  Chain of a step, us, 8 / 16 / 32 columns, d_v = 64:
+  // 16 x 32 118 / 121 / 138; 18 x 64 210 / 226 / 261; 32 x 32 208 / 188 / 207; d_v = 128: 9 x 64 170 / 180 / 219; 18 x 32 170 / 152 / 167.
   return c8 <= sms ? launch_scan_few<8>(p, adjoint, st) : launch_scan_few<16>(p, adjoint, st);
 }
 
