@@ -203,14 +203,16 @@ def test_scan_kernels_of_parts_and_of_the_whole_give_the_same_bits(V, H, L):
         assert torch.equal(getattr(part, n), getattr(ref, n)), n
 
 
-@pytest.mark.parametrize("gate,V,parts", [("scalar", 64, (18, 20)), ("scalar", 64, (1, 37)), ("scalar", 128, (9, 10)),
-                                          ("channel", 128, (1, 18)), ("none", 128, (3, 10, 10))])
-def test_a_shard_gives_the_bits_of_the_whole(gate, V, parts):
+@pytest.mark.parametrize("gate,delta,V,parts", [
+    ("scalar", True, 64, (18, 20)), ("scalar", True, 64, (1, 37)), ("scalar", True, 128, (9, 10)), ("channel", True, 128, (1, 18)),
+    ("none", True, 128, (3, 10, 10)), ("scalar", False, 64, (37, 38)), ("channel", False, 128, (1, 37))])
+def test_a_shard_gives_the_bits_of_the_whole(gate, delta, V, parts):
     """Heads cut into problems of their own, as over several GPUs: the whole takes the state scan of 64 columns per CTA, the parts
-    those of 8 and 16 (and one pair the shortest).  Gentle decays, so that the scan's products count; the last chunk is ragged."""
+    those of 8 and 16 (and one pair the shortest); without the delta term 8 and 16 records ahead.  Gentle decays, so that the scan's
+    products count; the last chunk is ragged."""
     K, L, H = 128, 620, sum(parts)
     dev = torch.device("cuda")
-    inp = make_inputs(1, L, H, K, V, gate=gate, delta=True, seed=8, mild=True)
+    inp = make_inputs(1, L, H, K, V, gate=gate, delta=delta, seed=8, mild=True)
     dhT = 0.1 * torch.randn(1, H, K, V, generator=torch.Generator().manual_seed(7))
 
     def run(heads):
