@@ -38,7 +38,7 @@
 // per chunk are 12 k cycles of an SM's share of HBM.  The CTA is persistent and fetches the next chunk's tiles into the ones that
 // are dead once its last products are issued, under the longest CUDA-core phase.  Inside a group the products that the chain waits
 // for are issued first and the rest of the epilogue before lies in the next group's shadow.
-// us at d_v = 128, before (dT, X = dT T^T and dM as three groups, 100 bytes of registers a thread in local memory, all copies
+// us at d_v = 128, before (dT, X = dT T^T and dM as three groups, 88 to 440 bytes a thread of spilled loads, 0 to 48 now, all copies
 // issued by one thread, beta and the per-channel gates read when they were needed) and now: 8192 chunks 920 -> 789; 4096 without the
 // delta term 301 -> 267; 512 with per-channel gates 113 -> 79.
 // Cycles per chunk by clock samples of one CTA (d_v = 128): operand columns and waits for the tiles 4.9 k, group 1 2.5 k, the rest
@@ -225,7 +225,8 @@ bwd_cw_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     float al[16];
     uint32_t kp[8], qp[8];
     // Between two phases: what the compiler has made from the channel (tile addresses) and from k and q (fp32 values) is made anew
-    // in the next one; kept, it goes to local memory (100 bytes a thread), which misses L1 beside 226 KB of shared memory.
+    // in the next one; kept, it goes to local memory, which misses L1 beside 226 KB of shared memory (88 to 440 bytes a thread; 16 to
+    // 48 are left in the instantiations with the delta term or without a WY half, none in Stage B by itself).
     auto anew = [&]() {
       asm volatile("" : "+r"(d));
 #pragma unroll

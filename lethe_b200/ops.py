@@ -173,12 +173,12 @@ def default_cut(gate: int, V: int, NT: int, BH: int, sms: int) -> int:
 
     That unit was a wave of the chunk kernels when they ran one CTA per chunk.  They are persistent now, with one
     to four CTAs per SM, and no wave ends at the cut: the unit is where the cut lies, not a reason for it.  Replay
-    in us, not cut / cut at half / cut here, BH x NT: scalar gate, d_v = 64: 8 x 32 64 / 66 / 67, 16 x 32 105 / 111
-    / 104, 36 x 47 256 / 264 / 261, 32 x 64 309 / 309 / 316, 64 x 64 570 / 554 / 553; d_v = 128: 16 x 32 137 / 141 /
-    134, 64 x 64 723 / 753 / 752; channel-wise, d_v = 64: 16 x 32 140 / 152 / 139; d_v = 128: 16 x 32 169 / 179 /
-    175, 32 x 64 518 / 524 / 524, 64 x 128 1827 / 1863 / 1862; without the delta term, d_v = 128, 64 x 64: scalar
-    461 / 468 / 467, channel-wise 636 / 629 / 629.  So a cut is worth 3 % at best and costs up to 4 %: a whole
-    sequence has the shorter scan step."""
+    in us, not cut / cut at half / cut here, BH x NT: scalar gate, d_v = 64: 8 x 32 66 / 66 / 66, 16 x 32 105 / 111
+    / 105, 36 x 47 255 / 266 / 262, 32 x 64 308 / 310 / 317, 64 x 64 571 / 554 / 554; d_v = 128: 16 x 32 136 / 141 /
+    134, 64 x 64 721 / 752 / 752; channel-wise, d_v = 64: 16 x 32 141 / 151 / 138; d_v = 128: 16 x 32 168 / 180 /
+    175, 32 x 64 518 / 525 / 524, 64 x 128 1825 / 1861 / 1860; without the delta term, d_v = 128, 64 x 64: scalar
+    460 / 467 / 467, channel-wise 636 / 628 / 629.  So a cut is worth 3 % at best and costs up to 4 %: a whole
+    sequence has the shorter scan step.  The rule has not been fitted to that yet."""
     if NT < 8:
         return 0
     per_sm = 2 if (gate != GATE_CHANNEL and V == 64) else 1
@@ -195,7 +195,7 @@ def default_bwd_cuts(gate: int, V: int, delta: bool, NT: int, BH: int, sms: int,
     """Where the backward is cut: at the forward's cut, and - scalar gate, d_v = 64, two units of ``default_cut`` at
     most - once more at half a unit, so that the last main kernel, which has nothing to hide behind, is short.
     At B=2, H=8, L=2048 that cut, placed when Stage B and the WY VJP were kernels of their own, is worth nothing
-    any more: 104 us with it, 102 without.  Elsewhere a second cut at half of the first costs 1 to
+    any more: 105 us with it, 103 without.  Elsewhere a second cut at half of the first costs 1 to
     9 % (d_v = 128, 512 chunks: 144 -> 153; channel-wise 193 -> 198; 4096 chunks 574 -> 587)."""
     if not cut:
         return ()
