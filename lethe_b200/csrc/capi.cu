@@ -83,6 +83,7 @@ static int fill_problem(const LetheGdnArgs* a, Problem* p, bool backward) {
   if (p->L > d.L || p->L <= d.L - kC || (p->Kr != 64 && p->Kr != kK)) return kErrDims;
   if (d.delta == 2 && (p->L != d.L || p->Kr != kK)) return kErrFlags;
   p->V = d.V; p->gate = d.gate; p->delta = d.delta ? 1 : 0;
+  p->Kw = d.delta || d.gate == LETHE_GATE_CHANNEL ? kK : p->Kr;
   if (a->bh_count == 0) {
     if (a->bh_begin != 0) return kErrDims;
     p->bh0 = 0;

@@ -61,22 +61,23 @@ struct ScBars {
 
 struct ScGates { float G[64], beta[64], de[64], gam[64]; };      // cumulative log decay, beta, de, gamma
 
-template <int V>
+// KW: 64 only in kScNoDelta, as in prepare_nodelta_kernel
+template <int V, int KW = kK>
 struct ScSmem {
-  static constexpr int kVT = V * 128;
+  static constexpr int kVT = V * 128, kHT = V * KW * 2;
   static constexpr int oQ = 0;                      // q; then (d_v = 64) dk on its way out
-  static constexpr int oK = oQ + 16384;             // k (directly behind q: early view)
-  static constexpr int oDO = oK + 16384;            // do; with v_new behind it, then dq on its way out, then (d_v = 64) w
+  static constexpr int oK = oQ + KW * 128;             // k (directly behind q: early view)
+  static constexpr int oDO = oK + KW * 128;            // do; with v_new behind it, then dq on its way out, then (d_v = 64) w
   static constexpr int oVN = oDO + kVT;             // v_new
   static constexpr int oV = oVN + kVT;              // v; then dv on its way out
   static constexpr int oT = oV + kVT;               // T; then dkk
   static constexpr int oA = oT + 8192;              // A (directly behind T: early view); then DS
   static constexpr int oH = oA + 8192;              // h; then dw, then dbgk [channel][token]
-  static constexpr int oDH = oH + V * 256;          // dh; then dv2, then dbv [token][V], and (d_v = 64) u behind it
-  static constexpr int oOwn = oDH + V * 256;        // d_v = 128 has room for tiles of their own: dk, w, u
+  static constexpr int oDH = oH + kHT;          // dh; then dv2, then dbv [token][V], and (d_v = 64) u behind it
+  static constexpr int oOwn = oDH + kHT;        // d_v = 128 has room for tiles of their own: dk, w, u
   static constexpr bool kOwn = V == 128;
   static constexpr int oDK = kOwn ? oOwn : oQ, oW = kOwn ? oOwn + 16384 : oDO, oU = kOwn ? oOwn + 32768 : oDH + kVT;
-  static constexpr int oF = kOwn ? oOwn + 49152 : oOwn;
+  static constexpr int oF = kOwn ? oOwn + (KW == kK ? 49152 : 8192) : oOwn;
   // warps that reach one lane quadrant: they split the columns of every epilogue
   static constexpr int kCg = V == 64 ? 2 : 4, kThreads = 128 * kCg;
   // floats: gates of this chunk and the next; t1q [4][64], pq [4][64]; t2p, t3p, ddep, rsp, dbm, rvp [kCg][64] each;
@@ -98,11 +99,12 @@ __device__ __forceinline__ void warp_sums(float* v, int lane, float* out) {
   }
 }
 
-template <int V, ScMode MODE>
-__global__ void __launch_bounds__(ScSmem<V>::kThreads, V == 64 ? 2 : 1)
+template <int V, ScMode MODE, int KW>
+__global__ void __launch_bounds__(ScSmem<V, KW>::kThreads, V == 64 ? 2 : 1)
 bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,
               const __grid_constant__ CUtensorMap mv, const __grid_constant__ CUtensorMap mdo, const __grid_constant__ OutMaps mo) {
-  using S = ScSmem<V>;
+  using S = ScSmem<V, KW>;
+  static_assert(KW == kK || MODE == kScNoDelta, "");
   constexpr bool SB = MODE != kScWy, WY = MODE == kScAll || MODE == kScWy, DELTA = MODE != kScNoDelta;
   constexpr int kCg = S::kCg, kU = 4 / kCg, kThreads = S::kThreads;
   constexpr bool CUT = MODE == kScStageB || MODE == kScWy;
@@ -124,7 +126,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
   CtaCtl ctl{p.status, &bars->abort_flag};
   const int nchunks = p.nbh * p.cn;
   // loads of a chunk (tid 0), by when their destinations fall free in the chunk before
-  constexpr uint32_t kIn0 = 32768u + (WY ? V * 128u : 0u) + (DELTA ? 16384u : 8192u) + (SB ? 2u * V * 128 + V * 256 : V * 128u);
+  constexpr uint32_t kIn0 = KW * 256u + (WY ? V * 128u : 0u) + (DELTA ? 16384u : 8192u) + (SB ? 2u * V * 128 + S::kHT : V * 128u);
   auto load_do = [&](const ChunkAt& a) {               // do, and without the delta term v as v_new
     mbar_expect_tx(&bars->in0, kIn0);
     for (int t = 0; t < V / 64; ++t) {
@@ -137,18 +139,18 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
   };
   auto load_rec = [&](const ChunkAt& a) {              // v_new, h (dv2 where the first half of the call left it)
     if (SB && DELTA) bulk_g2s(tVN, p.saved + p.lay.vn + static_cast<size_t>(a.z) * p.lay.sz_vn, V * 128, &bars->in0);
-    if (SB) bulk_g2s(tH, p.saved + p.lay.hc + static_cast<size_t>(a.z + a.b * p.H + a.h) * p.lay.sz_hc, V * 256, &bars->in0);
+    if (SB) load_image<V, KW>(tH, p.saved + p.lay.hc + static_cast<size_t>(a.z + a.b * p.H + a.h) * p.lay.sz_hc, &bars->in0);
     else bulk_g2s(tDV, p.scratch + p.lay.dv2 + static_cast<size_t>(a.z) * p.lay.sz_dv2, V * 128, &bars->in0);
   };
   auto load_dh = [&](const ChunkAt& a) {
-    mbar_expect_tx(&bars->in1, V * 256u);
-    bulk_g2s(tDH, p.scratch + p.lay.dh + static_cast<size_t>(a.z) * p.lay.sz_dh, V * 256, &bars->in1);
+    mbar_expect_tx(&bars->in1, static_cast<uint32_t>(S::kHT));
+    load_image<V, KW>(tDH, p.scratch + p.lay.dh + static_cast<size_t>(a.z) * p.lay.sz_dh, &bars->in1);
   };
   auto load_b = [&](const ChunkAt& a) {                // [T; A], k
     const unsigned char* ta = p.saved + p.lay.ta + static_cast<size_t>(a.z) * p.lay.sz_ta;
     if (DELTA) bulk_g2s(tT, ta, 16384, &bars->in0);
     else bulk_g2s(tA, ta + 8192, 8192, &bars->in0);
-    for (int t = 0; t < 2; ++t) tma_load_4d(tK + t * 8192, &mk, &bars->in0, t * 64, a.h, a.c * kC, a.b);
+    for (int t = 0; t < KW / 64; ++t) tma_load_4d(tK + t * 8192, &mk, &bars->in0, t * 64, a.h, a.c * kC, a.b);
   };
   auto load_w = [&](const ChunkAt& a) {                // the forward's WY factors
     mbar_expect_tx(&bars->inU, 16384u);
@@ -160,7 +162,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
   };
   // what a chunk will load, to L2: its tiles are free late (before this its loads were waited for, 2 to 5 k cycles per chunk)
   auto prefetch = [&](const ChunkAt& a) {
-    for (int t = 0; t < 2; ++t) {
+    for (int t = 0; t < KW / 64; ++t) {
       tma_prefetch_4d(&mq, t * 64, a.h, a.c * kC, a.b);
       tma_prefetch_4d(&mk, t * 64, a.h, a.c * kC, a.b);
     }
@@ -169,8 +171,8 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       tma_prefetch_4d(&mv, t * 64, a.h, a.c * kC, a.b);
     }
     if (DELTA) bulk_prefetch(p.saved + p.lay.vn + static_cast<size_t>(a.z) * p.lay.sz_vn, V * 128);
-    bulk_prefetch(p.saved + p.lay.hc + static_cast<size_t>(a.z + a.b * p.H + a.h) * p.lay.sz_hc, V * 256);
-    bulk_prefetch(p.scratch + p.lay.dh + static_cast<size_t>(a.z) * p.lay.sz_dh, V * 256);
+    prefetch_image<V, KW>(p.saved + p.lay.hc + static_cast<size_t>(a.z + a.b * p.H + a.h) * p.lay.sz_hc);
+    prefetch_image<V, KW>(p.scratch + p.lay.dh + static_cast<size_t>(a.z) * p.lay.sz_dh);
     if (WY) {
       bulk_prefetch(p.saved + p.lay.w + static_cast<size_t>(a.z) * 16384, 16384);
       bulk_prefetch(p.saved + p.lay.u + static_cast<size_t>(a.z) * p.lay.sz_u, V * 128);
@@ -178,7 +180,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     bulk_prefetch(p.saved + p.lay.ta + static_cast<size_t>(a.z) * p.lay.sz_ta, 16384);
   };
   auto load_q = [&](const ChunkAt& a) {
-    for (int t = 0; t < 2; ++t) tma_load_4d(tQ + t * 8192, &mq, &bars->in0, t * 64, a.h, a.c * kC, a.b);
+    for (int t = 0; t < KW / 64; ++t) tma_load_4d(tQ + t * 8192, &mq, &bars->in0, t * 64, a.h, a.c * kC, a.b);
   };
 
   if (tid == 0) {
@@ -283,7 +285,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     // ---- operands to fp16 in place
     mbar_wait_warp(&bars->in0, ph, ctl, 411);
     if (!p.qk16) {
-      for (int idx = tid; idx < 2 * 64 * 16; idx += kThreads) {      // q and k lie behind each other
+      for (int idx = tid; idx < 2 * KW * 8; idx += kThreads) {       // q and k lie behind each other
         uint4* c = reinterpret_cast<uint4*>(tQ + idx * 16);
         float x[8];
         unpack8_bf16(*c, x);
@@ -319,8 +321,8 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       if (warp == 0) {
         tc_fence_after();
         const uint32_t leader = elect_leader();
-        issue_product_led(leader, cD, Tile{smem_u32(tK) - 8192, 64, false}, Tile{smem_u32(tDH), 128, true}, V, 128, 0u);
-        issue_product_led(leader, cDK, Tile{smem_u32(tDH), 128, false}, Tile{smem_u32(tVN), 64, false}, 64, V, 0u);
+        issue_product_led(leader, cD, Tile{smem_u32(tK) - 8192, 64, false}, Tile{smem_u32(tDH), KW, true}, V, KW, 0u);
+        issue_product_led(leader, cDK, Tile{smem_u32(tDH), KW, false}, Tile{smem_u32(tVN), 64, false}, 64, V, 0u);
         umma_commit_led(leader, &bars->m1);
       } else if (warp == 4) {
         tc_fence_after();
@@ -334,7 +336,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       __syncwarp();
       // in their shadow: <dh, h>, element by element on two images of one layout
       float dhh = 0.f;
-      for (int idx = tid; idx < kK * V / 8; idx += kThreads) {
+      for (int idx = tid; idx < KW * V / 8; idx += kThreads) {
         float x[8], y[8];
         unpack8_f16(*reinterpret_cast<const uint4*>(tDH + idx * 16), x);
         unpack8_f16(*reinterpret_cast<const uint4*>(tH + idx * 16), y);
@@ -408,7 +410,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       if (warp == 0) {
         tc_fence_after();
         const uint32_t leader = elect_leader();
-        issue_product_led(leader, cDQ, Tile{smem_u32(tH), 128, false}, Tile{smem_u32(tDO), 64, false}, 64, V, 0u);
+        issue_product_led(leader, cDQ, Tile{smem_u32(tH), KW, false}, Tile{smem_u32(tDO), 64, false}, 64, V, 0u);
         umma_commit_led(leader, &bars->m2);
         if (tid == 0) {
           if (!DELTA) for (int t = 0; t < V / 64; ++t) tma_store_4d(&mo.dv, oVt + t * 8192, t * 64, a.h, a.c * kC, a.b);
@@ -428,41 +430,43 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       tc_fence_after();
       float t1[16 * kU];
       const f2 scale2 = pack2(p.scale, p.scale);
+      if (KW == kK || quad < 2) {                   // (with 64 channels the other lanes hold none)
 #pragma unroll
-      for (int u = 0; u < kU; ++u) {
-        uint32_t qp[8];
-        float x[16], y[16];
-        read_column(tQ, kU * cg + u, d, 1, qp);
-        tmem_ld16(cDQ + lane_base + c0 + 16 * u, x);
-        tmem_ld16(cQI + lane_base + c0 + 16 * u, y);
-        tmem_ld_wait();
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {               // two tokens
-          const int r = c0 + 16 * u + 2 * j;
-          f2 g;
-          g.u = *reinterpret_cast<const unsigned long long*>(gt.gam + r);
-          const f2 dq = mul2(mul2(scale2, g), pack2(x[2 * j], x[2 * j + 1]));
-          unpack2(mul2(dq, pair_of(qp[j])), t1[16 * u + 2 * j], t1[16 * u + 2 * j + 1]);
-          stage16_two(oQt, r, d, add2(dq, pack2(y[2 * j], y[2 * j + 1])), p.qk16);
-        }
-        if (DELTA) {
-          tmem_ld16(cDWt + lane_base + c0 + 16 * u, x);
+        for (int u = 0; u < kU; ++u) {
+          uint32_t qp[8];
+          float x[16], y[16];
+          read_column(tQ, kU * cg + u, d, 1, qp);
+          tmem_ld16(cDQ + lane_base + c0 + 16 * u, x);
+          tmem_ld16(cQI + lane_base + c0 + 16 * u, y);
           tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 16; ++i) x[i] = -x[i];
-          if (WY) write_column(tDW, kU * cg + u, d, x);
-          if (keep)
+          for (int j = 0; j < 8; ++j) {               // two tokens
+            const int r = c0 + 16 * u + 2 * j;
+            f2 g;
+            g.u = *reinterpret_cast<const unsigned long long*>(gt.gam + r);
+            const f2 dq = mul2(mul2(scale2, g), pack2(x[2 * j], x[2 * j + 1]));
+            unpack2(mul2(dq, pair_of(qp[j])), t1[16 * u + 2 * j], t1[16 * u + 2 * j + 1]);
+            stage16_two(oQt, r, d, add2(dq, pack2(y[2 * j], y[2 * j + 1])), p.qk16);
+          }
+          if (DELTA) {
+            tmem_ld16(cDWt + lane_base + c0 + 16 * u, x);
+            tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 16; ++i) store_f16_sat(dw_g + sw128_off(c0 + 16 * u + i, d, 64), x[i]);
-        }
-        if (MODE == kScStageB) {
-          tmem_ld16(cDK + lane_base + c0 + 16 * u, x);
-          tmem_ld_wait();
+            for (int i = 0; i < 16; ++i) x[i] = -x[i];
+            if (WY) write_column(tDW, kU * cg + u, d, x);
+            if (keep)
 #pragma unroll
-          for (int i = 0; i < 16; ++i) dkb_g[static_cast<size_t>(c0 + 16 * u + i) * kK + d] = x[i];
+              for (int i = 0; i < 16; ++i) store_f16_sat(dw_g + sw128_off(c0 + 16 * u + i, d, 64), x[i]);
+          }
+          if (MODE == kScStageB) {
+            tmem_ld16(cDK + lane_base + c0 + 16 * u, x);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 16; ++i) dkb_g[static_cast<size_t>(c0 + 16 * u + i) * kK + d] = x[i];
+          }
         }
+        warp_sums<16 * kU>(t1, lane, t1q + quad * 64 + c0);
       }
-      warp_sums<16 * kU>(t1, lane, t1q + quad * 64 + c0);
       if (tid == 0 && keep) bulk_wait_read();       // dv2 has left its tile, which becomes dbv
       sync_for_issue();
       if (tid == 96) {                              // (a thread that issues no products: it waits)
@@ -492,7 +496,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) sdde += __shfl_xor_sync(0xffffffffu, sdde, o);
         if (lane == 0) red[12 + warp] = sdde;
-        dG = ((t1q[tid] + t1q[64 + tid]) + (t1q[128 + tid] + t1q[192 + tid])) + over_cg(t2p) - over_cg(t3p);
+        dG = ((t1q[tid] + t1q[64 + tid]) + (KW == kK ? t1q[128 + tid] + t1q[192 + tid] : 0.f)) + over_cg(t2p) - over_cg(t3p);
       }
     } else if (tid < 64) {
       dG = dgb_g[tid];
@@ -660,6 +664,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     __syncwarp();
 #pragma unroll
     for (int u = 0; u < kU; ++u) {
+      if (KW < kK && quad >= 2) break;
       float x[16], y[16];
       if (SB) {
         tmem_ld16(cDK + lane_base + c0 + 16 * u, y);
@@ -726,17 +731,17 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
 }
 
 // ---------------------------------------------------------------------------------------------
-template <int V, ScMode MODE>
+template <int V, ScMode MODE, int KW = kK>
 static int launch_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                     const CUtensorMap& mdo, const OutMaps& mo, cudaStream_t st) {
-  constexpr int smem = ScSmem<V>::kBytes, per_sm = V == 64 ? 2 : 1;
+  constexpr int smem = ScSmem<V, KW>::kBytes, per_sm = V == 64 ? 2 : 1;
   static_assert(per_sm * (smem + 1024) <= 228 * 1024, "CTAs per SM");
   static SmemAttr attr;
-  if (attr.set(bwd_sc_kernel<V, MODE>, smem)) return kErrLaunch;
+  if (attr.set(bwd_sc_kernel<V, MODE, KW>, smem)) return kErrLaunch;
   const int sms = sm_count();
   if (sms <= 0) return kErrDevice;
   const int n = p.nbh * p.cn, most = per_sm * sms;
-  if (launch_dependent(bwd_sc_kernel<V, MODE>, dim3(n < most ? n : most), dim3(ScSmem<V>::kThreads), smem, st, p, mq, mk, mv, mdo, mo) !=
+  if (launch_dependent(bwd_sc_kernel<V, MODE, KW>, dim3(n < most ? n : most), dim3(ScSmem<V, KW>::kThreads), smem, st, p, mq, mk, mv, mdo, mo) !=
       cudaSuccess) return kErrLaunch;
   return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
 }
@@ -750,7 +755,10 @@ static int launch_v(const Problem& p, const CUtensorMap& mq, const CUtensorMap& 
 int launch_bwd_main(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                     const CUtensorMap& mdo, const OutMaps& mo, cudaStream_t st, uint32_t mask) {
   const bool sb = mask & 4u, wy = (mask & 8u) && p.delta;
-  if (!p.delta) return sb ? launch_v<kScNoDelta>(p, mq, mk, mv, mdo, mo, st) : kOk;
+  if (!p.delta && !sb) return kOk;
+  if (p.Kw == 64)
+    return p.V == 64 ? launch_t<64, kScNoDelta, 64>(p, mq, mk, mv, mdo, mo, st) : launch_t<128, kScNoDelta, 64>(p, mq, mk, mv, mdo, mo, st);
+  if (!p.delta) return launch_v<kScNoDelta>(p, mq, mk, mv, mdo, mo, st);
   if (sb && wy) return launch_v<kScAll>(p, mq, mk, mv, mdo, mo, st);
   return sb ? launch_v<kScStageB>(p, mq, mk, mv, mdo, mo, st) : launch_v<kScWy>(p, mq, mk, mv, mdo, mo, st);
 }

@@ -14,9 +14,10 @@ namespace lg {
 
 constexpr int kPreThreads = 256;
 
-template <int V, bool DELTA>
+// KW: 64 only without the delta term and with one decay or none, as in prepare_nodelta_kernel
+template <int V, bool DELTA, int KW = kK>
 struct PreSmem {
-  static constexpr int oW = 16384, oDO = DELTA ? oW + 16384 : V * 256;        // (Rb is staged over q and w)
+  static constexpr int oW = 16384, oDO = DELTA ? oW + 16384 : V * KW * 2;     // (Rb is staged over q and w)
   static constexpr int oA = oDO + V * 128;                                    // A (its 128-row view starts 64 rows early)
   static constexpr int oDV = oA;                                              // then A^T do (64 x V) in its place
   static constexpr int kUsed = DELTA ? oDV + V * 128 : oA, kCtas = DELTA && V == 128 ? 3 : 4;
@@ -24,10 +25,10 @@ struct PreSmem {
 };
 
 // ---------------------------------------------------------------------------------------------
-template <int V, bool DELTA, bool CW>
-__global__ void __launch_bounds__(kPreThreads, PreSmem<V, DELTA>::kCtas)
+template <int V, bool DELTA, bool CW, int KW>
+__global__ void __launch_bounds__(kPreThreads, PreSmem<V, DELTA, KW>::kCtas)
 bwd_pre_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mdo) {
-  using S = PreSmem<V, DELTA>;
+  using S = PreSmem<V, DELTA, KW>;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* sm = align1024(smem_raw);
   unsigned char *QG = sm, *Wt = sm + S::oW, *DO = sm + S::oDO, *At_ = sm + S::oA, *DVL = sm + S::oDV;
@@ -48,14 +49,14 @@ bwd_pre_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
     return a;
   };
   auto load_do = [&](const At& a) {
-    mbar_expect_tx(full, 16384u + V * 128u + (DELTA ? 16384u + 8192u : 0u));
+    mbar_expect_tx(full, KW * 128u + V * 128u + (DELTA ? 16384u + 8192u : 0u));
     for (int i = 0; i < V / 64; ++i) tma_load_4d(DO + i * 8192, &mdo, full, i * 64, a.h, a.c * kC, a.b);
     if (DELTA) bulk_g2s(At_, p.saved + p.lay.ta + static_cast<size_t>(a.z) * p.lay.sz_ta + 8192, 8192, full);
   };
   auto load_q = [&](const At& a) {
     // scale * gamma * q: built below from q, or - channel-wise gate - read as the record the forward's prepare kernel left
     if (CW) bulk_g2s(QG, p.saved + p.lay.qg + static_cast<size_t>(a.z) * 16384, 16384, full);
-    else for (int i = 0; i < 2; ++i) tma_load_4d(QG + i * 8192, &mq, full, i * 64, a.h, a.c * kC, a.b);
+    else for (int i = 0; i < KW / 64; ++i) tma_load_4d(QG + i * 8192, &mq, full, i * 64, a.h, a.c * kC, a.b);
     if (DELTA) bulk_g2s(Wt, p.saved + p.lay.w + static_cast<size_t>(a.z) * p.lay.sz_w, 16384, full);
   };
   auto fetch_gates = [&](const At& a, float* o) {
@@ -65,7 +66,7 @@ bwd_pre_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
   // with; scalar gate without the delta term, d_v = 64, 1692 chunks 22.5 without, 20 with)
   auto prefetch = [&](const At& a) {
     for (int i = 0; i < V / 64; ++i) tma_prefetch_4d(&mdo, i * 64, a.h, a.c * kC, a.b);
-    for (int i = 0; i < 2; ++i) tma_prefetch_4d(&mq, i * 64, a.h, a.c * kC, a.b);
+    for (int i = 0; i < KW / 64; ++i) tma_prefetch_4d(&mq, i * 64, a.h, a.c * kC, a.b);
     if (DELTA) {
       bulk_prefetch(p.saved + p.lay.ta + static_cast<size_t>(a.z) * p.lay.sz_ta + 8192, 8192);
       bulk_prefetch(p.saved + p.lay.w + static_cast<size_t>(a.z) * p.lay.sz_w, 16384);
@@ -107,8 +108,8 @@ bwd_pre_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
     mbar_wait_warp(full, ph, ctl, 401);
     if (!CW) {
       const float* sg = sgs + ph * 64;
-      for (int idx = tid; idx < 64 * 16; idx += kPreThreads) {
-        const int r = idx >> 4, ch = idx & 15;
+      for (int idx = tid; idx < KW * 8; idx += kPreThreads) {
+        const int r = idx / (KW / 8), ch = idx % (KW / 8);
         float x[8];
         unpack8_in(tile_ld_chunk(QG, r, ch, 64), x, p.qk16);
 #pragma unroll
@@ -169,7 +170,7 @@ bwd_pre_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         if (DELTA) *reinterpret_cast<uint4*>(SR + rrec_off(row, cb / 8 + i)) = pack8_f16(d + 8 * i);
-        else tile_st_chunk(SR, row, cb / 8 + i, 128, pack8_f16(d + 8 * i));     // no delta term: plain tile image
+        else if (row < KW) tile_st_chunk(SR, row, cb / 8 + i, KW, pack8_f16(d + 8 * i));     // no delta term: plain tile image
       }
     }
     fence_proxy_async();
@@ -177,7 +178,7 @@ bwd_pre_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
     __syncthreads();
     tc_fence_after();
     if (tid == 0) {
-      bulk_s2g(p.scratch + p.lay.rb + static_cast<size_t>(a.z) * p.lay.sz_rb, SR, V * 256);
+      store_image<V, KW>(p.scratch + p.lay.rb + static_cast<size_t>(a.z) * p.lay.sz_rb, SR);
       bulk_commit();
       bulk_wait_read();
       if (more) load_q(at(n + gridDim.x));
@@ -191,18 +192,18 @@ bwd_pre_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
 // ---------------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------------
-template <int V, bool DELTA, bool CW>
+template <int V, bool DELTA, bool CW, int KW = kK>
 static int launch_pre_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mdo, cudaStream_t st) {
-  using S = PreSmem<V, DELTA>;
+  using S = PreSmem<V, DELTA, KW>;
   static SmemAttr attr;
-  if (attr.set(bwd_pre_kernel<V, DELTA, CW>, S::kBytes)) return kErrLaunch;
+  if (attr.set(bwd_pre_kernel<V, DELTA, CW, KW>, S::kBytes)) return kErrLaunch;
   const int sms = sm_count(), n = p.nbh * p.cn;
   if (sms <= 0) return kErrDevice;
   // Not launched early: its CTAs would hold room that the kernel before, or one of another stream, could use.  Captured step,
   // us, plain / early, scalar gate, d_v = 64: 512 chunks 107 / 116, 2048 335 / 341, 4096 572 / 597; channel-wise, d_v = 128: 512
   // 190 / 199, 8192 2074 / 2046 (early is the better one at the largest, scalar d_v = 128 at 4096 842 / 815 too); one chain: no
   // more than 1 % either way up to 2048 chunks, 4096 596 / 614.
-  bwd_pre_kernel<V, DELTA, CW><<<n < S::kCtas * sms ? n : S::kCtas * sms, kPreThreads, S::kBytes, st>>>(p, mq, mdo);
+  bwd_pre_kernel<V, DELTA, CW, KW><<<n < S::kCtas * sms ? n : S::kCtas * sms, kPreThreads, S::kBytes, st>>>(p, mq, mdo);
   return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
 }
 int launch_bwd_pre(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mdo, cudaStream_t st) {
@@ -210,6 +211,7 @@ int launch_bwd_pre(const Problem& p, const CUtensorMap& mq, const CUtensorMap& m
     if (p.V == 64) return p.delta ? launch_pre_t<64, true, true>(p, mq, mdo, st) : launch_pre_t<64, false, true>(p, mq, mdo, st);
     return p.delta ? launch_pre_t<128, true, true>(p, mq, mdo, st) : launch_pre_t<128, false, true>(p, mq, mdo, st);
   }
+  if (p.Kw == 64) return p.V == 64 ? launch_pre_t<64, false, false, 64>(p, mq, mdo, st) : launch_pre_t<128, false, false, 64>(p, mq, mdo, st);
   if (p.V == 64) return p.delta ? launch_pre_t<64, true, false>(p, mq, mdo, st) : launch_pre_t<64, false, false>(p, mq, mdo, st);
   return p.delta ? launch_pre_t<128, true, false>(p, mq, mdo, st) : launch_pre_t<128, false, false>(p, mq, mdo, st);
 }

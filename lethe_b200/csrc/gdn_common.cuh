@@ -87,6 +87,7 @@ __host__ inline Layout make_layout(const LetheGdnDims& d) {
 struct Problem {
   int B, H, L, NT, V, gate, delta;   // L: tokens of the user tensors (the last chunk may be partly filled)
   int Kr;            // key channels of the user tensors (64 or 128); the kernels work on 128, missing ones are zero
+  int Kw;            // key channels that these calls work on: Kr for one decay or none without the delta term, 128 elsewhere
   int bh0, nbh;      // the (batch, head) pairs this call works on: [bh0, bh0 + nbh) of the B * H pairs
   int c0, cn;        // the chunks of every pair this call works on: [c0, c0 + cn) of the NT chunks
   uint32_t lean;     // 1: intermediates that no later kernel of the call reads are not written; 2: nor what only a backward reads
@@ -237,6 +238,23 @@ __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefe
 // scan_nodelta_kernel with full-line accesses):
 __device__ __forceinline__ uint32_t rrec_off(int row, int col8) {
   return static_cast<uint32_t>((col8 >> 1) * 4096 + row * 32 + (col8 & 1) * 16);
+}
+
+// A record of [128 rows][V] as a tile of its first KW rows in shared memory (atoms of KW rows), and back.
+template <int V, int KW>
+__device__ __forceinline__ void load_image(unsigned char* dst, const unsigned char* rec, uint64_t* bar) {
+  if (KW == kK) bulk_g2s(dst, rec, V * 256, bar);
+  else for (int i = 0; i < V / 64; ++i) bulk_g2s(dst + i * KW * 128, rec + i * 16384, KW * 128, bar);
+}
+template <int V, int KW>
+__device__ __forceinline__ void prefetch_image(const unsigned char* rec) {
+  if (KW == kK) bulk_prefetch(rec, V * 256);
+  else for (int i = 0; i < V / 64; ++i) bulk_prefetch(rec + i * 16384, KW * 128);
+}
+template <int V, int KW>
+__device__ __forceinline__ void store_image(unsigned char* rec, const unsigned char* src) {
+  if (KW == kK) bulk_s2g(rec, src, V * 256);
+  else for (int i = 0; i < V / 64; ++i) bulk_s2g(rec + i * 16384, src + i * KW * 128, KW * 128);
 }
 
 // Where the n-th chunk of a call is: record index, and batch, head and chunk in the user's tensors.  One thread works it out

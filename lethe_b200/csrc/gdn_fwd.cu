@@ -64,17 +64,18 @@ __device__ __forceinline__ void prep_gates(const Problem& p, int z, int lane, Pr
 }
 
 // k and q into the 128-row tile [k; q] (tid 0)
+template <int KW = kK>
 __device__ __forceinline__ void prep_load_kq(unsigned char* KQ, const CUtensorMap* mk, const CUtensorMap* mq, uint64_t* bar, const ChunkAt& a) {
-  mbar_expect_tx(bar, 32768u);
-  for (int t = 0; t < 2; ++t) {
+  mbar_expect_tx(bar, KW * 256u);
+  for (int t = 0; t < KW / 64; ++t) {
     tma_load_4d(KQ + t * 16384, mk, bar, t * 64, a.h, a.c * kC, a.b);
     tma_load_4d(KQ + t * 16384 + 8192, mq, bar, t * 64, a.h, a.c * kC, a.b);
   }
 }
 // ... and what a chunk will load to L2, under the products of the chunk before: its tiles are free late
-template <int V>
+template <int V, int KW = kK>
 __device__ __forceinline__ void prep_prefetch(const CUtensorMap* mk, const CUtensorMap* mq, const CUtensorMap* mv, const ChunkAt& a) {
-  for (int t = 0; t < 2; ++t) {
+  for (int t = 0; t < KW / 64; ++t) {
     tma_prefetch_4d(mk, t * 64, a.h, a.c * kC, a.b);
     tma_prefetch_4d(mq, t * 64, a.h, a.c * kC, a.b);
   }
@@ -363,18 +364,22 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
 }
 
 // Without the delta term u = v, and only A and R = kd^T v are left: two independent products, one wait.
-template <int V>
+// KW: key channels of the tensors.  With 64 the other half of every tile, product and record is left out, here and in the kernels
+// behind (what a product of 128 rows leaves in the lanes of the other 64 is not read): SSD, 36 pairs x 47 chunks, d_v = 64, us,
+// 128 / 64: prepare 32 / 18, output 17 / 12, scan input 16 / 13, main 53 / 45, the training step 156 / 135.
+template <int V, int KW>
 struct PrepNdSmem {
-  static constexpr int oA = 32768, oKD = oA + 8192, oV = oKD + 16384;    // R leaves from where kd (d_v = 128: and v) was
+  // R leaves from where kd (and as far as it is longer, v) was
+  static constexpr int oA = KW * 256, oKD = oA + 8192, oV = oKD + KW * 128;
   static constexpr int kUsed = oV + V * 128, kBytes = kUsed + 2 * static_cast<int>(sizeof(PrepGates) + sizeof(ChunkAt)) + static_cast<int>(sizeof(CtaShared)) + 1024;
   static constexpr int kCols = V == 64 ? 128 : 256, kCtas = V == 64 ? 3 : 2;      // q k^T and R side by side in tensor memory
 };
 
-template <int V>
-__global__ void __launch_bounds__(kPrepThreads, PrepNdSmem<V>::kCtas)
+template <int V, int KW>
+__global__ void __launch_bounds__(kPrepThreads, PrepNdSmem<V, KW>::kCtas)
 prepare_nodelta_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,
                        const __grid_constant__ CUtensorMap mv) {
-  using S = PrepNdSmem<V>;
+  using S = PrepNdSmem<V, KW>;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* sm = align1024(smem_raw);
   unsigned char *KQ = sm, *A = sm + S::oA, *KD = sm + S::oKD, *Vt = sm + S::oV;
@@ -406,7 +411,7 @@ prepare_nodelta_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, 
     const ChunkAt a = chunk_at(p, blockIdx.x);
     if (tid == 0) {
       where[0] = a;
-      prep_load_kq(KQ, &mk, &mq, full_kq, a);
+      prep_load_kq<KW>(KQ, &mk, &mq, full_kq, a);
       prep_load_v<V>(Vt, &mv, full_v, a);
     }
     if (warp == 1) {
@@ -424,8 +429,8 @@ prepare_nodelta_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, 
     if (tid == kPrepThreads - 1 && more) where[ph ^ 1u] = chunk_at(p, n + gridDim.x);
 
     mbar_wait_warp(full_kq, ph, ctl, 206);
-    for (int idx = tid; idx < 64 * 16; idx += kPrepThreads) {
-      const int r = idx >> 4, ch = idx & 15;
+    for (int idx = tid; idx < KW * 8; idx += kPrepThreads) {
+      const int r = idx / (KW / 8), ch = idx % (KW / 8);
       float x[8];
       unpack8_in(tile_ld_chunk(KQ, r, ch, 128), x, p.qk16);
       if (!p.qk16) tile_st_chunk(KQ, r, ch, 128, pack8_f16(x));
@@ -443,7 +448,7 @@ prepare_nodelta_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, 
     if (warp == 0) {
       tc_fence_after();
       const uint32_t leader = elect_leader();
-      issue_product_led(leader, tmem, Tile{smem_u32(KQ), 128, false}, Tile{smem_u32(KQ), 128, false}, 64, 128, 0u);
+      issue_product_led(leader, tmem, Tile{smem_u32(KQ), 128, false}, Tile{smem_u32(KQ), 128, false}, 64, KW, 0u);
       issue_product_led(leader, tmem + 64, Tile{smem_u32(KD), 64, true}, Tile{smem_u32(Vt), 64, true}, V, 64, 0u);
       umma_commit_led(leader, mma);
       if (tid == 0 && !p.lean) {
@@ -454,11 +459,11 @@ prepare_nodelta_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, 
       const ChunkAt nx = where[ph ^ 1u];
       prep_fetch_gates(p, nx.b, nx.c, nx.h, lane, gates + (ph ^ 1u));
     } else if (warp == 2 && lane == 0 && more) {
-      prep_prefetch<V>(&mk, &mq, &mv, where[ph ^ 1u]);
+      prep_prefetch<V, KW>(&mk, &mq, &mv, where[ph ^ 1u]);
     }
     __syncwarp();
     wait_products(mma, pm, ctl, 208);
-    if (tid == 0 && more) prep_load_kq(KQ, &mk, &mq, full_kq, where[ph ^ 1u]);
+    if (tid == 0 && more) prep_load_kq<KW>(KQ, &mk, &mq, full_kq, where[ph ^ 1u]);
     if (!p.lean) {
       if (tid == 0) bulk_wait_read();
       __syncthreads();
@@ -478,14 +483,15 @@ prepare_nodelta_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, 
       float d[32];
       tmem_ld32(tmem + 64 + lane_base + cb, d);
       tmem_ld_wait();
+      if (tq < KW)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) tile_st_chunk(KD, tq, cb / 8 + i, 128, pack8_f16(d + 8 * i));
+        for (int i = 0; i < 4; ++i) tile_st_chunk(KD, tq, cb / 8 + i, KW, pack8_f16(d + 8 * i));
     }
     fence_proxy_async();
     tc_fence_before();
     __syncthreads();
     if (tid == 0) {
-      bulk_s2g(p.saved + p.lay.r + static_cast<size_t>(a.z) * p.lay.sz_r, KD, V * 256);
+      store_image<V, KW>(p.saved + p.lay.r + static_cast<size_t>(a.z) * p.lay.sz_r, KD);
       bulk_s2g(p.saved + p.lay.ta + static_cast<size_t>(a.z) * p.lay.sz_ta + 8192, A, 8192);
       bulk_commit();
       bulk_wait_read();
@@ -516,20 +522,21 @@ prepare_nodelta_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, 
 // ---------------------------------------------------------------------------------------------
 constexpr int kOutThreads = 256;
 
-template <int V, bool CW>
+template <int V, bool CW, int KW = kK>
 struct OutSmem {
-  static constexpr int oA = 32768;                   // behind [w; qg]: A (its 128-row view starts 64 rows early)
+  static constexpr int oA = KW > V ? KW * 256 : V * 256;      // behind [w; qg], and o: A (its 128-row view starts 64 rows early)
   static constexpr int oH = oA + 8192;               // state image
-  static constexpr int oU = oH + V * 256;            // u, then v_new
-  static constexpr int kStage = oU + V * 128, kStages = V == 64 || !CW ? 1 : 2, kCtas = V == 64 ? 3 : CW ? 1 : 2;
+  static constexpr int oU = oH + V * KW * 2;         // u, then v_new
+  static constexpr int kStage = oU + V * 128, kStages = V == 64 || !CW ? 1 : 2, kCtas = V == 64 ? (KW == 64 ? 4 : 3) : CW ? 1 : 2;
   static constexpr int kBytes = kStages * kStage + 2 * 256 + static_cast<int>(sizeof(CtaShared)) + 1024;
 };
 
-template <int V, bool DELTA, bool CW>
-__global__ void __launch_bounds__(kOutThreads, OutSmem<V, CW>::kCtas)
+// KW: 64 only without the delta term and with one decay or none, as in prepare_nodelta_kernel
+template <int V, bool DELTA, bool CW, int KW>
+__global__ void __launch_bounds__(kOutThreads, OutSmem<V, CW, KW>::kCtas)
 output_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mv,
               const __grid_constant__ CUtensorMap mo) {
-  using S = OutSmem<V, CW>;
+  using S = OutSmem<V, CW, KW>;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* sm = align1024(smem_raw);
   float* sgs = reinterpret_cast<float*>(sm + S::kStages * S::kStage);      // [2][64] scale gamma (scalar gate)
@@ -550,8 +557,8 @@ output_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
   };
   auto load = [&](const At& a, int s) {              // everything but h (tid 0)
     unsigned char* t = sm + s * S::kStage;
-    mbar_expect_tx(&full[s], 16384u + (DELTA ? 16384u : 0u) + V * 128u + 8192u + V * 256u);
-    for (int i = 0; i < 2; ++i) {
+    mbar_expect_tx(&full[s], KW * 128u + (DELTA ? 16384u : 0u) + V * 128u + 8192u + V * KW * 2u);
+    for (int i = 0; i < KW / 64; ++i) {
       // the query operand: q from the user tensor (scaled below), or - channel-wise gate - the record of
       // scale * gamma * q that the prepare kernel left (two 64-row atoms of 8 KB)
       if (CW) bulk_g2s(t + i * 16384 + 8192, p.saved + p.lay.qg + static_cast<size_t>(a.z) * 16384 + i * 8192, 8192, &full[s]);
@@ -563,20 +570,20 @@ output_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     else for (int i = 0; i < V / 64; ++i) tma_load_4d(t + S::oU + i * 8192, &mv, &full[s], i * 64, a.h, a.c * kC, a.b);    // v_new = v
   };
   auto load_h = [&](const At& a, int s) {
-    bulk_g2s(sm + s * S::kStage + S::oH, p.saved + p.lay.hc + static_cast<size_t>(a.z + a.bh) * p.lay.sz_hc, V * 256, &full[s]);
+    load_image<V, KW>(sm + s * S::kStage + S::oH, p.saved + p.lay.hc + static_cast<size_t>(a.z + a.bh) * p.lay.sz_hc, &full[s]);
   };
   auto fetch_gates = [&](const At& a, float* o) {
     if (p.gate == LETHE_GATE_SCALAR) warp_copy_gates(p, p.g, a.b, a.c, a.h, lane, o);
   };
   auto prefetch = [&](const At& a) {                 // what load and load_h will want, to L2
-    for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < KW / 64; ++i)
       if (!CW) tma_prefetch_4d(&mq, i * 64, a.h, a.c * kC, a.b);
     if (CW) bulk_prefetch(p.saved + p.lay.qg + static_cast<size_t>(a.z) * 16384, 16384);
     if (DELTA) bulk_prefetch(p.saved + p.lay.w + static_cast<size_t>(a.z) * p.lay.sz_w, 16384);
     bulk_prefetch(p.saved + p.lay.ta + static_cast<size_t>(a.z) * p.lay.sz_ta + 8192, 8192);
     if (DELTA) bulk_prefetch(p.saved + p.lay.u + static_cast<size_t>(a.z) * p.lay.sz_u, V * 128);
     else for (int i = 0; i < V / 64; ++i) tma_prefetch_4d(&mv, i * 64, a.h, a.c * kC, a.b);
-    bulk_prefetch(p.saved + p.lay.hc + static_cast<size_t>(a.z + a.bh) * p.lay.sz_hc, V * 256);
+    prefetch_image<V, KW>(p.saved + p.lay.hc + static_cast<size_t>(a.z + a.bh) * p.lay.sz_hc);
   };
 
   const int n0 = blockIdx.x, n1 = n0 + gridDim.x;
@@ -618,8 +625,8 @@ output_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     mbar_wait_warp(&full[s], static_cast<uint32_t>((it / S::kStages) & 1), ctl, 211);
     if (!CW) {
       const float* sg = sgs + g2 * 64;
-      for (int idx = tid; idx < 64 * 16; idx += kOutThreads) {
-        const int r = idx >> 4, ch = idx & 15;
+      for (int idx = tid; idx < KW * 8; idx += kOutThreads) {
+        const int r = idx / (KW / 8), ch = idx % (KW / 8);
         float x[8];
         unpack8_in(tile_ld_chunk(WQ, 64 + r, ch, 128), x, p.qk16);
 #pragma unroll
@@ -639,7 +646,7 @@ output_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     if (warp == 0) {
       tc_fence_after();
       const uint32_t leader = elect_leader();
-      issue_product_led(leader, tmem, Tile{smem_u32(WQ), 128, false}, Tile{smem_u32(HT), 128, true}, V, 128, 0u);
+      issue_product_led(leader, tmem, Tile{smem_u32(WQ), 128, false}, Tile{smem_u32(HT), KW, true}, V, KW, 0u);
       if (!DELTA) issue_product_led(leader, tmem, Tile{smem_u32(At_) - 8192, 64, false}, Tile{smem_u32(VN), 64, true}, V, 64, 1u);
       umma_commit_led(leader, DELTA ? m1 : m2);
       if (S::kStages == 2 && tid == 0 && it > 0 && n + static_cast<int>(gridDim.x) < nchunks) {      // the other stage's results have left it
@@ -735,17 +742,18 @@ static int launch_persistent(Kern kern, SmemAttr& attr, int smem, int ctas, cons
 }
 template <int V>
 static int launch_prepare_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, cudaStream_t st) {
-  static SmemAttr attr[2];
+  static SmemAttr attr[3];
   // Not early for a later part of the sequences of at most two rounds: its CTAs would take the SMs that the scan of the first
   // part starts on.  Captured step, us, plain / early, by chunks of the later part: 224 (d_v = 64) 107.0 / 108.2, 224 (d_v = 128)
   // 143 / 140, 828 281 / 284, 896 328 / 336, 2048 584 / 573.  So the line could lie between 900 and 2000 as well; below it the
   // two differ by less than two captures of the same step do (2 %).
   const int sms = sm_count();
   const bool early = p.c0 == 0 || p.nbh * p.cn > 4 * sms;
-  return p.delta ? launch_persistent(prepare_kernel<V>, attr[0], PrepSmem<V>::kBytes, 2, p, mq, mk, mv, st, early)
-                 : launch_persistent(prepare_nodelta_kernel<V>, attr[1], PrepNdSmem<V>::kBytes, PrepNdSmem<V>::kCtas, p, mq, mk, mv, st, early);
+  if (p.delta) return launch_persistent(prepare_kernel<V>, attr[0], PrepSmem<V>::kBytes, 2, p, mq, mk, mv, st, early);
+  return p.Kw == 64 ? launch_persistent(prepare_nodelta_kernel<V, 64>, attr[2], PrepNdSmem<V, 64>::kBytes, PrepNdSmem<V, 64>::kCtas, p, mq, mk, mv, st, early)
+                    : launch_persistent(prepare_nodelta_kernel<V, kK>, attr[1], PrepNdSmem<V, kK>::kBytes, PrepNdSmem<V, kK>::kCtas, p, mq, mk, mv, st, early);
 }
-template <int V, bool DELTA, bool CW>
+template <int V, bool DELTA, bool CW, int KW = kK>
 static int launch_output_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mv, const CUtensorMap& mo, cudaStream_t st) {
   static SmemAttr attr;
   // A part of the sequences (a captured step that overlaps parts): early CTAs would wait in room that a scan or a chunk kernel
@@ -753,7 +761,7 @@ static int launch_output_t(const Problem& p, const CUtensorMap& mq, const CUtens
   // 335 / 341, 4096 572 / 586; channel-wise: 512 150 / 157 (d_v = 64) and 190 / 191 (128), 8192 2074 / 2057 (early is the better
   // one there).  Without the delta term the kernels are short and the gaps count: 512 59 / 57, 4096 553 / 541 and 727 / 695.
   const bool early = !DELTA || p.cn == p.NT;
-  return launch_persistent(output_kernel<V, DELTA, CW>, attr, OutSmem<V, CW>::kBytes, OutSmem<V, CW>::kCtas, p, mq, mv, mo, st, early);
+  return launch_persistent(output_kernel<V, DELTA, CW, KW>, attr, OutSmem<V, CW, KW>::kBytes, OutSmem<V, CW, KW>::kCtas, p, mq, mv, mo, st, early);
 }
 
 int launch_prepare(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
@@ -766,6 +774,7 @@ static int launch_output_cw(const Problem& p, const CUtensorMap& mq, const CUten
   return p.delta ? launch_output_t<128, true, CW>(p, mq, mv, mo, st) : launch_output_t<128, false, CW>(p, mq, mv, mo, st);
 }
 int launch_output(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mv, const CUtensorMap& mo, cudaStream_t st) {
+  if (p.Kw == 64) return p.V == 64 ? launch_output_t<64, false, false, 64>(p, mq, mv, mo, st) : launch_output_t<128, false, false, 64>(p, mq, mv, mo, st);
   return p.gate == LETHE_GATE_CHANNEL ? launch_output_cw<true>(p, mq, mv, mo, st) : launch_output_cw<false>(p, mq, mv, mo, st);
 }
 

@@ -530,14 +530,14 @@ scan_mma_kernel(const Problem p) {
 // of a record atom, so every access is a full line.  A thread keeps the R of the next
 // kDepth chunks on the way: 16 while two CTAs per SM hold the whole grid, 8 beyond that, where four do (B H = 36, d_v = 64, 47
 // chunks: forward and backward 184 us with 8, 176 with 16; B H = 64, d_v = 128, 64 chunks: 554 us with 8, 603 with 16).
-// R / Rb and the state records are 128-row tile images.
-// Grid: (V / 64 atoms x 4 row blocks, pairs) x 256 threads.
+// R / Rb and the state records are 128-row tile images, of which rows from Kw on are neither read nor written.
+// Grid: (V / 64 atoms x Kw / 32 row blocks, pairs) x 256 threads.
 // ---------------------------------------------------------------------------------------------
 template <bool ADJOINT, int kDepth>
 __global__ void __launch_bounds__(256, kDepth == 16 ? 2 : 4)
 scan_nodelta_kernel(const Problem p) {
-  const int tid = threadIdx.x;
-  const int atom = blockIdx.x >> 2, d = (blockIdx.x & 3) * 32 + (tid >> 3), c8 = tid & 7;
+  const int tid = threadIdx.x, blocks = p.Kw / 32;
+  const int atom = blockIdx.x / blocks, d = (blockIdx.x - atom * blocks) * 32 + (tid >> 3), c8 = tid & 7;
   const int bh = blockIdx.y + p.bh0, V = p.V, NT = p.NT, n = p.cn;
   const bool seg_first = ADJOINT ? (p.c0 + p.cn == NT) : (p.c0 == 0);        // chunk ranges as in scan_kernel
   const bool seg_last = ADJOINT ? (p.c0 == 0) : (p.c0 + p.cn == NT);
@@ -622,7 +622,7 @@ static int launch_scan_few(const Problem& p, bool adjoint, cudaStream_t st) {
 constexpr int kScanAloneBytes = 118000;      // more than half of an SM's memory, as above
 template <int kDepth>
 static int launch_scan_nodelta(const Problem& p, bool adjoint, bool alone, cudaStream_t st) {
-  const dim3 g((p.V / 64) * 4, p.nbh);
+  const dim3 g((p.V / 64) * (p.Kw / 32), p.nbh);
   const int smem = alone && p.cn == p.NT ? kScanAloneBytes : 0;      // as above: one CTA per SM
   static SmemAttr attr[2];
   if (attr[0].set(scan_nodelta_kernel<false, kDepth>, kScanAloneBytes) || attr[1].set(scan_nodelta_kernel<true, kDepth>, kScanAloneBytes)) return kErrLaunch;
@@ -635,7 +635,7 @@ int launch_scan(const Problem& p, bool adjoint, cudaStream_t st) {
   const int sms = sm_count();
   if (sms <= 0) return kErrDevice;
   if (!p.delta) {
-    const int ctas = (p.V / 64) * 4 * p.nbh;
+    const int ctas = (p.V / 64) * (p.Kw / 32) * p.nbh;
     return ctas <= 2 * sms ? launch_scan_nodelta<16>(p, adjoint, ctas <= sms, st) : launch_scan_nodelta<8>(p, adjoint, false, st);
   }
   // Warp-level products or tcgen05 (the same bits): by the whole problem, since calls on ranges of its pairs run beside one another.
