@@ -13,7 +13,7 @@ int launch_prepare_cw(const Problem&, const CUtensorMap&, const CUtensorMap&, co
 int launch_output(const Problem&, const CUtensorMap& mq, const CUtensorMap& mv, const CUtensorMap& mo, cudaStream_t);
 int launch_scan(const Problem&, bool adjoint, cudaStream_t);
 int launch_bwd_pre(const Problem&, const CUtensorMap& mq, const CUtensorMap& mdo, cudaStream_t);
-bool scan_io_serves(const Problem&);
+bool scan_io_serves(const Problem&, bool adjoint);
 int launch_scan_io(const Problem&, bool adjoint, const CUtensorMap& mio, const CUtensorMap& mv, cudaStream_t);
 int launch_bwd_main(const Problem&, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                     const CUtensorMap& mdo, const OutMaps& mo, cudaStream_t, uint32_t mask);
@@ -170,7 +170,7 @@ extern "C" int lethe_gdn_forward(const LetheGdnArgs* a, void* stream) {
   }
   CUtensorMap mo;
   if ((m & 4u) && (e = token_map(&mo, a->o, p, p.V))) return e;
-  if ((m & 6u) == 6u && scan_io_serves(p)) return launch_scan_io(p, false, mo, mv, st);
+  if ((m & 6u) == 6u && scan_io_serves(p, false)) return launch_scan_io(p, false, mo, mv, st);
   if ((m & 2u) && (e = launch_scan(p, false, st))) return e;
   if ((m & 4u) && (e = launch_output(p, mq, mv, mo, st))) return e;
   return kOk;
@@ -190,7 +190,7 @@ extern "C" int lethe_gdn_backward(const LetheGdnArgs* a, void* stream) {
   if ((e = token_map(&mv, a->v, p, p.V))) return e;
   if ((e = token_map(&mdo, a->d_o, p, p.V))) return e;
   uint32_t m = a->kernel_mask ? a->kernel_mask : 15u;
-  if ((m & 3u) == 3u && scan_io_serves(p)) {
+  if ((m & 3u) == 3u && scan_io_serves(p, true)) {
     if ((e = launch_scan_io(p, true, mdo, mv, st))) return e;
     m &= ~3u;
   }

@@ -527,15 +527,27 @@ scan_mma_kernel(const Problem p) {
 // Without the delta term the recurrence is x <- a x + R per element: no product, nothing serial but the
 // chunk order, and the kernel is bound by reading R and writing the state records once.  Every thread
 // owns one 16-byte piece (8 columns) of one row of the state; a warp covers four whole 128-byte rows
-// of a record atom, so every access is a full line.  A thread keeps the R of the next
-// kDepth chunks on the way: 16 while two CTAs per SM hold the whole grid, 8 beyond that, where four do (B H = 36, d_v = 64, 47
-// chunks: forward and backward 184 us with 8, 176 with 16; B H = 64, d_v = 128, 64 chunks: 554 us with 8, 603 with 16).
+// of a record atom, so every access is a full line.  What is on the way from HBM decides the speed: a thread copies the R of
+// the next kDepth chunks to shared memory behind its own back.  (As loads to registers, 16 or 8 of them, a wait for one was a wait for
+// all that shared its scoreboard, six for a warp, and a step took 0.6 us: 36 pairs x 94 and 188 chunks, d_v = 64, 55 and 114 us, now
+// 18 and 40; 64 pairs x 64, d_v = 128, 59, now 46.)  32 slots, one CTA per SM, for whole sequences (40, 48 and 80 pairs x 64, d_v = 128, us, 8 /
+// 16 / 32: 36 / 39 / 33, 46 / 39 / 36, 63 / 62 / 57).  A range of chunks (captured step) has chunk kernels beside it, which need the room:
+// 16 while two CTAs per SM hold the whole grid, 8 beyond (captured step, SSD, 16 pairs x 32, d_v = 128, 8 / 16 / 32 88 / 78 / 84; GLA, 64 pairs x
+// 64, 603 / 613 / 625).
 // R / Rb and the state records are 128-row tile images, of which rows from Kw on are neither read nor written.
 // Grid: (V / 64 atoms x Kw / 32 row blocks, pairs) x 256 threads.
 // ---------------------------------------------------------------------------------------------
+// A ring of kDepth slots of 16 bytes of R and the row's decay per thread, filled by the thread itself.
+template <int kDepth>
+struct ScanNdSmem {
+  static constexpr int kAd = kDepth * 256 * 16, kBytes = kAd + kDepth * 256 * 4;
+};
 template <bool ADJOINT, int kDepth>
-__global__ void __launch_bounds__(256, kDepth == 16 ? 2 : 4)
+__global__ void __launch_bounds__(256)
 scan_nodelta_kernel(const Problem p) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  uint4* ring = reinterpret_cast<uint4*>(smem_raw) + threadIdx.x;
+  float* ring_ad = reinterpret_cast<float*>(smem_raw + ScanNdSmem<kDepth>::kAd) + threadIdx.x;
   const int tid = threadIdx.x, blocks = p.Kw / 32;
   const int atom = blockIdx.x / blocks, d = (blockIdx.x - atom * blocks) * 32 + (tid >> 3), c8 = tid & 7;
   const int bh = blockIdx.y + p.bh0, V = p.V, NT = p.NT, n = p.cn;
@@ -545,12 +557,14 @@ scan_nodelta_kernel(const Problem p) {
   griddep_wait();
   griddep_launch();
   float* carry = reinterpret_cast<float*>(ADJOINT ? p.scratch + p.lay.carry_b : p.saved + p.lay.carry_f);
-  const unsigned char* Rg = ADJOINT ? p.scratch + p.lay.rb : p.saved + p.lay.r;
-  const float* ADg = reinterpret_cast<const float*>(p.saved + p.lay.ad);
-  unsigned char* Xg = ADJOINT ? p.scratch + p.lay.dh : p.saved + p.lay.hc;
   const size_t szx = p.lay.sz_hc;
   const uint32_t off = sw128_chunk(d, atom * 8 + c8, 128);     // this thread's piece inside any 128-row image
-  auto chunk_of = [&](int it) { return ADJOINT ? p.c0 + n - 1 - it : p.c0 + it; };
+  // records of the chunk that the walk starts with, and the way to the next
+  const size_t z0 = static_cast<size_t>(bh) * NT + (ADJOINT ? p.c0 + n - 1 : p.c0);
+  const long long dir = ADJOINT ? -1 : 1;
+  const unsigned char* Rg = (ADJOINT ? p.scratch + p.lay.rb : p.saved + p.lay.r) + z0 * p.lay.sz_r + off;
+  const float* ADg = reinterpret_cast<const float*>(p.saved + p.lay.ad) + z0 * kK + d;
+  unsigned char* X = (ADJOINT ? p.scratch + p.lay.dh : p.saved + p.lay.hc) + (ADJOINT ? z0 : z0 + bh) * szx + off;
 
   float x[8];
   {
@@ -559,33 +573,29 @@ scan_nodelta_kernel(const Problem p) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) x[j] = x0 && d < nrow ? x0[(static_cast<size_t>(bh) * nrow + d) * V + col0 + j] : 0.f;
   }
-  uint4 rb[kDepth];
-  float ab[kDepth];
-  auto load = [&](int j, int it) {
+  auto fetch = [&](int it) {                       // (a group for every step, empty behind the last)
     if (it < n) {
-      const size_t zj = static_cast<size_t>(bh) * NT + chunk_of(it);
-      rb[j] = *reinterpret_cast<const uint4*>(Rg + zj * p.lay.sz_r + off);
-      ab[j] = ADg[zj * kK + d];
+      const int s = it % kDepth;
+      async_copy16(ring + s * 256, Rg + it * dir * static_cast<long long>(p.lay.sz_r));
+      async_copy4(ring_ad + s * 256, ADg + it * dir * kK, true);
     }
+    async_copy_commit();
   };
+#pragma unroll 1
+  for (int it = 0; it < kDepth - 1; ++it) fetch(it);
+#pragma unroll 1
+  for (int it = 0; it < n; ++it, X += dir * static_cast<long long>(szx)) {
+    *reinterpret_cast<uint4*>(X) = pack8_f16(x);
+    async_copy_wait_but<kDepth - 2>();
+    fetch(it + kDepth - 1);                        // into the slot that the step before has read
+    const int s = it % kDepth;
+    const float a = ring_ad[s * 256];
+    float rr[8];
+    unpack8_f16(ring[s * 256], rr);
 #pragma unroll
-  for (int j = 0; j < kDepth; ++j) load(j, j);
-  for (int it0 = 0; it0 < n; it0 += kDepth) {
-#pragma unroll
-    for (int j = 0; j < kDepth; ++j) {
-      if (it0 + j < n) {
-        const size_t zj = static_cast<size_t>(bh) * NT + chunk_of(it0 + j);
-        *reinterpret_cast<uint4*>(Xg + (ADJOINT ? zj : zj + bh) * szx + off) = pack8_f16(x);
-        float rr[8];
-        unpack8_f16(rb[j], rr);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) x[e] = fmaf(ab[j], x[e], rr[e]);
-        load(j, it0 + j + kDepth);
-      }
-    }
+    for (int e = 0; e < 8; ++e) x[e] = fmaf(a, x[e], rr[e]);
   }
-  if (!ADJOINT && seg_last)   // the final state as one more record
-    *reinterpret_cast<uint4*>(Xg + (static_cast<size_t>(bh) * (NT + 1) + NT) * szx + off) = pack8_f16(x);
+  if (!ADJOINT && seg_last) *reinterpret_cast<uint4*>(X) = pack8_f16(x);      // the final state as one more record
   float* xT = seg_last ? (ADJOINT ? p.dh0 : p.hT) : carry;
   const int nrow = seg_last ? p.Kr : kK;
   if (xT && d < nrow) {
@@ -619,13 +629,12 @@ static int launch_scan_few(const Problem& p, bool adjoint, cudaStream_t st) {
   return e == cudaSuccess ? kOk : kErrLaunch;
 }
 
-constexpr int kScanAloneBytes = 118000;      // more than half of an SM's memory, as above
 template <int kDepth>
-static int launch_scan_nodelta(const Problem& p, bool adjoint, bool alone, cudaStream_t st) {
+static int launch_scan_nodelta(const Problem& p, bool adjoint, cudaStream_t st) {
   const dim3 g((p.V / 64) * (p.Kw / 32), p.nbh);
-  const int smem = alone && p.cn == p.NT ? kScanAloneBytes : 0;      // as above: one CTA per SM
+  constexpr int smem = ScanNdSmem<kDepth>::kBytes;
   static SmemAttr attr[2];
-  if (attr[0].set(scan_nodelta_kernel<false, kDepth>, kScanAloneBytes) || attr[1].set(scan_nodelta_kernel<true, kDepth>, kScanAloneBytes)) return kErrLaunch;
+  if (attr[0].set(scan_nodelta_kernel<false, kDepth>, smem) || attr[1].set(scan_nodelta_kernel<true, kDepth>, smem)) return kErrLaunch;
   const cudaError_t e = adjoint ? launch_dependent(scan_nodelta_kernel<true, kDepth>, g, dim3(256), smem, st, p)
                                 : launch_dependent(scan_nodelta_kernel<false, kDepth>, g, dim3(256), smem, st, p);
   return e == cudaSuccess ? kOk : kErrLaunch;
@@ -635,8 +644,9 @@ int launch_scan(const Problem& p, bool adjoint, cudaStream_t st) {
   const int sms = sm_count();
   if (sms <= 0) return kErrDevice;
   if (!p.delta) {
+    if (p.cn == p.NT) return launch_scan_nodelta<32>(p, adjoint, st);
     const int ctas = (p.V / 64) * (p.Kw / 32) * p.nbh;
-    return ctas <= 2 * sms ? launch_scan_nodelta<16>(p, adjoint, ctas <= sms, st) : launch_scan_nodelta<8>(p, adjoint, false, st);
+    return ctas <= 2 * sms ? launch_scan_nodelta<16>(p, adjoint, st) : launch_scan_nodelta<8>(p, adjoint, st);
   }
   // Warp-level products or tcgen05 (the same bits): by the whole problem, since calls on ranges of its pairs run beside one another.
   // The line is where 16 columns no longer give every CTA an SM of its own.  Beyond it 32 columns are the shorter scan (alone, us,

@@ -510,12 +510,17 @@ static int launch_scan_io_t(const Problem& p, const CUtensorMap& mio, const CUte
 
 // Whether a call takes this kernel instead of the two: its records are not for the caller (lean), the whole sequence in one call, and
 // pairs enough.  With the delta term that is where the scan has 64 columns per CTA anyway (launch_scan).  Without it the scan is
-// spread over four times as many CTAs, the others over all SMs, and the line lies at a third of the SMs (64 chunks, us, the two /
-// this one, forward and adjoint, by CTAs here: 38 63 / 78 and 54 / 54, 48 74 / 72 and 59 / 50, 64 83 / 74 and 71 / 49, 96 108 / 79 and
-// 92 / 48, 160 183 / 151 and 161 / 95).  By the whole problem, since calls on ranges of its pairs run beside one another.
-bool scan_io_serves(const Problem& p) {
-  const int sms = sm_count(), ctas = p.V / kIoW * p.B * p.H;
-  return p.gate == LETHE_GATE_CHANNEL && p.lean && p.cn == p.NT && sms > 0 && (p.delta ? 4 * ctas > sms : 3 * ctas > sms);
+// spread over four times as many CTAs, and the others over all SMs.  The adjoint is the faster from a third of the SMs on, the
+// forward where it fills three fifths of them in its last round too (64 chunks, us, the two / this one: forward, evaluation, adjoint, by
+// CTAs here: 48 51 / 50, 51 / 50, 37 / 41; 64 63 / 72, 63 / 61, 50 / 48; 96 92 / 79, 92 / 65, 76 / 48; 128 119 / 88, 119 / 70, 100 / 52;
+// 160 145 / 151, 145 / 128, 122 / 96; 250 chunks, 64 CTAs 229 / 254, 229 / 220, 196 / 166).  By the whole problem, since calls on
+// ranges of its pairs run beside one another.
+bool scan_io_serves(const Problem& p, bool adjoint) {
+  const int sms = sm_count();
+  if (p.gate != LETHE_GATE_CHANNEL || !p.lean || p.cn != p.NT || sms <= 0) return false;
+  const int ctas = p.V / kIoW * p.B * p.H, rounds = (ctas + sms - 1) / sms;
+  if (p.delta) return 4 * ctas > sms;
+  return adjoint ? 3 * ctas > sms : 5 * ctas > 3 * rounds * sms;
 }
 // mio: o (forward) or do (adjoint)
 int launch_scan_io(const Problem& p, bool adjoint, const CUtensorMap& mio, const CUtensorMap& mv, cudaStream_t st) {
