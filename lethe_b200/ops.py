@@ -206,6 +206,28 @@ def default_bwd_cuts(gate: int, V: int, delta: bool, NT: int, BH: int, sms: int,
     return (cut,)
 
 
+def step_is_cut(gate: int, delta: bool, NT: int, BH: int, sms: int) -> bool:
+    """Whether ``GdnStepGraph`` cuts the sequences at all when it is not told.  A cut adds launches and gives up the scan of a whole
+    sequence: without the delta term, and with the channel-wise gate while a CTA of its kernels has one chunk, that costs more than
+    the overlap gives.  Replay in us, cut / not, BH x NT: SSD, d_v = 64, 4 x 32 35 / 27, 16 x 32 56 / 47, 64 x 16 99 / 84, 36 x 47 131 / 127;
+    d_v = 128, 16 x 32 79 / 71, 32 x 64 234 / 223, 64 x 64 448 / 439; GLA 4 x 32 43 / 31, 16 x 32 85 / 77, 64 x 16 147 / 131, d_v = 128 32 x 64
+    320 / 311; KDA 1 x 32 66 / 58, 4 x 32 66 / 60, d_v = 128 16 x 32 173 / 165, 3 x 128 178 / 197; scalar 4 x 32 58 / 55, 16 x 32 103 / 102,
+    8 x 128 188 / 228.  From 4096 chunks on the 2 to 4 % that are left without the delta term are not worth another schedule."""
+    if not delta:
+        return NT * BH >= 4096
+    return gate != GATE_CHANNEL or NT * BH >= 2 * sms
+
+
+def step_is_chain(gate: int, V: int, delta: bool, BH: int, sms: int) -> bool:
+    """Whether one chain of whole calls is the faster captured step: where forward and backward take the scans that have the output,
+    or their input, beside them (``scan_io_serves`` of the library).  Replay in us, overlapped / chain, BH x NT: KDA, d_v = 64, 64 x 16
+    229 / 217, 64 x 64 801 / 766; d_v = 128 32 x 64 515 / 498, 64 x 64 960 / 868; GLA, d_v = 128, 32 x 64 (not this) 311 / 319, 64 x 64 606 / 549."""
+    ctas = V // 64 * BH
+    if gate != GATE_CHANNEL:
+        return False
+    return 4 * ctas > sms if delta else 5 * ctas > 3 * -(-ctas // sms) * sms
+
+
 class GdnStepGraph:
     """Forward + backward of one fixed problem, captured once into a CUDA graph and replayed.
 
@@ -214,10 +236,10 @@ class GdnStepGraph:
     leave idle (a scan occupies V / 64 to V / 8 CTAs per (batch, head) pair), both bitwise
     equal to the plain chain:
 
-    ``pipeline`` (default): only the serial chain of the step - prepare, forward scan, adjoint scan, Stage B
+    ``pipeline`` (default, but where ``step_is_chain``): only the serial chain of the step - prepare, forward scan, adjoint scan, Stage B
     and WY - stays on one stream; the output kernel and the kernel that builds the adjoint scan's input run
     on other streams of the graph beside the scans (the adjoint scan needs neither the outputs nor the
-    forward scan).  ``cut`` (default: ``default_cut``, about half of the chunks, for sequences of at least 8
+    forward scan).  ``cut`` (default: ``default_cut`` where ``step_is_cut``, about half of the chunks, for sequences of at least 8
     chunks; 0 = no cut) splits every sequence into an early and a late segment of
     chunks (``c_range`` of the C ABI): the late segment is prepared under the forward scan of the early one,
     and its Stage B and WY kernels run under the adjoint scan of the early one.  The scans hand their fp32
@@ -244,7 +266,7 @@ class GdnStepGraph:
         ranges = [(bounds[i], bounds[i + 1] - bounds[i]) for i in range(groups)]
         self.groups = groups
         if pipeline is None:
-            pipeline = groups == 1
+            pipeline = groups == 1 and not (cut is None and bwd_cuts is None and self._is_chain(buf, BH, dev))
         self.pipeline = bool(pipeline) and groups == 1
         if cut is None:
             cut = self._default_cut(buf, NT, BH, dev)
@@ -374,7 +396,14 @@ class GdnStepGraph:
     @staticmethod
     def _default_cut(buf, NT: int, BH: int, dev) -> int:
         sms = torch.cuda.get_device_properties(dev).multi_processor_count
+        if not step_is_cut(buf.dims.gate, buf.dims.delta != 0, NT, BH, sms):
+            return 0
         return default_cut(buf.dims.gate, buf.dims.V, NT, BH, sms)
+
+    @staticmethod
+    def _is_chain(buf, BH: int, dev) -> bool:
+        sms = torch.cuda.get_device_properties(dev).multi_processor_count
+        return step_is_chain(buf.dims.gate, buf.dims.V, buf.dims.delta != 0, BH, sms)
 
     @staticmethod
     def _default_bwd_cuts(buf, NT: int, BH: int, dev, cut: int) -> tuple:
