@@ -353,6 +353,10 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
         const int r = d - 64;
         const float de = gt.de[r];
         float t3 = 0.f, dde = 0.f;
+        constexpr int kNv = V / (8 * kCg);          // (all loads ahead of the first store: see output_kernel)
+        uint4 vc[kNv];
+#pragma unroll
+        for (int i = 0; i < kNv; ++i) vc[i] = tile_ld_chunk(tVN, r, cg * kNv + i, 64);
 #pragma unroll
         for (int jj = 0; jj < V / (16 * kCg); ++jj) {
           const int cb = cg * (V / kCg) + jj * 16;
@@ -363,7 +367,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
 #pragma unroll
           for (int q = 0; q < 2; ++q) {
             float vn[8];
-            unpack8_f16(tile_ld_chunk(tVN, r, cb / 8 + q, 64), vn);
+            unpack8_f16(vc[2 * jj + q], vn);
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
               const float kd_dh = de * y[8 * q + e];
@@ -381,6 +385,12 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
         const int r = d;
         const float Gr = gt.G[r];
         float t2 = 0.f;
+        uint4 ac[2 * kU];                           // A[r, s] (holds scale * ratio already)
+#pragma unroll
+        for (int i = 0; i < 2 * kU; ++i) ac[i] = tile_ld_chunk(tA, r, c0 / 8 + i, 64);
+        float e[16 * kU];
+#pragma unroll
+        for (int i = 0; i < 16 * kU; i += 8) ld8(gt.G + c0 + i, e + i);
 #pragma unroll
         for (int u = 0; u < kU; ++u) {
           float x[16];
@@ -390,13 +400,13 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
           for (int q = 0; q < 2; ++q) {
             const int s8 = c0 / 8 + 2 * u + q;
             float av[8], y[8];
-            unpack8_f16(tile_ld_chunk(tA, r, s8, 64), av);       // A[r, s] (holds scale * ratio already)
+            unpack8_f16(ac[2 * u + q], av);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               const int s = s8 * 8 + i;
               const float da = (s <= r) ? x[8 * q + i] : 0.f;
               t2 += da * av[i];
-              y[i] = (s <= r) ? p.scale * __expf(Gr - gt.G[s]) * da : 0.f;
+              y[i] = (s <= r) ? p.scale * __expf(Gr - e[16 * u + 8 * q + i]) * da : 0.f;
             }
             tile_st_chunk(tDS, r, s8, 64, pack8_f16(y));
           }
@@ -438,13 +448,14 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
           read_column(tQ, kU * cg + u, d, 1, qp);
           tmem_ld16(cDQ + lane_base + c0 + 16 * u, x);
           tmem_ld16(cQI + lane_base + c0 + 16 * u, y);
+          f2 g[8];
+#pragma unroll
+          for (int j = 0; j < 8; j += 2) ld_pairs(gt.gam + c0 + 16 * u + 2 * j, g + j);
           tmem_ld_wait();
 #pragma unroll
           for (int j = 0; j < 8; ++j) {               // two tokens
             const int r = c0 + 16 * u + 2 * j;
-            f2 g;
-            g.u = *reinterpret_cast<const unsigned long long*>(gt.gam + r);
-            const f2 dq = mul2(mul2(scale2, g), pack2(x[2 * j], x[2 * j + 1]));
+            const f2 dq = mul2(mul2(scale2, g[j]), pack2(x[2 * j], x[2 * j + 1]));
             unpack2(mul2(dq, pair_of(qp[j])), t1[16 * u + 2 * j], t1[16 * u + 2 * j + 1]);
             stage16_two(oQt, r, d, add2(dq, pack2(y[2 * j], y[2 * j + 1])), p.qk16);
           }
@@ -544,6 +555,11 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
       auto dbv_columns = [&](bool operand, bool result) {
         const int r = d;
         const float be = gt.beta[r];
+        constexpr int kNv = V / (8 * kCg);
+        uint4 vc[kNv];
+        if (result)
+#pragma unroll
+          for (int i = 0; i < kNv; ++i) vc[i] = tile_ld_chunk(tV, r, cg * kNv + i, 64);
 #pragma unroll
         for (int jj = 0; jj < V / (16 * kCg); ++jj) {
           const int cb = cg * (V / kCg) + jj * 16;
@@ -555,7 +571,7 @@ bwd_sc_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
             if (operand) tile_st_chunk(tBV, r, cb / 8 + q, 64, pack8_f16(x + 8 * q));
             if (!result) continue;
             float vv[8];
-            unpack8_bf16(tile_ld_chunk(tV, r, cb / 8 + q, 64), vv);
+            unpack8_bf16(vc[2 * jj + q], vv);
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
               rv += x[8 * q + e] * vv[e];

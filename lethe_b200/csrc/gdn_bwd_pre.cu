@@ -108,13 +108,23 @@ bwd_pre_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
     mbar_wait_warp(full, ph, ctl, 401);
     if (!CW) {
       const float* sg = sgs + ph * 64;
-      for (int idx = tid; idx < KW * 8; idx += kPreThreads) {
-        const int r = idx / (KW / 8), ch = idx % (KW / 8);
-        float x[8];
-        unpack8_in(tile_ld_chunk(QG, r, ch, 64), x, p.qk16);
+      constexpr int kN = KW * 8 / kPreThreads;
+      uint4 c[kN];
+      float f[kN];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) x[i] *= sg[r];
-        tile_st_chunk(QG, r, ch, 64, pack8_f16(x));
+      for (int u = 0; u < kN; ++u) {                 // (all loads ahead of the first store: see output_kernel)
+        const int idx = tid + u * kPreThreads, r = idx / (KW / 8);
+        c[u] = tile_ld_chunk(QG, r, idx % (KW / 8), 64);
+        f[u] = sg[r];
+      }
+#pragma unroll
+      for (int u = 0; u < kN; ++u) {
+        const int idx = tid + u * kPreThreads, r = idx / (KW / 8);
+        float x[8];
+        unpack8_in(c[u], x, p.qk16);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] *= f[u];
+        tile_st_chunk(QG, r, idx % (KW / 8), 64, pack8_f16(x));
       }
     }
     for (int idx = tid; idx < 64 * (V / 8); idx += kPreThreads) {

@@ -97,13 +97,23 @@ __device__ __forceinline__ void prep_to_f16(unsigned char* t, int bytes, int tid
 }
 // kd = k exp(G_last - G), a 64-row tile
 __device__ __forceinline__ void prep_kd(unsigned char* KD, const unsigned char* KQ, const float* dec, int tid) {
-  for (int idx = tid; idx < 64 * 16; idx += kPrepThreads) {
-    const int r = idx >> 4, ch = idx & 15;
-    float x[8];
-    unpack8_f16(tile_ld_chunk(KQ, r, ch, 128), x);
+  constexpr int kN = 64 * 16 / kPrepThreads;
+  uint4 c[kN];
+  float f[kN];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) x[i] *= dec[r];
-    tile_st_chunk(KD, r, ch, 64, pack8_f16(x));
+  for (int u = 0; u < kN; ++u) {                  // (all loads ahead of the first store: see output_kernel)
+    const int idx = tid + u * kPrepThreads;
+    c[u] = tile_ld_chunk(KQ, idx >> 4, idx & 15, 128);
+    f[u] = dec[idx >> 4];
+  }
+#pragma unroll
+  for (int u = 0; u < kN; ++u) {
+    const int idx = tid + u * kPrepThreads;
+    float x[8];
+    unpack8_f16(c[u], x);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] *= f[u];
+    tile_st_chunk(KD, idx >> 4, idx & 15, 64, pack8_f16(x));
   }
 }
 // 32 columns (from 32 half) of row r of a product, times the decay between the tokens and `f`; zero from column `end` on.
@@ -247,19 +257,24 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
       prep_to_f16(Vt, V * 128, tid);
     }
     __syncthreads();
+    {
+      const int ch = tid & 7, r0 = tid >> 3;
+      float bg[8], be[8];
+      ld8(gt.bg + ch * 8, bg);
+      ld8(gt.beta + ch * 8, be);
+      const uint4 c[2] = {tile_ld_chunk(TA, r0, ch, 128), tile_ld_chunk(TA, r0 + kPrepThreads / 8, ch, 128)};
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int idx = tid + u * kPrepThreads, r = idx >> 3, ch = idx & 7;
-      float t[8], x[8], b[8];
-      unpack8_f16(tile_ld_chunk(TA, r, ch, 128), t);
-      ld8(gt.bg + ch * 8, b);
+      for (int u = 0; u < 2; ++u) {
+        const int r = r0 + u * (kPrepThreads / 8);
+        float t[8], x[8];
+        unpack8_f16(c[u], t);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) x[i] = t[i] * b[i];
-      ld8(gt.beta + ch * 8, b);
-      tile_st_chunk(W, r, ch, 128, pack8_f16(x));
+        for (int i = 0; i < 8; ++i) x[i] = t[i] * bg[i];
+        tile_st_chunk(W, r, ch, 128, pack8_f16(x));
 #pragma unroll
-      for (int i = 0; i < 8; ++i) x[i] = t[i] * b[i];
-      tile_st_chunk(W, 64 + r, ch, 128, pack8_f16(x));
+        for (int i = 0; i < 8; ++i) x[i] = t[i] * be[i];
+        tile_st_chunk(W, 64 + r, ch, 128, pack8_f16(x));
+      }
     }
     sync_for_issue();
 
@@ -429,17 +444,33 @@ prepare_nodelta_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, 
     if (tid == kPrepThreads - 1 && more) where[ph ^ 1u] = chunk_at(p, n + gridDim.x);
 
     mbar_wait_warp(full_kq, ph, ctl, 206);
-    for (int idx = tid; idx < KW * 8; idx += kPrepThreads) {
-      const int r = idx / (KW / 8), ch = idx % (KW / 8);
-      float x[8];
-      unpack8_in(tile_ld_chunk(KQ, r, ch, 128), x, p.qk16);
-      if (!p.qk16) tile_st_chunk(KQ, r, ch, 128, pack8_f16(x));
+    {
+      constexpr int kAll = KW * 8 / kPrepThreads, kN = V == 64 && KW == kK ? 2 : kAll;      // (three CTAs per SM: registers)
 #pragma unroll
-      for (int i = 0; i < 8; ++i) x[i] *= gt.dec[r];
-      tile_st_chunk(KD, r, ch, 64, pack8_f16(x));
-      if (!p.qk16) {
-        unpack8_bf16(tile_ld_chunk(KQ, 64 + r, ch, 128), x);
-        tile_st_chunk(KQ, 64 + r, ch, 128, pack8_f16(x));
+      for (int u0 = 0; u0 < kAll; u0 += kN) {
+        uint4 ck[kN], cq[kN];
+        float f[kN];
+#pragma unroll
+        for (int u = 0; u < kN; ++u) {              // (all loads ahead of the first store: see output_kernel)
+          const int idx = tid + (u0 + u) * kPrepThreads, r = idx / (KW / 8), ch = idx % (KW / 8);
+          ck[u] = tile_ld_chunk(KQ, r, ch, 128);
+          cq[u] = tile_ld_chunk(KQ, 64 + r, ch, 128);
+          f[u] = gt.dec[r];
+        }
+#pragma unroll
+        for (int u = 0; u < kN; ++u) {
+          const int idx = tid + (u0 + u) * kPrepThreads, r = idx / (KW / 8), ch = idx % (KW / 8);
+          float x[8];
+          unpack8_in(ck[u], x, p.qk16);
+          if (!p.qk16) tile_st_chunk(KQ, r, ch, 128, pack8_f16(x));
+#pragma unroll
+          for (int i = 0; i < 8; ++i) x[i] *= f[u];
+          tile_st_chunk(KD, r, ch, 64, pack8_f16(x));
+          if (!p.qk16) {
+            unpack8_bf16(cq[u], x);
+            tile_st_chunk(KQ, 64 + r, ch, 128, pack8_f16(x));
+          }
+        }
       }
     }
     mbar_wait_warp(full_v, ph, ctl, 207);
@@ -531,9 +562,11 @@ struct OutSmem {
   static constexpr int kBytes = kStages * kStage + 2 * 256 + static_cast<int>(sizeof(CtaShared)) + 1024;
 };
 
-// KW: 64 only without the delta term and with one decay or none, as in prepare_nodelta_kernel
+// KW: 64 only without the delta term and with one decay or none, as in prepare_nodelta_kernel.  64 registers at d_v = 64, where the
+// memory holds three CTAs per SM: with more of them the next call's first kernel overlaps less (8 pairs x 16 chunks, forward 24.3
+// us, now 21.3).
 template <int V, bool DELTA, bool CW, int KW>
-__global__ void __launch_bounds__(kOutThreads, OutSmem<V, CW, KW>::kCtas)
+__global__ void __launch_bounds__(kOutThreads, V == 64 ? 4 : OutSmem<V, CW, KW>::kCtas)
 output_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mv,
               const __grid_constant__ CUtensorMap mo) {
   using S = OutSmem<V, CW, KW>;
@@ -625,13 +658,23 @@ output_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     mbar_wait_warp(&full[s], static_cast<uint32_t>((it / S::kStages) & 1), ctl, 211);
     if (!CW) {
       const float* sg = sgs + g2 * 64;
-      for (int idx = tid; idx < KW * 8; idx += kOutThreads) {
-        const int r = idx / (KW / 8), ch = idx % (KW / 8);
-        float x[8];
-        unpack8_in(tile_ld_chunk(WQ, 64 + r, ch, 128), x, p.qk16);
+      constexpr int kN = KW * 8 / kOutThreads;
+      uint4 c[kN];
+      float f[kN];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) x[i] *= sg[r];
-        tile_st_chunk(WQ, 64 + r, ch, 128, pack8_f16(x));
+      for (int u = 0; u < kN; ++u) {
+        const int idx = tid + u * kOutThreads, r = idx / (KW / 8);
+        c[u] = tile_ld_chunk(WQ, 64 + r, idx % (KW / 8), 128);
+        f[u] = sg[r];
+      }
+#pragma unroll
+      for (int u = 0; u < kN; ++u) {
+        const int idx = tid + u * kOutThreads, r = idx / (KW / 8);
+        float x[8];
+        unpack8_in(c[u], x, p.qk16);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] *= f[u];
+        tile_st_chunk(WQ, 64 + r, idx % (KW / 8), 128, pack8_f16(x));
       }
     }
     if (!DELTA) {
@@ -661,6 +704,12 @@ output_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
     __syncwarp();
     if (!CW && warp == 1 && more) warp_scaled_gammas(p, lane, sgs + (g2 ^ 1) * 64);
     if (DELTA) {
+      // A store to a swizzled tile keeps every later shared-memory load behind it, whatever the two addresses: loads come first, here
+      // while the products run.
+      uint4 un[V / 16];                              // this thread's pieces of u
+      if (quad < 2)
+#pragma unroll
+        for (int i = 0; i < V / 16; ++i) un[i] = tile_ld_chunk(VN, quad * 32 + lane, half * (V / 16) + i, 64);
       mbar_wait_warp(m1, ph, ctl, 212);
       tc_fence_after();
       if (quad < 2) {                                // v_new, where u was
@@ -674,7 +723,7 @@ output_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             float u8[8];
-            unpack8_f16(tile_ld_chunk(VN, r, cb / 8 + i, 64), u8);
+            unpack8_f16(un[4 * jj + i], u8);
 #pragma unroll
             for (int e = 0; e < 8; ++e) u8[e] -= d[8 * i + e];
             tile_st_chunk(VN, r, cb / 8 + i, 64, pack8_f16(u8));
