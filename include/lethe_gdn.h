@@ -128,9 +128,10 @@ typedef struct LetheGdnArgs {
   /* the backward read.  2 (forward only): not even the latter, no backward can follow.  0: also intermediates that a  */
   /* caller may want to look at (dv2, dw).                                                                             */
   uint32_t lean;
-  /* Forward, LETHE_GATE_CHANNEL only.  l2_eps > 0: q and k are normalised as they are read, x rsqrt(sum x^2 + l2_eps)   */
-  /* per token-head, in fp32 and rounded once to fp16 (what lethe_gdn_l2norm_qk does, without its pass over memory);    */
-  /* q_norm, k_norm (both or neither) take the normalised rows, fp16, for the backward.                                 */
+  /* Forward.  l2_eps > 0: q and k are normalised as they are read, x rsqrt(sum x^2 + l2_eps) per token-head, in fp32   */
+  /* and rounded once to fp16 (what lethe_gdn_l2norm_qk does, without its pass over memory).  q_norm, k_norm take the     */
+  /* normalised rows, fp16, for the backward: both or neither with LETHE_GATE_CHANNEL; otherwise q_norm is needed (the   */
+  /* output kernel reads it) and k_norm is for a backward.                                                                */
   float l2_eps;
   void* q_norm;
   void* k_norm;

@@ -7,7 +7,7 @@
 #include "host_util.h"
 
 namespace lg {
-int launch_prepare(const Problem&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, cudaStream_t);
+int launch_prepare(const Problem&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const NormMaps&, cudaStream_t);
 int launch_prepare_cw(const Problem&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap& mg,
                       const NormMaps&, cudaStream_t);
 int launch_output(const Problem&, const CUtensorMap& mq, const CUtensorMap& mv, const CUtensorMap& mo, cudaStream_t);
@@ -107,10 +107,10 @@ static int fill_problem(const LetheGdnArgs* a, Problem* p, bool backward) {
   p->lean = a->lean;
   if (p->lean > 2u || (backward && p->lean == 2u)) return kErrFlags;
   if (!backward && a->l2_eps != 0.f) {
-    if (!(a->l2_eps > 0.f) || d.gate != LETHE_GATE_CHANNEL || !a->q_norm != !a->k_norm) return kErrFlags;
-    if (a->q_norm && (!aligned16(a->q_norm) || !aligned16(a->k_norm))) return kErrAlign;
+    if (!(a->l2_eps > 0.f) || (d.gate == LETHE_GATE_CHANNEL ? !a->q_norm != !a->k_norm : !a->q_norm)) return kErrFlags;
+    if (!aligned16(a->q_norm) || !aligned16(a->k_norm)) return kErrAlign;
     p->l2_eps = a->l2_eps;
-    p->keep_norm = a->q_norm ? 1 : 0;
+    p->keep_norm = a->k_norm ? 1 : 0;
   }
   p->q = static_cast<const __nv_bfloat16*>(a->q);
   p->k = static_cast<const __nv_bfloat16*>(a->k);
@@ -159,14 +159,19 @@ extern "C" int lethe_gdn_forward(const LetheGdnArgs* a, void* stream) {
   if ((e = token_map(&mk, a->k, p, p.Kr))) return e;
   if ((e = token_map(&mv, a->v, p, p.V))) return e;
   const uint32_t m = a->kernel_mask ? a->kernel_mask : 7u;
+  NormMaps mn;
+  memset(&mn, 0, sizeof(mn));
+  if (p.l2_eps > 0.f && a->q_norm && (e = token_map(&mn.q, a->q_norm, p, p.Kr))) return e;
+  if (p.keep_norm && (e = token_map(&mn.k, a->k_norm, p, p.Kr))) return e;
   if ((m & 1u) && p.gate == LETHE_GATE_CHANNEL) {
     CUtensorMap mg;
-    NormMaps mn;
-    memset(&mn, 0, sizeof(mn));
-    if (p.keep_norm && ((e = token_map(&mn.q, a->q_norm, p, p.Kr)) || (e = token_map(&mn.k, a->k_norm, p, p.Kr)))) return e;
     if ((e = gate_map(&mg, a->g, p)) || (e = launch_prepare_cw(p, mq, mk, mv, mg, mn, st))) return e;
-  } else if ((m & 1u) && (e = launch_prepare(p, mq, mk, mv, st))) {
+  } else if ((m & 1u) && (e = launch_prepare(p, mq, mk, mv, mn, st))) {
     return e;
+  }
+  if (p.l2_eps > 0.f && p.gate != LETHE_GATE_CHANNEL) {      // the output kernel reads the normalised q
+    mq = mn.q;
+    p.qk16 = 1;
   }
   CUtensorMap mo;
   if ((m & 4u) && (e = token_map(&mo, a->o, p, p.V))) return e;

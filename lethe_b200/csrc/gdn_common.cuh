@@ -94,7 +94,7 @@ struct Problem {
   int qk16;          // non-zero: q, k, dq, dk hold fp16 instead of bf16
   float scale;
   int after_scan;    // the same call launched the adjoint scan just before the main kernel
-  float l2_eps;      // > 0: the channel-wise prepare kernel normalises q and k
+  float l2_eps;      // > 0: the prepare kernel normalises q and k (q for the output kernel too, where that reads it)
   int keep_norm;     // ... and stores the normalised rows
   const __nv_bfloat16 *q, *k, *v, *d_o;
   const float *g, *beta, *h0, *dhT;

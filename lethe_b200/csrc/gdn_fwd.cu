@@ -86,6 +86,52 @@ __device__ __forceinline__ void prep_load_v(unsigned char* Vt, const CUtensorMap
   mbar_expect_tx(bar, V * 128u);
   for (int t = 0; t < V / 64; ++t) tma_load_4d(Vt + t * 8192, mv, bar, t * 64, a.h, a.c * kC, a.b);
 }
+// The rows of the tile [k; q] normalised, as lethe_gdn_l2norm_qk does (x rsqrt(sum x^2 + eps) in fp32, one rounding to fp16).  Four lanes
+// have a row; the eight rows of a pass take the same 16-byte piece at a time, so the swizzle keeps them off one another's banks.  A
+// kernel of its own took a launch and another pass over q and k (prefill of 1000 tokens, 8 heads: 26.6 us, now 22.2).
+// kPass: passes whose loads come together, ahead of the first store
+template <int KW = kK, int kPass = 2>
+__device__ __forceinline__ void prep_normalise_rows(unsigned char* KQ, int r0, int part, int f16, float eps) {
+  constexpr int kN = KW / 32;
+  uint4 c[kPass][kN];
+#pragma unroll
+  for (int u = 0; u < kPass; ++u)
+#pragma unroll
+    for (int j = 0; j < kN; ++j) c[u][j] = tile_ld_chunk(KQ, r0 + 8 * u, part + 4 * j, 128);
+#pragma unroll
+  for (int u = 0; u < kPass; ++u) {
+    float x[kN][8], ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < kN; ++j) {
+      unpack8_in(c[u][j], x[j], f16);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) ss = fmaf(x[j][e], x[j][e], ss);
+    }
+    ss += __shfl_xor_sync(0xffffffffu, ss, 8);
+    ss += __shfl_xor_sync(0xffffffffu, ss, 16);
+    const float s = rsqrtf(ss + eps);
+#pragma unroll
+    for (int j = 0; j < kN; ++j) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[j][e] *= s;
+      tile_st_chunk(KQ, r0 + 8 * u, part + 4 * j, 128, pack8_f16(x[j]));
+    }
+  }
+}
+template <int KW = kK, int kPass = 2>
+__device__ __forceinline__ void prep_normalise(unsigned char* KQ, int warp, int lane, int f16, float eps) {
+  const int r0 = warp * 16 + (lane & 7), part = lane >> 3;
+#pragma unroll 1
+  for (int r = 0; r < 16; r += 8 * kPass) prep_normalise_rows<KW, kPass>(KQ, r0 + r, part, f16, eps);
+}
+// ... on their way out: q for the output kernel, both for a backward (tid 0, behind a barrier)
+__device__ __forceinline__ void prep_store_norm(const Problem& p, const NormMaps& mn, const unsigned char* KQ, const ChunkAt& a) {
+  for (int t = 0; t < p.Kr / 64; ++t) {
+    tma_store_4d(&mn.q, KQ + t * 16384 + 8192, t * 64, a.h, a.c * kC, a.b);
+    if (p.keep_norm) tma_store_4d(&mn.k, KQ + t * 16384, t * 64, a.h, a.c * kC, a.b);
+  }
+  bulk_commit();
+}
 // a tile of bf16 to fp16 in place, whatever its shape
 template <int N = kPrepThreads>
 __device__ __forceinline__ void prep_to_f16(unsigned char* t, int bytes, int tid) {      // on N threads
@@ -148,10 +194,11 @@ struct PrepSmem {
   static_assert((kInvMtFloats + kInvScratchFloats) * 4 <= 32768, "scratch of the inverse");
 };
 
-template <int V>
+// NORM: q and k are normalised on the way in (as a branch it cost 1 to 3 % where they are not)
+template <int V, bool NORM>
 __global__ void __launch_bounds__(kPrepThreads, 2)
 prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,
-               const __grid_constant__ CUtensorMap mv) {
+               const __grid_constant__ CUtensorMap mv, const __grid_constant__ NormMaps mn) {
   using S = PrepSmem<V>;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* sm = align1024(smem_raw);
@@ -205,7 +252,8 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
     if (tid == kPrepThreads - 1 && more) where[ph ^ 1u] = chunk_at(p, n + gridDim.x);
 
     mbar_wait_warp(full_kq, ph, ctl, 201);
-    if (!p.qk16) prep_to_f16(KQ, 32768, tid);
+    if (NORM) prep_normalise(KQ, warp, lane, p.qk16, p.l2_eps);
+    else if (!p.qk16) prep_to_f16(KQ, 32768, tid);
     if (tid == 0 && n != static_cast<int>(blockIdx.x)) {
       bulk_wait_read();                              // P and R of the chunk before have left their tiles
       if (V == 128) prep_load_v<V>(Vt, &mv, full_v, a);
@@ -213,6 +261,10 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
     sync_for_issue();
 
     // ---- product 1: [KK; QK] = [k; q] k^T
+    if (NORM) {
+      if (tid == kPrepThreads - 1) prep_store_norm(p, mn, KQ, a);
+      __syncwarp();
+    }
     if (warp == 0) {
       tc_fence_after();
       const uint32_t leader = elect_leader();
@@ -316,6 +368,7 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
       }
     }
     if (tid == 0) bulk_wait_read();                  // [T; A] have left their tile
+    if (NORM && tid == kPrepThreads - 1) bulk_wait_read();      // ... and the normalised rows
     sync_for_issue();
 
     // ---- product 3: [P | R] = kd^T [w | u]
@@ -390,10 +443,10 @@ struct PrepNdSmem {
   static constexpr int kCols = V == 64 ? 128 : 256, kCtas = V == 64 ? 3 : 2;      // q k^T and R side by side in tensor memory
 };
 
-template <int V, int KW>
+template <int V, int KW, bool NORM>
 __global__ void __launch_bounds__(kPrepThreads, PrepNdSmem<V, KW>::kCtas)
 prepare_nodelta_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,
-                       const __grid_constant__ CUtensorMap mv) {
+                       const __grid_constant__ CUtensorMap mv, const __grid_constant__ NormMaps mn) {
   using S = PrepNdSmem<V, KW>;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* sm = align1024(smem_raw);
@@ -444,33 +497,24 @@ prepare_nodelta_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, 
     if (tid == kPrepThreads - 1 && more) where[ph ^ 1u] = chunk_at(p, n + gridDim.x);
 
     mbar_wait_warp(full_kq, ph, ctl, 206);
-    {
-      constexpr int kAll = KW * 8 / kPrepThreads, kN = V == 64 && KW == kK ? 2 : kAll;      // (three CTAs per SM: registers)
+    const int f16 = NORM ? 1 : p.qk16;               // the type of the tile from here on
+    if (NORM) {
+      prep_normalise<KW, V == 64 && KW == kK ? 1 : 2>(KQ, warp, lane, p.qk16, p.l2_eps);
+      fence_proxy_async();
+      __syncthreads();
+      if (tid == kPrepThreads - 1) prep_store_norm(p, mn, KQ, a);
+    }
+    for (int idx = tid; idx < KW * 8; idx += kPrepThreads) {
+      const int r = idx / (KW / 8), ch = idx % (KW / 8);
+      float x[8];
+      unpack8_in(tile_ld_chunk(KQ, r, ch, 128), x, f16);
+      if (!f16) tile_st_chunk(KQ, r, ch, 128, pack8_f16(x));
 #pragma unroll
-      for (int u0 = 0; u0 < kAll; u0 += kN) {
-        uint4 ck[kN], cq[kN];
-        float f[kN];
-#pragma unroll
-        for (int u = 0; u < kN; ++u) {              // (all loads ahead of the first store: see output_kernel)
-          const int idx = tid + (u0 + u) * kPrepThreads, r = idx / (KW / 8), ch = idx % (KW / 8);
-          ck[u] = tile_ld_chunk(KQ, r, ch, 128);
-          cq[u] = tile_ld_chunk(KQ, 64 + r, ch, 128);
-          f[u] = gt.dec[r];
-        }
-#pragma unroll
-        for (int u = 0; u < kN; ++u) {
-          const int idx = tid + (u0 + u) * kPrepThreads, r = idx / (KW / 8), ch = idx % (KW / 8);
-          float x[8];
-          unpack8_in(ck[u], x, p.qk16);
-          if (!p.qk16) tile_st_chunk(KQ, r, ch, 128, pack8_f16(x));
-#pragma unroll
-          for (int i = 0; i < 8; ++i) x[i] *= f[u];
-          tile_st_chunk(KD, r, ch, 64, pack8_f16(x));
-          if (!p.qk16) {
-            unpack8_bf16(cq[u], x);
-            tile_st_chunk(KQ, 64 + r, ch, 128, pack8_f16(x));
-          }
-        }
+      for (int i = 0; i < 8; ++i) x[i] *= gt.dec[r];
+      tile_st_chunk(KD, r, ch, 64, pack8_f16(x));
+      if (!f16) {
+        unpack8_bf16(tile_ld_chunk(KQ, 64 + r, ch, 128), x);
+        tile_st_chunk(KQ, 64 + r, ch, 128, pack8_f16(x));
       }
     }
     mbar_wait_warp(full_v, ph, ctl, 207);
@@ -494,6 +538,10 @@ prepare_nodelta_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, 
     }
     __syncwarp();
     wait_products(mma, pm, ctl, 208);
+    if (NORM) {                                      // the normalised rows have left
+      if (tid == kPrepThreads - 1) bulk_wait_read();
+      __syncthreads();
+    }
     if (tid == 0 && more) prep_load_kq<KW>(KQ, &mk, &mq, full_kq, where[ph ^ 1u]);
     if (!p.lean) {
       if (tid == 0) bulk_wait_read();
@@ -778,29 +826,36 @@ output_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __g
 // ---------------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------------
-template <typename Kern>
-static int launch_persistent(Kern kern, SmemAttr& attr, int smem, int ctas, const Problem& p, const CUtensorMap& m0, const CUtensorMap& m1,
-                             const CUtensorMap& m2, cudaStream_t st, bool early = true) {
+template <typename Kern, typename... Maps>
+static int launch_persistent(Kern kern, SmemAttr& attr, int smem, int ctas, cudaStream_t st, bool early, const Problem& p, const Maps&... maps) {
   if (attr.set(kern, smem)) return kErrLaunch;
   const int sms = sm_count(), n = p.nbh * p.cn;
   if (sms <= 0) return kErrDevice;
   const int grid = n < ctas * sms ? n : ctas * sms;
-  if (!early) kern<<<grid, 256, smem, st>>>(p, m0, m1, m2);
-  else if (launch_dependent(kern, dim3(grid), dim3(256), smem, st, p, m0, m1, m2) != cudaSuccess) return kErrLaunch;
+  if (!early) kern<<<grid, 256, smem, st>>>(p, maps...);
+  else if (launch_dependent(kern, dim3(grid), dim3(256), smem, st, p, maps...) != cudaSuccess) return kErrLaunch;
   return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
 }
 template <int V>
-static int launch_prepare_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, cudaStream_t st) {
-  static SmemAttr attr[3];
+static int launch_prepare_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const NormMaps& mn, cudaStream_t st) {
+  static SmemAttr attr[6];
   // Not early for a later part of the sequences of at most two rounds: its CTAs would take the SMs that the scan of the first
   // part starts on.  Captured step, us, plain / early, by chunks of the later part: 224 (d_v = 64) 107.0 / 108.2, 224 (d_v = 128)
   // 143 / 140, 828 281 / 284, 896 328 / 336, 2048 584 / 573.  So the line could lie between 900 and 2000 as well; below it the
   // two differ by less than two captures of the same step do (2 %).
   const int sms = sm_count();
   const bool early = p.c0 == 0 || p.nbh * p.cn > 4 * sms;
-  if (p.delta) return launch_persistent(prepare_kernel<V>, attr[0], PrepSmem<V>::kBytes, 2, p, mq, mk, mv, st, early);
-  return p.Kw == 64 ? launch_persistent(prepare_nodelta_kernel<V, 64>, attr[2], PrepNdSmem<V, 64>::kBytes, PrepNdSmem<V, 64>::kCtas, p, mq, mk, mv, st, early)
-                    : launch_persistent(prepare_nodelta_kernel<V, kK>, attr[1], PrepNdSmem<V, kK>::kBytes, PrepNdSmem<V, kK>::kCtas, p, mq, mk, mv, st, early);
+  const bool norm = p.l2_eps > 0.f;
+  auto delta = [&](auto kern, SmemAttr& at) { return launch_persistent(kern, at, PrepSmem<V>::kBytes, 2, st, early, p, mq, mk, mv, mn); };
+  auto nodelta = [&](auto kern, SmemAttr& at, int smem, int ctas) { return launch_persistent(kern, at, smem, ctas, st, early, p, mq, mk, mv, mn); };
+  if (p.delta) return norm ? delta(prepare_kernel<V, true>, attr[0]) : delta(prepare_kernel<V, false>, attr[1]);
+  using S64 = PrepNdSmem<V, 64>;
+  using S128 = PrepNdSmem<V, kK>;
+  if (p.Kw == 64)
+    return norm ? nodelta(prepare_nodelta_kernel<V, 64, true>, attr[2], S64::kBytes, S64::kCtas)
+                : nodelta(prepare_nodelta_kernel<V, 64, false>, attr[3], S64::kBytes, S64::kCtas);
+  return norm ? nodelta(prepare_nodelta_kernel<V, kK, true>, attr[4], S128::kBytes, S128::kCtas)
+              : nodelta(prepare_nodelta_kernel<V, kK, false>, attr[5], S128::kBytes, S128::kCtas);
 }
 template <int V, bool DELTA, bool CW, int KW = kK>
 static int launch_output_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mv, const CUtensorMap& mo, cudaStream_t st) {
@@ -810,12 +865,12 @@ static int launch_output_t(const Problem& p, const CUtensorMap& mq, const CUtens
   // 335 / 341, 4096 572 / 586; channel-wise: 512 150 / 157 (d_v = 64) and 190 / 191 (128), 8192 2074 / 2057 (early is the better
   // one there).  Without the delta term the kernels are short and the gaps count: 512 59 / 57, 4096 553 / 541 and 727 / 695.
   const bool early = !DELTA || p.cn == p.NT;
-  return launch_persistent(output_kernel<V, DELTA, CW, KW>, attr, OutSmem<V, CW, KW>::kBytes, OutSmem<V, CW, KW>::kCtas, p, mq, mv, mo, st, early);
+  return launch_persistent(output_kernel<V, DELTA, CW, KW>, attr, OutSmem<V, CW, KW>::kBytes, OutSmem<V, CW, KW>::kCtas, st, early, p, mq, mv, mo);
 }
 
-int launch_prepare(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
+int launch_prepare(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const NormMaps& mn,
                    cudaStream_t st) {
-  return p.V == 64 ? launch_prepare_t<64>(p, mq, mk, mv, st) : launch_prepare_t<128>(p, mq, mk, mv, st);
+  return p.V == 64 ? launch_prepare_t<64>(p, mq, mk, mv, mn, st) : launch_prepare_t<128>(p, mq, mk, mv, mn, st);
 }
 template <bool CW>
 static int launch_output_cw(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mv, const CUtensorMap& mo, cudaStream_t st) {

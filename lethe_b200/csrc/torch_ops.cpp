@@ -202,15 +202,17 @@ Forward run_forward(const Problem& p, Operands x, bool keep) {
   Tensor qn, kn;
   if (x.raw) {
     a.l2_eps = kL2Eps;
-    if (keep) {
+    if (keep || p.gate != LETHE_GATE_CHANNEL) {      // (with one decay or none the output kernel reads q, too)
       qn = at::empty(x.q.sizes(), o16.dtype(at::kHalf));
-      kn = at::empty(x.k.sizes(), o16.dtype(at::kHalf));
       a.q_norm = ptr(qn);
+    }
+    if (keep) {
+      kn = at::empty(x.k.sizes(), o16.dtype(at::kHalf));
       a.k_norm = ptr(kn);
     }
   }
   check(lethe_gdn_forward(&a, stream_of(x.q)));
-  if (qn.defined()) {
+  if (keep && qn.defined()) {
     x.q = qn;
     x.k = kn;
     x.raw = false;
@@ -401,12 +403,12 @@ Problem describe(const Tensor& q, const Tensor& k, const Tensor& v, double scale
 
 // q and k as the kernels read them: normalised rows in fp16 (rounded once from fp32), fp16 when both came as fp16,
 // bf16 otherwise
-// `fuse`: the channel-wise prepare kernel may normalise 16-bit rows itself
+// `fuse`: the prepare kernel may normalise 16-bit rows itself
 void prepare_qk(const Problem& p, const Tensor& q, const Tensor& k, Operands* x, bool fuse = false) {
   if (p.l2) {
     Tensor qc, kc;
     const int flags = l2_inputs(q, k, &qc, &kc) | LETHE_L2_NORM_F16;
-    if (fuse && p.gate == LETHE_GATE_CHANNEL && !(flags & LETHE_L2_IN_F32)) {
+    if (fuse && !(flags & LETHE_L2_IN_F32)) {
       x->q = qc;
       x->k = kc;
       x->raw = true;
