@@ -228,6 +228,10 @@ int lethe_gdn_gate_regime(const float* g, const float* b, const float* w, int64_
 int lethe_gdn_gate_spread(const float* dg0, const float* db0, const float* dw0, int64_t rows, int32_t K, int32_t V,
                           float* dg, float* db, float* dw, void* cuda_stream);
 
+/* n values from bf16 to fp32 (to_f32 != 0) or from fp32 to bf16, rounded to nearest even; both pointers on 16-byte     */
+/* boundaries.  No counterpart in the reference.                                                                        */
+int lethe_gdn_convert(const void* src, void* dst, int64_t n, int32_t to_f32, void* cuda_stream);
+
 /* Text for a return code of the calls above or for a device status code. */
 const char* lethe_gdn_strerror(int code);
 

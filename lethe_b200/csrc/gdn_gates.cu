@@ -1,6 +1,8 @@
 // Gates of the six-input surface (reference gdn_layer.py:99-111), where g, b and w come per channel even when a model
 // has one decay and one beta per token-head: the test that finds this out and compacts them, and the way back.  Both
 // are element-wise and bound by HBM: one pass over the gates each.
+#include <cuda_bf16.h>
+
 #include <algorithm>
 
 #include "../../include/lethe_gdn.h"
@@ -111,6 +113,43 @@ gate_spread_kernel(const SpreadProblem p) {
   }
 }
 
+// bf16 to fp32 or back, 8 values a thread
+template <bool TO_F32>
+__global__ void __launch_bounds__(kGateThreads)
+convert_kernel(const void* __restrict__ src, void* __restrict__ dst, long long n) {
+  const long long i = (static_cast<long long>(blockIdx.x) * kGateThreads + threadIdx.x) * 8;
+  if (i >= n) return;
+  const __nv_bfloat16* s16 = static_cast<const __nv_bfloat16*>(src);
+  const float* s32 = static_cast<const float*>(src);
+  __nv_bfloat16* d16 = static_cast<__nv_bfloat16*>(dst);
+  float* d32 = static_cast<float*>(dst);
+  if (i + 8 > n) {
+    for (long long j = i; j < n; ++j) {
+      if (TO_F32) d32[j] = __bfloat162float(s16[j]);
+      else d16[j] = __float2bfloat16_rn(s32[j]);
+    }
+    return;
+  }
+  if (TO_F32) {
+    const uint4 u = *reinterpret_cast<const uint4*>(s16 + i);
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+    float4 o[2];
+    float* f = reinterpret_cast<float*>(o);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      f[2 * j] = __uint_as_float(w[j] << 16);
+      f[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
+    }
+    reinterpret_cast<float4*>(d32 + i)[0] = o[0];
+    reinterpret_cast<float4*>(d32 + i)[1] = o[1];
+  } else {
+    const float4 a = reinterpret_cast<const float4*>(s32 + i)[0], b = reinterpret_cast<const float4*>(s32 + i)[1];
+    const __nv_bfloat162 h[4] = {__floats2bfloat162_rn(a.x, a.y), __floats2bfloat162_rn(a.z, a.w), __floats2bfloat162_rn(b.x, b.y),
+                                 __floats2bfloat162_rn(b.z, b.w)};
+    *reinterpret_cast<uint4*>(d16 + i) = *reinterpret_cast<const uint4*>(h);
+  }
+}
+
 static bool gates_aligned(const void* a) { return (reinterpret_cast<uintptr_t>(a) & 15) == 0; }
 
 }  // namespace lg
@@ -148,5 +187,20 @@ extern "C" int lethe_gdn_gate_spread(const float* dg0, const float* db0, const f
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (V == 64) gate_spread_kernel<64><<<grid, kGateThreads, 0, st>>>(p);
   else gate_spread_kernel<128><<<grid, kGateThreads, 0, st>>>(p);
+  return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
+}
+
+extern "C" int lethe_gdn_convert(const void* src, void* dst, int64_t n, int32_t to_f32, void* stream) {
+  using namespace lg;
+  if (!src || !dst) return kErrNull;
+  if (n <= 0) return kErrDims;
+  if (!gates_aligned(src) || !gates_aligned(dst)) return kErrAlign;
+  DeviceGuard guard(src);
+  if (!guard.ok) return kErrDevice;
+  const int64_t per_cta = kGateThreads * 8, grid = (n + per_cta - 1) / per_cta;
+  if (grid > 0x7fffffff) return kErrDims;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (to_f32) convert_kernel<true><<<static_cast<unsigned>(grid), kGateThreads, 0, st>>>(src, dst, n);
+  else convert_kernel<false><<<static_cast<unsigned>(grid), kGateThreads, 0, st>>>(src, dst, n);
   return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
 }

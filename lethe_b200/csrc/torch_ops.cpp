@@ -132,6 +132,16 @@ constexpr float kL2Eps = 1e-6f;
 
 cudaStream_t stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
 
+// bf16 <-> fp32 by a kernel of the library, where `t` is that in one piece (Tensor::to costs the host three times a launch)
+bool converts(const Tensor& t, at::ScalarType from) {
+  return t.scalar_type() == from && t.is_contiguous() && t.numel() > 0 && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
+}
+Tensor to_f32(const Tensor& t) {
+  Tensor r = at::empty(t.sizes(), t.options().dtype(at::kFloat));
+  check(lethe_gdn_convert(t.data_ptr(), r.data_ptr(), t.numel(), 1, stream_of(t)));
+  return r;
+}
+
 // ---------------------------------------------------------------------------------------------
 // The chunked op.  One description serves every surface: g per row, per channel or absent; beta, or the erase / write
 // gates b, w of the full op; L2 normalisation of q, k inside; and the six-input surface, whose per-channel gates have
@@ -176,14 +186,27 @@ LetheGdnArgs base_args(const Problem& p, const Operands& x, void* saved, size_t 
   return a;
 }
 
+// One allocation for what a call needs for itself; pieces on 1024-byte boundaries.
+struct Slab {
+  size_t bytes = 0;
+  Tensor t;
+  size_t piece(size_t n) {
+    const size_t at = bytes;
+    bytes += (n + 1023) / 1024 * 1024;
+    return at;
+  }
+  void make(const at::TensorOptions& o) { t = workspace(bytes, o); }
+  void* at(size_t offset) const { return static_cast<char*>(t.data_ptr()) + offset; }
+};
+
 struct Forward {
   Tensor o, hT;
   Operands x;
   Tensor saved;
 };
 
-// `keep`: a backward follows, which reads the normalised rows
-Forward run_forward(const Problem& p, Operands x, bool keep) {
+// `keep`: a backward follows, which reads the normalised rows.  `state`: the final state is wanted
+Forward run_forward(const Problem& p, Operands x, bool keep, bool state) {
   Forward f;
   const LetheGdnDims d = p.dims();
   const size_t need = lethe_gdn_saved_bytes(&d);
@@ -194,7 +217,7 @@ Forward run_forward(const Problem& p, Operands x, bool keep) {
   const auto o32 = o16.dtype(at::kFloat);
   f.saved = workspace(need, o16);
   f.o = at::empty({p.B, p.L, p.H, p.V}, o16);
-  f.hT = at::empty({p.B, p.H, p.K, p.V}, o32);
+  if (state) f.hT = at::empty({p.B, p.H, p.K, p.V}, o32);
   LetheGdnArgs a = base_args(p, x, f.saved.data_ptr(), need);
   a.o = ptr(f.o);
   a.hT = ptr<float>(f.hT);
@@ -221,36 +244,60 @@ Forward run_forward(const Problem& p, Operands x, bool keep) {
   return f;
 }
 
+// Tensors for what the caller gets; pointers into `slab` for what is worked on further (or to the tensors).
 struct Grads {
-  Tensor dq, dk, dv, dg, dbeta, dbeta_w, dh0, db, dw;
+  Tensor dq, dk, dv, dg, dbeta, dh0, db, dw;
+  Slab slab;
+  void *p_dq = nullptr, *p_dk = nullptr, *p_dv = nullptr;
+  float *p_dg = nullptr, *p_dbeta = nullptr, *p_dbeta_w = nullptr;
 };
 
-Grads run_backward(const Problem& p, const Operands& x, const Tensor& saved, const Tensor& d_o, const Tensor& dhT,
-                   bool split_beta) {
+// `spread`: gate gradients per row are to be spread over the channels.  `dv32`: dv is to be fp32
+Grads run_backward(const Problem& p, const Operands& x, const Tensor& saved, const Tensor& d_o_in, const Tensor& dhT, bool spread,
+                   bool dv32) {
   Grads r;
   const LetheGdnDims d = p.dims();
-  const auto o16 = x.v.options();
-  const auto o32 = o16.dtype(at::kFloat);
-  const Tensor scratch = workspace(lethe_gdn_scratch_bytes(&d), o16);
-  r.dq = at::empty_like(x.q);
-  r.dk = at::empty_like(x.k);
-  r.dv = at::empty_like(x.v);
-  if (x.g.defined()) r.dg = at::empty_like(x.g);
+  const auto bytes = [](const Tensor& t) { return static_cast<size_t>(t.numel()) * t.element_size(); };
+  const size_t need = lethe_gdn_scratch_bytes(&d), o_bytes = bytes(x.v);
+  const bool cast_do = d_o_in.defined() && converts(d_o_in, at::kFloat), one = x.beta.defined() && p.delta == 1;
+  const bool row_g = spread && p.gate == LETHE_GATE_SCALAR;
+  Slab& s = r.slab;
+  s.piece(need);
+  const size_t at_do = cast_do ? s.piece(o_bytes) : 0, at_dq = p.l2 ? s.piece(bytes(x.q)) : 0, at_dk = p.l2 ? s.piece(bytes(x.k)) : 0;
+  const size_t at_dv = dv32 ? s.piece(o_bytes) : 0, at_dg = row_g ? s.piece(bytes(x.g)) : 0;
+  const size_t at_db = spread && one ? s.piece(bytes(x.beta)) : 0, at_dw = spread && one ? s.piece(bytes(x.beta)) : 0;
+  s.make(x.v.options());
+  auto place = [&](Tensor& t, const Tensor& like, bool inside, size_t at) -> void* {
+    if (inside) return s.at(at);
+    t = at::empty_like(like);
+    return t.data_ptr();
+  };
+  r.p_dq = place(r.dq, x.q, p.l2, at_dq);
+  r.p_dk = place(r.dk, x.k, p.l2, at_dk);
+  r.p_dv = place(r.dv, x.v, dv32, at_dv);
+  if (x.g.defined()) r.p_dg = static_cast<float*>(place(r.dg, x.g, row_g, at_dg));
+  if (one) r.p_dbeta = static_cast<float*>(place(r.dbeta, x.beta, spread, at_db));
+  if (one && spread) r.p_dbeta_w = static_cast<float*>(s.at(at_dw));
   if (x.h0.defined()) r.dh0 = at::empty_like(x.h0);
   LetheGdnArgs a = base_args(p, x, saved.data_ptr(), static_cast<size_t>(saved.numel()));
   if (p.delta == 2) {
     r.db = at::empty_like(x.b);
     r.dw = at::empty_like(x.w);
-  } else if (p.delta == 1) {
-    r.dbeta = at::empty_like(x.beta);
-    if (split_beta) r.dbeta_w = at::empty_like(x.beta);
   }
-  a.d_o = ptr(d_o); a.dhT = ptr<float>(dhT);
-  a.dq = ptr(r.dq); a.dk = ptr(r.dk); a.dv = ptr(r.dv); a.dg = ptr<float>(r.dg); a.dh0 = ptr<float>(r.dh0);
-  a.dbeta = ptr<float>(r.dbeta); a.dbeta_write = ptr<float>(r.dbeta_w);
+  Tensor d_o;
+  if (cast_do) {
+    check(lethe_gdn_convert(d_o_in.data_ptr(), s.at(at_do), d_o_in.numel(), 0, stream_of(x.q)));
+    a.d_o = s.at(at_do);
+  } else {
+    d_o = d_o_in.defined() ? as(d_o_in, at::kBFloat16) : at::zeros({p.B, p.L, p.H, p.V}, x.v.options());
+    a.d_o = ptr(d_o);
+  }
+  a.dhT = ptr<float>(dhT);
+  a.dq = r.p_dq; a.dk = r.p_dk; a.dv = r.p_dv; a.dg = r.p_dg; a.dh0 = ptr<float>(r.dh0);
+  a.dbeta = r.p_dbeta; a.dbeta_write = r.p_dbeta_w;
   a.db_gate = ptr<float>(r.db); a.dw_gate = ptr<float>(r.dw);
-  a.scratch = scratch.data_ptr();
-  a.scratch_bytes = static_cast<size_t>(scratch.numel());
+  a.scratch = s.at(0);
+  a.scratch_bytes = need;
   check(lethe_gdn_backward(&a, stream_of(x.q)));
   return r;
 }
@@ -272,11 +319,12 @@ struct GdnBackward : public torch::autograd::Node {
   }
   variable_list apply(variable_list&& grads) override {
     const bool second = torch::autograd::GradMode::is_enabled() &&
-                        ((grads[0].defined() && grads[0].requires_grad()) || (grads[1].defined() && grads[1].requires_grad()));
+                        ((grads[0].defined() && grads[0].requires_grad()) ||
+                         (grads.size() > 1 && grads[1].defined() && grads[1].requires_grad()));
     variable_list out;
     {
       at::NoGradGuard no_grad;
-      out = first_order(grads[0], grads[1]);
+      out = first_order(grads[0], grads.size() > 1 ? grads[1] : Tensor());
     }
     if (!second) return out;
     for (auto& t : out)
@@ -299,19 +347,23 @@ struct GdnBackward : public torch::autograd::Node {
       Tensor t = workspace(static_cast<size_t>(ws.numel()), ws.options());
       ws = t.copy_(ws);
     }
-    const Tensor d_o = d_o_in.defined() ? as(d_o_in, at::kBFloat16) : at::zeros({p.B, p.L, p.H, p.V}, x.v.options());
     const Tensor dhT = as32(dhT_in);
-    Grads r = run_backward(p, x, ws, d_o, dhT, six && p.delta == 1);
+    const bool rows = six && p.delta != 2, dv32 = dtypes[kV] == at::kFloat && task_should_compute_output(kV);
+    Grads r = run_backward(p, x, ws, d_o_in, dhT, rows, dv32);
     if (p.l2) {     // VJP of x / sqrt(|x|^2 + eps) (the reference gets it by autograd, gdn2_assemble.py:300-312)
       Tensor qc, kc;
       const int flags = l2_inputs(q_in.unpack(self), k_in.unpack(self), &qc, &kc) | LETHE_L2_NORM_F16;
       Tensor dq = at::empty_like(qc), dk = at::empty_like(kc);
-      check(lethe_gdn_l2norm_qk_vjp(qc.data_ptr(), kc.data_ptr(), r.dq.data_ptr(), r.dk.data_ptr(), dq.data_ptr(),
-                                    dk.data_ptr(), qc.numel() / p.K, static_cast<int32_t>(p.K), flags, kL2Eps, stream_of(qc)));
+      check(lethe_gdn_l2norm_qk_vjp(qc.data_ptr(), kc.data_ptr(), r.p_dq, r.p_dk, dq.data_ptr(), dk.data_ptr(),
+                                     qc.numel() / p.K, static_cast<int32_t>(p.K), flags, kL2Eps, stream_of(qc)));
       r.dq = dq;
       r.dk = dk;
     }
-    if (six && p.delta != 2) spread(x, &r);
+    if (rows) spread(x, &r);
+    if (dv32) {
+      r.dv = at::empty(x.v.sizes(), x.v.options().dtype(at::kFloat));
+      check(lethe_gdn_convert(r.p_dv, r.dv.data_ptr(), r.dv.numel(), 1, stream_of(x.v)));
+    }
     const Tensor got[kSlots] = {r.dq, r.dk, r.dv, r.dg, r.dbeta, r.dh0, r.db, r.dw};
     for (int i = 0; i < kSlots; ++i)
       if (got[i].defined() && task_should_compute_output(i)) out[i] = cast_back(got[i], dtypes[i]);
@@ -326,7 +378,7 @@ struct GdnBackward : public torch::autograd::Node {
     if (task_should_compute_output(kB)) db = at::empty({p.B, p.L, p.H, p.K}, o32);
     if (task_should_compute_output(kW)) dw = at::empty({p.B, p.L, p.H, p.V}, o32);
     if (dg.defined() || db.defined() || dw.defined())
-      check(lethe_gdn_gate_spread(ptr<float>(r->dg), ptr<float>(r->dbeta), ptr<float>(r->dbeta_w), p.B * p.L * p.H,
+      check(lethe_gdn_gate_spread(p.gate == LETHE_GATE_SCALAR ? r->p_dg : nullptr, r->p_dbeta, r->p_dbeta_w, p.B * p.L * p.H,
                                   static_cast<int32_t>(p.K), static_cast<int32_t>(p.V), ptr<float>(dg), ptr<float>(db),
                                   ptr<float>(dw), stream_of(x.q)));
     if (p.gate == LETHE_GATE_SCALAR) r->dg = dg;
@@ -347,8 +399,8 @@ std::pair<Tensor, Tensor> apply(const Problem& p, const Tensor (&in)[kSlots], Op
   Forward f;
   {
     at::NoGradGuard no_grad;
-    f = run_forward(p, std::move(x), need);
-    f.o = cast_back(f.o, in[kV].scalar_type());
+    f = run_forward(p, std::move(x), need, !six);
+    f.o = in[kV].scalar_type() == at::kFloat ? to_f32(f.o) : cast_back(f.o, in[kV].scalar_type());
   }
   if (need) {
     std::shared_ptr<GdnBackward> node(new GdnBackward(), torch::autograd::deleteNode);
@@ -371,7 +423,7 @@ std::pair<Tensor, Tensor> apply(const Problem& p, const Tensor (&in)[kSlots], Op
     node->w = SavedVariable(f.x.w, false);
     node->saved = SavedVariable(f.saved, false);
     torch::autograd::set_history(f.o, node);
-    torch::autograd::set_history(f.hT, node);
+    if (f.hT.defined()) torch::autograd::set_history(f.hT, node);
   }
   return {f.o, f.hT};
 }

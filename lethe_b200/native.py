@@ -68,4 +68,6 @@ def _declare(L: ctypes.CDLL) -> None:
     L.lethe_gdn_l2norm_qk_vjp.argtypes = [c_void_p] * 6 + [ctypes.c_int64, ctypes.c_int32, ctypes.c_int32,
                                                           ctypes.c_float, c_void_p]
     L.lethe_gdn_strerror.restype = ctypes.c_char_p
+    L.lethe_gdn_convert.restype = c_int
+    L.lethe_gdn_convert.argtypes = [c_void_p, c_void_p, ctypes.c_int64, ctypes.c_int32, c_void_p]
     L.lethe_gdn_strerror.argtypes = [c_int]
