@@ -200,12 +200,14 @@ int lethe_gdn_decode_step(const LetheGdnDecodeArgs* args, void* cuda_stream);
  *        LETHE_L2_IN_F16  - ... fp16 (at most one of the two);
  *        LETHE_L2_NORM_F16 - the normalised rows qn, kn and their gradients dqn, dkn are fp16 instead
  *                            of bf16 (pair it with LetheGdnArgs::qk_f16 on the forward / backward
- *                            calls: the rows are then rounded once, to the operand type).
+ *                            calls: the rows are then rounded once, to the operand type);
+ *        LETHE_L2_EARLY   - VJP only: the call directly follows lethe_gdn_backward on its stream and q, k are older
+ *                            than that call; they are read before its last kernel has ended.
  * q, k: [rows, D] contiguous; D in {64, 128}; rows = B L H.
  * qn, kn: 16-bit [rows, D], the tensors lethe_gdn_forward / lethe_gdn_backward then read.
  * dqn, dkn: 16-bit [rows, D], the dq / dk lethe_gdn_backward wrote; dq, dk: [rows, D] in the type of
  * q, k (may alias dqn, dkn when both are bf16).  One launch each; every pointer 16-byte aligned. */
-enum { LETHE_L2_IN_F32 = 1, LETHE_L2_NORM_F16 = 2, LETHE_L2_IN_F16 = 4 };
+enum { LETHE_L2_IN_F32 = 1, LETHE_L2_NORM_F16 = 2, LETHE_L2_IN_F16 = 4, LETHE_L2_EARLY = 8 };
 int lethe_gdn_l2norm_qk(const void* q, const void* k, void* qn, void* kn, int64_t rows, int32_t D,
                         int32_t flags, float eps, void* cuda_stream);
 int lethe_gdn_l2norm_qk_vjp(const void* q, const void* k, const void* dqn, const void* dkn, void* dq, void* dk,

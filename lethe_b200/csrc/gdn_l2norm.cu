@@ -122,6 +122,7 @@ l2norm_qk_kernel(const L2Problem p) {
 #pragma unroll
   for (int u = 0; u < kPieces; ++u) load8<IN>(p.x[t], idx[u], x[u]);
   if (BACKWARD) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");      // (x is older than the kernel that makes dy: LETHE_L2_EARLY)
 #pragma unroll
     for (int u = 0; u < kPieces; ++u) load8_16(p.dy[t], idx[u], dy[u], p.norm_f16);
   }
@@ -148,10 +149,13 @@ l2norm_qk_kernel(const L2Problem p) {
 }
 
 template <int LANES, bool BACKWARD>
-void launch_l2norm_t(const L2Problem& p, int in, const dim3& grid, cudaStream_t st) {
-  if (in == kInF32) l2norm_qk_kernel<LANES, kInF32, BACKWARD><<<grid, 256, 0, st>>>(p);
-  else if (in == kInF16) l2norm_qk_kernel<LANES, kInF16, BACKWARD><<<grid, 256, 0, st>>>(p);
-  else l2norm_qk_kernel<LANES, kInBf16, BACKWARD><<<grid, 256, 0, st>>>(p);
+cudaError_t launch_l2norm_t(const L2Problem& p, int in, bool early, const dim3& grid, cudaStream_t st) {
+  auto kern = in == kInF32 ? l2norm_qk_kernel<LANES, kInF32, BACKWARD>
+                           : in == kInF16 ? l2norm_qk_kernel<LANES, kInF16, BACKWARD> : l2norm_qk_kernel<LANES, kInBf16, BACKWARD>;
+  // Behind the main kernel, whose last round leaves SMs idle: launched early, x is there when dy is (KDA training step B2 H8 L2048 189.2 / 187.2 us).
+  if (BACKWARD && early) return launch_dependent(kern, grid, dim3(256), 0, st, p);
+  kern<<<grid, 256, 0, st>>>(p);
+  return cudaGetLastError();
 }
 template <bool BACKWARD>
 int launch_l2norm(const L2Problem& p, int D, int flags, cudaStream_t st) {
@@ -160,9 +164,9 @@ int launch_l2norm(const L2Problem& p, int D, int flags, cudaStream_t st) {
   const long long pieces = p.rows * lanes;
   const int per_cta = 256 * kPieces;
   const dim3 grid(static_cast<unsigned>((pieces + per_cta - 1) / per_cta), 2);
-  if (lanes == 16) launch_l2norm_t<16, BACKWARD>(p, in, grid, st);
-  else launch_l2norm_t<8, BACKWARD>(p, in, grid, st);
-  return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
+  const bool early = (flags & LETHE_L2_EARLY) != 0;
+  const cudaError_t e = lanes == 16 ? launch_l2norm_t<16, BACKWARD>(p, in, early, grid, st) : launch_l2norm_t<8, BACKWARD>(p, in, early, grid, st);
+  return e == cudaSuccess ? kOk : kErrLaunch;
 }
 
 inline bool aligned16(const void* a) { return (reinterpret_cast<uintptr_t>(a) & 15) == 0; }

@@ -348,11 +348,14 @@ struct GdnBackward : public torch::autograd::Node {
       ws = t.copy_(ws);
     }
     const Tensor dhT = as32(dhT_in);
+    // the raw rows come back before the backward is launched: older than its last kernel, unless they are converted below
+    const Tensor q_raw = p.l2 ? q_in.unpack(self) : Tensor(), k_raw = p.l2 ? k_in.unpack(self) : Tensor();
     const bool rows = six && p.delta != 2, dv32 = dtypes[kV] == at::kFloat && task_should_compute_output(kV);
     Grads r = run_backward(p, x, ws, d_o_in, dhT, rows, dv32);
     if (p.l2) {     // VJP of x / sqrt(|x|^2 + eps) (the reference gets it by autograd, gdn2_assemble.py:300-312)
       Tensor qc, kc;
-      const int flags = l2_inputs(q_in.unpack(self), k_in.unpack(self), &qc, &kc) | LETHE_L2_NORM_F16;
+      int flags = l2_inputs(q_raw, k_raw, &qc, &kc) | LETHE_L2_NORM_F16;
+      if (qc.data_ptr() == q_raw.data_ptr() && kc.data_ptr() == k_raw.data_ptr()) flags |= LETHE_L2_EARLY;
       Tensor dq = at::empty_like(qc), dk = at::empty_like(kc);
       check(lethe_gdn_l2norm_qk_vjp(qc.data_ptr(), kc.data_ptr(), r.p_dq, r.p_dk, dq.data_ptr(), dk.data_ptr(),
                                      qc.numel() / p.K, static_cast<int32_t>(p.K), flags, kL2Eps, stream_of(qc)));
