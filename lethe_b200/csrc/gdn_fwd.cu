@@ -228,19 +228,21 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = cs->tmem_slot, lane_base = static_cast<uint32_t>(quad * 32) << 16;
-  griddep_wait();
-  griddep_launch();
   {
-    const ChunkAt a = chunk_at(p, blockIdx.x);
+    const ChunkAt a = chunk_at(p, blockIdx.x);       // (divisions and the maps' way here lie under the kernel before)
     if (tid == 0) {
       where[0] = a;
+      prefetch_map(&mk);
+      prefetch_map(&mq);
+      prefetch_map(&mv);
+    }
+    griddep_wait();
+    griddep_launch();
+    if (tid == 0) {
       prep_load_kq(KQ, &mk, &mq, full_kq, a);
       prep_load_v<V>(Vt, &mv, full_v, a);
     }
-    if (warp == 1) {
-      prep_fetch_gates(p, a.b, a.c, a.h, lane, gates);
-      prep_gates(p, a.z, lane, gates);
-    }
+    if (warp == 1) prep_fetch_gates(p, a.b, a.c, a.h, lane, gates);      // (summed under product 1: waited for here, they held it up)
   }
   __syncthreads();
 
@@ -251,10 +253,11 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
     const PrepGates& gt = gates[ph];
     if (tid == kPrepThreads - 1 && more) where[ph ^ 1u] = chunk_at(p, n + gridDim.x);
 
+    const bool first = n == static_cast<int>(blockIdx.x);
     mbar_wait_warp(full_kq, ph, ctl, 201);
     if (NORM) prep_normalise(KQ, warp, lane, p.qk16, p.l2_eps);
     else if (!p.qk16) prep_to_f16(KQ, 32768, tid);
-    if (tid == 0 && n != static_cast<int>(blockIdx.x)) {
+    if (tid == 0 && !first) {
       bulk_wait_read();                              // P and R of the chunk before have left their tiles
       if (V == 128) prep_load_v<V>(Vt, &mv, full_v, a);
     }
@@ -270,12 +273,16 @@ prepare_kernel(const Problem p, const __grid_constant__ CUtensorMap mq, const __
       const uint32_t leader = elect_leader();
       issue_product_led(leader, tmem, Tile{smem_u32(KQ), 128, false}, Tile{smem_u32(KQ), 128, false}, 64, 128, 0u);
       umma_commit_led(leader, mma);
-    } else if (warp == 1 && more) {
-      const ChunkAt nx = where[ph ^ 1u];
-      prep_fetch_gates(p, nx.b, nx.c, nx.h, lane, gates + (ph ^ 1u));
+    } else if (warp == 1) {
+      if (first) prep_gates(p, a.z, lane, gates);
+      if (more) {
+        const ChunkAt nx = where[ph ^ 1u];
+        prep_fetch_gates(p, nx.b, nx.c, nx.h, lane, gates + (ph ^ 1u));
+      }
     } else if (V == 64 && warp == 2 && lane == 0 && more) {      // (4096 chunks, us, without / with: d_v = 64 135 / 131, 128 143 / 148)
       prep_prefetch<V>(&mk, &mq, &mv, where[ph ^ 1u]);
     }
+    if (first) __syncthreads();                      // the gates
     wait_products(mma, pm, ctl, 202);
     {
       // each half takes 32 of the 64 columns; rows 0-31 (lane quadrant 0 of either operand half) have
