@@ -33,7 +33,32 @@ gate_regime_kernel(const RegimeProblem p) {
   constexpr int R = kGateRowsPerWarp;
   constexpr int WV = V / 32;
   uint32_t bad = 0;
-  for (long long r0 = first * R; r0 < p.rows; r0 += warps * R) {
+  // what a row's values rule out
+  auto rules_out = [&](const float4& g, const float4& b, const float* w, float gf, float bf) {
+    const bool g_one = g.x == gf && g.y == gf && g.z == gf && g.w == gf;
+    bool one = b.x == bf && b.y == bf && b.z == bf && b.w == bf;
+    bool none = b.x == 0.f && b.y == 0.f && b.z == 0.f && b.w == 0.f;
+#pragma unroll
+    for (int e = 0; e < WV; ++e) {
+      one = one && w[e] == bf;
+      none = none && w[e] == 1.f;
+    }
+    return (g_one ? 0u : LETHE_REGIME_SCALAR_GATE) | (one ? 0u : LETHE_REGIME_ONE_BETA) | (none ? 0u : LETHE_REGIME_NO_DELTA);
+  };
+  auto load_w = [&](long long r, float* w) {
+    if (WV == 4) *reinterpret_cast<float4*>(w) = reinterpret_cast<const float4*>(p.w + r * V)[lane];
+    else *reinterpret_cast<float2*>(w) = reinterpret_cast<const float2*>(p.w + r * V)[lane];
+  };
+  // Many rows: one of each warp first.  Independent gates show there, and the first batch of all warps, 29 MB, is not read (32768 rows, the call
+  // that waits for it: 20.2 / 16.1 us; gates of one value per row take as long as before).
+  if (p.rows >= R * warps) {
+    const long long r = first * R;
+    const float4 g = reinterpret_cast<const float4*>(p.g + r * 128)[lane], b = reinterpret_cast<const float4*>(p.b + r * 128)[lane];
+    float w[WV];
+    load_w(r, w);
+    bad = __reduce_or_sync(0xffffffffu, rules_out(g, b, w, __shfl_sync(0xffffffffu, g.x, 0), __shfl_sync(0xffffffffu, b.x, 0)));
+  }
+  for (long long r0 = first * R; r0 < p.rows && bad != 7u; r0 += warps * R) {
     float4 g[R], b[R];
     float w[R][WV];
 #pragma unroll
@@ -41,28 +66,18 @@ gate_regime_kernel(const RegimeProblem p) {
       const long long r = min(r0 + u, p.rows - 1);
       g[u] = reinterpret_cast<const float4*>(p.g + r * 128)[lane];
       b[u] = reinterpret_cast<const float4*>(p.b + r * 128)[lane];
-      if (WV == 4) *reinterpret_cast<float4*>(w[u]) = reinterpret_cast<const float4*>(p.w + r * V)[lane];
-      else *reinterpret_cast<float2*>(w[u]) = reinterpret_cast<const float2*>(p.w + r * V)[lane];
+      load_w(r, w[u]);
     }
 #pragma unroll
     for (int u = 0; u < R; ++u) {
       const float gf = __shfl_sync(0xffffffffu, g[u].x, 0), bf = __shfl_sync(0xffffffffu, b[u].x, 0);
-      const bool g_one = g[u].x == gf && g[u].y == gf && g[u].z == gf && g[u].w == gf;
-      bool one = b[u].x == bf && b[u].y == bf && b[u].z == bf && b[u].w == bf;
-      bool none = b[u].x == 0.f && b[u].y == 0.f && b[u].z == 0.f && b[u].w == 0.f;
-#pragma unroll
-      for (int e = 0; e < WV; ++e) {
-        one = one && w[u][e] == bf;
-        none = none && w[u][e] == 1.f;
-      }
-      bad |= (g_one ? 0u : LETHE_REGIME_SCALAR_GATE) | (one ? 0u : LETHE_REGIME_ONE_BETA) | (none ? 0u : LETHE_REGIME_NO_DELTA);
+      bad |= rules_out(g[u], b[u], w[u], gf, bf);
       if (lane == 0 && r0 + u < p.rows) {
         p.g0[r0 + u] = gf;
         p.b0[r0 + u] = bf;
       }
     }
     bad = __reduce_or_sync(0xffffffffu, bad);
-    if (bad == 7u) break;
     if (*reinterpret_cast<volatile uint32_t*>(p.work) == 7u) break;
   }
   __shared__ uint32_t cta_bad;
