@@ -11,10 +11,9 @@ int launch_prepare(const Problem&, const CUtensorMap&, const CUtensorMap&, const
 int launch_prepare_cw(const Problem&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap&, const CUtensorMap& mg,
                       const NormMaps&, cudaStream_t);
 int launch_output(const Problem&, const CUtensorMap& mq, const CUtensorMap& mv, const CUtensorMap& mo, cudaStream_t);
-int launch_scan(const Problem&, bool adjoint, cudaStream_t);
+int launch_scan(const Problem&, bool adjoint, cudaStream_t, const CUtensorMap* mv = nullptr);
 int launch_bwd_pre(const Problem&, const CUtensorMap& mq, const CUtensorMap& mdo, cudaStream_t);
 bool scan_io_serves(const Problem&, bool adjoint);
-int launch_scan_io(const Problem&, bool adjoint, const CUtensorMap& mio, const CUtensorMap& mv, cudaStream_t);
 int launch_bwd_main(const Problem&, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                     const CUtensorMap& mdo, const OutMaps& mo, cudaStream_t, uint32_t mask);
 int launch_bwd_main_cw(const Problem&, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
@@ -175,9 +174,9 @@ extern "C" int lethe_gdn_forward(const LetheGdnArgs* a, void* stream) {
   }
   CUtensorMap mo;
   if ((m & 4u) && (e = token_map(&mo, a->o, p, p.V))) return e;
-  if ((m & 6u) == 6u && scan_io_serves(p, false)) return launch_scan_io(p, false, mo, mv, st);
-  if ((m & 2u) && (e = launch_scan(p, false, st))) return e;
-  if ((m & 4u) && (e = launch_output(p, mq, mv, mo, st))) return e;
+  if ((m & 6u) == 6u && scan_io_serves(p, false)) p.io = &mo;
+  if ((m & 2u) && (e = launch_scan(p, false, st, &mv))) return e;
+  if ((m & 4u) && !p.io && (e = launch_output(p, mq, mv, mo, st))) return e;
   return kOk;
 }
 
@@ -194,12 +193,9 @@ extern "C" int lethe_gdn_backward(const LetheGdnArgs* a, void* stream) {
   if ((e = token_map(&mk, a->k, p, p.Kr))) return e;
   if ((e = token_map(&mv, a->v, p, p.V))) return e;
   if ((e = token_map(&mdo, a->d_o, p, p.V))) return e;
-  uint32_t m = a->kernel_mask ? a->kernel_mask : 15u;
-  if ((m & 3u) == 3u && scan_io_serves(p, true)) {
-    if ((e = launch_scan_io(p, true, mdo, mv, st))) return e;
-    m &= ~3u;
-  }
-  if ((m & 1u) && (e = launch_bwd_pre(p, mq, mdo, st))) return e;
+  const uint32_t m = a->kernel_mask ? a->kernel_mask : 15u;
+  if ((m & 3u) == 3u && scan_io_serves(p, true)) p.io = &mdo;
+  if ((m & 1u) && !p.io && (e = launch_bwd_pre(p, mq, mdo, st))) return e;
   if ((m & 2u) && (e = launch_scan(p, true, st))) return e;
   p.after_scan = (m & 2u) ? 1 : 0;
   if (m & 12u) {

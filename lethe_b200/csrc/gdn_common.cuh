@@ -93,6 +93,7 @@ struct Problem {
   uint32_t lean;     // 1: intermediates that no later kernel of the call reads are not written; 2: nor what only a backward reads
   int qk16;          // non-zero: q, k, dq, dk hold fp16 instead of bf16
   float scale;
+  const CUtensorMap* io;      // host only: the scan takes the kernel beside it along (launch_scan), whose tensor this is
   int after_scan;    // the same call launched the adjoint scan just before the main kernel
   float l2_eps;      // > 0: the prepare kernel normalises q and k (q for the output kernel too, where that reads it)
   int keep_norm;     // ... and stores the normalised rows

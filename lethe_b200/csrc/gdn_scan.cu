@@ -640,7 +640,9 @@ static int launch_scan_nodelta(const Problem& p, bool adjoint, cudaStream_t st) 
   return e == cudaSuccess ? kOk : kErrLaunch;
 }
 
-int launch_scan(const Problem& p, bool adjoint, cudaStream_t st) {
+int launch_scan_io(const Problem&, bool adjoint, const CUtensorMap& mio, const CUtensorMap& mv, cudaStream_t);
+int launch_scan(const Problem& p, bool adjoint, cudaStream_t st, const CUtensorMap* mv) {
+  if (p.io) return launch_scan_io(p, adjoint, *p.io, mv ? *mv : *p.io, st);
   const int sms = sm_count();
   if (sms <= 0) return kErrDevice;
   if (!p.delta) {
