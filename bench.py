@@ -663,7 +663,7 @@ def main():
     # the timed step is the CUDA-graph replay of forward + backward (ops.GdnStepGraph: the public call for a
     # training step at fixed shapes); the per-kernel and fwd / bwd timings below are plain launches
     graph = ops.GdnStepGraph(buf, d["q"], d["k"], d["v"], g, beta, h0, d["do"], None, scale, groups=args.groups,
-                             pipeline=not args.plain_chain, cut=None if args.cut < 0 else args.cut,
+                             pipeline=False if args.plain_chain else None, cut=None if args.cut < 0 else args.cut,
                              bwd_cuts=[int(x) for x in args.bwd_cuts.split(",")] if args.bwd_cuts else None, **gates)
     ms = timed(graph.replay, args.steps, max(args.warmup, 3))
     ops.check_status(buf.status)
@@ -801,7 +801,7 @@ def main():
                     "host_link_floor_ms": max(h2d, d2h) / (pcie["both"]["slowest_rank_gbs"] * 1e9) * 1e3},
             "autograd_op_ms": op_ms,
             # kernels per replayed step: three per forward and per backward segment of the step graph
-            "gpu_launches": args.steps * 3 * (graph.segments + len(graph.bwd_cuts) + 1),
+            "gpu_launches": args.steps * (graph.launches * args.groups),
             "clocks": clocks,
             "roofline": {"kernel": top, "bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
                          "frac": achieved / hbm, "peak_source": which,

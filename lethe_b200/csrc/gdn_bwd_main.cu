@@ -37,7 +37,8 @@
 // of latencies that one CTA cannot fill.  CTAs are persistent and fetch the next chunk's tiles as theirs fall free, which is late
 // for most of them: all are prefetched to L2 under the first products, and copies are issued by threads that issue no products.
 // us, with six groups and without the prefetch, and now: d_v = 64, 512 chunks 44 -> 40, 4096 230 -> 226; d_v = 128, 512 chunks 62
-// -> 54; without the delta term d_v = 128, 4096 chunks 265 -> 191, d_v = 64, 1692 chunks 75 -> 64.
+// -> 54; without the delta term d_v = 128, 4096 chunks 265 -> 191, d_v = 64, 1692 chunks 75 -> 64, later 57 -> 55.5 (loads
+// ahead of the stores to swizzled tiles), with 64 key channels 45.
 #include "gdn_cw.cuh"
 #include "host_util.h"
 

@@ -39,7 +39,7 @@
 // are dead once its last products are issued, under the longest CUDA-core phase.  Inside a group the products that the chain waits
 // for are issued first and the rest of the epilogue before lies in the next group's shadow.
 // us at d_v = 128, before (dT, X = dT T^T and dM as three groups, 88 to 440 bytes a thread of spilled loads, 0 to 48 now, all copies
-// issued by one thread, beta and the per-channel gates read when they were needed) and now: 8192 chunks 920 -> 789; 4096 without the
+// issued by one thread, beta and the per-channel gates read when they were needed) and then: 8192 chunks 920 -> 789 (773 with the abort flag behind the waits); 4096 without the
 // delta term 301 -> 267; 512 with per-channel gates 113 -> 79.
 // Cycles per chunk by clock samples of one CTA (d_v = 128): operand columns and waits for the tiles 4.9 k, group 1 2.5 k, the rest
 // up to dM 7.0 k, column sums with the decay assembly 5.0 k, row sums with the gradients 5.6 k, gate gradient and stores 2.2 k; 27.1 k

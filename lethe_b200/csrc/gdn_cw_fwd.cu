@@ -23,7 +23,7 @@
 // one chunk's barriers, product waits and loads lie under the other's arithmetic; k, q and alpha go to registers after the diagonal
 // sums and the operands take their tiles.  1: 512 threads, for a launch that gives every SM one chunk at most, where only the
 // length of a chunk's own chain counts.  Measured (us, d_v = 128; one CTA of 512 threads with twice the memory / two of 256 /
-// these diagonal sums, loads that come early, beta a chunk ahead): 8192 chunks 590 / 559 / 486; 512 chunks 54 / 49 / 44; without the
+// these diagonal sums, loads that come early, beta a chunk ahead): 8192 chunks 590 / 559 / 486 (480 with the abort flag behind the waits); 512 chunks 54 / 49 / 44; without the
 // delta term 4096 chunks 209 / 190 / 158; per-channel gates 512 chunks 70 / 59 / 52; 128 chunks 20 in each.
 //
 // Loads: k and q of the next chunk as soon as the inverse is done, g when w and u have left its tiles, behind a prefetch to L2 that

@@ -24,7 +24,9 @@ namespace lg {
 // per SM; the next k, q and v are fetched as soon as their tiles are dead (k and q under product 3 and the last epilogue),
 // and the gates are summed a chunk ahead by one warp.  With one CTA per chunk instead, the wait for the first loads and the
 // start of the CTA were 40 % of its time.  The gates are applied to the columns of T, not to k and v: half the elements.
-// 4096 chunks: d_v = 64 167 -> 132 us, d_v = 128 183 -> 143; without the delta term (below) d_v = 128 121 -> 85.
+// 4096 chunks: d_v = 64 167 -> 132 us, d_v = 128 183 -> 143; without the delta term (below) d_v = 128 121 -> 85.  With loads ahead of the
+// stores to swizzled tiles, the abort flag behind the waits and the first gates summed under the first product 132 -> 127, 512 chunks 21.6
+// -> 20.3, 128 chunks 9.1 -> 8.5.
 // The gates of the next chunk come by asynchronous copies to shared memory, its place from one thread, and (not at d_v = 128) its
 // tiles are prefetched to L2 under product 1: without the delta term d_v = 128 79 -> 70, with it within 2 %.
 // ---------------------------------------------------------------------------------------------

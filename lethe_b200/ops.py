@@ -275,6 +275,10 @@ class GdnStepGraph:
         if bwd_cuts is None or not self.pipeline:
             bwd_cuts = self._default_bwd_cuts(buf, NT, BH, dev, self.cut)
         self.bwd_cuts = tuple(sorted(int(c) for c in bwd_cuts))
+        # kernels of one replay (and range of pairs)
+        self.launches = 3 * (self.segments + len(self.bwd_cuts) + 1)
+        if not self.pipeline:
+            self.launches = 6 - self._kernels_beside_scans(buf, BH, dev)
         if any(c <= 0 or c >= NT for c in self.bwd_cuts) or len(set(self.bwd_cuts)) != len(self.bwd_cuts):
             raise GdnError(f"lethe_gdn: backward cuts {self.bwd_cuts} must be distinct chunk indices inside (0, {NT})")
         gates = dict(b_gate=b_gate, w_gate=w_gate, lean=True)
@@ -399,6 +403,15 @@ class GdnStepGraph:
         if not step_is_cut(buf.dims.gate, buf.dims.delta != 0, NT, BH, sms):
             return 0
         return default_cut(buf.dims.gate, buf.dims.V, NT, BH, sms)
+
+    @staticmethod
+    def _kernels_beside_scans(buf, BH: int, dev) -> int:
+        """How many of a plain step's two scans take another kernel along."""
+        sms = torch.cuda.get_device_properties(dev).multi_processor_count
+        if buf.dims.gate != GATE_CHANNEL:
+            return 0
+        forward = step_is_chain(buf.dims.gate, buf.dims.V, buf.dims.delta != 0, BH, sms)
+        return int(forward) + int((4 if buf.dims.delta else 3) * (buf.dims.V // 64) * BH > sms)
 
     @staticmethod
     def _is_chain(buf, BH: int, dev) -> bool:
