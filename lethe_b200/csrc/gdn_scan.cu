@@ -99,7 +99,15 @@ scan_kernel(const Problem p) {
         const int st = it % kStages;
         if (it >= kStages) mbar_wait(&bar_free[st], static_cast<uint32_t>(((it / kStages) - 1) & 1), ctl, 303, true);
         mbar_expect_tx(&bar_full[st], 32768u);
-        bulk_g2s(Pst + st * 32768, Pg + (static_cast<size_t>(bh) * NT + chunk_of(it)) * 32768, 32768u, &bar_full[st]);
+        const size_t z = static_cast<size_t>(bh) * NT + chunk_of(it);
+        bulk_g2s(Pst + st * 32768, Pg + z * 32768, 32768u, &bar_full[st]);
+        // What the state warps load to registers a step ahead goes to L2 now, three steps ahead: a step is shorter than its way from
+        // HBM (us, without / with, forward and adjoint alike: 40 pairs x 128 chunks, d_v = 64, 109 / 94; 64 x 64 63 / 52; d_v = 128 19 x 128
+        // 105 / 93, 64 x 64 74 / 63; the decays alone 2 %).  In the adjoint not before the kernel that makes Rb has ended.
+        if (ADJOINT && it < kStages) continue;
+        if (ADJOINT && it == kStages) griddep_wait();
+        bulk_prefetch(p.saved + p.lay.ad + z * 512, 512);
+        bulk_prefetch((ADJOINT ? p.scratch + p.lay.rb : p.saved + p.lay.r) + z * p.lay.sz_r + static_cast<size_t>(v0 >> 6) * 16384, 16384);
       }
     }
   } else if (warp > kStateWarps) {
@@ -239,7 +247,7 @@ scan_kernel(const Problem p) {
 //
 // Bound by the matrix pipe (17 cycles for a product of 16 x 8 x 16 per SM quarter, so 0.14 us per 8 columns) behind 0.25 us of
 // barrier, operand loads and P's way to registers: 0.39 us a step with 8 columns, 0.51 with 16, 0.79 with 32; tcgen05 took 0.69
-// with 16 (same measure: slope over the number of chunks, L2 cold) and takes 0.83 with 64.  With the fetch behind the products
+// with 16 (same measure: slope over the number of chunks, L2 cold) and takes 0.72 with 64.  With the fetch behind the products
 // instead of between them 16 columns took 0.62, with four warps of kM = 2 at 32 columns the step is 0.92.
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t* r) {
