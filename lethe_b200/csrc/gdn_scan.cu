@@ -97,7 +97,7 @@ scan_kernel(const Problem p) {
       const unsigned char* Pg = p.saved + p.lay.p;
       for (int it = 0; it < n; ++it) {
         const int st = it % kStages;
-        if (it >= kStages) mbar_wait(&bar_free[st], static_cast<uint32_t>(((it / kStages) - 1) & 1), ctl, 303, true);
+        if (it >= kStages) mbar_wait(&bar_free[st], static_cast<uint32_t>(((it / kStages) - 1) & 1), ctl, 303);
         mbar_expect_tx(&bar_full[st], 32768u);
         const size_t z = static_cast<size_t>(bh) * NT + chunk_of(it);
         bulk_g2s(Pst + st * 32768, Pg + z * 32768, 32768u, &bar_full[st]);
@@ -123,7 +123,7 @@ scan_kernel(const Problem p) {
     const uint32_t acc = tmem + static_cast<uint32_t>(m * kW);
     for (int it = 0; it < n; ++it) {
       const int st = it % kStages;
-      mbar_wait_warp(&bar_full[st], static_cast<uint32_t>((it / kStages) & 1), ctl, 301, true);
+      mbar_wait_warp(&bar_full[st], static_cast<uint32_t>((it / kStages) & 1), ctl, 301);
       if (m == 0 && lane == 0) bulk_wait_read();     // the other operand tile is recorded: it may be written again
       step_sync<kStepBarrier>();
       tc_fence_after();
@@ -200,7 +200,7 @@ scan_kernel(const Problem p) {
         load_r(cn);
         a_next = ADg[(static_cast<size_t>(bh) * NT + cn) * kK + d];
       }
-      mbar_wait_warp(bar_mma, static_cast<uint32_t>(it & 1), ctl, 302, true);
+      mbar_wait_warp(bar_mma, static_cast<uint32_t>(it & 1), ctl, 302);
       tc_fence_after();
       static_assert(kMmaWarps == 2, "two accumulators of kW columns, one per half of the contraction");
       float a0[kVs], a1[kVs];

@@ -74,16 +74,11 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 // Bounded wait on phase `parity`.  `code` identifies the wait site in the status word.  The abort flag is looked at only where
-// the phase is not complete yet: ahead of the first look its load is part of every wait of a chunk's chain.
-// `flag_first` keeps that order for scan_kernel, which is the faster with it (32 pairs x 250 chunks, us: 218 / 224).
-__device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, const CtaCtl& ctl, int code, bool flag_first = false) {
-  if (flag_first) {
-    if (*ctl.abort_flag) return;
-    if (mbar_try(bar, parity)) return;
-  } else {
-    if (mbar_test(bar, parity)) return;
-    if (*ctl.abort_flag) return;
-  }
+// the phase is not complete yet: ahead of the first look its load is part of every wait of a chunk's chain (us, before / now:
+// channel-wise prepare, 8192 chunks, 486 / 480, main 780 / 772).
+__device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, const CtaCtl& ctl, int code) {
+  if (mbar_test(bar, parity)) return;
+  if (*ctl.abort_flag) return;
   const long long t0 = clock64();
   while (!mbar_try(bar, parity)) {
     if (*ctl.abort_flag) return;
@@ -97,8 +92,8 @@ __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, const 
 
 // Same, for a wait that every lane of the calling warp executes: the warp leaves it converged, which
 // the .sync.aligned tcgen05 instructions that usually follow require.
-__device__ __forceinline__ void mbar_wait_warp(uint64_t* bar, uint32_t parity, const CtaCtl& ctl, int code, bool flag_first = false) {
-  mbar_wait(bar, parity, ctl, code, flag_first);
+__device__ __forceinline__ void mbar_wait_warp(uint64_t* bar, uint32_t parity, const CtaCtl& ctl, int code) {
+  mbar_wait(bar, parity, ctl, code);
   __syncwarp();
 }
 
