@@ -88,9 +88,10 @@ __device__ __forceinline__ void prep_load_v(unsigned char* Vt, const CUtensorMap
   mbar_expect_tx(bar, V * 128u);
   for (int t = 0; t < V / 64; ++t) tma_load_4d(Vt + t * 8192, mv, bar, t * 64, a.h, a.c * kC, a.b);
 }
-// The rows of the tile [k; q] normalised, as lethe_gdn_l2norm_qk does (x rsqrt(sum x^2 + eps) in fp32, one rounding to fp16).  Four lanes
-// have a row; the eight rows of a pass take the same 16-byte piece at a time, so the swizzle keeps them off one another's banks.  A
-// kernel of its own took a launch and another pass over q and k (prefill of 1000 tokens, 8 heads: 26.6 us, now 22.2).
+// The rows of the tile [k; q] normalised, as lethe_gdn_l2norm_qk does (x rsqrt(sum x^2 + eps) in fp32, one rounding to fp16) and to its
+// bits: every sum is formed in its order.  Four lanes have a row; the eight rows of a pass take the same 16-byte piece at a time, so the
+// swizzle keeps them off one another's banks.  A kernel of its own took a launch and another pass over q and k (prefill of 1000 tokens,
+// 8 heads: 26.6 us, now 21.5).
 // kPass: passes whose loads come together, ahead of the first store
 template <int KW = kK, int kPass = 2>
 __device__ __forceinline__ void prep_normalise_rows(unsigned char* KQ, int r0, int part, int f16, float eps) {
@@ -102,15 +103,18 @@ __device__ __forceinline__ void prep_normalise_rows(unsigned char* KQ, int r0, i
     for (int j = 0; j < kN; ++j) c[u][j] = tile_ld_chunk(KQ, r0 + 8 * u, part + 4 * j, 128);
 #pragma unroll
   for (int u = 0; u < kPass; ++u) {
-    float x[kN][8], ss = 0.f;
+    float x[kN][8], sp[kN];
 #pragma unroll
     for (int j = 0; j < kN; ++j) {
       unpack8_in(c[u][j], x[j], f16);
+      sp[j] = 0.f;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) ss = fmaf(x[j][e], x[j][e], ss);
+      for (int e = 0; e < 8; ++e) sp[j] = fmaf(x[j][e], x[j][e], sp[j]);
     }
-    ss += __shfl_xor_sync(0xffffffffu, ss, 8);
+    // the order of row_sum: pieces 8 apart, then 4, 2 and 1
+    float ss = kN == 4 ? (sp[0] + sp[kN - 2]) + (sp[1] + sp[kN - 1]) : sp[0] + sp[1];
     ss += __shfl_xor_sync(0xffffffffu, ss, 16);
+    ss += __shfl_xor_sync(0xffffffffu, ss, 8);
     const float s = rsqrtf(ss + eps);
 #pragma unroll
     for (int j = 0; j < kN; ++j) {
