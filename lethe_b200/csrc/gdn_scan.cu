@@ -538,8 +538,12 @@ scan_mma_kernel(const Problem p) {
 // of a record atom, so every access is a full line.  What is on the way from HBM decides the speed: a thread copies the R of
 // the next kDepth chunks to shared memory behind its own back.  (As loads to registers, 16 or 8 of them, a wait for one was a wait for
 // all that shared its scoreboard, six for a warp, and a step took 0.6 us: 36 pairs x 94 and 188 chunks, d_v = 64, 55 and 114 us, now
-// 18 and 40; 64 pairs x 64, d_v = 128, 59, now 46.)  32 slots, one CTA per SM, for whole sequences (40, 48 and 80 pairs x 64, d_v = 128, us, 8 /
-// 16 / 32: 36 / 39 / 33, 46 / 39 / 36, 63 / 62 / 57).  A range of chunks (captured step) has chunk kernels beside it, which need the room:
+// 18 and 40; 64 pairs x 64, d_v = 128, 59, now 46.)  32 slots, one CTA per SM, for whole sequences of more than 16
+// chunks (40, 48 and 80 pairs x 64, d_v = 128, us, 8 / 16 / 32: 36 / 39 / 33, 46 / 39 / 36, 63 / 62 / 57).  Shorter ones do not fill that ring,
+// and with many pairs one CTA per SM is a long row of nearly empty rounds: 16 slots, and for 8 chunks at most and more CTAs than two per
+// SM 8, four CTAs per SM (three in the forward from 5 chunks on: more of them read in a worse order).  SSD, d_v = 128, us, forward and
+// backward, registers as above / always 32 slots / now: 256 pairs x 1 28 and 38 / 38 and 50 / 26 and 36; 1024 x 1 81 and 103 / 120 and 151 / 77
+// and 95; 256 x 4 58 and 83 / 70 and 95 / 58 and 82; d_v = 64, 1024 x 8 234 and 348 / 239 and 359 / 224 and 348.  A range of chunks (captured step) has chunk kernels beside it, which need the room:
 // 16 while two CTAs per SM hold the whole grid, 8 beyond (captured step, SSD, 16 pairs x 32, d_v = 128, 8 / 16 / 32 88 / 78 / 84; GLA, 64 pairs x
 // 64, 603 / 613 / 625).
 // R / Rb and the state records are 128-row tile images, of which rows from Kw on are neither read nor written.
@@ -637,12 +641,17 @@ static int launch_scan_few(const Problem& p, bool adjoint, cudaStream_t st) {
   return e == cudaSuccess ? kOk : kErrLaunch;
 }
 
-template <int kDepth>
+// Shared memory with which `most` CTAs fit an SM's 228 KB (each takes 1 KB more) and another does not.
+constexpr int scan_share(int most) { return 233472 / (most + 1) - 512; }
+// kMost: CTAs per SM at most, 3 or more (0: as many as the ring leaves room for)
+template <int kDepth, int kMost = 0>
 static int launch_scan_nodelta(const Problem& p, bool adjoint, cudaStream_t st) {
   const dim3 g((p.V / 64) * (p.Kw / 32), p.nbh);
-  constexpr int smem = ScanNdSmem<kDepth>::kBytes;
+  constexpr int ring = ScanNdSmem<kDepth>::kBytes, smem = kMost && scan_share(kMost) > ring ? scan_share(kMost) : ring;
+  constexpr int limit = ring > scan_share(3) ? ring : scan_share(3);      // (one limit per kernel, whatever kMost)
+  static_assert(kMost == 0 || (kMost >= 3 && smem <= limit), "");
   static SmemAttr attr[2];
-  if (attr[0].set(scan_nodelta_kernel<false, kDepth>, smem) || attr[1].set(scan_nodelta_kernel<true, kDepth>, smem)) return kErrLaunch;
+  if (attr[0].set(scan_nodelta_kernel<false, kDepth>, limit) || attr[1].set(scan_nodelta_kernel<true, kDepth>, limit)) return kErrLaunch;
   const cudaError_t e = adjoint ? launch_dependent(scan_nodelta_kernel<true, kDepth>, g, dim3(256), smem, st, p)
                                 : launch_dependent(scan_nodelta_kernel<false, kDepth>, g, dim3(256), smem, st, p);
   return e == cudaSuccess ? kOk : kErrLaunch;
@@ -654,9 +663,11 @@ int launch_scan(const Problem& p, bool adjoint, cudaStream_t st, const CUtensorM
   const int sms = sm_count();
   if (sms <= 0) return kErrDevice;
   if (!p.delta) {
-    if (p.cn == p.NT) return launch_scan_nodelta<32>(p, adjoint, st);
-    const int ctas = (p.V / 64) * (p.Kw / 32) * p.nbh;
-    return ctas <= 2 * sms ? launch_scan_nodelta<16>(p, adjoint, st) : launch_scan_nodelta<8>(p, adjoint, st);
+    const int ctas = (p.V / 64) * (p.Kw / 32) * p.nbh, n = p.cn;
+    if (n < p.NT) return ctas <= 2 * sms ? launch_scan_nodelta<16>(p, adjoint, st) : launch_scan_nodelta<8>(p, adjoint, st);
+    if (n > 16 || (n > 8 && ctas <= sms)) return launch_scan_nodelta<32>(p, adjoint, st);
+    if (n > 8 || ctas <= 2 * sms) return launch_scan_nodelta<16>(p, adjoint, st);
+    return n <= 4 || adjoint ? launch_scan_nodelta<8, 4>(p, adjoint, st) : launch_scan_nodelta<8, 3>(p, adjoint, st);
   }
   // Warp-level products or tcgen05 (the same bits): by the whole problem, since calls on ranges of its pairs run beside one another.
   // The line is where 16 columns no longer give every CTA an SM of its own.  Beyond it 32 columns are the shorter scan (alone, us,
