@@ -800,7 +800,7 @@ def main():
                     "host_link": pcie,
                     "host_link_floor_ms": max(h2d, d2h) / (pcie["both"]["slowest_rank_gbs"] * 1e9) * 1e3},
             "autograd_op_ms": op_ms,
-            # kernels per replayed step: three per forward and per backward segment of the step graph
+            # kernels per replayed step, as the step graph captured them (every range of pairs its own)
             "gpu_launches": args.steps * (graph.launches * args.groups),
             "clocks": clocks,
             "roofline": {"kernel": top, "bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",

@@ -141,6 +141,12 @@ typedef struct LetheGdnArgs {
 size_t lethe_gdn_saved_bytes(const LetheGdnDims* dims);
 size_t lethe_gdn_scratch_bytes(const LetheGdnDims* dims);
 
+/* Which scans of whole calls on these sizes do the work of the kernel beside them (output kernel, scan input) themselves, on a    */
+/* GPU of `sms` SMs (0: the current device): one launch less each, and the records between the two are not written.  0 for lean 0.  */
+/* No counterpart in the reference.                                                                                                */
+enum { LETHE_JOINT_FORWARD = 1, LETHE_JOINT_ADJOINT = 2 };
+int lethe_gdn_joint_scans(const LetheGdnDims* dims, uint32_t lean, int32_t sms);
+
 /* Forward: o (and hT) from q, k, v, g, beta, h0.  Replaces gdn_layer.py:17-67 of the reference. */
 int lethe_gdn_forward(const LetheGdnArgs* args, void* cuda_stream);
 

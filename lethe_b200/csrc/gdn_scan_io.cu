@@ -515,12 +515,19 @@ static int launch_scan_io_t(const Problem& p, const CUtensorMap& mio, const CUte
 // CTAs here: 48 51 / 50, 51 / 50, 37 / 41; 64 63 / 72, 63 / 61, 50 / 48; 96 92 / 79, 92 / 65, 76 / 48; 128 119 / 88, 119 / 70, 100 / 52;
 // 160 145 / 151, 145 / 128, 122 / 96; 250 chunks, 64 CTAs 229 / 254, 229 / 220, 196 / 166).  By the whole problem, since calls on
 // ranges of its pairs run beside one another.
-bool scan_io_serves(const Problem& p, bool adjoint) {
-  const int sms = sm_count();
-  if (p.gate != LETHE_GATE_CHANNEL || !p.lean || p.cn != p.NT || sms <= 0) return false;
-  const int ctas = p.V / kIoW * p.B * p.H, rounds = (ctas + sms - 1) / sms;
-  if (p.delta) return 4 * ctas > sms;
+static bool scan_io_rule(int gate, int delta, int V, int pairs, bool adjoint, int sms) {
+  if (gate != LETHE_GATE_CHANNEL || sms <= 0) return false;
+  const int ctas = V / kIoW * pairs, rounds = (ctas + sms - 1) / sms;
+  if (delta) return 4 * ctas > sms;
   return adjoint ? 3 * ctas > sms : 5 * ctas > 3 * rounds * sms;
+}
+bool scan_io_serves(const Problem& p, bool adjoint) {
+  return p.lean && p.cn == p.NT && scan_io_rule(p.gate, p.delta, p.V, p.B * p.H, adjoint, sm_count());
+}
+// ... for lethe_gdn_joint_scans, which a captured step is planned with
+int scan_io_joint(const LetheGdnDims& d, int sms) {
+  auto serves = [&](bool adjoint) { return scan_io_rule(d.gate, d.delta, d.V, d.B * d.H, adjoint, sms); };
+  return (serves(false) ? LETHE_JOINT_FORWARD : 0) | (serves(true) ? LETHE_JOINT_ADJOINT : 0);
 }
 // mio: o (forward) or do (adjoint)
 int launch_scan_io(const Problem& p, bool adjoint, const CUtensorMap& mio, const CUtensorMap& mv, cudaStream_t st) {

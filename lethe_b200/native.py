@@ -51,6 +51,8 @@ def _declare(L: ctypes.CDLL) -> None:
     L.lethe_gdn_saved_bytes.argtypes = [c_void_p]
     L.lethe_gdn_scratch_bytes.restype = ctypes.c_size_t
     L.lethe_gdn_scratch_bytes.argtypes = [c_void_p]
+    L.lethe_gdn_joint_scans.restype = c_int
+    L.lethe_gdn_joint_scans.argtypes = [c_void_p, ctypes.c_uint32, ctypes.c_int32]
     L.lethe_gdn_forward.restype = c_int
     L.lethe_gdn_forward.argtypes = [c_void_p, c_void_p]
     L.lethe_gdn_backward.restype = c_int

@@ -218,14 +218,17 @@ def step_is_cut(gate: int, delta: bool, NT: int, BH: int, sms: int) -> bool:
     return gate != GATE_CHANNEL or NT * BH >= 2 * sms
 
 
-def step_is_chain(gate: int, V: int, delta: bool, BH: int, sms: int) -> bool:
+def joint_scans(gate: int, V: int, delta: bool, BH: int, sms: int, NT: int = 64) -> int:
+    """Which scans of a whole lean call the library launches with the kernel beside them in one: 1 forward, 2 adjoint (bits)."""
+    dims = _Dims(1, BH, 64 * NT, 128, V, gate, int(delta))
+    return native.lib().lethe_gdn_joint_scans(ctypes.byref(dims), 1, sms)
+
+
+def step_is_chain(gate: int, V: int, delta: bool, BH: int, sms: int, NT: int = 64) -> bool:
     """Whether one chain of whole calls is the faster captured step: where forward and backward take the scans that have the output,
-    or their input, beside them (``scan_io_serves`` of the library).  Replay in us, overlapped / chain, BH x NT: KDA, d_v = 64, 64 x 16
+    or their input, beside them (``joint_scans``).  Replay in us, overlapped / chain, BH x NT: KDA, d_v = 64, 64 x 16
     229 / 217, 64 x 64 801 / 766; d_v = 128 32 x 64 515 / 498, 64 x 64 960 / 868; GLA, d_v = 128, 32 x 64 (not this) 311 / 319, 64 x 64 606 / 549."""
-    ctas = V // 64 * BH
-    if gate != GATE_CHANNEL:
-        return False
-    return 4 * ctas > sms if delta else 5 * ctas > 3 * -(-ctas // sms) * sms
+    return joint_scans(gate, V, delta, BH, sms, NT) == 3
 
 
 class GdnStepGraph:
@@ -266,7 +269,7 @@ class GdnStepGraph:
         ranges = [(bounds[i], bounds[i + 1] - bounds[i]) for i in range(groups)]
         self.groups = groups
         if pipeline is None:
-            pipeline = groups == 1 and not (cut is None and bwd_cuts is None and self._is_chain(buf, BH, dev))
+            pipeline = groups == 1 and not (cut is None and bwd_cuts is None and self._joint_scans(buf, BH, NT, dev) == 3)
         self.pipeline = bool(pipeline) and groups == 1
         if cut is None:
             cut = self._default_cut(buf, NT, BH, dev)
@@ -278,7 +281,7 @@ class GdnStepGraph:
         # kernels of one replay (and range of pairs)
         self.launches = 3 * (self.segments + len(self.bwd_cuts) + 1)
         if not self.pipeline:
-            self.launches = 6 - self._kernels_beside_scans(buf, BH, dev)
+            self.launches = 6 - self._joint_scans(buf, BH, NT, dev).bit_count()
         if any(c <= 0 or c >= NT for c in self.bwd_cuts) or len(set(self.bwd_cuts)) != len(self.bwd_cuts):
             raise GdnError(f"lethe_gdn: backward cuts {self.bwd_cuts} must be distinct chunk indices inside (0, {NT})")
         gates = dict(b_gate=b_gate, w_gate=w_gate, lean=True)
@@ -405,18 +408,9 @@ class GdnStepGraph:
         return default_cut(buf.dims.gate, buf.dims.V, NT, BH, sms)
 
     @staticmethod
-    def _kernels_beside_scans(buf, BH: int, dev) -> int:
-        """How many of a plain step's two scans take another kernel along."""
+    def _joint_scans(buf, BH: int, NT: int, dev) -> int:
         sms = torch.cuda.get_device_properties(dev).multi_processor_count
-        if buf.dims.gate != GATE_CHANNEL:
-            return 0
-        forward = step_is_chain(buf.dims.gate, buf.dims.V, buf.dims.delta != 0, BH, sms)
-        return int(forward) + int((4 if buf.dims.delta else 3) * (buf.dims.V // 64) * BH > sms)
-
-    @staticmethod
-    def _is_chain(buf, BH: int, dev) -> bool:
-        sms = torch.cuda.get_device_properties(dev).multi_processor_count
-        return step_is_chain(buf.dims.gate, buf.dims.V, buf.dims.delta != 0, BH, sms)
+        return joint_scans(buf.dims.gate, buf.dims.V, buf.dims.delta != 0, BH, sms, NT)
 
     @staticmethod
     def _default_bwd_cuts(buf, NT: int, BH: int, dev, cut: int) -> tuple:
