@@ -14,7 +14,7 @@ int launch_output(const Problem&, const CUtensorMap& mq, const CUtensorMap& mv, 
 int launch_scan(const Problem&, bool adjoint, cudaStream_t, const CUtensorMap* mv = nullptr);
 int launch_bwd_pre(const Problem&, const CUtensorMap& mq, const CUtensorMap& mdo, cudaStream_t);
 bool scan_io_serves(const Problem&, bool adjoint);
-int scan_io_joint(const LetheGdnDims&, int sms);
+int scan_io_joint(const LetheGdnDims&, uint32_t lean, int sms);
 int launch_bwd_main(const Problem&, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                     const CUtensorMap& mdo, const OutMaps& mo, cudaStream_t, uint32_t mask);
 int launch_bwd_main_cw(const Problem&, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
@@ -148,7 +148,7 @@ extern "C" size_t lethe_gdn_scratch_bytes(const LetheGdnDims* d) {
 
 extern "C" int lethe_gdn_joint_scans(const LetheGdnDims* d, uint32_t lean, int32_t sms) {
   if (!d || !lean || !dims_ok(*d)) return 0;
-  return scan_io_joint(*d, sms > 0 ? sms : sm_count());
+  return scan_io_joint(*d, lean, sms > 0 ? sms : sm_count());
 }
 
 extern "C" int lethe_gdn_forward(const LetheGdnArgs* a, void* stream) {

@@ -515,18 +515,26 @@ static int launch_scan_io_t(const Problem& p, const CUtensorMap& mio, const CUte
 // CTAs here: 48 51 / 50, 51 / 50, 37 / 41; 64 63 / 72, 63 / 61, 50 / 48; 96 92 / 79, 92 / 65, 76 / 48; 128 119 / 88, 119 / 70, 100 / 52;
 // 160 145 / 151, 145 / 128, 122 / 96; 250 chunks, 64 CTAs 229 / 254, 229 / 220, 196 / 166).  By the whole problem, since calls on
 // ranges of its pairs run beside one another.
-static bool scan_io_rule(int gate, int delta, int V, int pairs, bool adjoint, int sms) {
+//
+// Short sequences: a CTA has the whole SM, and its start (barriers, tensor memory, the first loads) is as long for one chunk as for many,
+// so a row of rounds of them loses to kernels that share the SMs.  us, the two / this one, pairs x chunks, without the delta term, d_v =
+// 128: forward 256 x 1 34 / 43, x 2 50 / 58, x 4 81 / 85, x 6 118 / 117, x 8 155 / 149; evaluation 256 x 2 50 / 54, x 3 69 / 69, x 4 81 / 79;
+// adjoint 1024 x 1 118 / 142, x 2 202 / 216, x 3 286 / 288, x 4 409 / 397; d_v = 64, forward 512 x 4 110 / 120, x 6 155 / 160, x 8 200 / 200,
+// evaluation x 4 110 / 116, x 6 155 / 155.  With it only the forward over one chunk: d_v = 128, 256 pairs 50 / 54, 512 90 / 93; two chunks 79 / 79.
+static bool scan_io_rule(int gate, int delta, int V, int pairs, int NT, uint32_t lean, bool adjoint, int sms) {
   if (gate != LETHE_GATE_CHANNEL || sms <= 0) return false;
   const int ctas = V / kIoW * pairs, rounds = (ctas + sms - 1) / sms;
-  if (delta) return 4 * ctas > sms;
-  return adjoint ? 3 * ctas > sms : 5 * ctas > 3 * rounds * sms;
+  if (delta) return 4 * ctas > sms && (adjoint || NT > 1 || rounds <= 2);
+  if (adjoint) return 3 * ctas > sms && (NT > 2 || rounds <= 2);
+  const int least = lean == 2u ? (V == 64 ? 6 : 3) : (V == 64 ? 8 : 6);
+  return 5 * ctas > 3 * rounds * sms && (NT >= least || rounds == 1);
 }
 bool scan_io_serves(const Problem& p, bool adjoint) {
-  return p.lean && p.cn == p.NT && scan_io_rule(p.gate, p.delta, p.V, p.B * p.H, adjoint, sm_count());
+  return p.lean && p.cn == p.NT && scan_io_rule(p.gate, p.delta, p.V, p.B * p.H, p.NT, p.lean, adjoint, sm_count());
 }
 // ... for lethe_gdn_joint_scans, which a captured step is planned with
-int scan_io_joint(const LetheGdnDims& d, int sms) {
-  auto serves = [&](bool adjoint) { return scan_io_rule(d.gate, d.delta, d.V, d.B * d.H, adjoint, sms); };
+int scan_io_joint(const LetheGdnDims& d, uint32_t lean, int sms) {
+  auto serves = [&](bool adjoint) { return scan_io_rule(d.gate, d.delta, d.V, d.B * d.H, d.L / kC, lean, adjoint, sms); };
   return (serves(false) ? LETHE_JOINT_FORWARD : 0) | (serves(true) ? LETHE_JOINT_ADJOINT : 0);
 }
 // mio: o (forward) or do (adjoint)

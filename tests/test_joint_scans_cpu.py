@@ -34,3 +34,17 @@ def test_none_for_a_call_that_leaves_every_record_or_for_bad_sizes():
     assert joint(ops.GATE_CHANNEL, 128, 1, 64, lean=0) == 0
     assert joint(ops.GATE_CHANNEL, 96, 1, 64) == 0
     assert native.lib().lethe_gdn_joint_scans(None, 1, B200_SMS) == 0
+
+
+F, A = 1, 2      # forward, adjoint
+
+
+@pytest.mark.parametrize("V,delta,BH,NT,lean,bits", [
+    # one CTA per SM: short sequences of many pairs are a row of rounds that are all start
+    (128, 0, 1024, 1, 1, 0), (128, 0, 256, 2, 1, 0), (128, 0, 256, 3, 1, A), (128, 0, 256, 5, 1, A), (128, 0, 256, 6, 1, F | A),
+    (64, 0, 512, 7, 1, A), (64, 0, 512, 8, 1, F | A), (64, 0, 512, 5, 2, A), (64, 0, 512, 6, 2, F | A), (128, 0, 256, 2, 2, 0),
+    (128, 0, 256, 3, 2, F | A), (128, 1, 1024, 1, 1, A), (128, 1, 1024, 2, 1, F | A), (128, 2, 149, 1, 1, A),
+    # one round (with the delta term, or in the adjoint: two) at any length
+    (128, 0, 64, 1, 1, F | A), (64, 0, 128, 1, 1, F | A), (128, 0, 128, 1, 1, A), (128, 1, 148, 1, 1, F | A), (64, 1, 38, 1, 1, F | A)])
+def test_short_sequences_of_many_pairs(V, delta, BH, NT, lean, bits):
+    assert joint(ops.GATE_CHANNEL, V, delta, BH, NT, lean) == bits
