@@ -92,8 +92,11 @@ int32_t* status_word(int dev) {
 // ---------------------------------------------------------------------------------------------
 // tensors
 // ---------------------------------------------------------------------------------------------
+// memory that does not hold the values: a negated view, a tensor of zeros without storage
+bool lazy(const Tensor& t) { return t.is_neg() || t._is_zerotensor(); }
 Tensor as(const Tensor& t, at::ScalarType dt) {
-  return t.scalar_type() == dt ? t.contiguous() : t.to(dt).contiguous();
+  const Tensor r = t.scalar_type() == dt ? t : t.to(dt);
+  return (lazy(r) ? r.clone() : r).contiguous();
 }
 Tensor as32(const Tensor& t) { return t.defined() ? as(t, at::kFloat) : t; }
 // a gate per channel is read through a tensor map, which wants its start on a 16-byte boundary
@@ -134,7 +137,7 @@ cudaStream_t stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream
 
 // bf16 <-> fp32 by a kernel of the library, where `t` is that in one piece (Tensor::to costs the host three times a launch)
 bool converts(const Tensor& t, at::ScalarType from) {
-  return t.scalar_type() == from && t.is_contiguous() && t.numel() > 0 && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
+  return t.scalar_type() == from && t.is_contiguous() && !lazy(t) && t.numel() > 0 && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
 }
 Tensor to_f32(const Tensor& t) {
   Tensor r = at::empty(t.sizes(), t.options().dtype(at::kFloat));
@@ -474,8 +477,8 @@ void prepare_qk(const Problem& p, const Tensor& q, const Tensor& k, Operands* x,
     check(lethe_gdn_l2norm_qk(qc.data_ptr(), kc.data_ptr(), x->q.data_ptr(), x->k.data_ptr(), qc.numel() / p.K,
                               static_cast<int32_t>(p.K), flags, kL2Eps, stream_of(qc)));
   } else if (q.scalar_type() == at::kHalf && k.scalar_type() == at::kHalf) {
-    x->q = q.contiguous();
-    x->k = k.contiguous();
+    x->q = as(q, at::kHalf);
+    x->k = as(k, at::kHalf);
   } else {
     x->q = as(q, at::kBFloat16);
     x->k = as(k, at::kBFloat16);
@@ -650,7 +653,7 @@ struct RegimeTest {
 };
 
 bool plain32(const Tensor& t) {
-  return t.scalar_type() == at::kFloat && t.is_contiguous() && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
+  return t.scalar_type() == at::kFloat && t.is_contiguous() && !lazy(t) && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
 }
 
 // the same tests with library operations, for gates of other types or layouts
