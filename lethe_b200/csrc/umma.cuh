@@ -105,9 +105,13 @@ __device__ __forceinline__ void mbar_wait_warp(uint64_t* bar, uint32_t parity, c
 // kernel here triggers only after its own wait, so when a kernel starts, everything older than its
 // immediate predecessors is complete: before the wait it may read anything except what those write.
 // Calls can be cut into kernels and ranges of chunks, so which kernels these are depends on the
-// caller.  The kernels therefore read, before they wait, only the caller's tensors and records of
-// prepare, behind which another kernel of the same chunks always comes first (prepare, scan, output;
-// prepare, scan input, adjoint scan, main).
+// caller.  The kernels therefore read, before they wait, only the caller's tensors and what prepare
+// writes - its records, and the normalised q and k, which the output and main kernels read through
+// tensor maps in the place of the caller's - behind which another kernel of the same chunks always
+// comes first (prepare, scan, output; prepare, scan input, adjoint scan, main; either scan may have
+// the kernel beside it in it).  The main kernels behind an adjoint scan of the same call read what is
+// older than that scan, and the normalisation's VJP behind a backward (LETHE_L2_EARLY) reads q and k,
+// which are older than that call.
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
