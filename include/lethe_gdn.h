@@ -83,7 +83,11 @@ typedef struct LetheGdnArgs {
   /* Profiling aid: 0 runs every kernel of the call.  Otherwise bit i selects kernel i of the call  */
   /* (forward: 1 prepare, 2 state scan, 4 output; backward: 1 scan input, 2 adjoint scan,           */
   /* 4 Stage B, 8 WY VJP); a partial call relies on the records left by an earlier full call (names   */
-  /* and layout: csrc/gdn_common.cuh).  Backward with the delta term, records read: 1: A (of TA), W,   */
+  /* and layout: csrc/gdn_common.cuh) - one with lean 0, where a scan of the full call would be joint  */
+  /* with the kernel beside it (lethe_gdn_joint_scans): a lean full call then leaves no RB behind the  */
+  /* adjoint and, with lean 2, no Hc behind the forward.  A partial call that has one of the two       */
+  /* kernels but not the other runs it by itself, lean or not.                                        */
+  /* Backward with the delta term, records read: 1: A (of TA), W,                                      */
   /* QG (channel-wise gate); 2: P, AD, RB; 4: A, VN, Hc, DH; 8: T (of TA), W and U (the WY factors     */
   /* w = T (beta gamma k) and u = T (beta v), which the gradient of the inverse is formed with), and   */
   /* DV2, DW, DKB, DGB, RB as bit 4 left them.  A caller that lays records down for 8 alone has to     */
@@ -126,7 +130,8 @@ typedef struct LetheGdnArgs {
   uint32_t k_channels;
   /* 1: the call leaves only results in memory, and in the workspaces what its own later kernels and, after a forward, */
   /* the backward read.  2 (forward only): not even the latter, no backward can follow.  0: also intermediates that a  */
-  /* caller may want to look at (dv2, dw).                                                                             */
+  /* caller may want to look at (dv2, dw), and whatever a partial call (kernel_mask) on the same workspaces may read:  */
+  /* a lean call may do the work of two kernels in one, and what goes between them is then not written.                */
   uint32_t lean;
   /* Forward.  l2_eps > 0: q and k are normalised as they are read, x rsqrt(sum x^2 + l2_eps) per token-head, in fp32   */
   /* and rounded once to fp16 (what lethe_gdn_l2norm_qk does, without its pass over memory).  q_norm, k_norm take the     */

@@ -137,7 +137,8 @@ def forward_into(buf: GdnBuffers, q, k, v, g, beta, h0, scale: float, kernel_mas
     ``bh_range = (begin, count)`` restricts the call to those (batch, head) pairs (count 0: all),
     ``c_range = (begin, count)`` to those 64-token chunks of every sequence (the scans carry their state from
     one range to the next: forward ranges in ascending order).  ``lean``: workspace records that no kernel of the
-    forward or the backward reads are not written."""
+    forward or the backward reads are not written (2: nor what only a backward reads); calls with ``kernel_mask`` that go on
+    from a full one need it made without ``lean``."""
     _same_device(q, k, v, g, beta, h0, b_gate, w_gate, buf.saved)
     a = _Args(dims=buf.dims, scale=scale, q=_ptr(q), k=_ptr(k), v=_ptr(v), g=_ptr(g), beta=_ptr(beta),
               h0=_ptr(h0), o=_ptr(buf.o), hT=_ptr(buf.hT), saved=_ptr(buf.saved),
@@ -151,7 +152,7 @@ def backward_into(buf: GdnBuffers, q, k, v, g, beta, h0, do, dhT, scale: float, 
                   b_gate=None, w_gate=None, bh_range: tuple[int, int] = (0, 0),
                   c_range: tuple[int, int] = (0, 0), lean: bool = False) -> None:
     """Enqueue the backward kernels; gradients land in ``buf.dq`` ... ``buf.dh0`` (``buf.db`` / ``buf.dw``
-    for the per-channel gates of buffers made with ``delta=2``)."""
+    for the per-channel gates of buffers made with ``delta=2``).  ``kernel_mask``, ranges and ``lean`` as in the forward."""
     _same_device(q, k, v, g, beta, h0, do, dhT, b_gate, w_gate, buf.saved)
     a = _Args(dims=buf.dims, scale=scale, q=_ptr(q), k=_ptr(k), v=_ptr(v), g=_ptr(g), beta=_ptr(beta),
               h0=_ptr(h0), d_o=_ptr(do), dhT=_ptr(dhT), dq=_ptr(buf.dq), dk=_ptr(buf.dk), dv=_ptr(buf.dv),
