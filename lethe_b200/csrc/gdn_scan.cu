@@ -246,8 +246,8 @@ scan_kernel(const Problem p) {
 // 0.39 / 0.39, 16 0.53 / 0.51, 32 0.79 / 0.79; fetching R and storing the record between the products pays for the additions).
 //
 // Bound by the matrix pipe (17 cycles for a product of 16 x 8 x 16 per SM quarter, so 0.14 us per 8 columns) behind 0.25 us of
-// barrier, operand loads and P's way to registers: 0.39 us a step with 8 columns, 0.51 with 16, 0.79 with 32; tcgen05 took 0.69
-// with 16 (same measure: slope over the number of chunks, L2 cold) and takes 0.72 with 64.  With the fetch behind the products
+// barrier, operand loads and P's way to registers: 0.38 us a step with 8 columns, 0.48 with 16, 0.79 with 32; tcgen05 took 0.69
+// with 16 (same measure: slope over the number of chunks, L2 cold) and takes 0.68 with 64.  With the fetch behind the products
 // instead of between them 16 columns took 0.62, with four warps of kM = 2 at 32 columns the step is 0.92.
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t* r) {
@@ -538,15 +538,15 @@ scan_mma_kernel(const Problem p) {
 // of a record atom, so every access is a full line.  What is on the way from HBM decides the speed: a thread copies the R of
 // the next kDepth chunks to shared memory behind its own back.  (As loads to registers, 16 or 8 of them, a wait for one was a wait for
 // all that shared its scoreboard, six for a warp, and a step took 0.6 us: 36 pairs x 94 and 188 chunks, d_v = 64, 55 and 114 us, now
-// 18 and 40; 64 pairs x 64, d_v = 128, 59, now 46.)  32 slots, one CTA per SM, for whole sequences of more than 16
-// chunks (40, 48 and 80 pairs x 64, d_v = 128, us, 8 / 16 / 32: 36 / 39 / 33, 46 / 39 / 36, 63 / 62 / 57).  Shorter ones do not fill that ring,
-// and with many pairs one CTA per SM is a long row of nearly empty rounds: 16 slots, and for 8 chunks at most and more CTAs than two per
-// SM 8, four CTAs per SM (1024 pairs x 8, d_v = 64, forward, three / four: 224 / 254, but with 64 key channels 169 / 151, and no difference
-// from d_v = 128 on).  SSD, d_v = 128, us, forward and
-// backward, registers as above / always 32 slots / now: 256 pairs x 1 28 and 38 / 38 and 50 / 26 and 36; 1024 x 1 81 and 103 / 120 and 151 / 77
-// and 95; 256 x 4 58 and 83 / 70 and 95 / 58 and 82; d_v = 64, 1024 x 8 234 and 348 / 239 and 359 / 224 and 348.  A range of chunks (captured step) has chunk kernels beside it, which need the room:
-// 16 while two CTAs per SM hold the whole grid, 8 beyond (captured step, SSD, 16 pairs x 32, d_v = 128, 8 / 16 / 32 88 / 78 / 84; GLA, 64 pairs x
-// 64, 603 / 613 / 625).
+// 18 and 40; 64 pairs x 64, d_v = 128, 59, now 46.)
+// Slots, whole sequences: 32, one CTA per SM, for more than 16 chunks (40, 48 and 80 pairs x 64, d_v = 128, us, 8 / 16 / 32: 36 / 39 / 33, 46 / 39 /
+// 36, 63 / 62 / 57).  Shorter ones do not fill that ring, and with many pairs one CTA per SM is a long row of nearly empty rounds: 16 slots, and
+// for 8 chunks at most and more CTAs than two per SM 8, four CTAs per SM (three in the forward over 5 to 8 chunks with d_v = 64: 1024 pairs
+// x 8, three / four 224 / 254; with 64 key channels 169 / 151, and no difference at d_v = 128).  SSD, d_v = 128, us, forward and backward,
+// registers as above / always 32 slots / now: 256 pairs x 1 28 and 38 / 38 and 50 / 26 and 36; 1024 x 1 81 and 103 / 120 and 151 / 77 and 95; 256 x
+// 4 58 and 83 / 70 and 95 / 58 and 82; d_v = 64, 1024 x 8 234 and 348 / 239 and 359 / 224 and 348.
+// A range of chunks (captured step) has chunk kernels beside it, which need the room: 16 while two CTAs per SM hold the whole grid, 8 beyond
+// (captured step, SSD, 16 pairs x 32, d_v = 128, 8 / 16 / 32 88 / 78 / 84; GLA, 64 pairs x 64, 603 / 613 / 625).
 // R / Rb and the state records are 128-row tile images, of which rows from Kw on are neither read nor written.
 // Grid: (V / 64 atoms x Kw / 32 row blocks, pairs) x 256 threads.
 // ---------------------------------------------------------------------------------------------
@@ -672,19 +672,21 @@ int launch_scan(const Problem& p, bool adjoint, cudaStream_t st, const CUtensorM
     return three ? launch_scan_nodelta<8, 3>(p, adjoint, st) : launch_scan_nodelta<8, 4>(p, adjoint, st);
   }
   // Warp-level products or tcgen05 (the same bits): by the whole problem, since calls on ranges of its pairs run beside one another.
-  // The line is where 16 columns no longer give every CTA an SM of its own.  Beyond it 32 columns are the shorter scan (alone, us,
-  // 32 / 64 columns, 64 chunks, d_v = 64: 64 pairs 63 / 76; d_v = 128: 20 61 / 66, 32 63 / 70) and in calls that repeat on the same
-  // inputs (32 pairs, d_v = 128, forward over 250 chunks 814 / 825; training step d_v = 64, 64 x 32 311 / 328, 48 x 128 889 / 914), but not
-  // where the inputs change from call to call, since P is read twice as often: the same forward 873 / 857.
+  // The line is where 16 columns no longer give every CTA an SM of its own: up to it they are the shorter scan (alone, us, 16 / 32 / 64
+  // columns, 64 chunks, d_v = 64, 37 pairs 43 / 61 / 59; d_v = 128, 18 pairs 41 / 60 / 58), beyond it not (38 pairs 74 / 60 / 59; 20 pairs
+  // 72 / 60 / 58).  There 32 and 64 are alike while 32 have an SM each and a little beyond (forward and backward, 32 / 64: d_v = 64, 38 x 64 172 and
+  // 222 / 170 and 225, 64 x 64 244 and 324 / 246 and 329; d_v = 128, 32 x 64 177 and 246 / 179 and 246), and 64 the better the more there is
+  // to read, since P is read half as often (32 x 250 639 and 981 / 619 and 919; 64 x 64 334 and 475 / 297 and 439).
   if ((p.V / 16) * p.B * p.H > sms) return launch_scan_wide(p, adjoint, st);
   const int c8 = (p.V / 8) * p.nbh;            // CTAs with 8 columns each
   if (p.cn < p.NT) {
     // A range of the sequences (captured step): chunk kernels of another range run beside the scan, and an SM that a scan CTA sits
-    // on is lost to them.  Few CTAs then count for more than a short step.  Captured step, us, 8 / 32 / 64 columns, d_v = 64, pairs x
-    // chunks: 8 x 32 66 / 86 / 90, 12 x 32 98 / 96 / 107, 12 x 64 154 / 168 / 174, 14 x 32 115 / 100 / 113, 16 x 32 126 / 105 / 117, 24 x 64 277 /
-    // 254 / 276, 32 x 64 351 / 317 / 344; d_v = 128: 3 x 16 50 / 60 / 70, 6 x 32 75 / 87 / 96, 7 x 32 94 / 88 / 97, 10 x 32 120 / 102 / 111, 16 x 32
-    // 171 / 133 / 138; the same with the channel-wise gate 207 / 174 / 161: its chunk kernels would be better off with 64, which this
-    // rule has not been fitted to (64 columns were out of the question here while their bits differed).
+    // on is lost to them.  Few CTAs then count for more than a short step.  Captured step, us, 8 / 16 / 32 / 64 columns, pairs x chunks, d_v = 64:
+    // 4 x 32 62 / 68 / 86 / 96, 8 x 32 71 / 76 / 89 / 98, 12 x 32 101 / 94 / 98 / 112, 16 x 32 129 / 116 / 107 / 121, 24 x 64 278 / 250 / 254 /
+    // 267, 32 x 64 347 / 321 / 316 / 327, 64 x 64 639 / 573 / 567 / 542; d_v = 128: 6 x 32 83 / 78 / 90 / 102, 10 x 32 121 / 105 / 106 / 117, 16 x 32
+    // 173 / 152 / 135 / 141, 8 x 128 274 / 249 / 302 / 311, 64 x 64 964 / 838 / 814 / 758; channel-wise, d_v = 128: 3 x 128 184 / 206 / 258 / 251, 16 x
+    // 32 210 / 189 / 179 / 167.  So 16 and 64 columns each have a range of sizes where they would be the better ones; the rule knows 8 and
+    // 32 only.
     return 3 * c8 <= 2 * sms ? launch_scan_few<8>(p, adjoint, st) : launch_scan_few<32>(p, adjoint, st);
   }
   // A whole sequence: the fewest columns with which every CTA has an SM of its own.  Chain of a step, us, 8 / 16 / 32 columns, d_v = 64:

@@ -173,13 +173,8 @@ def default_cut(gate: int, V: int, NT: int, BH: int, sms: int) -> int:
     the ``BH`` (batch, head) pairs takes the same number; half where that is nothing or everything.  ``sms``: SMs.
 
     That unit was a wave of the chunk kernels when they ran one CTA per chunk.  They are persistent now, with one
-    to four CTAs per SM, and no wave ends at the cut: the unit is where the cut lies, not a reason for it.  Replay
-    in us, not cut / cut at half / cut here, BH x NT: scalar gate, d_v = 64: 8 x 32 66 / 66 / 66, 16 x 32 105 / 111
-    / 105, 36 x 47 255 / 266 / 262, 32 x 64 308 / 310 / 317, 64 x 64 571 / 554 / 554; d_v = 128: 16 x 32 136 / 141 /
-    134, 64 x 64 721 / 752 / 752; channel-wise, d_v = 64: 16 x 32 141 / 151 / 138; d_v = 128: 16 x 32 168 / 180 /
-    175, 32 x 64 518 / 525 / 524, 64 x 128 1825 / 1861 / 1860; without the delta term, d_v = 128, 64 x 64: scalar
-    460 / 467 / 467, channel-wise 636 / 628 / 629.  So a cut is worth 3 % at best and costs up to 4 %: a whole
-    sequence has the shorter scan step.  The rule has not been fitted to that yet."""
+    to four CTAs per SM, and no wave ends at the cut: the unit is where the cut lies, not a reason for it.  ``step_is_cut``
+    has what a cut here is worth."""
     if NT < 8:
         return 0
     per_sm = 2 if (gate != GATE_CHANNEL and V == 64) else 1
@@ -195,9 +190,9 @@ def default_cut(gate: int, V: int, NT: int, BH: int, sms: int) -> int:
 def default_bwd_cuts(gate: int, V: int, delta: bool, NT: int, BH: int, sms: int, cut: int) -> tuple:
     """Where the backward is cut: at the forward's cut, and - scalar gate, d_v = 64, two units of ``default_cut`` at
     most - once more at half a unit, so that the last main kernel, which has nothing to hide behind, is short.
-    At B=2, H=8, L=2048 that cut, placed when Stage B and the WY VJP were kernels of their own, is worth nothing
-    any more: 105 us with it, 103 without.  Elsewhere a second cut at half of the first costs 1 to
-    9 % (d_v = 128, 512 chunks: 144 -> 153; channel-wise 193 -> 198; 4096 chunks 574 -> 587)."""
+    That cut was placed when Stage B and the WY VJP were kernels of their own.  Replay in us without / with it, where it is
+    made: 16 x 32 107 / 107, 8 x 64 113 / 122, 4 x 128 147 / 147.  Elsewhere a second cut at half of the first costs 1 to
+    9 % (d_v = 128, 16 x 32 136 / 147; channel-wise 179 / 189; 64 x 64 763 / 797).  So it is worth nothing any more."""
     if not cut:
         return ()
     two_per_sm = gate != GATE_CHANNEL and V == 64 and delta
@@ -210,10 +205,17 @@ def default_bwd_cuts(gate: int, V: int, delta: bool, NT: int, BH: int, sms: int,
 def step_is_cut(gate: int, delta: bool, NT: int, BH: int, sms: int) -> bool:
     """Whether ``GdnStepGraph`` cuts the sequences at all when it is not told.  A cut adds launches and gives up the scan of a whole
     sequence: without the delta term, and with the channel-wise gate while a CTA of its kernels has one chunk, that costs more than
-    the overlap gives.  Replay in us, cut / not, BH x NT: SSD, d_v = 64, 4 x 32 35 / 27, 16 x 32 56 / 47, 64 x 16 99 / 84, 36 x 47 131 / 127;
-    d_v = 128, 16 x 32 79 / 71, 32 x 64 234 / 223, 64 x 64 448 / 439; GLA 4 x 32 43 / 31, 16 x 32 85 / 77, 64 x 16 147 / 131, d_v = 128 32 x 64
-    320 / 311; KDA 1 x 32 66 / 58, 4 x 32 66 / 60, d_v = 128 16 x 32 173 / 165, 3 x 128 178 / 197; scalar 4 x 32 58 / 55, 16 x 32 103 / 102,
-    8 x 128 188 / 228.  From 4096 chunks on the 2 to 4 % that are left without the delta term are not worth another schedule."""
+    the overlap gives.  Replay in us, not cut / cut, BH x NT: SSD, d_v = 64, 4 x 32 33 / 41, 16 x 32 53 / 61, 64 x 16 91 / 98, 36 x 47 131 / 136;
+    d_v = 128, 16 x 32 74 / 85, 32 x 64 231 / 240, 64 x 64 445 / 463; GLA 4 x 32 39 / 53, 16 x 32 82 / 91, 64 x 16 132 / 154, d_v = 128 32 x 64
+    318 / 326; KDA 4 x 32 73 / 76, d_v = 128, 3 x 128 202 / 187, 4 x 64 125 / 129, 8 x 37 113 / 134, 16 x 32 171 / 179, 16 x 64 285 / 293; d_v = 64, 4 x 128
+    209 / 173, 16 x 128 451 / 513; scalar 4 x 16 51 / 61, 4 x 32 64 / 62, 4 x 64 94 / 87, 4 x 256 324 / 273, 8 x 32 77 / 72, 8 x 128 231 / 192, 16 x 32
+    109 / 107, 16 x 128 333 / 377, 36 x 47 260 / 264, 64 x 64 553 / 544; d_v = 128, 4 x 128 196 / 166, 8 x 32 86 / 92, 8 x 128 261 / 304, 16 x 32 138 / 136,
+    64 x 64 714 / 763.
+
+    The rule goes by the number of chunks in all, and is coarser than that.  A cut gains up to 17 % where the pairs are so few that both
+    scans keep 8 columns per CTA (up to 8 pairs of d_v = 64, 4 of 128) and the sequences have 32 chunks or more, where the serial scan is
+    what there is to hide; elsewhere it gives 2 % at best and costs up to 19 %.  The rule still cuts there - every scalar gate with the delta term, the
+    channel-wise one from two chunks per SM on, and SSD from 4096 chunks on - as it did before whole sequences had shorter scans."""
     if not delta:
         return NT * BH >= 4096
     return gate != GATE_CHANNEL or NT * BH >= 2 * sms
@@ -227,8 +229,9 @@ def joint_scans(gate: int, V: int, delta: bool, BH: int, sms: int, NT: int = 64)
 
 def step_is_chain(gate: int, V: int, delta: bool, BH: int, sms: int, NT: int = 64) -> bool:
     """Whether one chain of whole calls is the faster captured step: where forward and backward take the scans that have the output,
-    or their input, beside them (``joint_scans``).  Replay in us, overlapped / chain, BH x NT: KDA, d_v = 64, 64 x 16
-    229 / 217, 64 x 64 801 / 766; d_v = 128 32 x 64 515 / 498, 64 x 64 960 / 868; GLA, d_v = 128, 32 x 64 (not this) 311 / 319, 64 x 64 606 / 549."""
+    or their input, beside them (``joint_scans``).  Replay in us, overlapped with a cut / without / chain, BH x NT: KDA, d_v = 64, 64 x 16
+    237 / 227 / 227, 64 x 64 799 / 791 / 777; d_v = 128 32 x 64 514 / 505 / 511, 64 x 64 975 / 923 / 904; GLA, d_v = 128, 64 x 16 181 / 173 / 164, 64 x 64
+    613 / 609 / 562, 32 x 64 (not this) 326 / 318 / 326."""
     return joint_scans(gate, V, delta, BH, sms, NT) == 3
 
 
