@@ -95,8 +95,8 @@ int32_t* status_word(int dev) {
 // memory that does not hold the values: a negated view, a tensor of zeros without storage
 bool lazy(const Tensor& t) { return t.is_neg() || t._is_zerotensor(); }
 Tensor as(const Tensor& t, at::ScalarType dt) {
-  const Tensor r = t.scalar_type() == dt ? t : t.to(dt);
-  return (lazy(r) ? r.clone() : r).contiguous();
+  if (t.scalar_type() != dt) return t.to(dt).contiguous();      // (writes them out)
+  return lazy(t) ? t.clone().contiguous() : t.contiguous();
 }
 Tensor as32(const Tensor& t) { return t.defined() ? as(t, at::kFloat) : t; }
 // a gate per channel is read through a tensor map, which wants its start on a 16-byte boundary
