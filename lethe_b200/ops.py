@@ -231,8 +231,11 @@ def step_is_chain(gate: int, V: int, delta: bool, BH: int, sms: int, NT: int = 6
     """Whether one chain of whole calls is the faster captured step: where forward and backward take the scans that have the output,
     or their input, beside them (``joint_scans``).  Replay in us, overlapped with a cut / without / chain, BH x NT: KDA, d_v = 64, 64 x 16
     237 / 227 / 227, 64 x 64 799 / 791 / 777; d_v = 128 32 x 64 514 / 505 / 511, 64 x 64 975 / 923 / 904; GLA, d_v = 128, 64 x 16 181 / 173 / 164, 64 x 64
-    613 / 609 / 562, 32 x 64 (not this) 326 / 318 / 326."""
-    return joint_scans(gate, V, delta, BH, sms, NT) == 3
+    613 / 609 / 562, 32 x 64 (not this) 326 / 318 / 326.
+
+    Not below 8 chunks, where nothing is ever cut: the overlap hides more than the launches cost (without a cut / chain: KDA, d_v = 64, 38 x 7 84 /
+    92, 100 x 1 59 / 62; d_v = 128, 100 x 2 98 / 104; GLA, d_v = 64, 100 x 2 49 / 57; d_v = 128, 46 x 4 55 / 61, 256 x 6 255 / 279)."""
+    return NT >= 8 and joint_scans(gate, V, delta, BH, sms, NT) == 3
 
 
 class GdnStepGraph:
@@ -273,7 +276,7 @@ class GdnStepGraph:
         ranges = [(bounds[i], bounds[i + 1] - bounds[i]) for i in range(groups)]
         self.groups = groups
         if pipeline is None:
-            pipeline = groups == 1 and not (cut is None and bwd_cuts is None and self._joint_scans(buf, BH, NT, dev) == 3)
+            pipeline = groups == 1 and not (cut is None and bwd_cuts is None and self._is_chain(buf, BH, NT, dev))
         self.pipeline = bool(pipeline) and groups == 1
         if cut is None:
             cut = self._default_cut(buf, NT, BH, dev)
@@ -415,6 +418,11 @@ class GdnStepGraph:
     def _joint_scans(buf, BH: int, NT: int, dev) -> int:
         sms = torch.cuda.get_device_properties(dev).multi_processor_count
         return joint_scans(buf.dims.gate, buf.dims.V, buf.dims.delta != 0, BH, sms, NT)
+
+    @staticmethod
+    def _is_chain(buf, BH: int, NT: int, dev) -> bool:
+        sms = torch.cuda.get_device_properties(dev).multi_processor_count
+        return step_is_chain(buf.dims.gate, buf.dims.V, buf.dims.delta != 0, BH, sms, NT)
 
     @staticmethod
     def _default_bwd_cuts(buf, NT: int, BH: int, dev, cut: int) -> tuple:

@@ -1,5 +1,5 @@
-"""CPU: which scans the library launches with the kernel beside them in one, and that a captured step is planned by that and nothing
-else (``lethe_gdn_joint_scans``)."""
+"""CPU: which scans the library launches with the kernel beside them in one, and that a captured step is planned by what it says
+(``lethe_gdn_joint_scans``)."""
 import ctypes
 from types import SimpleNamespace
 
@@ -22,7 +22,7 @@ def test_a_captured_step_is_one_chain_where_both_scans_are_joint(monkeypatch, ga
     for NT in (1, 2, 4, 8, 64):
         for BH in list(range(1, 200)) + [256, 512, 1024]:
             bits = joint(gate, V, delta, BH, NT)
-            assert ops.step_is_chain(gate, V, delta != 0, BH, B200_SMS, NT) == (bits == 3)
+            assert ops.step_is_chain(gate, V, delta != 0, BH, B200_SMS, NT) == (bits == 3 and NT >= 8)      # (shorter ones are never cut)
             buf = SimpleNamespace(dims=SimpleNamespace(gate=gate, V=V, delta=delta))
             assert ops.GdnStepGraph._joint_scans(buf, BH, NT, None) == bits
             if gate != ops.GATE_CHANNEL:
