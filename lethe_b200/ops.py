@@ -212,13 +212,17 @@ def step_is_cut(gate: int, delta: bool, NT: int, BH: int, sms: int) -> bool:
     109 / 107, 16 x 128 333 / 377, 36 x 47 260 / 264, 64 x 64 553 / 544; d_v = 128, 4 x 128 196 / 166, 8 x 32 86 / 92, 8 x 128 261 / 304, 16 x 32 138 / 136,
     64 x 64 714 / 763.
 
-    The rule goes by the number of chunks in all, and is coarser than that.  A cut gains up to 17 % where the pairs are so few that both
+    Few pairs with long sequences are cut with the channel-wise gate, too: the serial scan is most of their step.  KDA, not cut / cut, d_v = 64:
+    1 x 64 94 / 92, 1 x 256 255 / 239, 2 x 96 135 / 121, 3 x 64 113 / 96, 3 x 96 138 / 141, 4 x 48 100 / 90, 4 x 64 115 / 102, 4 x 72 121 / 127, but 6 x 48 104 /
+    113, 8 x 32 92 / 101, 2 x 32 70 / 74; d_v = 128: 1 x 192 213 / 194, 2 x 128 172 / 151, 3 x 48 92 / 89, 4 x 40 100 / 102, 4 x 56 117 / 109.
+
+    Otherwise the rule goes by the number of chunks in all, and is coarser than its figures.  A cut gains up to 17 % where the pairs are so few that both
     scans keep 8 columns per CTA (up to 8 pairs of d_v = 64, 4 of 128) and the sequences have 32 chunks or more, where the serial scan is
     what there is to hide; elsewhere it gives 2 % at best and costs up to 19 %.  The rule still cuts there - every scalar gate with the delta term, the
     channel-wise one from two chunks per SM on, and SSD from 4096 chunks on - as it did before whole sequences had shorter scans."""
     if not delta:
         return NT * BH >= 4096
-    return gate != GATE_CHANNEL or NT * BH >= 2 * sms
+    return gate != GATE_CHANNEL or NT * BH >= 2 * sms or (BH <= 4 and NT >= 40)
 
 
 def joint_scans(gate: int, V: int, delta: bool, BH: int, sms: int, NT: int = 64) -> int:

@@ -48,3 +48,9 @@ F, A = 1, 2      # forward, adjoint
     (128, 0, 64, 1, 1, F | A), (64, 0, 128, 1, 1, F | A), (128, 0, 128, 1, 1, A), (128, 1, 148, 1, 1, F | A), (64, 1, 38, 1, 1, F | A)])
 def test_short_sequences_of_many_pairs(V, delta, BH, NT, lean, bits):
     assert joint(ops.GATE_CHANNEL, V, delta, BH, NT, lean) == bits
+
+
+@pytest.mark.parametrize("BH,NT,cut", [(1, 39, False), (1, 40, True), (2, 128, True), (4, 40, True), (4, 64, True), (5, 48, False), (8, 32, False), (5, 60, True)])
+def test_few_long_sequences_with_the_channel_gate_are_cut(BH, NT, cut):
+    assert ops.step_is_cut(ops.GATE_CHANNEL, True, NT, BH, B200_SMS) == cut
+    assert not ops.step_is_cut(ops.GATE_CHANNEL, False, NT, BH, B200_SMS)
