@@ -539,12 +539,13 @@ scan_mma_kernel(const Problem p) {
 // the next kDepth chunks to shared memory behind its own back.  (As loads to registers, 16 or 8 of them, a wait for one was a wait for
 // all that shared its scoreboard, six for a warp, and a step took 0.6 us: 36 pairs x 94 and 188 chunks, d_v = 64, 55 and 114 us, now
 // 18 and 40; 64 pairs x 64, d_v = 128, 59, now 46.)
-// Slots, whole sequences: 32, one CTA per SM, for more than 16 chunks (40, 48 and 80 pairs x 64, d_v = 128, us, 8 / 16 / 32: 36 / 39 / 33, 46 / 39 /
-// 36, 63 / 62 / 57).  Shorter ones do not fill that ring, and with many pairs one CTA per SM is a long row of nearly empty rounds: 16 slots, and
-// for 8 chunks at most and more CTAs than two per SM 8, four CTAs per SM (three in the forward over 5 to 8 chunks with d_v = 64: 1024 pairs
-// x 8, three / four 224 / 254; with 64 key channels 169 / 151, and no difference at d_v = 128).  SSD, d_v = 128, us, forward and backward,
-// registers as above / always 32 slots / now: 256 pairs x 1 28 and 38 / 38 and 50 / 26 and 36; 1024 x 1 81 and 103 / 120 and 151 / 77 and 95; 256 x
-// 4 58 and 83 / 70 and 95 / 58 and 82; d_v = 64, 1024 x 8 234 and 348 / 239 and 359 / 224 and 348.
+// Slots, whole sequences: 32, one CTA per SM, where that holds the whole grid (in pairs on the first free SMs they share their intake:
+// captured step, 16 pairs x 8, d_v = 64, us, 16 / 32 30.6 / 28.8) and for more than 16 chunks (40, 48 and 80 pairs x 64, d_v = 128, 8 / 16 /
+// 32: 36 / 39 / 33, 46 / 39 / 36, 63 / 62 / 57).  Shorter ones do not fill that ring, and with many pairs one CTA per SM is a long row of nearly
+// empty rounds: 16 slots, and for 8 chunks at most and more CTAs than two per SM 8, four CTAs per SM (three in the forward over 5 to 8
+// chunks with d_v = 64: 1024 pairs x 8, three / four 224 / 254; with 64 key channels 169 / 151, and no difference at d_v = 128).  SSD, d_v =
+// 128, forward and backward, registers as above / always 32 slots / now: 256 pairs x 1 28 and 38 / 38 and 50 / 26 and 36; 1024 x 1 81 and
+// 103 / 120 and 151 / 77 and 95; 256 x 4 58 and 83 / 70 and 95 / 58 and 82; d_v = 64, 1024 x 8 234 and 348 / 239 and 359 / 224 and 348.
 // A range of chunks (captured step) has chunk kernels beside it, which need the room: 16 while two CTAs per SM hold the whole grid, 8 beyond
 // (captured step, SSD, 16 pairs x 32, d_v = 128, 8 / 16 / 32 88 / 78 / 84; GLA, 64 pairs x 64, 603 / 613 / 625).
 // R / Rb and the state records are 128-row tile images, of which rows from Kw on are neither read nor written.
@@ -666,7 +667,7 @@ int launch_scan(const Problem& p, bool adjoint, cudaStream_t st, const CUtensorM
   if (!p.delta) {
     const int ctas = (p.V / 64) * (p.Kw / 32) * p.nbh, n = p.cn;
     if (n < p.NT) return ctas <= 2 * sms ? launch_scan_nodelta<16>(p, adjoint, st) : launch_scan_nodelta<8>(p, adjoint, st);
-    if (n > 16 || (n > 8 && ctas <= sms)) return launch_scan_nodelta<32>(p, adjoint, st);
+    if (n > 16 || ctas <= sms) return launch_scan_nodelta<32>(p, adjoint, st);
     if (n > 8 || ctas <= 2 * sms) return launch_scan_nodelta<16>(p, adjoint, st);
     const bool three = !adjoint && n > 4 && p.V == 64 && p.Kw == kK;
     return three ? launch_scan_nodelta<8, 3>(p, adjoint, st) : launch_scan_nodelta<8, 4>(p, adjoint, st);
