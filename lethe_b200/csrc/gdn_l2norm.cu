@@ -122,7 +122,7 @@ l2norm_qk_kernel(const L2Problem p) {
 #pragma unroll
   for (int u = 0; u < kPieces; ++u) load8<IN>(p.x[t], idx[u], x[u]);
   if (BACKWARD) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");      // (x is older than the kernel that makes dy: LETHE_L2_EARLY)
+    asm volatile("griddepcontrol.wait;" ::: "memory");      // (x is older than the kernel that makes dy: LETHE_L2_EARLY; dx may lie in what that kernel's scratch was)
 #pragma unroll
     for (int u = 0; u < kPieces; ++u) load8_16(p.dy[t], idx[u], dy[u], p.norm_f16);
   }

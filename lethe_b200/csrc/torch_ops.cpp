@@ -189,17 +189,49 @@ LetheGdnArgs base_args(const Problem& p, const Operands& x, void* saved, size_t 
   return a;
 }
 
-// One allocation for what a call needs for itself; pieces on 1024-byte boundaries.
-struct Slab {
-  size_t bytes = 0;
-  Tensor t;
-  size_t piece(size_t n) {
-    const size_t at = bytes;
-    bytes += (n + 1023) / 1024 * 1024;
-    return at;
+// What a backward needs for itself, by how long: the library's scratch and the converted gradient of o until its kernels are launched,
+// the gradients of normalised rows until their VJP is, the rest until the results are made.  One allocation for all of it where that is
+// small (an allocation costs the host a microsecond), one for each otherwise, given back when it is done with: a call of hundreds
+// of megabytes then peaks no higher than its scratch and its results ask for.  Pieces on 1024-byte boundaries.
+class Slab {
+ public:
+  enum Until { kKernels, kRows, kEnd, kGroups };
+  struct Piece {
+    Until until = kEnd;
+    size_t at = 0;
+  };
+  Piece piece(Until until, size_t n) {
+    const Piece p{until, bytes_[until]};
+    bytes_[until] += (n + 1023) / 1024 * 1024;
+    return p;
   }
-  void make(const at::TensorOptions& o) { t = workspace(bytes, o); }
-  void* at(size_t offset) const { return static_cast<char*>(t.data_ptr()) + offset; }
+  void make(const at::TensorOptions& o) {
+    const size_t all = bytes_[kKernels] + bytes_[kRows] + bytes_[kEnd];
+    if (all <= kOne) {
+      t_[kKernels] = workspace(all, o);
+      char* base = static_cast<char*>(t_[kKernels].data_ptr());
+      for (int i = 0; i < kGroups; base += bytes_[i++]) base_[i] = base;
+      return;
+    }
+    for (int i = 0; i < kGroups; ++i) {
+      if (!bytes_[i]) continue;
+      t_[i] = workspace(bytes_[i], o);
+      base_[i] = static_cast<char*>(t_[i].data_ptr());
+      own_ = true;
+    }
+  }
+  void* at(const Piece& p) const { return base_[p.until] + p.at; }
+  // what was for `until` is done with: on this stream, whose later kernels write it behind those that read it
+  void drop(Until until) {
+    if (own_) t_[until].reset();
+  }
+
+ private:
+  static constexpr size_t kOne = 16u << 20;
+  size_t bytes_[kGroups] = {};
+  char* base_[kGroups] = {};
+  Tensor t_[kGroups];
+  bool own_ = false;
 };
 
 struct Forward {
@@ -265,12 +297,15 @@ Grads run_backward(const Problem& p, const Operands& x, const Tensor& saved, con
   const bool cast_do = d_o_in.defined() && converts(d_o_in, at::kFloat), one = x.beta.defined() && p.delta == 1;
   const bool row_g = spread && p.gate == LETHE_GATE_SCALAR;
   Slab& s = r.slab;
-  s.piece(need);
-  const size_t at_do = cast_do ? s.piece(o_bytes) : 0, at_dq = p.l2 ? s.piece(bytes(x.q)) : 0, at_dk = p.l2 ? s.piece(bytes(x.k)) : 0;
-  const size_t at_dv = dv32 ? s.piece(o_bytes) : 0, at_dg = row_g ? s.piece(bytes(x.g)) : 0;
-  const size_t at_db = spread && one ? s.piece(bytes(x.beta)) : 0, at_dw = spread && one ? s.piece(bytes(x.beta)) : 0;
+  using P = Slab::Piece;
+  const P scratch = s.piece(Slab::kKernels, need);
+  const P at_do = cast_do ? s.piece(Slab::kKernels, o_bytes) : P();
+  const P at_dq = p.l2 ? s.piece(Slab::kRows, bytes(x.q)) : P(), at_dk = p.l2 ? s.piece(Slab::kRows, bytes(x.k)) : P();
+  const P at_dv = dv32 ? s.piece(Slab::kEnd, o_bytes) : P(), at_dg = row_g ? s.piece(Slab::kEnd, bytes(x.g)) : P();
+  const bool rows_b = spread && one;
+  const P at_db = rows_b ? s.piece(Slab::kEnd, bytes(x.beta)) : P(), at_dw = rows_b ? s.piece(Slab::kEnd, bytes(x.beta)) : P();
   s.make(x.v.options());
-  auto place = [&](Tensor& t, const Tensor& like, bool inside, size_t at) -> void* {
+  auto place = [&](Tensor& t, const Tensor& like, bool inside, const P& at) -> void* {
     if (inside) return s.at(at);
     t = at::empty_like(like);
     return t.data_ptr();
@@ -299,9 +334,10 @@ Grads run_backward(const Problem& p, const Operands& x, const Tensor& saved, con
   a.dq = r.p_dq; a.dk = r.p_dk; a.dv = r.p_dv; a.dg = r.p_dg; a.dh0 = ptr<float>(r.dh0);
   a.dbeta = r.p_dbeta; a.dbeta_write = r.p_dbeta_w;
   a.db_gate = ptr<float>(r.db); a.dw_gate = ptr<float>(r.dw);
-  a.scratch = s.at(0);
+  a.scratch = s.at(scratch);
   a.scratch_bytes = need;
   check(lethe_gdn_backward(&a, stream_of(x.q)));
+  s.drop(Slab::kKernels);
   return r;
 }
 
@@ -362,6 +398,7 @@ struct GdnBackward : public torch::autograd::Node {
       Tensor dq = at::empty_like(qc), dk = at::empty_like(kc);
       check(lethe_gdn_l2norm_qk_vjp(qc.data_ptr(), kc.data_ptr(), r.p_dq, r.p_dk, dq.data_ptr(), dk.data_ptr(),
                                      qc.numel() / p.K, static_cast<int32_t>(p.K), flags, kL2Eps, stream_of(qc)));
+      r.slab.drop(Slab::kRows);
       r.dq = dq;
       r.dk = dk;
     }
